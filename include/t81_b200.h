@@ -329,6 +329,13 @@ T81B200_API int64_t t81b200_t2_bytes(int64_t rows, int64_t cols);
  * same choice for the limb layout with the limb layout's cost). */
 T81B200_API int t81b200_prefers_streaming(int64_t M, int64_t N, int64_t K);
 T81B200_API int t81b200_pack_t2(const uint8_t *packed, int64_t rows, int64_t cols, uint8_t *t2, void *stream);
+/* One matrix in the decode-stream layout times any number of activation rows (token-major B, C): the streaming kernel
+ * up to 16 rows, tensor-core tiles beyond.  16-bit rows that start on 16-byte boundaries are read where they are;
+ * fp32 and unaligned ones are staged in the workspace (16-byte aligned, linear_t2_workspace_bytes for this very B). */
+T81B200_API size_t t81b200_linear_t2_workspace_bytes(const void *B, int b_dtype, int64_t ldb, int64_t M, int64_t N, int64_t K);
+T81B200_API int t81b200_linear_t2(const uint8_t *t2, const float *row_scale, const float *bias, void *C, int64_t M, const void *B,
+                                  int b_dtype, int64_t ldb, int c_dtype, int64_t ldc, int64_t N, int64_t K, float alpha, float beta,
+                                  void *workspace, size_t workspace_bytes, void *stream);
 /* gemm_trit_t2 for ONE matrix of a column-sharded Linear: t81b200_gemm_trit_peers (see there for peer_C, sync_local
  * and sync_slots) with the rank's rows given in the decode-stream layout; 1..16 rows of B, token-major. */
 T81B200_API int t81b200_gemm_trit_t2_peers(const uint8_t *t2, const float *row_scale, const float *bias, void *C, int64_t M,

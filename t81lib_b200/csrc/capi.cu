@@ -73,9 +73,10 @@ int gemv_trit_launch(const uint8_t *A, const float *row_scale, const void *X, in
 int gemm_trit_simt_launch(const uint8_t *A, const float *row_scale, const void *B, int b_dtype, int layout,
                           int64_t ldb, const float *bias, void *C, int c_dtype, int64_t ldc, int64_t M,
                           int64_t N, int64_t K, float alpha, float beta, cudaStream_t st);
-bool gemm_trit_tc_eligible(int b_dtype, int layout, int c_dtype, int64_t M, int64_t N, int64_t K);
-size_t gemm_trit_tc_workspace(int b_dtype, int layout, int c_dtype, int64_t M, int64_t N, int64_t K);
-int gemm_trit_tc_launch(const uint8_t *A, const float *row_scale, const void *B, int b_dtype, int layout,
+bool gemm_trit_tc_eligible(int64_t M, int64_t N, int64_t K);
+size_t gemm_trit_tc_scratch(const void *B, int b_dtype, int layout, int64_t ldb, int64_t N, int64_t K);
+size_t gemm_trit_tc_scratch_most(int b_dtype, int64_t N, int64_t K);
+int gemm_trit_tc_launch(int fmt, const uint8_t *A, const float *row_scale, const void *B, int b_dtype, int layout,
                         int64_t ldb, const float *bias, void *C, int c_dtype, int64_t ldc, int64_t M, int64_t N,
                         int64_t K, float alpha, float beta, void *workspace, size_t workspace_bytes,
                         cudaStream_t st, int n_peers, void *const *peer_C);
@@ -122,12 +123,21 @@ extern "C" int t81b200_device_available(void) { return check_device() == 0 ? 1 :
 
 static bool valid_dtype(int d) { return d == T81B200_F32 || d == T81B200_BF16 || d == T81B200_F16; }
 
+// The tensor-core kernel reads 16-bit token-major activations in place; everything else is staged in scratch memory
+// first, unless the problem is too small for that to pay (launch-bound either way: the general kernel takes it).
+static bool worth_staging(int64_t M, int64_t N, int64_t K) { return (double)M * (double)N * (double)K >= 1.6e7 && N >= 8; }
+
 extern "C" size_t t81b200_gemm_trit_workspace_bytes(int b_dtype, int layout, int c_dtype, int64_t M, int64_t N,
                                                     int64_t K) {
+    (void)c_dtype;
     if (M <= 0 || N <= 0 || K < 0) return 0;
-    if (!gemm_trit_tc_eligible(b_dtype, layout, c_dtype, M, N, K)) return 0;
-    return gemm_trit_tc_workspace(b_dtype, layout, c_dtype, M, N, K);
+    if (b_dtype == T81B200_BF16 && layout == T81B200_LAYOUT_NK) return 0;
+    if (!gemm_trit_tc_eligible(M, N, K) || !worth_staging(M, N, K)) return 0;
+    return gemm_trit_tc_scratch_most(b_dtype, N, K);
 }
+
+// Contractions up to this length always have a launch shape of the streaming kernel (16 fp32 rows of B included).
+constexpr int64_t kT2StreamingMaxK = 14336;
 
 static int gemm_trit_local(const uint8_t *A, const float *row_scale, const void *B, int b_dtype, int layout,
                            int64_t ldb, const float *bias, void *C, int c_dtype, int64_t ldc, int64_t M,
@@ -272,17 +282,18 @@ static int gemm_trit_local(const uint8_t *A, const float *row_scale, const void 
         ctx->waited = true;
     }
 
-    if (a_aligned && gemm_trit_tc_eligible(b_dtype, layout, c_dtype, M, N, K)) {
-        const size_t need = gemm_trit_tc_workspace(b_dtype, layout, c_dtype, M, N, K);
-        if (need > 0 && (!workspace || workspace_bytes < need))
-            return fail(T81B200_EWORKSPACE, "gemm_trit: workspace of %zu bytes needed, %zu given", need, workspace_bytes);
-        const int rc = gemm_trit_tc_launch(A, row_scale, B, b_dtype, layout, ldb, bias, C, c_dtype, ldc, M, N, K,
-                                           alpha, beta, workspace, workspace_bytes, st, ctx ? ctx->n_peers : 0,
-                                           ctx ? ctx->peer_C : nullptr);
-        if (rc != T81B200_EALIGN) {  // unaligned activations: the general kernel takes them
+    if (a_aligned && gemm_trit_tc_eligible(M, N, K)) {
+        const size_t need = gemm_trit_tc_scratch(B, b_dtype, layout, ldb, N, K);
+        const bool have = workspace && workspace_bytes >= need && reinterpret_cast<uintptr_t>(workspace) % 16 == 0;
+        if (need == 0 || (have && worth_staging(M, N, K))) {
+            const int rc = gemm_trit_tc_launch(0, A, row_scale, B, b_dtype, layout, ldb, bias, C, c_dtype, ldc, M, N, K, alpha, beta,
+                                               workspace, workspace_bytes, st, ctx ? ctx->n_peers : 0, ctx ? ctx->peer_C : nullptr);
             if (ctx) ctx->peers_done = rc == T81B200_OK;
             return rc;
         }
+        // unaligned bf16 rows without a workspace, and small problems: the general kernel
+        if (t81b200_gemm_trit_workspace_bytes(b_dtype, layout, c_dtype, M, N, K) > 0)
+            return fail(T81B200_EWORKSPACE, "gemm_trit: workspace of %zu bytes needed, %zu given", need, workspace_bytes);
     }
     return gemm_trit_simt_launch(A, row_scale, B, b_dtype, layout, ldb, bias, C, c_dtype, ldc, M, N, K, alpha, beta, st);
 }
@@ -323,6 +334,31 @@ extern "C" int t81b200_gemm_trit_t2(int n_group, const uint8_t *const *t2, const
     t81b200::g_hint_independent = hint;
     if (rc == T81B200_EALIGN) return fail(T81B200_ELIMIT, "gemm_trit_t2: K = %lld does not fit the kernel's shared memory", (long long)K);
     return rc;
+}
+
+extern "C" size_t t81b200_linear_t2_workspace_bytes(const void *B, int b_dtype, int64_t ldb, int64_t M, int64_t N, int64_t K) {
+    if (M <= 0 || N <= 0 || K <= 0 || !valid_dtype(b_dtype) || (N <= 16 && K <= kT2StreamingMaxK)) return 0;
+    return gemm_trit_tc_scratch(B, b_dtype, T81B200_LAYOUT_NK, ldb, N, K);
+}
+
+extern "C" int t81b200_linear_t2(const uint8_t *t2, const float *row_scale, const float *bias, void *C, int64_t M, const void *B,
+                                 int b_dtype, int64_t ldb, int c_dtype, int64_t ldc, int64_t N, int64_t K, float alpha, float beta,
+                                 void *workspace, size_t workspace_bytes, void *stream) {
+    if (M <= 0 || K <= 0 || N < 0) return fail(T81B200_EINVAL, "linear_t2: dimensions must be positive");
+    if (!valid_dtype(b_dtype) || !valid_dtype(c_dtype)) return fail(T81B200_EINVAL, "gemm_trit: unknown dtype");
+    if (ldb < K || ldc < M) return fail(T81B200_EINVAL, "gemm_trit: leading dimension below the row length");
+    if (N > 0 && (!t2 || !B || !C)) return fail(T81B200_EINVAL, "gemm_trit: null pointer");
+    if (reinterpret_cast<uintptr_t>(t2) % 16 != 0) return fail(T81B200_EALIGN, "gemm_trit_t2: matrices must be 16-byte aligned");
+    if (int rc = check_device()) return rc;
+    if (N == 0) return T81B200_OK;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (N <= 16) {
+        const int rc = gemv_trit_lut_launch(1, 1, &t2, &row_scale, &bias, &C, &M, B, b_dtype, ldb, c_dtype, ldc, (int)N, K, alpha, beta, st, nullptr);
+        if (rc != T81B200_EALIGN) return rc;  // a contraction too long for that kernel's shared memory: tiles take it
+    }
+    if (!gemm_trit_tc_eligible(M, N, K)) return fail(T81B200_ELIMIT, "linear_t2: dimensions beyond 2^31 (2^29 rows of B)");
+    return gemm_trit_tc_launch(1, t2, row_scale, B, b_dtype, T81B200_LAYOUT_NK, ldb, bias, C, c_dtype, ldc, M, N, K, alpha, beta, workspace,
+                               workspace_bytes, st, 0, nullptr);
 }
 
 extern "C" int t81b200_gemm_trit_t2_peers(const uint8_t *t2, const float *row_scale, const float *bias, void *C, int64_t M,

@@ -1,28 +1,42 @@
-// Prefill-shaped TRIT-mode kernel on the 5th-generation tensor cores (tcgen05).
+// TRIT-mode matmul on the 5th-generation tensor cores (tcgen05): more activation rows than the streaming kernel takes.
 //
-//   D[o][t] = sum_k T[o][k] * x[t][k]       o: output feature (UMMA M = 128 per CTA tile)
-//                                            t: token          (UMMA N = 256 per CTA tile)
-// Operand A is produced on the fly: the packed limbs of 128 weight rows arrive by TMA as
-// raw bytes, converter warps expand them to exact bf16 {-1,0,+1} (packed bf16 FMAs, see
-// common.cuh) and write them in the K-major, 128-byte-swizzled layout UMMA expects.
-// Operand B is the activations, brought by TMA (SWIZZLE_128B) straight from (tokens, K)
-// bf16 memory.  Accumulators live in TMEM (2 x 256 fp32 columns, double-buffered across
-// tiles) and are read back with tcgen05.ld for a fused scale/bias/beta epilogue.
+//   D[o][t] = sum_k T[o][k] * x[t][k]       o: output feature (256 per CTA pair, 128 per CTA)
+//                                            t: token          (up to 256 per tile)
+// A pair of CTAs (cta_group::2) works on one tile: each expands its own 128 weight rows into bf16 / fp16 operands in
+// its shared memory and loads half of the tile's activation rows by TMA; the even CTA issues the MMAs, which read both
+// halves, and each CTA keeps its 128 accumulator rows in TMEM (2 x 256 fp32 columns, double-buffered across tiles).
+// Measured against the one-CTA 128 x 256 kernel before it (bf16, weights in limbs there and in codes here):
+// 4096 x 14336 x 16384 tokens 1700 -> 1160 us (958 -> 1391 TFLOP/s in a long run under the power cap), 9216 x 3072 x 2048
+// 109 -> 86, 14336 x 4096 x 80 40.9 -> 20.3 us.
+// What bounds the kernel is shared-memory bandwidth: a 64-deep step writes and reads 16 KB of expanded weights per CTA
+// and writes and reads the activations, against 512 clocks of MMA at 256 tokens.  Halving the activation share is what
+// the pair is for: a single CTA with a 128 x 256 tile needs 768 clocks of shared memory per 512 of MMA.
 //
-// One persistent CTA per SM, 14 warps:
-//   warp 0      TMA producer (raw weight bytes + activation tiles)
-//   warp 1      MMA issuer (one elected lane), owns the TMEM allocation
-//   warps 2-5   epilogue (TMEM lanes 32*(warp%4) ...)
-//   warps 6-13  converters (256 threads; 2 limbs per thread per 192-trit super-block)
-// The contraction runs in k-atoms of 64 (one 128-byte swizzle row); 48-trit limbs do not
-// divide 64, so converters work in super-blocks of 4 limbs = 192 trits = 3 atoms.
+// Weights come in two formats (template FMT), both brought by bulk copies in 192-column chunks:
+//   0  packed limbs: a lane takes four limbs (rows 8 apart), packed bf16 FMAs expand them to {-1, 0, +1} (common.cuh);
+//   1  the decode-stream layout (pack_t2.cu): one word is 8 columns of 2 rows, i.e. two 16-byte pieces of the operand
+//      tile; a pair of trits is one shift and one AND (the 2-bit code IS the top of the 16-bit number +-2 or 0, in
+//      bf16 and in fp16 alike; the factor 2 leaves with alpha).  The 32 lanes of a warp store 8 rows x 4 column runs
+//      of 48: under the 128-byte swizzle every quarter of a warp store covers all banks once.
+// 192 columns are four limbs and three 64-column operand atoms: the unit in which converters hand weights to the MMAs.
 //
-// Every mbarrier wait is bounded; on expiry the role records a status code and all roles
-// fall through to the common teardown (TMEM is always released).
+// Activations: 16-bit types as they are (A and B of one MMA have the same type), fp32 as bf16 planes (x = hi + lo, 16
+// mantissa bits) that are multiplied one after the other with the same expanded weights.  Rows TMA cannot read
+// (unaligned, the (K, N) layout, fp32) are first copied into token-major planes in the caller's workspace.
+//
+// Few tiles (small matrices, short prompts): the contraction is split over S = 2 or 4 pairs of one cluster, whose
+// partial sums meet in the finishing CTA's shared memory (a tile's 32-token blocks go round the S pairs), added in rank
+// order: deterministic, no scratch memory.
+//
+// 14 warps per CTA:   0 TMA producer   1 MMA issuer (even CTA), TMEM allocation   2-5 epilogue   6-13 converters
+// (two groups of four: a warp per 32 rows, the groups take alternate chunks).  Every mbarrier wait is bounded; on
+// expiry the role records a status code and all roles fall through to the common teardown (TMEM is always released).
 #include "common.cuh"
 #include "tma.cuh"
+#include "umma.cuh"
 
 #include <atomic>
+#include <cmath>
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
@@ -31,48 +45,44 @@ namespace t81b200 {
 
 namespace {
 
-constexpr int BM = 128;          // output features per tile (UMMA M)
-constexpr int BN_MAX = 256;      // tokens per tile (UMMA N) with one activation plane; 128 with two
-constexpr int BK = 64;           // k-atom: 64 bf16 = 128 bytes
-constexpr int A_STAGES = 6;      // two super-blocks of expanded weights
-constexpr int B_STAGES = 3;
-constexpr int RAW_STAGES = 2;
-constexpr int A_STAGE_BYTES = BM * BK * 2;    // 16 KB
-constexpr int B_STAGE_BYTES = BN_MAX * BK * 2;  // 32 KB: one 256-token plane or two 128-token planes
-#ifndef T81B200_TC_CONVERTER_WARPS
-#define T81B200_TC_CONVERTER_WARPS 8
-#endif
-constexpr int CONVERTER_WARPS_ = T81B200_TC_CONVERTER_WARPS;
-constexpr int RAW_STAGE_BYTES = BM * 64;      // 4 limbs per row: 8 KB
-constexpr int NUM_THREADS = (6 + CONVERTER_WARPS_) * 32;
-constexpr int CONVERTER_WARP0 = 6;
-constexpr int CONVERTER_WARPS = CONVERTER_WARPS_;
-constexpr int CONVERTER_THREADS = CONVERTER_WARPS * 32;
-constexpr int LIMBS_PER_CONVERTER = BM * 4 / CONVERTER_THREADS;  // limbs of a 4-limb super-block per thread
-constexpr int OUT_TOKENS = 32;                      // tokens per staged output block (one tcgen05.ld of 32 columns)
+constexpr int BM = 128;          // output features per CTA
+constexpr int BK = 64;           // operand atom: 64 k = 128 bytes
+constexpr int CHUNK = 192;       // columns converted at a time: 3 atoms
+constexpr int A_ATOM_BYTES = BM * BK * 2;        // 16 KB
+constexpr int A_CHUNK_BYTES = 3 * A_ATOM_BYTES;  // 48 KB
+constexpr int A_MAX = 3, B_MAX = 12;             // ring slots that have barriers
+constexpr int RAW_STAGES = 3;                    // packed weights of a chunk (128 rows): 8 KB of limbs, 6 KB of codes
+constexpr int MAX_SPLITS = 4;                    // clusters of up to 8 CTAs
+constexpr int NUM_THREADS = 14 * 32;
+constexpr int EPILOGUE_WARP0 = 2, CONVERTER_WARP0 = 6;
+constexpr int OUT_TOKENS = 32;                        // tokens per staged output block (one tcgen05.ld of 32 columns)
 constexpr int OUT_STAGE_BYTES = OUT_TOKENS * BM * 2;  // [token][feature] block of a 16-bit output type: 8 KB
-constexpr int OUT_STAGES = 2;
-constexpr int SMEM_DATA_BYTES = A_STAGES * A_STAGE_BYTES + B_STAGES * B_STAGE_BYTES + RAW_STAGES * RAW_STAGE_BYTES +
-                                OUT_STAGES * OUT_STAGE_BYTES;
-constexpr int SMEM_BYTES = SMEM_DATA_BYTES + 256 /*barriers*/ + 1024 /*alignment slack*/;
-constexpr uint32_t TMEM_COLS = 512;
-
-// kind::f16 instruction descriptor: D fp32, A and B bf16, both K-major, N tokens, M = 128.
-__host__ __device__ constexpr uint32_t instr_desc(int bn) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
-}
+constexpr int BARRIER_BYTES = 512;
+constexpr int SMEM_LIMIT = 227 * 1024;
+template <int FMT> constexpr int kRawBytes = FMT == 1 ? 4 * 1536 : BM * 64;
+constexpr int SMEM_FIXED = RAW_STAGES * 8192 + 2 * OUT_STAGE_BYTES + BARRIER_BYTES + 1024 /*alignment*/;
 
 enum { STATUS_OK = 0, STATUS_TIMEOUT_PRODUCER = 1, STATUS_TIMEOUT_MMA = 2, STATUS_TIMEOUT_EPILOGUE = 3, STATUS_TIMEOUT_CONVERTER = 4 };
 
 __device__ int g_tc_status = 0;
 
 struct TcParams {
+    const uint8_t *A;
     const float *row_scale, *bias;
     void *C;
     int64_t c_row_stride, c_tok_stride;  // element strides of C along output features and tokens
-    int64_t M, N, K, kl;
-    int m_tiles, n_tiles, n_atoms;
-    int plane_rows;  // row distance between the activation planes in the tensor map
+    int64_t M, N, kl;
+    int tiles32;             // FMT 1: 32-row tiles of the matrix
+    int m_tiles, n_tiles;    // 256-row pair tiles, bn-token tiles
+    int bn;                  // tokens per tile: a multiple of 32
+    int n_atoms, n_chunks;
+    int planes, plane_rows;  // activation planes and their row distance in the tensor map
+    int splits;              // pairs of a cluster that share a tile's contraction
+    int a_stages, b_stages;
+    int b_step;              // atoms behind one barrier of the activation ring: 1, or 3 (a whole chunk)
+    int one_tile;            // no cluster has more than one tile: all warps but the first two finish it
+    uint32_t idesc;
+    uint32_t one_mask;       // FMT 0: bits of bf16 +-1 that stay (all for bf16, 0xBC00 per half for fp16)
     float alpha, beta;
     int n_out_maps;      // > 0: the epilogue stages output blocks in shared memory and stores them by TMA through
                          // this many tensor maps (the local C first, then the peers'); 0: per-element stores
@@ -86,49 +96,6 @@ struct TcParams {
 struct TcOutMaps {
     CUtensorMap m[1 + T81B200_MAX_PEERS];
 };
-
-__device__ __forceinline__ void tma_store_2d(const CUtensorMap *map, uint32_t src, int x, int y) {
-    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%2, %3}], [%1];"
-                 ::"l"(map), "r"(src), "r"(x), "r"(y)
-                 : "memory");
-}
-
-// K-major, SWIZZLE_128B shared-memory descriptor: rows are 128 bytes, 8-row groups 1024 bytes apart.
-__device__ __forceinline__ uint64_t umma_desc(uint32_t smem_addr) {
-    uint64_t d = 0;
-    d |= (uint64_t)((smem_addr >> 4) & 0x3FFF);  // start address
-    d |= (uint64_t)1 << 16;                       // leading byte offset (unused for swizzled K-major)
-    d |= (uint64_t)(1024 >> 4) << 32;             // stride byte offset
-    d |= (uint64_t)1 << 46;                       // descriptor version (Blackwell)
-    d |= (uint64_t)2 << 61;                       // SWIZZLE_128B
-    return d;
-}
-
-__device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                          uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
-          "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
-          "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-        : "r"(taddr)
-        : "memory");
-}
-
 
 // AND of a predicate over the 128 epilogue threads (named barrier 2); every one of them must call it.
 __device__ __forceinline__ bool epilogue_all(bool pred) {
@@ -144,433 +111,649 @@ __device__ __forceinline__ bool epilogue_all(bool pred) {
     return r != 0;
 }
 
-// PLANES = 1: bf16 activations as they are.  PLANES = 2: activations split into a bf16 "hi"
-// plane and a bf16 "lo" plane (x = hi + lo to 16 mantissa bits); both are multiplied with the
-// same expanded weights into the same accumulator, on a 128-token tile.
-// NSPLIT = 2 (one plane only): 128-token tiles, for launches whose 256-token tiles would leave most CTAs idle in
-// the last wave; the weight expansion is then done twice as often per flop, so it is only used where it pays.
-template <typename CT, int PLANES, int NSPLIT>
-__global__ void __launch_bounds__(NUM_THREADS, 1)
-gemm_trit_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
-                    const __grid_constant__ TcOutMaps omaps, const TcParams p) {
-    constexpr int BN = BN_MAX / PLANES / NSPLIT;
-    constexpr int PLANE_BYTES = BN * BK * 2;
-    constexpr uint32_t kInstrDesc = instr_desc(BN);
-    extern __shared__ uint8_t smem_raw[];
-    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    const uint32_t a_smem = base;
-    const uint32_t b_smem = a_smem + A_STAGES * A_STAGE_BYTES;
-    const uint32_t raw_smem = b_smem + B_STAGES * B_STAGE_BYTES;
-    const uint32_t out_smem = raw_smem + RAW_STAGES * RAW_STAGE_BYTES;
-    const uint32_t bars = out_smem + OUT_STAGES * OUT_STAGE_BYTES;
-    uint8_t *gen_base = smem_raw + (base - smem_u32(smem_raw));
-    // barrier slots (8 bytes each)
-    auto a_full = [&](int s) { return bars + 8u * s; };
-    auto a_empty = [&](int s) { return bars + 8u * (A_STAGES + s); };
-    auto b_full = [&](int s) { return bars + 8u * (2 * A_STAGES + s); };
-    auto b_empty = [&](int s) { return bars + 8u * (2 * A_STAGES + B_STAGES + s); };
-    auto raw_full = [&](int s) { return bars + 8u * (2 * A_STAGES + 2 * B_STAGES + s); };
-    auto raw_empty = [&](int s) { return bars + 8u * (2 * A_STAGES + 2 * B_STAGES + RAW_STAGES + s); };
-    auto acc_full = [&](int s) { return bars + 8u * (2 * A_STAGES + 2 * B_STAGES + 2 * RAW_STAGES + s); };
-    auto acc_empty = [&](int s) { return bars + 8u * (2 * A_STAGES + 2 * B_STAGES + 2 * RAW_STAGES + 2 + s); };
-    const uint32_t tmem_slot = bars + 8u * (2 * A_STAGES + 2 * B_STAGES + 2 * RAW_STAGES + 4);
-    volatile uint32_t *tmem_slot_gen = reinterpret_cast<volatile uint32_t *>(
-        gen_base + SMEM_DATA_BYTES + 8 * (2 * A_STAGES + 2 * B_STAGES + 2 * RAW_STAGES + 4));
+// Where a 32-token block is staged on its way to a TMA store, and which four warps share it.
+struct OutStage {
+    uint8_t *gen;      // [32 tokens][128 features] of a 16-bit type
+    uint32_t smem;
+    uint32_t barrier;  // named barrier of the 128 threads
+    bool first;        // this thread issues the store
+    bool reused;       // an earlier store may still be reading the buffer
+};
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < A_STAGES; ++s) { mbar_init(a_full(s), CONVERTER_WARPS); mbar_init(a_empty(s), 1); }
-        for (int s = 0; s < B_STAGES; ++s) { mbar_init(b_full(s), 1); mbar_init(b_empty(s), 1); }
-        for (int s = 0; s < RAW_STAGES; ++s) { mbar_init(raw_full(s), 1); mbar_init(raw_empty(s), CONVERTER_WARPS); }
-        for (int s = 0; s < 2; ++s) { mbar_init(acc_full(s), 1); mbar_init(acc_empty(s), 4); }
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_slot), "r"(TMEM_COLS) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem_base = *tmem_slot_gen;
-
-    const int total_tiles = p.m_tiles * p.n_tiles;
-    const int n_super = (p.n_atoms + 2) / 3;
-
-    if (warp == 0) {
-        // ---------------- TMA producer ----------------
-        if (lane == 0) {
-            Ring raw, b;
-            bool ok = true;
-            for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
-                const int m0 = (tile % p.m_tiles) * BM, n0 = (tile / p.m_tiles) * BN;
-                for (int s = 0; s < n_super && ok; ++s) {
-                    ok = mbar_wait(raw_empty(raw.stage), raw.phase ^ 1);
-                    if (!ok) break;
-                    mbar_arrive_expect_tx(raw_full(raw.stage), RAW_STAGE_BYTES);
-                    tma_load_2d(raw_smem + raw.stage * RAW_STAGE_BYTES, &map_w, s * 64, m0, raw_full(raw.stage));
-                    raw.advance(RAW_STAGES);
-                    for (int a = 3 * s; a < 3 * s + 3 && a < p.n_atoms; ++a) {
-                        ok = mbar_wait(b_empty(b.stage), b.phase ^ 1);
-                        if (!ok) break;
-                        mbar_arrive_expect_tx(b_full(b.stage), PLANES * PLANE_BYTES);
-#pragma unroll
-                        for (int pl = 0; pl < PLANES; ++pl)
-                            tma_load_2d(b_smem + b.stage * B_STAGE_BYTES + pl * PLANE_BYTES, &map_x, a * BK,
-                                        pl * p.plane_rows + n0, b_full(b.stage));
-                        b.advance(B_STAGES);
-                    }
-                }
-            }
-            if (!ok) atomicCAS(&g_tc_status, STATUS_OK, STATUS_TIMEOUT_PRODUCER);
+// One 32-token block of this thread's output feature: scale, bias, beta, store.
+template <typename CT>
+__device__ __forceinline__ void emit_block(const TcParams &p, const TcOutMaps &omaps, const uint32_t (&v)[32], int row0, int64_t row,
+                                           float scale, float bias, int tok0, const OutStage &out) {
+    const bool row_ok = row < p.M;
+    CT *crow = static_cast<CT *>(p.C) + row * p.c_row_stride;
+    if (p.n_out_maps > 0) {
+        // 16-bit output, token-major C: stage [32 tokens][128 features] blocks in shared memory and let
+        // TMA write them (whole 256-byte rows; the tensor map clips rows and tokens past the end)
+        if (out.reused) {
+            // two buffers in turn: the store issued from this one two blocks ago must have read it
+            if (out.first) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+            asm volatile("bar.sync %0, 128;" ::"r"(out.barrier) : "memory");
         }
-    } else if (warp == 1) {
-        // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            Ring a, b;
-            bool ok = true;
-            int it = 0;
-            for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++it) {
-                const int buf = it & 1;
-                const uint32_t acc_phase = (uint32_t)(it >> 1) & 1u;
-                ok = mbar_wait(acc_empty(buf), acc_phase ^ 1);
-                if (!ok) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t d_tmem = tmem_base + (uint32_t)buf * BN_MAX;
-                for (int at = 0; at < p.n_atoms; ++at) {
-                    ok = mbar_wait(a_full(a.stage), a.phase) && mbar_wait(b_full(b.stage), b.phase);
-                    if (!ok) break;
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint64_t ad = umma_desc(a_smem + a.stage * A_STAGE_BYTES);
+        CT *dst = reinterpret_cast<CT *>(out.gen) + (int)(row - row0);
 #pragma unroll
-                    for (int pl = 0; pl < PLANES; ++pl) {
-                        const uint64_t bd = umma_desc(b_smem + b.stage * B_STAGE_BYTES + pl * PLANE_BYTES);
-#pragma unroll
-                        for (int k = 0; k < BK / 16; ++k)
-                            umma_bf16(d_tmem, ad + (uint64_t)(2 * k), bd + (uint64_t)(2 * k), kInstrDesc,
-                                      (at | k | pl) != 0 ? 1u : 0u);
-                    }
-                    umma_commit(a_empty(a.stage));
-                    umma_commit(b_empty(b.stage));
-                    a.advance(A_STAGES);
-                    b.advance(B_STAGES);
-                }
-                if (!ok) break;
-                umma_commit(acc_full(buf));
-            }
-            if (!ok) atomicCAS(&g_tc_status, STATUS_OK, STATUS_TIMEOUT_MMA);
+        for (int i = 0; i < 32; ++i) dst[i * BM] = from_float<CT>(__uint_as_float(v[i]) * scale + bias);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        asm volatile("bar.sync %0, 128;" ::"r"(out.barrier) : "memory");
+        if (out.first) {
+            if (row0 < p.M && tok0 < p.N)
+                for (int j = 0; j < p.n_out_maps; ++j) tma_store_2d(&omaps.m[j], out.smem, row0, tok0);
+            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
         }
-    } else if (warp < CONVERTER_WARP0) {
-        // ---------------- epilogue ----------------
-        const int lane_group = warp & 3;  // TMEM lanes 32*lane_group .. +31 are this warp's
-        bool ok = true;
-        int it = 0;
-        int out_count = 0;  // staged output blocks so far (picks the staging buffer)
-        for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++it) {
-            const int m0 = (tile % p.m_tiles) * BM, n0 = (tile / p.m_tiles) * BN;
-            const int buf = it & 1;
-            const uint32_t acc_phase = (uint32_t)(it >> 1) & 1u;
-            // One decision for all four epilogue warps (tcgen05.ld is .aligned, and the staging path below
-            // meets at named barriers): every thread's bounded wait returns, then the 128 threads agree.
-            ok = epilogue_all(mbar_wait(acc_full(buf), acc_phase));
-            if (!ok) break;
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const int64_t row = (int64_t)m0 + lane_group * 32 + lane;
-            const bool row_ok = row < p.M;
-            const float scale = (row_ok && p.row_scale ? p.row_scale[row] : 1.0f) * p.alpha;
-            const float bias = row_ok && p.bias ? p.bias[row] : 0.0f;
-            CT *crow = static_cast<CT *>(p.C) + row * p.c_row_stride;
-            if (p.n_out_maps > 0) {
-                // 16-bit output, token-major C: stage [32 tokens][128 features] blocks in shared memory and let
-                // TMA write them (whole 256-byte rows; the tensor map clips rows and tokens past the end)
-                const int epi_tid = threadIdx.x - 2 * 32;  // 0..127
-                uint8_t *stage0 = gen_base + (out_smem - base);
-#pragma unroll 1
-                for (int c = 0; c < BN / 32; ++c, ++out_count) {
-                    uint32_t v[32];
-                    tmem_ld32(tmem_base + ((uint32_t)(lane_group * 32) << 16) + (uint32_t)(buf * BN_MAX + c * 32), v);
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    const int sb = out_count & 1;
-                    // the stores issued from this buffer two blocks ago must have read it
-                    if (epi_tid == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-                    asm volatile("bar.sync 2, 128;" ::: "memory");
-                    CT *dst = reinterpret_cast<CT *>(stage0 + sb * OUT_STAGE_BYTES) + lane_group * 32 + lane;
+    } else if (row_ok && p.c_vec && (int64_t)tok0 + 32 <= p.N) {
+        // (M, N) argument order: the thread's 32 tokens are contiguous — whole 16-byte pieces, and with
+        // beta the old values are all fetched before the first store
+        constexpr int PER = 16 / (int)sizeof(CT);  // elements per 128-bit access
+        uint4 *dst = reinterpret_cast<uint4 *>(crow + tok0);
+        uint4 old[32 / PER];
+        if (p.beta != 0.0f) {
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) dst[i * BM] = from_float<CT>(__uint_as_float(v[i]) * scale + bias);
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                    asm volatile("bar.sync 2, 128;" ::: "memory");
-                    if (epi_tid == 0) {
-                        for (int j = 0; j < p.n_out_maps; ++j)
-                            tma_store_2d(&omaps.m[j], out_smem + (uint32_t)sb * OUT_STAGE_BYTES, m0, n0 + c * 32);
-                        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-                    }
-                }
-            } else
-#pragma unroll 1
-            for (int c = 0; c < BN / 32; ++c) {
-                uint32_t v[32];
-                tmem_ld32(tmem_base + ((uint32_t)(lane_group * 32) << 16) + (uint32_t)(buf * BN_MAX + c * 32), v);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (row_ok && p.c_vec && (int64_t)n0 + c * 32 + 32 <= p.N) {
-                    // (M, N) argument order: the thread's 32 tokens are contiguous — whole 16-byte pieces, and with
-                    // beta the old values are all fetched before the first store
-                    constexpr int PER = 16 / (int)sizeof(CT);  // elements per 128-bit access
-                    uint4 *dst = reinterpret_cast<uint4 *>(crow + (int64_t)n0 + c * 32);
-                    uint4 old[32 / PER];
-                    if (p.beta != 0.0f) {
+            for (int q = 0; q < 32 / PER; ++q) old[q] = dst[q];
+        }
 #pragma unroll
-                        for (int q = 0; q < 32 / PER; ++q) old[q] = dst[q];
-                    }
+        for (int q = 0; q < 32 / PER; ++q) {
+            CT out[PER];
+            const CT *was = reinterpret_cast<const CT *>(&old[q]);
 #pragma unroll
-                    for (int q = 0; q < 32 / PER; ++q) {
-                        CT out[PER];
-                        const CT *was = reinterpret_cast<const CT *>(&old[q]);
+            for (int e = 0; e < PER; ++e) {
+                float y = __uint_as_float(v[q * PER + e]) * scale + bias;
+                if (p.beta != 0.0f) y += p.beta * to_float<CT>(was[e]);
+                out[e] = from_float<CT>(y);
+            }
+            dst[q] = *reinterpret_cast<const uint4 *>(out);
+        }
+    } else if (row_ok) {
 #pragma unroll
-                        for (int e = 0; e < PER; ++e) {
-                            float y = __uint_as_float(v[q * PER + e]) * scale + bias;
-                            if (p.beta != 0.0f) y += p.beta * to_float<CT>(was[e]);
-                            out[e] = from_float<CT>(y);
-                        }
-                        dst[q] = *reinterpret_cast<const uint4 *>(out);
-                    }
-                } else if (row_ok) {
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) {
-                        const int64_t tok = (int64_t)n0 + c * 32 + i;
-                        if (tok < p.N) {
-                            float y = __uint_as_float(v[i]) * scale + bias;
-                            CT *dst = crow + tok * p.c_tok_stride;
-                            if (p.beta != 0.0f) y += p.beta * to_float<CT>(*dst);
-                            *dst = from_float<CT>(y);
-                        }
-                    }
-                    // column-sharded Linear: the same elements go into every peer's result over NVLink
-                    for (int pj = 0; pj < p.n_peers; ++pj) {
-                        CT *prow = static_cast<CT *>(p.peer_C[pj]) + row * p.c_row_stride;
+        for (int i = 0; i < 32; ++i) {
+            const int64_t tok = (int64_t)tok0 + i;
+            if (tok < p.N) {
+                float y = __uint_as_float(v[i]) * scale + bias;
+                CT *dst = crow + tok * p.c_tok_stride;
+                if (p.beta != 0.0f) y += p.beta * to_float<CT>(*dst);
+                *dst = from_float<CT>(y);
+            }
+        }
+        // column-sharded Linear: the same elements go into every peer's result over NVLink
+        for (int pj = 0; pj < p.n_peers; ++pj) {
+            CT *prow = static_cast<CT *>(p.peer_C[pj]) + row * p.c_row_stride;
 #pragma unroll 1  // a rare path: unrolled it costs the whole kernel 40 registers
-                        for (int i = 0; i < 32; ++i) {
-                            const int64_t tok = (int64_t)n0 + c * 32 + i;
-                            if (tok < p.N) prow[tok * p.c_tok_stride] = crow[tok * p.c_tok_stride];
-                        }
-                    }
-                }
-            }
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) mbar_arrive(acc_empty(buf));
-        }
-        // every TMA store of this CTA has completed before the kernel ends
-        if (threadIdx.x == 2 * 32) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
-        if (!ok && lane == 0) atomicCAS(&g_tc_status, STATUS_OK, STATUS_TIMEOUT_EPILOGUE);
-    } else {
-        // ---------------- converters ----------------
-        const int cthread = threadIdx.x - CONVERTER_WARP0 * 32;  // 0..255
-        Ring raw, a;
-        bool ok = true;
-        for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
-            for (int s = 0; s < n_super && ok; ++s) {
-                ok = __all_sync(0xffffffffu, mbar_wait(raw_full(raw.stage), raw.phase));
-                if (!ok) break;
-                uint4 limb[LIMBS_PER_CONVERTER];
-#pragma unroll
-                for (int h = 0; h < LIMBS_PER_CONVERTER; ++h) {
-                    const int item = cthread + CONVERTER_THREADS * h;  // row = item / 4, limb = item % 4
-                    limb[h] = *reinterpret_cast<const uint4 *>(gen_base + A_STAGES * A_STAGE_BYTES + B_STAGES * B_STAGE_BYTES +
-                                                               raw.stage * RAW_STAGE_BYTES + item * 16);
-                    if ((int64_t)4 * s + (item & 3) >= p.kl)  // past the row's last limb: zero trits
-                        limb[h] = make_uint4(kZeroTryteWord, kZeroTryteWord, kZeroTryteWord, kZeroTryteWord);
-                }
-                __syncwarp();
-                if (lane == 0) mbar_arrive(raw_empty(raw.stage));
-                raw.advance(RAW_STAGES);
-
-                // the (up to) three atoms of this super-block
-                const int atoms_here = p.n_atoms - 3 * s < 3 ? p.n_atoms - 3 * s : 3;
-                Ring aw = a;
-                for (int j = 0; j < atoms_here && ok; ++j) {
-                    ok = mbar_wait(a_empty(aw.stage), aw.phase ^ 1);
-                    aw.advance(A_STAGES);
-                }
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
-#pragma unroll
-                for (int h = 0; h < LIMBS_PER_CONVERTER; ++h) {
-                    const int item = cthread + CONVERTER_THREADS * h;
-                    const int r = item >> 2, j = item & 3;
-                    uint32_t o[24];
-                    decode_limb(limb[h], o);
-                    // decode order -> natural order: pairs (trit 2m, trit 2m+1)
-                    uint32_t nat[24];
-#pragma unroll
-                    for (int pr = 0; pr < 8; ++pr) {
-                        nat[3 * pr + 0] = __byte_perm(o[3 * pr], o[3 * pr + 1], 0x5410);
-                        nat[3 * pr + 1] = __byte_perm(o[3 * pr + 2], o[3 * pr], 0x7610);
-                        nat[3 * pr + 2] = __byte_perm(o[3 * pr + 1], o[3 * pr + 2], 0x7632);
-                    }
-                    const uint32_t row_off = (uint32_t)(r >> 3) * 1024u + (uint32_t)(r & 7) * 128u;
-#pragma unroll
-                    for (int q = 0; q < 6; ++q) {
-                        const int chunk = 6 * j + q;         // 16-byte chunk inside the 384-byte super-block row
-                        const int atom = chunk >> 3, cc = chunk & 7;
-                        if (atom < atoms_here) {
-                            int st = a.stage + atom;
-                            st = st >= A_STAGES ? st - A_STAGES : st;
-                            const uint32_t off = (uint32_t)st * A_STAGE_BYTES + row_off + (uint32_t)((cc ^ (r & 7)) << 4);
-                            *reinterpret_cast<uint4 *>(gen_base + off) = make_uint4(nat[4 * q], nat[4 * q + 1], nat[4 * q + 2], nat[4 * q + 3]);
-                        }
-                    }
-                }
-                // generic-proxy writes must be visible to the tensor core's async proxy
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                __syncwarp();
-                if (lane == 0)
-                    for (int j = 0; j < atoms_here; ++j) {
-                        int st = a.stage + j;
-                        st = st >= A_STAGES ? st - A_STAGES : st;
-                        mbar_arrive(a_full(st));
-                    }
-                a = aw;
+            for (int i = 0; i < 32; ++i) {
+                const int64_t tok = (int64_t)tok0 + i;
+                if (tok < p.N) prow[tok * p.c_tok_stride] = crow[tok * p.c_tok_stride];
             }
         }
-        if (!ok && lane == 0) atomicCAS(&g_tc_status, STATUS_OK, STATUS_TIMEOUT_CONVERTER);
-    }
-
-    // ---------------- teardown ----------------
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    if (warp == 1) {
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
     }
 }
 
-template <typename CT, int PLANES, int NSPLIT>
-int launch_tc(const CUtensorMap &mw, const CUtensorMap &mx, const TcOutMaps &om, const TcParams &p, cudaStream_t st) {
-    auto kern = gemm_trit_tc_kernel<CT, PLANES, NSPLIT>;
+// One warp's share of a chunk (32 rows x 192 columns), read from the raw ring.
+template <int FMT> struct RawChunk;
+template <> struct RawChunk<0> { uint4 q[4]; };  // limb (lane % 4) of rows lane / 4 + 8 i
+template <> struct RawChunk<1> { uint4 q[3]; };  // the lane's twelve words
+
+template <int FMT>
+__device__ __forceinline__ void read_chunk(const TcParams &p, const uint8_t *raw_stage, int rt, int c, int lane, RawChunk<FMT> &raw) {
+    if constexpr (FMT == 1) {
+        const uint4 *src = reinterpret_cast<const uint4 *>(raw_stage + rt * 1536 + lane * 48);
+#pragma unroll
+        for (int j = 0; j < 3; ++j) raw.q[j] = src[j];
+    } else {
+        const bool there = (int64_t)4 * c + (lane & 3) < p.kl;  // past the row's last limb: zero trits
+        const uint4 *src = reinterpret_cast<const uint4 *>(raw_stage + rt * 2048) + lane;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            raw.q[i] = there ? src[32 * i] : make_uint4(kZeroTryteWord, kZeroTryteWord, kZeroTryteWord, kZeroTryteWord);
+    }
+}
+
+// Expands the share into the operand tile at `tile` (this warp's 32 rows of the chunk's first atom): K-major rows of
+// 128 bytes, 16-byte piece cc of row r at (cc ^ (r & 7)) * 16.
+template <int FMT>
+__device__ __forceinline__ void expand_chunk(const RawChunk<FMT> &raw, uint8_t *tile, int lane, uint32_t one_mask) {
+    const int g = lane >> 2, t = lane & 3;  // row within a group of 8; 48-column run
+    uint32_t off[6];
+#pragma unroll
+    for (int m = 0; m < 6; ++m) {
+        const int piece = 6 * t + m;
+        off[m] = (uint32_t)(piece >> 3) * A_ATOM_BYTES + (uint32_t)g * 128u + (uint32_t)(((piece & 7) ^ g) << 4);
+    }
+    if constexpr (FMT == 1) {
+        const uint32_t *w = reinterpret_cast<const uint32_t *>(&raw.q[0]);
+#pragma unroll
+        for (int gr = 0; gr < 2; ++gr)
+#pragma unroll
+            for (int m = 0; m < 6; ++m) {
+                const uint32_t x = w[6 * gr + m];
+                constexpr uint32_t k = 0xC000C000u;
+                uint8_t *dst = tile + gr * 2048 + off[m];
+                *reinterpret_cast<uint4 *>(dst) = make_uint4(x & k, (x << 4) & k, (x << 8) & k, (x << 12) & k);
+                *reinterpret_cast<uint4 *>(dst + 1024) = make_uint4((x << 2) & k, (x << 6) & k, (x << 10) & k, (x << 14) & k);
+            }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            uint32_t o[24], nat[24];
+            decode_limb(raw.q[i], o);
+            // decode order -> natural order: pairs (trit 2m, trit 2m+1)
+#pragma unroll
+            for (int pr = 0; pr < 8; ++pr) {
+                nat[3 * pr + 0] = __byte_perm(o[3 * pr], o[3 * pr + 1], 0x5410) & one_mask;
+                nat[3 * pr + 1] = __byte_perm(o[3 * pr + 2], o[3 * pr], 0x7610) & one_mask;
+                nat[3 * pr + 2] = __byte_perm(o[3 * pr + 1], o[3 * pr + 2], 0x7632) & one_mask;
+            }
+#pragma unroll
+            for (int m = 0; m < 6; ++m)
+                *reinterpret_cast<uint4 *>(tile + i * 1024 + off[m]) = make_uint4(nat[4 * m], nat[4 * m + 1], nat[4 * m + 2], nat[4 * m + 3]);
+        }
+    }
+}
+
+template <typename CT, int FMT>
+__global__ void __launch_bounds__(NUM_THREADS, 1)
+gemm_trit_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ TcOutMaps omaps, const __grid_constant__ TcParams p) {
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    uint8_t *gen_base = smem_raw + (base - smem_u32(smem_raw));
+    const uint32_t b_atom_bytes = (uint32_t)p.bn * (BK * 2 / 2);  // this CTA's half of the tokens
+    const uint32_t b_stage_bytes = b_atom_bytes * (uint32_t)p.b_step;
+    const uint32_t b_off = (uint32_t)p.a_stages * A_CHUNK_BYTES;
+    const uint32_t raw_off = b_off + (uint32_t)p.b_stages * b_stage_bytes;
+    const uint32_t out_off = raw_off + RAW_STAGES * kRawBytes<FMT>;
+    const uint32_t bars = base + out_off + 2 * OUT_STAGE_BYTES;
+    auto a_full = [&](int s) { return bars + 8u * s; };
+    auto a_empty = [&](int s) { return bars + 8u * (A_MAX + s); };
+    auto b_full = [&](int s) { return bars + 8u * (2 * A_MAX + s); };
+    auto b_empty = [&](int s) { return bars + 8u * (2 * A_MAX + B_MAX + s); };
+    auto acc_full = [&](int s) { return bars + 8u * (2 * A_MAX + 2 * B_MAX + s); };
+    auto acc_empty = [&](int s) { return bars + 8u * (2 * A_MAX + 2 * B_MAX + 2 + s); };
+    auto raw_full = [&](int s) { return bars + 8u * (2 * A_MAX + 2 * B_MAX + 4 + s); };
+    auto raw_empty = [&](int s) { return bars + 8u * (2 * A_MAX + 2 * B_MAX + 4 + RAW_STAGES + s); };
+    const uint32_t tmem_slot = bars + 8u * (2 * A_MAX + 2 * B_MAX + 4 + 2 * RAW_STAGES);
+
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+    const uint32_t rank = cluster_rank();
+    const int half = (int)(rank & 1u), slice = (int)(rank >> 1);
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < A_MAX; ++s) { mbar_init(a_full(s), 8); mbar_init(a_empty(s), 1); }
+        for (int s = 0; s < B_MAX; ++s) { mbar_init(b_full(s), 1); mbar_init(b_empty(s), 1); }
+        for (int s = 0; s < 2; ++s) { mbar_init(acc_full(s), 1); mbar_init(acc_empty(s), 8); }
+        for (int s = 0; s < RAW_STAGES; ++s) { mbar_init(raw_full(s), 1); mbar_init(raw_empty(s), 4); }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();  // barriers initialised (this CTA)
+    const int total_tiles = p.m_tiles * p.n_tiles;
+    const int n_clusters = (int)gridDim.x / (2 * p.splits), cluster_id = (int)blockIdx.x / (2 * p.splits);
+    // this pair's share of the contraction, in chunks
+    const int c0 = p.n_chunks * slice / p.splits, c1 = p.n_chunks * (slice + 1) / p.splits;
+    const uint16_t pair_mask = (uint16_t)(3u << (rank & ~1u));
+
+    // The producer's weight loads run two chunks ahead of the activations; the first ones touch nothing but this CTA's
+    // memory and start before the cluster has met.
+    Ring raw_fill;
+    bool fill_ok = true;
+    int raw_tile = cluster_id, raw_c = c0;
+    auto load_raw = [&]() {
+        if (raw_tile >= total_tiles || !fill_ok) return;
+        fill_ok = mbar_wait(raw_empty(raw_fill.stage), raw_fill.phase ^ 1);
+        if (!fill_ok) return;
+        const int row0 = ((raw_tile % p.m_tiles) * 2 + half) * BM;
+        const uint32_t dst = base + raw_off + (uint32_t)raw_fill.stage * (uint32_t)kRawBytes<FMT>, bar = raw_full(raw_fill.stage);
+        if (elect_one()) {
+            if constexpr (FMT == 1) {
+                // the row tiles of a chunk are contiguous; past the matrix's last one nothing is loaded (those rows
+                // of the result are not stored)
+                int n = p.tiles32 - (row0 >> 5);
+                n = n < 0 ? 0 : (n > 4 ? 4 : n);
+                if (n > 0) {
+                    mbar_arrive_expect_tx(bar, (uint32_t)n * 1536u);
+                    bulk_load(dst, p.A + ((int64_t)raw_c * p.tiles32 + (row0 >> 5)) * 1536, (uint32_t)n * 1536u, bar);
+                } else mbar_arrive(bar);
+            } else {
+                mbar_arrive_expect_tx(bar, (uint32_t)kRawBytes<FMT>);
+                tma_load_2d(dst, &map_w, raw_c * 64, row0, bar);
+            }
+        }
+        __syncwarp();
+        raw_fill.advance(RAW_STAGES);
+        if (++raw_c >= c1) { raw_c = c0; raw_tile += n_clusters; }
+    };
+
+    // launched with programmatic stream serialization: everything above overlaps the tail of the previous kernel
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (warp == 0) {
+        load_raw();
+        load_raw();
+    } else if (warp == 1) tmem_alloc_pair(tmem_slot);
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    cluster_barrier();  // the other CTAs' barriers are initialised before anything arrives on them
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t *>(gen_base + (tmem_slot - base));
+
+    if (warp == 0) {
+        // ---------------- TMA producer: this CTA's packed weights and its half of the activation rows ----------------
+        Ring b;
+        bool ok = fill_ok;
+        for (int tile = cluster_id; tile < total_tiles && ok; tile += n_clusters) {
+            const int row = (tile / p.m_tiles) * p.bn + half * (p.bn / 2);
+            for (int c = c0; c < c1 && ok; ++c) {
+                load_raw();
+                ok = fill_ok;
+                const int a_end = 3 * c + 3 < p.n_atoms ? 3 * c + 3 : p.n_atoms;
+                for (int a0 = 3 * c; a0 < a_end && ok; a0 += p.b_step) {
+                    const int a1 = a0 + p.b_step < a_end ? a0 + p.b_step : a_end;
+                    for (int pl = 0; pl < p.planes; ++pl) {
+                        ok = mbar_wait(b_empty(b.stage), b.phase ^ 1);
+                        if (!ok) break;
+                        if (elect_one()) {
+                            if (half == 0) mbar_arrive_expect_tx(b_full(b.stage), 2 * (uint32_t)(a1 - a0) * b_atom_bytes);
+                            uint32_t dst = base + b_off + (uint32_t)b.stage * b_stage_bytes;
+                            for (int a = a0; a < a1; ++a, dst += b_atom_bytes)
+                                tma_load_2d_pair(dst, &map_x, a * BK, pl * p.plane_rows + row, b_full(b.stage));
+                        }
+                        __syncwarp();
+                        b.advance(p.b_stages);
+                    }
+                }
+            }
+        }
+        if (!ok && lane == 0) atomicCAS(&g_tc_status, STATUS_OK, STATUS_TIMEOUT_PRODUCER);
+    } else if (warp == 1) {
+        // ---------------- MMA issuer ----------------
+        if (half == 0) {
+            Ring a, b;
+            bool ok = true;
+            int it = 0;
+            for (int tile = cluster_id; tile < total_tiles && ok; tile += n_clusters, ++it) {
+                const int buf = it & 1;
+                ok = mbar_wait(acc_empty(buf), ((uint32_t)(it >> 1) & 1u) ^ 1u);
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t d_tmem = tmem_base + (uint32_t)buf * 256u;
+                uint32_t accumulate = 0;
+                for (int c = c0; c < c1 && ok; ++c) {
+                    ok = mbar_wait(a_full(a.stage), a.phase);
+                    if (!ok) break;
+                    const int atoms = p.n_atoms - 3 * c < 3 ? p.n_atoms - 3 * c : 3;
+                    const uint32_t a_base = base + (uint32_t)a.stage * A_CHUNK_BYTES;
+                    for (int j0 = 0; j0 < atoms && ok; j0 += p.b_step) {
+                        const int j1 = j0 + p.b_step < atoms ? j0 + p.b_step : atoms;
+                        for (int pl = 0; pl < p.planes; ++pl) {
+                            ok = mbar_wait(b_full(b.stage), b.phase);
+                            if (!ok) break;
+                            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                            if (elect_one()) {
+                                uint64_t bd = umma_desc_k(base + b_off + (uint32_t)b.stage * b_stage_bytes);
+                                uint64_t ad = umma_desc_k(a_base + (uint32_t)j0 * A_ATOM_BYTES);
+                                for (int j = j0; j < j1; ++j, ad += A_ATOM_BYTES >> 4, bd += b_atom_bytes >> 4) {
+#pragma unroll
+                                    for (int k = 0; k < BK / 16; ++k)
+                                        umma_pair(d_tmem, ad + (uint64_t)(2 * k), bd + (uint64_t)(2 * k), p.idesc, k == 0 && j == j0 ? accumulate : 1u);
+                                }
+                                umma_commit_pair(b_empty(b.stage), pair_mask);
+                            }
+                            __syncwarp();
+                            accumulate = 1;
+                            b.advance(p.b_stages);
+                        }
+                    }
+                    if (!ok) break;
+                    if (elect_one()) umma_commit_pair(a_empty(a.stage), pair_mask);
+                    __syncwarp();
+                    a.advance(p.a_stages);
+                }
+                if (ok && elect_one()) umma_commit_pair(acc_full(buf), pair_mask);
+                __syncwarp();
+            }
+            if (!ok && lane == 0) atomicCAS(&g_tc_status, STATUS_OK, STATUS_TIMEOUT_MMA);
+        }
+    } else if (warp < CONVERTER_WARP0) {
+        // ---------------- epilogue of all but one-tile launches, which are finished below ----------------
+        const int quarter = warp & 3;  // TMEM lanes 32 * quarter .. + 31 are this warp's
+        bool ok = true;
+        int it = 0, out_count = 0;
+        for (int tile = cluster_id; tile < total_tiles && ok; tile += n_clusters, ++it) {
+            const int buf = it & 1;
+            // One decision for all four epilogue warps (tcgen05.ld is .aligned, and the staging path meets at named
+            // barriers): every thread's bounded wait returns, then the 128 threads agree.
+            ok = epilogue_all(mbar_wait(acc_full(buf), (uint32_t)(it >> 1) & 1u));
+            if (!ok) break;
+            if (p.one_tile) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const int row0 = ((tile % p.m_tiles) * 2 + half) * BM, n0 = (tile / p.m_tiles) * p.bn;
+            const int64_t row = (int64_t)row0 + quarter * 32 + lane;
+            const float scale = (row < p.M && p.row_scale ? p.row_scale[row] : 1.0f) * p.alpha;
+            const float bias = row < p.M && p.bias ? p.bias[row] : 0.0f;
+#pragma unroll 1
+            for (int c = 0; c < p.bn / 32; ++c) {
+                uint32_t v[32];
+                tmem_ld32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * 256 + c * 32), v);
+                const uint32_t stage = out_off + (uint32_t)(out_count++ & 1) * OUT_STAGE_BYTES;
+                emit_block<CT>(p, omaps, v, row0, row, scale, bias, n0 + c * 32,
+                               OutStage{gen_base + stage, base + stage, 2, threadIdx.x == EPILOGUE_WARP0 * 32, true});
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive_leader(acc_empty(buf));
+        }
+        if (!ok && lane == 0) atomicCAS(&g_tc_status, STATUS_OK, STATUS_TIMEOUT_EPILOGUE);
+    } else {
+        // ---------------- converters ----------------
+        const int rt = (warp - CONVERTER_WARP0) & 3, group = (warp - CONVERTER_WARP0) >> 2;
+        const int span = c1 - c0, my_tiles = cluster_id < total_tiles ? (total_tiles - 1 - cluster_id) / n_clusters + 1 : 0;
+        Ring a, raw;
+        if (group == 1) { a.advance(p.a_stages); raw.advance(RAW_STAGES); }
+        bool ok = true;
+        int c = c0 + group;  // the groups take alternate chunks of the CTA's whole sequence
+        for (int left = my_tiles * span - group; left > 0; left -= 2) {
+            while (c >= c1) c -= span;
+            ok = __all_sync(0xffffffffu, mbar_wait(raw_full(raw.stage), raw.phase));
+            if (!ok) break;
+            RawChunk<FMT> words;
+            read_chunk<FMT>(p, gen_base + raw_off + raw.stage * kRawBytes<FMT>, rt, c, lane, words);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(raw_empty(raw.stage));
+            ok = __all_sync(0xffffffffu, mbar_wait(a_empty(a.stage), a.phase ^ 1));
+            if (!ok) break;
+            expand_chunk<FMT>(words, gen_base + a.stage * A_CHUNK_BYTES + rt * 4096, lane, p.one_mask);
+            // generic-proxy writes must be visible to the tensor core's async proxy
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive_leader(a_full(a.stage));
+            a.advance(p.a_stages);
+            a.advance(p.a_stages);
+            raw.advance(RAW_STAGES);
+            raw.advance(RAW_STAGES);
+            c += 2;
+        }
+        if (!ok && lane == 0) atomicCAS(&g_tc_status, STATUS_OK, STATUS_TIMEOUT_CONVERTER);
+    }
+    __syncwarp();
+
+    if (p.one_tile) {
+        // Three groups of four warps take the tile's 32-token blocks in turn; what they stage goes into the activation
+        // ring, idle by now.  With splits > 1 the pairs of the cluster hold partial sums: block b is finished by slice
+        // b % splits, the others write theirs into its shared memory first (the weight ring, idle once every CTA of
+        // the cluster has its last MMA behind it).
+        const int group = (warp - EPILOGUE_WARP0) >> 2, quarter = warp & 3, S = p.splits, blocks = p.bn / 32;
+        const int row0 = ((cluster_id % p.m_tiles) * 2 + half) * BM, n0 = (cluster_id / p.m_tiles) * p.bn;
+        const uint32_t lane_row = (uint32_t)(quarter * 32 + lane);
+        const uint32_t t_lane = tmem_base + ((uint32_t)(quarter * 32) << 16);
+        __syncthreads();
+        if (S > 1) cluster_barrier();
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (S > 1) {
+            if (warp >= EPILOGUE_WARP0)
+                for (int b = group; b < blocks; b += 3) {
+                    const int to = b % S;
+                    if (to == slice) continue;
+                    uint32_t v[32];
+                    tmem_ld32(t_lane + (uint32_t)(b * 32), v);
+                    const int slot = (b / S) * (S - 1) + (slice < to ? slice : slice - 1);
+                    uint32_t dst;
+                    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(base + (uint32_t)slot * 16384u + lane_row * 4u), "r"((uint32_t)(2 * to + half)));
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(dst + (uint32_t)i * 512u), "r"(v[i]) : "memory");
+                }
+            __syncthreads();
+            cluster_barrier();
+        }
+        if (warp >= EPILOGUE_WARP0) {
+            const int64_t row = (int64_t)row0 + lane_row;
+            const float scale = (row < p.M && p.row_scale ? p.row_scale[row] : 1.0f) * p.alpha;
+            const float bias = row < p.M && p.bias ? p.bias[row] : 0.0f;
+            const bool first = quarter == 2 && lane == 0;
+            for (int b = slice + S * group; b < blocks; b += 3 * S) {
+                uint32_t v[32];
+                tmem_ld32(t_lane + (uint32_t)(b * 32), v);
+                if (S > 1) {
+                    uint32_t sum[32];
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) sum[i] = 0u;
+                    for (int s = 0; s < S; ++s) {  // in rank order
+                        const float *src = reinterpret_cast<const float *>(gen_base + (size_t)((b / S) * (S - 1) + (s < slice ? s : s - 1)) * 16384) + lane_row;
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) sum[i] = __float_as_uint(__uint_as_float(sum[i]) + (s == slice ? __uint_as_float(v[i]) : src[i * 128]));
+                    }
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) v[i] = sum[i];
+                }
+                const uint32_t stage = b_off + (uint32_t)b * OUT_STAGE_BYTES;
+                emit_block<CT>(p, omaps, v, row0, row, scale, bias, n0 + b * 32, OutStage{gen_base + stage, base + stage, (uint32_t)(2 + group), first, false});
+            }
+            if (first) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+        }
+    } else if (threadIdx.x == EPILOGUE_WARP0 * 32) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");  // every store has completed
+
+    // ---------------- teardown: no CTA leaves while its peer may still arrive on its barriers or read its operands ----
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    cluster_barrier();
+    if (warp == 1) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        tmem_free_pair(tmem_base);
+    }
+}
+
+// Everything a launch needs to know about the sizes.
+struct TcShape {
+    int bn = 0, n_tiles = 0, splits = 1, a_stages = 2, b_stages = 2, b_step = 1;
+    size_t smem = 0;
+};
+
+// Clusters of 2 * splits CTAs (one CTA per SM) that the device runs at a time: clusters do not straddle GPCs, so fewer
+// fit than the SM count suggests (74, 33, 22 and 15 for 1 to 4 splits).
+int resident_clusters(int splits);
+
+TcShape pick_shape(int64_t M, int64_t N, int64_t K, int planes) {
+    const int64_t m_tiles = (M + 255) / 256, chunks = (K + CHUNK - 1) / CHUNK, least = (N + 255) / 256;
+    TcShape best;
+    double best_t = 1e30;
+    for (int64_t want = least; want <= least + 8 && want <= (N + 31) / 32; ++want) {
+        const int bn = (int)(((N + want - 1) / want + 31) / 32 * 32);
+        const int64_t n_tiles = (N + bn - 1) / bn, tiles = m_tiles * n_tiles;
+        for (int s = 1; s <= MAX_SPLITS; ++s) {
+            const int resident = resident_clusters(s);
+            if (s > chunks || (s > 1 && tiles > resident)) continue;
+            const double mma = 2.0 * planes * bn, smem = 128.0 + planes * (128.0 + bn);
+            const double atom = mma > smem ? mma : smem;
+            const double t = (double)((tiles + resident - 1) / resident) * (3.0 * (double)((chunks + s - 1) / s) * atom + 400.0) +
+                             4.0 * bn + (s > 1 ? 1500.0 + 4.0 * bn : 0.0);
+            if (t < best_t) { best_t = t; best.bn = bn; best.n_tiles = (int)n_tiles; best.splits = s; }
+        }
+    }
+    // narrow tiles are bound by the issue of their MMAs: one barrier per chunk instead of one per atom
+    best.b_step = best.bn <= 128 ? 3 : 1;
+    best.a_stages = best.bn <= 96 ? 3 : 2;
+    const int stage = best.bn * BK * best.b_step;
+    int b = (SMEM_LIMIT - SMEM_FIXED - best.a_stages * A_CHUNK_BYTES) / stage;
+    best.b_stages = b > B_MAX ? B_MAX : b;
+    best.smem = (size_t)best.a_stages * A_CHUNK_BYTES + (size_t)best.b_stages * stage + SMEM_FIXED;
+    return best;
+}
+
+int resident_clusters(int splits) {
+    static std::atomic<int> known[64][MAX_SPLITS + 1];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return sm_count() / (2 * splits + 1);
+    int n = known[dev][splits].load(std::memory_order_relaxed);
+    if (n > 0) return n;
+    auto kern = gemm_trit_tc_kernel<__nv_bfloat16, 1>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(2 * splits), 1, 1);
+    cfg.blockDim = dim3(NUM_THREADS, 1, 1);
+    cfg.dynamicSmemBytes = SMEM_LIMIT;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = (unsigned)(2 * splits);
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 1) {
+        (void)cudaGetLastError();
+        n = sm_count() / (2 * splits + 1);
+    }
+    known[dev][splits].store(n, std::memory_order_relaxed);
+    return n;
+}
+
+template <typename CT, int FMT>
+int launch_tc(const TcShape &shape, const CUtensorMap &mw, const CUtensorMap &mx, const TcOutMaps &om, const TcParams &p, cudaStream_t st) {
+    auto kern = gemm_trit_tc_kernel<CT, FMT>;
     // the shared-memory limit is a per-device attribute of the function: set it once on every device
     static std::atomic<bool> configured[64];
     int dev = 0;
     T81_CUDA_TRY(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64 || !configured[dev].load(std::memory_order_acquire)) {
-        T81_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+        T81_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT));
         if (dev >= 0 && dev < 64) configured[dev].store(true, std::memory_order_release);
     }
     const int tiles = p.m_tiles * p.n_tiles;
-    const int sms = sm_count();
-    const int grid = tiles < sms ? tiles : sms;
-    kern<<<grid, NUM_THREADS, SMEM_BYTES, st>>>(mw, mx, om, p);
-    T81_LAUNCH_CHECK("gemm_trit_tc_kernel");
+    const int clusters = p.one_tile ? tiles : resident_clusters(1);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(clusters * 2 * p.splits), 1, 1);
+    cfg.blockDim = dim3(NUM_THREADS, 1, 1);
+    cfg.dynamicSmemBytes = shape.smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)(2 * p.splits);
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    T81_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, mw, mx, om, p));
     return T81B200_OK;
 }
 
-template <int PLANES, int NSPLIT>
-int launch_tc_ct(int c_dtype, const CUtensorMap &mw, const CUtensorMap &mx, const TcOutMaps &om, const TcParams &p, cudaStream_t st) {
+template <int FMT>
+int launch_tc_ct(int c_dtype, const TcShape &shape, const CUtensorMap &mw, const CUtensorMap &mx, const TcOutMaps &om, const TcParams &p, cudaStream_t st) {
     switch (c_dtype) {
-        case T81B200_F32: return launch_tc<float, PLANES, NSPLIT>(mw, mx, om, p, st);
-        case T81B200_BF16: return launch_tc<__nv_bfloat16, PLANES, NSPLIT>(mw, mx, om, p, st);
-        case T81B200_F16: return launch_tc<__half, PLANES, NSPLIT>(mw, mx, om, p, st);
+        case T81B200_F32: return launch_tc<float, FMT>(shape, mw, mx, om, p, st);
+        case T81B200_BF16: return launch_tc<__nv_bfloat16, FMT>(shape, mw, mx, om, p, st);
+        case T81B200_F16: return launch_tc<__half, FMT>(shape, mw, mx, om, p, st);
     }
     return fail(T81B200_EINVAL, "gemm_trit: unknown output dtype %d", c_dtype);
 }
 
-// Pre-pass for activations the TMA path cannot read directly (fp32 / fp16 values, the
-// (K, N) layout, unaligned rows): writes token-major bf16 planes into scratch memory,
-//   plane 0 = bf16(x), plane 1 = bf16(x - plane 0)      (PLANES == 2)
-// as scratch[plane][token][k], row length kpad.  32 x 32 tiles through shared memory so
-// that both the read (along n for KN, along k for NK) and the write (along k) coalesce.
-template <typename BT, int PLANES>
-__global__ void __launch_bounds__(256) stage_planes_kernel(const BT *__restrict__ B, int64_t sbk, int64_t sbn, int64_t N,
-                                                           int64_t K, __nv_bfloat16 *__restrict__ out, int64_t kpad,
-                                                           int64_t plane_elems) {
-    __shared__ float tile[32][33];
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
-    const int64_t n0 = (int64_t)blockIdx.x * 32, k0 = (int64_t)blockIdx.y * 32;
-    const bool k_fast = sbk == 1;  // NK layout: k is the contiguous index of the source
+// Pre-pass for activations TMA cannot read in place: token-major rows of kpad elements in scratch memory.  16-bit
+// values are copied bit for bit; fp32 values become PLANES bf16 planes, plane i = bf16(x - planes before it).
+// Bound by memory: every element is read once and written once (PLANES x 2 bytes).
+template <int PLANES>
+__device__ __forceinline__ void store_planes(const float (&v)[4], __nv_bfloat16 *out, int64_t plane_elems) {
+    float r[4] = {v[0], v[1], v[2], v[3]};
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int a = ty + 8 * i;
-        const int64_t n = k_fast ? n0 + a : n0 + tx, k = k_fast ? k0 + tx : k0 + a;
-        float v = 0.0f;
-        if (n < N && k < K) v = to_float<BT>(B[k * sbk + n * sbn]);
-        if (k_fast) tile[a][tx] = v; else tile[tx][a] = v;  // tile[n][k]
+    for (int pl = 0; pl < PLANES; ++pl) {
+        __nv_bfloat162 a = __floats2bfloat162_rn(r[0], r[1]), b = __floats2bfloat162_rn(r[2], r[3]);
+        *reinterpret_cast<uint2 *>(out + pl * plane_elems) = make_uint2(bf162_bits(a), bf162_bits(b));
+        r[0] -= __low2float(a); r[1] -= __high2float(a); r[2] -= __low2float(b); r[3] -= __high2float(b);
+    }
+}
+
+// (N, K) layout: a thread moves four consecutive k of one token; whole 16- / 8-byte loads where the rows allow them.
+template <typename T, int PLANES>
+__global__ void __launch_bounds__(256) stage_rows_kernel(const T *__restrict__ B, int64_t ldb, int64_t K, __nv_bfloat16 *__restrict__ out,
+                                                         int64_t kpad, int64_t plane_elems, bool vec) {
+    const int64_t n = blockIdx.x, k = ((int64_t)blockIdx.y * 256 + threadIdx.x) * 4;
+    if (k >= kpad) return;
+    const T *src = B + n * ldb + k;
+    __nv_bfloat16 *dst = out + n * kpad + k;
+    if constexpr (PLANES == 0) {  // bit copy of a 16-bit type
+        uint16_t e[4] = {0, 0, 0, 0};
+        const uint16_t *s16 = reinterpret_cast<const uint16_t *>(src);
+        if (vec && k + 4 <= K) *reinterpret_cast<uint2 *>(e) = *reinterpret_cast<const uint2 *>(src);
+        else
+#pragma unroll
+            for (int i = 0; i < 4; ++i) if (k + i < K) e[i] = s16[i];
+        *reinterpret_cast<uint2 *>(dst) = *reinterpret_cast<const uint2 *>(e);
+    } else {
+        float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        if (vec && k + 4 <= K) *reinterpret_cast<float4 *>(v) = *reinterpret_cast<const float4 *>(src);
+        else
+#pragma unroll
+            for (int i = 0; i < 4; ++i) if (k + i < K) v[i] = to_float<T>(src[i]);
+        store_planes<PLANES>(v, dst, plane_elems);
+    }
+}
+
+// (K, N) layout: 64 k x 32 n tiles through shared memory, so that the reads (along n) and the writes (along k) coalesce.
+template <typename T, int PLANES>
+__global__ void __launch_bounds__(256) stage_columns_kernel(const T *__restrict__ B, int64_t ldb, int64_t N, int64_t K, __nv_bfloat16 *__restrict__ out,
+                                                            int64_t kpad, int64_t plane_elems) {
+    __shared__ T tile[32][65];
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
+    const int64_t n0 = (int64_t)blockIdx.x * 32, k0 = (int64_t)blockIdx.y * 64;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int64_t k = k0 + ty + 8 * i, n = n0 + tx;
+        tile[tx][ty + 8 * i] = n < N && k < K ? B[k * ldb + n] : from_float<T>(0.0f);
     }
     __syncthreads();
+    const int kq = (threadIdx.x & 15) * 4;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int a = ty + 8 * i;
-        const int64_t n = n0 + a, k = k0 + tx;
-        if (n < N && k < kpad) {
-            const float v = tile[a][tx];
-            const __nv_bfloat16 hi = __float2bfloat16_rn(v);
-            out[n * kpad + k] = hi;
-            if (PLANES == 2) out[plane_elems + n * kpad + k] = __float2bfloat16_rn(v - __bfloat162float(hi));
+    for (int i = 0; i < 2; ++i) {
+        const int a = (threadIdx.x >> 4) + 16 * i;
+        const int64_t n = n0 + a, k = k0 + kq;
+        if (n >= N || k >= kpad) continue;
+        __nv_bfloat16 *dst = out + n * kpad + k;
+        if constexpr (PLANES == 0) {
+            T e[4] = {tile[a][kq], tile[a][kq + 1], tile[a][kq + 2], tile[a][kq + 3]};
+            *reinterpret_cast<uint2 *>(dst) = *reinterpret_cast<const uint2 *>(e);
+        } else {
+            const float v[4] = {to_float<T>(tile[a][kq]), to_float<T>(tile[a][kq + 1]), to_float<T>(tile[a][kq + 2]), to_float<T>(tile[a][kq + 3])};
+            store_planes<PLANES>(v, dst, plane_elems);
         }
     }
 }
 
-template <typename BT>
-int launch_stage(const void *B, int layout, int64_t ldb, int64_t N, int64_t K, int planes, __nv_bfloat16 *out,
-                 int64_t kpad, int64_t plane_elems, cudaStream_t st) {
-    const int64_t sbk = layout == T81B200_LAYOUT_KN ? ldb : 1, sbn = layout == T81B200_LAYOUT_KN ? 1 : ldb;
-    dim3 grid((unsigned)((N + 31) / 32), (unsigned)((kpad + 31) / 32));
-    if (grid.y > 65535u) return fail(T81B200_ELIMIT, "gemm_trit: K too large");
-    if (planes == 2)
-        stage_planes_kernel<BT, 2><<<grid, 256, 0, st>>>(static_cast<const BT *>(B), sbk, sbn, N, K, out, kpad, plane_elems);
-    else
-        stage_planes_kernel<BT, 1><<<grid, 256, 0, st>>>(static_cast<const BT *>(B), sbk, sbn, N, K, out, kpad, plane_elems);
-    T81_LAUNCH_CHECK("stage_planes_kernel");
+template <typename T, int PLANES>
+int launch_stage(const void *B, int layout, int64_t ldb, int64_t N, int64_t K, __nv_bfloat16 *out, int64_t kpad, cudaStream_t st) {
+    const T *src = static_cast<const T *>(B);
+    const int64_t plane_elems = N * kpad;
+    if (layout == T81B200_LAYOUT_KN) {
+        const dim3 grid((unsigned)((N + 31) / 32), (unsigned)((kpad + 63) / 64));
+        if (grid.y > 65535u) return fail(T81B200_ELIMIT, "gemm_trit: K too large");
+        stage_columns_kernel<T, PLANES><<<grid, 256, 0, st>>>(src, ldb, N, K, out, kpad, plane_elems);
+        T81_LAUNCH_CHECK("stage_columns_kernel");
+    } else {
+        const dim3 grid((unsigned)N, (unsigned)((kpad + 1023) / 1024));
+        if (grid.y > 65535u) return fail(T81B200_ELIMIT, "gemm_trit: K too large");
+        const bool vec = reinterpret_cast<uintptr_t>(B) % (4 * sizeof(T)) == 0 && ldb % 4 == 0;
+        stage_rows_kernel<T, PLANES><<<grid, 256, 0, st>>>(src, ldb, K, out, kpad, plane_elems, vec);
+        T81_LAUNCH_CHECK("stage_rows_kernel");
+    }
     return T81B200_OK;
 }
 
-// How the dense operand reaches the tensor-core kernel.
-struct TcPlan {
-    bool direct;       // bf16, token-major: TMA reads the caller's buffer
-    int planes;        // 1 or 2
-    int bn;            // tokens per tile
-    int64_t kpad;      // scratch row length (elements)
-    int64_t rows_pad;  // scratch rows per plane (a whole number of tiles)
-    size_t scratch_bytes;
-};
-
-TcPlan make_plan(int b_dtype, int layout, int64_t M, int64_t N, int64_t K) {
-    TcPlan pl;
-    pl.direct = b_dtype == T81B200_BF16 && layout == T81B200_LAYOUT_NK;
-    pl.planes = b_dtype == T81B200_BF16 ? 1 : 2;
-    pl.bn = BN_MAX / pl.planes;
-    if (pl.planes == 1 && M > 0) {
-        // 128-token tiles only when 256-token tiles would leave more than half of the SMs without any tile: every
-        // tile expands its own 128 x K block of weights, and at 128 tokens the eight converter warps cannot keep
-        // up with the MMAs (measured: 612 instead of 1128 TFLOP/s on 4096 x 4096 x 16384, 470 instead of 627 on
-        // 3072 x 3072 x 2048), so the smaller tile pays only where the extra expansions run on idle SMs
-        // (1024 x 4096 x 1024: 39.5 instead of 42.6 us).  T81B200_TC_TILE_TOKENS=128|256 (read once) forces one.
-        static const int forced = [] { const char *e = getenv("T81B200_TC_TILE_TOKENS"); return e ? atoi(e) : 0; }();
-        const int64_t sms = sm_count(), tiles256 = ((M + BM - 1) / BM) * ((N + 255) / 256);
-        if (forced == 128 || (forced == 0 && tiles256 * 2 <= sms && N > 128)) pl.bn = 128;
-    }
-    pl.kpad = (K + 7) & ~(int64_t)7;
-    pl.rows_pad = (N + pl.bn - 1) / pl.bn * pl.bn;
-    pl.scratch_bytes = pl.direct ? 0 : (size_t)pl.planes * pl.rows_pad * pl.kpad * 2;
-    return pl;
+// 16-bit token-major rows that TMA can read where they are.
+bool reads_in_place(const void *B, int b_dtype, int layout, int64_t ldb) {
+    return b_dtype != T81B200_F32 && layout == T81B200_LAYOUT_NK && reinterpret_cast<uintptr_t>(B) % 16 == 0 && (ldb * 2) % 16 == 0;
 }
+
+int64_t scratch_row(int64_t K) { return (K + 7) & ~(int64_t)7; }
+size_t scratch_size(int b_dtype, int64_t N, int64_t K) { return (size_t)(b_dtype == T81B200_F32 ? 2 : 1) * N * scratch_row(K) * 2; }
 
 }  // namespace
 
-// The tensor-core path reads bf16 token-major activations in place; other dtypes and the
-// (K, N) layout go through the staging pre-pass into scratch memory first.  Small problems
-// stay on the general kernel (they are launch-bound either way).
-bool gemm_trit_tc_eligible(int b_dtype, int layout, int c_dtype, int64_t M, int64_t N, int64_t K) {
-    (void)c_dtype;
-    if (M < 1 || N < 1 || K < 1 || M >= (1ll << 31) || N >= (1ll << 31) || K >= (1ll << 31)) return false;
-    const bool direct = b_dtype == T81B200_BF16 && layout == T81B200_LAYOUT_NK;
-    if (direct) return N >= 1;  // the dispatcher sends N <= 16 to the streaming kernel first
-    return (double)M * (double)N * (double)K >= 1.6e7 && N >= 8;
+bool gemm_trit_tc_eligible(int64_t M, int64_t N, int64_t K) {
+    return M >= 1 && N >= 1 && K >= 1 && M < (1ll << 31) && N < (1ll << 29) && K < (1ll << 31);
 }
 
-size_t gemm_trit_tc_workspace(int b_dtype, int layout, int c_dtype, int64_t M, int64_t N, int64_t K) {
-    (void)c_dtype; (void)M;
-    return make_plan(b_dtype, layout, 0, N, K).scratch_bytes;
+// Scratch bytes for activations that cannot be read in place.  What the C entry points promise for bf16 token-major
+// activations (no workspace, whatever their alignment) is kept by gemm_trit_local, which sends unaligned ones without
+// a workspace to the general kernel.
+size_t gemm_trit_tc_scratch(const void *B, int b_dtype, int layout, int64_t ldb, int64_t N, int64_t K) {
+    return reads_in_place(B, b_dtype, layout, ldb) ? 0 : scratch_size(b_dtype, N, K);
 }
+size_t gemm_trit_tc_scratch_most(int b_dtype, int64_t N, int64_t K) { return scratch_size(b_dtype, N, K); }
 
 int gemm_trit_tc_status(int reset) {
     int v = 0;
@@ -582,59 +765,70 @@ int gemm_trit_tc_status(int reset) {
     return v;
 }
 
-int gemm_trit_tc_launch(const uint8_t *A, const float *row_scale, const void *B, int b_dtype, int layout,
+// fmt 0: A holds packed limbs, 1: the decode-stream layout.  A is 16-byte aligned; the workspace holds
+// gemm_trit_tc_scratch bytes.
+int gemm_trit_tc_launch(int fmt, const uint8_t *A, const float *row_scale, const void *B, int b_dtype, int layout,
                         int64_t ldb, const float *bias, void *C, int c_dtype, int64_t ldc, int64_t M, int64_t N,
                         int64_t K, float alpha, float beta, void *workspace, size_t workspace_bytes, cudaStream_t st,
                         int n_peers, void *const *peer_C) {
-    const TcPlan plan = make_plan(b_dtype, layout, M, N, K);
     const void *x_ptr = B;
     int64_t x_ld = ldb, x_rows = N;
-    if (plan.direct) {
-        if (reinterpret_cast<uintptr_t>(B) % 16 != 0 || (ldb * 2) % 16 != 0)
-            return T81B200_EALIGN;  // caller falls back to the general kernel
-    } else {
-        if (!workspace || workspace_bytes < plan.scratch_bytes || reinterpret_cast<uintptr_t>(workspace) % 16 != 0)
-            return fail(T81B200_EWORKSPACE, "gemm_trit: %zu bytes of 16-byte aligned workspace needed, %zu given",
-                        plan.scratch_bytes, workspace_bytes);
+    const int planes = b_dtype == T81B200_F32 ? 2 : 1;
+    if (!reads_in_place(B, b_dtype, layout, ldb)) {
+        const size_t need = scratch_size(b_dtype, N, K);
+        if (!workspace || workspace_bytes < need || reinterpret_cast<uintptr_t>(workspace) % 16 != 0)
+            return fail(T81B200_EWORKSPACE, "gemm_trit: %zu bytes of 16-byte aligned workspace needed, %zu given", need, workspace_bytes);
         __nv_bfloat16 *scratch = static_cast<__nv_bfloat16 *>(workspace);
-        const int64_t plane_elems = plan.rows_pad * plan.kpad;
+        const int64_t kpad = scratch_row(K);
         int rc = T81B200_EINVAL;
         switch (b_dtype) {
-            case T81B200_F32: rc = launch_stage<float>(B, layout, ldb, N, K, plan.planes, scratch, plan.kpad, plane_elems, st); break;
-            case T81B200_BF16: rc = launch_stage<__nv_bfloat16>(B, layout, ldb, N, K, plan.planes, scratch, plan.kpad, plane_elems, st); break;
-            case T81B200_F16: rc = launch_stage<__half>(B, layout, ldb, N, K, plan.planes, scratch, plan.kpad, plane_elems, st); break;
+            case T81B200_F32: rc = launch_stage<float, 2>(B, layout, ldb, N, K, scratch, kpad, st); break;
+            case T81B200_BF16: case T81B200_F16: rc = launch_stage<__nv_bfloat16, 0>(B, layout, ldb, N, K, scratch, kpad, st); break;
         }
         if (rc) return rc;
-        x_ptr = scratch; x_ld = plan.kpad; x_rows = (int64_t)plan.planes * plan.rows_pad;
+        x_ptr = scratch; x_ld = kpad; x_rows = (int64_t)planes * N;
     }
-    const int64_t kl = (K + 47) / 48;
+    const TcShape shape = pick_shape(M, N, K, planes);
+    const bool f16 = b_dtype == T81B200_F16;
     CUtensorMap mw, mx;
-    if (int rc = make_map_2d(&mw, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, A, (uint64_t)kl * 16, (uint64_t)M, (uint64_t)kl * 16, 64, BM,
-                             CU_TENSOR_MAP_SWIZZLE_NONE))
-        return rc;
-    if (int rc = make_map_2d(&mx, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, x_ptr, (uint64_t)K, (uint64_t)x_rows, (uint64_t)x_ld * 2, BK,
-                             (uint32_t)plan.bn, CU_TENSOR_MAP_SWIZZLE_128B))
+    memset(&mw, 0, sizeof mw);
+    if (fmt == 0) {
+        const int64_t row_bytes = (K + 47) / 48 * 16;
+        if (int rc = make_map_2d(&mw, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, A, (uint64_t)row_bytes, (uint64_t)M, (uint64_t)row_bytes, 64, BM,
+                                 CU_TENSOR_MAP_SWIZZLE_NONE))
+            return rc;
+    }
+    if (int rc = make_map_2d(&mx, f16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, x_ptr, (uint64_t)K,
+                             (uint64_t)x_rows, (uint64_t)x_ld * 2, BK, (uint32_t)shape.bn / 2, CU_TENSOR_MAP_SWIZZLE_128B))
         return rc;
     TcParams p;
-    p.row_scale = row_scale; p.bias = bias; p.C = C; p.M = M; p.N = N; p.K = K; p.kl = kl;
+    memset(&p, 0, sizeof p);
+    p.A = A; p.row_scale = row_scale; p.bias = bias; p.C = C; p.M = M; p.N = N; p.kl = (K + 47) / 48;
     if (layout == T81B200_LAYOUT_NK) { p.c_row_stride = 1; p.c_tok_stride = ldc; }
     else { p.c_row_stride = ldc; p.c_tok_stride = 1; }
-    p.m_tiles = (int)((M + BM - 1) / BM);
-    p.n_tiles = (int)((N + plan.bn - 1) / plan.bn);
+    p.tiles32 = (int)((M + 31) / 32);
+    p.m_tiles = (int)((M + 255) / 256);
+    p.n_tiles = shape.n_tiles;
+    p.bn = shape.bn;
     p.n_atoms = (int)((K + BK - 1) / BK);
-    p.plane_rows = (int)plan.rows_pad;
-    p.alpha = alpha; p.beta = beta;
+    p.n_chunks = (int)((K + CHUNK - 1) / CHUNK);
+    p.planes = planes; p.plane_rows = (int)N;
+    p.splits = shape.splits;
+    p.a_stages = shape.a_stages; p.b_stages = shape.b_stages; p.b_step = shape.b_step;
+    p.one_tile = shape.splits > 1 || p.m_tiles * p.n_tiles <= resident_clusters(1) ? 1 : 0;
+    p.idesc = umma_instr_desc(shape.bn, f16);
+    p.one_mask = f16 ? 0xBC00BC00u : 0xFFFFFFFFu;
+    p.alpha = fmt == 1 ? 0.5f * alpha : alpha;
+    p.beta = beta;
     p.n_peers = n_peers;
-    for (int i = 0; i < T81B200_MAX_PEERS; ++i) p.peer_C[i] = i < n_peers ? peer_C[i] : nullptr;
+    for (int i = 0; i < n_peers; ++i) p.peer_C[i] = peer_C[i];
     p.c_vec = layout == T81B200_LAYOUT_KN && n_peers == 0 && reinterpret_cast<uintptr_t>(C) % 16 == 0 &&
                       (ldc * (int64_t)dtype_size(c_dtype)) % 16 == 0 ? 1 : 0;
     // TMA-store epilogue: 16-bit output, token-major C (features contiguous), no read-modify-write, and every
     // result 16-byte aligned with a 16-byte multiple as its row pitch
     TcOutMaps om;
     memset(&om, 0, sizeof om);
-    p.n_out_maps = 0;
-    const size_t esz = dtype_size(c_dtype);
-    bool tma_out = esz == 2 && layout == T81B200_LAYOUT_NK && beta == 0.0f && (ldc * 2) % 16 == 0 &&
+    bool tma_out = dtype_size(c_dtype) == 2 && layout == T81B200_LAYOUT_NK && beta == 0.0f && (ldc * 2) % 16 == 0 &&
                    reinterpret_cast<uintptr_t>(C) % 16 == 0;
     for (int i = 0; i < n_peers; ++i) tma_out = tma_out && reinterpret_cast<uintptr_t>(peer_C[i]) % 16 == 0;
     if (tma_out) {
@@ -647,8 +841,7 @@ int gemm_trit_tc_launch(const uint8_t *A, const float *row_scale, const void *B,
         }
         p.n_out_maps = 1 + n_peers;
     }
-    if (plan.planes == 2) return launch_tc_ct<2, 1>(c_dtype, mw, mx, om, p, st);
-    return plan.bn == 128 ? launch_tc_ct<1, 2>(c_dtype, mw, mx, om, p, st) : launch_tc_ct<1, 1>(c_dtype, mw, mx, om, p, st);
+    return fmt == 1 ? launch_tc_ct<1>(c_dtype, shape, mw, mx, om, p, st) : launch_tc_ct<0>(c_dtype, shape, mw, mx, om, p, st);
 }
 
 }  // namespace t81b200

@@ -196,12 +196,6 @@ __device__ __forceinline__ void lut_decode_word(uint32_t w, uint32_t lane_key, u
     o[3] = e1x; o[4] = e1y | o1x; o[5] = o1y;
 }
 
-__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
-                 : "memory");
-}
-
 template <typename XT> struct LutPlanes { static constexpr int value = 2; };
 template <> struct LutPlanes<__nv_bfloat16> { static constexpr int value = 1; };
 

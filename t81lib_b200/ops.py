@@ -190,15 +190,21 @@ def gemm_trit(packed: torch.Tensor, B: torch.Tensor, *, M: int, K: int, layout: 
     bs = bias
     if bs is not None and (bs.dtype != torch.float32 or bs.device != dev or not bs.is_contiguous()):
         bs = bs.detach().to(device=dev, dtype=torch.float32).contiguous()
-    direct = b_code == _capi.BF16 and code == _capi.LAYOUT_NK  # no scratch needed
+    # 16-bit token-major rows on 16-byte boundaries are read in place; up to 16 of them always are
+    direct = code == _capi.LAYOUT_NK and (N <= 16 or (b_code != _capi.F32 and B.data_ptr() % 16 == 0 and ldb % 8 == 0))
+
+    def scratch():
+        need = 0 if direct else _capi.lib.t81b200_gemm_trit_workspace_bytes(b_code, code, c_code, M, N, K)
+        if need == 0 and not direct and code == _capi.LAYOUT_NK and M * N * K >= 16_000_000:
+            need = N * ((K + 7) // 8 * 8) * 2  # unaligned bf16 rows: staged, as the other types are
+        return _workspace(dev, need)
     if peers:
         for t in peers:
             if tuple(t.shape) != tuple(C.shape) or t.stride() != C.stride() or t.dtype != C.dtype:
                 raise ValueError("peer results must have C's shape, strides and dtype")
         ptrs = (ctypes.c_void_p * len(peers))(*[t.data_ptr() for t in peers])
         with torch.cuda.device(dev):
-            need = 0 if direct else _capi.lib.t81b200_gemm_trit_workspace_bytes(b_code, code, c_code, M, N, K)
-            ws = _workspace(dev, need)
+            ws = scratch()
             _capi.check(_capi.lib.t81b200_gemm_trit_peers(
                 _ptr(packed), _ptr(rs), _ptr(B), b_code, code, ldb, _ptr(bs), _ptr(C), c_code, ldc,
                 M, N, K, float(alpha), float(beta), _ptr(ws), 0 if ws is None else ws.numel(), len(peers), ptrs,
@@ -210,8 +216,7 @@ def gemm_trit(packed: torch.Tensor, B: torch.Tensor, *, M: int, K: int, layout: 
             M, N, K, float(alpha), float(beta), None, 0, torch.cuda.current_stream(dev).cuda_stream))
         return C
     with torch.cuda.device(dev):
-        need = 0 if direct else _capi.lib.t81b200_gemm_trit_workspace_bytes(b_code, code, c_code, M, N, K)
-        ws = _workspace(dev, need)
+        ws = scratch()
         _capi.check(_capi.lib.t81b200_gemm_trit(
             _ptr(packed), _ptr(rs), _ptr(B), b_code, code, ldb, _ptr(bs), _ptr(C), c_code, ldc,
             M, N, K, float(alpha), float(beta), _ptr(ws), 0 if ws is None else ws.numel(), _stream(dev)))
@@ -231,28 +236,28 @@ def pack_t2(packed: torch.Tensor, rows: int, cols: int) -> torch.Tensor:
     return out
 
 
-def gemm_trit_t2_one(t2: torch.Tensor, M: int, x: torch.Tensor, K: int, row_scale: Optional[torch.Tensor] = None,
-                     bias: Optional[torch.Tensor] = None, out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
-    """``gemm_trit_t2`` for one matrix with as little host work as the call allows (the kernel runs a few
-    microseconds: list handling and conversions would outweigh it).  ``x`` is (1..16 tokens, K) with unit column
-    stride on ``t2``'s device; ``row_scale`` and ``bias`` are contiguous float32 on that device or None."""
+def linear_t2(t2: torch.Tensor, M: int, x: torch.Tensor, K: int, row_scale: Optional[torch.Tensor] = None,
+              bias: Optional[torch.Tensor] = None, out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
+    """One matrix in the decode-stream layout times any number of activation rows, with as little host work as the
+    call allows (a decode-sized kernel runs a few microseconds).  ``x`` is (tokens, K) with unit column stride on
+    ``t2``'s device; ``row_scale`` and ``bias`` are contiguous float32 on that device or None."""
     tokens = x.shape[0]
     dev = x.device
     C = torch.empty((tokens, M), dtype=out_dtype or x.dtype, device=dev)
-    vp = ctypes.c_void_p
-    a = vp(t2.data_ptr())
-    c = vp(C.data_ptr())
-    m = ctypes.c_int64(M)
-    rs = None if row_scale is None else ctypes.byref(vp(row_scale.data_ptr()))
-    bs = None if bias is None else ctypes.byref(vp(bias.data_ptr()))
-    args = (1, ctypes.byref(a), rs, bs, ctypes.byref(c), ctypes.byref(m), x.data_ptr(), _DTYPES[x.dtype],
-            x.stride(0) if tokens > 1 else max(K, 1), _DTYPES[C.dtype], M, tokens, K, 1.0, 0.0,
-            torch.cuda.current_stream(dev).cuda_stream)
+    if tokens == 0:
+        return C
+    ldx = x.stride(0) if tokens > 1 else max(K, 1)
+    code, xp = _DTYPES[x.dtype], x.data_ptr()
+    ws, need = None, _capi.lib.t81b200_linear_t2_workspace_bytes(xp, code, ldx, M, tokens, K) if tokens > 16 else 0
+    if need:
+        ws = torch.empty(need, dtype=torch.uint8, device=dev)
+    args = (t2.data_ptr(), _ptr(row_scale), _ptr(bias), C.data_ptr(), M, xp, code, ldx, _DTYPES[C.dtype], max(M, 1), tokens, K,
+            1.0, 0.0, _ptr(ws), need, torch.cuda.current_stream(dev).cuda_stream)
     if torch.cuda.current_device() == dev.index:
-        rc = _capi.lib.t81b200_gemm_trit_t2(*args)
+        rc = _capi.lib.t81b200_linear_t2(*args)
     else:
         with torch.cuda.device(dev):
-            rc = _capi.lib.t81b200_gemm_trit_t2(*args)
+            rc = _capi.lib.t81b200_linear_t2(*args)
     if rc:
         _capi.check(rc)
     return C

@@ -61,8 +61,8 @@ def _to_device_float(tensor: torch.Tensor) -> torch.Tensor:
     return tensor
 
 
-# Decode-sized products (1..16 activation rows) of a TernaryTensor run on a second copy of the weight in the
-# decode-stream layout (ops.pack_t2), made on first use: 0.25 byte per weight on top of the 0.33 of the limbs.
+# Products of a TernaryTensor run on a second copy of the weight in the decode-stream layout (ops.pack_t2), made on
+# first use: 0.25 byte per weight on top of the 0.33 of the limbs.
 # False keeps every product on the limb layout.
 DECODE_STREAM_LAYOUT = True
 
@@ -111,7 +111,7 @@ class TernaryTensor(torch.Tensor):
         tensor._base_device = packed.device
         tensor._threshold = _clamp_threshold(threshold)
         tensor._rule = rule
-        tensor._t2 = None  # the decode-stream layout, made by the first decode-sized product; False: does not apply
+        tensor._t2 = None  # the decode-stream layout, made by the first product
         return tensor
 
     @property
@@ -172,10 +172,6 @@ class TernaryTensor(torch.Tensor):
             w = w * self._row_scale.to(dtype)[:, None]
         return w
 
-    def _streams(self, tokens: int) -> bool:
-        """17..128 activation rows: slices of the streaming kernel or tensor-core tiles (the library's estimate)."""
-        return 16 < tokens <= _capi.T2_MAX_TOKENS and bool(_capi.lib.t81b200_prefers_streaming(self._rows, tokens, self._k_actual))
-
     def matmul_input(self, input: torch.Tensor, bias: Optional[torch.Tensor] = None,
                      out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
         """``input @ W.T (+ bias)`` for activations (tokens, cols) -> (tokens, rows).
@@ -187,19 +183,17 @@ class TernaryTensor(torch.Tensor):
             # inference fast path: no autograd node, no device shuffling — one kernel call
             if input.shape[1] != self._k_actual:
                 raise ValueError("rhs dimension does not match ternary weight width")
-            if DECODE_STREAM_LAYOUT and (1 <= input.shape[0] <= 16 or self._streams(input.shape[0])) and self._t2 is not False and self._rows > 0 and self._k_actual > 0:
-                # decode-sized: the weight in the decode-stream layout (made once, a quarter fewer bytes to stream)
+            if DECODE_STREAM_LAYOUT and self._rows > 0 and self._k_actual > 0:
+                # the weight in the decode-stream layout (made once): a quarter fewer bytes to stream, and two
+                # instructions per pair of trits to expand
                 if self._t2 is None:
                     self._t2 = ops.pack_t2(self._packed, self._rows, self._k_actual)
-                try:
-                    x = input if input.stride(1) == 1 else input.contiguous()
-                    if x.dtype not in (torch.float32, torch.bfloat16, torch.float16):
-                        raise ValueError(f"x must be float32, bfloat16 or float16, got {x.dtype}")
-                    if bias is not None and (bias.dtype != torch.float32 or bias.device != x.device or not bias.is_contiguous()):
-                        bias = bias.detach().to(device=x.device, dtype=torch.float32).contiguous()
-                    return ops.gemm_trit_t2_one(self._t2, self._rows, x, self._k_actual, self._row_scale, bias, out_dtype)
-                except _capi.LimitError:
-                    self._t2 = False  # a contraction too long for that kernel: the limb layout serves it
+                x = input if input.stride(1) == 1 else input.contiguous()
+                if x.dtype not in (torch.float32, torch.bfloat16, torch.float16):
+                    raise ValueError(f"x must be float32, bfloat16 or float16, got {x.dtype}")
+                if bias is not None and (bias.dtype != torch.float32 or bias.device != x.device or not bias.is_contiguous()):
+                    bias = bias.detach().to(device=x.device, dtype=torch.float32).contiguous()
+                return ops.linear_t2(self._t2, self._rows, x, self._k_actual, self._row_scale, bias, out_dtype)
             return ops.gemm_trit(self._packed, input, M=self._rows, K=self._k_actual, layout="nk",
                                  row_scale=self._row_scale, bias=bias, out_dtype=out_dtype)
         return _TernaryLinearFunction.apply(self, input, bias, out_dtype)

@@ -1,0 +1,51 @@
+"""The paired tensor-core kernel behind ``ops.linear_t2`` (decode-stream layout) and ``ops.gemm_trit`` (limbs) at the
+edges of its tiles, contraction splits and staging rules, against the CPU oracle."""
+
+import numpy as np
+import pytest
+import torch
+
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def dev(lib_built):
+    from t81lib_b200 import _capi
+    assert _capi.device_available(), _capi.last_error()
+    return torch.device("cuda", 0)
+
+
+# (rows, K, tokens): one row and column; 17 tokens on a 32-token tile; two CTAs with the second one empty (rows <= 128) or
+# nearly so (129, 257); K below, at and just past an atom (64) and a chunk (192); splits of 2 to 4 with unequal shares; a
+# 224- and a 256-token tile; several tiles per cluster with a ragged last one in both directions
+SHAPES = [(1, 1, 17), (128, 64, 32), (129, 65, 33), (257, 192, 64), (256, 193, 96), (300, 385, 97), (512, 1001, 129),
+          (1024, 4096, 40), (4096, 1536, 80), (100, 14336, 18), (260, 256, 777), (9500, 200, 1100)]
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("rows,K,tokens", SHAPES)
+def test_products_match_the_oracle(dev, rows, K, tokens, dtype):
+    from t81lib_b200 import _capi, ops
+    rng = np.random.default_rng(rows + 31 * K + 977 * tokens)
+    trits = rng.integers(-1, 2, (rows, K)).astype(np.int8)
+    limbs = oracle.pack_trits_rowwise(trits)
+    scale, bias = rng.uniform(0.01, 0.03, rows).astype(np.float32), rng.normal(0, 0.01, rows).astype(np.float32)
+    packed, sd, bd = (torch.from_numpy(a).to(dev) for a in (limbs, scale, bias))
+    t2 = ops.pack_t2(packed, rows, K)
+    wide = torch.from_numpy(rng.normal(size=(tokens, K + 3)).astype(np.float32)).to(dev).to(dtype)
+    # products are exact, sums fp32 in another order: about sqrt(K) ulp of the sum's size; fp32 activations enter with 16
+    # mantissa bits (2^-17 each, averaging out over K)
+    tol = 2e-5 if dtype != torch.float32 else 5e-5
+    for x in (wide[:, :K].contiguous(), wide[:, 1:K + 1]):  # rows on 16-byte boundaries where K allows, and not
+        want = (x.double().cpu().numpy() @ trits.T.astype(np.float64)) * scale + bias
+        rms = float(np.sqrt(np.mean(want ** 2)))
+        y = ops.linear_t2(t2, rows, x, K, sd, bd, torch.float32)
+        z = ops.gemm_trit(packed, x, M=rows, K=K, layout="nk", row_scale=sd, bias=bd, out_dtype=torch.float32)
+        assert np.abs(y.cpu().numpy() - want).max() < tol * rms
+        assert np.abs(z.cpu().numpy() - want).max() < tol * rms
+        # 16-bit results: one rounding of the fp32 ones (TMA-store epilogue where rows are a multiple of 8)
+        h = ops.linear_t2(t2, rows, x, K, sd, bd, torch.bfloat16)
+        assert torch.equal(h, y.to(torch.bfloat16))
+    assert _capi.kernel_status(reset=True) == 0
