@@ -331,11 +331,12 @@ T81B200_API int t81b200_prefers_streaming(int64_t M, int64_t N, int64_t K);
 T81B200_API int t81b200_pack_t2(const uint8_t *packed, int64_t rows, int64_t cols, uint8_t *t2, void *stream);
 /* One matrix in the decode-stream layout times any number of activation rows (token-major B, C): the streaming kernel
  * up to 16 rows, tensor-core tiles beyond.  16-bit rows that start on 16-byte boundaries are read where they are;
- * fp32 and unaligned ones are staged in the workspace (16-byte aligned, linear_t2_workspace_bytes for this very B). */
-T81B200_API size_t t81b200_linear_t2_workspace_bytes(const void *B, int b_dtype, int64_t ldb, int64_t M, int64_t N, int64_t K);
+ * fp32 and unaligned ones are staged in the workspace (16-byte aligned, linear_t2_workspace_bytes for this very B).
+ * fp32_planes: bf16 planes that fp32 activations enter the products as — 2: 16 mantissa bits, 3: all of them. */
+T81B200_API size_t t81b200_linear_t2_workspace_bytes(const void *B, int b_dtype, int64_t ldb, int64_t M, int64_t N, int64_t K, int fp32_planes);
 T81B200_API int t81b200_linear_t2(const uint8_t *t2, const float *row_scale, const float *bias, void *C, int64_t M, const void *B,
                                   int b_dtype, int64_t ldb, int c_dtype, int64_t ldc, int64_t N, int64_t K, float alpha, float beta,
-                                  void *workspace, size_t workspace_bytes, void *stream);
+                                  int fp32_planes, void *workspace, size_t workspace_bytes, void *stream);
 /* gemm_trit_t2 for ONE matrix of a column-sharded Linear: t81b200_gemm_trit_peers (see there for peer_C, sync_local
  * and sync_slots) with the rank's rows given in the decode-stream layout; 1..16 rows of B, token-major. */
 T81B200_API int t81b200_gemm_trit_t2_peers(const uint8_t *t2, const float *row_scale, const float *bias, void *C, int64_t M,
@@ -361,6 +362,19 @@ T81B200_API int t81b200_qat_update_scale(const void *w, int w_dtype, int64_t row
                                          float *state, void *stream);
 T81B200_API int t81b200_qat_quantize_pack(const void *w, int w_dtype, int64_t rows, int64_t cols, int64_t ld, float threshold,
                                           const float *scale, uint8_t *packed, float *row_scale, void *stream);
+/* Training step on the decode-stream layout.  qat_quantize_t2: the same quantiser (fp32 weight) writing the layout of the
+ * weight and, unless null, of its transpose (what the input gradient multiplies with); scale_out receives n_scales
+ * copies of the scale (the row scales of either product).  qat_weight_grad: out (rows, cols) fp32, contiguous, =
+ * slope * g^T x for token-major g (tokens, rows) and x (tokens, cols) of one dtype, slope = 2 where |w / scale| < 0.5 and
+ * 0 elsewhere (t81/nn/linear.py:72-80 through t81/qat.py:28-57); 16-bit operands are multiplied exactly, fp32 ones in
+ * three bf16 planes; operands that TMA cannot read where they are need the workspace (256-byte aligned). */
+T81B200_API int t81b200_qat_quantize_t2(const float *w, int64_t rows, int64_t cols, int64_t ld, float threshold, const float *scale, uint8_t *t2,
+                                        uint8_t *t2_transposed, float *scale_out, int64_t n_scales, void *stream);
+T81B200_API size_t t81b200_qat_weight_grad_workspace_bytes(const void *g, int64_t ldg, const void *x, int64_t ldx, int dtype, int64_t tokens,
+                                                           int64_t rows, int64_t cols);
+T81B200_API int t81b200_qat_weight_grad(const void *g, int64_t ldg, const void *x, int64_t ldx, int dtype, int64_t tokens, int64_t rows, int64_t cols,
+                                        const float *w, int64_t ldw, const float *scale, float *out, void *workspace, size_t workspace_bytes,
+                                        void *stream);
 
 /* Transcoders between the packed-limb layout and the GGUF ternary block formats the reference writes and reads
  * on the CPU through float arrays (t81/gguf.py:518-662: _quantize_blocks_tq1 / _tq2, _dequantize_blocks_tq1 / _tq2;

@@ -28,7 +28,7 @@ EXPORTS = (
     "t81b200_copy_columns", "t81b200_gemm_trit_peers", "t81b200_exchange_wait", "t81b200_hint_independent",
     "t81b200_gemm_limb_auto", "t81b200_gemm_trit_auto", "t81b200_elementwise", "t81b200_elementwise_auto",
     "t81b200_release_staging", "t81b200_exchange_signal", "t81b200_gemm_trit_grouped", "t81b200_t2_bytes", "t81b200_pack_t2", "t81b200_prefers_streaming", "t81b200_gemm_trit_t2", "t81b200_gemm_trit_t2_peers", "t81b200_linear_t2_workspace_bytes", "t81b200_linear_t2", "t81b200_tq_bytes", "t81b200_packed_to_tq", "t81b200_tq_to_packed",
-    "t81b200_qat_update_scale", "t81b200_qat_quantize_pack",
+    "t81b200_qat_update_scale", "t81b200_qat_quantize_pack", "t81b200_qat_quantize_t2", "t81b200_qat_weight_grad_workspace_bytes", "t81b200_qat_weight_grad",
 )
 TQ1_0, TQ2_0 = 0, 1
 T2_MAX_TOKENS = 128  # T81B200_T2_MAX_ROWS
@@ -82,6 +82,10 @@ def _load() -> ctypes.CDLL:
     lib.t81b200_elementwise_auto.argtypes = [ci, vp, vp, vp, vp, i64, f32, f32]
     lib.t81b200_qat_update_scale.argtypes = [vp, ci, i64, i64, i64, f32, vp, vp]
     lib.t81b200_qat_quantize_pack.argtypes = [vp, ci, i64, i64, i64, f32, vp, vp, vp, vp]
+    lib.t81b200_qat_quantize_t2.argtypes = [vp, i64, i64, i64, f32, vp, vp, vp, vp, i64, vp]
+    lib.t81b200_qat_weight_grad_workspace_bytes.argtypes = [vp, i64, vp, i64, ci, i64, i64, i64]
+    lib.t81b200_qat_weight_grad_workspace_bytes.restype = ctypes.c_size_t
+    lib.t81b200_qat_weight_grad.argtypes = [vp, i64, vp, i64, ci, i64, i64, i64, vp, i64, vp, vp, vp, ctypes.c_size_t, vp]
     lib.t81b200_tq_bytes.argtypes = [ci, i64, i64]
     lib.t81b200_tq_bytes.restype = i64
     lib.t81b200_packed_to_tq.argtypes = [vp, vp, i64, i64, ci, vp, vp]
@@ -94,9 +98,9 @@ def _load() -> ctypes.CDLL:
     lib.t81b200_gemm_trit_t2.argtypes = lib.t81b200_gemm_trit_grouped.argtypes
     lib.t81b200_gemm_trit_t2_peers.argtypes = [vp, vp, vp, vp, i64, vp, ci, i64, ci, i64, i64, i64, f32, f32, ci,
                                                ctypes.POINTER(vp), vp, ctypes.POINTER(vp), vp]
-    lib.t81b200_linear_t2_workspace_bytes.argtypes = [vp, ci, i64, i64, i64, i64]
+    lib.t81b200_linear_t2_workspace_bytes.argtypes = [vp, ci, i64, i64, i64, i64, ci]
     lib.t81b200_linear_t2_workspace_bytes.restype = ctypes.c_size_t
-    lib.t81b200_linear_t2.argtypes = [vp, vp, vp, vp, i64, vp, ci, i64, ci, i64, i64, i64, f32, f32, vp, ctypes.c_size_t, vp]
+    lib.t81b200_linear_t2.argtypes = [vp, vp, vp, vp, i64, vp, ci, i64, ci, i64, i64, i64, f32, f32, ci, vp, ctypes.c_size_t, vp]
     lib.t81b200_t2_bytes.argtypes = [i64, i64]
     lib.t81b200_t2_bytes.restype = i64
     lib.t81b200_pack_t2.argtypes = [vp, i64, i64, vp, vp]

@@ -74,14 +74,15 @@ int gemm_trit_simt_launch(const uint8_t *A, const float *row_scale, const void *
                           int64_t ldb, const float *bias, void *C, int c_dtype, int64_t ldc, int64_t M,
                           int64_t N, int64_t K, float alpha, float beta, cudaStream_t st);
 bool gemm_trit_tc_eligible(int64_t M, int64_t N, int64_t K);
-size_t gemm_trit_tc_scratch(const void *B, int b_dtype, int layout, int64_t ldb, int64_t N, int64_t K);
-size_t gemm_trit_tc_scratch_most(int b_dtype, int64_t N, int64_t K);
-int gemm_trit_tc_launch(int fmt, const uint8_t *A, const float *row_scale, const void *B, int b_dtype, int layout,
+size_t gemm_trit_tc_scratch(const void *B, int b_dtype, int layout, int64_t ldb, int64_t N, int64_t K, int planes);
+size_t gemm_trit_tc_scratch_most(int b_dtype, int64_t N, int64_t K, int planes);
+int gemm_trit_tc_launch(int fmt, int fp32_planes, const uint8_t *A, const float *row_scale, const void *B, int b_dtype, int layout,
                         int64_t ldb, const float *bias, void *C, int c_dtype, int64_t ldc, int64_t M, int64_t N,
                         int64_t K, float alpha, float beta, void *workspace, size_t workspace_bytes,
                         cudaStream_t st, int n_peers, void *const *peer_C);
 
 int gemm_trit_tc_status(int reset);
+int gemm_wgrad_status(int reset);
 int gemv_trit_status(int reset);
 int gemv_trit_lut_status(int reset);
 int quantize_pack_status(int reset);
@@ -99,6 +100,8 @@ extern "C" int t81b200_kernel_status(int reset) {
     const int gv = gemv_trit_status(reset);
     const int lut = gemv_trit_lut_status(reset);
     const int qp = quantize_pack_status(reset);
+    const int wg = gemm_wgrad_status(reset);
+    if (wg != 0) return wg;
     return tc != 0 ? tc : (gv != 0 ? gv : (lut != 0 ? lut : qp));
 }
 
@@ -133,7 +136,7 @@ extern "C" size_t t81b200_gemm_trit_workspace_bytes(int b_dtype, int layout, int
     if (M <= 0 || N <= 0 || K < 0) return 0;
     if (b_dtype == T81B200_BF16 && layout == T81B200_LAYOUT_NK) return 0;
     if (!gemm_trit_tc_eligible(M, N, K) || !worth_staging(M, N, K)) return 0;
-    return gemm_trit_tc_scratch_most(b_dtype, N, K);
+    return gemm_trit_tc_scratch_most(b_dtype, N, K, 2);
 }
 
 // Contractions up to this length always have a launch shape of the streaming kernel (16 fp32 rows of B included).
@@ -283,10 +286,10 @@ static int gemm_trit_local(const uint8_t *A, const float *row_scale, const void 
     }
 
     if (a_aligned && gemm_trit_tc_eligible(M, N, K)) {
-        const size_t need = gemm_trit_tc_scratch(B, b_dtype, layout, ldb, N, K);
+        const size_t need = gemm_trit_tc_scratch(B, b_dtype, layout, ldb, N, K, 2);
         const bool have = workspace && workspace_bytes >= need && reinterpret_cast<uintptr_t>(workspace) % 16 == 0;
         if (need == 0 || (have && worth_staging(M, N, K))) {
-            const int rc = gemm_trit_tc_launch(0, A, row_scale, B, b_dtype, layout, ldb, bias, C, c_dtype, ldc, M, N, K, alpha, beta,
+            const int rc = gemm_trit_tc_launch(0, 2, A, row_scale, B, b_dtype, layout, ldb, bias, C, c_dtype, ldc, M, N, K, alpha, beta,
                                                workspace, workspace_bytes, st, ctx ? ctx->n_peers : 0, ctx ? ctx->peer_C : nullptr);
             if (ctx) ctx->peers_done = rc == T81B200_OK;
             return rc;
@@ -336,29 +339,33 @@ extern "C" int t81b200_gemm_trit_t2(int n_group, const uint8_t *const *t2, const
     return rc;
 }
 
-extern "C" size_t t81b200_linear_t2_workspace_bytes(const void *B, int b_dtype, int64_t ldb, int64_t M, int64_t N, int64_t K) {
-    if (M <= 0 || N <= 0 || K <= 0 || !valid_dtype(b_dtype) || (N <= 16 && K <= kT2StreamingMaxK)) return 0;
-    return gemm_trit_tc_scratch(B, b_dtype, T81B200_LAYOUT_NK, ldb, N, K);
+// Decode-sized calls the streaming kernel takes: up to 16 rows, fp32 ones in two planes.
+static bool linear_t2_streams(int b_dtype, int64_t N, int fp32_planes) { return N <= 16 && (b_dtype != T81B200_F32 || fp32_planes <= 2); }
+
+extern "C" size_t t81b200_linear_t2_workspace_bytes(const void *B, int b_dtype, int64_t ldb, int64_t M, int64_t N, int64_t K, int fp32_planes) {
+    if (M <= 0 || N <= 0 || K <= 0 || !valid_dtype(b_dtype) || (linear_t2_streams(b_dtype, N, fp32_planes) && K <= kT2StreamingMaxK)) return 0;
+    return gemm_trit_tc_scratch(B, b_dtype, T81B200_LAYOUT_NK, ldb, N, K, fp32_planes);
 }
 
 extern "C" int t81b200_linear_t2(const uint8_t *t2, const float *row_scale, const float *bias, void *C, int64_t M, const void *B,
                                  int b_dtype, int64_t ldb, int c_dtype, int64_t ldc, int64_t N, int64_t K, float alpha, float beta,
-                                 void *workspace, size_t workspace_bytes, void *stream) {
+                                 int fp32_planes, void *workspace, size_t workspace_bytes, void *stream) {
     if (M <= 0 || K <= 0 || N < 0) return fail(T81B200_EINVAL, "linear_t2: dimensions must be positive");
     if (!valid_dtype(b_dtype) || !valid_dtype(c_dtype)) return fail(T81B200_EINVAL, "gemm_trit: unknown dtype");
+    if (fp32_planes != 2 && fp32_planes != 3) return fail(T81B200_EINVAL, "linear_t2: fp32 activations take 2 or 3 planes");
     if (ldb < K || ldc < M) return fail(T81B200_EINVAL, "gemm_trit: leading dimension below the row length");
     if (N > 0 && (!t2 || !B || !C)) return fail(T81B200_EINVAL, "gemm_trit: null pointer");
     if (reinterpret_cast<uintptr_t>(t2) % 16 != 0) return fail(T81B200_EALIGN, "gemm_trit_t2: matrices must be 16-byte aligned");
     if (int rc = check_device()) return rc;
     if (N == 0) return T81B200_OK;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (N <= 16) {
+    if (linear_t2_streams(b_dtype, N, fp32_planes)) {
         const int rc = gemv_trit_lut_launch(1, 1, &t2, &row_scale, &bias, &C, &M, B, b_dtype, ldb, c_dtype, ldc, (int)N, K, alpha, beta, st, nullptr);
         if (rc != T81B200_EALIGN) return rc;  // a contraction too long for that kernel's shared memory: tiles take it
     }
     if (!gemm_trit_tc_eligible(M, N, K)) return fail(T81B200_ELIMIT, "linear_t2: dimensions beyond 2^31 (2^29 rows of B)");
-    return gemm_trit_tc_launch(1, t2, row_scale, B, b_dtype, T81B200_LAYOUT_NK, ldb, bias, C, c_dtype, ldc, M, N, K, alpha, beta, workspace,
-                               workspace_bytes, st, 0, nullptr);
+    return gemm_trit_tc_launch(1, fp32_planes, t2, row_scale, B, b_dtype, T81B200_LAYOUT_NK, ldb, bias, C, c_dtype, ldc, M, N, K, alpha, beta,
+                               workspace, workspace_bytes, st, 0, nullptr);
 }
 
 extern "C" int t81b200_gemm_trit_t2_peers(const uint8_t *t2, const float *row_scale, const float *bias, void *C, int64_t M,

@@ -494,11 +494,7 @@ gemm_trit_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                     if (to == slice) continue;
                     uint32_t v[32];
                     tmem_ld32(t_lane + (uint32_t)(b * 32), v);
-                    const int slot = (b / S) * (S - 1) + (slice < to ? slice : slice - 1);
-                    uint32_t dst;
-                    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(base + (uint32_t)slot * 16384u + lane_row * 4u), "r"((uint32_t)(2 * to + half)));
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(dst + (uint32_t)i * 512u), "r"(v[i]) : "memory");
+                    push_partial(v, base + partial_slot(b, S, slice, to) * 16384u + lane_row * 4u, (uint32_t)(2 * to + half));
                 }
             __syncthreads();
             cluster_barrier();
@@ -511,18 +507,7 @@ gemm_trit_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             for (int b = slice + S * group; b < blocks; b += 3 * S) {
                 uint32_t v[32];
                 tmem_ld32(t_lane + (uint32_t)(b * 32), v);
-                if (S > 1) {
-                    uint32_t sum[32];
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) sum[i] = 0u;
-                    for (int s = 0; s < S; ++s) {  // in rank order
-                        const float *src = reinterpret_cast<const float *>(gen_base + (size_t)((b / S) * (S - 1) + (s < slice ? s : s - 1)) * 16384) + lane_row;
-#pragma unroll
-                        for (int i = 0; i < 32; ++i) sum[i] = __float_as_uint(__uint_as_float(sum[i]) + (s == slice ? __uint_as_float(v[i]) : src[i * 128]));
-                    }
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) v[i] = sum[i];
-                }
+                if (S > 1) fold_partials(v, gen_base, b, S, slice, lane_row);
                 const uint32_t stage = b_off + (uint32_t)b * OUT_STAGE_BYTES;
                 emit_block<CT>(p, omaps, v, row0, row, scale, bias, n0 + b * 32, OutStage{gen_base + stage, base + stage, (uint32_t)(2 + group), first, false});
             }
@@ -546,10 +531,6 @@ struct TcShape {
     size_t smem = 0;
 };
 
-// Clusters of 2 * splits CTAs (one CTA per SM) that the device runs at a time: clusters do not straddle GPCs, so fewer
-// fit than the SM count suggests (74, 33, 22 and 15 for 1 to 4 splits).
-int resident_clusters(int splits);
-
 TcShape pick_shape(int64_t M, int64_t N, int64_t K, int planes) {
     const int64_t m_tiles = (M + 255) / 256, chunks = (K + CHUNK - 1) / CHUNK, least = (N + 255) / 256;
     TcShape best;
@@ -558,7 +539,7 @@ TcShape pick_shape(int64_t M, int64_t N, int64_t K, int planes) {
         const int bn = (int)(((N + want - 1) / want + 31) / 32 * 32);
         const int64_t n_tiles = (N + bn - 1) / bn, tiles = m_tiles * n_tiles;
         for (int s = 1; s <= MAX_SPLITS; ++s) {
-            const int resident = resident_clusters(s);
+            const int resident = resident_pair_clusters(s);
             if (s > chunks || (s > 1 && tiles > resident)) continue;
             const double mma = 2.0 * planes * bn, smem = 128.0 + planes * (128.0 + bn);
             const double atom = mma > smem ? mma : smem;
@@ -577,32 +558,6 @@ TcShape pick_shape(int64_t M, int64_t N, int64_t K, int planes) {
     return best;
 }
 
-int resident_clusters(int splits) {
-    static std::atomic<int> known[64][MAX_SPLITS + 1];
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return sm_count() / (2 * splits + 1);
-    int n = known[dev][splits].load(std::memory_order_relaxed);
-    if (n > 0) return n;
-    auto kern = gemm_trit_tc_kernel<__nv_bfloat16, 1>;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(2 * splits), 1, 1);
-    cfg.blockDim = dim3(NUM_THREADS, 1, 1);
-    cfg.dynamicSmemBytes = SMEM_LIMIT;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = (unsigned)(2 * splits);
-    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT) != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 1) {
-        (void)cudaGetLastError();
-        n = sm_count() / (2 * splits + 1);
-    }
-    known[dev][splits].store(n, std::memory_order_relaxed);
-    return n;
-}
-
 template <typename CT, int FMT>
 int launch_tc(const TcShape &shape, const CUtensorMap &mw, const CUtensorMap &mx, const TcOutMaps &om, const TcParams &p, cudaStream_t st) {
     auto kern = gemm_trit_tc_kernel<CT, FMT>;
@@ -615,7 +570,7 @@ int launch_tc(const TcShape &shape, const CUtensorMap &mw, const CUtensorMap &mx
         if (dev >= 0 && dev < 64) configured[dev].store(true, std::memory_order_release);
     }
     const int tiles = p.m_tiles * p.n_tiles;
-    const int clusters = p.one_tile ? tiles : resident_clusters(1);
+    const int clusters = p.one_tile ? tiles : resident_pair_clusters(1);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(clusters * 2 * p.splits), 1, 1);
     cfg.blockDim = dim3(NUM_THREADS, 1, 1);
@@ -739,21 +694,53 @@ bool reads_in_place(const void *B, int b_dtype, int layout, int64_t ldb) {
 }
 
 int64_t scratch_row(int64_t K) { return (K + 7) & ~(int64_t)7; }
-size_t scratch_size(int b_dtype, int64_t N, int64_t K) { return (size_t)(b_dtype == T81B200_F32 ? 2 : 1) * N * scratch_row(K) * 2; }
 
 }  // namespace
+
+int resident_pair_clusters(int splits) {
+    static std::atomic<int> known[64][MAX_SPLITS + 1];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return sm_count() / (2 * splits + 1);
+    int n = known[dev][splits].load(std::memory_order_relaxed);
+    if (n > 0) return n;
+    auto kern = gemm_trit_tc_kernel<__nv_bfloat16, 1>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(2 * splits), 1, 1);
+    cfg.blockDim = dim3(NUM_THREADS, 1, 1);
+    cfg.dynamicSmemBytes = SMEM_LIMIT;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = (unsigned)(2 * splits);
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 1) {
+        (void)cudaGetLastError();
+        n = sm_count() / (2 * splits + 1);
+    }
+    known[dev][splits].store(n, std::memory_order_relaxed);
+    return n;
+}
+
+int stage_planes(const void *B, int dtype, int layout, int64_t ld, int64_t tokens, int64_t K, int planes, void *scratch, cudaStream_t st) {
+    __nv_bfloat16 *out = static_cast<__nv_bfloat16 *>(scratch);
+    const int64_t kpad = scratch_row(K);
+    if (dtype != T81B200_F32) return launch_stage<__nv_bfloat16, 0>(B, layout, ld, tokens, K, out, kpad, st);
+    return planes == 3 ? launch_stage<float, 3>(B, layout, ld, tokens, K, out, kpad, st) : launch_stage<float, 2>(B, layout, ld, tokens, K, out, kpad, st);
+}
 
 bool gemm_trit_tc_eligible(int64_t M, int64_t N, int64_t K) {
     return M >= 1 && N >= 1 && K >= 1 && M < (1ll << 31) && N < (1ll << 29) && K < (1ll << 31);
 }
 
-// Scratch bytes for activations that cannot be read in place.  What the C entry points promise for bf16 token-major
-// activations (no workspace, whatever their alignment) is kept by gemm_trit_local, which sends unaligned ones without
-// a workspace to the general kernel.
-size_t gemm_trit_tc_scratch(const void *B, int b_dtype, int layout, int64_t ldb, int64_t N, int64_t K) {
-    return reads_in_place(B, b_dtype, layout, ldb) ? 0 : scratch_size(b_dtype, N, K);
+// Scratch bytes for the activations: none when they are read in place.  `planes`: bf16 planes of fp32 activations.
+size_t gemm_trit_tc_scratch_most(int b_dtype, int64_t N, int64_t K, int planes) {
+    return (size_t)(b_dtype == T81B200_F32 ? planes : 1) * N * scratch_row(K) * 2;
 }
-size_t gemm_trit_tc_scratch_most(int b_dtype, int64_t N, int64_t K) { return scratch_size(b_dtype, N, K); }
+size_t gemm_trit_tc_scratch(const void *B, int b_dtype, int layout, int64_t ldb, int64_t N, int64_t K, int planes) {
+    return reads_in_place(B, b_dtype, layout, ldb) ? 0 : gemm_trit_tc_scratch_most(b_dtype, N, K, planes);
+}
 
 int gemm_trit_tc_status(int reset) {
     int v = 0;
@@ -766,27 +753,20 @@ int gemm_trit_tc_status(int reset) {
 }
 
 // fmt 0: A holds packed limbs, 1: the decode-stream layout.  A is 16-byte aligned; the workspace holds
-// gemm_trit_tc_scratch bytes.
-int gemm_trit_tc_launch(int fmt, const uint8_t *A, const float *row_scale, const void *B, int b_dtype, int layout,
+// gemm_trit_tc_scratch bytes for `fp32_planes` (2: 16 mantissa bits of fp32 activations, 3: all of them).
+int gemm_trit_tc_launch(int fmt, int fp32_planes, const uint8_t *A, const float *row_scale, const void *B, int b_dtype, int layout,
                         int64_t ldb, const float *bias, void *C, int c_dtype, int64_t ldc, int64_t M, int64_t N,
                         int64_t K, float alpha, float beta, void *workspace, size_t workspace_bytes, cudaStream_t st,
                         int n_peers, void *const *peer_C) {
     const void *x_ptr = B;
     int64_t x_ld = ldb, x_rows = N;
-    const int planes = b_dtype == T81B200_F32 ? 2 : 1;
+    const int planes = b_dtype == T81B200_F32 ? fp32_planes : 1;
     if (!reads_in_place(B, b_dtype, layout, ldb)) {
-        const size_t need = scratch_size(b_dtype, N, K);
+        const size_t need = gemm_trit_tc_scratch_most(b_dtype, N, K, planes);
         if (!workspace || workspace_bytes < need || reinterpret_cast<uintptr_t>(workspace) % 16 != 0)
             return fail(T81B200_EWORKSPACE, "gemm_trit: %zu bytes of 16-byte aligned workspace needed, %zu given", need, workspace_bytes);
-        __nv_bfloat16 *scratch = static_cast<__nv_bfloat16 *>(workspace);
-        const int64_t kpad = scratch_row(K);
-        int rc = T81B200_EINVAL;
-        switch (b_dtype) {
-            case T81B200_F32: rc = launch_stage<float, 2>(B, layout, ldb, N, K, scratch, kpad, st); break;
-            case T81B200_BF16: case T81B200_F16: rc = launch_stage<__nv_bfloat16, 0>(B, layout, ldb, N, K, scratch, kpad, st); break;
-        }
-        if (rc) return rc;
-        x_ptr = scratch; x_ld = kpad; x_rows = (int64_t)planes * N;
+        if (int rc = stage_planes(B, b_dtype, layout, ldb, N, K, planes, workspace, st)) return rc;
+        x_ptr = workspace; x_ld = scratch_row(K); x_rows = (int64_t)planes * N;
     }
     const TcShape shape = pick_shape(M, N, K, planes);
     const bool f16 = b_dtype == T81B200_F16;
@@ -815,7 +795,7 @@ int gemm_trit_tc_launch(int fmt, const uint8_t *A, const float *row_scale, const
     p.planes = planes; p.plane_rows = (int)N;
     p.splits = shape.splits;
     p.a_stages = shape.a_stages; p.b_stages = shape.b_stages; p.b_step = shape.b_step;
-    p.one_tile = shape.splits > 1 || p.m_tiles * p.n_tiles <= resident_clusters(1) ? 1 : 0;
+    p.one_tile = shape.splits > 1 || p.m_tiles * p.n_tiles <= resident_pair_clusters(1) ? 1 : 0;
     p.idesc = umma_instr_desc(shape.bn, f16);
     p.one_mask = f16 ? 0xBC00BC00u : 0xFFFFFFFFu;
     p.alpha = fmt == 1 ? 0.5f * alpha : alpha;

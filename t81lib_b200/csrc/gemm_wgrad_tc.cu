@@ -1,0 +1,414 @@
+// Weight gradient of the ternary Linear's training step (t81/nn/linear.py:72-80 through t81/qat.py:28-57 of the
+// reference) on the tensor cores:
+//
+//   out[o][k] = slope(w[o][k]) * sum_t g[t][o] * x[t][k]        slope = 2 where |w / scale| < 0.5, else 0
+//
+// g (tokens, rows) and x (tokens, cols) are token-major, so both operands are contiguous along the output index and
+// strided along the contraction: they are loaded as they lie (boxes of 64 columns x 64 tokens, 128-byte swizzle) and
+// read by tcgen05.mma as M- / N-major operands; nothing is transposed in memory.  One pair of CTAs (cta_group::2) per
+// 256 x bn tile; each loads its own 128 columns of g and half of the tile's columns of x.
+//
+// 16-bit operands multiply as they are: products exact, accumulation fp32.  fp32 operands are staged as three bf16
+// planes (x = p0 + p1 + p2 exactly, 24 mantissa bits) and the six plane products of weight 2^-16 and above are
+// accumulated; the three left out lie below an fp32 ulp of the product.  The five small products have an accumulator of
+// their own, and long contractions of fp32 operands are cut into segments of about 1024 tokens that meet in `out`: the tensor cores
+// cut an accumulator off at every 16-token step instead of rounding it, which over 4096 tokens in one piece left the
+// result 4.4e-6 (root mean square) from the exact sums, against 1.1e-6 for fp32 arithmetic on CUDA cores.
+//
+// Bound by the operands' way from L2: a pair tile takes 32 KB per CTA and 64-token step, whatever the MMAs do.  Tiles
+// are walked in groups of eight row tiles so that what runs at a time shares its operands in L2.  The slope is applied in
+// the epilogue, on values that a trip through shared memory has turned into whole 128-byte rows, beside the weights.
+#include "common.cuh"
+#include "tma.cuh"
+#include "umma.cuh"
+
+#include <atomic>
+#include <cstring>
+
+namespace t81b200 {
+
+namespace {
+
+constexpr int BT = 64;                        // tokens per operand stage
+constexpr int BOX_BYTES = 64 * BT * 2;        // 64 columns x 64 tokens: 8 KB
+constexpr int A_BYTES = 2 * BOX_BYTES;        // this CTA's 128 columns of g
+constexpr int MAX_STAGES = 8;
+constexpr int NUM_THREADS = 6 * 32;
+constexpr int EPILOGUE_WARP0 = 2;
+constexpr int MAX_SPLITS = 4;
+constexpr int TURN_PITCH = 36;                // floats per row of the turning buffer: 16-byte aligned, conflict-free
+constexpr int TURN_BYTES = 4 * 32 * TURN_PITCH * 4;
+constexpr int BARRIER_BYTES = 256;
+constexpr int SMEM_LIMIT = 227 * 1024;
+
+enum { WGRAD_STATUS_PRODUCER = 11, WGRAD_STATUS_MMA = 12, WGRAD_STATUS_EPILOGUE = 13 };
+__device__ int g_wgrad_status = 0;
+
+struct WgradParams {
+    const float *w, *scale;
+    float *out;
+    int64_t rows, cols, ldw;
+    int m_tiles, n_tiles, bn;
+    int pairs, token_steps;           // plane products (1 or 6), 64-token steps
+    int segments;                     // parts of the contraction that are added up in `out` (one if split)
+    int splits, stages;
+    uint32_t idesc;
+    int vec;                          // 128-bit accesses to w and out
+};
+
+// Plane pair i of an fp32 product: planes of g and of x.
+__device__ __forceinline__ void plane_pair(int i, int &a, int &b) {
+    a = i == 2 || i == 3 ? 1 : (i == 5 ? 2 : 0);   // 0 0 1 1 0 2
+    b = i == 1 || i == 3 ? 1 : (i == 4 ? 2 : 0);   // 0 1 0 1 2 0
+}
+
+// M- / N-major SWIZZLE_128B operand: 64-column groups 8 KB apart, 8-token groups 1 KB apart.
+__device__ __forceinline__ uint64_t umma_desc_mn(uint32_t smem_addr) {
+    return (uint64_t)((smem_addr >> 4) & 0x3FFF) | ((uint64_t)(BOX_BYTES >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) |
+           ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
+}
+
+__device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const CUtensorMap *map, int x, int y, int z, uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+        ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(pair_leader(bar))
+        : "memory");
+}
+
+// Tile number -> row and column tile: groups of eight row tiles, row fastest inside a group.
+__device__ __forceinline__ void tile_at(const WgradParams &p, int tile, int &m, int &n) {
+    const int group = 8 * p.n_tiles, first = tile / group * 8;
+    const int height = p.m_tiles - first < 8 ? p.m_tiles - first : 8;
+    const int r = tile - first * p.n_tiles;
+    m = first + r % height;
+    n = r / height;
+}
+
+// 32 columns of this warp's 32 rows: turned through shared memory, multiplied with the slope, stored.
+__device__ __forceinline__ void emit_block(const WgradParams &p, const uint32_t (&v)[32], float *turn, int64_t row0, int64_t col0, int lane, float half_scale, bool add) {
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+        *reinterpret_cast<uint4 *>(turn + lane * TURN_PITCH + 4 * i) = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+    __syncwarp();
+    const int64_t col = col0 + (lane & 7) * 4;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int r = 4 * i + (lane >> 3);
+        const int64_t row = row0 + r;
+        if (row >= p.rows || col >= p.cols) continue;
+        const float4 s = *reinterpret_cast<const float4 *>(turn + r * TURN_PITCH + (lane & 7) * 4);
+        const float *w = p.w + row * p.ldw + col;
+        float *o = p.out + row * p.cols + col;
+        // |w / scale| < 0.5 exactly where |w| < scale / 2: two floats that differ do so by 2^-24 of their size or more,
+        // and a quotient 2^-24 below one half does not round up to it
+        if (p.vec) {
+            const float4 wv = __ldg(reinterpret_cast<const float4 *>(w));
+            float4 y = make_float4(fabsf(wv.x) < half_scale ? 2.0f * s.x : 0.0f * s.x, fabsf(wv.y) < half_scale ? 2.0f * s.y : 0.0f * s.y,
+                                                         fabsf(wv.z) < half_scale ? 2.0f * s.z : 0.0f * s.z, fabsf(wv.w) < half_scale ? 2.0f * s.w : 0.0f * s.w);
+            if (add) {
+                const float4 was = *reinterpret_cast<const float4 *>(o);
+                y.x += was.x; y.y += was.y; y.z += was.z; y.w += was.w;
+            }
+            *reinterpret_cast<float4 *>(o) = y;
+        } else {
+            const float e[4] = {s.x, s.y, s.z, s.w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (col + j < p.cols) o[j] = e[j] * (fabsf(w[j]) < half_scale ? 2.0f : 0.0f) + (add ? o[j] : 0.0f);
+        }
+    }
+}
+
+// 32 columns of the tile's sums: fp32 operands have the small products beside the large one.
+__device__ __forceinline__ void load_sums(const WgradParams &p, uint32_t taddr, uint32_t (&v)[32]) {
+    tmem_ld32(taddr, v);
+    if (p.pairs > 1) {
+        uint32_t small[32];
+        tmem_ld32(taddr + 256u, small);
+#pragma unroll
+        for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) + __uint_as_float(small[i]));
+    }
+}
+
+__global__ void __launch_bounds__(NUM_THREADS, 1)
+gemm_wgrad_tc_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ WgradParams p) {
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    uint8_t *gen_base = smem_raw + (base - smem_u32(smem_raw));
+    const uint32_t b_bytes = (uint32_t)p.bn / 2 / 64 * BOX_BYTES, stage_bytes = A_BYTES + b_bytes;
+    const uint32_t turn_off = (uint32_t)p.stages * stage_bytes, bars = base + turn_off + TURN_BYTES;
+    auto full = [&](int s) { return bars + 8u * s; };
+    auto empty = [&](int s) { return bars + 8u * (MAX_STAGES + s); };
+    auto acc_full = [&](int s) { return bars + 8u * (2 * MAX_STAGES + s); };
+    auto acc_empty = [&](int s) { return bars + 8u * (2 * MAX_STAGES + 2 + s); };
+    const uint32_t tmem_slot = bars + 8u * (2 * MAX_STAGES + 4);
+
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+    const uint32_t rank = cluster_rank();
+    const int half = (int)(rank & 1u), slice = (int)(rank >> 1);
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < MAX_STAGES; ++s) { mbar_init(full(s), 1); mbar_init(empty(s), 1); }
+        for (int s = 0; s < 2; ++s) { mbar_init(acc_full(s), 1); mbar_init(acc_empty(s), 8); }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncwarp();
+    if (warp == 1) tmem_alloc_pair(tmem_slot);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    cluster_barrier();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t *>(gen_base + (tmem_slot - base));
+
+    const int total_pieces = p.m_tiles * p.n_tiles * p.segments;
+    const int n_clusters = (int)gridDim.x / (2 * p.splits), cluster_id = (int)blockIdx.x / (2 * p.splits);
+    // a piece of work is one segment of one tile; this pair's share of a segment: token steps, each with all plane products
+    const int parts = p.splits * p.segments;
+    auto share_begin = [&](int piece) { return (int)((int64_t)p.token_steps * (piece % p.segments * p.splits + slice) / parts) * p.pairs; };
+    auto share_end = [&](int piece) { return (int)((int64_t)p.token_steps * (piece % p.segments * p.splits + slice + 1) / parts) * p.pairs; };
+    const int n_bufs = p.pairs == 1 ? 2 : 1;  // fp32: the second buffer holds the small products
+    auto next_piece = [&](int piece) { return (piece + 1) % p.segments ? piece + 1 : piece + 1 + (n_clusters - 1) * p.segments; };
+    const uint16_t pair_mask = (uint16_t)(3u << (rank & ~1u));
+    const float half_scale = 0.5f * *p.scale;
+
+    if (warp == 0) {
+        Ring ring;
+        bool ok = true;
+        for (int piece = cluster_id * p.segments; piece < total_pieces && ok; piece = next_piece(piece)) {
+            int m, n;
+            tile_at(p, piece / p.segments, m, n);
+            const int s0 = share_begin(piece), s1 = share_end(piece);
+            const int o0 = (2 * m + half) * 128, k0 = n * p.bn + half * (p.bn / 2);
+            for (int s = s0; s < s1; ++s) {
+                ok = mbar_wait(empty(ring.stage), ring.phase ^ 1);
+                if (!ok) break;
+                int pa, pb;
+                plane_pair(s % p.pairs, pa, pb);
+                const int t0 = s / p.pairs * BT;
+                if (elect_one()) {
+                    if (half == 0) mbar_arrive_expect_tx(full(ring.stage), 2 * stage_bytes);
+                    uint32_t dst = base + (uint32_t)ring.stage * stage_bytes;
+                    for (int b = 0; b < 2; ++b, dst += BOX_BYTES) tma_load_3d_pair(dst, &map_g, o0 + 64 * b, t0, pa, full(ring.stage));
+                    for (int b = 0; b < p.bn / 128; ++b, dst += BOX_BYTES) tma_load_3d_pair(dst, &map_x, k0 + 64 * b, t0, pb, full(ring.stage));
+                }
+                __syncwarp();
+                ring.advance(p.stages);
+            }
+        }
+        if (!ok && lane == 0) atomicCAS(&g_wgrad_status, 0, WGRAD_STATUS_PRODUCER);
+    } else if (warp == 1) {
+        if (half == 0) {
+            Ring ring;
+            bool ok = true;
+            int it = 0;
+            for (int piece = cluster_id * p.segments; piece < total_pieces && ok; piece = next_piece(piece), ++it) {
+                const int s0 = share_begin(piece), s1 = share_end(piece);
+                const int buf = it % n_bufs;
+                ok = mbar_wait(acc_empty(buf), ((uint32_t)(it / n_bufs) & 1u) ^ 1u);
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t d_tmem = tmem_base + (uint32_t)buf * 256u;
+                for (int s = s0; s < s1; ++s) {
+                    ok = mbar_wait(full(ring.stage), ring.phase);
+                    if (!ok) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint64_t ad = umma_desc_mn(base + (uint32_t)ring.stage * stage_bytes);
+                    const uint64_t bd = umma_desc_mn(base + (uint32_t)ring.stage * stage_bytes + A_BYTES);
+                    const int pair = s % p.pairs;
+                    const uint32_t d = d_tmem + (pair == 0 ? 0u : 256u), more = s - s0 >= (pair == 0 ? 1 : 2) ? 1u : 0u;
+                    if (elect_one()) {
+#pragma unroll
+                        for (int k = 0; k < BT / 16; ++k)  // 16 tokens: two 1 KB groups
+                            umma_pair(d, ad + (uint64_t)(128 * k), bd + (uint64_t)(128 * k), p.idesc, k == 0 ? more : 1u);
+                        umma_commit_pair(empty(ring.stage), pair_mask);
+                    }
+                    __syncwarp();
+                    ring.advance(p.stages);
+                }
+                if (ok && elect_one()) umma_commit_pair(acc_full(buf), pair_mask);
+                __syncwarp();
+            }
+            if (!ok && lane == 0) atomicCAS(&g_wgrad_status, 0, WGRAD_STATUS_MMA);
+        }
+    } else {
+        const int quarter = warp & 3;
+        float *turn = reinterpret_cast<float *>(gen_base + turn_off) + quarter * 32 * TURN_PITCH;
+        bool ok = true;
+        int it = 0;
+        for (int piece = cluster_id * p.segments; piece < total_pieces && ok; piece = next_piece(piece), ++it) {
+            const int buf = it % n_bufs;
+            ok = __all_sync(0xffffffffu, mbar_wait(acc_full(buf), (uint32_t)(it / n_bufs) & 1u));
+            if (!ok || p.splits > 1) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            int m, n;
+            tile_at(p, piece / p.segments, m, n);
+            for (int c = 0; c < p.bn / 32; ++c) {
+                uint32_t v[32];
+                load_sums(p, tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * 256 + c * 32), v);
+                emit_block(p, v, turn, (int64_t)(2 * m + half) * 128 + quarter * 32, (int64_t)n * p.bn + c * 32, lane, half_scale, piece % p.segments != 0);
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive_leader(acc_empty(buf));
+        }
+        if (!ok && lane == 0) atomicCAS(&g_wgrad_status, 0, WGRAD_STATUS_EPILOGUE);
+    }
+    __syncwarp();
+
+    if (p.splits > 1) {
+        // one tile per cluster, its tokens shared by the pairs: 32-column block b is finished by slice b % splits, the others
+        // push their partial sums into its operand ring (idle once every CTA has its last MMA behind it)
+        const int quarter = warp & 3, S = p.splits, blocks = p.bn / 32;
+        const bool epi = warp >= EPILOGUE_WARP0;
+        const uint32_t t_lane = tmem_base + ((uint32_t)(quarter * 32) << 16), lane_row = (uint32_t)(quarter * 32 + lane);
+        __syncthreads();
+        cluster_barrier();
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (epi)
+            for (int b = 0; b < blocks; ++b)
+                if (b % S != slice) {
+                    uint32_t v[32];
+                    load_sums(p, t_lane + (uint32_t)(b * 32), v);
+                    push_partial(v, base + partial_slot(b, S, slice, b % S) * 16384u + lane_row * 4u, (uint32_t)(2 * (b % S) + half));
+                }
+        __syncthreads();
+        cluster_barrier();
+        if (epi) {
+            int m, n;
+            tile_at(p, cluster_id, m, n);
+            float *turn = reinterpret_cast<float *>(gen_base + turn_off) + quarter * 32 * TURN_PITCH;
+            for (int b = slice; b < blocks; b += S) {
+                uint32_t v[32];
+                load_sums(p, t_lane + (uint32_t)(b * 32), v);
+                fold_partials(v, gen_base, b, S, slice, lane_row);
+                emit_block(p, v, turn, (int64_t)(2 * m + half) * 128 + quarter * 32, (int64_t)n * p.bn + b * 32, lane, half_scale, false);
+            }
+        }
+    }
+
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    cluster_barrier();
+    if (warp == 1) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        tmem_free_pair(tmem_base);
+    }
+}
+
+int make_map_3d(CUtensorMap *map, CUtensorMapDataType dt, const void *ptr, uint64_t inner, uint64_t tokens, uint64_t planes, uint64_t ld_bytes) {
+    const cuuint64_t dims[3] = {inner, tokens, planes}, strides[2] = {ld_bytes, ld_bytes * tokens};
+    const cuuint32_t box[3] = {64, BT, 1};
+    return make_map(map, dt, 3, ptr, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+
+bool in_place(const void *p, int dtype, int64_t ld) { return dtype != T81B200_F32 && reinterpret_cast<uintptr_t>(p) % 16 == 0 && (ld * 2) % 16 == 0; }
+size_t operand_scratch(const void *p, int dtype, int64_t ld, int64_t tokens, int64_t width) {
+    if (in_place(p, dtype, ld)) return 0;
+    return ((size_t)(dtype == T81B200_F32 ? 3 : 1) * tokens * ((width + 7) & ~(int64_t)7) * 2 + 255) / 256 * 256;
+}
+
+}  // namespace
+
+int gemm_wgrad_status(int reset) {
+    int v = 0;
+    if (cudaMemcpyFromSymbol(&v, g_wgrad_status, sizeof v) != cudaSuccess) return T81B200_ECUDA;
+    if (reset && v != 0) {
+        const int zero = 0;
+        if (cudaMemcpyToSymbol(g_wgrad_status, &zero, sizeof zero) != cudaSuccess) return T81B200_ECUDA;
+    }
+    return v;
+}
+
+}  // namespace t81b200
+
+using namespace t81b200;
+
+extern "C" size_t t81b200_qat_weight_grad_workspace_bytes(const void *g, int64_t ldg, const void *x, int64_t ldx, int dtype, int64_t tokens,
+                                                          int64_t rows, int64_t cols) {
+    if (tokens <= 0 || rows <= 0 || cols <= 0) return 0;
+    return operand_scratch(g, dtype, ldg, tokens, rows) + operand_scratch(x, dtype, ldx, tokens, cols);
+}
+
+extern "C" int t81b200_qat_weight_grad(const void *g, int64_t ldg, const void *x, int64_t ldx, int dtype, int64_t tokens, int64_t rows, int64_t cols,
+                                       const float *w, int64_t ldw, const float *scale, float *out, void *workspace, size_t workspace_bytes, void *stream) {
+    if (tokens < 0 || rows < 0 || cols < 0 || ldg < rows || ldx < cols || ldw < cols) return fail(T81B200_EINVAL, "qat_weight_grad: bad dimensions");
+    if (dtype != T81B200_F32 && dtype != T81B200_BF16 && dtype != T81B200_F16) return fail(T81B200_EINVAL, "qat_weight_grad: unknown dtype %d", dtype);
+    if (int rc = check_device()) return rc;
+    if (rows == 0 || cols == 0) return T81B200_OK;
+    if (!w || !scale || !out || (tokens > 0 && (!g || !x))) return fail(T81B200_EINVAL, "qat_weight_grad: null pointer");
+    if (rows >= (1ll << 30) || cols >= (1ll << 30) || tokens >= (1ll << 27)) return fail(T81B200_ELIMIT, "qat_weight_grad: dimensions too large");
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (tokens == 0) {
+        T81_CUDA_TRY(cudaMemsetAsync(out, 0, (size_t)rows * cols * 4, st));
+        return T81B200_OK;
+    }
+    const size_t need_g = operand_scratch(g, dtype, ldg, tokens, rows), need_x = operand_scratch(x, dtype, ldx, tokens, cols);
+    if (need_g + need_x > 0 && (!workspace || workspace_bytes < need_g + need_x || reinterpret_cast<uintptr_t>(workspace) % 256 != 0))
+        return fail(T81B200_EWORKSPACE, "qat_weight_grad: %zu bytes of 256-byte aligned workspace needed, %zu given", need_g + need_x, workspace_bytes);
+    const int planes = dtype == T81B200_F32 ? 3 : 1;
+    const CUtensorMapDataType dt = dtype == T81B200_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+    CUtensorMap mg, mx;
+    struct { const void *src; int64_t ld, width; size_t need; char *scratch; CUtensorMap *map; } ops[2] = {
+        {g, ldg, rows, need_g, static_cast<char *>(workspace), &mg}, {x, ldx, cols, need_x, static_cast<char *>(workspace) + need_g, &mx}};
+    for (auto &o : ops) {
+        const void *src = o.src;
+        int64_t ld = o.ld;
+        if (o.need) {
+            ld = (o.width + 7) & ~(int64_t)7;
+            if (int rc = stage_planes(o.src, dtype, T81B200_LAYOUT_NK, o.ld, tokens, o.width, planes, o.scratch, st)) return rc;
+            src = o.scratch;
+        }
+        if (int rc = make_map_3d(o.map, dt, src, (uint64_t)o.width, (uint64_t)tokens, (uint64_t)planes, (uint64_t)ld * 2)) return rc;
+    }
+
+    static std::atomic<bool> configured[64];
+    int dev = 0;
+    T81_CUDA_TRY(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64 || !configured[dev].load(std::memory_order_acquire)) {
+        T81_CUDA_TRY(cudaFuncSetAttribute(gemm_wgrad_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT));
+        if (dev >= 0 && dev < 64) configured[dev].store(true, std::memory_order_release);
+    }
+    WgradParams p;
+    memset(&p, 0, sizeof p);
+    p.w = w; p.scale = scale; p.out = out; p.rows = rows; p.cols = cols; p.ldw = ldw;
+    p.token_steps = (int)((tokens + BT - 1) / BT);
+    p.pairs = planes == 3 ? 6 : 1;
+    p.m_tiles = (int)((rows + 255) / 256);
+    // 256- or 128-column tiles, tokens split over up to four pairs of a cluster while that fits the GPU at once: whichever
+    // needs fewer steps one after the other (a 128-column step costs about 0.65 of a 256-column one)
+    double best = 1e30;
+    for (int bn = 256; bn >= 128; bn -= 128)
+        for (int s = 1; s <= MAX_SPLITS; ++s) {
+            const int64_t tiles = (int64_t)p.m_tiles * ((cols + bn - 1) / bn), resident = resident_pair_clusters(s);
+            if (s > p.token_steps || (s > 1 && tiles > resident)) continue;
+            const double t = (double)((tiles + resident - 1) / resident) * ((p.token_steps + s - 1) / s) * p.pairs * (bn == 256 ? 1.0 : 0.65) + (s > 1 ? 6.0 : 0.0);
+            if (t < best) { best = t; p.bn = bn; p.splits = s; }
+        }
+    p.segments = p.pairs > 1 && p.splits == 1 ? (p.token_steps + 15) / 16 : 1;
+    p.n_tiles = (int)((cols + p.bn - 1) / p.bn);
+    const int stage = A_BYTES + p.bn / 2 / 64 * BOX_BYTES;
+    const int fit = (SMEM_LIMIT - 1024 - TURN_BYTES - BARRIER_BYTES) / stage;
+    p.stages = fit < MAX_STAGES ? fit : MAX_STAGES;
+    p.idesc = umma_instr_desc(p.bn, dtype == T81B200_F16, true, true);
+    p.vec = cols % 4 == 0 && ldw % 4 == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0 && reinterpret_cast<uintptr_t>(out) % 16 == 0 ? 1 : 0;
+    const int64_t tiles = (int64_t)p.m_tiles * p.n_tiles;
+    const int64_t clusters = p.splits > 1 || tiles < resident_pair_clusters(1) ? tiles : resident_pair_clusters(1);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(clusters * 2 * p.splits), 1, 1);
+    cfg.blockDim = dim3(NUM_THREADS, 1, 1);
+    cfg.dynamicSmemBytes = (size_t)p.stages * stage + TURN_BYTES + BARRIER_BYTES + 1024;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)(2 * p.splits);
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    T81_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_wgrad_tc_kernel, mg, mx, p));
+    return T81B200_OK;
+}

@@ -80,19 +80,28 @@ inline EncodeTiledFn encode_tiled() {
     return fn;
 }
 
-inline int make_map_2d(CUtensorMap *map, CUtensorMapDataType dt, size_t elem, const void *ptr, uint64_t inner, uint64_t outer,
-                uint64_t row_stride_bytes, uint32_t box_inner, uint32_t box_outer, CUtensorMapSwizzle swz) {
+// Tensor map of `rank` dimensions; dims, strides (bytes, of dimensions 1 ..) and box as the driver wants them.
+inline int make_map(CUtensorMap *map, CUtensorMapDataType dt, int rank, const void *ptr, const cuuint64_t *dims, const cuuint64_t *strides,
+                    const cuuint32_t *box, CUtensorMapSwizzle swz) {
     EncodeTiledFn fn = encode_tiled();
     if (!fn) return fail(T81B200_ECUDA, "cuTensorMapEncodeTiled is not available from the driver");
-    cuuint64_t dims[2] = {inner, outer};
-    cuuint64_t strides[1] = {row_stride_bytes};
-    cuuint32_t box[2] = {box_inner, box_outer};
-    cuuint32_t estr[2] = {1, 1};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    for (int attempt = 0;; ++attempt) {
+        const CUresult rc = fn(map, dt, (cuuint32_t)rank, const_cast<void *>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swz,
+                               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (rc == CUDA_SUCCESS) return T81B200_OK;
+        // a thread that has made no runtime call with an effect yet (an autograd worker) has no current context: bind it
+        if (rc != CUDA_ERROR_INVALID_CONTEXT || attempt > 0) return fail(T81B200_ECUDA, "cuTensorMapEncodeTiled failed with code %d", (int)rc);
+        T81_CUDA_TRY(cudaFree(nullptr));
+    }
+}
+
+inline int make_map_2d(CUtensorMap *map, CUtensorMapDataType dt, size_t elem, const void *ptr, uint64_t inner, uint64_t outer,
+                uint64_t row_stride_bytes, uint32_t box_inner, uint32_t box_outer, CUtensorMapSwizzle swz) {
     (void)elem;
-    CUresult rc = fn(map, dt, 2, const_cast<void *>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swz,
-                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (rc != CUDA_SUCCESS) return fail(T81B200_ECUDA, "cuTensorMapEncodeTiled failed with code %d", (int)rc);
-    return T81B200_OK;
+    const cuuint64_t dims[2] = {inner, outer}, strides[1] = {row_stride_bytes};
+    const cuuint32_t box[2] = {box_inner, box_outer};
+    return make_map(map, dt, 2, ptr, dims, strides, box, swz);
 }
 
 }  // namespace t81b200

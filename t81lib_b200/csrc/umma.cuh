@@ -108,4 +108,38 @@ __device__ __forceinline__ void cluster_barrier() {
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
+// ---- a tile whose contraction is split over S pairs of a cluster ----
+// 32-column block b of the accumulator is finished by slice b % S; each other slice owns one 16 KB slot per block
+// ([column][128 rows] fp32) in that CTA's shared memory.
+__device__ __forceinline__ uint32_t partial_slot(int b, int S, int from, int to) { return (uint32_t)((b / S) * (S - 1) + (from < to ? from : from - 1)); }
+
+// v[i] (column i of the block) of this thread's row -> the slot at `dst` in the CTA of that cluster rank.
+__device__ __forceinline__ void push_partial(const uint32_t (&v)[32], uint32_t dst, uint32_t to_rank) {
+    asm("mapa.shared::cluster.u32 %0, %0, %1;" : "+r"(dst) : "r"(to_rank));
+#pragma unroll
+    for (int i = 0; i < 32; ++i) asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(dst + (uint32_t)i * 512u), "r"(v[i]) : "memory");
+}
+
+// v (this slice's own sums of block b) += the other slices' slots, in slice order whoever finishes the block.
+__device__ __forceinline__ void fold_partials(uint32_t (&v)[32], const uint8_t *slots, int b, int S, int slice, uint32_t lane_row) {
+    float sum[32];
+#pragma unroll
+    for (int i = 0; i < 32; ++i) sum[i] = 0.0f;
+    for (int s = 0; s < S; ++s) {
+        const float *src = reinterpret_cast<const float *>(slots + (size_t)partial_slot(b, S, s, slice) * 16384) + lane_row;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) sum[i] += s == slice ? __uint_as_float(v[i]) : src[i * 128];
+    }
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(sum[i]);
+}
+
+// ---- host ----
+// Clusters of `splits` CTA pairs (one CTA per SM) that the device runs at a time: clusters do not straddle GPCs, so
+// fewer fit than the SM count suggests (74, 33, 22 and 15 for 1 to 4 splits on a B200).
+int resident_pair_clusters(int splits);
+// Token-major planes of a (tokens, K) or (K, tokens) operand in scratch memory, rows of K rounded up to 8 elements:
+// 16-bit types are copied bit for bit (planes == 1), fp32 becomes two or three bf16 planes.
+int stage_planes(const void *B, int dtype, int layout, int64_t ld, int64_t tokens, int64_t K, int planes, void *scratch, cudaStream_t st);
+
 }  // namespace t81b200

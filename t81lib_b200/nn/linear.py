@@ -61,8 +61,9 @@ def ternary(x: torch.Tensor, threshold: float = 0.45, stochastic: bool = False) 
 
 
 class _FusedQATLinear(torch.autograd.Function):
-    """Training forward on the device kernels: the weight is quantised with the running scale and packed in one
-    pass (``ops.qat_quantize_pack``), the product runs on the packed-trit matmul with the scale as row scale.
+    """Training step on the device kernels: one pass over the weight quantises it with the running scale into the
+    decode-stream layout of the weight and of its transpose; the products of the forward and of the input gradient run
+    on them with the scale as row scale, the weight gradient on the transposed operands.
     Backward is the reference's (t81/nn/linear.py:72-80 through t81/qat.py:28-57): the input gradient is
     grad @ (trits * scale); the weight gradient is grad^T @ x times the surrogate's slope, 2 where
     |weight / scale| < 0.5 and 0 elsewhere (the scale itself carries no gradient)."""
@@ -70,15 +71,20 @@ class _FusedQATLinear(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight, bias, scale, threshold):
         from .. import ops
-        packed, row_scale = ops.qat_quantize_pack(weight.detach(), threshold, scale)
         rows, cols = weight.shape
-        x2 = x.reshape(-1, cols)
+        w = weight.detach()
+        t2, t2_t, scales = ops.qat_quantize_t2(w if w.stride(1) == 1 else w.contiguous(), threshold, scale, ctx.needs_input_grad[0])
+        x2 = x.detach().reshape(-1, cols)
         if x2.dtype not in (torch.float32, torch.bfloat16, torch.float16):
             x2 = x2.float()
-        y = ops.gemm_trit(packed, x2.detach(), M=rows, K=cols, layout="nk", row_scale=row_scale,
-                          bias=None if bias is None else bias.detach())
+        if x2.stride(1) != 1:
+            x2 = x2.contiguous()
+        b = bias
+        if b is not None:
+            b = b.detach().to(device=x2.device, dtype=torch.float32).contiguous()
+        y = ops.linear_t2(t2, rows, x2, cols, scales, b)
         ctx.save_for_backward(x2, weight, scale)
-        ctx.packed, ctx.has_bias, ctx.x_shape = packed, bias is not None, x.shape
+        ctx.t2_t, ctx.scales, ctx.has_bias, ctx.x_shape = t2_t, scales, bias is not None, x.shape
         return y.reshape(*x.shape[:-1], rows)
 
     @staticmethod
@@ -87,13 +93,15 @@ class _FusedQATLinear(torch.autograd.Function):
         x2, weight, scale = ctx.saved_tensors
         rows, cols = weight.shape
         g = grad_output.reshape(-1, rows)
+        if g.stride(1) != 1 or (g.shape[0] > 1 and g.stride(0) < rows):
+            g = g.contiguous()
         grad_x = grad_w = grad_b = None
         if ctx.needs_input_grad[0]:
-            w_eff = ops.unpack(ctx.packed, rows, cols).to(g.dtype) * scale.to(g.dtype)
-            grad_x = (g @ w_eff).reshape(ctx.x_shape).to(x2.dtype)
+            # every mantissa bit of a float32 gradient counts here: three planes
+            grad_x = ops.linear_t2(ctx.t2_t, cols, g, rows, ctx.scales, fp32_planes=3).reshape(ctx.x_shape)
         if ctx.needs_input_grad[1]:
-            slope = ((weight.detach() / scale).abs() < 0.5).to(weight.dtype) * 2.0
-            grad_w = (g.t().to(weight.dtype) @ x2.to(weight.dtype)) * slope
+            w = weight.detach()
+            grad_w = ops.qat_weight_grad(g, x2, w if w.stride(1) == 1 else w.contiguous(), scale)
         if ctx.has_bias and ctx.needs_input_grad[2]:
             grad_b = g.sum(dim=0)
         return grad_x, grad_w, grad_b, None, None
