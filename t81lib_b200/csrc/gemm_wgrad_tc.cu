@@ -33,11 +33,12 @@ constexpr int BT = 64;                        // tokens per operand stage
 constexpr int BOX_BYTES = 64 * BT * 2;        // 64 columns x 64 tokens: 8 KB
 constexpr int A_BYTES = 2 * BOX_BYTES;        // this CTA's 128 columns of g
 constexpr int MAX_STAGES = 8;
-constexpr int NUM_THREADS = 6 * 32;
+constexpr int EPILOGUE_WARPS = 8;             // two per quarter of the rows: each takes every other 32-column block
+constexpr int NUM_THREADS = (2 + EPILOGUE_WARPS) * 32;
 constexpr int EPILOGUE_WARP0 = 2;
 constexpr int MAX_SPLITS = 4;
 constexpr int TURN_PITCH = 36;                // floats per row of the turning buffer: 16-byte aligned, conflict-free
-constexpr int TURN_BYTES = 4 * 32 * TURN_PITCH * 4;
+constexpr int TURN_BYTES = EPILOGUE_WARPS * 32 * TURN_PITCH * 4;
 constexpr int BARRIER_BYTES = 256;
 constexpr int SMEM_LIMIT = 227 * 1024;
 
@@ -84,38 +85,59 @@ __device__ __forceinline__ void tile_at(const WgradParams &p, int tile, int &m, 
     n = r / height;
 }
 
-// 32 columns of this warp's 32 rows: turned through shared memory, multiplied with the slope, stored.
-__device__ __forceinline__ void emit_block(const WgradParams &p, const uint32_t (&v)[32], float *turn, int64_t row0, int64_t col0, int lane, float half_scale, bool add) {
+// A block is 32 columns of this warp's 32 rows.  VEC: a lane moves four columns of rows 4 i + lane / 8 (whole 128-byte
+// row pieces, 16 bytes a lane); otherwise one column of all 32 rows.
+template <bool VEC>
+__device__ __forceinline__ void load_weights(const WgradParams &p, int64_t row0, int64_t col0, int lane, float (&w)[32]) {
+    if constexpr (VEC) {
+        const int64_t col = col0 + (lane & 7) * 4;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int64_t row = row0 + 4 * i + (lane >> 3);
+            const float4 q = row < p.rows && col < p.cols ? __ldg(reinterpret_cast<const float4 *>(p.w + row * p.ldw + col)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            w[4 * i] = q.x; w[4 * i + 1] = q.y; w[4 * i + 2] = q.z; w[4 * i + 3] = q.w;
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) w[i] = row0 + i < p.rows && col0 + lane < p.cols ? __ldg(p.w + (row0 + i) * p.ldw + col0 + lane) : 0.0f;
+    }
+}
+
+// The block's sums, turned through shared memory, multiplied with the slope and stored (or added to what is there).
+template <bool VEC>
+__device__ __forceinline__ void emit_block(const WgradParams &p, const uint32_t (&v)[32], const float (&w)[32], float *turn, int64_t row0, int64_t col0,
+                                           int lane, float half_scale, bool add) {
     __syncwarp();
 #pragma unroll
     for (int i = 0; i < 8; ++i)
         *reinterpret_cast<uint4 *>(turn + lane * TURN_PITCH + 4 * i) = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
     __syncwarp();
-    const int64_t col = col0 + (lane & 7) * 4;
+    // |w / scale| < 0.5 exactly where |w| < scale / 2: two floats that differ do so by 2^-24 of their size or more,
+    // and a quotient 2^-24 below one half does not round up to it
+    auto sloped = [&](float sum, float weight) { return sum * (fabsf(weight) < half_scale ? 2.0f : 0.0f); };
+    if constexpr (VEC) {
+        const int64_t col = col0 + (lane & 7) * 4;
+        if (col >= p.cols) return;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int r = 4 * i + (lane >> 3);
-        const int64_t row = row0 + r;
-        if (row >= p.rows || col >= p.cols) continue;
-        const float4 s = *reinterpret_cast<const float4 *>(turn + r * TURN_PITCH + (lane & 7) * 4);
-        const float *w = p.w + row * p.ldw + col;
-        float *o = p.out + row * p.cols + col;
-        // |w / scale| < 0.5 exactly where |w| < scale / 2: two floats that differ do so by 2^-24 of their size or more,
-        // and a quotient 2^-24 below one half does not round up to it
-        if (p.vec) {
-            const float4 wv = __ldg(reinterpret_cast<const float4 *>(w));
-            float4 y = make_float4(fabsf(wv.x) < half_scale ? 2.0f * s.x : 0.0f * s.x, fabsf(wv.y) < half_scale ? 2.0f * s.y : 0.0f * s.y,
-                                                         fabsf(wv.z) < half_scale ? 2.0f * s.z : 0.0f * s.z, fabsf(wv.w) < half_scale ? 2.0f * s.w : 0.0f * s.w);
+        for (int i = 0; i < 8; ++i) {
+            const int r = 4 * i + (lane >> 3);
+            if (row0 + r >= p.rows) continue;
+            const float4 s = *reinterpret_cast<const float4 *>(turn + r * TURN_PITCH + (lane & 7) * 4);
+            float4 *o = reinterpret_cast<float4 *>(p.out + (row0 + r) * p.cols + col);
+            float4 y = make_float4(sloped(s.x, w[4 * i]), sloped(s.y, w[4 * i + 1]), sloped(s.z, w[4 * i + 2]), sloped(s.w, w[4 * i + 3]));
             if (add) {
-                const float4 was = *reinterpret_cast<const float4 *>(o);
+                const float4 was = *o;
                 y.x += was.x; y.y += was.y; y.z += was.z; y.w += was.w;
             }
-            *reinterpret_cast<float4 *>(o) = y;
-        } else {
-            const float e[4] = {s.x, s.y, s.z, s.w};
+            *o = y;
+        }
+    } else {
+        if (col0 + lane >= p.cols) return;
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
-                if (col + j < p.cols) o[j] = e[j] * (fabsf(w[j]) < half_scale ? 2.0f : 0.0f) + (add ? o[j] : 0.0f);
+        for (int i = 0; i < 32; ++i) {
+            if (row0 + i >= p.rows) break;
+            float *o = p.out + (row0 + i) * p.cols + col0 + lane;
+            *o = sloped(turn[i * TURN_PITCH + lane], w[i]) + (add ? *o : 0.0f);
         }
     }
 }
@@ -131,6 +153,7 @@ __device__ __forceinline__ void load_sums(const WgradParams &p, uint32_t taddr, 
     }
 }
 
+template <bool VEC>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_wgrad_tc_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ WgradParams p) {
     extern __shared__ uint8_t smem_raw[];
@@ -150,7 +173,7 @@ gemm_wgrad_tc_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_con
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < MAX_STAGES; ++s) { mbar_init(full(s), 1); mbar_init(empty(s), 1); }
-        for (int s = 0; s < 2; ++s) { mbar_init(acc_full(s), 1); mbar_init(acc_empty(s), 8); }
+        for (int s = 0; s < 2; ++s) { mbar_init(acc_full(s), 1); mbar_init(acc_empty(s), 2 * EPILOGUE_WARPS); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncwarp();
@@ -234,21 +257,28 @@ gemm_wgrad_tc_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_con
             if (!ok && lane == 0) atomicCAS(&g_wgrad_status, 0, WGRAD_STATUS_MMA);
         }
     } else {
-        const int quarter = warp & 3;
-        float *turn = reinterpret_cast<float *>(gen_base + turn_off) + quarter * 32 * TURN_PITCH;
+        const int quarter = warp & 3, first = (warp - EPILOGUE_WARP0) >> 2;
+        float *turn = reinterpret_cast<float *>(gen_base + turn_off) + (warp - EPILOGUE_WARP0) * 32 * TURN_PITCH;
         bool ok = true;
         int it = 0;
         for (int piece = cluster_id * p.segments; piece < total_pieces && ok; piece = next_piece(piece), ++it) {
             const int buf = it % n_bufs;
+            int m, n;
+            tile_at(p, piece / p.segments, m, n);
+            const int64_t row0 = (int64_t)(2 * m + half) * 128 + quarter * 32, col0 = (int64_t)n * p.bn;
+            float w[32];  // the weights of a block are fetched while the one before it is put out: their latency bounded this loop
+            load_weights<VEC>(p, row0, col0 + first * 32, lane, w);
             ok = __all_sync(0xffffffffu, mbar_wait(acc_full(buf), (uint32_t)(it / n_bufs) & 1u));
             if (!ok || p.splits > 1) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            int m, n;
-            tile_at(p, piece / p.segments, m, n);
-            for (int c = 0; c < p.bn / 32; ++c) {
+            for (int c = first; c < p.bn / 32; c += 2) {
+                float next[32];
+                load_weights<VEC>(p, row0, col0 + (c + 2 < p.bn / 32 ? c + 2 : c) * 32, lane, next);
                 uint32_t v[32];
                 load_sums(p, tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * 256 + c * 32), v);
-                emit_block(p, v, turn, (int64_t)(2 * m + half) * 128 + quarter * 32, (int64_t)n * p.bn + c * 32, lane, half_scale, piece % p.segments != 0);
+                emit_block<VEC>(p, v, w, turn, row0, col0 + c * 32, lane, half_scale, piece % p.segments != 0);
+#pragma unroll
+                for (int i = 0; i < 32; ++i) w[i] = next[i];
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
@@ -261,14 +291,14 @@ gemm_wgrad_tc_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_con
     if (p.splits > 1) {
         // one tile per cluster, its tokens shared by the pairs: 32-column block b is finished by slice b % splits, the others
         // push their partial sums into its operand ring (idle once every CTA has its last MMA behind it)
-        const int quarter = warp & 3, S = p.splits, blocks = p.bn / 32;
+        const int quarter = warp & 3, first = (warp - EPILOGUE_WARP0) >> 2, S = p.splits, blocks = p.bn / 32;
         const bool epi = warp >= EPILOGUE_WARP0;
         const uint32_t t_lane = tmem_base + ((uint32_t)(quarter * 32) << 16), lane_row = (uint32_t)(quarter * 32 + lane);
         __syncthreads();
         cluster_barrier();
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         if (epi)
-            for (int b = 0; b < blocks; ++b)
+            for (int b = first; b < blocks; b += 2)
                 if (b % S != slice) {
                     uint32_t v[32];
                     load_sums(p, t_lane + (uint32_t)(b * 32), v);
@@ -279,12 +309,16 @@ gemm_wgrad_tc_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_con
         if (epi) {
             int m, n;
             tile_at(p, cluster_id, m, n);
-            float *turn = reinterpret_cast<float *>(gen_base + turn_off) + quarter * 32 * TURN_PITCH;
-            for (int b = slice; b < blocks; b += S) {
+            float *turn = reinterpret_cast<float *>(gen_base + turn_off) + (warp - EPILOGUE_WARP0) * 32 * TURN_PITCH;
+            const int64_t row0 = (int64_t)(2 * m + half) * 128 + quarter * 32;
+            for (int b = slice + S * first; b < blocks; b += 2 * S) {
+                const int64_t col = (int64_t)n * p.bn + b * 32;
+                float w[32];
+                load_weights<VEC>(p, row0, col, lane, w);
                 uint32_t v[32];
                 load_sums(p, t_lane + (uint32_t)(b * 32), v);
                 fold_partials(v, gen_base, b, S, slice, lane_row);
-                emit_block(p, v, turn, (int64_t)(2 * m + half) * 128 + quarter * 32, (int64_t)n * p.bn + b * 32, lane, half_scale, false);
+                emit_block<VEC>(p, v, w, turn, row0, col, lane, half_scale, false);
             }
         }
     }
@@ -302,6 +336,20 @@ int make_map_3d(CUtensorMap *map, CUtensorMapDataType dt, const void *ptr, uint6
     const cuuint64_t dims[3] = {inner, tokens, planes}, strides[2] = {ld_bytes, ld_bytes * tokens};
     const cuuint32_t box[3] = {64, BT, 1};
     return make_map(map, dt, 3, ptr, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+
+template <bool VEC>
+int launch_wgrad(const cudaLaunchConfig_t &cfg, const CUtensorMap &mg, const CUtensorMap &mx, const WgradParams &p) {
+    // the shared-memory limit is a per-device attribute of the function: set it once on every device
+    static std::atomic<bool> configured[64];
+    int dev = 0;
+    T81_CUDA_TRY(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64 || !configured[dev].load(std::memory_order_acquire)) {
+        T81_CUDA_TRY(cudaFuncSetAttribute(gemm_wgrad_tc_kernel<VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT));
+        if (dev >= 0 && dev < 64) configured[dev].store(true, std::memory_order_release);
+    }
+    T81_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_wgrad_tc_kernel<VEC>, mg, mx, p));
+    return T81B200_OK;
 }
 
 bool in_place(const void *p, int dtype, int64_t ld) { return dtype != T81B200_F32 && reinterpret_cast<uintptr_t>(p) % 16 == 0 && (ld * 2) % 16 == 0; }
@@ -364,13 +412,6 @@ extern "C" int t81b200_qat_weight_grad(const void *g, int64_t ldg, const void *x
         if (int rc = make_map_3d(o.map, dt, src, (uint64_t)o.width, (uint64_t)tokens, (uint64_t)planes, (uint64_t)ld * 2)) return rc;
     }
 
-    static std::atomic<bool> configured[64];
-    int dev = 0;
-    T81_CUDA_TRY(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 64 || !configured[dev].load(std::memory_order_acquire)) {
-        T81_CUDA_TRY(cudaFuncSetAttribute(gemm_wgrad_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT));
-        if (dev >= 0 && dev < 64) configured[dev].store(true, std::memory_order_release);
-    }
     WgradParams p;
     memset(&p, 0, sizeof p);
     p.w = w; p.scale = scale; p.out = out; p.rows = rows; p.cols = cols; p.ldw = ldw;
@@ -409,6 +450,5 @@ extern "C" int t81b200_qat_weight_grad(const void *g, int64_t ldg, const void *x
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    T81_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_wgrad_tc_kernel, mg, mx, p));
-    return T81B200_OK;
+    return p.vec ? launch_wgrad<true>(cfg, mg, mx, p) : launch_wgrad<false>(cfg, mg, mx, p);
 }
