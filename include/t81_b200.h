@@ -367,7 +367,9 @@ T81B200_API int t81b200_qat_quantize_pack(const void *w, int w_dtype, int64_t ro
  * copies of the scale (the row scales of either product).  qat_weight_grad: out (rows, cols) fp32, contiguous, =
  * slope * g^T x for token-major g (tokens, rows) and x (tokens, cols) of one dtype, slope = 2 where |w / scale| < 0.5 and
  * 0 elsewhere (t81/nn/linear.py:72-80 through t81/qat.py:28-57); 16-bit operands are multiplied exactly, fp32 ones in
- * three bf16 planes; operands that TMA cannot read where they are need the workspace (256-byte aligned). */
+ * three bf16 planes; operands that TMA cannot read where they are need the workspace (256-byte aligned).
+ * column_sums: fp32 sums over the tokens of a token-major matrix (the bias gradient). */
+T81B200_API int t81b200_column_sums(const void *g, int dtype, int64_t tokens, int64_t cols, int64_t ld, float *out, void *stream);
 T81B200_API int t81b200_qat_quantize_t2(const float *w, int64_t rows, int64_t cols, int64_t ld, float threshold, const float *scale, uint8_t *t2,
                                         uint8_t *t2_transposed, float *scale_out, int64_t n_scales, void *stream);
 T81B200_API size_t t81b200_qat_weight_grad_workspace_bytes(const void *g, int64_t ldg, const void *x, int64_t ldx, int dtype, int64_t tokens,

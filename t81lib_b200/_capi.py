@@ -28,7 +28,7 @@ EXPORTS = (
     "t81b200_copy_columns", "t81b200_gemm_trit_peers", "t81b200_exchange_wait", "t81b200_hint_independent",
     "t81b200_gemm_limb_auto", "t81b200_gemm_trit_auto", "t81b200_elementwise", "t81b200_elementwise_auto",
     "t81b200_release_staging", "t81b200_exchange_signal", "t81b200_gemm_trit_grouped", "t81b200_t2_bytes", "t81b200_pack_t2", "t81b200_prefers_streaming", "t81b200_gemm_trit_t2", "t81b200_gemm_trit_t2_peers", "t81b200_linear_t2_workspace_bytes", "t81b200_linear_t2", "t81b200_tq_bytes", "t81b200_packed_to_tq", "t81b200_tq_to_packed",
-    "t81b200_qat_update_scale", "t81b200_qat_quantize_pack", "t81b200_qat_quantize_t2", "t81b200_qat_weight_grad_workspace_bytes", "t81b200_qat_weight_grad",
+    "t81b200_qat_update_scale", "t81b200_qat_quantize_pack", "t81b200_qat_quantize_t2", "t81b200_qat_weight_grad_workspace_bytes", "t81b200_qat_weight_grad", "t81b200_column_sums",
 )
 TQ1_0, TQ2_0 = 0, 1
 T2_MAX_TOKENS = 128  # T81B200_T2_MAX_ROWS
@@ -86,6 +86,7 @@ def _load() -> ctypes.CDLL:
     lib.t81b200_qat_weight_grad_workspace_bytes.argtypes = [vp, i64, vp, i64, ci, i64, i64, i64]
     lib.t81b200_qat_weight_grad_workspace_bytes.restype = ctypes.c_size_t
     lib.t81b200_qat_weight_grad.argtypes = [vp, i64, vp, i64, ci, i64, i64, i64, vp, i64, vp, vp, vp, ctypes.c_size_t, vp]
+    lib.t81b200_column_sums.argtypes = [vp, ci, i64, i64, i64, vp, vp]
     lib.t81b200_tq_bytes.argtypes = [ci, i64, i64]
     lib.t81b200_tq_bytes.restype = i64
     lib.t81b200_packed_to_tq.argtypes = [vp, vp, i64, i64, ci, vp, vp]
@@ -113,6 +114,22 @@ def _load() -> ctypes.CDLL:
 
 
 lib = _load()
+
+
+def _load_native():
+    """``_t81_torch``: the Python layer's per-call host work in native code (torch's headers, entering ``lib``)."""
+    import importlib.machinery
+    import importlib.util
+
+    import torch  # noqa: F401  (its libraries are what the module links against)
+    from . import build as _build
+    loader = importlib.machinery.ExtensionFileLoader("t81lib_b200._t81_torch", _build.NATIVE_PATH)
+    module = importlib.util.module_from_spec(importlib.util.spec_from_file_location(loader.name, _build.NATIVE_PATH, loader=loader))
+    loader.exec_module(module)
+    return module
+
+
+native = _load_native()
 
 
 def last_error() -> str:

@@ -17,6 +17,7 @@ _PKG = os.path.dirname(os.path.abspath(__file__))
 _CSRC = os.path.join(_PKG, "csrc")
 _LIBDIR = os.path.join(_PKG, "lib")
 LIB_PATH = os.path.join(_LIBDIR, "libt81_b200.so")
+NATIVE_PATH = os.path.join(_LIBDIR, "_t81_torch.so")  # torch_binding.cpp: the Python layer's host path
 
 SOURCES = ["capi.cu", "quantize_pack.cu", "gemm_limb.cu", "gemv_trit.cu", "gemv_trit_lut.cu", "gemm_trit_simt.cu", "gemm_trit_tc.cu", "gemm_wgrad_tc.cu", "elementwise.cu", "tq_codec.cu", "qat.cu", "pack_t2.cu"]
 NVCC_FLAGS = [
@@ -29,6 +30,24 @@ NVCC_FLAGS = [
 def _flags() -> list:
     """The nvcc flags, plus whatever T81B200_NVCC_EXTRA adds (instrumented builds, e.g. -DT81B200_GEMV_TRACE)."""
     return NVCC_FLAGS + os.environ.get("T81B200_NVCC_EXTRA", "").split()
+
+
+def _torch_dir() -> str:
+    """torch's installation, without importing it (an import takes seconds; its version is part of the stamp)."""
+    import importlib.util
+    return os.path.dirname(importlib.util.find_spec("torch").origin)
+
+
+def _native_cmd(obj: str, compile_only: bool = False) -> list:
+    import sysconfig
+    root = _torch_dir()
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    if compile_only:
+        return ["g++", "-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-D_GLIBCXX_USE_CXX11_ABI=1", "-w", "-c",
+                os.path.join(_CSRC, "torch_binding.cpp"), "-o", obj, f"-I{root}/include", f"-I{root}/include/torch/csrc/api/include",
+                f"-I{sysconfig.get_paths()['include']}", f"-I{cuda}/include"]
+    return ["g++", "-shared", obj, "-o", NATIVE_PATH, f"-L{_LIBDIR}", "-l:libt81_b200.so", "-Wl,-rpath,$ORIGIN",
+            f"-L{root}/lib", "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda", f"-Wl,-rpath,{root}/lib"]
 
 
 def _nvcc() -> str:
@@ -52,11 +71,13 @@ def source_hash() -> str:
         with open(d, "rb") as fh:
             h.update(fh.read())
     h.update(" ".join(_flags()).encode())
+    with open(os.path.join(_torch_dir(), "version.py"), "rb") as fh:  # the binding is compiled against torch's headers
+        h.update(fh.read())
     return h.hexdigest()
 
 
 def _stale() -> bool:
-    if not os.path.exists(LIB_PATH) or not os.path.exists(_STAMP):
+    if not all(os.path.exists(p) for p in (LIB_PATH, NATIVE_PATH, _STAMP)):
         return True
     with open(_STAMP) as fh:
         return fh.read().strip() != source_hash()
@@ -87,6 +108,8 @@ def _build_locked(verbose: bool) -> str:
         if verbose:
             cmd.insert(1, "-Xptxas=-v")
         procs.append((src, obj, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
+    binding_obj = os.path.join(objdir, "torch_binding.o")
+    native = subprocess.Popen(_native_cmd(binding_obj, compile_only=True), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     objs = []
     for src, obj, proc in procs:
         out, _ = proc.communicate()
@@ -99,6 +122,12 @@ def _build_locked(verbose: bool) -> str:
     res = subprocess.run(link, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     if res.returncode != 0:
         raise RuntimeError(f"link failed:\n{res.stdout}")
+    out, _ = native.communicate()
+    if native.returncode != 0:
+        raise RuntimeError(f"g++ failed on torch_binding.cpp:\n{out}")
+    res = subprocess.run(_native_cmd(binding_obj), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"link of torch_binding failed:\n{res.stdout}")
     with open(_STAMP, "w") as fh:
         fh.write(source_hash())
     return LIB_PATH

@@ -74,9 +74,7 @@ def _convert_linear_layer(linear: nn.Module, threshold: float, keep_biases_bf16:
         if t81_torch.DECODE_STREAM_LAYOUT:
             # the decode-stream copy too (0.25 byte per weight), so that the first decode step — possibly inside a
             # CUDA graph capture — does not have to make it
-            from . import ops
-            tw = ternary.ternary_weight
-            tw._t2 = ops.pack_t2(tw.packed, tw._rows, tw._k_actual)
+            ternary.ternary_weight._native_product()
         stats.packed_on_device += 1
         if release_float:
             # inference-only deployment: the packed bytes (2.67 bits per weight) replace the float weight

@@ -107,22 +107,42 @@ __global__ void __launch_bounds__(256) qat_quantize_pack_kernel(const T *__restr
 }
 
 // Quantise straight into the decode-stream layout of the weight (forward product) and of its transpose (input
-// gradient), in one pass over the weight.  A CTA takes 192 x 192 weights: six blocks of either layout.  Warp w owns
-// columns 32 w .. + 31, a lane one column, and walks the 192 rows (whole 128-byte reads):
+// gradient), in one pass over the weight.  A CTA takes 96 rows x 192 columns: three blocks of the weight's layout and half of six
+// of the transpose's.  Warp w owns columns 32 w .. + 31, a lane one column, and walks the 96 rows (whole 128-byte
+// reads, eight rows ahead of use: with nothing in flight while eight rows are packed the pass took 90 us):
 //   transpose: the lane's column is a row of it; eight rows in turn fill one half of a word (two bits each, at the
 //              places the layout wants), the lane eight columns on supplies the other half;
 //   weight:    two ballots per row hold 32 columns of it; lane r keeps those of row r of a 32-row tile and spreads its
 //              four bytes of each to word positions with a table.
-// Blocks are put together in shared memory and leave as contiguous 9 KB runs.  About 12 instructions per weight;
-// 14336 x 4096: 66 us, against 235 MB read and 29 MB written (41 us at the measured copy rate); writing limbs and
-// unpacking them for the gradient took 0.6 ms.
+// Blocks are put together in shared memory and leave as contiguous runs (4.5 KB, and 96 bytes of the transpose).  The rows
+// are taken last first: the scale's reduction has just read the weight front to back, and its end is still in L2.
 __device__ __forceinline__ uint32_t spread_place(int c) { return (c & 1 ? 30u : 14u) - 4u * (uint32_t)(c >> 1); }  // of column c of eight, first row of the pair
+
+// The rule compares w / scale, rounded, with the threshold, and keeps zeros (t81/qat.py:12-25).  Rounded division is
+// monotonic, so that is a comparison of |w| with the smallest value whose quotient reaches the threshold and is not
+// zero: bisected over the floats' bit patterns, from within four ulp of thr * scale where that brackets it.  (A division
+// per weight in the unrolled loop below would not fit the instruction cache: 33 us for 4096 x 4096 instead of 14.)
+__device__ float quotient_cut(float thr, float scale) {
+    auto reaches = [&](uint32_t bits) {
+        const float q = __fdiv_rn(__uint_as_float(bits), scale);
+        return q >= thr && q > 0.0f;
+    };
+    const uint32_t guess = __float_as_uint(__fmul_rn(thr, scale));
+    uint32_t lo = guess > 4u ? guess - 4u : 0u, hi = guess + 4u;  // lo: below the cut, hi: at or above it
+    if (reaches(lo) || !reaches(hi)) { lo = 0u; hi = 0x7F800000u; }
+    while (hi - lo > 1u) {
+        const uint32_t mid = lo + (hi - lo) / 2u;
+        if (reaches(mid)) hi = mid;
+        else lo = mid;
+    }
+    return __uint_as_float(hi);
+}
 
 __global__ void __launch_bounds__(192) qat_quantize_t2_kernel(const float *__restrict__ w, int64_t rows, int64_t cols, int64_t ld, float thr,
                                                               const float *__restrict__ scale_ptr, uint8_t *__restrict__ t2,
                                                               uint8_t *__restrict__ t2_t, float *__restrict__ scale_out, int64_t n_scales) {
     __shared__ uint32_t spread[256];
-    __shared__ __align__(16) uint32_t fwd[6 * 384], trn[6 * 384];
+    __shared__ __align__(16) uint32_t fwd[3 * 384], trn[6 * 192];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const float scale = *scale_ptr;
     for (int64_t i = ((int64_t)blockIdx.y * gridDim.x + blockIdx.x) * 192 + tid; i < n_scales; i += (int64_t)gridDim.x * gridDim.y * 192) scale_out[i] = scale;
@@ -131,69 +151,94 @@ __global__ void __launch_bounds__(192) qat_quantize_t2_kernel(const float *__res
         for (int c = 0; c < 8; ++c) v |= (uint32_t)((b >> c) & 1) << spread_place(c);
         spread[b] = v;
     }
-    // The rule compares w / scale, rounded, with the threshold (t81/qat.py:12-25).  Rounded division is monotonic, so that
-    // is a comparison of |w| with the smallest value whose quotient reaches the threshold: an ulp or two from thr * scale.
-    // Thresholds whose cut is not a normal number keep the division.
-    float cut = __fmul_rn(thr, scale);
-    const bool by_cut = cut >= 1e-30f && cut < 1e30f;
-    if (by_cut) {
-        for (int i = 0; i < 8 && __fdiv_rn(cut, scale) < thr; ++i) cut = __uint_as_float(__float_as_uint(cut) + 1u);
-        for (int i = 0; i < 8 && __fdiv_rn(__uint_as_float(__float_as_uint(cut) - 1u), scale) >= thr; ++i) cut = __uint_as_float(__float_as_uint(cut) - 1u);
-    }
+    const float cut = quotient_cut(thr, scale);
     __syncthreads();
-    const int64_t row0 = (int64_t)blockIdx.y * 192, col = (int64_t)blockIdx.x * 192 + 32 * warp + lane;
+    const int64_t rb = gridDim.y - 1 - blockIdx.y, row0 = rb * 96, col = (int64_t)blockIdx.x * 192 + 32 * warp + lane;
     const bool col_ok = col < cols;
     const float *src = w + row0 * ld + col;
     const int gr = lane >> 4, g = lane & 7;
-    for (int T = 0; T < 6; ++T) {
-        uint32_t my_nz = 0, my_neg = 0;
+    auto load8 = [&](int first, float (&v)[8]) {
 #pragma unroll
-        for (int r8 = 0; r8 < 4; ++r8) {
-            float v[8];
+        for (int i = 0; i < 8; ++i) v[i] = col_ok && first < 96 && row0 + first + i < rows ? __ldg(src + (int64_t)(first + i) * ld) : 0.0f;
+    };
+    float v[8];
+    load8(0, v);
+    uint32_t my_nz = 0, my_neg = 0;
+#pragma unroll 4
+    for (int og = 0; og < 12; ++og) {  // groups of eight rows of the weight = eight columns of the transpose
+        float ahead[8];
+        load8(8 * og + 8, ahead);
+        uint32_t half = 0;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const int64_t r = 32 * T + 8 * r8 + i;
-                v[i] = col_ok && row0 + r < rows ? __ldg(src + r * ld) : 0.0f;
-            }
-            uint32_t half = 0;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                bool nz;
-                if (by_cut) nz = fabsf(v[i]) >= cut;
-                else {
-                    const float q = __fdiv_rn(v[i], scale);
-                    nz = fabsf(q) >= thr && q != 0.0f;
-                }
-                const bool neg = nz && v[i] < 0.0f;
-                const uint32_t nz_mask = __ballot_sync(0xffffffffu, nz), neg_mask = __ballot_sync(0xffffffffu, neg);
-                if (lane == 8 * r8 + i) { my_nz = nz_mask; my_neg = neg_mask; }
-                half |= ((neg ? 2u : 0u) | (nz ? 1u : 0u)) << spread_place(i);
-            }
-            if (t2_t) {
-                const uint32_t word = half | (__shfl_down_sync(0xffffffffu, half, 8) >> 2);
-                const int og = 4 * T + r8;  // group of eight rows of the weight = eight columns of the transpose
-                if (!(lane & 8)) trn[warp * 384 + (4 * g + og / 6) * 12 + 6 * gr + og % 6] = word;
-            }
+        for (int i = 0; i < 8; ++i) {
+            const bool nz = fabsf(v[i]) >= cut;
+            const bool neg = nz && v[i] < 0.0f;
+            const uint32_t nz_mask = __ballot_sync(0xffffffffu, nz), neg_mask = __ballot_sync(0xffffffffu, neg);
+            if (lane == 8 * (og & 3) + i) { my_nz = nz_mask; my_neg = neg_mask; }
+            half |= ((neg ? 2u : 0u) | (nz ? 1u : 0u)) << spread_place(i);
         }
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            const uint32_t half = spread[(my_nz >> (8 * b)) & 0xFFu] | (spread[(my_neg >> (8 * b)) & 0xFFu] << 1);
+        if (t2_t) {
+            // word 6 gr + og % 6 of lane 4 g + t, t = 2 * (rb % 2) + og / 6: two of a block's four runs are this CTA's
             const uint32_t word = half | (__shfl_down_sync(0xffffffffu, half, 8) >> 2);
-            const int kg = 4 * warp + b;
-            if (!(lane & 8)) fwd[T * 384 + (4 * g + kg / 6) * 12 + 6 * gr + kg % 6] = word;
+            if (!(lane & 8)) trn[warp * 192 + (2 * g + og / 6) * 12 + 6 * gr + og % 6] = word;
         }
+        if ((og & 3) == 3) {
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                const uint32_t h = spread[(my_nz >> (8 * b)) & 0xFFu] | (spread[(my_neg >> (8 * b)) & 0xFFu] << 1);
+                const uint32_t word = h | (__shfl_down_sync(0xffffffffu, h, 8) >> 2);
+                const int kg = 4 * warp + b;
+                if (!(lane & 8)) fwd[(og >> 2) * 384 + (4 * g + kg / 6) * 12 + 6 * gr + kg % 6] = word;
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = ahead[i];
     }
     __syncthreads();
-    // block (chunk, row tile) of the weight: chunk = blockIdx.x, row tiles 6 blockIdx.y ..; of the transpose the other way round
+    // block (chunk, row tile) of the weight: chunk = blockIdx.x, row tiles 3 rb ..; of the transpose: chunk rb / 2, row tiles 6 blockIdx.x ..
     const int64_t tiles = (rows + 31) / 32, tiles_t = (cols + 31) / 32;
-    auto put = [&](uint8_t *out, const uint32_t *blocks, int64_t chunk, int64_t first, int64_t n_tiles) {
-        const int64_t left = n_tiles - first;
-        const int n = (int)(left < 6 ? left : 6) * 96;
-        uint4 *dst = reinterpret_cast<uint4 *>(out + (chunk * n_tiles + first) * 1536);
-        for (int i = tid; i < n; i += 192) dst[i] = reinterpret_cast<const uint4 *>(blocks)[i];
-    };
-    put(t2, fwd, blockIdx.x, (int64_t)blockIdx.y * 6, tiles);
-    if (t2_t) put(t2_t, trn, blockIdx.y, (int64_t)blockIdx.x * 6, tiles_t);
+    {
+        const int64_t left = tiles - rb * 3;
+        const int n = (int)(left < 3 ? left : 3) * 96;
+        uint4 *dst = reinterpret_cast<uint4 *>(t2 + ((int64_t)blockIdx.x * tiles + rb * 3) * 1536);
+        for (int i = tid; i < n; i += 192) dst[i] = reinterpret_cast<const uint4 *>(fwd)[i];
+    }
+    if (t2_t) {
+        const int64_t left = tiles_t - (int64_t)blockIdx.x * 6;
+        const int n = (int)(left < 6 ? left : 6) * 48;  // per block: 8 runs of 6 pieces
+        uint8_t *out = t2_t + ((rb >> 1) * tiles_t + (int64_t)blockIdx.x * 6) * 1536 + (rb & 1) * 96;
+        for (int i = tid; i < n; i += 192) *reinterpret_cast<uint4 *>(out + i / 6 * 192 + i % 6 * 16) = reinterpret_cast<const uint4 *>(trn)[i];
+        // an odd number of 96-row parts: the last chunk's other half is past the matrix
+        if (rb == gridDim.y - 1 && !(rb & 1))
+            for (int i = tid; i < n; i += 192) *reinterpret_cast<uint4 *>(out + 96 + i / 6 * 192 + i % 6 * 16) = make_uint4(0u, 0u, 0u, 0u);
+    }
+}
+
+// Column sums of a token-major matrix (the bias gradient): 32 columns per CTA, 32 warps of it take every 32nd row, eight
+// rows in flight; fp32 sums, folded in a fixed order.
+template <typename T>
+__global__ void __launch_bounds__(1024) column_sums_kernel(const T *__restrict__ g, int64_t tokens, int64_t cols, int64_t ld, float *__restrict__ out) {
+    __shared__ float part[32][33];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t col = (int64_t)blockIdx.x * 32 + lane;
+    float sum = 0.0f;
+    if (col < cols) {
+        int64_t t = warp;
+        for (; t + 7 * 32 < tokens; t += 8 * 32) {
+            float v[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] = to_float<T>(g[(t + 32 * i) * ld + col]);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) sum += v[i];
+        }
+        for (; t < tokens; t += 32) sum += to_float<T>(g[t * ld + col]);
+    }
+    part[warp][lane] = sum;
+    __syncthreads();
+    float v = part[lane][warp];  // warp = column now
+#pragma unroll
+    for (int off = 16; off >= 1; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+    if (lane == 0 && (int64_t)blockIdx.x * 32 + warp < cols) out[(int64_t)blockIdx.x * 32 + warp] = v;
 }
 
 template <typename T>
@@ -266,9 +311,26 @@ extern "C" int t81b200_qat_quantize_t2(const float *w, int64_t rows, int64_t col
     if (!w || !scale || !t2 || (n_scales > 0 && !scale_out)) return fail(T81B200_EINVAL, "qat_quantize_t2: null pointer");
     if (reinterpret_cast<uintptr_t>(t2) % 16 != 0 || reinterpret_cast<uintptr_t>(t2_transposed) % 16 != 0)
         return fail(T81B200_EALIGN, "qat_quantize_t2: the outputs must be 16-byte aligned");
-    const dim3 grid((unsigned)((cols + 191) / 192), (unsigned)((rows + 191) / 192));
+    const dim3 grid((unsigned)((cols + 191) / 192), (unsigned)((rows + 95) / 96));
     if (cols > (1ll << 31) || grid.y > 65535u) return fail(T81B200_ELIMIT, "qat_quantize_t2: matrix too large for one call");
     qat_quantize_t2_kernel<<<grid, 192, 0, static_cast<cudaStream_t>(stream)>>>(w, rows, cols, ld, threshold, scale, t2, t2_transposed, scale_out, n_scales);
     T81_LAUNCH_CHECK("qat_quantize_t2_kernel");
+    return T81B200_OK;
+}
+
+extern "C" int t81b200_column_sums(const void *g, int dtype, int64_t tokens, int64_t cols, int64_t ld, float *out, void *stream) {
+    if (tokens < 0 || cols < 0 || ld < cols) return fail(T81B200_EINVAL, "column_sums: bad dimensions");
+    if (int rc = check_device()) return rc;
+    if (cols == 0) return T81B200_OK;
+    if (!out || (tokens > 0 && !g)) return fail(T81B200_EINVAL, "column_sums: null pointer");
+    const unsigned blocks = (unsigned)((cols + 31) / 32);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    switch (dtype) {
+        case T81B200_F32: column_sums_kernel<float><<<blocks, 1024, 0, st>>>(static_cast<const float *>(g), tokens, cols, ld, out); break;
+        case T81B200_BF16: column_sums_kernel<__nv_bfloat16><<<blocks, 1024, 0, st>>>(static_cast<const __nv_bfloat16 *>(g), tokens, cols, ld, out); break;
+        case T81B200_F16: column_sums_kernel<__half><<<blocks, 1024, 0, st>>>(static_cast<const __half *>(g), tokens, cols, ld, out); break;
+        default: return fail(T81B200_EINVAL, "column_sums: unknown dtype %d", dtype);
+    }
+    T81_LAUNCH_CHECK("column_sums_kernel");
     return T81B200_OK;
 }

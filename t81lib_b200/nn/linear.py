@@ -7,8 +7,8 @@ ternary matmul, optional per-row scale, bias — on the activations where they
 live.  Training mode keeps the reference's quantisation-aware forward — the
 ternary quantiser with its surrogate gradient on ``weight / scale`` and a running
 absmax scale (t81/nn/linear.py:72-99, t81/qat.py:12-57): with the weight on a CUDA
-device the scale update, quantise + pack and the product run on the device kernels
-(``_FusedQATLinear``); stochastic rounding and CPU weights take the PyTorch form.
+device the scale update, quantise + pack, the product and the gradients run on the device
+kernels (``qat_linear`` of the native binding); stochastic rounding and CPU weights take the PyTorch form.
 """
 
 from __future__ import annotations
@@ -20,6 +20,7 @@ import torch
 from torch import nn
 from torch.nn import functional as F
 
+from .. import _capi
 from .. import torch as t81_torch
 
 _DEFAULT_THRESHOLD = 0.45
@@ -60,53 +61,6 @@ def ternary(x: torch.Tensor, threshold: float = 0.45, stochastic: bool = False) 
     return _StraightThrough.apply(dorso_round(x), quantized)
 
 
-class _FusedQATLinear(torch.autograd.Function):
-    """Training step on the device kernels: one pass over the weight quantises it with the running scale into the
-    decode-stream layout of the weight and of its transpose; the products of the forward and of the input gradient run
-    on them with the scale as row scale, the weight gradient on the transposed operands.
-    Backward is the reference's (t81/nn/linear.py:72-80 through t81/qat.py:28-57): the input gradient is
-    grad @ (trits * scale); the weight gradient is grad^T @ x times the surrogate's slope, 2 where
-    |weight / scale| < 0.5 and 0 elsewhere (the scale itself carries no gradient)."""
-
-    @staticmethod
-    def forward(ctx, x, weight, bias, scale, threshold):
-        from .. import ops
-        rows, cols = weight.shape
-        w = weight.detach()
-        t2, t2_t, scales = ops.qat_quantize_t2(w if w.stride(1) == 1 else w.contiguous(), threshold, scale, ctx.needs_input_grad[0])
-        x2 = x.detach().reshape(-1, cols)
-        if x2.dtype not in (torch.float32, torch.bfloat16, torch.float16):
-            x2 = x2.float()
-        if x2.stride(1) != 1:
-            x2 = x2.contiguous()
-        b = bias
-        if b is not None:
-            b = b.detach().to(device=x2.device, dtype=torch.float32).contiguous()
-        y = ops.linear_t2(t2, rows, x2, cols, scales, b)
-        ctx.save_for_backward(x2, weight, scale)
-        ctx.t2_t, ctx.scales, ctx.has_bias, ctx.x_shape = t2_t, scales, bias is not None, x.shape
-        return y.reshape(*x.shape[:-1], rows)
-
-    @staticmethod
-    def backward(ctx, grad_output):
-        from .. import ops
-        x2, weight, scale = ctx.saved_tensors
-        rows, cols = weight.shape
-        g = grad_output.reshape(-1, rows)
-        if g.stride(1) != 1 or (g.shape[0] > 1 and g.stride(0) < rows):
-            g = g.contiguous()
-        grad_x = grad_w = grad_b = None
-        if ctx.needs_input_grad[0]:
-            # every mantissa bit of a float32 gradient counts here: three planes
-            grad_x = ops.linear_t2(ctx.t2_t, cols, g, rows, ctx.scales, fp32_planes=3).reshape(ctx.x_shape)
-        if ctx.needs_input_grad[1]:
-            w = weight.detach()
-            grad_w = ops.qat_weight_grad(g, x2, w if w.stride(1) == 1 else w.contiguous(), scale)
-        if ctx.has_bias and ctx.needs_input_grad[2]:
-            grad_b = g.sum(dim=0)
-        return grad_x, grad_w, grad_b, None, None
-
-
 class Linear(nn.Linear):
     """Balanced-ternary ``nn.Linear``; ``rule`` selects the eval-mode quantiser
     ("fixed": the reference's fixed threshold; "absmean": per-row scaled)."""
@@ -131,13 +85,22 @@ class Linear(nn.Linear):
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         if self.training:
             if self.weight.is_cuda and x.is_cuda and not self._stochastic_rounding and self.weight.dtype == torch.float32:
-                # fused path: running scale, quantise + pack and the product all on the device kernels
-                scale = self._update_training_scale_on_device()
-                return _FusedQATLinear.apply(x, self.weight, self.bias, scale, float(max(0.0, min(self.ternary_threshold, 1.0))))
+                # fused path: running scale, quantise + pack, the product and the gradients all on the device kernels
+                state = self._qat_state_on_device()
+                y = _capi.native.qat_linear(x, self.weight, self.bias, state[0], 0.99, float(max(0.0, min(self.ternary_threshold, 1.0))))
+                if self._buffers["training_scale"] is not state[1]:
+                    self.training_scale = state[1]
+                return y
             return F.linear(x, self._quantize_training_weight(), self.bias)
-        if self.ternary_weight is None:
-            self.ternary_weight = t81_torch.TernaryTensor.from_float(
+        ternary_weight = self.ternary_weight
+        if ternary_weight is None:
+            ternary_weight = self.ternary_weight = t81_torch.TernaryTensor.from_float(
                 self.weight.detach(), threshold=self.ternary_threshold, rule=self.ternary_rule)
+        product = ternary_weight._product
+        if product is not None and t81_torch.DECODE_STREAM_LAYOUT:
+            y = product(x, self._parameters["bias"])  # None: a call that needs a conversion, a copy or an autograd node
+            if y is not None:
+                return y
         return self._packed_linear(x)
 
     def _packed_linear(self, x: torch.Tensor) -> torch.Tensor:
@@ -154,22 +117,19 @@ class Linear(nn.Linear):
                             stochastic=self._stochastic_rounding)
         return quantized * scale
 
-    def _update_training_scale_on_device(self) -> torch.Tensor:
-        """``_update_training_scale`` as one reduction kernel: no host synchronisation, the scale stays on the
-        device.  ``training_scale`` keeps its meaning (a 0-dim float32 tensor holding the running scale)."""
-        from .. import ops
+    def _qat_state_on_device(self):
+        """The running scale of the fused path: (four floats on the weight's device, the 0-dim view of the scale), no host
+        synchronisation.  ``training_scale`` keeps its meaning (a 0-dim float32 tensor holding the running scale)."""
         device = self.weight.device
         state = self.__dict__.get("_qat_state")
-        if state is None or state.device != device:
-            state = torch.zeros(4, dtype=torch.float32, device=device)
+        if state is None or state[0].device != device:
+            values = torch.zeros(4, dtype=torch.float32, device=device)
             existing = self.training_scale
             if existing is not None:  # carried over from the PyTorch path or another device
-                state[0] = existing.to(device=device, dtype=torch.float32)
-                state[3] = 1.0
-            self.__dict__["_qat_state"] = state
-        scale = ops.qat_update_scale(self.weight.detach(), state)
-        self.training_scale = state[0]
-        return scale
+                values[0] = existing.to(device=device, dtype=torch.float32)
+                values[3] = 1.0
+            state = self.__dict__["_qat_state"] = (values, values[0])
+        return state
 
     def _update_training_scale(self) -> torch.Tensor:
         device = self.weight.device

@@ -238,30 +238,10 @@ def pack_t2(packed: torch.Tensor, rows: int, cols: int) -> torch.Tensor:
 
 def linear_t2(t2: torch.Tensor, M: int, x: torch.Tensor, K: int, row_scale: Optional[torch.Tensor] = None,
               bias: Optional[torch.Tensor] = None, out_dtype: Optional[torch.dtype] = None, fp32_planes: int = 2) -> torch.Tensor:
-    """One matrix in the decode-stream layout times any number of activation rows, with as little host work as the
-    call allows (a decode-sized kernel runs a few microseconds).  ``x`` is (tokens, K) with unit column stride on
+    """One matrix in the decode-stream layout times any number of activation rows.  ``x`` is (tokens, K) with unit column stride on
     ``t2``'s device; ``row_scale`` and ``bias`` are contiguous float32 on that device or None.  ``fp32_planes``: bf16 planes
     that float32 activations enter the products as (2: 16 mantissa bits, 3: all 24)."""
-    tokens = x.shape[0]
-    dev = x.device
-    C = torch.empty((tokens, M), dtype=out_dtype or x.dtype, device=dev)
-    if tokens == 0:
-        return C
-    ldx = x.stride(0) if tokens > 1 else max(K, 1)
-    code, xp = _DTYPES[x.dtype], x.data_ptr()
-    ws, need = None, _capi.lib.t81b200_linear_t2_workspace_bytes(xp, code, ldx, M, tokens, K, fp32_planes)
-    if need:
-        ws = torch.empty(need, dtype=torch.uint8, device=dev)
-    args = (t2.data_ptr(), _ptr(row_scale), _ptr(bias), C.data_ptr(), M, xp, code, ldx, _DTYPES[C.dtype], max(M, 1), tokens, K,
-            1.0, 0.0, fp32_planes, _ptr(ws), need, torch.cuda.current_stream(dev).cuda_stream)
-    if torch.cuda.current_device() == dev.index:
-        rc = _capi.lib.t81b200_linear_t2(*args)
-    else:
-        with torch.cuda.device(dev):
-            rc = _capi.lib.t81b200_linear_t2(*args)
-    if rc:
-        _capi.check(rc)
-    return C
+    return _capi.native.linear_t2(t2, M, x, K, row_scale, bias, out_dtype, fp32_planes)
 
 
 def gemm_trit_t2(t2, rows, x: torch.Tensor, *, K: int, row_scales=None, biases=None, outs=None,
@@ -445,15 +425,4 @@ def qat_quantize_t2(weight: torch.Tensor, threshold: float, scale: torch.Tensor,
 def qat_weight_grad(grad: torch.Tensor, x: torch.Tensor, weight: torch.Tensor, scale: torch.Tensor) -> torch.Tensor:
     """``(grad^T x) * slope`` in float32 for token-major ``grad`` (tokens, rows) and ``x`` (tokens, cols) of one dtype;
     slope is 2 where ``|weight / scale| < 0.5`` and 0 elsewhere (t81/qat.py:28-57)."""
-    rows, cols = weight.shape
-    tokens, dev = x.shape[0], weight.device
-    grad = grad if grad.stride(1) == 1 and (tokens < 2 or grad.stride(0) >= rows) else grad.contiguous()
-    x = x if x.stride(1) == 1 and (tokens < 2 or x.stride(0) >= cols) else x.contiguous()
-    ldg, ldx = (grad.stride(0), x.stride(0)) if tokens > 1 else (rows, cols)
-    out = torch.empty((rows, cols), dtype=torch.float32, device=dev)
-    need = _capi.lib.t81b200_qat_weight_grad_workspace_bytes(_ptr(grad), ldg, _ptr(x), ldx, _DTYPES[x.dtype], tokens, rows, cols)
-    ws = torch.empty(need, dtype=torch.uint8, device=dev) if need else None
-    with torch.cuda.device(dev):
-        _capi.check(_capi.lib.t81b200_qat_weight_grad(_ptr(grad), ldg, _ptr(x), ldx, _DTYPES[x.dtype], tokens, rows, cols, _ptr(weight),
-                                                      weight.stride(0) if rows > 1 else max(cols, 1), _ptr(scale), _ptr(out), _ptr(ws), need, _stream(dev)))
-    return out
+    return _capi.native.qat_weight_grad(grad, x, weight, scale)

@@ -86,6 +86,7 @@ class TernaryTensor(torch.Tensor):
         "_threshold",
         "_rule",
         "_t2",
+        "_product",
     )
 
     def __new__(
@@ -112,6 +113,7 @@ class TernaryTensor(torch.Tensor):
         tensor._threshold = _clamp_threshold(threshold)
         tensor._rule = rule
         tensor._t2 = None  # the decode-stream layout, made by the first product
+        tensor._product = None  # the native call on it
         return tensor
 
     @property
@@ -160,7 +162,7 @@ class TernaryTensor(torch.Tensor):
         ops.quantize_pack(dev_float, self._threshold, self._rule, out=self._packed,
                           row_scale_out=self._row_scale)
         self._float_source = dev_float
-        self._t2 = None
+        self._t2 = self._product = None
 
     def to_trits(self) -> torch.Tensor:
         """int8 (rows, cols) trits (the inverse of the packer)."""
@@ -171,6 +173,14 @@ class TernaryTensor(torch.Tensor):
         if self._row_scale is not None:
             w = w * self._row_scale.to(dtype)[:, None]
         return w
+
+    def _native_product(self):
+        """The native call on the decode-stream layout, both made on first use."""
+        if self._product is None:
+            if self._t2 is None:
+                self._t2 = ops.pack_t2(self._packed, self._rows, self._k_actual)
+            self._product = _capi.native.Product(self._t2, self._rows, self._k_actual, self._row_scale)
+        return self._product
 
     def matmul_input(self, input: torch.Tensor, bias: Optional[torch.Tensor] = None,
                      out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
@@ -186,14 +196,15 @@ class TernaryTensor(torch.Tensor):
             if DECODE_STREAM_LAYOUT and self._rows > 0 and self._k_actual > 0:
                 # the weight in the decode-stream layout (made once): a quarter fewer bytes to stream, and two
                 # instructions per pair of trits to expand
-                if self._t2 is None:
-                    self._t2 = ops.pack_t2(self._packed, self._rows, self._k_actual)
-                x = input if input.stride(1) == 1 else input.contiguous()
-                if x.dtype not in (torch.float32, torch.bfloat16, torch.float16):
-                    raise ValueError(f"x must be float32, bfloat16 or float16, got {x.dtype}")
-                if bias is not None and (bias.dtype != torch.float32 or bias.device != x.device or not bias.is_contiguous()):
-                    bias = bias.detach().to(device=x.device, dtype=torch.float32).contiguous()
-                return ops.linear_t2(self._t2, self._rows, x, self._k_actual, self._row_scale, bias, out_dtype)
+                product = self._native_product()
+                if input.dtype not in (torch.float32, torch.bfloat16, torch.float16):
+                    raise ValueError(f"x must be float32, bfloat16 or float16, got {input.dtype}")
+                if bias is not None and (bias.dtype != torch.float32 or bias.device != input.device or not bias.is_contiguous() or bias.requires_grad):
+                    bias = bias.detach().to(device=input.device, dtype=torch.float32).contiguous()
+                y = product(input, bias, out_dtype)
+                if y is None:  # columns that are not contiguous, overlapping rows, a tensor subclass
+                    y = ops.linear_t2(self._t2, self._rows, input.as_subclass(torch.Tensor).contiguous(), self._k_actual, self._row_scale, bias, out_dtype)
+                return y
             return ops.gemm_trit(self._packed, input, M=self._rows, K=self._k_actual, layout="nk",
                                  row_scale=self._row_scale, bias=bias, out_dtype=out_dtype)
         return _TernaryLinearFunction.apply(self, input, bias, out_dtype)
