@@ -52,6 +52,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 #include <unordered_map>
 
 namespace cg = cooperative_groups;
@@ -123,7 +124,7 @@ struct GemvLutParams {
     int stages, stage_bytes;
     int ring0_stages;        // ring slots [0, ring0_stages) lie at offset 0, the others at ring1_offset
     int ring1_offset, xs_offset, part_offset, sb_offset, bar_offset;
-    int bulk_x;              // 1: bf16 activations, 16-byte aligned rows, K % 8 == 0: fetched by bulk copies
+    int bulk_x;              // 1: 16-bit activations, 16-byte aligned rows, K % 8 == 0: fetched by bulk copies
     int independent;         // 1: reads nothing the previous kernel of the stream wrote
     int n_peers;             // other GPUs whose result receives every output element too (one segment only)
     void *peer_C[T81B200_MAX_PEERS];
@@ -134,13 +135,19 @@ struct GemvLutParams {
                              // the shifts of the decode on the multiply-add pipe, beside the masks on the logic pipe
 };
 
-__device__ __forceinline__ void mma_bf16_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                               uint32_t b0, uint32_t b1) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-        "{%0,%1,%2,%3};\n"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+// fp16 activations multiply as fp16, everything else as bf16 (fp32 in two planes); weights are exact in both.
+template <bool F16>
+__device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    if constexpr (F16)
+        asm volatile(
+            "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+            : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+            : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+    else
+        asm volatile(
+            "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+            : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+            : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
 __device__ __forceinline__ uint32_t pack_bf16_pair(float lo, float hi) {
@@ -163,8 +170,8 @@ template <> __device__ __forceinline__ uint32_t pack_pair<float>(float lo, float
 struct LutImage {
     uint32_t w[32 * 2 * 16 * 2];
 };
-constexpr uint32_t trit_bits(int d) { return d == 0 ? 0xBF80u : (d == 2 ? 0x3F80u : 0u); }  // digit d = trit + 1
-constexpr LutImage make_lut_image() {
+constexpr LutImage make_lut_image(uint32_t one) {
+    auto trit_bits = [one](int d) { return d == 0 ? 0x8000u | one : (d == 2 ? one : 0u); };  // digit d = trit + 1
     LutImage im{};
     for (int b = 0; b < 32; ++b) {
         const uint32_t t0 = b < 27 ? trit_bits(b % 3) : 0u, t1 = b < 27 ? trit_bits((b / 3) % 3) : 0u, t2 = b < 27 ? trit_bits(b / 9) : 0u;
@@ -177,7 +184,8 @@ constexpr LutImage make_lut_image() {
     }
     return im;
 }
-__device__ __align__(128) const LutImage g_lut_image = make_lut_image();
+__device__ __align__(128) const LutImage g_lut_image = make_lut_image(0x3F80u);
+__device__ __align__(128) const LutImage g_lut_image_f16 = make_lut_image(0x3C00u);
 
 // One 32-bit word of a limb (4 trytes = 12 trits) -> 6 registers of adjacent trit pairs.
 // lane_key = the CTA's shared-memory window (top byte) | kLutAbs | (lane % 16) * 8.
@@ -196,28 +204,51 @@ __device__ __forceinline__ void lut_decode_word(uint32_t w, uint32_t lane_key, u
     o[3] = e1x; o[4] = e1y | o1x; o[5] = o1y;
 }
 
-template <typename XT> struct LutPlanes { static constexpr int value = 2; };
-template <> struct LutPlanes<__nv_bfloat16> { static constexpr int value = 1; };
+template <typename XT> struct LutPlanes { static constexpr int value = 1; };
+template <> struct LutPlanes<float> { static constexpr int value = 2; };
 
 // Activations of the CTA's limbs [0, nl) (limb 0 = limb L0 of the row) for every token, element by element
-// (fp32 / fp16 values, unaligned rows), in natural order, zero beyond K.  Plane 0 holds bf16(x); plane 1
-// (PLANES == 2) holds bf16(x - plane 0), so that plane 0 + plane 1 carries 16 mantissa bits of an fp32 / fp16 input.
+// (fp32 values, rows a bulk copy cannot take), in natural order, zero beyond K.  Plane 0 holds bf16(x); plane 1
+// (PLANES == 2) holds bf16(x - plane 0), so that plane 0 + plane 1 carries 16 mantissa bits of an fp32 input.  A thread has
+// the loads of four pairs in flight: one at a time, their latency was most of the call.
 template <typename XT, int PLANES>
 __device__ __forceinline__ void stage_elements(const GemvLutParams &p, int L0, int nl, uint32_t *xs, int tok_stride,
                                                int plane_stride, int tid, int nthreads) {
     const XT *X = static_cast<const XT *>(p.X);
     const int per_tok = nl * 24;
-    for (int item = tid; item < p.ntok * per_tok; item += nthreads) {
-        const int tok = item / per_tok, r = item - tok * per_tok;
-        const int64_t k = (int64_t)L0 * 48 + 2 * r;
-        const float e0 = k < p.K ? to_float<XT>(X[(int64_t)tok * p.ldx + k]) : 0.0f;
-        const float e1 = k + 1 < p.K ? to_float<XT>(X[(int64_t)tok * p.ldx + k + 1]) : 0.0f;
-        const uint32_t hi = pack_bf16_pair(e0, e1);
-        uint32_t *dst = xs + tok * tok_stride + r;
-        *dst = hi;
-        if constexpr (PLANES == 2) {
-            const __nv_bfloat162 hv = *reinterpret_cast<const __nv_bfloat162 *>(&hi);
-            dst[plane_stride] = pack_bf16_pair(e0 - __low2float(hv), e1 - __high2float(hv));
+    if (per_tok == 0) return;
+    const int64_t k_first = (int64_t)L0 * 48;
+    int tok = 0, r = tid;  // pair r of token tok
+    auto settle = [&]() { while (r >= per_tok && tok < p.ntok) { r -= per_tok; ++tok; } };
+    settle();
+    while (tok < p.ntok) {
+        XT e[4][2];
+        uint32_t *dst[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int64_t k = k_first + 2 * r;
+            const bool there = tok < p.ntok;
+            const XT *src = X + (int64_t)tok * p.ldx + k;
+            dst[u] = there ? xs + tok * tok_stride + r : nullptr;
+            e[u][0] = there && k < p.K ? src[0] : from_float<XT>(0.0f);
+            e[u][1] = there && k + 1 < p.K ? src[1] : from_float<XT>(0.0f);
+            r += nthreads;
+            settle();
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            if (!dst[u]) break;
+            if constexpr (PLANES == 1) {
+                uint32_t both;
+                memcpy(&both, e[u], 4);
+                *dst[u] = both;
+            } else {
+                const float e0 = to_float<XT>(e[u][0]), e1 = to_float<XT>(e[u][1]);
+                const uint32_t hi = pack_bf16_pair(e0, e1);
+                const __nv_bfloat162 hv = *reinterpret_cast<const __nv_bfloat162 *>(&hi);
+                *dst[u] = hi;
+                dst[u][plane_stride] = pack_bf16_pair(e0 - __low2float(hv), e1 - __high2float(hv));
+            }
         }
     }
 }
@@ -227,6 +258,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 gemv_trit_lut_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ CUtensorMap map1,
                      const __grid_constant__ CUtensorMap map2, const GemvLutParams p) {
     constexpr int PLANES = LutPlanes<XT>::value;
+    constexpr bool kF16 = std::is_same<XT, __half>::value;
     constexpr int kTokPad = 8 * TOKB;
     extern __shared__ __align__(128) uint8_t smem[];
     TRACE_STAMP(0);
@@ -295,7 +327,7 @@ gemv_trit_lut_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
     // "everything before it has".
     if (p.independent) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
-    // Activations by bulk copy (bf16, 16-byte aligned rows, K a multiple of 8): the copies bring exactly the
+    // Activations by bulk copy (16-bit types, 16-byte aligned rows, K a multiple of 8): the copies bring exactly the
     // elements below K, one copy per token and piece; piece j holds the elements of chunks
     // [j * x_group, (j + 1) * x_group) that exist.  Issuing a copy costs its warp tens of nanoseconds, so the
     // consumer warps share them out (lane 0 of each), in piece order: no warp starts its chunks late.
@@ -315,7 +347,7 @@ gemv_trit_lut_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
         }
     };
     auto issue_x = [&](int who, int n_who) {  // copies who, who + n_who, ... in piece order
-        const __nv_bfloat16 *X = static_cast<const __nv_bfloat16 *>(p.X);
+        const uint16_t *X = static_cast<const uint16_t *>(p.X);  // either 16-bit type
         for (int i = who; i < kXPieces * p.ntok; i += n_who) {
             const int j = i / p.ntok, tok = i - j * p.ntok;
             int e0, e1;
@@ -366,7 +398,7 @@ gemv_trit_lut_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
                 if (bias_by_copy) bytes += (uint32_t)rows_per_cta * 4u;
                 if (bytes) mbar_arrive_expect_tx(pro_bar, bytes);
                 else mbar_arrive(pro_bar);
-                if constexpr (FMT == 0) bulk_load(smem_u32(lut), &g_lut_image, (uint32_t)kLutBytes, pro_bar);
+                if constexpr (FMT == 0) bulk_load(smem_u32(lut), kF16 ? &g_lut_image_f16 : &g_lut_image, (uint32_t)kLutBytes, pro_bar);
                 if (scale_by_copy) bulk_load(smem_u32(sb), S.row_scale + cta_row0, (uint32_t)rows_per_cta * 4u, pro_bar);
                 if (bias_by_copy) bulk_load(smem_u32(sb + rows_per_cta), S.bias + cta_row0, (uint32_t)rows_per_cta * 4u, pro_bar);
             }
@@ -468,7 +500,7 @@ gemv_trit_lut_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
 #pragma unroll
                             for (int pl = 0; pl < PLANES; ++pl) {
                                 const uint32_t *xw = reinterpret_cast<const uint32_t *>(&xr[b][pl][0]) + 2 * m;
-                                mma_bf16_16816(acc[gr][m % NACC][b], a0, a1, a2, a3, xw[0], xw[1]);
+                                mma_16816<kF16>(acc[gr][m % NACC][b], a0, a1, a2, a3, xw[0], xw[1]);
                             }
                     }
                 }
@@ -508,9 +540,9 @@ gemv_trit_lut_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
                         for (int pl = 0; pl < PLANES; ++pl) {
                             // registers 6w .. 6w+5 of the limb <-> activation registers 6w .. 6w+5
                             const uint32_t *xw = reinterpret_cast<const uint32_t *>(&xr[b][pl][0]) + 6 * w;
-                            mma_bf16_16816(acc[gr][(3 * w) % NACC][b], oa[0], ob[0], oa[1], ob[1], xw[0], xw[1]);
-                            mma_bf16_16816(acc[gr][(3 * w + 1) % NACC][b], oa[2], ob[2], oa[3], ob[3], xw[2], xw[3]);
-                            mma_bf16_16816(acc[gr][(3 * w + 2) % NACC][b], oa[4], ob[4], oa[5], ob[5], xw[4], xw[5]);
+                            mma_16816<kF16>(acc[gr][(3 * w) % NACC][b], oa[0], ob[0], oa[1], ob[1], xw[0], xw[1]);
+                            mma_16816<kF16>(acc[gr][(3 * w + 1) % NACC][b], oa[2], ob[2], oa[3], ob[3], xw[2], xw[3]);
+                            mma_16816<kF16>(acc[gr][(3 * w + 2) % NACC][b], oa[4], ob[4], oa[5], ob[5], xw[4], xw[5]);
                         }
                 }
             }
@@ -731,7 +763,7 @@ bool lay_out(Plan &pl, int fmt, int planes, int ntok, int tokpad, int rwv, int k
 }
 
 int make_plan(Plan &pl, const PlanKey &key) {
-    const int planes = key.x_dtype == T81B200_BF16 ? 1 : 2;
+    const int planes = key.x_dtype == T81B200_F32 ? 2 : 1;
     const int tokpad = key.ntok > 8 ? 16 : 8;
     const int64_t kl = (key.K + 47) / 48;
     const int kl4 = (int)((kl + 3) & ~(int64_t)3);
@@ -899,7 +931,7 @@ int gemv_trit_lut_launch(int fmt, int n_seg, const uint8_t *const *A, const floa
     p.row_warps = pl.row_warps; p.k_warps = pl.k_warps; p.limbs_per_slice = pl.limbs_per_slice;
     p.stages = pl.stages; p.stage_bytes = pl.stage_bytes; p.ring0_stages = pl.ring0_stages; p.ring1_offset = pl.ring1_offset;
     p.xs_offset = pl.xs_offset; p.part_offset = pl.part_offset; p.sb_offset = pl.sb_offset; p.bar_offset = pl.bar_offset;
-    p.bulk_x = x_dtype == T81B200_BF16 && reinterpret_cast<uintptr_t>(X) % 16 == 0 && (ldx * 2) % 16 == 0 && K % 8 == 0 ? 1 : 0;
+    p.bulk_x = x_dtype != T81B200_F32 && reinterpret_cast<uintptr_t>(X) % 16 == 0 && (ldx * 2) % 16 == 0 && K % 8 == 0 ? 1 : 0;
     p.n_peers = ctx ? ctx->n_peers : 0;
     for (int i = 0; i < T81B200_MAX_PEERS; ++i) p.peer_C[i] = i < p.n_peers ? ctx->peer_C[i] : nullptr;
     p.sync_local = ctx ? ctx->sync_local : nullptr;

@@ -290,7 +290,7 @@ quantize_pack_ring_kernel(const T *__restrict__ w, int rows, int cols, int64_t l
     __syncthreads();
     // launched with programmatic stream serialization: everything above overlaps the tail of the kernel before
     // this one in the stream; nothing below reads or writes global memory before that kernel has completed
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // (the kernel does not release its successor early: a decode-sized product reads its weights before it waits)
     asm volatile("griddepcontrol.wait;" ::: "memory");
 
     if (warp_in_cta == TEAMS * 4) {

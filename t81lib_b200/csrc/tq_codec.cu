@@ -24,14 +24,19 @@ constexpr int kBlock = 256;
 
 __host__ __device__ constexpr int block_bytes(int format) { return format == T81B200_TQ2_0 ? 66 : 54; }
 
-// Both directions work in groups of three blocks: 768 elements, 256 trytes.  A warp takes one group at a time, turns it
-// into one byte per digit (trit + 1) in shared memory with four trytes or four block bytes per arithmetic step — digits
-// are small enough for byte- or halfword-wise sums in a 32-bit register — and puts the other form together from there.
-// Global memory is touched in whole words (trytes) and halfwords (blocks start on even bytes), each byte once; buffers
-// that start on odd addresses (`wide` false) are taken byte by byte.  The
-// byte-at-a-time form (one CTA per block) took 349 us for 14336 x 4096 TQ1_0 out and back; 65 MB cross memory (10 us).
-constexpr int kGroup = 3 * kBlock;
-constexpr int kWarps = 8;
+// Both directions work in runs of twelve blocks of a row: 3072 elements, 1024 trytes (three blocks are the least that end
+// on a tryte).  A warp takes one run at a time, turns it into one byte per digit (trit + 1) in shared memory with four
+// trytes or four block bytes per arithmetic step — digits are small enough for byte- or halfword-wise sums in a 32-bit
+// register — and puts the other form together from there.  Twelve, because a TQ1_0 block is 13 words of work: 156 items fill
+// five warp passes, where the 39 of three blocks leave most of a second one idle; and its four loads of a lane are in
+// flight together.  Global memory is touched in whole words (trytes) and halfwords (blocks start on even bytes), each byte
+// once; buffers that start on odd addresses (`wide` false) are taken byte by byte.  Bound by instructions.
+// 14336 x 4096 TQ1_0 out and back: 349 us byte at a time (one CTA per block), 100 us with three blocks a warp, 58 us this
+// way; 65 MB cross memory (10 us).
+constexpr int kRunBlocks = 12;
+constexpr int kRun = kRunBlocks * kBlock;      // elements
+constexpr int kPieces = kRun / 768;            // 256 trytes each: eight per lane
+constexpr int kWarps = 4;
 
 // Four trytes -> their twelve digits in element order.
 __device__ __forceinline__ void word_digits(uint32_t b, uint32_t (&w)[3]) {
@@ -72,156 +77,187 @@ __device__ __forceinline__ void clear_past(uint32_t (&w)[WORDS], int64_t left) {
             if (4 * i + j >= left) w[i] = (w[i] & ~(0xFFu << (8 * j))) | (1u << (8 * j));
 }
 
+// Word k of a block's payload: the digit words it is made of, first + m * pitch.  TQ2_0: four; TQ1_0: five, or four and
+// a zero digit for the last word.
+template <int FORMAT>
+__device__ __forceinline__ void digit_words(int k, int &first, int &pitch) {
+    if constexpr (FORMAT == T81B200_TQ2_0) {
+        first = (k >> 3) * 32 + (k & 7);
+        pitch = 8;
+    } else {
+        first = k < 8 ? k : (k < 12 ? 32 + k : 60);
+        pitch = k < 8 ? 8 : (k < 12 ? 4 : 1);
+    }
+}
+
 template <int FORMAT>
 __global__ void __launch_bounds__(kWarps * 32) packed_to_tq_kernel(const uint8_t *__restrict__ packed, const float *__restrict__ row_scale, int64_t rows,
                                                                    int64_t cols, int64_t row_bytes, uint8_t *__restrict__ blocks, int64_t blocks_per_row,
-                                                                   int64_t groups_per_row, bool wide) {
-    constexpr int kBytes = block_bytes(FORMAT), kWords = FORMAT == T81B200_TQ2_0 ? 16 : 13;  // digit words of a block's payload
-    __shared__ __align__(16) uint32_t digits[kWarps][kGroup / 4];
-    __shared__ __align__(16) uint8_t staged[kWarps][3 * 66 + 2];
+                                                                   int runs_per_row, bool wide) {
+    constexpr int kBytes = block_bytes(FORMAT), kWords = FORMAT == T81B200_TQ2_0 ? 16 : 13;  // words of a block's payload
+    __shared__ __align__(16) uint32_t digits[kWarps][kRun / 4];
+    __shared__ __align__(16) uint8_t staged[kWarps][kRunBlocks * 66];
+    __shared__ uint8_t nonzero[kWarps][kRunBlocks];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t *q = digits[warp];
-    const int64_t total = rows * groups_per_row, stride = (int64_t)gridDim.x * kWarps;
-    for (int64_t item = (int64_t)blockIdx.x * kWarps + warp; item < total; item += stride) {
-        const int64_t row = item / groups_per_row, group = item - row * groups_per_row;
-        // eight trytes a lane
-        const int64_t byte0 = group * 256 + lane * 8, e0 = group * kGroup + lane * 24;
-        uint2 in = make_uint2(kZeroTryteWord, kZeroTryteWord);
-        if (byte0 < row_bytes) {  // limbs are 16 bytes: all eight or none
-            const uint8_t *src = packed + row * row_bytes + byte0;
-            if (wide) in = __ldg(reinterpret_cast<const uint2 *>(src));
-            else in = make_uint2(bytes_word(src), bytes_word(src + 4));
+    const int64_t total = rows * runs_per_row;
+    for (int64_t at = (int64_t)blockIdx.x * kWarps + warp; at < total; at += (int64_t)gridDim.x * kWarps) {
+        const int64_t row = total < (1ll << 32) ? (int64_t)((uint32_t)at / (uint32_t)runs_per_row) : at / runs_per_row;
+        const int run = (int)(at - row * runs_per_row);
+        uint2 in[kPieces];
+        const int64_t byte0 = (int64_t)run * (kRun / 3) + lane * 8;
+#pragma unroll
+        for (int i = 0; i < kPieces; ++i) {
+            in[i] = make_uint2(kZeroTryteWord, kZeroTryteWord);
+            if (byte0 + 256 * i < row_bytes) {  // limbs are 16 bytes: all eight or none
+                const uint8_t *src = packed + row * row_bytes + byte0 + 256 * i;
+                if (wide) in[i] = __ldg(reinterpret_cast<const uint2 *>(src));
+                else in[i] = make_uint2(bytes_word(src), bytes_word(src + 4));
+            }
         }
-        uint32_t lo[3], hi[3];
-        word_digits(in.x, lo);
-        word_digits(in.y, hi);
-        uint32_t w[6] = {lo[0], lo[1], lo[2], hi[0], hi[1], hi[2]};
-        if (e0 + 24 > cols) clear_past<6>(w, cols - e0);
         __syncwarp();
+        if (lane < kRunBlocks) nonzero[warp][lane] = 0;
 #pragma unroll
-        for (int i = 0; i < 3; ++i) *reinterpret_cast<uint2 *>(q + lane * 6 + 2 * i) = make_uint2(w[2 * i], w[2 * i + 1]);
+        for (int i = 0; i < kPieces; ++i) {
+            uint32_t lo[3], hi[3];
+            word_digits(in[i].x, lo);
+            word_digits(in[i].y, hi);
+            uint32_t w[6] = {lo[0], lo[1], lo[2], hi[0], hi[1], hi[2]};
+            const int64_t e0 = (int64_t)run * kRun + 768 * i + lane * 24;
+            if (e0 + 24 > cols) clear_past<6>(w, cols - e0);
+#pragma unroll
+            for (int j = 0; j < 3; ++j) *reinterpret_cast<uint2 *>(q + i * 192 + lane * 6 + 2 * j) = make_uint2(w[2 * j], w[2 * j + 1]);
+        }
         __syncwarp();
-        const int n_blocks = (int)(blocks_per_row - 3 * group < 3 ? blocks_per_row - 3 * group : 3);
+        const int64_t left = blocks_per_row - (int64_t)run * kRunBlocks;
+        const int n_blocks = (int)(left < kRunBlocks ? left : kRunBlocks);
+        for (int item = lane; item < n_blocks * kWords; item += 32) {
+            const int b = item / kWords, k = item - b * kWords;
+            int first, pitch;
+            digit_words<FORMAT>(k, first, pitch);
+            const uint32_t *blk = q + b * 64 + first;
+            uint32_t v = 0, differs = 0;
+            if constexpr (FORMAT == T81B200_TQ2_0) {
 #pragma unroll
-        for (int b = 0; b < 3; ++b) {
-            uint32_t v = 0;
-            bool nonzero = false;
-            if (b < n_blocks && lane < kWords) {
-                const uint32_t *blk = q + b * 64;  // words of four digits
-                auto at = [&](int word) { const uint32_t x = blk[word]; nonzero |= x != 0x01010101u; return x; };
-                if constexpr (FORMAT == T81B200_TQ2_0) {
-                    const int half = lane >> 3, j = lane & 7;
-#pragma unroll
-                    for (int m = 0; m < 4; ++m) v |= at(half * 32 + 8 * m + j) << (2 * m);
-                } else {
-                    uint32_t n = 0;  // base-3 numbers 0..242, byte by byte
-                    if (lane < 8) {
-#pragma unroll
-                        for (int m = 0; m < 5; ++m) n = 3u * n + at(8 * m + lane);
-                    } else if (lane < 12) {
-#pragma unroll
-                        for (int m = 0; m < 5; ++m) n = 3u * n + at(40 + 4 * m + lane - 8);
-                    } else {
-#pragma unroll
-                        for (int m = 0; m < 4; ++m) n = 3u * n + at(60 + m);
-                        n = 3u * n;
-                    }
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) v |= ((((n >> (8 * j)) & 0xFFu) * 256u + 242u) / 243u) << (8 * j);
+                for (int m = 0; m < 4; ++m) {
+                    const uint32_t x = blk[m * pitch];
+                    differs |= x ^ 0x01010101u;
+                    v |= x << (2 * m);
                 }
-                uint16_t *dst = reinterpret_cast<uint16_t *>(staged[warp] + b * kBytes) + lane * 2;
-                dst[0] = (uint16_t)v;
-                dst[1] = (uint16_t)(v >> 16);
+            } else {
+                uint32_t n = 0;  // base-3 numbers 0..242, byte by byte
+#pragma unroll
+                for (int m = 0; m < 5; ++m) {
+                    const bool there = m < 4 || k < 12;
+                    const uint32_t x = there ? blk[m * pitch] : 0u;
+                    differs |= there ? x ^ 0x01010101u : 0u;
+                    n = 3u * n + x;
+                }
+                // ceil(256 n / 243), exact for all 243 values
+#pragma unroll
+                for (int j = 0; j < 4; ++j) v |= ((((n >> (8 * j)) & 0xFFu) * 8631u + 8100u) >> 13) << (8 * j);
             }
-            // the scale of a block with no non-zero trit is 0, like the absmax of an all-zero block
-            nonzero = __any_sync(0xffffffffu, nonzero);
-            if (b < n_blocks && lane == 0) {
-                const float d = nonzero ? (row_scale ? row_scale[row] : 1.0f) : 0.0f;
-                *reinterpret_cast<uint16_t *>(staged[warp] + b * kBytes + kBytes - 2) = __half_as_ushort(__float2half_rn(d));
-            }
+            if (differs) nonzero[warp][b] = 1;
+            uint16_t *dst = reinterpret_cast<uint16_t *>(staged[warp] + b * kBytes) + k * 2;
+            dst[0] = (uint16_t)v;
+            dst[1] = (uint16_t)(v >> 16);
         }
         __syncwarp();
-        uint16_t *out = reinterpret_cast<uint16_t *>(blocks + (row * blocks_per_row + 3 * group) * kBytes);
+        // the scale of a block with no non-zero trit is 0, like the absmax of an all-zero block
+        if (lane < n_blocks) {
+            const float d = nonzero[warp][lane] ? (row_scale ? row_scale[row] : 1.0f) : 0.0f;
+            *reinterpret_cast<uint16_t *>(staged[warp] + lane * kBytes + kBytes - 2) = __half_as_ushort(__float2half_rn(d));
+        }
+        __syncwarp();
+        uint8_t *out = blocks + (row * blocks_per_row + (int64_t)run * kRunBlocks) * kBytes;
         if (wide)
-            for (int i = lane; i < n_blocks * kBytes / 2; i += 32) out[i] = reinterpret_cast<const uint16_t *>(staged[warp])[i];
+            for (int i = lane; i < n_blocks * kBytes / 2; i += 32) reinterpret_cast<uint16_t *>(out)[i] = reinterpret_cast<const uint16_t *>(staged[warp])[i];
         else
-            for (int i = lane; i < n_blocks * kBytes; i += 32) reinterpret_cast<uint8_t *>(out)[i] = staged[warp][i];
+            for (int i = lane; i < n_blocks * kBytes; i += 32) out[i] = staged[warp][i];
     }
 }
 
 template <int FORMAT>
 __global__ void __launch_bounds__(kWarps * 32) tq_to_packed_kernel(const uint8_t *__restrict__ blocks, int64_t rows, int64_t cols, int64_t row_bytes,
                                                                    uint8_t *__restrict__ packed, float *__restrict__ block_scale, int64_t blocks_per_row,
-                                                                   int64_t groups_per_row, bool wide) {
-    constexpr int kBytes = block_bytes(FORMAT), kWords = FORMAT == T81B200_TQ2_0 ? 16 : 13;
-    __shared__ __align__(16) uint32_t digits[kWarps][kGroup / 4];
-    __shared__ __align__(16) uint8_t staged[kWarps][3 * 66 + 2];
+                                                                   int runs_per_row, bool wide) {
+    constexpr int kBytes = block_bytes(FORMAT), kWords = FORMAT == T81B200_TQ2_0 ? 16 : 13, kHalves = kRunBlocks * kBytes / 2, kLoads = (kHalves + 31) / 32;
+    __shared__ __align__(16) uint32_t digits[kWarps][kRun / 4];
+    __shared__ __align__(16) uint8_t staged[kWarps][kRunBlocks * 66];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t *q = digits[warp];
-    const int64_t total = rows * groups_per_row, stride = (int64_t)gridDim.x * kWarps;
-    for (int64_t item = (int64_t)blockIdx.x * kWarps + warp; item < total; item += stride) {
-        const int64_t row = item / groups_per_row, group = item - row * groups_per_row;
-        const int n_blocks = (int)(blocks_per_row - 3 * group < 3 ? blocks_per_row - 3 * group : 3);
-        const uint16_t *in = reinterpret_cast<const uint16_t *>(blocks + (row * blocks_per_row + 3 * group) * kBytes);
+    const int64_t total = rows * runs_per_row;
+    for (int64_t at = (int64_t)blockIdx.x * kWarps + warp; at < total; at += (int64_t)gridDim.x * kWarps) {
+        const int64_t row = total < (1ll << 32) ? (int64_t)((uint32_t)at / (uint32_t)runs_per_row) : at / runs_per_row;
+        const int run = (int)(at - row * runs_per_row);
+        const int64_t left = blocks_per_row - (int64_t)run * kRunBlocks;
+        const int n_blocks = (int)(left < kRunBlocks ? left : kRunBlocks);
+        const uint8_t *in = blocks + (row * blocks_per_row + (int64_t)run * kRunBlocks) * kBytes;
         __syncwarp();
-        if (wide)
-            for (int i = lane; i < n_blocks * kBytes / 2; i += 32) reinterpret_cast<uint16_t *>(staged[warp])[i] = __ldg(in + i);
-        else
-            for (int i = lane; i < n_blocks * kBytes; i += 32) staged[warp][i] = reinterpret_cast<const uint8_t *>(in)[i];
+        if (wide) {
+            uint16_t h[kLoads];
+#pragma unroll
+            for (int i = 0; i < kLoads; ++i) h[i] = lane + 32 * i < n_blocks * kBytes / 2 ? __ldg(reinterpret_cast<const uint16_t *>(in) + lane + 32 * i) : (uint16_t)0;
+#pragma unroll
+            for (int i = 0; i < kLoads; ++i)
+                if (lane + 32 * i < kHalves) reinterpret_cast<uint16_t *>(staged[warp])[lane + 32 * i] = h[i];
+        } else
+            for (int i = lane; i < n_blocks * kBytes; i += 32) staged[warp][i] = in[i];
         __syncwarp();
-        for (int i = lane; i < 3 * kWords; i += 32) {
-            const int b = i / kWords, k = i - b * kWords;
-            if (b >= n_blocks) break;  // elements past the row: cleared below
+        for (int item = lane; item < n_blocks * kWords; item += 32) {
+            const int b = item / kWords, k = item - b * kWords;
             const uint16_t *src = reinterpret_cast<const uint16_t *>(staged[warp] + b * kBytes) + 2 * k;
             const uint32_t x = (uint32_t)src[0] | ((uint32_t)src[1] << 16);
-            uint32_t *blk = q + b * 64;
+            int first, pitch;
+            digit_words<FORMAT>(k, first, pitch);
+            uint32_t *blk = q + b * 64 + first;
             if constexpr (FORMAT == T81B200_TQ2_0) {
-                const int half = k >> 3, j = k & 7;
 #pragma unroll
                 for (int m = 0; m < 4; ++m) {
                     const uint32_t d = (x >> (2 * m)) & 0x03030303u;
-                    blk[half * 32 + 8 * m + j] = d - (d & (d >> 1) & 0x01010101u);  // 3 reads as 2
+                    blk[m * pitch] = d - (d & (d >> 1) & 0x01010101u);  // 3 reads as 2
                 }
             } else {
                 // digit m of a byte is the top of byte * 3^m (mod 256) * 3 (t81/gguf.py:629-637)
                 uint32_t even = x & 0x00FF00FFu, odd = (x >> 8) & 0x00FF00FFu;
-                const int pitch = k < 8 ? 8 : (k < 12 ? 4 : 1), first = k < 8 ? k : (k < 12 ? 40 + k - 8 : 60), n = k < 12 ? 5 : 4;
 #pragma unroll
                 for (int m = 0; m < 5; ++m) {
                     even *= 3u;
                     odd *= 3u;
-                    if (m < n) blk[first + m * pitch] = ((even >> 8) & 0x00FF00FFu) | (odd & 0xFF00FF00u);
+                    if (m < 4 || k < 12) blk[m * pitch] = ((even >> 8) & 0x00FF00FFu) | (odd & 0xFF00FF00u);
                     even &= 0x00FF00FFu;
                     odd &= 0x00FF00FFu;
                 }
             }
         }
         __syncwarp();
-        const int64_t byte0 = group * 256 + lane * 8, e0 = group * kGroup + lane * 24;
-        if (byte0 < row_bytes) {
+#pragma unroll
+        for (int i = 0; i < kPieces; ++i) {
+            const int64_t byte0 = (int64_t)run * (kRun / 3) + 256 * i + lane * 8, e0 = (int64_t)run * kRun + 768 * i + lane * 24;
+            if (byte0 >= row_bytes) break;
             uint32_t w[6];
 #pragma unroll
-            for (int i = 0; i < 3; ++i) {
-                const uint2 d = *reinterpret_cast<const uint2 *>(q + lane * 6 + 2 * i);
-                w[2 * i] = d.x;
-                w[2 * i + 1] = d.y;
+            for (int j = 0; j < 3; ++j) {
+                const uint2 d = *reinterpret_cast<const uint2 *>(q + i * 192 + lane * 6 + 2 * j);
+                w[2 * j] = d.x;
+                w[2 * j + 1] = d.y;
             }
             if (e0 + 24 > cols) clear_past<6>(w, cols - e0);
             const uint32_t t0 = digits_word(w[0], w[1], w[2]), t1 = digits_word(w[3], w[4], w[5]);
             uint8_t *dst = packed + row * row_bytes + byte0;
             if (wide) *reinterpret_cast<uint2 *>(dst) = make_uint2(t0, t1);
             else
-                for (int i = 0; i < 4; ++i) { dst[i] = (uint8_t)(t0 >> (8 * i)); dst[4 + i] = (uint8_t)(t1 >> (8 * i)); }
+                for (int j = 0; j < 4; ++j) { dst[j] = (uint8_t)(t0 >> (8 * j)); dst[4 + j] = (uint8_t)(t1 >> (8 * j)); }
         }
         if (block_scale && lane < n_blocks)
-            block_scale[row * blocks_per_row + 3 * group + lane] =
+            block_scale[row * blocks_per_row + (int64_t)run * kRunBlocks + lane] =
                 __half2float(__ushort_as_half(*reinterpret_cast<const uint16_t *>(staged[warp] + lane * kBytes + kBytes - 2)));
     }
 }
 
-// A few groups per warp: enough CTAs to fill the GPU, no more than are resident at a time.
-unsigned tq_grid(int64_t groups) {
-    const int64_t ctas = (groups + kWarps - 1) / kWarps, most = (int64_t)sm_count() * 8;
+// A warp per run, up to about what is resident at a time.
+unsigned tq_grid(int64_t runs) {
+    const int64_t ctas = (runs + kWarps - 1) / kWarps, most = (int64_t)sm_count() * 12;
     return (unsigned)(ctas < most ? ctas : most);
 }
 
@@ -245,12 +281,12 @@ extern "C" int t81b200_packed_to_tq(const uint8_t *packed, const float *row_scal
     const int64_t bpr = (cols + kBlock - 1) / kBlock, row_bytes = (cols + 47) / 48 * 16;
     if (bpr > 65535 || rows >= (1ll << 31)) return fail(T81B200_ELIMIT, "tq: matrix too large for one call");
     const bool wide = reinterpret_cast<uintptr_t>(packed) % 8 == 0 && reinterpret_cast<uintptr_t>(blocks) % 2 == 0;
-    const int64_t groups = (bpr + 2) / 3;
+    const int64_t runs = (bpr + kRunBlocks - 1) / kRunBlocks;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (format == T81B200_TQ2_0)
-        packed_to_tq_kernel<T81B200_TQ2_0><<<tq_grid(rows * groups), kWarps * 32, 0, st>>>(packed, row_scale, rows, cols, row_bytes, blocks, bpr, groups, wide);
+        packed_to_tq_kernel<T81B200_TQ2_0><<<tq_grid(rows * runs), kWarps * 32, 0, st>>>(packed, row_scale, rows, cols, row_bytes, blocks, bpr, (int)runs, wide);
     else
-        packed_to_tq_kernel<T81B200_TQ1_0><<<tq_grid(rows * groups), kWarps * 32, 0, st>>>(packed, row_scale, rows, cols, row_bytes, blocks, bpr, groups, wide);
+        packed_to_tq_kernel<T81B200_TQ1_0><<<tq_grid(rows * runs), kWarps * 32, 0, st>>>(packed, row_scale, rows, cols, row_bytes, blocks, bpr, (int)runs, wide);
     T81_LAUNCH_CHECK("packed_to_tq_kernel");
     return T81B200_OK;
 }
@@ -265,12 +301,12 @@ extern "C" int t81b200_tq_to_packed(const uint8_t *blocks, int64_t rows, int64_t
     const int64_t bpr = (cols + kBlock - 1) / kBlock, row_bytes = (cols + 47) / 48 * 16;
     if (bpr > 65535 || rows >= (1ll << 31)) return fail(T81B200_ELIMIT, "tq: matrix too large for one call");
     const bool wide = reinterpret_cast<uintptr_t>(packed) % 8 == 0 && reinterpret_cast<uintptr_t>(blocks) % 2 == 0;
-    const int64_t groups = (bpr + 2) / 3;
+    const int64_t runs = (bpr + kRunBlocks - 1) / kRunBlocks;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (format == T81B200_TQ2_0)
-        tq_to_packed_kernel<T81B200_TQ2_0><<<tq_grid(rows * groups), kWarps * 32, 0, st>>>(blocks, rows, cols, row_bytes, packed, block_scale, bpr, groups, wide);
+        tq_to_packed_kernel<T81B200_TQ2_0><<<tq_grid(rows * runs), kWarps * 32, 0, st>>>(blocks, rows, cols, row_bytes, packed, block_scale, bpr, (int)runs, wide);
     else
-        tq_to_packed_kernel<T81B200_TQ1_0><<<tq_grid(rows * groups), kWarps * 32, 0, st>>>(blocks, rows, cols, row_bytes, packed, block_scale, bpr, groups, wide);
+        tq_to_packed_kernel<T81B200_TQ1_0><<<tq_grid(rows * runs), kWarps * 32, 0, st>>>(blocks, rows, cols, row_bytes, packed, block_scale, bpr, (int)runs, wide);
     T81_LAUNCH_CHECK("tq_to_packed_kernel");
     return T81B200_OK;
 }
