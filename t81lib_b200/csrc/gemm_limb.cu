@@ -6,6 +6,7 @@
 // A and 16 of B to doubles once (32 threads, one limb each), so a decode is
 // shared by 16 outputs instead of being redone per output element.
 #include "common.cuh"
+#include "host_staging.cuh"
 
 #include <mutex>
 
@@ -68,39 +69,10 @@ gemm_limb_kernel(const uint8_t *__restrict__ A, const uint8_t *__restrict__ B, f
     if (live) C[i * N + j] = (float)acc;
 }
 
-// Staging buffers of the entry points that take host pointers: one set per device, kept for
-// the life of the process and grown on demand.
-struct HostStaging {
-    std::mutex mu;
-    void *a = nullptr, *b = nullptr, *c = nullptr, *ws = nullptr;
-    size_t a_cap = 0, b_cap = 0, c_cap = 0, ws_cap = 0;
-};
-constexpr int kMaxDevices = 64;
-HostStaging g_staging[kMaxDevices];
-
-int staging_for_current_device(HostStaging **out) {
-    int dev = 0;
-    T81_CUDA_TRY(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= kMaxDevices) return fail(T81B200_ELIMIT, "device index %d not supported", dev);
-    *out = &g_staging[dev];
-    return T81B200_OK;
-}
-
-int grow(void **p, size_t *cap, size_t need) {
-    if (need <= *cap) return T81B200_OK;
-    if (*p) cudaFree(*p);
-    *p = nullptr; *cap = 0;
-    T81_CUDA_TRY(cudaMalloc(p, need));
-    *cap = need;
-    return T81B200_OK;
-}
-
 }  // namespace
 
 // 1: memory a kernel of the current device can dereference (device or managed memory);
 // 0: host memory (pageable or pinned).  Null pointers count as "either".
-void release_elementwise_staging();  // elementwise.cu
-
 int pointer_is_device(const void *p, int *is_device) {
     *is_device = 0;
     if (!p) return T81B200_OK;
@@ -117,26 +89,6 @@ int pointer_is_device(const void *p, int *is_device) {
 }  // namespace t81b200
 
 using namespace t81b200;
-
-extern "C" int t81b200_release_staging(void) {
-    if (int rc = check_device()) return rc;
-    int cur = 0, count = 0;
-    T81_CUDA_TRY(cudaGetDevice(&cur));
-    T81_CUDA_TRY(cudaGetDeviceCount(&count));
-    for (int d = 0; d < count && d < kMaxDevices; ++d) {
-        HostStaging &s = g_staging[d];
-        std::lock_guard<std::mutex> lock(s.mu);
-        if (!s.a && !s.b && !s.c && !s.ws) continue;
-        T81_CUDA_TRY(cudaSetDevice(d));
-        void **bufs[4] = {&s.a, &s.b, &s.c, &s.ws};
-        for (void **b : bufs) { if (*b) cudaFree(*b); *b = nullptr; }
-        s.a_cap = s.b_cap = s.c_cap = s.ws_cap = 0;
-    }
-    T81_CUDA_TRY(cudaSetDevice(cur));
-    release_elementwise_staging();
-    T81_CUDA_TRY(cudaSetDevice(cur));
-    return T81B200_OK;
-}
 
 extern "C" int t81b200_gemm_limb(const uint8_t *A, const uint8_t *B, float *C, int64_t M, int64_t N,
                                  int64_t k_limbs, float alpha, float beta, void *stream) {
@@ -158,21 +110,19 @@ extern "C" int t81b200_gemm_limb_host(const uint8_t *A, const uint8_t *B, float 
     if (M == 0 || N == 0) return T81B200_OK;
     if (!C || (k_limbs > 0 && (!A || !B))) return fail(T81B200_EINVAL, "gemm_limb_host: null pointer");
     HostStaging *stg = nullptr;
-    if (int rc = staging_for_current_device(&stg)) return rc;
+    if (int rc = host_staging(&stg)) return rc;
     std::lock_guard<std::mutex> lock(stg->mu);
+    if (int rc = host_staging_ready(*stg)) return rc;
     const size_t a_bytes = (size_t)M * k_limbs * 16, b_bytes = (size_t)k_limbs * N * 16, c_bytes = (size_t)M * N * 4;
-    if (int rc = grow(&stg->a, &stg->a_cap, a_bytes ? a_bytes : 16)) return rc;
-    if (int rc = grow(&stg->b, &stg->b_cap, b_bytes ? b_bytes : 16)) return rc;
-    if (int rc = grow(&stg->c, &stg->c_cap, c_bytes)) return rc;
-    if (a_bytes) T81_CUDA_TRY(cudaMemcpyAsync(stg->a, A, a_bytes, cudaMemcpyHostToDevice, 0));
-    if (b_bytes) T81_CUDA_TRY(cudaMemcpyAsync(stg->b, B, b_bytes, cudaMemcpyHostToDevice, 0));
-    T81_CUDA_TRY(cudaMemcpyAsync(stg->c, C, c_bytes, cudaMemcpyHostToDevice, 0));
-    if (int rc = t81b200_gemm_limb((const uint8_t *)stg->a, (const uint8_t *)stg->b, (float *)stg->c,
-                                   M, N, k_limbs, alpha, beta, nullptr))
+    if (int rc = host_staging_buffer(*stg, HostStaging::A, a_bytes ? a_bytes : 16)) return rc;
+    if (int rc = host_staging_buffer(*stg, HostStaging::B, b_bytes ? b_bytes : 16)) return rc;
+    if (int rc = host_staging_buffer(*stg, HostStaging::C, c_bytes)) return rc;
+    const HostOperand ops[3] = {{stg->dev[HostStaging::A], A, a_bytes}, {stg->dev[HostStaging::B], B, b_bytes}, {stg->dev[HostStaging::C], C, c_bytes}};
+    if (int rc = host_upload(*stg, ops, 3)) return rc;
+    if (int rc = t81b200_gemm_limb(static_cast<const uint8_t *>(stg->dev[HostStaging::A]), static_cast<const uint8_t *>(stg->dev[HostStaging::B]),
+                                   static_cast<float *>(stg->dev[HostStaging::C]), M, N, k_limbs, alpha, beta, stg->stream))
         return rc;
-    T81_CUDA_TRY(cudaMemcpyAsync(C, stg->c, c_bytes, cudaMemcpyDeviceToHost, 0));
-    T81_CUDA_TRY(cudaStreamSynchronize(0));
-    return T81B200_OK;
+    return host_download(*stg, C, stg->dev[HostStaging::C], c_bytes);
 }
 
 extern "C" int t81b200_gemm_limb_auto(const uint8_t *A, const uint8_t *B, float *C, int64_t M, int64_t N,
@@ -196,24 +146,24 @@ extern "C" int t81b200_gemm_limb_auto(const uint8_t *A, const uint8_t *B, float 
 static int gemm_trit_host_impl(const uint8_t *A, const float *B, float *C, int64_t M, int64_t N, int64_t K,
                                float alpha, float beta) {
     HostStaging *stg = nullptr;
-    if (int rc = staging_for_current_device(&stg)) return rc;
+    if (int rc = host_staging(&stg)) return rc;
     std::lock_guard<std::mutex> lock(stg->mu);
+    if (int rc = host_staging_ready(*stg)) return rc;
     const int64_t kl = (K + 47) / 48;
     const size_t a_bytes = (size_t)M * kl * 16, b_bytes = (size_t)K * N * 4, c_bytes = (size_t)M * N * 4;
     const size_t ws_bytes = t81b200_gemm_trit_workspace_bytes(T81B200_F32, T81B200_LAYOUT_KN, T81B200_F32, M, N, K);
-    if (int rc = grow(&stg->a, &stg->a_cap, a_bytes ? a_bytes : 16)) return rc;
-    if (int rc = grow(&stg->b, &stg->b_cap, b_bytes ? b_bytes : 16)) return rc;
-    if (int rc = grow(&stg->c, &stg->c_cap, c_bytes)) return rc;
-    if (ws_bytes) if (int rc = grow(&stg->ws, &stg->ws_cap, ws_bytes)) return rc;
-    if (a_bytes) T81_CUDA_TRY(cudaMemcpyAsync(stg->a, A, a_bytes, cudaMemcpyHostToDevice, 0));
-    if (b_bytes) T81_CUDA_TRY(cudaMemcpyAsync(stg->b, B, b_bytes, cudaMemcpyHostToDevice, 0));
-    if (beta != 0.0f) T81_CUDA_TRY(cudaMemcpyAsync(stg->c, C, c_bytes, cudaMemcpyHostToDevice, 0));
-    if (int rc = t81b200_gemm_trit((const uint8_t *)stg->a, nullptr, stg->b, T81B200_F32, T81B200_LAYOUT_KN, N,
-                                   nullptr, stg->c, T81B200_F32, N, M, N, K, alpha, beta, stg->ws, stg->ws_cap, nullptr))
+    if (int rc = host_staging_buffer(*stg, HostStaging::A, a_bytes ? a_bytes : 16)) return rc;
+    if (int rc = host_staging_buffer(*stg, HostStaging::B, b_bytes ? b_bytes : 16)) return rc;
+    if (int rc = host_staging_buffer(*stg, HostStaging::C, c_bytes)) return rc;
+    if (ws_bytes) if (int rc = host_staging_buffer(*stg, HostStaging::WORKSPACE, ws_bytes)) return rc;
+    const HostOperand ops[3] = {{stg->dev[HostStaging::B], B, b_bytes}, {stg->dev[HostStaging::A], A, a_bytes},
+                                {stg->dev[HostStaging::C], C, beta != 0.0f ? c_bytes : 0}};
+    if (int rc = host_upload(*stg, ops, 3)) return rc;
+    if (int rc = t81b200_gemm_trit(static_cast<const uint8_t *>(stg->dev[HostStaging::A]), nullptr, stg->dev[HostStaging::B], T81B200_F32,
+                                   T81B200_LAYOUT_KN, N, nullptr, stg->dev[HostStaging::C], T81B200_F32, N, M, N, K, alpha, beta,
+                                   stg->dev[HostStaging::WORKSPACE], stg->dev_cap[HostStaging::WORKSPACE], stg->stream))
         return rc;
-    T81_CUDA_TRY(cudaMemcpyAsync(C, stg->c, c_bytes, cudaMemcpyDeviceToHost, 0));
-    T81_CUDA_TRY(cudaStreamSynchronize(0));
-    return T81B200_OK;
+    return host_download(*stg, C, stg->dev[HostStaging::C], c_bytes);
 }
 
 extern "C" int t81b200_gemm_trit_host(const uint8_t *A, const float *B, float *C, int64_t M, int64_t N, int64_t K,
@@ -238,12 +188,12 @@ extern "C" int t81b200_gemm_trit_auto(const uint8_t *A, const float *B, float *C
         return fail(T81B200_EINVAL, "gemm_ternary: A, B and C must all be host memory or all be device memory");
     if (!dc) return gemm_trit_host_impl(A, B, C, M, N, K, alpha, beta);
     HostStaging *stg = nullptr;
-    if (int rc = staging_for_current_device(&stg)) return rc;
+    if (int rc = host_staging(&stg)) return rc;
     std::lock_guard<std::mutex> lock(stg->mu);
     const size_t ws_bytes = t81b200_gemm_trit_workspace_bytes(T81B200_F32, T81B200_LAYOUT_KN, T81B200_F32, M, N, K);
-    if (ws_bytes) if (int rc = grow(&stg->ws, &stg->ws_cap, ws_bytes)) return rc;
+    if (ws_bytes) if (int rc = host_staging_buffer(*stg, HostStaging::WORKSPACE, ws_bytes)) return rc;
     if (int rc = t81b200_gemm_trit(A, nullptr, B, T81B200_F32, T81B200_LAYOUT_KN, N, nullptr, C, T81B200_F32, N, M, N, K,
-                                   alpha, beta, stg->ws, stg->ws_cap, nullptr))
+                                   alpha, beta, stg->dev[HostStaging::WORKSPACE], stg->dev_cap[HostStaging::WORKSPACE], nullptr))
         return rc;
     T81_CUDA_TRY(cudaStreamSynchronize(0));
     return T81B200_OK;

@@ -1,0 +1,38 @@
+// Operands that live in ordinary host memory: device buffers, page-locked buffers on the way there and a stream, one set
+// per device, grown on demand, kept between calls and given back by t81b200_release_staging.
+#pragma once
+
+#include <mutex>
+
+#include "common.cuh"
+
+namespace t81b200 {
+
+struct HostStaging {
+    std::mutex mu;  // held for a whole call
+    enum { A, B, C, WORKSPACE, N_BUFFERS };
+    void *dev[N_BUFFERS] = {nullptr};
+    size_t dev_cap[N_BUFFERS] = {0};
+    char *pinned = nullptr;
+    size_t pinned_cap = 0;
+    cudaStream_t stream = nullptr;
+    static constexpr int kMaxPieces = 64;
+    cudaEvent_t landed[kMaxPieces] = {nullptr};
+};
+
+// The current device's set, with its stream made on first use (call with `mu` held).
+int host_staging(HostStaging **out);
+int host_staging_ready(HostStaging &s);
+int host_staging_buffer(HostStaging &s, int which, size_t bytes);
+
+struct HostOperand {
+    void *device;
+    const void *host;
+    size_t bytes;
+};
+// Queues the operands' copies to the device on s.stream, first to last.
+int host_upload(HostStaging &s, const HostOperand *ops, int n);
+// Copies device memory to the host behind what s.stream holds; returns when it is there.
+int host_download(HostStaging &s, void *host, const void *device, size_t bytes);
+
+}  // namespace t81b200

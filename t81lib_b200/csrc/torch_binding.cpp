@@ -352,7 +352,162 @@ PyObject *qat_weight_grad(PyObject *, PyObject *const *args, Py_ssize_t n) {
     END_HANDLE_TH_ERRORS
 }
 
+int64_t limbs_of(int64_t cols) { return (cols + 47) / 48; }
+
+// quantize_pack(w, threshold, rule, out or None, row_scale_out or None) -> (packed, row_scale or None)
+PyObject *quantize_pack(PyObject *, PyObject *const *args, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    if (n != 5) return PyErr_Format(PyExc_TypeError, "quantize_pack takes 5 arguments");
+    const Tensor *w = &tensor_of(args[0]);
+    const double threshold = PyFloat_AsDouble(args[1]);
+    const int rule = (int)PyLong_AsLong(args[2]);
+    std::optional<Tensor> packed = optional_tensor(args[3]), scale = optional_tensor(args[4]);
+    if (PyErr_Occurred()) return nullptr;
+    TORCH_CHECK_VALUE(w->dim() == 2, "pack_dense_matrix expects a 2D array");
+    TORCH_CHECK_VALUE(w->is_cuda(), "w must be a CUDA tensor (there is no CPU path)");
+    const int dtype = dtype_code(w->scalar_type());
+    TORCH_CHECK_VALUE(dtype >= 0, "w must be float32, bfloat16 or float16, got ", w->dtype());
+    const c10::Device device = w->device();
+    const int64_t rows = w->size(0), cols = w->size(1), kl = limbs_of(cols);
+    OnDevice on(device);
+    Tensor unit;
+    if (w->numel() > 0 && (w->stride(1) != 1 || (rows > 1 && w->stride(0) < cols))) {
+        unit = w->contiguous();
+        w = &unit;
+    }
+    if (packed) {
+        TORCH_CHECK_VALUE(packed->numel() == rows * kl * 16 && packed->scalar_type() == at::kByte && packed->is_contiguous() && packed->device() == device,
+                          "packed output buffer has the wrong size");
+    } else packed = at::empty({rows, kl, 16}, at::TensorOptions().dtype(at::kByte).device(device));
+    if (rule == T81B200_RULE_ABSMEAN) {
+        if (scale) {
+            TORCH_CHECK_VALUE(float_vector(*scale, device, rows), "row_scale output must be float32 (rows,) on the weight's device");
+        } else scale = at::empty({rows}, at::TensorOptions().dtype(at::kFloat).device(device));
+    } else scale.reset();
+    try {
+        check(t81b200_quantize_pack(w->const_data_ptr(), dtype, rows, cols, rows > 1 ? w->stride(0) : (cols > 1 ? cols : 1), (float)threshold, rule,
+                                    packed->mutable_data_ptr<uint8_t>(), scale ? scale->mutable_data_ptr<float>() : nullptr, stream_of(device)));
+    } catch (const LibraryError &e) {
+        return raise_library_error(e.code);
+    }
+    PyObject *result = PyTuple_New(2);
+    if (!result) return nullptr;
+    PyTuple_SET_ITEM(result, 0, THPVariable_Wrap(*packed));
+    PyTuple_SET_ITEM(result, 1, scale ? THPVariable_Wrap(*scale) : Py_NewRef(Py_None));
+    return result;
+    END_HANDLE_TH_ERRORS
+}
+
+// tensor_body(device_of, rows, cols): a (rows, cols) view of one element, the data-less body of a TernaryTensor.
+PyObject *tensor_body(PyObject *, PyObject *const *args, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    if (n != 3) return PyErr_Format(PyExc_TypeError, "tensor_body takes 3 arguments");
+    const Tensor &like = tensor_of(args[0]);
+    const int64_t rows = PyLong_AsLongLong(args[1]), cols = PyLong_AsLongLong(args[2]);
+    if (PyErr_Occurred()) return nullptr;
+    at::AutoDispatchBelowADInplaceOrView below;
+    return THPVariable_Wrap(at::empty({1}, at::TensorOptions().dtype(at::kFloat).device(like.device())).expand({rows, cols}));
+    END_HANDLE_TH_ERRORS
+}
+
+// packed_to_tq(packed, rows, cols, format, row_scale or None) -> blocks
+PyObject *packed_to_tq(PyObject *, PyObject *const *args, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    if (n != 5) return PyErr_Format(PyExc_TypeError, "packed_to_tq takes 5 arguments");
+    const Tensor packed = tensor_of(args[0]).contiguous();
+    const int64_t rows = PyLong_AsLongLong(args[1]), cols = PyLong_AsLongLong(args[2]);
+    const int format = (int)PyLong_AsLong(args[3]);
+    std::optional<Tensor> scale = optional_tensor(args[4]);
+    if (PyErr_Occurred()) return nullptr;
+    const c10::Device device = packed.device();
+    TORCH_CHECK_VALUE(packed.is_cuda(), "packed must be a CUDA tensor (there is no CPU path)");
+    TORCH_CHECK_VALUE(rows >= 0 && cols >= 0 && packed.nbytes() >= (size_t)(rows * limbs_of(cols) * 16), "packed does not hold rows x ceil(cols/48) limbs");
+    if (scale) {
+        scale = scale->to(device, at::kFloat).contiguous();
+        TORCH_CHECK_VALUE(scale->numel() >= rows, "row_scale must have one value per row");
+    }
+    OnDevice on(device);
+    Tensor out = at::empty({rows, (cols + 255) / 256, format == T81B200_TQ2_0 ? 66 : 54}, at::TensorOptions().dtype(at::kByte).device(device));
+    try {
+        check(t81b200_packed_to_tq(static_cast<const uint8_t *>(packed.const_data_ptr()), float_ptr(scale), rows, cols, format, out.mutable_data_ptr<uint8_t>(),
+                                   stream_of(device)));
+    } catch (const LibraryError &e) {
+        return raise_library_error(e.code);
+    }
+    return THPVariable_Wrap(out);
+    END_HANDLE_TH_ERRORS
+}
+
+// tq_to_packed(blocks, rows, cols, format) -> (packed, block_scales)
+PyObject *tq_to_packed(PyObject *, PyObject *const *args, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    if (n != 4) return PyErr_Format(PyExc_TypeError, "tq_to_packed takes 4 arguments");
+    const Tensor blocks = tensor_of(args[0]).contiguous();
+    const int64_t rows = PyLong_AsLongLong(args[1]), cols = PyLong_AsLongLong(args[2]);
+    const int format = (int)PyLong_AsLong(args[3]);
+    if (PyErr_Occurred()) return nullptr;
+    const c10::Device device = blocks.device();
+    TORCH_CHECK_VALUE(blocks.is_cuda(), "blocks must be a CUDA tensor (there is no CPU path)");
+    TORCH_CHECK_VALUE((int64_t)blocks.numel() == t81b200_tq_bytes(format, rows, cols) && blocks.element_size() == 1, "block payload size does not match (rows, cols)");
+    OnDevice on(device);
+    const auto options = at::TensorOptions().device(device);
+    Tensor packed = at::empty({rows, limbs_of(cols), 16}, options.dtype(at::kByte)), scales = at::empty({rows, (cols + 255) / 256}, options.dtype(at::kFloat));
+    try {
+        check(t81b200_tq_to_packed(static_cast<const uint8_t *>(blocks.const_data_ptr()), rows, cols, format, packed.mutable_data_ptr<uint8_t>(),
+                                   scales.mutable_data_ptr<float>(), stream_of(device)));
+    } catch (const LibraryError &e) {
+        return raise_library_error(e.code);
+    }
+    PyObject *result = PyTuple_New(2);
+    if (!result) return nullptr;
+    PyTuple_SET_ITEM(result, 0, THPVariable_Wrap(packed));
+    PyTuple_SET_ITEM(result, 1, THPVariable_Wrap(scales));
+    return result;
+    END_HANDLE_TH_ERRORS
+}
+
+// gemm_trit(packed, B, C, layout, M, N, K, row_scale or None, bias or None, alpha, beta): operands checked by the caller.
+PyObject *gemm_trit(PyObject *, PyObject *const *args, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    if (n != 11) return PyErr_Format(PyExc_TypeError, "gemm_trit takes 11 arguments");
+    const Tensor &packed = tensor_of(args[0]), &B = tensor_of(args[1]), &C = tensor_of(args[2]);
+    const int layout = (int)PyLong_AsLong(args[3]);
+    const int64_t M = PyLong_AsLongLong(args[4]), N = PyLong_AsLongLong(args[5]), K = PyLong_AsLongLong(args[6]);
+    const std::optional<Tensor> scale = optional_tensor(args[7]), bias = optional_tensor(args[8]);
+    const double alpha = PyFloat_AsDouble(args[9]), beta = PyFloat_AsDouble(args[10]);
+    if (PyErr_Occurred()) return nullptr;
+    const int b_dtype = dtype_code(B.scalar_type()), c_dtype = dtype_code(C.scalar_type());
+    const c10::Device device = B.device();
+    const int64_t ldb = B.size(0) > 1 ? B.stride(0) : (B.size(1) > 1 ? B.size(1) : 1), ldc = C.size(0) > 1 ? C.stride(0) : (C.size(1) > 1 ? C.size(1) : 1);
+    OnDevice on(device);
+    // 16-bit token-major rows on 16-byte boundaries are read in place, and up to 16 rows always are; the rest is staged
+    // (bf16 rows off those boundaries too, where the problem is large enough)
+    size_t need = 0;
+    const bool token_major = layout == T81B200_LAYOUT_NK;
+    const bool in_place = token_major && (N <= 16 || (b_dtype != T81B200_F32 && reinterpret_cast<uintptr_t>(B.const_data_ptr()) % 16 == 0 && ldb % 8 == 0));
+    if (!in_place) {
+        need = t81b200_gemm_trit_workspace_bytes(b_dtype, layout, c_dtype, M, N, K);
+        if (need == 0 && token_major && (double)M * N * K >= 1.6e7) need = (size_t)N * ((K + 7) / 8 * 8) * 2;
+    }
+    Tensor ws;
+    if (need) ws = at::empty({(int64_t)need}, at::TensorOptions().dtype(at::kByte).device(device));
+    try {
+        check(t81b200_gemm_trit(static_cast<const uint8_t *>(packed.const_data_ptr()), float_ptr(scale), B.const_data_ptr(), b_dtype, layout, ldb,
+                                float_ptr(bias), C.mutable_data_ptr(), c_dtype, ldc, M, N, K, (float)alpha, (float)beta,
+                                need ? ws.mutable_data_ptr() : nullptr, need, stream_of(device)));
+    } catch (const LibraryError &e) {
+        return raise_library_error(e.code);
+    }
+    Py_RETURN_NONE;
+    END_HANDLE_TH_ERRORS
+}
+
 PyMethodDef methods[] = {
+    {"quantize_pack", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(quantize_pack)), METH_FASTCALL, nullptr},
+    {"tensor_body", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(tensor_body)), METH_FASTCALL, nullptr},
+    {"packed_to_tq", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(packed_to_tq)), METH_FASTCALL, nullptr},
+    {"tq_to_packed", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(tq_to_packed)), METH_FASTCALL, nullptr},
+    {"gemm_trit", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(gemm_trit)), METH_FASTCALL, nullptr},
     {"qat_linear", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(qat_linear)), METH_FASTCALL, nullptr},
     {"linear_t2", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(linear_t2)), METH_FASTCALL, nullptr},
     {"qat_weight_grad", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(qat_weight_grad)), METH_FASTCALL, nullptr},

@@ -84,27 +84,10 @@ def quantize_pack(w: torch.Tensor, threshold: float = 0.5, rule: str = "fixed",
 
     Returns ``(packed uint8 (rows, k_limbs, 16), row_scale float32 (rows,) or None)``.
     """
-    if w.ndim != 2:
-        raise ValueError("pack_dense_matrix expects a 2D array")
-    _require_cuda(w, "w")
-    if rule not in _RULES:
+    code = _RULES.get(rule)
+    if code is None:
         raise ValueError(f"unknown quantiser rule {rule!r}")
-    if w.stride(1) != 1 and w.numel() > 0:
-        w = w.contiguous()
-    rows, cols = w.shape
-    kl = k_limbs(cols)
-    with torch.cuda.device(w.device):
-        packed = out if out is not None else torch.empty((rows, kl, 16), dtype=torch.uint8, device=w.device)
-        if out is not None and (out.numel() != rows * kl * 16 or out.dtype != torch.uint8 or not out.is_contiguous()):
-            raise ValueError("packed output buffer has the wrong size")
-        scale = None
-        if rule == "absmean":
-            scale = row_scale_out if row_scale_out is not None else torch.empty(rows, dtype=torch.float32, device=w.device)
-        ld = w.stride(0) if rows > 1 else max(cols, 1)
-        _capi.check(_capi.lib.t81b200_quantize_pack(
-            _ptr(w), _dtype_code(w, "w"), rows, cols, max(ld, cols), float(threshold), _RULES[rule],
-            _ptr(packed), _ptr(scale), _stream(w.device)))
-    return packed, scale
+    return _capi.native.quantize_pack(w, threshold, code, out, row_scale_out)
 
 
 def quantize_trits(values: torch.Tensor, threshold: float = 0.5) -> torch.Tensor:
@@ -181,8 +164,6 @@ def gemm_trit(packed: torch.Tensor, B: torch.Tensor, *, M: int, K: int, layout: 
         if tuple(C.shape) != c_shape or C.stride(1) != 1:
             raise ValueError(f"C must have shape {c_shape} with unit inner stride")
     b_code, c_code = _dtype_code(B, "B"), _dtype_code(C, "C")
-    ldb = B.stride(0) if B.shape[0] > 1 else max(B.shape[1], 1)
-    ldc = C.stride(0) if C.shape[0] > 1 else max(C.shape[1], 1)
     dev = B.device
     rs = row_scale
     if rs is not None and (rs.dtype != torch.float32 or rs.device != dev or not rs.is_contiguous()):
@@ -190,36 +171,23 @@ def gemm_trit(packed: torch.Tensor, B: torch.Tensor, *, M: int, K: int, layout: 
     bs = bias
     if bs is not None and (bs.dtype != torch.float32 or bs.device != dev or not bs.is_contiguous()):
         bs = bs.detach().to(device=dev, dtype=torch.float32).contiguous()
-    # 16-bit token-major rows on 16-byte boundaries are read in place; up to 16 of them always are
-    direct = code == _capi.LAYOUT_NK and (N <= 16 or (b_code != _capi.F32 and B.data_ptr() % 16 == 0 and ldb % 8 == 0))
-
-    def scratch():
-        need = 0 if direct else _capi.lib.t81b200_gemm_trit_workspace_bytes(b_code, code, c_code, M, N, K)
-        if need == 0 and not direct and code == _capi.LAYOUT_NK and M * N * K >= 16_000_000:
-            need = N * ((K + 7) // 8 * 8) * 2  # unaligned bf16 rows: staged, as the other types are
-        return _workspace(dev, need)
-    if peers:
-        for t in peers:
-            if tuple(t.shape) != tuple(C.shape) or t.stride() != C.stride() or t.dtype != C.dtype:
-                raise ValueError("peer results must have C's shape, strides and dtype")
-        ptrs = (ctypes.c_void_p * len(peers))(*[t.data_ptr() for t in peers])
-        with torch.cuda.device(dev):
-            ws = scratch()
-            _capi.check(_capi.lib.t81b200_gemm_trit_peers(
-                _ptr(packed), _ptr(rs), _ptr(B), b_code, code, ldb, _ptr(bs), _ptr(C), c_code, ldc,
-                M, N, K, float(alpha), float(beta), _ptr(ws), 0 if ws is None else ws.numel(), len(peers), ptrs,
-                None if sync is None else sync.local_ptr, None if sync is None else sync.slot_ptrs, _stream(dev)))
+    if not peers:
+        _capi.native.gemm_trit(packed, B, C, code, M, N, K, rs, bs, float(alpha), float(beta))
         return C
-    if direct and dev.index == torch.cuda.current_device():
-        _capi.check(_capi.lib.t81b200_gemm_trit(
-            packed.data_ptr(), _ptr(rs), B.data_ptr(), b_code, code, ldb, _ptr(bs), C.data_ptr(), c_code, ldc,
-            M, N, K, float(alpha), float(beta), None, 0, torch.cuda.current_stream(dev).cuda_stream))
-        return C
+    for t in peers:
+        if tuple(t.shape) != tuple(C.shape) or t.stride() != C.stride() or t.dtype != C.dtype:
+            raise ValueError("peer results must have C's shape, strides and dtype")
+    ldb = B.stride(0) if B.shape[0] > 1 else max(B.shape[1], 1)
+    ldc = C.stride(0) if C.shape[0] > 1 else max(C.shape[1], 1)
+    ptrs = (ctypes.c_void_p * len(peers))(*[t.data_ptr() for t in peers])
+    # 16-bit token-major rows on 16-byte boundaries are read in place
+    in_place = code == _capi.LAYOUT_NK and b_code != _capi.F32 and B.data_ptr() % 16 == 0 and ldb % 8 == 0
     with torch.cuda.device(dev):
-        ws = scratch()
-        _capi.check(_capi.lib.t81b200_gemm_trit(
+        ws = None if in_place else _workspace(dev, _capi.lib.t81b200_gemm_trit_workspace_bytes(b_code, code, c_code, M, N, K))
+        _capi.check(_capi.lib.t81b200_gemm_trit_peers(
             _ptr(packed), _ptr(rs), _ptr(B), b_code, code, ldb, _ptr(bs), _ptr(C), c_code, ldc,
-            M, N, K, float(alpha), float(beta), _ptr(ws), 0 if ws is None else ws.numel(), _stream(dev)))
+            M, N, K, float(alpha), float(beta), _ptr(ws), 0 if ws is None else ws.numel(), len(peers), ptrs,
+            None if sync is None else sync.local_ptr, None if sync is None else sync.slot_ptrs, _stream(dev)))
     return C
 
 
@@ -339,37 +307,17 @@ def packed_to_tq(packed: torch.Tensor, rows: int, cols: int, fmt: str = "TQ2_0",
                  row_scale: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Packed limbs (+ per-row scale) -> GGUF TQ1_0 / TQ2_0 block payload, uint8 (rows, ceil(cols/256), 54 | 66),
     on the device; the trits are carried over exactly (t81/gguf.py:518-600 without the float round trip)."""
-    _require_cuda(packed, "packed")
     if fmt not in _TQ:
         raise ValueError(f"unknown block format {fmt!r}")
-    packed = packed.contiguous()
-    nbytes = _capi.lib.t81b200_tq_bytes(_TQ[fmt], rows, cols)
-    per_block = 66 if fmt == "TQ2_0" else 54
-    out = torch.empty((rows, (cols + 255) // 256, per_block), dtype=torch.uint8, device=packed.device)
-    assert out.numel() == nbytes
-    rs = row_scale
-    if rs is not None and (rs.dtype != torch.float32 or rs.device != packed.device or not rs.is_contiguous()):
-        rs = rs.to(device=packed.device, dtype=torch.float32).contiguous()
-    with torch.cuda.device(packed.device):
-        _capi.check(_capi.lib.t81b200_packed_to_tq(_ptr(packed), _ptr(rs), rows, cols, _TQ[fmt], _ptr(out), _stream(packed.device)))
-    return out
+    return _capi.native.packed_to_tq(packed, rows, cols, _TQ[fmt], row_scale)
 
 
 def tq_to_packed(blocks: torch.Tensor, rows: int, cols: int, fmt: str = "TQ2_0"):
     """GGUF TQ1_0 / TQ2_0 block payload -> (packed limbs uint8 (rows, ceil(cols/48), 16), block scales fp32
     (rows, ceil(cols/256))), on the device."""
-    _require_cuda(blocks, "blocks")
     if fmt not in _TQ:
         raise ValueError(f"unknown block format {fmt!r}")
-    blocks = blocks.contiguous()
-    if blocks.numel() != _capi.lib.t81b200_tq_bytes(_TQ[fmt], rows, cols):
-        raise ValueError("block payload size does not match (rows, cols)")
-    packed = torch.empty((rows, k_limbs(cols), 16), dtype=torch.uint8, device=blocks.device)
-    scales = torch.empty((rows, (cols + 255) // 256), dtype=torch.float32, device=blocks.device)
-    with torch.cuda.device(blocks.device):
-        _capi.check(_capi.lib.t81b200_tq_to_packed(_ptr(blocks), rows, cols, _TQ[fmt], _ptr(packed), _ptr(scales),
-                                                   _stream(blocks.device)))
-    return packed, scales
+    return _capi.native.tq_to_packed(blocks, rows, cols, _TQ[fmt])
 
 
 def qat_update_scale(weight: torch.Tensor, state: torch.Tensor, momentum: float = 0.99) -> torch.Tensor:

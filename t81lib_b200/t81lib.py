@@ -14,10 +14,14 @@ LIMB semantics (python/bindings.cpp:769-810, src/linalg/gemm_cpu.cpp:8-71).
 
 from __future__ import annotations
 
+import warnings
+
 import numpy as np
 import torch
 
 from . import _capi, ops
+
+_NUMPY_DTYPES = {np.dtype(np.uint8): torch.uint8, np.dtype(np.float32): torch.float32}
 
 TRITS_PER_LIMB = 48
 TRYTES_PER_LIMB = 16
@@ -61,7 +65,7 @@ def _packed_to_device(obj, rows: int, cols: int) -> torch.Tensor:
         if obj.nbytes != rows * cols * BYTES_PER_LIMB:
             raise ValueError("packed limb buffer byte size mismatch")
         flat = obj.reshape(-1).view(np.uint8) if obj.nbytes else np.zeros(0, np.uint8)
-        return torch.from_numpy(flat.copy()).to(_device())
+        return _host_to_device(flat)
     try:
         view = memoryview(obj)
     except TypeError:
@@ -71,7 +75,30 @@ def _packed_to_device(obj, rows: int, cols: int) -> torch.Tensor:
     if view.nbytes != rows * cols * BYTES_PER_LIMB:
         raise ValueError("packed limb buffer byte size mismatch")
     flat = np.frombuffer(view, dtype=np.uint8) if view.nbytes else np.zeros(0, np.uint8)
-    return torch.from_numpy(flat.copy()).to(_device())
+    return _host_to_device(flat)
+
+
+def _host_to_device(array: np.ndarray) -> torch.Tensor:
+    """A device copy of a host array, read-only ones included (torch warns about those, and only reads here)."""
+    out = torch.empty(array.shape, dtype=_NUMPY_DTYPES[array.dtype], device=_device())
+    if array.size:
+        with warnings.catch_warnings():
+            warnings.simplefilter("ignore")
+            out.copy_(torch.from_numpy(array))
+    return out
+
+
+def _gemm_on_host(A, B, C, M: int, N: int, K: int, kl: int, alpha: float, beta: float) -> bool:
+    """TRIT mode with all three operands in host memory as numpy arrays of the exact types: one call that copies in,
+    multiplies and copies out.  Anything else (and every argument error) is left to the general path."""
+    if not (isinstance(A, np.ndarray) and isinstance(B, np.ndarray) and isinstance(C, np.ndarray)):
+        return False
+    if not (A.flags.c_contiguous and A.nbytes == M * kl * BYTES_PER_LIMB and B.dtype == np.float32 and B.flags.c_contiguous
+            and B.shape == (K, N) and C.dtype == np.float32 and C.flags.c_contiguous and C.flags.writeable
+            and (C.shape == (M, N) or C.shape == (M * N,))):
+        return False
+    _capi.check(_capi.lib.t81b200_gemm_trit_host(A.ctypes.data, B.ctypes.data, C.ctypes.data, M, N, K, float(alpha), float(beta)))
+    return True
 
 
 def gemm_ternary(A, B, C, M: int, N: int, K: int, alpha: float = 1.0, beta: float = 0.0) -> None:
@@ -84,6 +111,8 @@ def gemm_ternary(A, B, C, M: int, N: int, K: int, alpha: float = 1.0, beta: floa
     if K % TRITS_PER_LIMB != 0:
         raise ValueError("K must be divisible by the limb trit count")
     kl = K // TRITS_PER_LIMB
+    if M and N and _gemm_on_host(A, B, C, M, N, K, kl, alpha, beta):
+        return None
     dense_b = (_is_tensor(B) and B.is_floating_point()) or (
         isinstance(B, np.ndarray) and B.dtype.kind == "f")
     a_dev = _packed_to_device(A, M, kl)
@@ -116,7 +145,7 @@ def gemm_ternary(A, B, C, M: int, N: int, K: int, alpha: float = 1.0, beta: floa
         if not ((view.ndim == 2 and tuple(view.shape) == (M, N)) or (view.ndim == 1 and view.shape[0] == M * N)):
             raise ValueError("C tensor shape must match (M, N)")
         c_np = np.frombuffer(view, dtype=np.float32).reshape(M, N)
-        c_dev = torch.from_numpy(c_np.copy()).to(a_dev.device)
+        c_dev = _host_to_device(c_np)
         c_host = c_np
     if M == 0 or N == 0:
         return None

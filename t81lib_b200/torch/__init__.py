@@ -101,8 +101,7 @@ class TernaryTensor(torch.Tensor):
         row_scale: Optional[torch.Tensor] = None,
         rule: str = "fixed",
     ) -> "TernaryTensor":
-        body = torch.empty(1, dtype=torch.float32, device=packed.device).expand(shape)
-        tensor = torch.Tensor._make_subclass(cls, body, False)
+        tensor = torch.Tensor._make_subclass(cls, _capi.native.tensor_body(packed, *shape), False)
         tensor._packed = packed
         tensor._row_scale = row_scale
         tensor._rows = shape[0]
