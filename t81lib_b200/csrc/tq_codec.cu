@@ -24,37 +24,44 @@ constexpr int kBlock = 256;
 
 __host__ __device__ constexpr int block_bytes(int format) { return format == T81B200_TQ2_0 ? 66 : 54; }
 
-// Both directions work in runs of twelve blocks of a row: 3072 elements, 1024 trytes (three blocks are the least that end
-// on a tryte).  A warp takes one run at a time, turns it into one byte per digit (trit + 1) in shared memory with four
-// trytes or four block bytes per arithmetic step — digits are small enough for byte- or halfword-wise sums in a 32-bit
-// register — and puts the other form together from there.  Twelve, because a TQ1_0 block is 13 words of work: 156 items fill
-// five warp passes, where the 39 of three blocks leave most of a second one idle; and its four loads of a lane are in
-// flight together.  Global memory is touched in whole words (trytes) and halfwords (blocks start on even bytes), each byte
-// once; buffers that start on odd addresses (`wide` false) are taken byte by byte.  Bound by instructions.
-// 14336 x 4096 TQ1_0 out and back: 349 us byte at a time (one CTA per block), 100 us with three blocks a warp, 58 us this
-// way; 65 MB cross memory (10 us).
-constexpr int kRunBlocks = 12;
-constexpr int kRun = kRunBlocks * kBlock;      // elements
-constexpr int kPieces = kRun / 768;            // 256 trytes each: eight per lane
+// Both directions work in runs of up to nine blocks of a row: 2304 elements, 768 trytes (three blocks are the least that
+// end on a tryte; a row is cut into equal runs).  A warp takes one run at a time, turns it into one byte per digit
+// (trit + 1) in shared memory, four digits to a word, and puts the other form together from there.  Trytes become digits
+// by a table with a copy per lane (one look-up per tryte, no bank conflicts); a block's words of digits lie 76 words from
+// the next block's, so that the items of a pass (13 words of payload a TQ1_0 block) meet few of each other's banks; where
+// an item reads and writes is worked out once per warp, not once per run.  Global memory is touched in whole words
+// (trytes) and halfwords (blocks start on even bytes), each byte once; buffers that start on odd addresses (`wide` false)
+// are taken byte by byte.  Bound by instructions.
+// 14336 x 4096 TQ1_0 out and back: 349 us byte at a time (one CTA per block), 100 us with three blocks a warp and digits
+// by arithmetic, 61 us with twelve, 45 us now; 65 MB cross memory (10 us).
+constexpr int kRunBlocks = 9;
+constexpr int kPieces = kRunBlocks / 3;        // 256 trytes each: eight per lane
+constexpr int kBlockPitch = 76;                // words of digits from one block to the next
+constexpr int kDigitWords = kRunBlocks * kBlockPitch;
 constexpr int kWarps = 4;
 
-// Four trytes -> their twelve digits in element order.
-__device__ __forceinline__ void word_digits(uint32_t b, uint32_t (&w)[3]) {
-    const uint32_t bad = __vcmpgtu4(b, 0x1A1A1A1Au);  // not a tryte: reads as zero
-    b = (b & ~bad) | (kZeroTryteWord & bad);
-    uint32_t d0 = 0, d1 = 0, d2 = 0;
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const uint32_t x = (b >> (8 * h)) & 0x00FF00FFu;
-        const uint32_t e2 = ((x * 57u) >> 9) & 0x00030003u, r = x - 9u * e2;   // x / 9
-        const uint32_t e1 = ((r * 11u) >> 5) & 0x00030003u;                    // r / 3
-        d0 |= (r - 3u * e1) << (8 * h);
-        d1 |= e1 << (8 * h);
-        d2 |= e2 << (8 * h);
+__device__ __forceinline__ int digit_place(int word) { return word + (word >> 6) * (kBlockPitch - 64); }
+
+// table[value * 32 + lane]: the three digits of a tryte, first element in the low byte; 27..31 read as the zero tryte.
+__device__ __forceinline__ void fill_tryte_table(uint32_t *table, int tid, int threads) {
+    for (int i = tid; i < 32 * 32; i += threads) {
+        int d0, d1, d2;
+        tryte_digits((uint32_t)(i >> 5), d0, d1, d2);
+        table[i] = (uint32_t)(d0 | (d1 << 8) | (d2 << 16));
     }
-    w[0] = __byte_perm(__byte_perm(d0, d1, 0x1040), d2, 0x3410);                // d0[0] d1[0] d2[0] d0[1]
-    w[1] = __byte_perm(__byte_perm(d1, d2, 0x2051), __byte_perm(d0, d1, 0x0062), 0x5410);  // d1[1] d2[1] d0[2] d1[2]
-    w[2] = __byte_perm(__byte_perm(d2, d0, 0x0072), __byte_perm(d1, d2, 0x0073), 0x5410);  // d2[2] d0[3] d1[3] d2[3]
+}
+
+// Four trytes -> their twelve digits in element order.  `column` = table + lane.
+__device__ __forceinline__ void word_digits(uint32_t b, const uint32_t *column, uint32_t (&w)[3]) {
+    if (b & 0xE0E0E0E0u) {  // not trytes: they read as zero
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if ((b >> (8 * i)) & 0xE0u) b |= 0x1Fu << (8 * i);
+    }
+    const uint32_t e0 = column[(b & 31u) << 5], e1 = column[((b >> 8) & 31u) << 5], e2 = column[((b >> 16) & 31u) << 5], e3 = column[((b >> 24) & 31u) << 5];
+    w[0] = __byte_perm(e0, e1, 0x4210);
+    w[1] = __byte_perm(e1, e2, 0x5421);
+    w[2] = __byte_perm(e2, e3, 0x6542);
 }
 
 // Twelve digits -> four trytes: d0 + 3 d1 + 9 d2 (the offset 13 is the three digits' own 1 + 3 + 9).
@@ -93,72 +100,97 @@ __device__ __forceinline__ void digit_words(int k, int &first, int &pitch) {
 template <int FORMAT>
 __global__ void __launch_bounds__(kWarps * 32) packed_to_tq_kernel(const uint8_t *__restrict__ packed, const float *__restrict__ row_scale, int64_t rows,
                                                                    int64_t cols, int64_t row_bytes, uint8_t *__restrict__ blocks, int64_t blocks_per_row,
-                                                                   int runs_per_row, bool wide) {
+                                                                   int runs_per_row, int run_blocks, bool wide) {
     constexpr int kBytes = block_bytes(FORMAT), kWords = FORMAT == T81B200_TQ2_0 ? 16 : 13;  // words of a block's payload
-    __shared__ __align__(16) uint32_t digits[kWarps][kRun / 4];
-    __shared__ __align__(16) uint8_t staged[kWarps][kRunBlocks * 66];
+    constexpr int kPasses = (kRunBlocks * kWords + 31) / 32, kHalves = kRunBlocks * kBytes / 2;
+    __shared__ uint32_t table[32 * 32];
+    __shared__ __align__(16) uint32_t digits[kWarps][kDigitWords];
+    __shared__ __align__(16) uint8_t staged[kWarps][kRunBlocks * 66 + 2];
     __shared__ uint8_t nonzero[kWarps][kRunBlocks];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    fill_tryte_table(table, threadIdx.x, kWarps * 32);
+    __syncthreads();
     uint32_t *q = digits[warp];
-    const int64_t total = rows * runs_per_row;
-    for (int64_t at = (int64_t)blockIdx.x * kWarps + warp; at < total; at += (int64_t)gridDim.x * kWarps) {
-        const int64_t row = total < (1ll << 32) ? (int64_t)((uint32_t)at / (uint32_t)runs_per_row) : at / runs_per_row;
-        const int run = (int)(at - row * runs_per_row);
+    // item lane + 32 i of a run: word k of block b
+    int from[kPasses], pitch[kPasses], to[kPasses], block[kPasses];
+#pragma unroll
+    for (int i = 0; i < kPasses; ++i) {
+        const int item = lane + 32 * i, b = item / kWords, k = item - b * kWords;
+        digit_words<FORMAT>(k, from[i], pitch[i]);
+        from[i] += b * kBlockPitch;
+        to[i] = b * (kBytes / 2) + 2 * k;
+        block[i] = b;
+    }
+    const int64_t total = rows * runs_per_row, stride = (int64_t)gridDim.x * kWarps;
+    auto locate = [&](int64_t at, int64_t &row, int64_t &block0, int &n_blocks) {
+        row = total < (1ll << 32) ? (int64_t)((uint32_t)at / (uint32_t)runs_per_row) : at / runs_per_row;
+        block0 = (at - row * runs_per_row) * run_blocks;  // run_blocks is a multiple of 3
+        const int64_t left = blocks_per_row - block0;
+        n_blocks = (int)(left < run_blocks ? left : run_blocks);
+    };
+    for (int64_t at = (int64_t)blockIdx.x * kWarps + warp; at < total; at += stride) {
+        int64_t row, block0;
+        int n_blocks;
+        locate(at, row, block0, n_blocks);
         uint2 in[kPieces];
-        const int64_t byte0 = (int64_t)run * (kRun / 3) + lane * 8;
+        const int64_t byte0 = block0 * kBlock / 3 + lane * 8;
 #pragma unroll
         for (int i = 0; i < kPieces; ++i) {
             in[i] = make_uint2(kZeroTryteWord, kZeroTryteWord);
-            if (byte0 + 256 * i < row_bytes) {  // limbs are 16 bytes: all eight or none
+            if (3 * i < n_blocks && byte0 + 256 * i < row_bytes) {  // limbs are 16 bytes: all eight or none
                 const uint8_t *src = packed + row * row_bytes + byte0 + 256 * i;
                 if (wide) in[i] = __ldg(reinterpret_cast<const uint2 *>(src));
                 else in[i] = make_uint2(bytes_word(src), bytes_word(src + 4));
             }
         }
+        const int n_pieces = (n_blocks + 2) / 3;
         __syncwarp();
         if (lane < kRunBlocks) nonzero[warp][lane] = 0;
 #pragma unroll
         for (int i = 0; i < kPieces; ++i) {
+            if (i >= n_pieces) break;
             uint32_t lo[3], hi[3];
-            word_digits(in[i].x, lo);
-            word_digits(in[i].y, hi);
+            word_digits(in[i].x, table + lane, lo);
+            word_digits(in[i].y, table + lane, hi);
             uint32_t w[6] = {lo[0], lo[1], lo[2], hi[0], hi[1], hi[2]};
-            const int64_t e0 = (int64_t)run * kRun + 768 * i + lane * 24;
+            const int64_t e0 = block0 * kBlock + 768 * i + lane * 24;
             if (e0 + 24 > cols) clear_past<6>(w, cols - e0);
 #pragma unroll
-            for (int j = 0; j < 3; ++j) *reinterpret_cast<uint2 *>(q + i * 192 + lane * 6 + 2 * j) = make_uint2(w[2 * j], w[2 * j + 1]);
+            for (int j = 0; j < 3; ++j) *reinterpret_cast<uint2 *>(q + digit_place(i * 192 + lane * 6 + 2 * j)) = make_uint2(w[2 * j], w[2 * j + 1]);
         }
         __syncwarp();
-        const int64_t left = blocks_per_row - (int64_t)run * kRunBlocks;
-        const int n_blocks = (int)(left < kRunBlocks ? left : kRunBlocks);
-        for (int item = lane; item < n_blocks * kWords; item += 32) {
-            const int b = item / kWords, k = item - b * kWords;
-            int first, pitch;
-            digit_words<FORMAT>(k, first, pitch);
-            const uint32_t *blk = q + b * 64 + first;
+#pragma unroll
+        for (int i = 0; i < kPasses; ++i) {
+            if (lane + 32 * i >= n_blocks * kWords) break;
+            const uint32_t *blk = q + from[i];
             uint32_t v = 0, differs = 0;
             if constexpr (FORMAT == T81B200_TQ2_0) {
 #pragma unroll
                 for (int m = 0; m < 4; ++m) {
-                    const uint32_t x = blk[m * pitch];
+                    const uint32_t x = blk[m * 8];
                     differs |= x ^ 0x01010101u;
                     v |= x << (2 * m);
                 }
             } else {
+                const bool last = pitch[i] == 1;  // four digits and a zero one
                 uint32_t n = 0;  // base-3 numbers 0..242, byte by byte
 #pragma unroll
-                for (int m = 0; m < 5; ++m) {
-                    const bool there = m < 4 || k < 12;
-                    const uint32_t x = there ? blk[m * pitch] : 0u;
-                    differs |= there ? x ^ 0x01010101u : 0u;
+                for (int m = 0; m < 4; ++m) {
+                    const uint32_t x = blk[m * pitch[i]];
+                    differs |= x ^ 0x01010101u;
                     n = 3u * n + x;
                 }
-                // ceil(256 n / 243), exact for all 243 values
+                const uint32_t x = last ? 0x01010101u : blk[4 * pitch[i]];
+                differs |= x ^ 0x01010101u;
+                n = 3u * n + (last ? 0u : x);
+                // ceil(256 n / 243) = (69045 n + 65000) >> 16, exact for all 243 values: byte 2 of each product
+                uint32_t y[4];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) v |= ((((n >> (8 * j)) & 0xFFu) * 8631u + 8100u) >> 13) << (8 * j);
+                for (int j = 0; j < 4; ++j) y[j] = __byte_perm(n, 0u, 0x4440 | j) * 69045u + 65000u;
+                v = __byte_perm(__byte_perm(y[0], y[1], 0x0062), __byte_perm(y[2], y[3], 0x0062), 0x5410);
             }
-            if (differs) nonzero[warp][b] = 1;
-            uint16_t *dst = reinterpret_cast<uint16_t *>(staged[warp] + b * kBytes) + k * 2;
+            if (differs) nonzero[warp][block[i]] = 1;
+            uint16_t *dst = reinterpret_cast<uint16_t *>(staged[warp]) + to[i];
             dst[0] = (uint16_t)v;
             dst[1] = (uint16_t)(v >> 16);
         }
@@ -169,10 +201,12 @@ __global__ void __launch_bounds__(kWarps * 32) packed_to_tq_kernel(const uint8_t
             *reinterpret_cast<uint16_t *>(staged[warp] + lane * kBytes + kBytes - 2) = __half_as_ushort(__float2half_rn(d));
         }
         __syncwarp();
-        uint8_t *out = blocks + (row * blocks_per_row + (int64_t)run * kRunBlocks) * kBytes;
-        if (wide)
-            for (int i = lane; i < n_blocks * kBytes / 2; i += 32) reinterpret_cast<uint16_t *>(out)[i] = reinterpret_cast<const uint16_t *>(staged[warp])[i];
-        else
+        uint8_t *out = blocks + (row * blocks_per_row + block0) * kBytes;
+        if (wide) {
+#pragma unroll
+            for (int i = 0; i < (kHalves + 31) / 32; ++i)
+                if (lane + 32 * i < n_blocks * kBytes / 2) reinterpret_cast<uint16_t *>(out)[lane + 32 * i] = reinterpret_cast<const uint16_t *>(staged[warp])[lane + 32 * i];
+        } else
             for (int i = lane; i < n_blocks * kBytes; i += 32) out[i] = staged[warp][i];
     }
 }
@@ -180,19 +214,33 @@ __global__ void __launch_bounds__(kWarps * 32) packed_to_tq_kernel(const uint8_t
 template <int FORMAT>
 __global__ void __launch_bounds__(kWarps * 32) tq_to_packed_kernel(const uint8_t *__restrict__ blocks, int64_t rows, int64_t cols, int64_t row_bytes,
                                                                    uint8_t *__restrict__ packed, float *__restrict__ block_scale, int64_t blocks_per_row,
-                                                                   int runs_per_row, bool wide) {
-    constexpr int kBytes = block_bytes(FORMAT), kWords = FORMAT == T81B200_TQ2_0 ? 16 : 13, kHalves = kRunBlocks * kBytes / 2, kLoads = (kHalves + 31) / 32;
-    __shared__ __align__(16) uint32_t digits[kWarps][kRun / 4];
-    __shared__ __align__(16) uint8_t staged[kWarps][kRunBlocks * 66];
+                                                                   int runs_per_row, int run_blocks, bool wide) {
+    constexpr int kBytes = block_bytes(FORMAT), kWords = FORMAT == T81B200_TQ2_0 ? 16 : 13, kHalves = kRunBlocks * kBytes / 2;
+    constexpr int kPasses = (kRunBlocks * kWords + 31) / 32, kLoads = (kHalves + 31) / 32;
+    __shared__ __align__(16) uint32_t digits[kWarps][kDigitWords];
+    __shared__ __align__(16) uint8_t staged[kWarps][kRunBlocks * 66 + 2];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t *q = digits[warp];
-    const int64_t total = rows * runs_per_row;
-    for (int64_t at = (int64_t)blockIdx.x * kWarps + warp; at < total; at += (int64_t)gridDim.x * kWarps) {
-        const int64_t row = total < (1ll << 32) ? (int64_t)((uint32_t)at / (uint32_t)runs_per_row) : at / runs_per_row;
-        const int run = (int)(at - row * runs_per_row);
-        const int64_t left = blocks_per_row - (int64_t)run * kRunBlocks;
-        const int n_blocks = (int)(left < kRunBlocks ? left : kRunBlocks);
-        const uint8_t *in = blocks + (row * blocks_per_row + (int64_t)run * kRunBlocks) * kBytes;
+    int to[kPasses], pitch[kPasses], from[kPasses];
+#pragma unroll
+    for (int i = 0; i < kPasses; ++i) {
+        const int item = lane + 32 * i, b = item / kWords, k = item - b * kWords;
+        digit_words<FORMAT>(k, to[i], pitch[i]);
+        to[i] += b * kBlockPitch;
+        from[i] = b * (kBytes / 2) + 2 * k;
+    }
+    const int64_t total = rows * runs_per_row, stride = (int64_t)gridDim.x * kWarps;
+    auto locate = [&](int64_t at, int64_t &row, int64_t &block0, int &n_blocks) {
+        row = total < (1ll << 32) ? (int64_t)((uint32_t)at / (uint32_t)runs_per_row) : at / runs_per_row;
+        block0 = (at - row * runs_per_row) * run_blocks;
+        const int64_t left = blocks_per_row - block0;
+        n_blocks = (int)(left < run_blocks ? left : run_blocks);
+    };
+    for (int64_t at = (int64_t)blockIdx.x * kWarps + warp; at < total; at += stride) {
+        int64_t row, block0;
+        int n_blocks;
+        locate(at, row, block0, n_blocks);
+        const uint8_t *in = blocks + (row * blocks_per_row + block0) * kBytes;
         __syncwarp();
         if (wide) {
             uint16_t h[kLoads];
@@ -204,18 +252,17 @@ __global__ void __launch_bounds__(kWarps * 32) tq_to_packed_kernel(const uint8_t
         } else
             for (int i = lane; i < n_blocks * kBytes; i += 32) staged[warp][i] = in[i];
         __syncwarp();
-        for (int item = lane; item < n_blocks * kWords; item += 32) {
-            const int b = item / kWords, k = item - b * kWords;
-            const uint16_t *src = reinterpret_cast<const uint16_t *>(staged[warp] + b * kBytes) + 2 * k;
+#pragma unroll
+        for (int i = 0; i < kPasses; ++i) {
+            if (lane + 32 * i >= n_blocks * kWords) break;
+            const uint16_t *src = reinterpret_cast<const uint16_t *>(staged[warp]) + from[i];
             const uint32_t x = (uint32_t)src[0] | ((uint32_t)src[1] << 16);
-            int first, pitch;
-            digit_words<FORMAT>(k, first, pitch);
-            uint32_t *blk = q + b * 64 + first;
+            uint32_t *blk = q + to[i];
             if constexpr (FORMAT == T81B200_TQ2_0) {
 #pragma unroll
                 for (int m = 0; m < 4; ++m) {
                     const uint32_t d = (x >> (2 * m)) & 0x03030303u;
-                    blk[m * pitch] = d - (d & (d >> 1) & 0x01010101u);  // 3 reads as 2
+                    blk[m * 8] = d - (d & (d >> 1) & 0x01010101u);  // 3 reads as 2
                 }
             } else {
                 // digit m of a byte is the top of byte * 3^m (mod 256) * 3 (t81/gguf.py:629-637)
@@ -224,7 +271,7 @@ __global__ void __launch_bounds__(kWarps * 32) tq_to_packed_kernel(const uint8_t
                 for (int m = 0; m < 5; ++m) {
                     even *= 3u;
                     odd *= 3u;
-                    if (m < 4 || k < 12) blk[m * pitch] = ((even >> 8) & 0x00FF00FFu) | (odd & 0xFF00FF00u);
+                    if (m < 4 || pitch[i] != 1) blk[m * pitch[i]] = __byte_perm(even, odd, 0x7351);
                     even &= 0x00FF00FFu;
                     odd &= 0x00FF00FFu;
                 }
@@ -233,12 +280,12 @@ __global__ void __launch_bounds__(kWarps * 32) tq_to_packed_kernel(const uint8_t
         __syncwarp();
 #pragma unroll
         for (int i = 0; i < kPieces; ++i) {
-            const int64_t byte0 = (int64_t)run * (kRun / 3) + 256 * i + lane * 8, e0 = (int64_t)run * kRun + 768 * i + lane * 24;
-            if (byte0 >= row_bytes) break;
+            const int64_t byte0 = block0 * kBlock / 3 + 256 * i + lane * 8, e0 = block0 * kBlock + 768 * i + lane * 24;
+            if (3 * i >= n_blocks || byte0 >= row_bytes) break;
             uint32_t w[6];
 #pragma unroll
             for (int j = 0; j < 3; ++j) {
-                const uint2 d = *reinterpret_cast<const uint2 *>(q + i * 192 + lane * 6 + 2 * j);
+                const uint2 d = *reinterpret_cast<const uint2 *>(q + digit_place(i * 192 + lane * 6 + 2 * j));
                 w[2 * j] = d.x;
                 w[2 * j + 1] = d.y;
             }
@@ -250,12 +297,12 @@ __global__ void __launch_bounds__(kWarps * 32) tq_to_packed_kernel(const uint8_t
                 for (int j = 0; j < 4; ++j) { dst[j] = (uint8_t)(t0 >> (8 * j)); dst[4 + j] = (uint8_t)(t1 >> (8 * j)); }
         }
         if (block_scale && lane < n_blocks)
-            block_scale[row * blocks_per_row + (int64_t)run * kRunBlocks + lane] =
+            block_scale[row * blocks_per_row + block0 + lane] =
                 __half2float(__ushort_as_half(*reinterpret_cast<const uint16_t *>(staged[warp] + lane * kBytes + kBytes - 2)));
     }
 }
 
-// A warp per run, up to about what is resident at a time.
+// A few runs a warp: the tables are made once per CTA.
 unsigned tq_grid(int64_t runs) {
     const int64_t ctas = (runs + kWarps - 1) / kWarps, most = (int64_t)sm_count() * 12;
     return (unsigned)(ctas < most ? ctas : most);
@@ -281,12 +328,14 @@ extern "C" int t81b200_packed_to_tq(const uint8_t *packed, const float *row_scal
     const int64_t bpr = (cols + kBlock - 1) / kBlock, row_bytes = (cols + 47) / 48 * 16;
     if (bpr > 65535 || rows >= (1ll << 31)) return fail(T81B200_ELIMIT, "tq: matrix too large for one call");
     const bool wide = reinterpret_cast<uintptr_t>(packed) % 8 == 0 && reinterpret_cast<uintptr_t>(blocks) % 2 == 0;
-    const int64_t runs = (bpr + kRunBlocks - 1) / kRunBlocks;
+    const int64_t runs0 = (bpr + kRunBlocks - 1) / kRunBlocks;
+    const int run_blocks = (int)(((bpr + runs0 - 1) / runs0 + 2) / 3 * 3);
+    const int64_t runs = (bpr + run_blocks - 1) / run_blocks;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (format == T81B200_TQ2_0)
-        packed_to_tq_kernel<T81B200_TQ2_0><<<tq_grid(rows * runs), kWarps * 32, 0, st>>>(packed, row_scale, rows, cols, row_bytes, blocks, bpr, (int)runs, wide);
+        packed_to_tq_kernel<T81B200_TQ2_0><<<tq_grid(rows * runs), kWarps * 32, 0, st>>>(packed, row_scale, rows, cols, row_bytes, blocks, bpr, (int)runs, run_blocks, wide);
     else
-        packed_to_tq_kernel<T81B200_TQ1_0><<<tq_grid(rows * runs), kWarps * 32, 0, st>>>(packed, row_scale, rows, cols, row_bytes, blocks, bpr, (int)runs, wide);
+        packed_to_tq_kernel<T81B200_TQ1_0><<<tq_grid(rows * runs), kWarps * 32, 0, st>>>(packed, row_scale, rows, cols, row_bytes, blocks, bpr, (int)runs, run_blocks, wide);
     T81_LAUNCH_CHECK("packed_to_tq_kernel");
     return T81B200_OK;
 }
@@ -301,12 +350,14 @@ extern "C" int t81b200_tq_to_packed(const uint8_t *blocks, int64_t rows, int64_t
     const int64_t bpr = (cols + kBlock - 1) / kBlock, row_bytes = (cols + 47) / 48 * 16;
     if (bpr > 65535 || rows >= (1ll << 31)) return fail(T81B200_ELIMIT, "tq: matrix too large for one call");
     const bool wide = reinterpret_cast<uintptr_t>(packed) % 8 == 0 && reinterpret_cast<uintptr_t>(blocks) % 2 == 0;
-    const int64_t runs = (bpr + kRunBlocks - 1) / kRunBlocks;
+    const int64_t runs0 = (bpr + kRunBlocks - 1) / kRunBlocks;
+    const int run_blocks = (int)(((bpr + runs0 - 1) / runs0 + 2) / 3 * 3);
+    const int64_t runs = (bpr + run_blocks - 1) / run_blocks;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (format == T81B200_TQ2_0)
-        tq_to_packed_kernel<T81B200_TQ2_0><<<tq_grid(rows * runs), kWarps * 32, 0, st>>>(blocks, rows, cols, row_bytes, packed, block_scale, bpr, (int)runs, wide);
+        tq_to_packed_kernel<T81B200_TQ2_0><<<tq_grid(rows * runs), kWarps * 32, 0, st>>>(blocks, rows, cols, row_bytes, packed, block_scale, bpr, (int)runs, run_blocks, wide);
     else
-        tq_to_packed_kernel<T81B200_TQ1_0><<<tq_grid(rows * runs), kWarps * 32, 0, st>>>(blocks, rows, cols, row_bytes, packed, block_scale, bpr, (int)runs, wide);
+        tq_to_packed_kernel<T81B200_TQ1_0><<<tq_grid(rows * runs), kWarps * 32, 0, st>>>(blocks, rows, cols, row_bytes, packed, block_scale, bpr, (int)runs, run_blocks, wide);
     T81_LAUNCH_CHECK("tq_to_packed_kernel");
     return T81B200_OK;
 }
