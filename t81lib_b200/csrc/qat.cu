@@ -106,22 +106,9 @@ __global__ void __launch_bounds__(256) qat_quantize_pack_kernel(const T *__restr
     }
 }
 
-// Quantise straight into the decode-stream layout of the weight (forward product) and of its transpose (input
-// gradient), in one pass over the weight.  A CTA takes 96 rows x 192 columns: three blocks of the weight's layout and half of six
-// of the transpose's.  Warp w owns columns 32 w .. + 31, a lane one column, and walks the 96 rows (whole 128-byte
-// reads, eight rows ahead of use: with nothing in flight while eight rows are packed the pass took 90 us):
-//   transpose: the lane's column is a row of it; eight rows in turn fill one half of a word (two bits each, at the
-//              places the layout wants), the lane eight columns on supplies the other half;
-//   weight:    two ballots per row hold 32 columns of it; lane r keeps those of row r of a 32-row tile and spreads its
-//              four bytes of each to word positions with a table.
-// Blocks are put together in shared memory and leave as contiguous runs (4.5 KB, and 96 bytes of the transpose).  The rows
-// are taken last first: the scale's reduction has just read the weight front to back, and its end is still in L2.
-__device__ __forceinline__ uint32_t spread_place(int c) { return (c & 1 ? 30u : 14u) - 4u * (uint32_t)(c >> 1); }  // of column c of eight, first row of the pair
-
 // The rule compares w / scale, rounded, with the threshold, and keeps zeros (t81/qat.py:12-25).  Rounded division is
 // monotonic, so that is a comparison of |w| with the smallest value whose quotient reaches the threshold and is not
-// zero: bisected over the floats' bit patterns, from within four ulp of thr * scale where that brackets it.  (A division
-// per weight in the unrolled loop below would not fit the instruction cache: 33 us for 4096 x 4096 instead of 14.)
+// zero: bisected over the floats' bit patterns, from within four ulp of thr * scale where that brackets it.  
 __device__ float quotient_cut(float thr, float scale) {
     auto reaches = [&](uint32_t bits) {
         const float q = __fdiv_rn(__uint_as_float(bits), scale);
@@ -138,75 +125,110 @@ __device__ float quotient_cut(float thr, float scale) {
     return __uint_as_float(hi);
 }
 
+// Quantise straight into the decode-stream layout of the weight (forward product) and of its transpose (input
+// gradient), in one pass over the weight.  A CTA takes 96 rows x 384 columns: six blocks of the weight's layout and half
+// of twelve of the transpose's.  A warp takes 16 rows x 128 columns at a time, a lane four columns: whole 512-byte row
+// pieces, 16 loads in flight per lane.
+//   A trit y = -1, 0, +1 is a compare and a sign; its code in the layout is the 2-bit two's complement of y.  Fields that
+//   hold y + 2 do not borrow from each other, and (y + 2) ^ 2 is that code: so a lane's share of a word is a float sum of
+//   y * 4^place (eight fields in two bytes 16 bits apart: exact), turned to an integer, plus 0xAA in each byte, exclusive-or
+//   the same.  Four instructions a weight for both layouts.
+//   A word of the weight's layout is 8 columns of 2 rows (g, g + 8): two neighbouring lanes' shares; a word of the
+//   transpose's is 8 rows of 2 columns (c, c + 8): those of two lanes 2 apart.  Each pair of lanes exchanges half its shares
+//   and finishes the other half.
+// Blocks are put together in shared memory and leave as contiguous runs.  The rows are taken last first: the scale's
+// reduction has just read the weight front to back, and its end is still in L2.  14336 x 4096: 110 us with two ballots and
+// ten bit operations a weight (issue-bound), 51 us this way, 39 behind that reduction; 264 MB cross memory (41 us).
+template <bool VEC>
 __global__ void __launch_bounds__(192) qat_quantize_t2_kernel(const float *__restrict__ w, int64_t rows, int64_t cols, int64_t ld, float thr,
                                                               const float *__restrict__ scale_ptr, uint8_t *__restrict__ t2,
                                                               uint8_t *__restrict__ t2_t, float *__restrict__ scale_out, int64_t n_scales) {
-    __shared__ uint32_t spread[256];
-    __shared__ __align__(16) uint32_t fwd[3 * 384], trn[6 * 192];
+    __shared__ __align__(16) uint32_t fwd[6 * 384], trn[12 * 192];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const float scale = *scale_ptr;
     for (int64_t i = ((int64_t)blockIdx.y * gridDim.x + blockIdx.x) * 192 + tid; i < n_scales; i += (int64_t)gridDim.x * gridDim.y * 192) scale_out[i] = scale;
-    for (int b = tid; b < 256; b += 192) {
-        uint32_t v = 0;
-        for (int c = 0; c < 8; ++c) v |= (uint32_t)((b >> c) & 1) << spread_place(c);
-        spread[b] = v;
-    }
     const float cut = quotient_cut(thr, scale);
-    __syncthreads();
-    const int64_t rb = gridDim.y - 1 - blockIdx.y, row0 = rb * 96, col = (int64_t)blockIdx.x * 192 + 32 * warp + lane;
-    const bool col_ok = col < cols;
+    const int64_t rb = gridDim.y - 1 - blockIdx.y, row0 = rb * 96, col0 = (int64_t)blockIdx.x * 384;
+    const int wx = warp % 3, col8 = wx * 16 + (lane >> 1);  // this lane's group of eight columns in the CTA's 48
+    const int64_t col = col0 + wx * 128 + lane * 4;
     const float *src = w + row0 * ld + col;
-    const int gr = lane >> 4, g = lane & 7;
-    auto load8 = [&](int first, float (&v)[8]) {
+    // word q of the weight's layout goes to fwd_at + q * 48 (its row pair) + tile; half of the row pairs each
+    const int odd = lane & 1, upper = (lane >> 1) & 1;
+    const int fwd_at = (col8 / 24) * (3 * 384) + (col8 % 24 / 6) * 12 + col8 % 6 + odd * (4 * 48);
+    const int trn_at = (wx * 4 + (lane >> 3)) * 192 + (8 * odd) * 12 + ((lane >> 2) & 1) * 6;
+    for (int rs = warp / 3; rs < 6; rs += 2) {
+        float4 v[16];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] = col_ok && first < 96 && row0 + first + i < rows ? __ldg(src + (int64_t)(first + i) * ld) : 0.0f;
-    };
-    float v[8];
-    load8(0, v);
-    uint32_t my_nz = 0, my_neg = 0;
-#pragma unroll 4
-    for (int og = 0; og < 12; ++og) {  // groups of eight rows of the weight = eight columns of the transpose
-        float ahead[8];
-        load8(8 * og + 8, ahead);
-        uint32_t half = 0;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const bool nz = fabsf(v[i]) >= cut;
-            const bool neg = nz && v[i] < 0.0f;
-            const uint32_t nz_mask = __ballot_sync(0xffffffffu, nz), neg_mask = __ballot_sync(0xffffffffu, neg);
-            if (lane == 8 * (og & 3) + i) { my_nz = nz_mask; my_neg = neg_mask; }
-            half |= ((neg ? 2u : 0u) | (nz ? 1u : 0u)) << spread_place(i);
-        }
-        if (t2_t) {
-            // word 6 gr + og % 6 of lane 4 g + t, t = 2 * (rb % 2) + og / 6: two of a block's four runs are this CTA's
-            const uint32_t word = half | (__shfl_down_sync(0xffffffffu, half, 8) >> 2);
-            if (!(lane & 8)) trn[warp * 192 + (2 * g + og / 6) * 12 + 6 * gr + og % 6] = word;
-        }
-        if ((og & 3) == 3) {
-#pragma unroll
-            for (int b = 0; b < 4; ++b) {
-                const uint32_t h = spread[(my_nz >> (8 * b)) & 0xFFu] | (spread[(my_neg >> (8 * b)) & 0xFFu] << 1);
-                const uint32_t word = h | (__shfl_down_sync(0xffffffffu, h, 8) >> 2);
-                const int kg = 4 * warp + b;
-                if (!(lane & 8)) fwd[(og >> 2) * 384 + (4 * g + kg / 6) * 12 + 6 * gr + kg % 6] = word;
+        for (int r = 0; r < 16; ++r) {
+            const float *p = src + (int64_t)(16 * rs + r) * ld;
+            v[r] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (row0 + 16 * rs + r < rows) {
+                if constexpr (VEC) {
+                    if (col < cols) v[r] = __ldg(reinterpret_cast<const float4 *>(p));
+                } else {
+                    if (col < cols) v[r].x = __ldg(p);
+                    if (col + 1 < cols) v[r].y = __ldg(p + 1);
+                    if (col + 2 < cols) v[r].z = __ldg(p + 2);
+                    if (col + 3 < cols) v[r].w = __ldg(p + 3);
+                }
             }
         }
+        float fs[8], ts[4][4];  // shares: row pairs; columns x groups of four rows
 #pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] = ahead[i];
+        for (int i = 0; i < 8; ++i) fs[i] = 0.0f;
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) ts[c][i] = 0.0f;
+#pragma unroll
+        for (int r = 0; r < 16; ++r) {
+            const float e[4] = {v[r].x, v[r].y, v[r].z, v[r].w};
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const float nz = fabsf(e[c]) >= cut ? 1.0f : 0.0f;
+                const float y = __uint_as_float(__float_as_uint(nz) | (__float_as_uint(e[c]) & 0x80000000u));
+                // fields of four: the first two of a parity at bits 6 and 2, odd ones 16 higher; the second of a pair 2 lower
+                fs[r & 7] = fmaf(y, (float)(1 << ((c & 1 ? 22 : 6) - 4 * (c >> 1) - (r >> 3 ? 2 : 0))), fs[r & 7]);
+                ts[c][r >> 2] = fmaf(y, (float)(1 << ((r & 1 ? 22 : 6) - 4 * ((r & 3) >> 1))), ts[c][r >> 2]);
+            }
+        }
+        // every place taken (0xAA per byte), and every other one (0x88)
+        auto part = [](float sum) { return (uint32_t)((int)sum + 0x00880088) ^ 0x00880088u; };
+        auto codes = [](float sum) { return (uint32_t)((int)sum + 0x00AA00AA) ^ 0x00AA00AAu; };
+        uint32_t *out = fwd + fwd_at + (rs >> 1) * 384 + 6 * (rs & 1);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint32_t a = codes(fs[i]), b = codes(fs[4 + i]);
+            const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? a : b, 1);
+            out[i * 48] = odd ? (got << 8) | b : (a << 8) | got;
+        }
+        if (t2_t) {
+            // fields 2 bits apart are this column's; the column 8 on takes the places between them
+            const int group = 2 * rs + upper;  // eight rows: 0 .. 11
+            uint32_t *to = trn + trn_at + (group / 6) * 12 + group % 6;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const uint32_t a = (part(ts[c][0]) << 8) | part(ts[c][1]), b = (part(ts[c][2]) << 8) | part(ts[c][3]);
+                const uint32_t got = __shfl_xor_sync(0xffffffffu, upper ? a : b, 2);
+                to[c * 24] = upper ? got | (b >> 2) : a | (got >> 2);
+            }
+        }
     }
     __syncthreads();
-    // block (chunk, row tile) of the weight: chunk = blockIdx.x, row tiles 3 rb ..; of the transpose: chunk rb / 2, row tiles 6 blockIdx.x ..
-    const int64_t tiles = (rows + 31) / 32, tiles_t = (cols + 31) / 32;
-    {
+    // block (chunk, row tile) of the weight: chunks 2 blockIdx.x, + 1, row tiles 3 rb ..; of the transpose: chunk rb / 2, row tiles 12 blockIdx.x ..
+    const int64_t tiles = (rows + 31) / 32, tiles_t = (cols + 31) / 32, chunks = (cols + 191) / 192;
+    for (int ch = 0; ch < 2; ++ch) {
+        const int64_t chunk = (int64_t)blockIdx.x * 2 + ch;
+        if (chunk >= chunks) break;
         const int64_t left = tiles - rb * 3;
         const int n = (int)(left < 3 ? left : 3) * 96;
-        uint4 *dst = reinterpret_cast<uint4 *>(t2 + ((int64_t)blockIdx.x * tiles + rb * 3) * 1536);
-        for (int i = tid; i < n; i += 192) dst[i] = reinterpret_cast<const uint4 *>(fwd)[i];
+        uint4 *dst = reinterpret_cast<uint4 *>(t2 + (chunk * tiles + rb * 3) * 1536);
+        for (int i = tid; i < n; i += 192) dst[i] = reinterpret_cast<const uint4 *>(fwd + ch * 1152)[i];
     }
     if (t2_t) {
-        const int64_t left = tiles_t - (int64_t)blockIdx.x * 6;
-        const int n = (int)(left < 6 ? left : 6) * 48;  // per block: 8 runs of 6 pieces
-        uint8_t *out = t2_t + ((rb >> 1) * tiles_t + (int64_t)blockIdx.x * 6) * 1536 + (rb & 1) * 96;
+        const int64_t left = tiles_t - (int64_t)blockIdx.x * 12;
+        const int n = (int)(left < 12 ? left : 12) * 48;  // per block: 8 runs of 6 pieces
+        uint8_t *out = t2_t + ((rb >> 1) * tiles_t + (int64_t)blockIdx.x * 12) * 1536 + (rb & 1) * 96;
         for (int i = tid; i < n; i += 192) *reinterpret_cast<uint4 *>(out + i / 6 * 192 + i % 6 * 16) = reinterpret_cast<const uint4 *>(trn)[i];
         // an odd number of 96-row parts: the last chunk's other half is past the matrix
         if (rb == gridDim.y - 1 && !(rb & 1))
@@ -311,9 +333,13 @@ extern "C" int t81b200_qat_quantize_t2(const float *w, int64_t rows, int64_t col
     if (!w || !scale || !t2 || (n_scales > 0 && !scale_out)) return fail(T81B200_EINVAL, "qat_quantize_t2: null pointer");
     if (reinterpret_cast<uintptr_t>(t2) % 16 != 0 || reinterpret_cast<uintptr_t>(t2_transposed) % 16 != 0)
         return fail(T81B200_EALIGN, "qat_quantize_t2: the outputs must be 16-byte aligned");
-    const dim3 grid((unsigned)((cols + 191) / 192), (unsigned)((rows + 95) / 96));
+    const dim3 grid((unsigned)((cols + 383) / 384), (unsigned)((rows + 95) / 96));
     if (cols > (1ll << 31) || grid.y > 65535u) return fail(T81B200_ELIMIT, "qat_quantize_t2: matrix too large for one call");
-    qat_quantize_t2_kernel<<<grid, 192, 0, static_cast<cudaStream_t>(stream)>>>(w, rows, cols, ld, threshold, scale, t2, t2_transposed, scale_out, n_scales);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (reinterpret_cast<uintptr_t>(w) % 16 == 0 && ld % 4 == 0 && cols % 4 == 0)
+        qat_quantize_t2_kernel<true><<<grid, 192, 0, st>>>(w, rows, cols, ld, threshold, scale, t2, t2_transposed, scale_out, n_scales);
+    else
+        qat_quantize_t2_kernel<false><<<grid, 192, 0, st>>>(w, rows, cols, ld, threshold, scale, t2, t2_transposed, scale_out, n_scales);
     T81_LAUNCH_CHECK("qat_quantize_t2_kernel");
     return T81B200_OK;
 }
