@@ -52,7 +52,7 @@ enum {
     T81B200_ELIMIT = -6      /* size beyond a stated fixed maximum               */
 };
 
-enum { T81B200_F32 = 0, T81B200_BF16 = 1, T81B200_F16 = 2 };
+enum { T81B200_F32 = 0, T81B200_BF16 = 1, T81B200_F16 = 2, T81B200_BF16X3 = 3 /* see stage_rows */ };
 
 /* Quantiser rule. FIXED is the reference rule (python/bindings.cpp:405-414,
  * t81/torch/__init__.py:44-50).  ABSMEAN compares each weight with threshold times
@@ -365,18 +365,24 @@ T81B200_API int t81b200_qat_quantize_pack(const void *w, int w_dtype, int64_t ro
 /* Training step on the decode-stream layout.  qat_quantize_t2: the same quantiser (fp32 weight) writing the layout of the
  * weight and, unless null, of its transpose (what the input gradient multiplies with); scale_out receives n_scales
  * copies of the scale (the row scales of either product).  qat_weight_grad: out (rows, cols) fp32, contiguous, =
- * slope * g^T x for token-major g (tokens, rows) and x (tokens, cols) of one dtype, slope = 2 where |w / scale| < 0.5 and
+ * slope * g^T x for token-major g (tokens, rows) and x (tokens, cols) of one dtype (or fp32 and BF16X3), slope = 2 where |w / scale| < 0.5 and
  * 0 elsewhere (t81/nn/linear.py:72-80 through t81/qat.py:28-57); 16-bit operands are multiplied exactly, fp32 ones in
  * three bf16 planes; operands that TMA cannot read where they are need the workspace (256-byte aligned).
  * column_sums: fp32 sums over the tokens of a token-major matrix (the bias gradient). */
 T81B200_API int t81b200_column_sums(const void *g, int dtype, int64_t tokens, int64_t cols, int64_t ld, float *out, void *stream);
 T81B200_API int t81b200_qat_quantize_t2(const float *w, int64_t rows, int64_t cols, int64_t ld, float threshold, const float *scale, uint8_t *t2,
                                         uint8_t *t2_transposed, float *scale_out, int64_t n_scales, void *stream);
-T81B200_API size_t t81b200_qat_weight_grad_workspace_bytes(const void *g, int64_t ldg, const void *x, int64_t ldx, int dtype, int64_t tokens,
-                                                           int64_t rows, int64_t cols);
-T81B200_API int t81b200_qat_weight_grad(const void *g, int64_t ldg, const void *x, int64_t ldx, int dtype, int64_t tokens, int64_t rows, int64_t cols,
-                                        const float *w, int64_t ldw, const float *scale, float *out, void *workspace, size_t workspace_bytes,
-                                        void *stream);
+T81B200_API size_t t81b200_qat_weight_grad_workspace_bytes(const void *g, int g_dtype, int64_t ldg, const void *x, int x_dtype, int64_t ldx,
+                                                           int64_t tokens, int64_t rows, int64_t cols);
+T81B200_API int t81b200_qat_weight_grad(const void *g, int g_dtype, int64_t ldg, const void *x, int x_dtype, int64_t ldx, int64_t tokens, int64_t rows,
+                                        int64_t cols, const float *w, int64_t ldw, const float *scale, float *out, void *workspace,
+                                        size_t workspace_bytes, void *stream);
+/* Activation rows that TMA cannot read in place, staged once for several products: fp32 becomes three bf16 planes
+ * (T81B200_BF16X3: (3, tokens, stage_rows_ld(width)) bf16, plane 0 + 1 + 2 = the value, all 24 mantissa bits), a 16-bit type
+ * keeps its type.  linear_t2 and qat_weight_grad take BF16X3 operands. */
+T81B200_API int64_t t81b200_stage_rows_ld(int64_t width);
+T81B200_API size_t t81b200_stage_rows_bytes(int dtype, int64_t tokens, int64_t width);
+T81B200_API int t81b200_stage_rows(const void *src, int dtype, int64_t ld, int64_t tokens, int64_t width, void *out, void *stream);
 
 /* Transcoders between the packed-limb layout and the GGUF ternary block formats the reference writes and reads
  * on the CPU through float arrays (t81/gguf.py:518-662: _quantize_blocks_tq1 / _tq2, _dequantize_blocks_tq1 / _tq2;

@@ -13,7 +13,7 @@ _PKG = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_PKG, "lib", "libt81_b200.so")
 
 OK, EINVAL, ENODEVICE, ECUDA, EWORKSPACE, EALIGN, ELIMIT = 0, -1, -2, -3, -4, -5, -6
-F32, BF16, F16 = 0, 1, 2
+F32, BF16, F16, BF16X3 = 0, 1, 2, 3
 RULE_FIXED, RULE_ABSMEAN = 0, 1
 LAYOUT_KN, LAYOUT_NK = 0, 1
 STATIC_SCRATCH_BYTES = 16 << 20
@@ -29,6 +29,7 @@ EXPORTS = (
     "t81b200_gemm_limb_auto", "t81b200_gemm_trit_auto", "t81b200_elementwise", "t81b200_elementwise_auto",
     "t81b200_release_staging", "t81b200_exchange_signal", "t81b200_gemm_trit_grouped", "t81b200_t2_bytes", "t81b200_pack_t2", "t81b200_prefers_streaming", "t81b200_gemm_trit_t2", "t81b200_gemm_trit_t2_peers", "t81b200_linear_t2_workspace_bytes", "t81b200_linear_t2", "t81b200_tq_bytes", "t81b200_packed_to_tq", "t81b200_tq_to_packed",
     "t81b200_qat_update_scale", "t81b200_qat_quantize_pack", "t81b200_qat_quantize_t2", "t81b200_qat_weight_grad_workspace_bytes", "t81b200_qat_weight_grad", "t81b200_column_sums",
+    "t81b200_stage_rows_ld", "t81b200_stage_rows_bytes", "t81b200_stage_rows",
 )
 TQ1_0, TQ2_0 = 0, 1
 T2_MAX_TOKENS = 128  # T81B200_T2_MAX_ROWS
@@ -83,9 +84,14 @@ def _load() -> ctypes.CDLL:
     lib.t81b200_qat_update_scale.argtypes = [vp, ci, i64, i64, i64, f32, vp, vp]
     lib.t81b200_qat_quantize_pack.argtypes = [vp, ci, i64, i64, i64, f32, vp, vp, vp, vp]
     lib.t81b200_qat_quantize_t2.argtypes = [vp, i64, i64, i64, f32, vp, vp, vp, vp, i64, vp]
-    lib.t81b200_qat_weight_grad_workspace_bytes.argtypes = [vp, i64, vp, i64, ci, i64, i64, i64]
+    lib.t81b200_qat_weight_grad_workspace_bytes.argtypes = [vp, ci, i64, vp, ci, i64, i64, i64, i64]
     lib.t81b200_qat_weight_grad_workspace_bytes.restype = ctypes.c_size_t
-    lib.t81b200_qat_weight_grad.argtypes = [vp, i64, vp, i64, ci, i64, i64, i64, vp, i64, vp, vp, vp, ctypes.c_size_t, vp]
+    lib.t81b200_qat_weight_grad.argtypes = [vp, ci, i64, vp, ci, i64, i64, i64, i64, vp, i64, vp, vp, vp, ctypes.c_size_t, vp]
+    lib.t81b200_stage_rows_ld.argtypes = [i64]
+    lib.t81b200_stage_rows_ld.restype = i64
+    lib.t81b200_stage_rows_bytes.argtypes = [ci, i64, i64]
+    lib.t81b200_stage_rows_bytes.restype = ctypes.c_size_t
+    lib.t81b200_stage_rows.argtypes = [vp, ci, i64, i64, i64, vp, vp]
     lib.t81b200_column_sums.argtypes = [vp, ci, i64, i64, i64, vp, vp]
     lib.t81b200_tq_bytes.argtypes = [ci, i64, i64]
     lib.t81b200_tq_bytes.restype = i64

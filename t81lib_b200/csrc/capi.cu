@@ -340,10 +340,12 @@ extern "C" int t81b200_gemm_trit_t2(int n_group, const uint8_t *const *t2, const
 }
 
 // Decode-sized calls the streaming kernel takes: up to 16 rows, fp32 ones in two planes.
-static bool linear_t2_streams(int b_dtype, int64_t N, int fp32_planes) { return N <= 16 && (b_dtype != T81B200_F32 || fp32_planes <= 2); }
+static bool linear_t2_streams(int b_dtype, int64_t N, int fp32_planes) {
+    return N <= 16 && b_dtype != T81B200_BF16X3 && (b_dtype != T81B200_F32 || fp32_planes <= 2);
+}
 
 extern "C" size_t t81b200_linear_t2_workspace_bytes(const void *B, int b_dtype, int64_t ldb, int64_t M, int64_t N, int64_t K, int fp32_planes) {
-    if (M <= 0 || N <= 0 || K <= 0 || !valid_dtype(b_dtype) || (linear_t2_streams(b_dtype, N, fp32_planes) && K <= kT2StreamingMaxK)) return 0;
+    if (M <= 0 || N <= 0 || K <= 0 || b_dtype == T81B200_BF16X3 || !valid_dtype(b_dtype) || (linear_t2_streams(b_dtype, N, fp32_planes) && K <= kT2StreamingMaxK)) return 0;
     return gemm_trit_tc_scratch(B, b_dtype, T81B200_LAYOUT_NK, ldb, N, K, fp32_planes);
 }
 
@@ -351,7 +353,8 @@ extern "C" int t81b200_linear_t2(const uint8_t *t2, const float *row_scale, cons
                                  int b_dtype, int64_t ldb, int c_dtype, int64_t ldc, int64_t N, int64_t K, float alpha, float beta,
                                  int fp32_planes, void *workspace, size_t workspace_bytes, void *stream) {
     if (M <= 0 || K <= 0 || N < 0) return fail(T81B200_EINVAL, "linear_t2: dimensions must be positive");
-    if (!valid_dtype(b_dtype) || !valid_dtype(c_dtype)) return fail(T81B200_EINVAL, "gemm_trit: unknown dtype");
+    if ((!valid_dtype(b_dtype) && b_dtype != T81B200_BF16X3) || !valid_dtype(c_dtype)) return fail(T81B200_EINVAL, "gemm_trit: unknown dtype");
+    if (b_dtype == T81B200_BF16X3 && (reinterpret_cast<uintptr_t>(B) % 16 != 0 || ldb % 8 != 0)) return fail(T81B200_EALIGN, "linear_t2: planes must be 16-byte aligned rows");
     if (fp32_planes != 2 && fp32_planes != 3) return fail(T81B200_EINVAL, "linear_t2: fp32 activations take 2 or 3 planes");
     if (ldb < K || ldc < M) return fail(T81B200_EINVAL, "gemm_trit: leading dimension below the row length");
     if (N > 0 && (!t2 || !B || !C)) return fail(T81B200_EINVAL, "gemm_trit: null pointer");

@@ -760,13 +760,14 @@ int gemm_trit_tc_launch(int fmt, int fp32_planes, const uint8_t *A, const float 
                         int n_peers, void *const *peer_C) {
     const void *x_ptr = B;
     int64_t x_ld = ldb, x_rows = N;
-    const int planes = b_dtype == T81B200_F32 ? fp32_planes : 1;
+    const int planes = b_dtype == T81B200_F32 ? fp32_planes : (b_dtype == T81B200_BF16X3 ? 3 : 1);
+    x_rows = (int64_t)planes * N;
     if (!reads_in_place(B, b_dtype, layout, ldb)) {
         const size_t need = gemm_trit_tc_scratch_most(b_dtype, N, K, planes);
         if (!workspace || workspace_bytes < need || reinterpret_cast<uintptr_t>(workspace) % 16 != 0)
             return fail(T81B200_EWORKSPACE, "gemm_trit: %zu bytes of 16-byte aligned workspace needed, %zu given", need, workspace_bytes);
         if (int rc = stage_planes(B, b_dtype, layout, ldb, N, K, planes, workspace, st)) return rc;
-        x_ptr = workspace; x_ld = scratch_row(K); x_rows = (int64_t)planes * N;
+        x_ptr = workspace; x_ld = scratch_row(K);
     }
     const TcShape shape = pick_shape(M, N, K, planes);
     const bool f16 = b_dtype == T81B200_F16;
@@ -825,6 +826,26 @@ int gemm_trit_tc_launch(int fmt, int fp32_planes, const uint8_t *A, const float 
 }
 
 }  // namespace t81b200
+
+// ---- staging by itself: what several products of one operand share ------------------------
+
+extern "C" int64_t t81b200_stage_rows_ld(int64_t width) { return (width + 7) & ~(int64_t)7; }
+
+extern "C" size_t t81b200_stage_rows_bytes(int dtype, int64_t tokens, int64_t width) {
+    if (tokens <= 0 || width <= 0) return 0;
+    return (size_t)(dtype == T81B200_F32 ? 3 : 1) * tokens * t81b200_stage_rows_ld(width) * 2;
+}
+
+extern "C" int t81b200_stage_rows(const void *src, int dtype, int64_t ld, int64_t tokens, int64_t width, void *out, void *stream) {
+    using namespace t81b200;
+    if (tokens < 0 || width < 0 || ld < width) return fail(T81B200_EINVAL, "stage_rows: bad dimensions");
+    if (dtype != T81B200_F32 && dtype != T81B200_BF16 && dtype != T81B200_F16) return fail(T81B200_EINVAL, "stage_rows: unknown dtype %d", dtype);
+    if (int rc = check_device()) return rc;
+    if (tokens == 0 || width == 0) return T81B200_OK;
+    if (!src || !out) return fail(T81B200_EINVAL, "stage_rows: null pointer");
+    if (reinterpret_cast<uintptr_t>(out) % 16 != 0) return fail(T81B200_EALIGN, "stage_rows: the output must be 16-byte aligned");
+    return stage_planes(src, dtype, T81B200_LAYOUT_NK, ld, tokens, width, 3, out, static_cast<cudaStream_t>(stream));
+}
 
 // ---- entry point that allocates nothing -------------------------------------------------
 

@@ -4,7 +4,7 @@
 //   out[o][k] = slope(w[o][k]) * sum_t g[t][o] * x[t][k]        slope = 2 where |w / scale| < 0.5, else 0
 //
 // g (tokens, rows) and x (tokens, cols) are token-major, so both operands are contiguous along the output index and
-// strided along the contraction: they are loaded as they lie (boxes of 64 columns x 64 tokens, 128-byte swizzle) and
+// strided along the contraction: they are loaded as they lie (boxes of 64 columns, 128-byte swizzle) and
 // read by tcgen05.mma as M- / N-major operands; nothing is transposed in memory.  One pair of CTAs (cta_group::2) per
 // 256 x bn tile; each loads its own 128 columns of g and half of the tile's columns of x.
 //
@@ -15,7 +15,9 @@
 // cut an accumulator off at every 16-token step instead of rounding it, which over 4096 tokens in one piece left the
 // result 4.4e-6 (root mean square) from the exact sums, against 1.1e-6 for fp32 arithmetic on CUDA cores.
 //
-// Bound by the operands' way from L2: a pair tile takes 32 KB per CTA and 64-token step, whatever the MMAs do.  Tiles
+// Bound by the operands' way from L2: a pair tile takes 32 KB per CTA and 64 tokens of 16-bit operands.  The planes of
+// fp32 operands are loaded together, once for all six products (2050 x 1537 x 1000 tokens: 64 us with a load per product,
+// 56 us this way).  Tiles
 // are walked in groups of eight row tiles so that what runs at a time shares its operands in L2.  The slope is applied in
 // the epilogue, on values that a trip through shared memory has turned into whole 128-byte rows, beside the weights.
 #include "common.cuh"
@@ -29,9 +31,9 @@ namespace t81b200 {
 
 namespace {
 
-constexpr int BT = 64;                        // tokens per operand stage
-constexpr int BOX_BYTES = 64 * BT * 2;        // 64 columns x 64 tokens: 8 KB
-constexpr int A_BYTES = 2 * BOX_BYTES;        // this CTA's 128 columns of g
+// A stage of the operand ring: per 64 columns of this CTA (two groups of g, bn / 128 of x) one box of all planes.
+__host__ __device__ constexpr int token_step(int planes) { return planes == 1 ? 64 : 32; }
+__host__ __device__ constexpr int group_bytes(int planes) { return planes * token_step(planes) * 128; }  // 8 KB, or 12 KB
 constexpr int MAX_STAGES = 8;
 constexpr int EPILOGUE_WARPS = 8;             // two per quarter of the rows: each takes every other 32-column block
 constexpr int NUM_THREADS = (2 + EPILOGUE_WARPS) * 32;
@@ -50,7 +52,7 @@ struct WgradParams {
     float *out;
     int64_t rows, cols, ldw;
     int m_tiles, n_tiles, bn;
-    int pairs, token_steps;           // plane products (1 or 6), 64-token steps
+    int planes, token_steps;          // 1 or 3 planes (6 plane products); stages of tokens
     int segments;                     // parts of the contraction that are added up in `out` (one if split)
     int splits, stages;
     uint32_t idesc;
@@ -63,9 +65,9 @@ __device__ __forceinline__ void plane_pair(int i, int &a, int &b) {
     b = i == 1 || i == 3 ? 1 : (i == 4 ? 2 : 0);   // 0 1 0 1 2 0
 }
 
-// M- / N-major SWIZZLE_128B operand: 64-column groups 8 KB apart, 8-token groups 1 KB apart.
-__device__ __forceinline__ uint64_t umma_desc_mn(uint32_t smem_addr) {
-    return (uint64_t)((smem_addr >> 4) & 0x3FFF) | ((uint64_t)(BOX_BYTES >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) |
+// M- / N-major SWIZZLE_128B operand: 64-column groups `group` bytes apart, 8-token groups 1 KB apart.
+__device__ __forceinline__ uint64_t umma_desc_mn(uint32_t smem_addr, uint32_t group) {
+    return (uint64_t)((smem_addr >> 4) & 0x3FFF) | ((uint64_t)(group >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) |
            ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
 
@@ -145,7 +147,7 @@ __device__ __forceinline__ void emit_block(const WgradParams &p, const uint32_t 
 // 32 columns of the tile's sums: fp32 operands have the small products beside the large one.
 __device__ __forceinline__ void load_sums(const WgradParams &p, uint32_t taddr, uint32_t (&v)[32]) {
     tmem_ld32(taddr, v);
-    if (p.pairs > 1) {
+    if (p.planes > 1) {
         uint32_t small[32];
         tmem_ld32(taddr + 256u, small);
 #pragma unroll
@@ -159,7 +161,7 @@ gemm_wgrad_tc_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_con
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t *gen_base = smem_raw + (base - smem_u32(smem_raw));
-    const uint32_t b_bytes = (uint32_t)p.bn / 2 / 64 * BOX_BYTES, stage_bytes = A_BYTES + b_bytes;
+    const uint32_t group = (uint32_t)group_bytes(p.planes), stage_bytes = (2u + (uint32_t)p.bn / 128u) * group;
     const uint32_t turn_off = (uint32_t)p.stages * stage_bytes, bars = base + turn_off + TURN_BYTES;
     auto full = [&](int s) { return bars + 8u * s; };
     auto empty = [&](int s) { return bars + 8u * (MAX_STAGES + s); };
@@ -190,9 +192,9 @@ gemm_wgrad_tc_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_con
     const int n_clusters = (int)gridDim.x / (2 * p.splits), cluster_id = (int)blockIdx.x / (2 * p.splits);
     // a piece of work is one segment of one tile; this pair's share of a segment: token steps, each with all plane products
     const int parts = p.splits * p.segments;
-    auto share_begin = [&](int piece) { return (int)((int64_t)p.token_steps * (piece % p.segments * p.splits + slice) / parts) * p.pairs; };
-    auto share_end = [&](int piece) { return (int)((int64_t)p.token_steps * (piece % p.segments * p.splits + slice + 1) / parts) * p.pairs; };
-    const int n_bufs = p.pairs == 1 ? 2 : 1;  // fp32: the second buffer holds the small products
+    auto share_begin = [&](int piece) { return (int)((int64_t)p.token_steps * (piece % p.segments * p.splits + slice) / parts); };
+    auto share_end = [&](int piece) { return (int)((int64_t)p.token_steps * (piece % p.segments * p.splits + slice + 1) / parts); };
+    const int n_bufs = p.planes == 1 ? 2 : 1;  // fp32: the second buffer holds the small products
     auto next_piece = [&](int piece) { return (piece + 1) % p.segments ? piece + 1 : piece + 1 + (n_clusters - 1) * p.segments; };
     const uint16_t pair_mask = (uint16_t)(3u << (rank & ~1u));
     const float half_scale = 0.5f * *p.scale;
@@ -208,14 +210,12 @@ gemm_wgrad_tc_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_con
             for (int s = s0; s < s1; ++s) {
                 ok = mbar_wait(empty(ring.stage), ring.phase ^ 1);
                 if (!ok) break;
-                int pa, pb;
-                plane_pair(s % p.pairs, pa, pb);
-                const int t0 = s / p.pairs * BT;
+                const int t0 = s * token_step(p.planes);
                 if (elect_one()) {
                     if (half == 0) mbar_arrive_expect_tx(full(ring.stage), 2 * stage_bytes);
                     uint32_t dst = base + (uint32_t)ring.stage * stage_bytes;
-                    for (int b = 0; b < 2; ++b, dst += BOX_BYTES) tma_load_3d_pair(dst, &map_g, o0 + 64 * b, t0, pa, full(ring.stage));
-                    for (int b = 0; b < p.bn / 128; ++b, dst += BOX_BYTES) tma_load_3d_pair(dst, &map_x, k0 + 64 * b, t0, pb, full(ring.stage));
+                    for (int b = 0; b < 2; ++b, dst += group) tma_load_3d_pair(dst, &map_g, o0 + 64 * b, t0, 0, full(ring.stage));
+                    for (int b = 0; b < p.bn / 128; ++b, dst += group) tma_load_3d_pair(dst, &map_x, k0 + 64 * b, t0, 0, full(ring.stage));
                 }
                 __syncwarp();
                 ring.advance(p.stages);
@@ -238,14 +238,26 @@ gemm_wgrad_tc_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_con
                     ok = mbar_wait(full(ring.stage), ring.phase);
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint64_t ad = umma_desc_mn(base + (uint32_t)ring.stage * stage_bytes);
-                    const uint64_t bd = umma_desc_mn(base + (uint32_t)ring.stage * stage_bytes + A_BYTES);
-                    const int pair = s % p.pairs;
-                    const uint32_t d = d_tmem + (pair == 0 ? 0u : 256u), more = s - s0 >= (pair == 0 ? 1 : 2) ? 1u : 0u;
-                    if (elect_one()) {
+                    const uint64_t ad = umma_desc_mn(base + (uint32_t)ring.stage * stage_bytes, group);
+                    const uint64_t bd = umma_desc_mn(base + (uint32_t)ring.stage * stage_bytes + 2 * group, group);
+                    const uint32_t more = s != s0 ? 1u : 0u;
+                    if (elect_one()) {  // 16 tokens: two 1 KB groups
+                        if (p.planes == 1) {
 #pragma unroll
-                        for (int k = 0; k < BT / 16; ++k)  // 16 tokens: two 1 KB groups
-                            umma_pair(d, ad + (uint64_t)(128 * k), bd + (uint64_t)(128 * k), p.idesc, k == 0 ? more : 1u);
+                            for (int k = 0; k < token_step(1) / 16; ++k)
+                                umma_pair(d_tmem, ad + (uint64_t)(128 * k), bd + (uint64_t)(128 * k), p.idesc, k != 0 ? 1u : more);
+                        } else {
+                            constexpr uint64_t plane = token_step(3) * 128 >> 4;
+#pragma unroll
+                            for (int k = 0; k < token_step(3) / 16; ++k)
+#pragma unroll
+                                for (int i = 0; i < 6; ++i) {
+                                    int pa, pb;
+                                    plane_pair(i, pa, pb);
+                                    umma_pair(d_tmem + (i == 0 ? 0u : 256u), ad + pa * plane + (uint64_t)(128 * k), bd + pb * plane + (uint64_t)(128 * k),
+                                              p.idesc, k != 0 || i > 1 ? 1u : more);
+                                }
+                        }
                         umma_commit_pair(empty(ring.stage), pair_mask);
                     }
                     __syncwarp();
@@ -332,9 +344,9 @@ gemm_wgrad_tc_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_con
     }
 }
 
-int make_map_3d(CUtensorMap *map, CUtensorMapDataType dt, const void *ptr, uint64_t inner, uint64_t tokens, uint64_t planes, uint64_t ld_bytes) {
-    const cuuint64_t dims[3] = {inner, tokens, planes}, strides[2] = {ld_bytes, ld_bytes * tokens};
-    const cuuint32_t box[3] = {64, BT, 1};
+int make_map_3d(CUtensorMap *map, CUtensorMapDataType dt, const void *ptr, uint64_t inner, uint64_t tokens, int planes, uint64_t ld_bytes) {
+    const cuuint64_t dims[3] = {inner, tokens, (cuuint64_t)planes}, strides[2] = {ld_bytes, ld_bytes * tokens};
+    const cuuint32_t box[3] = {64, (cuuint32_t)token_step(planes), (cuuint32_t)planes};
     return make_map(map, dt, 3, ptr, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
@@ -352,10 +364,10 @@ int launch_wgrad(const cudaLaunchConfig_t &cfg, const CUtensorMap &mg, const CUt
     return T81B200_OK;
 }
 
-bool in_place(const void *p, int dtype, int64_t ld) { return dtype != T81B200_F32 && reinterpret_cast<uintptr_t>(p) % 16 == 0 && (ld * 2) % 16 == 0; }
+// Scratch of one operand: none when it is 16-bit (or staged planes already) and TMA can read it where it is.
 size_t operand_scratch(const void *p, int dtype, int64_t ld, int64_t tokens, int64_t width) {
-    if (in_place(p, dtype, ld)) return 0;
-    return ((size_t)(dtype == T81B200_F32 ? 3 : 1) * tokens * ((width + 7) & ~(int64_t)7) * 2 + 255) / 256 * 256;
+    if (dtype != T81B200_F32 && reinterpret_cast<uintptr_t>(p) % 16 == 0 && (ld * 2) % 16 == 0) return 0;
+    return (t81b200_stage_rows_bytes(dtype, tokens, width) + 255) / 256 * 256;
 }
 
 }  // namespace
@@ -374,16 +386,20 @@ int gemm_wgrad_status(int reset) {
 
 using namespace t81b200;
 
-extern "C" size_t t81b200_qat_weight_grad_workspace_bytes(const void *g, int64_t ldg, const void *x, int64_t ldx, int dtype, int64_t tokens,
-                                                          int64_t rows, int64_t cols) {
+extern "C" size_t t81b200_qat_weight_grad_workspace_bytes(const void *g, int g_dtype, int64_t ldg, const void *x, int x_dtype, int64_t ldx,
+                                                          int64_t tokens, int64_t rows, int64_t cols) {
     if (tokens <= 0 || rows <= 0 || cols <= 0) return 0;
-    return operand_scratch(g, dtype, ldg, tokens, rows) + operand_scratch(x, dtype, ldx, tokens, cols);
+    return operand_scratch(g, g_dtype, ldg, tokens, rows) + operand_scratch(x, x_dtype, ldx, tokens, cols);
 }
 
-extern "C" int t81b200_qat_weight_grad(const void *g, int64_t ldg, const void *x, int64_t ldx, int dtype, int64_t tokens, int64_t rows, int64_t cols,
-                                       const float *w, int64_t ldw, const float *scale, float *out, void *workspace, size_t workspace_bytes, void *stream) {
+extern "C" int t81b200_qat_weight_grad(const void *g, int g_dtype, int64_t ldg, const void *x, int x_dtype, int64_t ldx, int64_t tokens, int64_t rows,
+                                       int64_t cols, const float *w, int64_t ldw, const float *scale, float *out, void *workspace, size_t workspace_bytes,
+                                       void *stream) {
     if (tokens < 0 || rows < 0 || cols < 0 || ldg < rows || ldx < cols || ldw < cols) return fail(T81B200_EINVAL, "qat_weight_grad: bad dimensions");
-    if (dtype != T81B200_F32 && dtype != T81B200_BF16 && dtype != T81B200_F16) return fail(T81B200_EINVAL, "qat_weight_grad: unknown dtype %d", dtype);
+    auto wide = [](int d) { return d == T81B200_F32 || d == T81B200_BF16X3; };
+    auto narrow = [](int d) { return d == T81B200_BF16 || d == T81B200_F16; };
+    if (!(wide(g_dtype) && wide(x_dtype)) && !(narrow(g_dtype) && g_dtype == x_dtype))
+        return fail(T81B200_EINVAL, "qat_weight_grad: operand dtypes %d and %d", g_dtype, x_dtype);
     if (int rc = check_device()) return rc;
     if (rows == 0 || cols == 0) return T81B200_OK;
     if (!w || !scale || !out || (tokens > 0 && (!g || !x))) return fail(T81B200_EINVAL, "qat_weight_grad: null pointer");
@@ -393,47 +409,45 @@ extern "C" int t81b200_qat_weight_grad(const void *g, int64_t ldg, const void *x
         T81_CUDA_TRY(cudaMemsetAsync(out, 0, (size_t)rows * cols * 4, st));
         return T81B200_OK;
     }
-    const size_t need_g = operand_scratch(g, dtype, ldg, tokens, rows), need_x = operand_scratch(x, dtype, ldx, tokens, cols);
+    const size_t need_g = operand_scratch(g, g_dtype, ldg, tokens, rows), need_x = operand_scratch(x, x_dtype, ldx, tokens, cols);
     if (need_g + need_x > 0 && (!workspace || workspace_bytes < need_g + need_x || reinterpret_cast<uintptr_t>(workspace) % 256 != 0))
         return fail(T81B200_EWORKSPACE, "qat_weight_grad: %zu bytes of 256-byte aligned workspace needed, %zu given", need_g + need_x, workspace_bytes);
-    const int planes = dtype == T81B200_F32 ? 3 : 1;
-    const CUtensorMapDataType dt = dtype == T81B200_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
-    CUtensorMap mg, mx;
-    struct { const void *src; int64_t ld, width; size_t need; char *scratch; CUtensorMap *map; } ops[2] = {
-        {g, ldg, rows, need_g, static_cast<char *>(workspace), &mg}, {x, ldx, cols, need_x, static_cast<char *>(workspace) + need_g, &mx}};
-    for (auto &o : ops) {
-        const void *src = o.src;
-        int64_t ld = o.ld;
-        if (o.need) {
-            ld = (o.width + 7) & ~(int64_t)7;
-            if (int rc = stage_planes(o.src, dtype, T81B200_LAYOUT_NK, o.ld, tokens, o.width, planes, o.scratch, st)) return rc;
-            src = o.scratch;
-        }
-        if (int rc = make_map_3d(o.map, dt, src, (uint64_t)o.width, (uint64_t)tokens, (uint64_t)planes, (uint64_t)ld * 2)) return rc;
-    }
-
+    if ((g_dtype == T81B200_BF16X3 && need_g) || (x_dtype == T81B200_BF16X3 && need_x)) return fail(T81B200_EALIGN, "qat_weight_grad: planes must be 16-byte aligned rows");
     WgradParams p;
     memset(&p, 0, sizeof p);
+    p.planes = wide(g_dtype) ? 3 : 1;
+    const CUtensorMapDataType dt = g_dtype == T81B200_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+    CUtensorMap mg, mx;
+    struct { const void *src; int dtype; int64_t ld, width; size_t need; char *scratch; CUtensorMap *map; } ops[2] = {
+        {g, g_dtype, ldg, rows, need_g, static_cast<char *>(workspace), &mg}, {x, x_dtype, ldx, cols, need_x, static_cast<char *>(workspace) + need_g, &mx}};
+    for (auto &o : ops) {
+        if (o.need) {
+            if (int rc = t81b200_stage_rows(o.src, o.dtype, o.ld, tokens, o.width, o.scratch, stream)) return rc;
+            o.src = o.scratch;
+            o.ld = t81b200_stage_rows_ld(o.width);
+        }
+        if (int rc = make_map_3d(o.map, dt, o.src, (uint64_t)o.width, (uint64_t)tokens, p.planes, (uint64_t)o.ld * 2)) return rc;
+    }
     p.w = w; p.scale = scale; p.out = out; p.rows = rows; p.cols = cols; p.ldw = ldw;
-    p.token_steps = (int)((tokens + BT - 1) / BT);
-    p.pairs = planes == 3 ? 6 : 1;
+    p.token_steps = (int)((tokens + token_step(p.planes) - 1) / token_step(p.planes));
     p.m_tiles = (int)((rows + 255) / 256);
     // 256- or 128-column tiles, tokens split over up to four pairs of a cluster while that fits the GPU at once: whichever
-    // needs fewer steps one after the other (a 128-column step costs about 0.65 of a 256-column one)
+    // needs fewer steps one after the other (a 128-column step costs about 0.65 of a 256-column one, a split six of 64 tokens)
+    const double per_step = p.planes == 1 ? 1.0 : 3.0;
     double best = 1e30;
     for (int bn = 256; bn >= 128; bn -= 128)
         for (int s = 1; s <= MAX_SPLITS; ++s) {
             const int64_t tiles = (int64_t)p.m_tiles * ((cols + bn - 1) / bn), resident = resident_pair_clusters(s);
             if (s > p.token_steps || (s > 1 && tiles > resident)) continue;
-            const double t = (double)((tiles + resident - 1) / resident) * ((p.token_steps + s - 1) / s) * p.pairs * (bn == 256 ? 1.0 : 0.65) + (s > 1 ? 6.0 : 0.0);
+            const double t = (double)((tiles + resident - 1) / resident) * ((p.token_steps + s - 1) / s) * per_step * (bn == 256 ? 1.0 : 0.65) + (s > 1 ? 6.0 : 0.0);
             if (t < best) { best = t; p.bn = bn; p.splits = s; }
         }
-    p.segments = p.pairs > 1 && p.splits == 1 ? (p.token_steps + 15) / 16 : 1;
+    p.segments = p.planes > 1 && p.splits == 1 ? (int)((tokens + 1023) / 1024) : 1;
     p.n_tiles = (int)((cols + p.bn - 1) / p.bn);
-    const int stage = A_BYTES + p.bn / 2 / 64 * BOX_BYTES;
+    const int stage = (2 + p.bn / 128) * group_bytes(p.planes);
     const int fit = (SMEM_LIMIT - 1024 - TURN_BYTES - BARRIER_BYTES) / stage;
     p.stages = fit < MAX_STAGES ? fit : MAX_STAGES;
-    p.idesc = umma_instr_desc(p.bn, dtype == T81B200_F16, true, true);
+    p.idesc = umma_instr_desc(p.bn, g_dtype == T81B200_F16, true, true);
     p.vec = cols % 4 == 0 && ldw % 4 == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0 && reinterpret_cast<uintptr_t>(out) % 16 == 0 ? 1 : 0;
     const int64_t tiles = (int64_t)p.m_tiles * p.n_tiles;
     const int64_t clusters = p.splits > 1 || tiles < resident_pair_clusters(1) ? tiles : resident_pair_clusters(1);

@@ -186,19 +186,39 @@ PyTypeObject ProductType = {PyVarObject_HEAD_INIT(nullptr, 0)};
 
 Tensor with_unit_columns(const Tensor &t) { return t.stride(1) == 1 && (t.size(0) < 2 || t.stride(0) >= t.size(1)) ? t : t.contiguous(); }
 
-Tensor weight_grad(const Tensor &g_, const Tensor &x_, const Tensor &w, const Tensor &scale) {
-    const Tensor g = with_unit_columns(g_), x = with_unit_columns(x_);
-    const int64_t tokens = x.size(0), rows = w.size(0), cols = w.size(1);
-    const int64_t ldg = tokens > 1 ? g.stride(0) : rows, ldx = tokens > 1 ? x.stride(0) : cols;
-    const int code = dtype_code(x.scalar_type());
+// Token-major rows as an operand of the gradient products.
+Rows rows_of(const Tensor &t) {
+    Rows r;
+    r.data = t.const_data_ptr();
+    r.dtype = dtype_code(t.scalar_type());
+    r.tokens = t.size(0);
+    r.ld = r.tokens > 1 ? t.stride(0) : t.size(1);
+    return r;
+}
+
+// The same rows staged for TMA where they cannot be read in place; `keep` holds the copy.
+Rows staged(const Rows &r, int64_t width, const c10::Device &device, Tensor &keep) {
+    if (r.tokens == 0 || (r.dtype != T81B200_F32 && reinterpret_cast<uintptr_t>(r.data) % 16 == 0 && r.ld % 8 == 0)) return r;
+    OnDevice on(device);
+    keep = at::empty({(int64_t)t81b200_stage_rows_bytes(r.dtype, r.tokens, width)}, at::TensorOptions().dtype(at::kByte).device(device));
+    check(t81b200_stage_rows(r.data, r.dtype, r.ld, r.tokens, width, keep.mutable_data_ptr(), stream_of(device)));
+    Rows s = r;
+    s.data = keep.const_data_ptr();
+    s.ld = t81b200_stage_rows_ld(width);
+    if (r.dtype == T81B200_F32) s.dtype = T81B200_BF16X3;
+    return s;
+}
+
+Tensor weight_grad(const Rows &g, const Rows &x, const Tensor &w, const Tensor &scale) {
+    const int64_t rows = w.size(0), cols = w.size(1);
     OnDevice on(w.device());
     Tensor out = at::empty({rows, cols}, w.options());
-    const size_t need = t81b200_qat_weight_grad_workspace_bytes(g.const_data_ptr(), ldg, x.const_data_ptr(), ldx, code, tokens, rows, cols);
+    const size_t need = t81b200_qat_weight_grad_workspace_bytes(g.data, g.dtype, g.ld, x.data, x.dtype, x.ld, x.tokens, rows, cols);
     Tensor ws;
     if (need) ws = at::empty({(int64_t)need}, w.options().dtype(at::kByte));
-    check(t81b200_qat_weight_grad(g.const_data_ptr(), ldg, x.const_data_ptr(), ldx, code, tokens, rows, cols, w.const_data_ptr<float>(),
-                                  rows > 1 ? w.stride(0) : cols, scale.const_data_ptr<float>(), out.mutable_data_ptr<float>(),
-                                  need ? ws.mutable_data_ptr() : nullptr, need, stream_of(w.device())));
+    check(t81b200_qat_weight_grad(g.data, g.dtype, g.ld, x.data, x.dtype, x.ld, x.tokens, rows, cols, w.const_data_ptr<float>(), rows > 1 ? w.stride(0) : cols,
+                                  scale.const_data_ptr<float>(), out.mutable_data_ptr<float>(), need ? ws.mutable_data_ptr() : nullptr, need,
+                                  stream_of(w.device())));
     return out;
 }
 
@@ -248,14 +268,16 @@ struct QatLinear : public torch::autograd::Function<QatLinear> {
         const Tensor g = with_unit_columns(grads[0].reshape({-1, rows}).to(x2.scalar_type()));
         const Tensor scales = ctx->saved_data["scales"].toTensor(), t2_t = ctx->saved_data["t2_t"].toTensor();
         Tensor grad_x, grad_w, grad_b;
+        const bool want_w = ctx->saved_data["weight"].toBool();
+        Rows r = rows_of(g);
+        Tensor keep;  // both products read one staged copy
+        if (t2_t.defined() && want_w) r = staged(r, rows, weight.device(), keep);
         if (t2_t.defined()) {
-            Rows r;
-            as_rows(g, rows, r);
             // every mantissa bit of a float32 gradient counts here: three planes
             grad_x = product(t2_t, cols, rows, scales.const_data_ptr<float>(), nullptr, r, {r.tokens, cols}, g.scalar_type(), weight.device(), 3)
                          .reshape(ctx->saved_data["shape"].toIntVector());
         }
-        if (ctx->saved_data["weight"].toBool()) grad_w = weight_grad(g, x2, with_unit_columns(weight), scale);
+        if (want_w) grad_w = weight_grad(r, rows_of(x2), with_unit_columns(weight), scale);
         if (ctx->saved_data["bias"].toBool()) {
             OnDevice on(g.device());
             grad_b = at::empty({rows}, weight.options());
@@ -345,7 +367,7 @@ PyObject *qat_weight_grad(PyObject *, PyObject *const *args, Py_ssize_t n) {
                           g.size(0) == x.size(0) && g.size(1) == w.size(0) && x.size(1) == w.size(1) && float_vector(scale, w.device(), 1),
                       "qat_weight_grad: operands do not match");
     try {
-        return THPVariable_Wrap(weight_grad(g, x, w, scale));
+        return THPVariable_Wrap(weight_grad(rows_of(with_unit_columns(g)), rows_of(with_unit_columns(x)), w, scale));
     } catch (const LibraryError &e) {
         return raise_library_error(e.code);
     }
