@@ -124,6 +124,7 @@ struct GemvLutParams {
     int stages, stage_bytes;
     int ring0_stages;        // ring slots [0, ring0_stages) lie at offset 0, the others at ring1_offset
     int ring1_offset, xs_offset, part_offset, sb_offset, bar_offset;
+    int vec_x;               // 1: rows of X start on 16-byte boundaries
     int bulk_x;              // 1: 16-bit activations, 16-byte aligned rows, K % 8 == 0: fetched by bulk copies
     int independent;         // 1: reads nothing the previous kernel of the stream wrote
     int n_peers;             // other GPUs whose result receives every output element too (one segment only)
@@ -207,47 +208,130 @@ __device__ __forceinline__ void lut_decode_word(uint32_t w, uint32_t lane_key, u
 template <typename XT> struct LutPlanes { static constexpr int value = 1; };
 template <> struct LutPlanes<float> { static constexpr int value = 2; };
 
-// Activations of the CTA's limbs [0, nl) (limb 0 = limb L0 of the row) for every token, element by element
-// (fp32 values, rows a bulk copy cannot take), in natural order, zero beyond K.  Plane 0 holds bf16(x); plane 1
-// (PLANES == 2) holds bf16(x - plane 0), so that plane 0 + plane 1 carries 16 mantissa bits of an fp32 input.  A thread has
-// the loads of four pairs in flight: one at a time, their latency was most of the call.
+// Activations of the CTA's limbs [0, nl) (limb 0 = limb L0 of the row) for every token, in natural order, zero beyond
+// K, eight elements at a time.  16-bit values as they are; fp32 as bf16(x) and bf16(x - that) (PLANES == 2: 16 mantissa
+// bits).  Rows on 16-byte boundaries (vec_x) are read with 128-bit loads, others element by element, four (two) eights in
+// flight per thread.  For what bulk copies cannot take (see bulk_x).
 template <typename XT, int PLANES>
-__device__ __forceinline__ void stage_elements(const GemvLutParams &p, int L0, int nl, uint32_t *xs, int tok_stride,
-                                               int plane_stride, int tid, int nthreads) {
+__device__ __forceinline__ void stage_activations(const GemvLutParams &p, int L0, int nl, uint32_t *xs, int tok_stride, int plane_stride,
+                                                  int tid, int nthreads) {
     const XT *X = static_cast<const XT *>(p.X);
-    const int per_tok = nl * 24;
+    const int per_tok = nl * 6;
     if (per_tok == 0) return;
     const int64_t k_first = (int64_t)L0 * 48;
-    int tok = 0, r = tid;  // pair r of token tok
+    int tok = 0, r = tid;  // eight r of token tok
     auto settle = [&]() { while (r >= per_tok && tok < p.ntok) { r -= per_tok; ++tok; } };
-    settle();
-    while (tok < p.ntok) {
-        XT e[4][2];
-        uint32_t *dst[4];
+    auto put = [&](uint32_t *dst, const XT (&e)[8]) {
+        if constexpr (PLANES == 1) {
+            uint4 q;
+            memcpy(&q, e, 16);
+            *reinterpret_cast<uint4 *>(dst) = q;
+        } else {
+            uint32_t hi[4], lo[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int64_t k = k_first + 2 * r;
-            const bool there = tok < p.ntok;
-            const XT *src = X + (int64_t)tok * p.ldx + k;
-            dst[u] = there ? xs + tok * tok_stride + r : nullptr;
-            e[u][0] = there && k < p.K ? src[0] : from_float<XT>(0.0f);
-            e[u][1] = there && k + 1 < p.K ? src[1] : from_float<XT>(0.0f);
-            r += nthreads;
-            settle();
+            for (int i = 0; i < 4; ++i) {
+                const float e0 = to_float<XT>(e[2 * i]), e1 = to_float<XT>(e[2 * i + 1]);
+                hi[i] = pack_bf16_pair(e0, e1);
+                const __nv_bfloat162 hv = *reinterpret_cast<const __nv_bfloat162 *>(&hi[i]);
+                lo[i] = pack_bf16_pair(e0 - __low2float(hv), e1 - __high2float(hv));
+            }
+            *reinterpret_cast<uint4 *>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+            *reinterpret_cast<uint4 *>(dst + plane_stride) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
         }
+    };
+    auto load_elements = [&](const XT *src, int64_t k, XT (&e)[8]) {
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            if (!dst[u]) break;
-            if constexpr (PLANES == 1) {
-                uint32_t both;
-                memcpy(&both, e[u], 4);
-                *dst[u] = both;
-            } else {
-                const float e0 = to_float<XT>(e[u][0]), e1 = to_float<XT>(e[u][1]);
-                const uint32_t hi = pack_bf16_pair(e0, e1);
-                const __nv_bfloat162 hv = *reinterpret_cast<const __nv_bfloat162 *>(&hi);
-                *dst[u] = hi;
-                dst[u][plane_stride] = pack_bf16_pair(e0 - __low2float(hv), e1 - __high2float(hv));
+        for (int i = 0; i < 8; ++i) e[i] = k + i < p.K ? __ldcg(src + i) : from_float<XT>(0.0f);
+    };
+    settle();
+    if (p.vec_x) {
+        constexpr int U = 4, LOADS = (int)sizeof(XT) / 2;
+        while (tok < p.ntok) {
+            uint4 q[U][LOADS];
+            uint32_t *dst[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int64_t k = k_first + 8 * r;
+                const XT *src = X + (int64_t)tok * p.ldx + k;
+                dst[u] = tok < p.ntok ? xs + tok * tok_stride + 4 * r : nullptr;
+                if (dst[u] && k + 8 <= p.K) {
+#pragma unroll
+                    for (int l = 0; l < LOADS; ++l) q[u][l] = __ldcg(reinterpret_cast<const uint4 *>(src) + l);
+                } else {
+                    XT e[8];
+                    if (dst[u]) load_elements(src, k, e);
+                    memcpy(&q[u], e, sizeof e);
+                }
+                r += nthreads;
+                settle();
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if (!dst[u]) break;
+                XT e[8];
+                memcpy(e, &q[u], sizeof e);
+                put(dst[u], e);
+            }
+        }
+    } else if constexpr (PLANES == 1) {
+        // 16-bit rows off those boundaries: three or four whole words, and single elements where the row starts on an odd
+        // place.  The loads of all eights come first and are put together afterwards: a wait per eight cost 3 us a call.
+        constexpr int U = 4;
+        while (tok < p.ntok) {
+            uint32_t w[U][5];
+            const XT *src[U];
+            uint32_t *dst[U];
+            int64_t at[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int64_t k = k_first + 8 * r;
+                src[u] = X + (int64_t)tok * p.ldx + k;
+                dst[u] = tok < p.ntok ? xs + tok * tok_stride + 4 * r : nullptr;
+                at[u] = k;
+                const bool odd = reinterpret_cast<uintptr_t>(src[u]) % 4 != 0;
+                const uint32_t *words = reinterpret_cast<const uint32_t *>(src[u] + (odd ? 1 : 0));
+                const uint16_t *halves = reinterpret_cast<const uint16_t *>(src[u]);
+                const bool load = dst[u] && k + 8 <= p.K;
+#pragma unroll
+                for (int i = 0; i < 3; ++i) w[u][i] = load ? __ldcg(words + i) : 0u;
+                w[u][3] = load && !odd ? __ldcg(words + 3) : 0u;
+                w[u][4] = 0u;
+                if (load && odd) {
+                    w[u][3] = __ldcg(halves + 7);
+                    w[u][4] = __ldcg(halves);
+                }
+                r += nthreads;
+                settle();
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if (!dst[u]) break;
+                uint4 q = make_uint4(w[u][0], w[u][1], w[u][2], w[u][3]);
+                if (reinterpret_cast<uintptr_t>(src[u]) % 4 != 0)
+                    q = make_uint4(__byte_perm(w[u][4], q.x, 0x5410), __funnelshift_l(q.x, q.y, 16), __funnelshift_l(q.y, q.z, 16), __byte_perm(q.z, q.w, 0x5432));
+                XT e[8];
+                if (at[u] + 8 <= p.K) memcpy(e, &q, 16);
+                else load_elements(src[u], at[u], e);
+                put(dst[u], e);
+            }
+        }
+    } else {
+        constexpr int U = 2;
+        while (tok < p.ntok) {
+            XT e[U][8];
+            uint32_t *dst[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int64_t k = k_first + 8 * r;
+                dst[u] = tok < p.ntok ? xs + tok * tok_stride + 4 * r : nullptr;
+                if (dst[u]) load_elements(X + (int64_t)tok * p.ldx + k, k, e[u]);
+                r += nthreads;
+                settle();
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if (!dst[u]) break;
+                put(dst[u], e[u]);
             }
         }
     }
@@ -448,7 +532,7 @@ gemv_trit_lut_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
         if (p.bulk_x) {
             issue_x(warp + lane * consumer_warps, 32 * consumer_warps);  // one copy per lane at most: one instruction per warp
         } else {
-            stage_elements<XT, PLANES>(p, L0, nl, xs, tok_stride, plane_stride, threadIdx.x, consumer_threads);
+            stage_activations<XT, PLANES>(p, L0, nl, xs, tok_stride, plane_stride, threadIdx.x, consumer_threads);
             asm volatile("bar.sync 1, %0;" ::"r"(consumer_threads) : "memory");
         }
         TRACE_STAMP(3);
@@ -931,6 +1015,7 @@ int gemv_trit_lut_launch(int fmt, int n_seg, const uint8_t *const *A, const floa
     p.row_warps = pl.row_warps; p.k_warps = pl.k_warps; p.limbs_per_slice = pl.limbs_per_slice;
     p.stages = pl.stages; p.stage_bytes = pl.stage_bytes; p.ring0_stages = pl.ring0_stages; p.ring1_offset = pl.ring1_offset;
     p.xs_offset = pl.xs_offset; p.part_offset = pl.part_offset; p.sb_offset = pl.sb_offset; p.bar_offset = pl.bar_offset;
+    p.vec_x = reinterpret_cast<uintptr_t>(X) % 16 == 0 && (ldx * (int64_t)dtype_size(x_dtype)) % 16 == 0 ? 1 : 0;
     p.bulk_x = x_dtype != T81B200_F32 && reinterpret_cast<uintptr_t>(X) % 16 == 0 && (ldx * 2) % 16 == 0 && K % 8 == 0 ? 1 : 0;
     p.n_peers = ctx ? ctx->n_peers : 0;
     for (int i = 0; i < T81B200_MAX_PEERS; ++i) p.peer_C[i] = i < p.n_peers ? ctx->peer_C[i] : nullptr;

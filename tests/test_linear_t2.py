@@ -49,3 +49,20 @@ def test_products_match_the_oracle(dev, rows, K, tokens, dtype):
         h = ops.linear_t2(t2, rows, x, K, sd, bd, torch.bfloat16)
         assert torch.equal(h, y.to(torch.bfloat16))
     assert _capi.kernel_status(reset=True) == 0
+
+
+# decode-sized calls whose rows lie on 16-byte, 4-byte and odd 2-byte places, and end inside a group of eight
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("rows,K,tokens", [(40, 7, 1), (70, 1905, 16), (100, 130, 5), (33, 1538, 9), (64, 14336, 16)])
+def test_decode_rows_off_boundaries(dev, rows, K, tokens, dtype):
+    from t81lib_b200 import _capi, ops
+    rng = np.random.default_rng(rows + K)
+    trits = rng.integers(-1, 2, (rows, K)).astype(np.int8)
+    t2 = ops.pack_t2(torch.from_numpy(oracle.pack_trits_rowwise(trits)).to(dev), rows, K)
+    wide = torch.from_numpy(rng.normal(size=(tokens, K + 3)).astype(np.float32)).to(dev).to(dtype)
+    tol = 2e-5 if dtype != torch.float32 else 1e-4  # as above; short contractions average fp32's 2^-17 roundings less
+    for x in (wide[:, :K].contiguous(), wide[:, 1:K + 1], wide[:, 2:K + 2]):
+        want = x.double().cpu().numpy() @ trits.T.astype(np.float64)
+        y = ops.linear_t2(t2, rows, x, K, None, None, torch.float32)
+        assert np.abs(y.cpu().numpy() - want).max() < tol * float(np.sqrt(np.mean(want ** 2)))
+    assert _capi.kernel_status(reset=True) == 0
