@@ -167,16 +167,16 @@ __device__ __forceinline__ void emit_block(const TcParams &p, const TcOutMaps &o
             dst[q] = *reinterpret_cast<const uint4 *>(out);
         }
     } else if (row_ok) {
+        // with beta the old values are all fetched before the first store (the compiler cannot know the stores to miss them)
+        float y[32];
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
-            const int64_t tok = (int64_t)tok0 + i;
-            if (tok < p.N) {
-                float y = __uint_as_float(v[i]) * scale + bias;
-                CT *dst = crow + tok * p.c_tok_stride;
-                if (p.beta != 0.0f) y += p.beta * to_float<CT>(*dst);
-                *dst = from_float<CT>(y);
-            }
+            y[i] = __uint_as_float(v[i]) * scale + bias;
+            if (p.beta != 0.0f && (int64_t)tok0 + i < p.N) y[i] += p.beta * to_float<CT>(crow[((int64_t)tok0 + i) * p.c_tok_stride]);
         }
+#pragma unroll
+        for (int i = 0; i < 32; ++i)
+            if ((int64_t)tok0 + i < p.N) crow[((int64_t)tok0 + i) * p.c_tok_stride] = from_float<CT>(y[i]);
         // column-sharded Linear: the same elements go into every peer's result over NVLink
         for (int pj = 0; pj < p.n_peers; ++pj) {
             CT *prow = static_cast<CT *>(p.peer_C[pj]) + row * p.c_row_stride;

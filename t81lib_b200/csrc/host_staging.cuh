@@ -13,8 +13,8 @@ struct HostStaging {
     enum { A, B, C, WORKSPACE, N_BUFFERS };
     void *dev[N_BUFFERS] = {nullptr};
     size_t dev_cap[N_BUFFERS] = {0};
-    char *pinned = nullptr;
-    size_t pinned_cap = 0;
+    char *pinned[2] = {nullptr, nullptr};  // on the way up and down
+    size_t pinned_cap[2] = {0, 0};
     cudaStream_t stream = nullptr;
     static constexpr int kMaxPieces = 64;
     cudaEvent_t landed[kMaxPieces] = {nullptr};
