@@ -28,7 +28,7 @@ constexpr int kMaxDevices = 64;
 HostStaging g_staging[kMaxDevices];
 
 constexpr size_t kPinnedMost = 96u << 20;      // larger calls are copied by the driver, from where the operands are
-constexpr size_t kHelpedBytes = 2u << 20;      // below, waking helpers costs what they save
+constexpr size_t kHelpedUp = 2u << 20, kHelpedDown = 1u << 20;  // below, waking helpers costs what they save
 constexpr int kHelpers = 3;
 
 inline void pause() {
@@ -216,7 +216,7 @@ int host_upload(HostStaging &s, const HostOperand *ops, int n) {
         moved[i].store(true, std::memory_order_release);
         return true;
     };
-    const bool helped = total >= kHelpedBytes && helpers().begin([&]() { while (move_one()) {} });
+    const bool helped = total >= kHelpedUp && helpers().begin([&]() { while (move_one()) {} });
     cudaError_t status = cudaSuccess;
     for (size_t queued = 0; queued < pieces.size();) {
         const bool more = move_one();
@@ -270,7 +270,7 @@ int host_download(HostStaging &s, void *host, const void *device, size_t bytes) 
         memcpy(static_cast<char *>(host) + i * piece, s.pinned[DOWN] + i * piece, size_of(i));
         return true;
     };
-    const bool helped = bytes >= kHelpedBytes && helpers().begin([&]() { while (move_one(true)) {} });
+    const bool helped = bytes >= kHelpedDown && helpers().begin([&]() { while (move_one(true)) {} });
     cudaError_t status = cudaSuccess;
     for (int seen = 0; seen < pieces;) {
         const cudaError_t e = cudaEventQuery(s.landed[seen]);
