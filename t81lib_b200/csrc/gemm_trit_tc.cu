@@ -334,6 +334,11 @@ gemm_trit_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     cluster_barrier();  // the other CTAs' barriers are initialised before anything arrives on them
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t *>(gen_base + (tmem_slot - base));
+    // scale and bias of this thread's output row, fetched long before the epilogue (a microsecond from HBM)
+    auto row_scale = [&](int64_t row) { return (row < p.M && p.row_scale ? __ldg(p.row_scale + row) : 1.0f) * p.alpha; };
+    auto row_bias = [&](int64_t row) { return row < p.M && p.bias ? __ldg(p.bias + row) : 0.0f; };
+    const int own_row = ((cluster_id % p.m_tiles) * 2 + half) * BM + (warp & 3) * 32 + lane;
+    const float own_scale = p.one_tile ? row_scale(own_row) : 0.0f, own_bias = p.one_tile ? row_bias(own_row) : 0.0f;
 
     if (warp == 0) {
         // ---------------- TMA producer: this CTA's packed weights and its half of the activation rows ----------------
@@ -421,14 +426,13 @@ gemm_trit_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             const int buf = it & 1;
             // One decision for all four epilogue warps (tcgen05.ld is .aligned, and the staging path meets at named
             // barriers): every thread's bounded wait returns, then the 128 threads agree.
+            const int row0 = ((tile % p.m_tiles) * 2 + half) * BM, n0 = (tile / p.m_tiles) * p.bn;
+            const int64_t row = (int64_t)row0 + quarter * 32 + lane;
+            const float scale = p.one_tile ? 0.0f : row_scale(row), bias = p.one_tile ? 0.0f : row_bias(row);
             ok = epilogue_all(mbar_wait(acc_full(buf), (uint32_t)(it >> 1) & 1u));
             if (!ok) break;
             if (p.one_tile) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const int row0 = ((tile % p.m_tiles) * 2 + half) * BM, n0 = (tile / p.m_tiles) * p.bn;
-            const int64_t row = (int64_t)row0 + quarter * 32 + lane;
-            const float scale = (row < p.M && p.row_scale ? p.row_scale[row] : 1.0f) * p.alpha;
-            const float bias = row < p.M && p.bias ? p.bias[row] : 0.0f;
 #pragma unroll 1
             for (int c = 0; c < p.bn / 32; ++c) {
                 uint32_t v[32];
@@ -500,16 +504,13 @@ gemm_trit_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             cluster_barrier();
         }
         if (warp >= EPILOGUE_WARP0) {
-            const int64_t row = (int64_t)row0 + lane_row;
-            const float scale = (row < p.M && p.row_scale ? p.row_scale[row] : 1.0f) * p.alpha;
-            const float bias = row < p.M && p.bias ? p.bias[row] : 0.0f;
             const bool first = quarter == 2 && lane == 0;
             for (int b = slice + S * group; b < blocks; b += 3 * S) {
                 uint32_t v[32];
                 tmem_ld32(t_lane + (uint32_t)(b * 32), v);
                 if (S > 1) fold_partials(v, gen_base, b, S, slice, lane_row);
                 const uint32_t stage = b_off + (uint32_t)b * OUT_STAGE_BYTES;
-                emit_block<CT>(p, omaps, v, row0, row, scale, bias, n0 + b * 32, OutStage{gen_base + stage, base + stage, (uint32_t)(2 + group), first, false});
+                emit_block<CT>(p, omaps, v, row0, own_row, own_scale, own_bias, n0 + b * 32, OutStage{gen_base + stage, base + stage, (uint32_t)(2 + group), first, false});
             }
             if (first) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
         }
