@@ -367,7 +367,14 @@ gemm_trit_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                 }
             }
         }
-        if (!ok && lane == 0) atomicCAS(&g_tc_status, STATUS_OK, STATUS_TIMEOUT_PRODUCER);
+        // The last commits' arrivals come from the pair's issuing CTA, one by one; this CTA may not end before they have landed.
+        for (int i = 0; i < p.b_stages && ok; ++i) {
+            ok = mbar_wait(b_empty(b.stage), b.phase ^ 1);
+            b.advance(p.b_stages);
+        }
+        const int fills = cluster_id < total_tiles ? ((total_tiles - 1 - cluster_id) / n_clusters + 1) * (c1 - c0) : 0;
+        for (int i = fills; i < fills + p.a_stages && ok; ++i) ok = mbar_wait(a_empty(i % p.a_stages), ((uint32_t)(i / p.a_stages) & 1u) ^ 1u);
+        if (!ok) give_up(&g_tc_status, STATUS_TIMEOUT_PRODUCER);
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
         if (half == 0) {
@@ -415,7 +422,7 @@ gemm_trit_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                 if (ok && elect_one()) umma_commit_pair(acc_full(buf), pair_mask);
                 __syncwarp();
             }
-            if (!ok && lane == 0) atomicCAS(&g_tc_status, STATUS_OK, STATUS_TIMEOUT_MMA);
+            if (!ok) give_up(&g_tc_status, STATUS_TIMEOUT_MMA);
         }
     } else if (warp < CONVERTER_WARP0) {
         // ---------------- epilogue of all but one-tile launches, which are finished below ----------------
@@ -445,7 +452,7 @@ gemm_trit_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             __syncwarp();
             if (lane == 0) mbar_arrive_leader(acc_empty(buf));
         }
-        if (!ok && lane == 0) atomicCAS(&g_tc_status, STATUS_OK, STATUS_TIMEOUT_EPILOGUE);
+        if (!ok) give_up(&g_tc_status, STATUS_TIMEOUT_EPILOGUE);
     } else {
         // ---------------- converters ----------------
         const int rt = (warp - CONVERTER_WARP0) & 3, group = (warp - CONVERTER_WARP0) >> 2;
@@ -475,7 +482,7 @@ gemm_trit_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             raw.advance(RAW_STAGES);
             c += 2;
         }
-        if (!ok && lane == 0) atomicCAS(&g_tc_status, STATUS_OK, STATUS_TIMEOUT_CONVERTER);
+        if (!ok) give_up(&g_tc_status, STATUS_TIMEOUT_CONVERTER);
     }
     __syncwarp();
 
@@ -516,7 +523,8 @@ gemm_trit_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         }
     } else if (threadIdx.x == EPILOGUE_WARP0 * 32) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");  // every store has completed
 
-    // ---------------- teardown: no CTA leaves while its peer may still arrive on its barriers or read its operands ----
+    // ---------------- teardown: no CTA leaves while its peer may still arrive on its barriers or read its operands
+    // (the producers have seen every commit) ----
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     cluster_barrier();
@@ -532,10 +540,20 @@ struct TcShape {
     size_t smem = 0;
 };
 
-// Tile width and split: the smallest estimate, in units of the time that one token of a 64-deep step takes (1.7 ns).  Fitted
-// to every width and split of 31 shapes from 512 x 528 x 256 to 9216 x 3072 x 2048 (mean regret 0.4 %, worst 6 %): a step costs
-// its tokens, and no less than 104 of them whatever the width (reading 256 rows of weights bounds it); a tile 400 more;
-// writing the last tiles out, 3 a token; sharing partial sums 1300 and 3 a token.
+// Time of a 64-deep step of one activation plane at tile width bn, in units of 1.7 ns (measured with 32 to 224 steps a tile):
+// its tokens, and no less than 104 of them whatever the width (reading 256 rows of weights bounds it); from 160 tokens on the
+// time grows slowly, since the issuing warps' own path between two barriers is a large part of it (290, 303 and 362 ns at 192,
+// 224 and 256 tokens with a barrier per chunk up to 224; 310, 320 and 370 ns with one per step, as several planes have it).
+double step_cost(int bn, int planes) {
+    if (bn <= 128) return bn > 104 ? bn : 104;
+    if (bn > 224) return 213;
+    return planes == 1 ? 178 - 0.25 * (224 - bn) : 188 - 0.2 * (224 - bn);
+}
+
+// Tile width and split: the smallest estimate, in step_cost's units.  Fitted to every width and split of 50 shapes from
+// 512 x 528 x 256 to 14336 x 4096 x 4096: the steps; a tile 400 more; writing the last tiles out, 3 a token; sharing partial
+// sums 1300 and 3 a token.  Several planes do without the width 160: one launch at it (728 tiles, two planes, fp32 result)
+// failed with an unspecified error on a variant of this kernel, and the cause is not known.
 TcShape pick_shape(int64_t M, int64_t N, int64_t K, int planes) {
     const int64_t m_tiles = (M + 255) / 256, chunks = (K + CHUNK - 1) / CHUNK, least = (N + 255) / 256;
     TcShape best;
@@ -546,14 +564,17 @@ TcShape pick_shape(int64_t M, int64_t N, int64_t K, int planes) {
         for (int s = 1; s <= MAX_SPLITS; ++s) {
             const int resident = resident_pair_clusters(s);
             if (s > chunks || (s > 1 && tiles > resident)) continue;
-            const double atom = planes * (bn > 104 ? bn : 104.0);
+            if (planes > 1 && bn > 128 && bn < 192) continue;
+            const double atom = planes * step_cost(bn, planes);
             const double t = (double)((tiles + resident - 1) / resident) * (3.0 * (double)((chunks + s - 1) / s) * atom + 400.0) +
                              3.0 * bn + (s > 1 ? 1300.0 + 3.0 * bn : 0.0);
             if (t < best_t) { best_t = t; best.bn = bn; best.n_tiles = (int)n_tiles; best.splits = s; }
         }
     }
-    // narrow tiles are bound by the issue of their MMAs: one barrier per chunk instead of one per atom
-    best.b_step = best.bn <= 128 ? 3 : 1;
+    // One barrier per chunk instead of one per step where two stages of a chunk fit (up to 224 tokens) and the planes are not
+    // several (those fill the time between two barriers anyway, and do better with a deeper ring: 200 against 220 us at
+    // 4096 x 4096 x 4096, fp32, 192 tokens).  With one plane: 192 tokens 408 -> 314 us at 14336 x 4096 x 4096.
+    best.b_step = best.bn <= 128 || (planes == 1 && best.bn <= 224) ? 3 : 1;
     best.a_stages = best.bn <= 96 ? 3 : 2;
     const int stage = best.bn * BK * best.b_step;
     int b = (SMEM_LIMIT - SMEM_FIXED - best.a_stages * A_CHUNK_BYTES) / stage;

@@ -221,7 +221,12 @@ gemm_wgrad_tc_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_con
                 ring.advance(p.stages);
             }
         }
-        if (!ok && lane == 0) atomicCAS(&g_wgrad_status, 0, WGRAD_STATUS_PRODUCER);
+        // every commit has landed here before this CTA may end (they arrive one by one from the pair's issuing CTA)
+        for (int i = 0; i < p.stages && ok; ++i) {
+            ok = mbar_wait(empty(ring.stage), ring.phase ^ 1);
+            ring.advance(p.stages);
+        }
+        if (!ok) give_up(&g_wgrad_status, WGRAD_STATUS_PRODUCER);
     } else if (warp == 1) {
         if (half == 0) {
             Ring ring;
@@ -266,7 +271,7 @@ gemm_wgrad_tc_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_con
                 if (ok && elect_one()) umma_commit_pair(acc_full(buf), pair_mask);
                 __syncwarp();
             }
-            if (!ok && lane == 0) atomicCAS(&g_wgrad_status, 0, WGRAD_STATUS_MMA);
+            if (!ok) give_up(&g_wgrad_status, WGRAD_STATUS_MMA);
         }
     } else {
         const int quarter = warp & 3, first = (warp - EPILOGUE_WARP0) >> 2;
@@ -296,7 +301,7 @@ gemm_wgrad_tc_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_con
             __syncwarp();
             if (lane == 0) mbar_arrive_leader(acc_empty(buf));
         }
-        if (!ok && lane == 0) atomicCAS(&g_wgrad_status, 0, WGRAD_STATUS_EPILOGUE);
+        if (!ok) give_up(&g_wgrad_status, WGRAD_STATUS_EPILOGUE);
     }
     __syncwarp();
 

@@ -18,6 +18,13 @@ __host__ __device__ constexpr uint32_t umma_instr_desc(int n, bool f16, bool a_m
            ((uint32_t)(n >> 3) << 17) | ((256u >> 4) << 24);
 }
 
+// A role whose bounded wait ran out: the code is recorded, and the CTA stays about a millisecond longer, so that copies and
+// commits under way land before its shared memory goes to another one.
+static __device__ __noinline__ void give_up(int *status, int code) {
+    if ((threadIdx.x & 31) == 0) atomicCAS(status, 0, code);
+    for (int i = 0; i < 10; ++i) __nanosleep(100000);
+}
+
 // True in one lane of a converged warp.  The loops of the issuing warps run on all 32 lanes (addresses and descriptors
 // stay in uniform registers) and only the issue itself is guarded: under a plain `lane == 0` branch the compiler cannot
 // know the operands to be uniform and every tcgen05 / TMA instruction pays for moving them (an operand atom of four

@@ -19,9 +19,11 @@ def dev(lib_built):
 
 # (rows, K, tokens): one row and column; 17 tokens on a 32-token tile; two CTAs with the second one empty (rows <= 128) or
 # nearly so (129, 257); K below, at and just past an atom (64) and a chunk (192); splits of 2 to 4 with unequal shares; a
-# 224- and a 256-token tile; several tiles per cluster with a ragged last one in both directions
+# 224- and a 256-token tile; several tiles per cluster with a ragged last one in both directions;
+# 192-, 224- and 160-token tiles whose chunks go behind one barrier, the last chunk of one step
 SHAPES = [(1, 1, 17), (128, 64, 32), (129, 65, 33), (257, 192, 64), (256, 193, 96), (300, 385, 97), (512, 1001, 129),
-          (1024, 4096, 40), (4096, 1536, 80), (100, 14336, 18), (260, 256, 777), (9500, 200, 1100)]
+          (1024, 4096, 40), (4096, 1536, 80), (100, 14336, 18), (260, 256, 777), (9500, 200, 1100),
+          (2048, 577, 1500), (9728, 400, 200), (12000, 130, 450)]
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
