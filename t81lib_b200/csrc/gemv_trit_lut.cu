@@ -790,7 +790,7 @@ struct PlanKey {
     const void *A[kMaxSeg];
     int64_t M[kMaxSeg];
     int64_t K;
-    int n_seg, ntok, x_dtype, c_dtype, device, fmt;
+    int n_seg, ntok, x_dtype, c_dtype, device, fmt, bulk_x;
     bool operator==(const PlanKey &o) const { return memcmp(this, &o, sizeof *this) == 0; }
 };
 struct PlanKeyHash {
@@ -852,7 +852,20 @@ int make_plan(Plan &pl, const PlanKey &key) {
     const int64_t kl = (key.K + 47) / 48;
     const int kl4 = (int)((kl + 3) & ~(int64_t)3);
     const int sms = sm_count();
-    const Switches sw = switches();
+    Switches sw = switches();
+    if (key.fmt == 1 && key.bulk_x && !sw.rw) {
+        // Where bulk copies bring the activations (no warp converts them), short rows need no cluster: its fold costs about a
+        // microsecond, and one CTA's copy of the activations is small.  Over 122 shapes in every launch shape the model below is
+        // 16 and 11 % behind the best for K up to 1152 and 1728, and a warp row of four K-slices is within 4 % of it for every
+        // number of tokens as long as the CTAs are at most three per SM (5504 x 1536, 8 tokens: 4.65 -> 3.85 us; 9216 x 1280, 10
+        // tokens: 6.25 -> 4.76).  With more than 8 tokens, where every CTA has twice the partial sums to fold, two slices are
+        // the better split for K up to 3456 (9216 x 3072, 13 tokens: 8.69 -> 7.39).
+        const int chunks = kl4 / 4;
+        int64_t tiles32 = 0, tiles64 = 0;
+        for (int i = 0; i < key.n_seg; ++i) { tiles32 += (key.M[i] + 31) / 32; tiles64 += (key.M[i] + 63) / 64; }
+        if (chunks >= 4 && chunks <= 9 && tiles32 <= 3 * sms) { sw.rw = 1; sw.kw = 4; sw.s = 1; }
+        else if (key.ntok > 8 && chunks >= 10 && chunks <= 18 && tiles64 <= sms) { sw.rw = 2; sw.kw = 4; sw.s = 2; }
+    }
     double best_t = 1e30;
     Plan best;
     for (int rwv = 1; rwv <= 8; ++rwv)
@@ -983,6 +996,8 @@ int gemv_trit_lut_launch(int fmt, int n_seg, const uint8_t *const *A, const floa
     PlanKey key;
     memset(&key, 0, sizeof key);
     for (int i = 0; i < n_seg; ++i) { key.A[i] = A[i]; key.M[i] = M[i]; }
+    const int bulk_x = x_dtype != T81B200_F32 && reinterpret_cast<uintptr_t>(X) % 16 == 0 && (ldx * 2) % 16 == 0 && K % 8 == 0 ? 1 : 0;
+    key.bulk_x = bulk_x;
     key.K = K; key.n_seg = n_seg; key.ntok = ntok; key.x_dtype = x_dtype; key.c_dtype = c_dtype; key.fmt = fmt;
     T81_CUDA_TRY(cudaGetDevice(&key.device));
     Plan pl;
@@ -1016,7 +1031,7 @@ int gemv_trit_lut_launch(int fmt, int n_seg, const uint8_t *const *A, const floa
     p.stages = pl.stages; p.stage_bytes = pl.stage_bytes; p.ring0_stages = pl.ring0_stages; p.ring1_offset = pl.ring1_offset;
     p.xs_offset = pl.xs_offset; p.part_offset = pl.part_offset; p.sb_offset = pl.sb_offset; p.bar_offset = pl.bar_offset;
     p.vec_x = reinterpret_cast<uintptr_t>(X) % 16 == 0 && (ldx * (int64_t)dtype_size(x_dtype)) % 16 == 0 ? 1 : 0;
-    p.bulk_x = x_dtype != T81B200_F32 && reinterpret_cast<uintptr_t>(X) % 16 == 0 && (ldx * 2) % 16 == 0 && K % 8 == 0 ? 1 : 0;
+    p.bulk_x = bulk_x;
     p.n_peers = ctx ? ctx->n_peers : 0;
     for (int i = 0; i < T81B200_MAX_PEERS; ++i) p.peer_C[i] = i < p.n_peers ? ctx->peer_C[i] : nullptr;
     p.sync_local = ctx ? ctx->sync_local : nullptr;

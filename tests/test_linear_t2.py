@@ -68,3 +68,20 @@ def test_decode_rows_off_boundaries(dev, rows, K, tokens, dtype):
         y = ops.linear_t2(t2, rows, x, K, None, None, torch.float32)
         assert np.abs(y.cpu().numpy() - want).max() < tol * float(np.sqrt(np.mean(want ** 2)))
     assert _capi.kernel_status(reset=True) == 0
+
+
+# launch shapes of short rows: K from 4 to 9 chunks with up to and past three 32-row CTAs per SM, 10 to 18 chunks with up to
+# and past one pair of 64-row CTAs per SM
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows,K,tokens", [(33, 584, 1), (1000, 1728, 16), (14208, 768, 5), (14240, 768, 9), (3200, 1736, 9),
+                                           (129, 3456, 16), (9472, 1920, 12), (9536, 1920, 12)])
+def test_decode_short_rows(dev, rows, K, tokens, dtype):
+    from t81lib_b200 import _capi, ops
+    rng = np.random.default_rng(rows + K)
+    trits = rng.integers(-1, 2, (rows, K)).astype(np.int8)
+    t2 = ops.pack_t2(torch.from_numpy(oracle.pack_trits_rowwise(trits)).to(dev), rows, K)
+    x = torch.from_numpy(rng.normal(size=(tokens, K)).astype(np.float32)).to(dev).to(dtype)
+    want = x.double().cpu().numpy() @ trits.T.astype(np.float64)
+    y = ops.linear_t2(t2, rows, x, K, None, None, torch.float32)
+    assert np.abs(y.cpu().numpy() - want).max() < 2e-5 * float(np.sqrt(np.mean(want ** 2)))  # exact products, fp32 sums
+    assert _capi.kernel_status(reset=True) == 0
