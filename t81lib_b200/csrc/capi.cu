@@ -74,6 +74,7 @@ int gemm_trit_simt_launch(const uint8_t *A, const float *row_scale, const void *
                           int64_t ldb, const float *bias, void *C, int c_dtype, int64_t ldc, int64_t M,
                           int64_t N, int64_t K, float alpha, float beta, cudaStream_t st);
 bool gemm_trit_tc_eligible(int64_t M, int64_t N, int64_t K);
+double gemm_trit_tc_estimate_us(int64_t M, int64_t N, int64_t K);
 size_t gemm_trit_tc_scratch(const void *B, int b_dtype, int layout, int64_t ldb, int64_t N, int64_t K, int planes);
 size_t gemm_trit_tc_scratch_most(int b_dtype, int64_t N, int64_t K, int planes);
 int gemm_trit_tc_launch(int fmt, int fp32_planes, const uint8_t *A, const float *row_scale, const void *B, int b_dtype, int layout,
@@ -227,16 +228,13 @@ extern "C" int t81b200_exchange_wait(uint32_t *sync_local, int n_peers, void *st
 // 17 .. T81B200_T2_MAX_ROWS rows of B: slices of the streaming kernel, or tensor-core tiles?  Estimates fitted to
 // measurements on the Llama- and Phi-shaped layers: a slice of 16 rows on the decode-stream layout costs about
 // 1.5 us plus its weight bytes at 1.35 TB/s (overlapping slices included), 1.4 times that on the limbs; the
-// tensor-core kernel runs its 128 x 256 tiles in waves of one per SM at about 8.5 ns per contraction step, whatever
-// part of a tile the rows of B fill.
+// tensor-core kernel's planner knows its own time.  Slices win for 17 to 32 rows of small matrices only.
 static bool streaming_wins(int64_t M, int64_t N, int64_t K, double layout_factor) {
     if (N <= 16) return true;
     if (N > T81B200_T2_MAX_ROWS || M <= 0 || K <= 0) return false;
     const double slices = (double)((N + 15) / 16);
     const double stream_us = layout_factor * slices * (1.5 + (double)M * (double)K * 0.25 / 1.35e6);
-    const int64_t tiles = ((M + 127) / 128) * ((N + 255) / 256);
-    const double waves = (double)((tiles + sm_count() - 1) / sm_count());
-    return stream_us < 5.0 + waves * (double)K * 8.5e-3;
+    return stream_us < gemm_trit_tc_estimate_us(M, N, K);
 }
 
 extern "C" int t81b200_prefers_streaming(int64_t M, int64_t N, int64_t K) { return streaming_wins(M, N, K, 1.0) ? 1 : 0; }
@@ -261,11 +259,13 @@ static int gemm_trit_local(const uint8_t *A, const float *row_scale, const void 
 
     if (a_aligned && layout == T81B200_LAYOUT_NK && N <= 16 && K > 0)
         return gemv_trit_launch(A, row_scale, B, b_dtype, ldb, bias, C, c_dtype, ldc, M, (int)N, K, alpha, beta, st, ctx);
-    // 17 to 128 rows of B: one launch of the streaming kernel per 16 rows often beats tensor-core tiles that would be
-    // mostly empty (4096 x 4096 x 32: 10 us instead of 42); streaming_wins decides.  A later slice reads and writes nothing an earlier one
-    // touches and is released by it only once its own input is complete: the slices are flagged independent and
-    // overlap.  Not with peers: the exchange protocol counts calls, not slices.
-    if (a_aligned && layout == T81B200_LAYOUT_NK && K > 0 && !ctx && streaming_wins(M, N, K, 1.4)) {
+    // 17 to 128 rows of B: one launch of the streaming kernel per 16 rows where streaming_wins says so, or where the tiles would
+    // need scratch memory that the caller has not lent.  A later slice reads and writes nothing an earlier one touches and is
+    // released by it only once its own input is complete: the slices are flagged independent and overlap.  Not with peers: the
+    // exchange protocol counts calls, not slices.
+    const size_t need = gemm_trit_tc_scratch(B, b_dtype, layout, ldb, N, K, 2);
+    const bool tiles = need == 0 || (workspace && workspace_bytes >= need && reinterpret_cast<uintptr_t>(workspace) % 16 == 0 && worth_staging(M, N, K));
+    if (a_aligned && layout == T81B200_LAYOUT_NK && K > 0 && !ctx && N <= T81B200_T2_MAX_ROWS && (!tiles || streaming_wins(M, N, K, 1.4))) {
         const int64_t esz_b = (int64_t)dtype_size(b_dtype), esz_c = (int64_t)dtype_size(c_dtype);
         const int hint = t81b200::g_hint_independent;
         int rc = T81B200_OK;
@@ -286,9 +286,7 @@ static int gemm_trit_local(const uint8_t *A, const float *row_scale, const void 
     }
 
     if (a_aligned && gemm_trit_tc_eligible(M, N, K)) {
-        const size_t need = gemm_trit_tc_scratch(B, b_dtype, layout, ldb, N, K, 2);
-        const bool have = workspace && workspace_bytes >= need && reinterpret_cast<uintptr_t>(workspace) % 16 == 0;
-        if (need == 0 || (have && worth_staging(M, N, K))) {
+        if (tiles) {
             const int rc = gemm_trit_tc_launch(0, 2, A, row_scale, B, b_dtype, layout, ldb, bias, C, c_dtype, ldc, M, N, K, alpha, beta,
                                                workspace, workspace_bytes, st, ctx ? ctx->n_peers : 0, ctx ? ctx->peer_C : nullptr);
             if (ctx) ctx->peers_done = rc == T81B200_OK;

@@ -538,6 +538,7 @@ gemm_trit_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 struct TcShape {
     int bn = 0, n_tiles = 0, splits = 1, a_stages = 2, b_stages = 2, b_step = 1;
     size_t smem = 0;
+    double cost = 0.0;  // pick_shape's estimate, in units of 1.7 ns
 };
 
 // Time of a 64-deep step of one activation plane at tile width bn, in units of 1.7 ns (measured with 32 to 224 steps a tile):
@@ -571,6 +572,7 @@ TcShape pick_shape(int64_t M, int64_t N, int64_t K, int planes) {
             if (t < best_t) { best_t = t; best.bn = bn; best.n_tiles = (int)n_tiles; best.splits = s; }
         }
     }
+    best.cost = best_t;
     // One barrier per chunk instead of one per step where two stages of a chunk fit (up to 224 tokens) and the planes are not
     // several (those fill the time between two barriers anyway, and do better with a deeper ring: 200 against 220 us at
     // 4096 x 4096 x 4096, fp32, 192 tokens).  With one plane: 192 tokens 408 -> 314 us at 14336 x 4096 x 4096.
@@ -758,6 +760,10 @@ int stage_planes(const void *B, int dtype, int layout, int64_t ld, int64_t token
 bool gemm_trit_tc_eligible(int64_t M, int64_t N, int64_t K) {
     return M >= 1 && N >= 1 && K >= 1 && M < (1ll << 31) && N < (1ll << 29) && K < (1ll << 31);
 }
+
+// Time of a launch without staging: 6 us of launch, set-up and last stores on top of the planner's figure (13.5 us estimated and 12.4
+// measured at 4096 x 4096 x 32, 18.8 and 20.3 at 14336 x 4096 x 80, both bf16).
+double gemm_trit_tc_estimate_us(int64_t M, int64_t N, int64_t K) { return 6.0 + 1.7e-3 * pick_shape(M, N, K, 1).cost; }
 
 // Scratch bytes for the activations: none when they are read in place.  `planes`: bf16 planes of fp32 activations.
 size_t gemm_trit_tc_scratch_most(int b_dtype, int64_t N, int64_t K, int planes) {
