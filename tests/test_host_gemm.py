@@ -1,0 +1,25 @@
+"""``gemm_ternary`` on numpy buffers at the sizes where its staging changes: single copies, pieces, helper threads."""
+
+import numpy as np
+import pytest
+
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+# B of 2 MiB and one row less and more of it (helpers on the way up), C of 1 MiB and a row more (on the way down), rows of no
+# multiple of 16 bytes, one element, and more than one piece in both directions
+@pytest.mark.parametrize("M,N,K", [(1, 1, 48), (64, 33, 48), (128, 1024, 480), (128, 1024, 528), (96, 993, 528), (512, 512, 96),
+                                   (513, 512, 96), (300, 4097, 576), (2048, 1500, 96)])
+@pytest.mark.parametrize("beta", [0.0, 0.5])
+def test_host_buffers(lib_built, M, N, K, beta):
+    from t81lib_b200 import t81lib
+    rng = np.random.default_rng(M + N + K)
+    trits = rng.integers(-1, 2, (M, K)).astype(np.int8)
+    b, c = rng.normal(size=(K, N)).astype(np.float32), rng.normal(size=(M, N)).astype(np.float32)
+    want = 1.5 * (trits.astype(np.float64) @ b) + beta * c
+    t81lib.gemm_ternary(oracle.pack_trits_rowwise(trits), b, c, M, N, K, alpha=1.5, beta=beta)
+    # fp32 activations enter with 16 mantissa bits (2^-17 each, averaging out over K), as in the device tests; relative to the
+    # product's root mean square
+    assert np.abs(c - want).max() < 5e-5 * 1.5 * float(np.sqrt(np.mean(np.abs(trits).sum(1))))
