@@ -859,12 +859,16 @@ int make_plan(Plan &pl, const PlanKey &key) {
         // 16 and 11 % behind the best for K up to 1152 and 1728, and a warp row of four K-slices is within 4 % of it for every
         // number of tokens as long as the CTAs are at most three per SM (5504 x 1536, 8 tokens: 4.65 -> 3.85 us; 9216 x 1280, 10
         // tokens: 6.25 -> 4.76).  With more than 8 tokens, where every CTA has twice the partial sums to fold, two slices are
-        // the better split for K up to 3456 (9216 x 3072, 13 tokens: 8.69 -> 7.39).
+        // the better split for K up to 3456 (9216 x 3072, 13 tokens: 8.69 -> 7.39).  Up to 8 tokens and from K = 8192 on, eight
+        // slices of small CTAs, all resident at once (2048 x 14336, 3 tokens: 9.36 -> 6.95) — for up to 2048 rows: at 4096 x 14336
+        // they win alone (10.5 -> 9.3), but in a chain of dependent launches they keep the next one from starting early and two
+        // decoder blocks lose 10 %.
         const int chunks = kl4 / 4;
         int64_t tiles32 = 0, tiles64 = 0;
         for (int i = 0; i < key.n_seg; ++i) { tiles32 += (key.M[i] + 31) / 32; tiles64 += (key.M[i] + 63) / 64; }
         if (chunks >= 4 && chunks <= 9 && tiles32 <= 3 * sms) { sw.rw = 1; sw.kw = 4; sw.s = 1; }
         else if (key.ntok > 8 && chunks >= 10 && chunks <= 18 && tiles64 <= sms) { sw.rw = 2; sw.kw = 4; sw.s = 2; }
+        else if (key.ntok <= 8 && chunks >= 43 && tiles64 >= 8 && tiles64 <= 32) { sw.rw = 2; sw.kw = 2; sw.s = 8; }
     }
     double best_t = 1e30;
     Plan best;

@@ -71,10 +71,11 @@ def test_decode_rows_off_boundaries(dev, rows, K, tokens, dtype):
 
 
 # launch shapes of short rows: K from 4 to 9 chunks with up to and past three 32-row CTAs per SM, 10 to 18 chunks with up to
-# and past one pair of 64-row CTAs per SM
+# and past one pair of 64-row CTAs per SM; long rows in eight slices, and a row too many for them
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("rows,K,tokens", [(33, 584, 1), (1000, 1728, 16), (14208, 768, 5), (14240, 768, 9), (3200, 1736, 9),
-                                           (129, 3456, 16), (9472, 1920, 12), (9536, 1920, 12)])
+                                           (129, 3456, 16), (9472, 1920, 12), (9536, 1920, 12), (449, 8208, 3),
+                                           (2048, 14336, 8), (2049, 8208, 1)])
 def test_decode_short_rows(dev, rows, K, tokens, dtype):
     from t81lib_b200 import _capi, ops
     rng = np.random.default_rng(rows + K)
