@@ -846,14 +846,15 @@ bool lay_out(Plan &pl, int fmt, int planes, int ntok, int tokpad, int rwv, int k
     return true;
 }
 
-int make_plan(Plan &pl, const PlanKey &key) {
+int make_plan(Plan &pl, const PlanKey &key, bool rules = true) {
     const int planes = key.x_dtype == T81B200_F32 ? 2 : 1;
     const int tokpad = key.ntok > 8 ? 16 : 8;
     const int64_t kl = (key.K + 47) / 48;
     const int kl4 = (int)((kl + 3) & ~(int64_t)3);
     const int sms = sm_count();
     Switches sw = switches();
-    if (key.fmt == 1 && key.bulk_x && !sw.rw) {
+    const bool forced = sw.rw != 0;
+    if (rules && key.fmt == 1 && key.bulk_x && !forced) {
         // Where bulk copies bring the activations (no warp converts them), short rows need no cluster: its fold costs about a
         // microsecond, and one CTA's copy of the activations is small.  Over 122 shapes in every launch shape the model below is
         // 16 and 11 % behind the best for K up to 1152 and 1728, and a warp row of four K-slices is within 4 % of it for every
@@ -919,6 +920,8 @@ int make_plan(Plan &pl, const PlanKey &key) {
                     best.tiles = (int)row_tiles;
                 }
             }
+    // a rule's shape need not exist (49 chunks leave the last of eight slices empty): the cost model decides then
+    if (best_t >= 1e30 && rules && !forced && sw.rw) return make_plan(pl, key, false);
     if (best_t >= 1e30) return T81B200_EALIGN;  // nothing fits: the caller uses the register-prefetch kernel
     const int rows = 32 * best.row_warps;
     int tile = 0;

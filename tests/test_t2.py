@@ -133,3 +133,21 @@ def test_t2_alpha_beta_and_strided_results(dev, dtype):
         # nothing outside the slice was touched
         assert torch.equal(wide[:, :8], before[:, :8]) and torch.equal(wide[:, 8 + out_f:], before[:, 8 + out_f:])
     assert _capi.kernel_status(reset=True) == 0
+
+
+# Every number of 192-column chunks the launch-shape rules take, and those beside them: a shape that a rule asks for and that does
+# not exist (49 chunks in eight slices) must not turn into a refusal.  Products are exact, so whole numbers come back whole.
+@pytest_gpu
+@pytest.mark.parametrize("rows,tokens", [(33, 8), (512, 1), (2048, 8), (449, 16), (2049, 5)])
+def test_every_row_length_has_a_launch_shape(dev, rows, tokens):
+    from t81lib_b200 import _capi, ops
+    gen = torch.Generator(device="cuda").manual_seed(rows)
+    for K in [192 * c for c in range(1, 76)] + [9224, 9232, 9400]:
+        trits = torch.randint(-1, 2, (rows, K), generator=gen, device=dev, dtype=torch.float32)
+        x = torch.randint(-3, 4, (tokens, K), generator=gen, device=dev).to(torch.bfloat16)
+        t2 = ops.pack_t2(ops.quantize_pack(trits, 0.5, "fixed")[0], rows, K)
+        want = (x.double() @ trits.double().t()).float()  # below 2^24: exact in fp32 in any order
+        got = ops.gemm_trit_t2([t2], [rows], x, K=K, out_dtype=torch.float32)[0]
+        assert torch.equal(got, want), K
+        assert torch.equal(ops.linear_t2(t2, rows, x, K, None, None, torch.float32), want), K
+    assert _capi.kernel_status(reset=True) == 0
