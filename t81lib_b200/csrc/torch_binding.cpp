@@ -51,6 +51,21 @@ PyObject *raise_library_error(int code) {
     return nullptr;
 }
 
+// The library's failures inside autograd travel as the Python exception they stand for: a backward runs in a worker thread of
+// torch's, which carries std::exceptions to the caller and ends the process on anything else.
+template <typename F> auto as_python_error(F &&f) {
+    try {
+        return f();
+    } catch (const LibraryError &e) {
+        const PyGILState_STATE gil = PyGILState_Ensure();
+        raise_library_error(e.code);
+        python_error error;
+        error.persist();
+        PyGILState_Release(gil);
+        throw error;
+    }
+}
+
 const float *float_ptr(const std::optional<Tensor> &t) { return t ? t->const_data_ptr<float>() : nullptr; }
 
 bool float_vector(const Tensor &t, const c10::Device &device, int64_t n) {
@@ -262,6 +277,10 @@ struct QatLinear : public torch::autograd::Function<QatLinear> {
     }
 
     static torch::autograd::variable_list backward(Context *ctx, torch::autograd::variable_list grads) {
+        return as_python_error([&] { return gradients(ctx, grads); });
+    }
+
+    static torch::autograd::variable_list gradients(Context *ctx, const torch::autograd::variable_list &grads) {
         const auto saved = ctx->get_saved_variables();
         const Tensor &x2 = saved[0], &weight = saved[1], &scale = saved[2];
         const int64_t rows = weight.size(0), cols = weight.size(1);
@@ -288,15 +307,6 @@ struct QatLinear : public torch::autograd::Function<QatLinear> {
     }
 };
 
-// The library's failures inside autograd (a worker thread in the backward) travel as C++ exceptions torch knows.
-template <typename F> auto as_torch_error(F &&f) {
-    try {
-        return f();
-    } catch (const LibraryError &e) {
-        TORCH_CHECK(false, "t81_b200 error ", e.code, ": ", t81b200_last_error());
-    }
-}
-
 std::optional<Tensor> optional_tensor(PyObject *o) {
     if (o == Py_None) return std::nullopt;
     TORCH_CHECK_TYPE(THPVariable_Check(o), "expected a tensor or None");
@@ -318,7 +328,7 @@ PyObject *qat_linear(PyObject *, PyObject *const *args, Py_ssize_t n) {
     TORCH_CHECK_VALUE(weight.dim() == 2 && weight.scalar_type() == at::kFloat && weight.is_cuda() && x.device() == weight.device() && x.dim() >= 1 &&
                           x.size(-1) == weight.size(1) && float_vector(state, weight.device(), 4),
                       "qat_linear: x and weight do not match");
-    return THPVariable_Wrap(as_torch_error([&] {
+    return THPVariable_Wrap(as_python_error([&] {
         const Tensor w = with_unit_columns(weight.detach());
         {
             OnDevice on(w.device());
