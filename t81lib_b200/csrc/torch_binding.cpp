@@ -240,7 +240,7 @@ Tensor weight_grad(const Rows &g, const Rows &x, const Tensor &w, const Tensor &
 struct QatLinear : public torch::autograd::Function<QatLinear> {
     using Context = torch::autograd::AutogradContext;
 
-    // state: the layer's four floats, the scale updated by the caller; threshold in [0, 1]
+    // x: token-major rows; state: the layer's four floats, the scale updated by the caller; threshold in [0, 1]
     static Tensor forward(Context *ctx, const Tensor &x, const Tensor &weight, const std::optional<Tensor> &bias, const Tensor &state, double threshold) {
         const c10::Device device = weight.device();
         const int64_t rows = weight.size(0), cols = weight.size(1);
@@ -253,26 +253,18 @@ struct QatLinear : public torch::autograd::Function<QatLinear> {
         check(t81b200_qat_quantize_t2(w.const_data_ptr<float>(), rows, cols, rows > 1 ? w.stride(0) : cols, (float)threshold, state.const_data_ptr<float>(),
                                       t2.mutable_data_ptr<uint8_t>(), grad_x ? t2_t.mutable_data_ptr<uint8_t>() : nullptr, scales.mutable_data_ptr<float>(),
                                       scales.numel(), stream_of(device)));
-        Tensor x2 = x.dim() == 2 ? x : x.reshape({-1, cols});
-        if (dtype_code(x2.scalar_type()) < 0) x2 = x2.to(at::kFloat);
-        x2 = with_unit_columns(x2);
         std::optional<Tensor> b = bias;
         if (b) b = b->to(device, at::kFloat).contiguous();
         Rows r;
-        TORCH_CHECK_VALUE(as_rows(x2, cols, r), "t81.nn.Linear: input does not match in_features");
-        Tensor y = product(t2, rows, cols, scales.const_data_ptr<float>(), float_ptr(b), r, {r.tokens, rows}, x2.scalar_type(), device, 2);
+        TORCH_CHECK_VALUE(as_rows(x, cols, r), "t81.nn.Linear: input does not match in_features");
+        Tensor y = product(t2, rows, cols, scales.const_data_ptr<float>(), float_ptr(b), r, {r.tokens, rows}, x.scalar_type(), device, 2);
         // the gradients use this step's scale, whatever later steps make of the layer's state
-        ctx->save_for_backward({x2, weight, scales.narrow(0, 0, 1)});
+        ctx->save_for_backward({x, weight, scales.narrow(0, 0, 1)});
         ctx->saved_data["scales"] = scales;
         ctx->saved_data["t2_t"] = t2_t;
         ctx->saved_data["bias"] = bias ? bias->requires_grad() : false;
         ctx->saved_data["weight"] = weight.requires_grad();
-        ctx->saved_data["shape"] = x.sizes().vec();
-        if (x.dim() != 2) {
-            auto shape = x.sizes().vec();
-            shape.back() = rows;
-            y = y.reshape(shape);
-        }
+        ctx->saved_data["threshold"] = threshold;
         return y;
     }
 
@@ -284,7 +276,8 @@ struct QatLinear : public torch::autograd::Function<QatLinear> {
         const auto saved = ctx->get_saved_variables();
         const Tensor &x2 = saved[0], &weight = saved[1], &scale = saved[2];
         const int64_t rows = weight.size(0), cols = weight.size(1);
-        const Tensor g = with_unit_columns(grads[0].reshape({-1, rows}).to(x2.scalar_type()));
+        if (at::GradMode::is_enabled() || !grads[0].has_storage() || grads[0].is_neg()) return recorded_gradients(ctx, grads[0], x2, weight, scale);
+        const Tensor g = with_unit_columns(grads[0]);
         const Tensor scales = ctx->saved_data["scales"].toTensor(), t2_t = ctx->saved_data["t2_t"].toTensor();
         Tensor grad_x, grad_w, grad_b;
         const bool want_w = ctx->saved_data["weight"].toBool();
@@ -293,8 +286,7 @@ struct QatLinear : public torch::autograd::Function<QatLinear> {
         if (t2_t.defined() && want_w) r = staged(r, rows, weight.device(), keep);
         if (t2_t.defined()) {
             // every mantissa bit of a float32 gradient counts here: three planes
-            grad_x = product(t2_t, cols, rows, scales.const_data_ptr<float>(), nullptr, r, {r.tokens, cols}, g.scalar_type(), weight.device(), 3)
-                         .reshape(ctx->saved_data["shape"].toIntVector());
+            grad_x = product(t2_t, cols, rows, scales.const_data_ptr<float>(), nullptr, r, {r.tokens, cols}, g.scalar_type(), weight.device(), 3);
         }
         if (want_w) grad_w = weight_grad(r, rows_of(x2), with_unit_columns(weight), scale);
         if (ctx->saved_data["bias"].toBool()) {
@@ -303,6 +295,22 @@ struct QatLinear : public torch::autograd::Function<QatLinear> {
             check(t81b200_column_sums(g.const_data_ptr(), dtype_code(g.scalar_type()), g.size(0), rows, g.size(0) > 1 ? g.stride(0) : rows,
                                       grad_b.mutable_data_ptr<float>(), stream_of(g.device())));
         }
+        return {grad_x, grad_w, grad_b, Tensor(), Tensor()};
+    }
+
+    // The same gradients in torch's operations: where they are differentiated again (create_graph) or the output's gradient is no
+    // plain memory (a batch of them under vmap).  The weight enters through its surrogate, as in the PyTorch form of the step.
+    static torch::autograd::variable_list recorded_gradients(Context *ctx, const Tensor &g, const Tensor &x, const Tensor &weight, const Tensor &scale) {
+        const double threshold = ctx->saved_data["threshold"].toDouble();
+        const Tensor ratio = weight.detach() / scale, slope = (ratio.abs() < 0.5).to(at::kFloat) * 2.0;
+        Tensor grad_x, grad_w, grad_b;
+        if (ctx->saved_data["t2_t"].toTensor().defined()) {
+            const Tensor trits = at::logical_and(ratio >= threshold, ratio > 0).to(at::kFloat) - at::logical_and(ratio <= -threshold, ratio < 0).to(at::kFloat);
+            const Tensor w = trits * scale + slope * (weight - weight.detach()).nan_to_num(0.0, 0.0, 0.0);
+            grad_x = g.matmul(w.to(g.scalar_type()));
+        }
+        if (ctx->saved_data["weight"].toBool()) grad_w = g.to(at::kFloat).t().matmul(x.to(at::kFloat)) * slope;
+        if (ctx->saved_data["bias"].toBool()) grad_b = g.sum(at::IntArrayRef{0});
         return {grad_x, grad_w, grad_b, Tensor(), Tensor()};
     }
 };
@@ -335,7 +343,14 @@ PyObject *qat_linear(PyObject *, PyObject *const *args, Py_ssize_t n) {
             check(t81b200_qat_update_scale(w.const_data_ptr(), T81B200_F32, w.size(0), w.size(1), w.size(0) > 1 ? w.stride(0) : w.size(1), (float)momentum,
                                            state.mutable_data_ptr<float>(), stream_of(w.device())));
         }
-        return QatLinear::apply(x, weight, bias, state, threshold);
+        // what the input needs on its way in and out is torch's to record; the node itself takes token-major rows
+        Tensor rows = x.dim() == 2 ? x : x.reshape({-1, weight.size(1)});
+        if (dtype_code(rows.scalar_type()) < 0) rows = rows.to(at::kFloat);
+        const Tensor y = QatLinear::apply(with_unit_columns(rows), weight, bias, state, threshold);
+        if (x.dim() == 2) return y;
+        auto shape = x.sizes().vec();
+        shape.back() = weight.size(0);
+        return y.reshape(shape);
     }));
     END_HANDLE_TH_ERRORS
 }

@@ -24,3 +24,40 @@ def test_a_library_error_in_the_backward_is_raised(Linear):
         y.sum().backward()
     layer(x).sum().backward()  # and the next step is none the worse
     assert layer.weight.grad.isfinite().all()
+
+
+def _twins(Linear, shape, dtype=torch.float32):
+    """The same layer on the device and in its PyTorch form on the CPU, and an input for each."""
+    torch.manual_seed(7)
+    layer, twin = Linear(48, 32, device="cuda").train(), Linear(48, 32).train()
+    twin.load_state_dict({k: v.cpu() for k, v in layer.state_dict().items()}, strict=False)
+    x = torch.randn(*shape, dtype=dtype)
+    return ((layer, x.cuda().requires_grad_(True)), (twin, x.clone().requires_grad_(True)))
+
+
+# a gradient penalty on the input and on the weight: derivatives of the step's gradients, against the PyTorch form
+@pytest.mark.parametrize("shape", [(20, 48), (2, 9, 48)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+def test_gradients_of_gradients(Linear, shape, dtype):
+    results = []
+    for layer, x in _twins(Linear, shape, dtype):
+        if dtype == torch.float64 and not x.is_cuda:
+            x = x.detach().float().requires_grad_(True)  # the device layer computes in float32
+        y = torch.tanh(layer(x))
+        gx, gw = torch.autograd.grad(y.sum(), [x, layer.weight], create_graph=True)
+        penalty = (gx ** 2).sum() + (gw ** 2).sum()
+        results.append([t.detach().cpu().double() for t in torch.autograd.grad(penalty, [x, layer.weight, layer.bias])])
+    for got, want in zip(*results):
+        # fp32 throughout; the device forward takes activations with 16 mantissa bits (2^-17 each)
+        assert float((got - want).norm() / want.norm()) < 4 * 2.0 ** -16
+        assert float(want.norm()) > 0
+
+
+def test_a_batch_of_output_gradients(Linear):
+    (layer, x), _ = _twins(Linear, (20, 48))
+    y, v = layer(x), torch.randn(3, 20, 32, device="cuda")
+    inputs = [x, layer.weight, layer.bias]
+    got = torch.autograd.grad(y, inputs, v, retain_graph=True, is_grads_batched=True)
+    for i in range(3):
+        for a, b in zip(got, torch.autograd.grad(y, inputs, v[i], retain_graph=True)):
+            assert float((a[i] - b).norm() / b.norm()) < 1e-6  # both exact products summed in fp32
