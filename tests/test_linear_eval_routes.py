@@ -1,0 +1,33 @@
+"""The eval-mode forward of ``Linear`` on its routes around the native call: biases that are no plain parameter."""
+
+import pytest
+import torch
+import torch.nn.utils.prune as prune
+from torch.nn.utils import parametrize
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def Linear(lib_built):
+    from t81lib_b200 import _capi
+    from t81lib_b200.nn import Linear
+    assert _capi.device_available(), _capi.last_error()
+    return Linear
+
+
+class _Doubled(torch.nn.Module):
+    def forward(self, t):
+        return 2.0 * t
+
+
+@pytest.mark.parametrize("change", [lambda l: prune.random_unstructured(l, "bias", 0.5),
+                                    lambda l: parametrize.register_parametrization(l, "bias", _Doubled())])
+def test_a_bias_that_is_no_parameter(Linear, change):
+    layer = Linear(96, 64, device="cuda").eval().requires_grad_(False)
+    x = torch.randn(4, 96, device="cuda")
+    before, bias = layer(x), layer.bias.clone()
+    change(layer)
+    assert not torch.equal(layer.bias, bias)
+    # fp32 sums of the same products with another last term
+    torch.testing.assert_close(layer(x) - layer.bias, before - bias, rtol=0, atol=1e-5)
