@@ -174,8 +174,11 @@ class TernaryTensor(torch.Tensor):
         return w
 
     def _native_product(self):
-        """The native call on the decode-stream layout, both made on first use."""
+        """The native call on the decode-stream layout, both made on first use.  None while a CUDA graph is being captured: what a
+        capture makes holds nothing until the graph is replayed, and lies in the graph's memory."""
         if self._product is None:
+            if torch.cuda.is_current_stream_capturing():
+                return None
             if self._t2 is None:
                 self._t2 = ops.pack_t2(self._packed, self._rows, self._k_actual)
             self._product = _capi.native.Product(self._t2, self._rows, self._k_actual, self._row_scale)
@@ -192,10 +195,10 @@ class TernaryTensor(torch.Tensor):
             # inference fast path: no autograd node, no device shuffling — one kernel call
             if input.shape[1] != self._k_actual:
                 raise ValueError("rhs dimension does not match ternary weight width")
-            if DECODE_STREAM_LAYOUT and self._rows > 0 and self._k_actual > 0:
-                # the weight in the decode-stream layout (made once): a quarter fewer bytes to stream, and two
-                # instructions per pair of trits to expand
-                product = self._native_product()
+            # the weight in the decode-stream layout (made once): a quarter fewer bytes to stream, and two instructions per pair
+            # of trits to expand
+            product = self._native_product() if DECODE_STREAM_LAYOUT and self._rows > 0 and self._k_actual > 0 else None
+            if product is not None:
                 if input.dtype not in (torch.float32, torch.bfloat16, torch.float16):
                     raise ValueError(f"x must be float32, bfloat16 or float16, got {input.dtype}")
                 if bias is not None and (bias.dtype != torch.float32 or bias.device != input.device or not bias.is_contiguous() or bias.requires_grad):

@@ -1,4 +1,5 @@
-"""The eval-mode forward of ``Linear`` on its routes around the native call: biases that are no plain parameter."""
+"""The eval-mode forward of ``Linear`` and ``TernaryTensor`` on the routes around the native call: biases that are no plain parameter,
+first calls inside a graph capture."""
 
 import pytest
 import torch
@@ -31,3 +32,21 @@ def test_a_bias_that_is_no_parameter(Linear, change):
     assert not torch.equal(layer.bias, bias)
     # fp32 sums of the same products with another last term
     torch.testing.assert_close(layer(x) - layer.bias, before - bias, rtol=0, atol=1e-5)
+
+
+# A weight's first call lies inside a capture: the graph's result is right on replay, and so is a call outside the graph before it
+@pytest.mark.parametrize("tokens", [4, 100, 300])
+def test_first_call_inside_a_capture(lib_built, tokens):
+    from t81lib_b200.torch import TernaryTensor
+    gen = torch.Generator(device="cuda").manual_seed(tokens)
+    w = TernaryTensor.from_float(torch.randn(512, 768, device="cuda", generator=gen), threshold=0.45)
+    x = torch.randint(-3, 4, (tokens, 768), device="cuda", generator=gen).to(torch.bfloat16)
+    want = (x.double() @ w.to_trits().double().t()).float()  # whole numbers: exact in any order
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = w.matmul_input(x, out_dtype=torch.float32)
+    assert torch.equal(w.matmul_input(x, out_dtype=torch.float32), want)
+    y.zero_()
+    graph.replay()
+    assert torch.equal(y, want)
