@@ -175,8 +175,12 @@ class TernaryTensor(torch.Tensor):
 
     def _native_product(self):
         """The native call on the decode-stream layout, both made on first use.  None while a CUDA graph is being captured: what a
-        capture makes holds nothing until the graph is replayed, and lies in the graph's memory."""
+        capture makes holds nothing until the graph is replayed, and lies in the graph's memory.  None, too, for row scales
+        that the native call cannot read where they are (``ops.gemm_trit`` converts them call by call)."""
         if self._product is None:
+            scale = self._row_scale
+            if scale is not None and (scale.dtype != torch.float32 or scale.device != self._base_device or not scale.is_contiguous()):
+                return None
             if torch.cuda.is_current_stream_capturing():
                 return None
             if self._t2 is None:

@@ -50,3 +50,19 @@ def test_first_call_inside_a_capture(lib_built, tokens):
     y.zero_()
     graph.replay()
     assert torch.equal(y, want)
+
+
+# Row scales a caller brings in another type or stride are converted, whatever the number of rows of the input
+@pytest.mark.parametrize("tokens", [4, 100, 300])
+@pytest.mark.parametrize("form", [lambda s: s.half(), lambda s: s.double(), lambda s: s.repeat_interleave(2)[::2]])
+def test_row_scales_of_another_form(lib_built, tokens, form):
+    from t81lib_b200 import ops
+    from t81lib_b200.torch import TernaryTensor
+    gen = torch.Generator(device="cuda").manual_seed(tokens)
+    trits = torch.randint(-1, 2, (512, 768), device="cuda", generator=gen).float()
+    scale = torch.randint(1, 9, (512,), device="cuda", generator=gen).float() / 8
+    packed, _ = ops.quantize_pack(trits, 0.5, "fixed")
+    w = TernaryTensor(packed, (512, 768), k_actual=768, k_limbs=16, row_scale=form(scale))
+    x = torch.randint(-3, 4, (tokens, 768), device="cuda", generator=gen).to(torch.bfloat16)
+    want = ((x.double() @ trits.double().t()) * scale).float()  # eighths of whole numbers: exact
+    assert torch.equal(w.matmul_input(x, out_dtype=torch.float32), want)
