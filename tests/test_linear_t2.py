@@ -86,3 +86,19 @@ def test_decode_short_rows(dev, rows, K, tokens, dtype):
     y = ops.linear_t2(t2, rows, x, K, None, None, torch.float32)
     assert np.abs(y.cpu().numpy() - want).max() < 2e-5 * float(np.sqrt(np.mean(want ** 2)))  # exact products, fp32 sums
     assert _capi.kernel_status(reset=True) == 0
+
+
+# fp32 rows in three planes, weights without zeros to thin the sums out: tiles alone, split over a cluster, several per cluster and
+# the widest the two accumulators of a tile leave room for
+@pytest.mark.parametrize("rows,K,tokens", [(100, 512, 33), (512, 1537, 1000), (9500, 700, 1100), (300, 4096, 257), (2048, 14336, 600)])
+def test_three_planes_are_as_exact_as_fp32(dev, rows, K, tokens):
+    from t81lib_b200 import _capi, ops
+    gen = torch.Generator(device="cuda").manual_seed(rows + K)
+    trits = torch.randint(0, 2, (rows, K), generator=gen, device=dev).float() * 2 - 1
+    t2 = ops.pack_t2(ops.quantize_pack(trits, 0.5, "fixed")[0], rows, K)
+    x = torch.randn(tokens, K, generator=gen, device=dev)
+    want = x.double() @ trits.double().t()
+    rms = lambda y: float((y.double() - want).norm() / want.norm())
+    plain = rms(torch.cat([x[i:i + 256] @ trits.t() for i in range(0, tokens, 256)]))  # fp32 on CUDA cores
+    assert rms(ops.linear_t2(t2, rows, x, K, None, None, torch.float32, 3)) <= plain
+    assert _capi.kernel_status(reset=True) == 0
