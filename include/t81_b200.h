@@ -332,7 +332,8 @@ T81B200_API int t81b200_pack_t2(const uint8_t *packed, int64_t rows, int64_t col
 /* One matrix in the decode-stream layout times any number of activation rows (token-major B, C): the streaming kernel
  * up to 16 rows, tensor-core tiles beyond.  16-bit rows that start on 16-byte boundaries are read where they are;
  * fp32 and unaligned ones are staged in the workspace (16-byte aligned, linear_t2_workspace_bytes for this very B).
- * fp32_planes: bf16 planes that fp32 activations enter the products as — 2: 16 mantissa bits, 3: all of them. */
+ * fp32_planes: bf16 planes that fp32 activations enter the products as — 2: at least 16 mantissa bits (small products keep all),
+ * 3: all of them. */
 T81B200_API size_t t81b200_linear_t2_workspace_bytes(const void *B, int b_dtype, int64_t ldb, int64_t M, int64_t N, int64_t K, int fp32_planes);
 T81B200_API int t81b200_linear_t2(const uint8_t *t2, const float *row_scale, const float *bias, void *C, int64_t M, const void *B,
                                   int b_dtype, int64_t ldb, int c_dtype, int64_t ldc, int64_t N, int64_t K, float alpha, float beta,

@@ -131,6 +131,15 @@ static bool valid_dtype(int d) { return d == T81B200_F32 || d == T81B200_BF16 ||
 // first, unless the problem is too small for that to pay (launch-bound either way: the general kernel takes it).
 static bool worth_staging(int64_t M, int64_t N, int64_t K) { return (double)M * (double)N * (double)K >= 1.6e7 && N >= 8; }
 
+// fp32 products below that line keep every mantissa bit: on the limbs the general kernel takes them, on the decode-stream layout
+// the tiles in three planes.  Two planes (16 bits) serve 17 to 128 rows in slices of the streaming kernel where those are expected
+// to be the quicker way: a slice 1.4 x (1.5 us and its weight bytes), against 5 us and 8.5 ns a column.
+static bool fp32_exact(int64_t M, int64_t N, int64_t K) {
+    if (N <= 16 || worth_staging(M, N, K)) return false;
+    const double slices = (double)((N + 15) / 16);
+    return N > T81B200_T2_MAX_ROWS || 1.4 * slices * (1.5 + (double)M * (double)K * 0.25 / 1.35e6) >= 5.0 + (double)K * 8.5e-3;
+}
+
 extern "C" size_t t81b200_gemm_trit_workspace_bytes(int b_dtype, int layout, int c_dtype, int64_t M, int64_t N,
                                                     int64_t K) {
     (void)c_dtype;
@@ -265,7 +274,7 @@ static int gemm_trit_local(const uint8_t *A, const float *row_scale, const void 
     // exchange protocol counts calls, not slices.
     const size_t need = gemm_trit_tc_scratch(B, b_dtype, layout, ldb, N, K, 2);
     const bool tiles = need == 0 || (workspace && workspace_bytes >= need && reinterpret_cast<uintptr_t>(workspace) % 16 == 0 && worth_staging(M, N, K));
-    if (a_aligned && layout == T81B200_LAYOUT_NK && K > 0 && !ctx && N <= T81B200_T2_MAX_ROWS && (!tiles || streaming_wins(M, N, K, 1.4))) {
+    if (a_aligned && layout == T81B200_LAYOUT_NK && K > 0 && !ctx && N <= T81B200_T2_MAX_ROWS && !(b_dtype == T81B200_F32 && fp32_exact(M, N, K)) && (!tiles || streaming_wins(M, N, K, 1.4))) {
         const int64_t esz_b = (int64_t)dtype_size(b_dtype), esz_c = (int64_t)dtype_size(c_dtype);
         const int hint = t81b200::g_hint_independent;
         int rc = T81B200_OK;
@@ -343,6 +352,7 @@ static bool linear_t2_streams(int b_dtype, int64_t N, int fp32_planes) {
 }
 
 extern "C" size_t t81b200_linear_t2_workspace_bytes(const void *B, int b_dtype, int64_t ldb, int64_t M, int64_t N, int64_t K, int fp32_planes) {
+    if (fp32_exact(M, N, K)) fp32_planes = 3;
     if (M <= 0 || N <= 0 || K <= 0 || b_dtype == T81B200_BF16X3 || !valid_dtype(b_dtype) || (linear_t2_streams(b_dtype, N, fp32_planes) && K <= kT2StreamingMaxK)) return 0;
     return gemm_trit_tc_scratch(B, b_dtype, T81B200_LAYOUT_NK, ldb, N, K, fp32_planes);
 }
@@ -359,6 +369,7 @@ extern "C" int t81b200_linear_t2(const uint8_t *t2, const float *row_scale, cons
     if (reinterpret_cast<uintptr_t>(t2) % 16 != 0) return fail(T81B200_EALIGN, "gemm_trit_t2: matrices must be 16-byte aligned");
     if (int rc = check_device()) return rc;
     if (N == 0) return T81B200_OK;
+    if (fp32_exact(M, N, K)) fp32_planes = 3;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (linear_t2_streams(b_dtype, N, fp32_planes)) {
         const int rc = gemv_trit_lut_launch(1, 1, &t2, &row_scale, &bias, &C, &M, B, b_dtype, ldb, c_dtype, ldc, (int)N, K, alpha, beta, st, nullptr);

@@ -102,3 +102,21 @@ def test_three_planes_are_as_exact_as_fp32(dev, rows, K, tokens):
     plain = rms(torch.cat([x[i:i + 256] @ trits.t() for i in range(0, tokens, 256)]))  # fp32 on CUDA cores
     assert rms(ops.linear_t2(t2, rows, x, K, None, None, torch.float32, 3)) <= plain
     assert _capi.kernel_status(reset=True) == 0
+
+
+# small fp32 products keep every mantissa bit on either layout: more than 128 rows, and 17 to 128 where slices of the streaming
+# kernel would be the slower way (K short against the number of slices)
+@pytest.mark.parametrize("rows,K,tokens", [(256, 256, 128), (64, 512, 100), (128, 100, 300), (16, 512, 1000), (2000, 8, 500), (64, 64, 40), (64, 128, 64)])
+def test_small_fp32_products_are_exact(dev, rows, K, tokens):
+    from t81lib_b200 import _capi, ops
+    gen = torch.Generator(device="cuda").manual_seed(rows + K)
+    trits = torch.randint(-1, 2, (rows, K), generator=gen, device=dev).float()
+    packed = ops.quantize_pack(trits, 0.5, "fixed")[0]
+    t2 = ops.pack_t2(packed, rows, K)
+    wide = torch.randn(tokens, K + 1, generator=gen, device=dev)
+    for x in (wide[:, :K].contiguous(), wide[:, 1:]):
+        want = x.double() @ trits.double().t()
+        for y in (ops.linear_t2(t2, rows, x, K, None, None, torch.float32), ops.gemm_trit(packed, x, M=rows, K=K, layout="nk")):
+            # a rounding of up to half an ulp of the running sum per addition, K of them at random
+            assert float((y.double() - want).norm() / want.norm()) < 2.0 ** -25 * (K ** 0.5 + 1)
+    assert _capi.kernel_status(reset=True) == 0
