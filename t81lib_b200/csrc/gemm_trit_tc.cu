@@ -23,11 +23,12 @@
 // Activations: 16-bit types as they are (A and B of one MMA have the same type), fp32 as bf16 planes (x = hi + lo, 16
 // mantissa bits) that are multiplied one after the other with the same expanded weights.  Rows TMA cannot read
 // (unaligned, the (K, N) layout, fp32) are first copied into token-major planes in the caller's workspace.
-// Three planes (all 24 mantissa bits, the gradients): the second and third have an accumulator of their own, 128 columns beside
-// the first one's, and the epilogue adds the two.  The tensor core cuts an accumulator off at every 16 columns instead of rounding
-// it.  With the first plane alone little is cut (trits times 8-bit mantissas mostly fit), with small terms mixed in a bit is lost
-// at every step: relative to the exact sums, trits and N(0, 1) values, 1537 x 2050 x 1000 tokens 5.1e-6 in one accumulator and
-// 4.9e-8 in two (40 us either way), 4096 x 14336 x 300 3.2e-5 and 2.6e-7; fp32 on CUDA cores has 6.6e-7 and 1.8e-6.
+// All planes but the first have an accumulator of their own beside it, and the epilogue adds the two.  The tensor core cuts an
+// accumulator off at every 16 columns instead of rounding it.  With the first plane alone little is cut (trits times 8-bit
+// mantissas mostly fit); with small terms mixed in a bit is lost at every step.  Relative to the exact sums of trits and N(0, 1)
+// values, one accumulator -> two: two planes 4096 x 14336 x 300 tokens 1.7e-5 -> 2.5e-6, at any size now (what 16 mantissa bits
+// leave); three planes (all 24 bits, the gradients) 3.2e-5 -> 2.6e-7, 1537 x 2050 x 1000 5.1e-6 -> 4.9e-8, where fp32 on CUDA
+// cores has 1.8e-6 and 6.6e-7.
 //
 // Few tiles (small matrices, short prompts): the contraction is split over S = 2 or 4 pairs of one cluster, whose
 // partial sums meet in the finishing CTA's shared memory (a tile's 32-token blocks go round the S pairs), added in rank
@@ -45,6 +46,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 
 namespace t81b200 {
 
@@ -60,7 +62,6 @@ constexpr int RAW_STAGES = 3;                    // packed weights of a chunk (1
 constexpr int MAX_SPLITS = 4;                    // clusters of up to 8 CTAs
 constexpr int NUM_THREADS = 14 * 32;
 constexpr int EPILOGUE_WARP0 = 2, CONVERTER_WARP0 = 6;
-constexpr int SMALL_COLS = 128;                       // three planes: from a tile's accumulator to the one of its second and third
 constexpr int OUT_TOKENS = 32;                        // tokens per staged output block (one tcgen05.ld of 32 columns)
 constexpr int OUT_STAGE_BYTES = OUT_TOKENS * BM * 2;  // [token][feature] block of a 16-bit output type: 8 KB
 constexpr int BARRIER_BYTES = 512;
@@ -196,14 +197,14 @@ __device__ __forceinline__ void emit_block(const TcParams &p, const TcOutMaps &o
 }
 
 // 32 columns of a tile's sums.
-template <bool THREE>
+template <int SMALL>
 __device__ __forceinline__ void load_sums(uint32_t taddr, uint32_t (&v)[32]) {
     tmem_ld32(taddr, v);
-    if constexpr (THREE) {
+    if constexpr (SMALL > 0) {
 #pragma unroll
         for (int q = 0; q < 4; ++q) {  // eight at a time: a whole block beside v costs the kernel spills
             uint32_t small[8];
-            tmem_ld8(taddr + (uint32_t)(SMALL_COLS + 8 * q), small);
+            tmem_ld8(taddr + (uint32_t)(SMALL + 8 * q), small);
 #pragma unroll
             for (int i = 0; i < 8; ++i) v[8 * q + i] = __float_as_uint(__uint_as_float(v[8 * q + i]) + __uint_as_float(small[i]));
         }
@@ -272,8 +273,8 @@ __device__ __forceinline__ void expand_chunk(const RawChunk<FMT> &raw, uint8_t *
     }
 }
 
-// THREE: three activation planes, the second and third with an accumulator of their own.
-template <typename CT, int FMT, bool THREE>
+// SMALL: 0, or with two or three activation planes the columns from a tile's accumulator to the one of all planes but the first.
+template <typename CT, int FMT, int SMALL>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_trit_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ TcOutMaps omaps, const __grid_constant__ TcParams p) {
     extern __shared__ uint8_t smem_raw[];
@@ -420,8 +421,8 @@ gemm_trit_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                             ok = mbar_wait(b_full(b.stage), b.phase);
                             if (!ok) break;
                             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                            const uint32_t d_tmem = d_tile + (THREE && pl > 0 ? (uint32_t)SMALL_COLS : 0u);
-                            const uint32_t accumulate = c > c0 || j0 > 0 || pl > (THREE ? 1 : 0) ? 1u : 0u;
+                            const uint32_t d_tmem = d_tile + (pl > 0 ? (uint32_t)SMALL : 0u);
+                            const uint32_t accumulate = c > c0 || j0 > 0 || pl > (SMALL > 0 ? 1 : 0) ? 1u : 0u;
                             if (elect_one()) {
                                 uint64_t bd = umma_desc_k(base + b_off + (uint32_t)b.stage * b_stage_bytes);
                                 uint64_t ad = umma_desc_k(a_base + (uint32_t)j0 * A_ATOM_BYTES);
@@ -465,7 +466,7 @@ gemm_trit_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 #pragma unroll 1
             for (int c = 0; c < p.bn / 32; ++c) {
                 uint32_t v[32];
-                load_sums<THREE>(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * 256 + c * 32), v);
+                load_sums<SMALL>(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * 256 + c * 32), v);
                 const uint32_t stage = out_off + (uint32_t)(out_count++ & 1) * OUT_STAGE_BYTES;
                 emit_block<CT>(p, omaps, v, row0, row, scale, bias, n0 + c * 32,
                                OutStage{gen_base + stage, base + stage, 2, threadIdx.x == EPILOGUE_WARP0 * 32, true});
@@ -526,7 +527,7 @@ gemm_trit_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                     const int to = b % S;
                     if (to == slice) continue;
                     uint32_t v[32];
-                    load_sums<THREE>(t_lane + (uint32_t)(b * 32), v);
+                    load_sums<SMALL>(t_lane + (uint32_t)(b * 32), v);
                     push_partial(v, base + partial_slot(b, S, slice, to) * 16384u + lane_row * 4u, (uint32_t)(2 * to + half));
                 }
             __syncthreads();
@@ -536,7 +537,7 @@ gemm_trit_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             const bool first = quarter == 2 && lane == 0;
             for (int b = slice + S * group; b < blocks; b += 3 * S) {
                 uint32_t v[32];
-                load_sums<THREE>(t_lane + (uint32_t)(b * 32), v);
+                load_sums<SMALL>(t_lane + (uint32_t)(b * 32), v);
                 if (S > 1) fold_partials(v, gen_base, b, S, slice, lane_row);
                 const uint32_t stage = b_off + (uint32_t)b * OUT_STAGE_BYTES;
                 emit_block<CT>(p, omaps, v, row0, own_row, own_scale, own_bias, n0 + b * 32, OutStage{gen_base + stage, base + stage, (uint32_t)(2 + group), first, false});
@@ -575,20 +576,23 @@ double step_cost(int bn, int planes) {
 
 // Tile width and split: the smallest estimate, in step_cost's units.  Fitted to every width and split of 50 shapes from
 // 512 x 528 x 256 to 14336 x 4096 x 4096: the steps; a tile 400 more; writing the last tiles out, 3 a token; sharing partial
-// sums 1300 and 3 a token.  Several planes do without the width 160: one launch at it (728 tiles, two planes, fp32 result)
-// failed with an unspecified error on a variant of this kernel, and the cause is not known.
+// sums 1300 and 3 a token.  Several planes take two accumulators a tile, so tiles that follow one another in a pair are at most
+// 128 tokens wide there (4096 x 4096 x 4096 in two planes 202 us, 208 at 256 tokens with one accumulator); wider ones only where
+// no pair has a second tile (5530 x 11021 x 249: 83 us at 128 tokens, 66 at 256).  The width 160 is left out for several planes:
+// a launch at it (728 tiles, two planes, fp32 result) failed with an unspecified error on a variant of this kernel that had other
+// issuing loops, and the cause is not known.
 TcShape pick_shape(int64_t M, int64_t N, int64_t K, int planes) {
-    const int widest = planes > 2 ? SMALL_COLS : 256;  // three planes take two accumulators a tile
-    const int64_t m_tiles = (M + 255) / 256, chunks = (K + CHUNK - 1) / CHUNK, least = (N + widest - 1) / widest;
+    const int64_t m_tiles = (M + 255) / 256, chunks = (K + CHUNK - 1) / CHUNK, wide = (N + 255) / 256, narrow = (N + 127) / 128;
+    const int64_t least = planes > 1 && wide > resident_pair_clusters(1) ? narrow : wide, most = (planes > 1 ? narrow : wide) + 8;
     TcShape best;
     double best_t = 1e30;
-    for (int64_t want = least; want <= least + 8 && want <= (N + 31) / 32; ++want) {
+    for (int64_t want = least; want <= most && want <= (N + 31) / 32; ++want) {
         const int bn = (int)(((N + want - 1) / want + 31) / 32 * 32);
         const int64_t n_tiles = (N + bn - 1) / bn, tiles = m_tiles * n_tiles;
         for (int s = 1; s <= MAX_SPLITS; ++s) {
             const int resident = resident_pair_clusters(s);
             if (s > chunks || (s > 1 && tiles > resident)) continue;
-            if (planes > 1 && bn > 128 && bn < 192) continue;
+            if (planes > 1 && bn > 128 && (bn < 192 || tiles > resident)) continue;
             const double atom = planes * step_cost(bn, planes);
             const double t = (double)((tiles + resident - 1) / resident) * (3.0 * (double)((chunks + s - 1) / s) * atom + 400.0) +
                              3.0 * bn + (s > 1 ? 1300.0 + 3.0 * bn : 0.0);
@@ -608,9 +612,9 @@ TcShape pick_shape(int64_t M, int64_t N, int64_t K, int planes) {
     return best;
 }
 
-template <typename CT, int FMT, bool THREE>
+template <typename CT, int FMT, int SMALL>
 int launch_tc(const TcShape &shape, const CUtensorMap &mw, const CUtensorMap &mx, const TcOutMaps &om, const TcParams &p, cudaStream_t st) {
-    auto kern = gemm_trit_tc_kernel<CT, FMT, THREE>;
+    auto kern = gemm_trit_tc_kernel<CT, FMT, SMALL>;
     // the shared-memory limit is a per-device attribute of the function: set it once on every device
     static std::atomic<bool> configured[64];
     int dev = 0;
@@ -639,12 +643,12 @@ int launch_tc(const TcShape &shape, const CUtensorMap &mw, const CUtensorMap &mx
     return T81B200_OK;
 }
 
-template <int FMT, bool THREE>
+template <int FMT, int SMALL>
 int launch_tc_ct(int c_dtype, const TcShape &shape, const CUtensorMap &mw, const CUtensorMap &mx, const TcOutMaps &om, const TcParams &p, cudaStream_t st) {
     switch (c_dtype) {
-        case T81B200_F32: return launch_tc<float, FMT, THREE>(shape, mw, mx, om, p, st);
-        case T81B200_BF16: return launch_tc<__nv_bfloat16, FMT, THREE>(shape, mw, mx, om, p, st);
-        case T81B200_F16: return launch_tc<__half, FMT, THREE>(shape, mw, mx, om, p, st);
+        case T81B200_F32: return launch_tc<float, FMT, SMALL>(shape, mw, mx, om, p, st);
+        case T81B200_BF16: return launch_tc<__nv_bfloat16, FMT, SMALL>(shape, mw, mx, om, p, st);
+        case T81B200_F16: return launch_tc<__half, FMT, SMALL>(shape, mw, mx, om, p, st);
     }
     return fail(T81B200_EINVAL, "gemm_trit: unknown output dtype %d", c_dtype);
 }
@@ -753,7 +757,7 @@ int resident_pair_clusters(int splits) {
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return sm_count() / (2 * splits + 1);
     int n = known[dev][splits].load(std::memory_order_relaxed);
     if (n > 0) return n;
-    auto kern = gemm_trit_tc_kernel<__nv_bfloat16, 1, false>;
+    auto kern = gemm_trit_tc_kernel<__nv_bfloat16, 1, 0>;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(2 * splits), 1, 1);
     cfg.blockDim = dim3(NUM_THREADS, 1, 1);
@@ -876,8 +880,12 @@ int gemm_trit_tc_launch(int fmt, int fp32_planes, const uint8_t *A, const float 
         }
         p.n_out_maps = 1 + n_peers;
     }
-    if (planes > 2) return fmt == 1 ? launch_tc_ct<1, true>(c_dtype, shape, mw, mx, om, p, st) : fail(T81B200_EINVAL, "gemm_trit: limbs take one or two planes");
-    return fmt == 1 ? launch_tc_ct<1, false>(c_dtype, shape, mw, mx, om, p, st) : launch_tc_ct<0, false>(c_dtype, shape, mw, mx, om, p, st);
+    auto launch = [&](auto small) {
+        constexpr int S = decltype(small)::value;
+        return fmt == 1 ? launch_tc_ct<1, S>(c_dtype, shape, mw, mx, om, p, st) : launch_tc_ct<0, S>(c_dtype, shape, mw, mx, om, p, st);
+    };
+    if (planes == 1) return launch(std::integral_constant<int, 0>{});
+    return shape.bn <= 128 ? launch(std::integral_constant<int, 128>{}) : launch(std::integral_constant<int, 256>{});
 }
 
 }  // namespace t81b200

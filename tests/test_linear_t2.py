@@ -120,3 +120,20 @@ def test_small_fp32_products_are_exact(dev, rows, K, tokens):
             # a rounding of up to half an ulp of the running sum per addition, K of them at random
             assert float((y.double() - want).norm() / want.norm()) < 2.0 ** -25 * (K ** 0.5 + 1)
     assert _capi.kernel_status(reset=True) == 0
+
+
+# two planes on either layout: 16 mantissa bits leave 2^-17 / sqrt(3) of a value at most, whatever the length of the sums; tiles of
+# one and two accumulators' widths, alone, split and several per cluster, and the rows that slices of the streaming kernel served
+@pytest.mark.parametrize("rows,K,tokens", [(512, 1537, 1000), (9500, 700, 1100), (300, 4096, 257), (2048, 14336, 250), (4096, 14336, 100), (512, 6000, 17)])
+def test_two_planes_lose_only_the_inputs_bits(dev, rows, K, tokens):
+    from t81lib_b200 import _capi, ops
+    gen = torch.Generator(device="cuda").manual_seed(rows + K)
+    trits = torch.randint(-1, 2, (rows, K), generator=gen, device=dev).float()
+    packed = ops.quantize_pack(trits, 0.5, "fixed")[0]
+    t2 = ops.pack_t2(packed, rows, K)
+    x = torch.randn(tokens, K, generator=gen, device=dev)
+    want = x.double() @ trits.double().t()
+    for y in (ops.linear_t2(t2, rows, x, K, None, None, torch.float32), ops.gemm_trit(packed, x, M=rows, K=K, layout="nk"),
+              ops.gemm_trit(packed, x.t().contiguous(), M=rows, K=K, layout="kn").t()):
+        assert float((y.double() - want).norm() / want.norm()) < 2.0 ** -17 / 3 ** 0.5
+    assert _capi.kernel_status(reset=True) == 0
