@@ -11,9 +11,13 @@
 // 16-bit operands multiply as they are: products exact, accumulation fp32.  fp32 operands are staged as three bf16
 // planes (x = p0 + p1 + p2 exactly, 24 mantissa bits) and the six plane products of weight 2^-16 and above are
 // accumulated; the three left out lie below an fp32 ulp of the product.  The five small products have an accumulator of
-// their own, and long contractions of fp32 operands are cut into segments of about 1024 tokens that meet in `out`: the tensor cores
-// cut an accumulator off at every 16-token step instead of rounding it, which over 4096 tokens in one piece left the
-// result 4.4e-6 (root mean square) from the exact sums, against 1.1e-6 for fp32 arithmetic on CUDA cores.
+// their own.  The tensor cores cut an accumulator off at every 16-token step instead of rounding it: 0.9e-9 of the result (root
+// mean square) a token, 4.4e-6 over 4096 tokens in one piece, where fp32 sums on CUDA cores had 6e-7 for 16-bit operands and
+// 1.1e-6 for fp32 ones.  So an accumulator takes a segment of the tokens only, and the epilogue warps add the segments up in
+// registers, while the MMAs fill the other accumulator: 16-bit operands 64 tokens below 512 of them, 128 below 1024 and 192 from
+// there on, fp32 ones 256; each the longest that is no further off than those sums were.  The results are 1.9e-7 to 2.9e-7 off at
+// 4096 tokens.  14336 x 4096 x 4096 tokens, bf16: 339 us in one piece, 405 in segments of 192, 375 with the weights brought to L2
+// ahead and long first segments (below); fp32 2048 x 2048 x 8192: 430 us in segments that met in memory, 329.
 //
 // Bound by the operands' way from L2: a pair tile takes 32 KB per CTA and 64 tokens of 16-bit operands.  The planes of
 // fp32 operands are loaded together, once for all six products (2050 x 1537 x 1000 tokens: 64 us with a load per product,
@@ -53,7 +57,7 @@ struct WgradParams {
     int64_t rows, cols, ldw;
     int m_tiles, n_tiles, bn;
     int planes, token_steps;          // 1 or 3 planes (6 plane products); stages of tokens
-    int segments;                     // parts of the contraction that are added up in `out` (one if split)
+    int segment, lead;                // token stages an accumulator takes before the epilogue adds it up; those of a tile's first two
     int splits, stages;
     uint32_t idesc;
     int vec;                          // 128-bit accesses to w and out
@@ -87,33 +91,40 @@ __device__ __forceinline__ void tile_at(const WgradParams &p, int tile, int &m, 
     n = r / height;
 }
 
-// A block is 32 columns of this warp's 32 rows.  VEC: a lane moves four columns of rows 4 i + lane / 8 (whole 128-byte
-// row pieces, 16 bytes a lane); otherwise one column of all 32 rows.
+// A block is 32 columns of this warp's 32 rows, half a block 16 of the rows.  VEC: a lane moves four columns of rows 4 i + lane / 8
+// (whole 128-byte row pieces, 16 bytes a lane); otherwise one column of all rows.
 template <bool VEC>
-__device__ __forceinline__ void load_weights(const WgradParams &p, int64_t row0, int64_t col0, int lane, float (&w)[32]) {
+__device__ __forceinline__ void load_weights(const WgradParams &p, int64_t row0, int64_t col0, int lane, int half, float (&w)[16]) {
     if constexpr (VEC) {
         const int64_t col = col0 + (lane & 7) * 4;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int64_t row = row0 + 4 * i + (lane >> 3);
+        for (int i = 0; i < 4; ++i) {
+            const int64_t row = row0 + 16 * half + 4 * i + (lane >> 3);
             const float4 q = row < p.rows && col < p.cols ? __ldg(reinterpret_cast<const float4 *>(p.w + row * p.ldw + col)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             w[4 * i] = q.x; w[4 * i + 1] = q.y; w[4 * i + 2] = q.z; w[4 * i + 3] = q.w;
         }
     } else {
+        const int64_t row = row0 + 16 * half;
+        const int n = col0 + lane < p.cols ? (int)(p.rows - row < 16 ? p.rows - row : 16) : 0;
+        const float *src = p.w + row * p.ldw + col0 + lane;
 #pragma unroll
-        for (int i = 0; i < 32; ++i) w[i] = row0 + i < p.rows && col0 + lane < p.cols ? __ldg(p.w + (row0 + i) * p.ldw + col0 + lane) : 0.0f;
+        for (int i = 0; i < 16; ++i, src += p.ldw) w[i] = i < n ? __ldg(src) : 0.0f;
     }
 }
 
-// The block's sums, turned through shared memory, multiplied with the slope and stored (or added to what is there).
-template <bool VEC>
-__device__ __forceinline__ void emit_block(const WgradParams &p, const uint32_t (&v)[32], const float (&w)[32], float *turn, int64_t row0, int64_t col0,
-                                           int lane, float half_scale, bool add) {
+// The block's sums into the turning buffer.
+__device__ __forceinline__ void turn_block(const float (&sum)[32], float *turn, int lane) {
     __syncwarp();
 #pragma unroll
     for (int i = 0; i < 8; ++i)
-        *reinterpret_cast<uint4 *>(turn + lane * TURN_PITCH + 4 * i) = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+        *reinterpret_cast<float4 *>(turn + lane * TURN_PITCH + 4 * i) = make_float4(sum[4 * i], sum[4 * i + 1], sum[4 * i + 2], sum[4 * i + 3]);
     __syncwarp();
+}
+
+// Half of the block in the turning buffer, multiplied with the slope and stored.
+template <bool VEC>
+__device__ __forceinline__ void emit_half(const WgradParams &p, const float (&w)[16], const float *turn, int64_t row0, int64_t col0, int lane, int half,
+                                          float half_scale) {
     // |w / scale| < 0.5 exactly where |w| < scale / 2: two floats that differ do so by 2^-24 of their size or more,
     // and a quotient 2^-24 below one half does not round up to it
     auto sloped = [&](float sum, float weight) { return sum * (fabsf(weight) < half_scale ? 2.0f : 0.0f); };
@@ -121,37 +132,41 @@ __device__ __forceinline__ void emit_block(const WgradParams &p, const uint32_t 
         const int64_t col = col0 + (lane & 7) * 4;
         if (col >= p.cols) return;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int r = 4 * i + (lane >> 3);
+        for (int i = 0; i < 4; ++i) {
+            const int r = 16 * half + 4 * i + (lane >> 3);
             if (row0 + r >= p.rows) continue;
             const float4 s = *reinterpret_cast<const float4 *>(turn + r * TURN_PITCH + (lane & 7) * 4);
-            float4 *o = reinterpret_cast<float4 *>(p.out + (row0 + r) * p.cols + col);
-            float4 y = make_float4(sloped(s.x, w[4 * i]), sloped(s.y, w[4 * i + 1]), sloped(s.z, w[4 * i + 2]), sloped(s.w, w[4 * i + 3]));
-            if (add) {
-                const float4 was = *o;
-                y.x += was.x; y.y += was.y; y.z += was.z; y.w += was.w;
-            }
-            *o = y;
+            *reinterpret_cast<float4 *>(p.out + (row0 + r) * p.cols + col) =
+                make_float4(sloped(s.x, w[4 * i]), sloped(s.y, w[4 * i + 1]), sloped(s.z, w[4 * i + 2]), sloped(s.w, w[4 * i + 3]));
         }
     } else {
-        if (col0 + lane >= p.cols) return;
+        const int64_t row = row0 + 16 * half;
+        const int n = col0 + lane < p.cols ? (int)(p.rows - row < 16 ? p.rows - row : 16) : 0;
+        float *out = p.out + row * p.cols + col0 + lane;
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-            if (row0 + i >= p.rows) break;
-            float *o = p.out + (row0 + i) * p.cols + col0 + lane;
-            *o = sloped(turn[i * TURN_PITCH + lane], w[i]) + (add ? *o : 0.0f);
-        }
+        for (int i = 0; i < 16; ++i, out += p.cols)
+            if (i < n) *out = sloped(turn[(16 * half + i) * TURN_PITCH + lane], w[i]);
     }
 }
 
-// 32 columns of the tile's sums: fp32 operands have the small products beside the large one.
-__device__ __forceinline__ void load_sums(const WgradParams &p, uint32_t taddr, uint32_t (&v)[32]) {
-    tmem_ld32(taddr, v);
-    if (p.planes > 1) {
-        uint32_t small[32];
-        tmem_ld32(taddr + 256u, small);
+// sum += 32 columns of an accumulator, 16 at a time (the sums of a whole tile take most of a thread's registers).
+__device__ __forceinline__ void add_columns(uint32_t taddr, float (&sum)[32]) {
 #pragma unroll
-        for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) + __uint_as_float(small[i]));
+    for (int h = 0; h < 2; ++h) {
+        uint32_t v[16];
+        tmem_ld16(taddr + 16u * h, v);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) sum[16 * h + i] += __uint_as_float(v[i]);
+    }
+}
+
+__device__ __forceinline__ void store_columns(uint32_t taddr, const float (&sum)[32]) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        uint32_t v[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(sum[16 * h + i]);
+        tmem_st16(taddr + 16u * h, v);
     }
 }
 
@@ -188,24 +203,24 @@ gemm_wgrad_tc_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_con
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t *>(gen_base + (tmem_slot - base));
 
-    const int total_pieces = p.m_tiles * p.n_tiles * p.segments;
+    const int total_tiles = p.m_tiles * p.n_tiles;
     const int n_clusters = (int)gridDim.x / (2 * p.splits), cluster_id = (int)blockIdx.x / (2 * p.splits);
-    // a piece of work is one segment of one tile; this pair's share of a segment: token steps, each with all plane products
-    const int parts = p.splits * p.segments;
-    auto share_begin = [&](int piece) { return (int)((int64_t)p.token_steps * (piece % p.segments * p.splits + slice) / parts); };
-    auto share_end = [&](int piece) { return (int)((int64_t)p.token_steps * (piece % p.segments * p.splits + slice + 1) / parts); };
+    // this pair's share of the tokens, in stages
+    const int s0 = (int)((int64_t)p.token_steps * slice / p.splits), s1 = (int)((int64_t)p.token_steps * (slice + 1) / p.splits);
+    auto segment_end = [&](int begin) {
+        const int end = begin + (begin - s0 < 2 * p.lead ? p.lead : p.segment);
+        return end < s1 ? end : s1;
+    };
     const int n_bufs = p.planes == 1 ? 2 : 1;  // fp32: the second buffer holds the small products
-    auto next_piece = [&](int piece) { return (piece + 1) % p.segments ? piece + 1 : piece + 1 + (n_clusters - 1) * p.segments; };
     const uint16_t pair_mask = (uint16_t)(3u << (rank & ~1u));
     const float half_scale = 0.5f * *p.scale;
 
     if (warp == 0) {
         Ring ring;
         bool ok = true;
-        for (int piece = cluster_id * p.segments; piece < total_pieces && ok; piece = next_piece(piece)) {
+        for (int tile = cluster_id; tile < total_tiles && ok; tile += n_clusters) {
             int m, n;
-            tile_at(p, piece / p.segments, m, n);
-            const int s0 = share_begin(piece), s1 = share_end(piece);
+            tile_at(p, tile, m, n);
             const int o0 = (2 * m + half) * 128, k0 = n * p.bn + half * (p.bn / 2);
             for (int s = s0; s < s1; ++s) {
                 ok = mbar_wait(empty(ring.stage), ring.phase ^ 1);
@@ -232,20 +247,21 @@ gemm_wgrad_tc_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_con
             Ring ring;
             bool ok = true;
             int it = 0;
-            for (int piece = cluster_id * p.segments; piece < total_pieces && ok; piece = next_piece(piece), ++it) {
-                const int s0 = share_begin(piece), s1 = share_end(piece);
-                const int buf = it % n_bufs;
+            // a segment of a tile after the other: `it` counts them
+            int begin = s0;
+            for (int tile = cluster_id; tile < total_tiles && ok; ++it) {
+                const int end = segment_end(begin), buf = it % n_bufs;
                 ok = mbar_wait(acc_empty(buf), ((uint32_t)(it / n_bufs) & 1u) ^ 1u);
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t d_tmem = tmem_base + (uint32_t)buf * 256u;
-                for (int s = s0; s < s1; ++s) {
+                for (int s = begin; s < end; ++s) {
                     ok = mbar_wait(full(ring.stage), ring.phase);
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint64_t ad = umma_desc_mn(base + (uint32_t)ring.stage * stage_bytes, group);
                     const uint64_t bd = umma_desc_mn(base + (uint32_t)ring.stage * stage_bytes + 2 * group, group);
-                    const uint32_t more = s != s0 ? 1u : 0u;
+                    const uint32_t more = s != begin ? 1u : 0u;
                     if (elect_one()) {  // 16 tokens: two 1 KB groups
                         if (p.planes == 1) {
 #pragma unroll
@@ -270,36 +286,73 @@ gemm_wgrad_tc_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_con
                 }
                 if (ok && elect_one()) umma_commit_pair(acc_full(buf), pair_mask);
                 __syncwarp();
+                begin = end;
+                if (begin >= s1) { begin = s0; tile += n_clusters; }
             }
             if (!ok) give_up(&g_wgrad_status, WGRAD_STATUS_MMA);
         }
-    } else {
-        const int quarter = warp & 3, first = (warp - EPILOGUE_WARP0) >> 2;
-        float *turn = reinterpret_cast<float *>(gen_base + turn_off) + (warp - EPILOGUE_WARP0) * 32 * TURN_PITCH;
+    }
+
+    // ---- epilogue: two warps per quarter of the rows, each with every other 32-column block of the tile ----
+    const bool epilogue = warp >= EPILOGUE_WARP0;
+    const int quarter = warp & 3, first = (warp - EPILOGUE_WARP0) >> 2;
+    float *turn = reinterpret_cast<float *>(gen_base + turn_off) + (warp - EPILOGUE_WARP0) * 32 * TURN_PITCH;
+    const uint32_t t_lane = tmem_base + ((uint32_t)(quarter * 32) << 16);
+    if (epilogue) {
+        constexpr int MOST = 4;  // blocks of a warp: 256 columns / 64
+        const int blocks = p.bn / 64;
         bool ok = true;
         int it = 0;
-        for (int piece = cluster_id * p.segments; piece < total_pieces && ok; piece = next_piece(piece), ++it) {
-            const int buf = it % n_bufs;
+        for (int tile = cluster_id; tile < total_tiles && ok; tile += n_clusters) {
             int m, n;
-            tile_at(p, piece / p.segments, m, n);
-            const int64_t row0 = (int64_t)(2 * m + half) * 128 + quarter * 32, col0 = (int64_t)n * p.bn;
-            float w[32];  // the weights of a block are fetched while the one before it is put out: their latency bounded this loop
-            load_weights<VEC>(p, row0, col0 + first * 32, lane, w);
-            ok = __all_sync(0xffffffffu, mbar_wait(acc_full(buf), (uint32_t)(it / n_bufs) & 1u));
-            if (!ok || p.splits > 1) break;
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            for (int c = first; c < p.bn / 32; c += 2) {
-                float next[32];
-                load_weights<VEC>(p, row0, col0 + (c + 2 < p.bn / 32 ? c + 2 : c) * 32, lane, next);
-                uint32_t v[32];
-                load_sums(p, tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * 256 + c * 32), v);
-                emit_block<VEC>(p, v, w, turn, row0, col0 + c * 32, lane, half_scale, piece % p.segments != 0);
+            tile_at(p, tile, m, n);
+            const int64_t row0 = (int64_t)(2 * m + half) * 128 + quarter * 32, col0 = (int64_t)n * p.bn + first * 32;
+            // the tile's weights on their way to L2 while its products are summed: what follows the last segment keeps the MMAs waiting
+            if (p.splits == 1 && row0 + lane < p.rows)
+                for (int c = 0; c < blocks && col0 + 64 * c < p.cols; ++c)
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(p.w + (row0 + lane) * p.ldw + col0 + 64 * c));
+            float sum[MOST][32];
 #pragma unroll
-                for (int i = 0; i < 32; ++i) w[i] = next[i];
+            for (int c = 0; c < MOST; ++c)
+#pragma unroll
+                for (int i = 0; i < 32; ++i) sum[c][i] = 0.0f;
+            for (int s = s0; s < s1; s = segment_end(s), ++it) {
+                const int buf = it % n_bufs;
+                ok = __all_sync(0xffffffffu, mbar_wait(acc_full(buf), (uint32_t)(it / n_bufs) & 1u));
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t acc = t_lane + (uint32_t)(buf * 256 + first * 32);
+#pragma unroll
+                for (int c = 0; c < MOST; ++c)
+                    if (c < blocks) {
+                        add_columns(acc + 64u * c, sum[c]);
+                        if (p.planes > 1) add_columns(acc + 64u * c + 256u, sum[c]);  // fp32: the small products beside the large one
+                    }
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive_leader(acc_empty(buf));
             }
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) mbar_arrive_leader(acc_empty(buf));
+            if (!ok) break;
+            if (p.splits > 1) {  // back to where the pairs of the cluster take them from
+#pragma unroll
+                for (int c = 0; c < MOST; ++c)
+                    if (c < blocks) store_columns(t_lane + (uint32_t)(first * 32 + 64 * c), sum[c]);
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                break;
+            }
+            float w[2][16];  // the weights of half a block are fetched while the half before it is put out: their latency bounded this loop
+            turn_block(sum[0], turn, lane);
+            load_weights<VEC>(p, row0, col0, lane, 0, w[0]);
+#pragma unroll
+            for (int c = 0; c < MOST; ++c)
+                if (c < blocks) {
+                    if (c > 0) turn_block(sum[c], turn, lane);
+                    load_weights<VEC>(p, row0, col0 + 64 * c, lane, 1, w[1]);
+                    emit_half<VEC>(p, w[0], turn, row0, col0 + 64 * c, lane, 0, half_scale);
+                    if (c + 1 < blocks) load_weights<VEC>(p, row0, col0 + 64 * (c + 1), lane, 0, w[0]);
+                    emit_half<VEC>(p, w[1], turn, row0, col0 + 64 * c, lane, 1, half_scale);
+                }
         }
         if (!ok) give_up(&g_wgrad_status, WGRAD_STATUS_EPILOGUE);
     }
@@ -308,34 +361,37 @@ gemm_wgrad_tc_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_con
     if (p.splits > 1) {
         // one tile per cluster, its tokens shared by the pairs: 32-column block b is finished by slice b % splits, the others
         // push their partial sums into its operand ring (idle once every CTA has its last MMA behind it)
-        const int quarter = warp & 3, first = (warp - EPILOGUE_WARP0) >> 2, S = p.splits, blocks = p.bn / 32;
-        const bool epi = warp >= EPILOGUE_WARP0;
-        const uint32_t t_lane = tmem_base + ((uint32_t)(quarter * 32) << 16), lane_row = (uint32_t)(quarter * 32 + lane);
+        const int S = p.splits, blocks = p.bn / 32;
+        const uint32_t lane_row = (uint32_t)(quarter * 32 + lane);
         __syncthreads();
         cluster_barrier();
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (epi)
+        if (epilogue)
             for (int b = first; b < blocks; b += 2)
                 if (b % S != slice) {
                     uint32_t v[32];
-                    load_sums(p, t_lane + (uint32_t)(b * 32), v);
+                    tmem_ld32(t_lane + (uint32_t)(b * 32), v);
                     push_partial(v, base + partial_slot(b, S, slice, b % S) * 16384u + lane_row * 4u, (uint32_t)(2 * (b % S) + half));
                 }
         __syncthreads();
         cluster_barrier();
-        if (epi) {
+        if (epilogue) {
             int m, n;
             tile_at(p, cluster_id, m, n);
-            float *turn = reinterpret_cast<float *>(gen_base + turn_off) + (warp - EPILOGUE_WARP0) * 32 * TURN_PITCH;
             const int64_t row0 = (int64_t)(2 * m + half) * 128 + quarter * 32;
             for (int b = slice + S * first; b < blocks; b += 2 * S) {
                 const int64_t col = (int64_t)n * p.bn + b * 32;
-                float w[32];
-                load_weights<VEC>(p, row0, col, lane, w);
+                float w[2][16], sums[32];
+                load_weights<VEC>(p, row0, col, lane, 0, w[0]);
+                load_weights<VEC>(p, row0, col, lane, 1, w[1]);
                 uint32_t v[32];
-                load_sums(p, t_lane + (uint32_t)(b * 32), v);
+                tmem_ld32(t_lane + (uint32_t)(b * 32), v);
                 fold_partials(v, gen_base, b, S, slice, lane_row);
-                emit_block<VEC>(p, v, w, turn, row0, col, lane, half_scale, false);
+#pragma unroll
+                for (int i = 0; i < 32; ++i) sums[i] = __uint_as_float(v[i]);
+                turn_block(sums, turn, lane);
+                emit_half<VEC>(p, w[0], turn, row0, col, lane, 0, half_scale);
+                emit_half<VEC>(p, w[1], turn, row0, col, lane, 1, half_scale);
             }
         }
     }
@@ -447,7 +503,7 @@ extern "C" int t81b200_qat_weight_grad(const void *g, int g_dtype, int64_t ldg, 
             const double t = (double)((tiles + resident - 1) / resident) * ((p.token_steps + s - 1) / s) * per_step * (bn == 256 ? 1.0 : 0.65) + (s > 1 ? 6.0 : 0.0);
             if (t < best) { best = t; p.bn = bn; p.splits = s; }
         }
-    p.segments = p.planes > 1 && p.splits == 1 ? (int)((tokens + 1023) / 1024) : 1;
+    p.segment = p.planes > 1 ? 256 / token_step(3) : (tokens < 512 ? 1 : (tokens < 1024 ? 2 : 3));  // how long: see the top
     p.n_tiles = (int)((cols + p.bn - 1) / p.bn);
     const int stage = (2 + p.bn / 128) * group_bytes(p.planes);
     const int fit = (SMEM_LIMIT - 1024 - TURN_BYTES - BARRIER_BYTES) / stage;
@@ -456,6 +512,10 @@ extern "C" int t81b200_qat_weight_grad(const void *g, int g_dtype, int64_t ldg, 
     p.vec = cols % 4 == 0 && ldw % 4 == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0 && reinterpret_cast<uintptr_t>(out) % 16 == 0 ? 1 : 0;
     const int64_t tiles = (int64_t)p.m_tiles * p.n_tiles;
     const int64_t clusters = p.splits > 1 || tiles < resident_pair_clusters(1) ? tiles : resident_pair_clusters(1);
+    // While the epilogue puts a tile out, the MMAs of the next one have two accumulators to go on with: an eighth of the tokens each
+    // where that is more, which leaves the whole tile's sums within the same bound.
+    const int eighth = (int)(tokens / 8) / token_step(p.planes);
+    p.lead = p.planes == 1 && tiles > clusters && eighth > p.segment ? eighth : p.segment;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(clusters * 2 * p.splits), 1, 1);
     cfg.blockDim = dim3(NUM_THREADS, 1, 1);

@@ -57,3 +57,19 @@ def test_weight_gradient(lib_built, tokens, rows, cols, dtype):
         assert float(err) < bound
         assert bool((got[slope == 0] == 0).all())
     assert _capi.kernel_status(reset=True) == 0
+
+
+# no further from the exact sums than fp32 on CUDA cores, whatever the number of tokens: segments of every length, in one and in
+# several accumulators a tile, tiles alone, split over a cluster and several per cluster
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("tokens,rows,cols", [(256, 512, 512), (500, 4000, 4300), (777, 1537, 1001), (1000, 2050, 1537), (4096, 1024, 1024),
+                                              (8192, 512, 512), (8192, 128, 100), (3000, 4000, 4300)])
+def test_weight_gradient_is_as_exact_as_fp32(lib_built, tokens, rows, cols, dtype):
+    from t81lib_b200 import _capi, ops
+    gen = torch.Generator(device="cuda").manual_seed(tokens + rows + cols)
+    w, scale = torch.zeros(rows, cols, device="cuda"), torch.ones(1, device="cuda")  # slope 2 everywhere
+    g, x = (torch.randn(tokens, n, device="cuda", generator=gen).to(dtype) for n in (rows, cols))
+    want = 2.0 * (g.double().t() @ x.double())
+    rms = lambda t: float((t.double() - want).norm() / want.norm())
+    assert rms(ops.qat_weight_grad(g, x, w, scale)) <= rms(2.0 * (g.float().t() @ x.float()))
+    assert _capi.kernel_status(reset=True) == 0
