@@ -278,6 +278,11 @@ T81B200_API int t81b200_exchange_signal(uint32_t *sync_local, uint32_t *const *s
  * reference. */
 T81B200_API void t81b200_hint_independent(int on);
 
+/* Decode-sized calls fetch their weights (limbs or codes, nothing else) before the kernel directly ahead of them on the
+ * stream is complete.  Behind a kernel of this library that writes weights they wait for it; behind a kernel of the
+ * caller's that does, the caller says so here, after launching it and before the call.  No counterpart in the reference. */
+T81B200_API void t81b200_weights_written(void *stream);
+
 /* Column-block copy for the column-sharded Linear: copies `rows` rows of `width_bytes`
  * bytes from src (row pitch src_pitch bytes) to dst (row pitch dst_pitch bytes) on the
  * copy engines, stream-ordered.  dst may be memory of another GPU of the same node

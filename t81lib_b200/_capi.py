@@ -25,7 +25,7 @@ EXPORTS = (
     "t81b200_device_available", "t81b200_last_error", "t81b200_version", "t81b200_quantize_pack",
     "t81b200_quantize_trits", "t81b200_unpack", "t81b200_gemm_limb", "t81b200_gemm_limb_host",
     "t81b200_gemm_trit", "t81b200_gemm_trit_host", "t81b200_gemm_trit_static", "t81b200_gemm_trit_workspace_bytes", "t81b200_kernel_status",
-    "t81b200_copy_columns", "t81b200_gemm_trit_peers", "t81b200_exchange_wait", "t81b200_hint_independent",
+    "t81b200_copy_columns", "t81b200_gemm_trit_peers", "t81b200_exchange_wait", "t81b200_hint_independent", "t81b200_weights_written",
     "t81b200_gemm_limb_auto", "t81b200_gemm_trit_auto", "t81b200_elementwise", "t81b200_elementwise_auto",
     "t81b200_release_staging", "t81b200_exchange_signal", "t81b200_gemm_trit_grouped", "t81b200_t2_bytes", "t81b200_pack_t2", "t81b200_prefers_streaming", "t81b200_gemm_trit_t2", "t81b200_gemm_trit_t2_peers", "t81b200_linear_t2_workspace_bytes", "t81b200_linear_t2", "t81b200_tq_bytes", "t81b200_packed_to_tq", "t81b200_tq_to_packed",
     "t81b200_qat_update_scale", "t81b200_qat_quantize_pack", "t81b200_qat_quantize_t2", "t81b200_qat_weight_grad_workspace_bytes", "t81b200_qat_weight_grad", "t81b200_column_sums",
@@ -112,6 +112,8 @@ def _load() -> ctypes.CDLL:
     lib.t81b200_t2_bytes.restype = i64
     lib.t81b200_pack_t2.argtypes = [vp, i64, i64, vp, vp]
     lib.t81b200_hint_independent.restype = None
+    lib.t81b200_weights_written.argtypes = [vp]
+    lib.t81b200_weights_written.restype = None
     for name in EXPORTS:
         fn = getattr(lib, name)
         if fn.restype is ctypes.c_int and name not in ("t81b200_device_available",):

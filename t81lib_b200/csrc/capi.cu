@@ -1,8 +1,12 @@
 // C ABI glue: error state, device probing and the TRIT-mode dispatcher.
 #include "common.cuh"
+#include "launch_order.cuh"
 
+#include <algorithm>
+#include <atomic>
 #include <cstring>
 #include <mutex>
+#include <vector>
 
 namespace t81b200 {
 
@@ -219,6 +223,58 @@ extern "C" int t81b200_gemm_trit_peers(const uint8_t *A, const float *row_scale,
 namespace t81b200 { extern thread_local int g_hint_independent; }
 
 extern "C" void t81b200_hint_independent(int on) { t81b200::g_hint_independent = on ? 1 : 0; }
+
+extern "C" void t81b200_weights_written(void *stream) { t81b200::note_weights_written(static_cast<cudaStream_t>(stream)); }
+
+namespace t81b200 {
+
+namespace {
+
+struct NotedStream {
+    int device;
+    const void *stream;
+    bool operator==(const NotedStream &o) const { return device == o.device && stream == o.stream; }
+};
+constexpr size_t kMostNoted = 1024;  // more streams than that with weights written and no product since: none is told apart then
+std::mutex g_noted_mu;
+std::vector<NotedStream> g_noted;
+std::atomic<size_t> g_noted_count{0};  // what a product looks at first
+bool g_noted_all = false;
+
+NotedStream noted_stream(cudaStream_t st) {
+    static thread_local char own;
+    int dev = -1;
+    (void)cudaGetDevice(&dev);
+    if (st == cudaStreamLegacy) st = nullptr;
+    return {dev, st == cudaStreamPerThread ? static_cast<const void *>(&own) : st};
+}
+
+}  // namespace
+
+void note_weights_written(cudaStream_t st) {
+    const NotedStream key = noted_stream(st);
+    std::lock_guard<std::mutex> lock(g_noted_mu);
+    if (std::find(g_noted.begin(), g_noted.end(), key) != g_noted.end()) return;
+    if (g_noted.capacity() == 0) g_noted.reserve(kMostNoted);
+    if (g_noted.size() < kMostNoted) g_noted.push_back(key);
+    else g_noted_all = true;
+    g_noted_count.store(g_noted.size(), std::memory_order_release);
+}
+
+bool take_weights_written(cudaStream_t st) {
+    if (g_noted_count.load(std::memory_order_acquire) == 0) return false;
+    const NotedStream key = noted_stream(st);
+    std::lock_guard<std::mutex> lock(g_noted_mu);
+    const auto at = std::find(g_noted.begin(), g_noted.end(), key);
+    if (at == g_noted.end()) return g_noted_all;
+    if (g_noted_all) return true;
+    *at = g_noted.back();
+    g_noted.pop_back();
+    g_noted_count.store(g_noted.size(), std::memory_order_release);
+    return true;
+}
+
+}  // namespace t81b200
 
 extern "C" int t81b200_exchange_signal(uint32_t *sync_local, uint32_t *const *sync_slots, int n_peers, void *stream) {
     if (int rc = check_device()) return rc;

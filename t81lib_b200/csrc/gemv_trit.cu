@@ -18,6 +18,7 @@
 //   MMA is free as long as both operands agree, so the activations are staged in
 //   shared memory already permuted into the register order decode_limb produces.
 #include "common.cuh"
+#include "launch_order.cuh"
 #include "tma.cuh"
 #include "exchange.cuh"
 
@@ -617,7 +618,7 @@ int launch_tma(const CUtensorMap &map, const GemvTmaParams &tp, int slices, size
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     static const bool pdl = !(getenv("T81B200_NO_PDL"));
-    cfg.numAttrs = pdl ? 2 : 1;
+    cfg.numAttrs = pdl && !take_weights_written(st) ? 2 : 1;
     T81_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, map, tp));
     return T81B200_OK;
 }

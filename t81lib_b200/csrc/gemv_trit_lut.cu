@@ -19,7 +19,7 @@
 //     fragments serve both 16-row groups of the warp.
 //   * fp32 accumulation in registers; the K-slices of a CTA meet in shared memory, the K-slices of a
 //     cluster (shapes with few rows) through distributed shared memory in rank order: deterministic,
-//     no global scratch, no atomics.  Row scales and biases are fetched into shared memory at the start.
+//     no global scratch, no atomics.  Row scales and biases are fetched into shared memory beside the activations.
 //
 // Up to three weight matrices that share their activations (q/k/v, gate/up) can be served by one launch:
 // row tiles are numbered through the segments.
@@ -42,6 +42,7 @@
 // tiles of a chunk) is contiguous in memory: one bulk copy, no tensor map.  A quarter fewer bytes than the
 // limb layout cross HBM.
 #include "common.cuh"
+#include "launch_order.cuh"
 #include "tma.cuh"
 #include "exchange.cuh"
 
@@ -366,7 +367,7 @@ gemv_trit_lut_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
     auto full_bar = [&](int st) { return bars + 8u * st; };
     auto empty_bar = [&](int st) { return bars + 8u * (p.stages + st); };
     const uint32_t x_bar = bars + 8u * (2 * p.stages);
-    const uint32_t pro_bar = x_bar + 8u * kXPieces;  // decode tables, row scales and biases have landed
+    const uint32_t lut_bar = x_bar + 8u * kXPieces, sb_bar = lut_bar + 8u;  // decode tables; row scales and biases have landed
     auto ring_offset = [&](int st) { return st < p.ring0_stages ? st * p.stage_bytes : p.ring1_offset + (st - p.ring0_stages) * p.stage_bytes; };
 
     cg::cluster_group cluster = cg::this_cluster();
@@ -401,7 +402,7 @@ gemv_trit_lut_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
     const int x_group = (chunks_cta + kXPieces - 1) / kXPieces > 0 ? (chunks_cta + kXPieces - 1) / kXPieces : 1;
     if (threadIdx.x < p.stages) { mbar_init(full_bar(threadIdx.x), 1); mbar_init(empty_bar(threadIdx.x), p.row_warps); }
     if (threadIdx.x >= kMaxStages && threadIdx.x < kMaxStages + kXPieces) mbar_init(x_bar + 8u * (threadIdx.x - kMaxStages), 1);
-    if (threadIdx.x == kMaxStages + kXPieces) mbar_init(pro_bar, 1);
+    if (threadIdx.x == kMaxStages + kXPieces) { mbar_init(lut_bar, 1); mbar_init(sb_bar, 1); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     __syncthreads();
     TRACE_STAMP(1);
@@ -473,22 +474,28 @@ gemv_trit_lut_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
                 }
                 return true;
             };
-            // decode tables (a compile-time image in global memory), row scales and biases: bulk copies, none of
-            // them the previous kernel's output.  Scales and biases that a copy cannot take (unaligned, or a tile
-            // that reaches past the last row) are fetched by the consumer threads instead.
-            if (layout_ok) {
-                uint32_t bytes = FMT == 1 ? 0u : (uint32_t)kLutBytes;
-                if (scale_by_copy) bytes += (uint32_t)rows_per_cta * 4u;
-                if (bias_by_copy) bytes += (uint32_t)rows_per_cta * 4u;
-                if (bytes) mbar_arrive_expect_tx(pro_bar, bytes);
-                else mbar_arrive(pro_bar);
-                if constexpr (FMT == 0) bulk_load(smem_u32(lut), kF16 ? &g_lut_image_f16 : &g_lut_image, (uint32_t)kLutBytes, pro_bar);
-                if (scale_by_copy) bulk_load(smem_u32(sb), S.row_scale + cta_row0, (uint32_t)rows_per_cta * 4u, pro_bar);
-                if (bias_by_copy) bulk_load(smem_u32(sb + rows_per_cta), S.bias + cta_row0, (uint32_t)rows_per_cta * 4u, pro_bar);
-            }
-            // the ring's first pass needs nothing but the weights: start it before the wait
+            // decode tables: a compile-time image in global memory
+            if constexpr (FMT == 0)
+                if (layout_ok) {
+                    mbar_arrive_expect_tx(lut_bar, (uint32_t)kLutBytes);
+                    bulk_load(smem_u32(lut), kF16 ? &g_lut_image_f16 : &g_lut_image, (uint32_t)kLutBytes, lut_bar);
+                }
+            // the ring's first pass needs nothing but the weights (never the output of the kernel directly ahead:
+            // launch_order.cuh): start it before the wait
             const int first = chunks_cta < p.stages ? chunks_cta : p.stages;
             for (int c = 0; c < first && ok; ++c) ok = load_weights(c);
+            // Row scales and biases, which a conversion directly ahead may have written, after it: only brought to L2 before
+            // (against reading them there, a decode step of 14 launches takes 1 % longer, and 3 % without the prefetch).  What a copy cannot take
+            // (unaligned, or a tile that reaches past the last row) is fetched by the consumer threads instead.
+            const uint32_t sb_bytes = (uint32_t)rows_per_cta * 4u;
+            if (scale_by_copy) bulk_prefetch(S.row_scale + cta_row0, sb_bytes);
+            if (bias_by_copy) bulk_prefetch(S.bias + cta_row0, sb_bytes);
+            if (!p.independent) asm volatile("griddepcontrol.wait;" ::: "memory");
+            const uint32_t expected = (scale_by_copy ? sb_bytes : 0u) + (bias_by_copy ? sb_bytes : 0u);
+            if (expected) mbar_arrive_expect_tx(sb_bar, expected);
+            else mbar_arrive(sb_bar);
+            if (scale_by_copy) bulk_load(smem_u32(sb), S.row_scale + cta_row0, sb_bytes, sb_bar);
+            if (bias_by_copy) bulk_load(smem_u32(sb + rows_per_cta), S.bias + cta_row0, sb_bytes, sb_bar);
             for (int c = first; c < chunks_cta && ok; ++c) ok = load_weights(c);
             if (!ok) atomicCAS(&g_lut_status, LUT_STATUS_OK, LUT_STATUS_TIMEOUT_PRODUCER);
         }
@@ -500,13 +507,6 @@ gemv_trit_lut_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
         // ---------------- consumers ----------------
         rw = warp % p.row_warps;
         kw = warp / p.row_warps;
-        // row scales and biases the producer's bulk copies do not bring (see there); absent ones are 1 and 0
-        if (!scale_by_copy)
-            for (int r = threadIdx.x; r < rows_per_cta; r += consumer_threads)
-                sb[r] = cta_row0 + r < S.M && S.row_scale ? S.row_scale[cta_row0 + r] : 1.0f;
-        if (!bias_by_copy)
-            for (int r = threadIdx.x; r < rows_per_cta; r += consumer_threads)
-                sb[rows_per_cta + r] = cta_row0 + r < S.M && S.bias ? S.bias[cta_row0 + r] : 0.0f;
         // what lies between K and the end of the CTA's padded range is zero and is written now, before the wait
         if (p.bulk_x) {
             const int zero_words = nl * 24 - (int)(valid / 2);
@@ -516,7 +516,7 @@ gemv_trit_lut_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
             }
         }
         if (p.bulk_x && threadIdx.x == 0) expect_x();
-        asm volatile("bar.sync 1, %0;" ::"r"(consumer_threads) : "memory");  // thread-written scales, zero padding, expected bytes
+        asm volatile("bar.sync 1, %0;" ::"r"(consumer_threads) : "memory");  // zero padding, expected bytes
         if (!p.independent) {
             asm volatile("griddepcontrol.wait;" ::: "memory");  // the activations may be the previous kernel's output
             asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -535,6 +535,13 @@ gemv_trit_lut_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
             stage_activations<XT, PLANES>(p, L0, nl, xs, tok_stride, plane_stride, threadIdx.x, consumer_threads);
             asm volatile("bar.sync 1, %0;" ::"r"(consumer_threads) : "memory");
         }
+        // row scales and biases the producer's bulk copies do not bring (see there), while the activations land; absent ones are 1 and 0
+        if (!scale_by_copy)
+            for (int r = threadIdx.x; r < rows_per_cta; r += consumer_threads)
+                sb[r] = cta_row0 + r < S.M && S.row_scale ? S.row_scale[cta_row0 + r] : 1.0f;
+        if (!bias_by_copy)
+            for (int r = threadIdx.x; r < rows_per_cta; r += consumer_threads)
+                sb[rows_per_cta + r] = cta_row0 + r < S.M && S.bias ? S.bias[cta_row0 + r] : 0.0f;
         TRACE_STAMP(3);
 
         int tok_off[TOKB];
@@ -542,7 +549,7 @@ gemv_trit_lut_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
         for (int b = 0; b < TOKB; ++b) tok_off[b] = (8 * b + g < p.ntok ? 8 * b + g : 0) * tok_stride + t * 24;
         const uint32_t lane_off = (uint32_t)((rw * 32 + g) * 64 + t * 16);
         const uint32_t lane_key = window | kLutAbs | (uint32_t)((lane & 15) << 3);
-        if (layout_ok) ok = __all_sync(0xffffffffu, mbar_wait(pro_bar, 0));
+        if (FMT == 0 && layout_ok) ok = __all_sync(0xffffffffu, mbar_wait(lut_bar, 0));
         // ring slot, its phase and the activation piece of chunk c, carried along instead of divided out
         // (the ring has at least k_warps slots)
         int st = kw % p.stages, xg = 0, xc = kw;
@@ -637,6 +644,7 @@ gemv_trit_lut_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
         // acc[..][b][0]: (row g, token 8b+2t), [1]: (row g, 8b+2t+1), [2]: (row g+8, 8b+2t), [3]: (row g+8, 8b+2t+1)
         // partials are kept token-major, part[kw][token][row] with rows padded by 4: the eight rows a finishing
         // thread reads are contiguous, and the four tokens a quad writes fall on different banks
+        if (!__all_sync(0xffffffffu, mbar_wait(sb_bar, 0)) && lane == 0) atomicCAS(&g_lut_status, LUT_STATUS_OK, LUT_STATUS_TIMEOUT_CONSUMER);
         float *pw = part + (size_t)kw * kTokPad * prow;
 #pragma unroll
         for (int gr = 0; gr < 2; ++gr) {
@@ -823,7 +831,7 @@ bool lay_out(Plan &pl, int fmt, int planes, int ntok, int tokpad, int rwv, int k
     // partial sums of the K-slices, and behind them the receive slots of the cluster fold (one per rank)
     const size_t part_bytes = align_up((size_t)kwv * tokpad * (rows + 4) * 4 + (s > 1 ? (size_t)tokpad * (rows + 4 * s) * 4 : 0), 128);
     const size_t sb_bytes = align_up((size_t)2 * rows * 4, 128);
-    const size_t bar_bytes = 1024;  // 2 * 48 + 1 barriers
+    const size_t bar_bytes = 1024;  // 2 * 48 + 4 + 2 barriers
     size_t off = fmt == 1 ? 0 : kWindowHi;  // no table, no window to keep free
     pl.xs_offset = (int)off; off += xs_bytes;
     pl.part_offset = (int)off; off += part_bytes;
@@ -964,7 +972,7 @@ int launch_lut(const Plan &pl, const GemvLutParams &p, cudaStream_t st) {
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = switches().pdl ? 2 : 1;
+    cfg.numAttrs = switches().pdl && !take_weights_written(st) ? 2 : 1;
     T81_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, pl.map[0], pl.map[1], pl.map[2], p));
     return T81B200_OK;
 }

@@ -10,6 +10,7 @@
 //   register r, trit h  <->  row 32 T + 16 gr + g + 8 (r % 2),  column 192 c + 48 t + 4 m + 2 (r / 2) + h;
 //   code 01 = +1, 11 = -1, 00 = 0; rows and columns past the matrix are 0.
 #include "common.cuh"
+#include "launch_order.cuh"
 
 namespace t81b200 {
 
@@ -72,5 +73,6 @@ extern "C" int t81b200_pack_t2(const uint8_t *packed, int64_t rows, int64_t cols
     pack_t2_kernel<<<(unsigned)blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(packed, rows, cols, (cols + 47) / 48 * 16, tiles32, words,
                                                                                    reinterpret_cast<uint32_t *>(t2));
     T81_LAUNCH_CHECK("pack_t2_kernel");
+    note_weights_written(static_cast<cudaStream_t>(stream));
     return T81B200_OK;
 }

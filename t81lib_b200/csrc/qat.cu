@@ -8,6 +8,7 @@
 //      no fp32 copy of the quantised weight is ever materialised (the reference builds quantized * scale in full).
 // Both read the weight once (4 bytes per weight for fp32) and write 1/3 byte per weight: HBM-bound streams.
 #include "common.cuh"
+#include "launch_order.cuh"
 
 namespace t81b200 {
 
@@ -321,6 +322,7 @@ extern "C" int t81b200_qat_quantize_pack(const void *w, int w_dtype, int64_t row
         default: return fail(T81B200_EINVAL, "qat_quantize_pack: unknown dtype %d", w_dtype);
     }
     T81_LAUNCH_CHECK("qat_quantize_pack_kernel");
+    note_weights_written(st);
     return T81B200_OK;
 }
 
@@ -341,6 +343,7 @@ extern "C" int t81b200_qat_quantize_t2(const float *w, int64_t rows, int64_t col
     else
         qat_quantize_t2_kernel<false><<<grid, 192, 0, st>>>(w, rows, cols, ld, threshold, scale, t2, t2_transposed, scale_out, n_scales);
     T81_LAUNCH_CHECK("qat_quantize_t2_kernel");
+    note_weights_written(st);
     return T81B200_OK;
 }
 

@@ -14,6 +14,7 @@
 // stores: one coalesced 128-byte warp store per chunk.
 //
 #include "common.cuh"
+#include "launch_order.cuh"
 #include "tma.cuh"
 
 #include <atomic>
@@ -290,7 +291,7 @@ quantize_pack_ring_kernel(const T *__restrict__ w, int rows, int cols, int64_t l
     __syncthreads();
     // launched with programmatic stream serialization: everything above overlaps the tail of the kernel before
     // this one in the stream; nothing below reads or writes global memory before that kernel has completed
-    // (the kernel does not release its successor early: a decode-sized product reads its weights before it waits)
+    // (the kernel does not release its successor early; a decode-sized product behind it is launched without overlap)
     asm volatile("griddepcontrol.wait;" ::: "memory");
 
     if (warp_in_cta == TEAMS * 4) {
@@ -496,6 +497,7 @@ extern "C" int t81b200_quantize_pack(const void *w, int w_dtype, int64_t rows, i
     if (reinterpret_cast<uintptr_t>(packed) % 4 != 0)
         return fail(T81B200_EALIGN, "quantize_pack: packed must be 4-byte aligned");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    note_weights_written(st);
     switch (w_dtype) {
         case T81B200_F32: return launch_quantize_pack<float>(w, rows, cols, ld, threshold, rule, packed, row_scale, st);
         case T81B200_BF16: return launch_quantize_pack<__nv_bfloat16>(w, rows, cols, ld, threshold, rule, packed, row_scale, st);

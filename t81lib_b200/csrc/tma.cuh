@@ -52,6 +52,11 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_
                  : "memory");
 }
 
+// The same bytes to L2 only.
+__device__ __forceinline__ void bulk_prefetch(const void *src, uint32_t bytes) {
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
+}
+
 struct Ring {
     int stage = 0;
     uint32_t phase = 0;

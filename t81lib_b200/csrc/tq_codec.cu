@@ -15,6 +15,7 @@
 // In the limb layout a row is a flat stream of tryte bytes, byte = t0 + 3 t1 + 9 t2 + 13: element e of a row sits
 // in byte e / 3 as digit e % 3, whatever the limb boundaries (48 trits = 16 bytes).
 #include "common.cuh"
+#include "launch_order.cuh"
 
 namespace t81b200 {
 
@@ -359,5 +360,6 @@ extern "C" int t81b200_tq_to_packed(const uint8_t *blocks, int64_t rows, int64_t
     else
         tq_to_packed_kernel<T81B200_TQ1_0><<<tq_grid(rows * runs), kWarps * 32, 0, st>>>(blocks, rows, cols, row_bytes, packed, block_scale, bpr, (int)runs, run_blocks, wide);
     T81_LAUNCH_CHECK("tq_to_packed_kernel");
+    note_weights_written(st);
     return T81B200_OK;
 }
