@@ -6,7 +6,6 @@
 #include <atomic>
 #include <cstring>
 #include <mutex>
-#include <vector>
 
 namespace t81b200 {
 
@@ -237,7 +236,7 @@ struct NotedStream {
 };
 constexpr size_t kMostNoted = 1024;  // more streams than that with weights written and no product since: none is told apart then
 std::mutex g_noted_mu;
-std::vector<NotedStream> g_noted;
+NotedStream g_noted[kMostNoted];
 std::atomic<size_t> g_noted_count{0};  // what a product looks at first
 bool g_noted_all = false;
 
@@ -254,23 +253,26 @@ NotedStream noted_stream(cudaStream_t st) {
 void note_weights_written(cudaStream_t st) {
     const NotedStream key = noted_stream(st);
     std::lock_guard<std::mutex> lock(g_noted_mu);
-    if (std::find(g_noted.begin(), g_noted.end(), key) != g_noted.end()) return;
-    if (g_noted.capacity() == 0) g_noted.reserve(kMostNoted);
-    if (g_noted.size() < kMostNoted) g_noted.push_back(key);
-    else g_noted_all = true;
-    g_noted_count.store(g_noted.size(), std::memory_order_release);
+    const size_t n = g_noted_count.load(std::memory_order_relaxed);
+    if (std::find(g_noted, g_noted + n, key) != g_noted + n) return;
+    if (n == kMostNoted) {
+        g_noted_all = true;
+        return;
+    }
+    g_noted[n] = key;
+    g_noted_count.store(n + 1, std::memory_order_release);
 }
 
 bool take_weights_written(cudaStream_t st) {
     if (g_noted_count.load(std::memory_order_acquire) == 0) return false;
     const NotedStream key = noted_stream(st);
     std::lock_guard<std::mutex> lock(g_noted_mu);
-    const auto at = std::find(g_noted.begin(), g_noted.end(), key);
-    if (at == g_noted.end()) return g_noted_all;
     if (g_noted_all) return true;
-    *at = g_noted.back();
-    g_noted.pop_back();
-    g_noted_count.store(g_noted.size(), std::memory_order_release);
+    const size_t n = g_noted_count.load(std::memory_order_relaxed);
+    NotedStream *const at = std::find(g_noted, g_noted + n, key);
+    if (at == g_noted + n) return false;
+    *at = g_noted[n - 1];
+    g_noted_count.store(n - 1, std::memory_order_release);
     return true;
 }
 

@@ -11,11 +11,9 @@
 #include <atomic>
 #include <condition_variable>
 #include <cstring>
-#include <functional>
-#include <memory>
-#include <system_error>
+#include <exception>
+#include <new>
 #include <thread>
-#include <vector>
 #if defined(__SSE2__)
 #include <emmintrin.h>
 #endif
@@ -60,20 +58,21 @@ void copy_for_device(char *dst, const char *src, size_t bytes) {
 }
 
 // Helper threads shared by all calls of the process, one job at a time; a call that finds them busy does without.  A job
-// is a function that claims its own work, so nothing depends on how many helpers take part.
+// is a function that claims its own work, so nothing depends on how many helpers take part.  Nothing here allocates or throws (the
+// callers are C entry points) but the start of a thread, which is caught.
 class Helpers {
 public:
-    // Offers `work` to the helpers; false when they are busy or cannot be started.
-    bool begin(std::function<void()> work) {
+    // Offers `work` (a function object that outlives end()) to the helpers; false when they are busy.
+    template <typename F> bool begin(F &work) {
         if (!busy_.try_lock()) return false;
         std::lock_guard<std::mutex> lock(mu_);
         try {
-            while ((int)threads_.size() < kHelpers && (int)threads_.size() + 1 < (int)std::thread::hardware_concurrency())
-                threads_.emplace_back([this] { run(); });
-        } catch (const std::system_error &) {
+            for (; count_ < kHelpers && count_ + 1 < (int)std::thread::hardware_concurrency(); ++count_) threads_[count_] = std::thread([this] { run(); });
+        } catch (const std::exception &) {
             // no more threads to be had: those there are help
         }
-        work_ = std::move(work);
+        call_ = [](void *f) { (*static_cast<F *>(f))(); };
+        work_ = &work;
         ++job_;
         wake_.notify_all();
         return true;
@@ -94,8 +93,7 @@ public:
             stopping_ = true;
             wake_.notify_all();
         }
-        for (std::thread &t : threads_) t.join();
-        threads_.clear();
+        for (; count_ > 0; --count_) threads_[count_ - 1].join();
         stopping_ = false;
     }
 
@@ -107,24 +105,29 @@ private:
             wake_.wait(lock, [&] { return stopping_ || (work_ && job_ != seen); });
             if (stopping_) return;
             seen = job_;
-            std::function<void()> work = work_;
+            void (*const call)(void *) = call_;
+            void *const work = work_;
             ++active_;
             lock.unlock();
-            work();
+            call(work);
             lock.lock();
             if (--active_ == 0) idle_.notify_all();
         }
     }
     std::mutex busy_, mu_;
     std::condition_variable wake_, idle_;
-    std::vector<std::thread> threads_;
-    std::function<void()> work_;
+    std::thread threads_[kHelpers];
+    int count_ = 0;
+    void (*call_)(void *) = nullptr;
+    void *work_ = nullptr;
     uint64_t job_ = 0;
     int active_ = 0;
     bool stopping_ = false;
 };
 Helpers &helpers() {
-    static Helpers *h = new Helpers;  // outlives every static destructor that might still copy
+    // outlives every static destructor that might still copy
+    alignas(Helpers) static unsigned char place[sizeof(Helpers)];
+    static Helpers *h = new (place) Helpers;
     return *h;
 }
 
@@ -150,11 +153,9 @@ int ensure_pinned(HostStaging &s, int way, size_t bytes, bool *fits) {
     return T81B200_OK;
 }
 
-struct Piece {
-    char *pinned, *device;
-    const char *host;
-    size_t bytes;
-};
+constexpr int kMostOperands = 3;
+constexpr size_t kUpPiece = 512u << 10;
+constexpr int kMostUpPieces = (int)(kPinnedMost / kUpPiece) + kMostOperands;
 
 int cuda_status(cudaError_t e, const char *what) {
     return e == cudaSuccess ? T81B200_OK : fail(T81B200_ECUDA, "%s failed: %s", what, cudaGetErrorString(e));
@@ -188,6 +189,7 @@ int host_staging_buffer(HostStaging &s, int which, size_t bytes) {
 }
 
 int host_upload(HostStaging &s, const HostOperand *ops, int n) {
+    if (n > kMostOperands) return fail(T81B200_ELIMIT, "host_upload: %d operands", n);
     size_t total = 0;
     for (int i = 0; i < n; ++i) total += (ops[i].bytes + 255) / 256 * 256;
     bool fits;
@@ -197,32 +199,48 @@ int host_upload(HostStaging &s, const HostOperand *ops, int n) {
             if (ops[i].bytes) T81_CUDA_TRY(cudaMemcpyAsync(ops[i].device, ops[i].host, ops[i].bytes, cudaMemcpyHostToDevice, s.stream));
         return T81B200_OK;
     }
-    const size_t piece = total < (4u << 20) ? 256u << 10 : 512u << 10;
-    std::vector<Piece> pieces;
-    size_t base = 0;
-    for (int i = 0; i < n; ++i) {
-        for (size_t at = 0; at < ops[i].bytes; at += piece)
-            pieces.push_back({s.pinned[UP] + base + at, static_cast<char *>(ops[i].device) + at, static_cast<const char *>(ops[i].host) + at,
-                              ops[i].bytes - at < piece ? ops[i].bytes - at : piece});
+    // piece j of operand i, numbered through: begins[i] is the number of the operand's first one
+    const size_t piece = total < (4u << 20) ? kUpPiece / 2 : kUpPiece;
+    size_t bases[kMostOperands];
+    int begins[kMostOperands + 1] = {0}, pieces = 0;
+    for (size_t i = 0, base = 0; i < (size_t)n; ++i) {
+        bases[i] = base;
         base += (ops[i].bytes + 255) / 256 * 256;
+        begins[i + 1] = pieces += (int)((ops[i].bytes + piece - 1) / piece);
     }
-    std::unique_ptr<std::atomic<bool>[]> moved(new std::atomic<bool>[pieces.size()]);
-    for (size_t i = 0; i < pieces.size(); ++i) moved[i].store(false, std::memory_order_relaxed);
-    std::atomic<size_t> next{0};
+    std::atomic<bool> moved[kMostUpPieces];
+    for (int i = 0; i < pieces; ++i) moved[i].store(false, std::memory_order_relaxed);
+    auto at = [&](int i, char *&pinned, char *&device, const char *&host) {  // returns the piece's size
+        int o = 0;
+        while (i >= begins[o + 1]) ++o;
+        const size_t off = (size_t)(i - begins[o]) * piece;
+        pinned = s.pinned[UP] + bases[o] + off;
+        device = static_cast<char *>(ops[o].device) + off;
+        host = static_cast<const char *>(ops[o].host) + off;
+        return ops[o].bytes - off < piece ? ops[o].bytes - off : piece;
+    };
+    std::atomic<int> next{0};
     auto move_one = [&]() {
-        const size_t i = next.fetch_add(1, std::memory_order_relaxed);
-        if (i >= pieces.size()) return false;
-        copy_for_device(pieces[i].pinned, pieces[i].host, pieces[i].bytes);
+        const int i = next.fetch_add(1, std::memory_order_relaxed);
+        if (i >= pieces) return false;
+        char *pinned, *device;
+        const char *host;
+        const size_t bytes = at(i, pinned, device, host);
+        copy_for_device(pinned, host, bytes);
         moved[i].store(true, std::memory_order_release);
         return true;
     };
-    const bool helped = total >= kHelpedUp && helpers().begin([&]() { while (move_one()) {} });
+    auto move_all = [&]() { while (move_one()) {} };
+    const bool helped = total >= kHelpedUp && helpers().begin(move_all);
     cudaError_t status = cudaSuccess;
-    for (size_t queued = 0; queued < pieces.size();) {
+    for (int queued = 0; queued < pieces;) {
         const bool more = move_one();
-        for (; queued < pieces.size() && moved[queued].load(std::memory_order_acquire); ++queued)
-            if (status == cudaSuccess)
-                status = cudaMemcpyAsync(pieces[queued].device, pieces[queued].pinned, pieces[queued].bytes, cudaMemcpyHostToDevice, s.stream);
+        for (; queued < pieces && moved[queued].load(std::memory_order_acquire); ++queued) {
+            char *pinned, *device;
+            const char *host;
+            const size_t bytes = at(queued, pinned, device, host);
+            if (status == cudaSuccess) status = cudaMemcpyAsync(device, pinned, bytes, cudaMemcpyHostToDevice, s.stream);
+        }
         if (!more) pause();
     }
     if (helped) helpers().end();
@@ -270,7 +288,8 @@ int host_download(HostStaging &s, void *host, const void *device, size_t bytes) 
         memcpy(static_cast<char *>(host) + i * piece, s.pinned[DOWN] + i * piece, size_of(i));
         return true;
     };
-    const bool helped = bytes >= kHelpedDown && helpers().begin([&]() { while (move_one(true)) {} });
+    auto move_all = [&]() { while (move_one(true)) {} };
+    const bool helped = bytes >= kHelpedDown && helpers().begin(move_all);
     cudaError_t status = cudaSuccess;
     for (int seen = 0; seen < pieces;) {
         const cudaError_t e = cudaEventQuery(s.landed[seen]);
