@@ -121,7 +121,7 @@ extern "C" int t81b200_gemm_limb_host(const uint8_t *A, const uint8_t *B, float 
     if (int rc = host_upload(*stg, ops, 3)) return rc;
     if (int rc = t81b200_gemm_limb(static_cast<const uint8_t *>(stg->dev[HostStaging::A]), static_cast<const uint8_t *>(stg->dev[HostStaging::B]),
                                    static_cast<float *>(stg->dev[HostStaging::C]), M, N, k_limbs, alpha, beta, stg->stream))
-        return rc;
+        return host_abandon(*stg, rc);
     return host_download(*stg, C, stg->dev[HostStaging::C], c_bytes);
 }
 
@@ -162,7 +162,7 @@ static int gemm_trit_host_impl(const uint8_t *A, const float *B, float *C, int64
     if (int rc = t81b200_gemm_trit(static_cast<const uint8_t *>(stg->dev[HostStaging::A]), nullptr, stg->dev[HostStaging::B], T81B200_F32,
                                    T81B200_LAYOUT_KN, N, nullptr, stg->dev[HostStaging::C], T81B200_F32, N, M, N, K, alpha, beta,
                                    stg->dev[HostStaging::WORKSPACE], stg->dev_cap[HostStaging::WORKSPACE], stg->stream))
-        return rc;
+        return host_abandon(*stg, rc);
     return host_download(*stg, C, stg->dev[HostStaging::C], c_bytes);
 }
 

@@ -195,9 +195,11 @@ int host_upload(HostStaging &s, const HostOperand *ops, int n) {
     bool fits;
     if (int rc = ensure_pinned(s, UP, total, &fits)) return rc;
     if (!fits) {
-        for (int i = 0; i < n; ++i)
-            if (ops[i].bytes) T81_CUDA_TRY(cudaMemcpyAsync(ops[i].device, ops[i].host, ops[i].bytes, cudaMemcpyHostToDevice, s.stream));
-        return T81B200_OK;
+        cudaError_t status = cudaSuccess;
+        for (int i = 0; i < n && status == cudaSuccess; ++i)
+            if (ops[i].bytes) status = cudaMemcpyAsync(ops[i].device, ops[i].host, ops[i].bytes, cudaMemcpyHostToDevice, s.stream);
+        if (status != cudaSuccess) cudaStreamSynchronize(s.stream);  // what was queued still reads the caller's memory
+        return cuda_status(status, "copy to the device");
     }
     // piece j of operand i, numbered through: begins[i] is the number of the operand's first one
     const size_t piece = total < (4u << 20) ? kUpPiece / 2 : kUpPiece;
@@ -246,6 +248,11 @@ int host_upload(HostStaging &s, const HostOperand *ops, int n) {
     if (helped) helpers().end();
     if (status != cudaSuccess) cudaStreamSynchronize(s.stream);  // what was queued still reads the page-locked buffer
     return cuda_status(status, "copy to the device");
+}
+
+int host_abandon(HostStaging &s, int code) {
+    cudaStreamSynchronize(s.stream);
+    return code;
 }
 
 int host_download(HostStaging &s, void *host, const void *device, size_t bytes) {

@@ -32,6 +32,8 @@ struct HostOperand {
 };
 // Queues the operands' copies to the device on s.stream, first to last.
 int host_upload(HostStaging &s, const HostOperand *ops, int n);
+// Ends a call that failed behind its upload: waits for the copies, which read the caller's or the page-locked memory; returns `code`.
+int host_abandon(HostStaging &s, int code);
 // Copies device memory to the host behind what s.stream holds; returns when it is there.
 int host_download(HostStaging &s, void *host, const void *device, size_t bytes);
 
