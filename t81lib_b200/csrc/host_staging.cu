@@ -172,6 +172,8 @@ int host_staging(HostStaging **out) {
 }
 
 int host_staging_ready(HostStaging &s) {
+    // page-locked operands may still be written by copies on the default stream, behind which these calls have always stood
+    T81_CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));
     if (!s.stream) T81_CUDA_TRY(cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking));
     for (cudaEvent_t &e : s.landed)
         if (!e) T81_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));

@@ -20,7 +20,7 @@ struct HostStaging {
     cudaEvent_t landed[kMaxPieces] = {nullptr};
 };
 
-// The current device's set, with its stream made on first use (call with `mu` held).
+// The current device's set, with its stream made on first use (call with `mu` held); ready: behind what the default stream holds.
 int host_staging(HostStaging **out);
 int host_staging_ready(HostStaging &s);
 int host_staging_buffer(HostStaging &s, int which, size_t bytes);

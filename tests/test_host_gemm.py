@@ -23,3 +23,23 @@ def test_host_buffers(lib_built, M, N, K, beta):
     # fp32 activations enter with 16 mantissa bits (2^-17 each, averaging out over K), as in the device tests; relative to the
     # product's root mean square
     assert np.abs(c - want).max() < 5e-5 * 1.5 * float(np.sqrt(np.mean(np.abs(trits).sum(1))))
+
+
+def test_operands_that_the_default_stream_still_writes(lib_built):
+    """A page-locked operand whose copy from the device is queued on the default stream: the call stands behind it."""
+    import torch
+    from t81lib_b200 import t81lib
+    M, N, K = 64, 96, 96
+    rng = np.random.default_rng(0)
+    trits = rng.integers(-1, 2, (M, K)).astype(np.int8)
+    a, c = oracle.pack_trits_rowwise(trits), np.zeros((M, N), np.float32)
+    b = torch.zeros(K, N, pin_memory=True)
+    there = torch.from_numpy(rng.integers(-3, 4, (K, N)).astype(np.float32)).cuda()
+    t81lib.gemm_ternary(a, b.numpy(), c, M, N, K)  # buffers and plans
+    busy = torch.ones(16384, 16384, device="cuda")
+    torch.cuda.synchronize()
+    for _ in range(4):
+        busy.mul_(1.0)  # a millisecond of work ahead of the copy
+    b.copy_(there, non_blocking=True)
+    t81lib.gemm_ternary(a, b.numpy(), c, M, N, K)
+    assert np.array_equal(c, trits.astype(np.float32) @ there.cpu().numpy())  # small whole numbers: exact
