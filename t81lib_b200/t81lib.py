@@ -14,7 +14,7 @@ LIMB semantics (python/bindings.cpp:769-810, src/linalg/gemm_cpu.cpp:8-71).
 
 from __future__ import annotations
 
-import warnings
+import ctypes
 
 import numpy as np
 import torch
@@ -79,11 +79,14 @@ def _packed_to_device(obj, rows: int, cols: int) -> torch.Tensor:
 
 
 def _host_to_device(array: np.ndarray) -> torch.Tensor:
-    """A device copy of a host array, read-only ones included (torch warns about those, and only reads here)."""
+    """A device copy of a host array.  torch warns about read-only ones; it only reads here, so it is handed a view of the same
+    memory that does not say so (switching the warning off would switch it off for every thread)."""
     out = torch.empty(array.shape, dtype=_NUMPY_DTYPES[array.dtype], device=_device())
     if array.size:
-        with warnings.catch_warnings():
-            warnings.simplefilter("ignore")
+        if not array.flags.writeable:
+            memory = (ctypes.c_ubyte * array.nbytes).from_address(array.ctypes.data)
+            out.copy_(torch.from_numpy(np.frombuffer(memory, dtype=array.dtype).reshape(array.shape)))
+        else:
             out.copy_(torch.from_numpy(array))
     return out
 

@@ -43,3 +43,27 @@ def test_operands_that_the_default_stream_still_writes(lib_built):
     b.copy_(there, non_blocking=True)
     t81lib.gemm_ternary(a, b.numpy(), c, M, N, K)
     assert np.array_equal(c, trits.astype(np.float32) @ there.cpu().numpy())  # small whole numbers: exact
+
+
+def test_read_only_operands_leave_the_warning_filters_alone(lib_built, monkeypatch):
+    """bytes and read-only arrays are taken without a warning, and without touching what other threads' warnings depend on."""
+    import warnings
+
+    import torch
+    from t81lib_b200 import t81lib
+    M, N, K = 8, 5, 96
+    rng = np.random.default_rng(1)
+    trits = rng.integers(-1, 2, (M, K)).astype(np.int8)
+    b = rng.integers(-3, 4, (K, N)).astype(np.float32)
+    from_numpy, seen = torch.from_numpy, []
+    with warnings.catch_warnings():
+        warnings.simplefilter("error")
+        filters = list(warnings.filters)
+        monkeypatch.setattr(torch, "from_numpy", lambda a: (seen.append(warnings.filters == filters), from_numpy(a))[1])
+        limbs = oracle.pack_trits_rowwise(trits)
+        limbs.flags.writeable = False
+        for a in (limbs, limbs.tobytes()):
+            c = torch.zeros(M, N, device="cuda")  # not all numpy: the general path
+            t81lib.gemm_ternary(a, b, c, M, N, K)
+            assert np.array_equal(c.cpu().numpy(), trits.astype(np.float32) @ b)
+    assert seen and all(seen)
