@@ -274,8 +274,12 @@ struct QatLinear : public torch::autograd::Function<QatLinear> {
 
     static torch::autograd::variable_list gradients(Context *ctx, const torch::autograd::variable_list &grads) {
         const auto saved = ctx->get_saved_variables();
-        const Tensor &x2 = saved[0], &weight = saved[1], &scale = saved[2];
+        const Tensor &weight = saved[1], &scale = saved[2];
         const int64_t rows = weight.size(0), cols = weight.size(1);
+        // hooks on saved tensors may hand them back elsewhere and laid out otherwise
+        const c10::Device device = grads[0].device();
+        TORCH_CHECK_VALUE(saved[0].device() == device && weight.device() == device && scale.device() == device, "saved tensors of the training step are not on ", device);
+        const Tensor x2 = with_unit_columns(saved[0]);
         if (at::GradMode::is_enabled() || !grads[0].has_storage() || grads[0].is_neg()) return recorded_gradients(ctx, grads[0], x2, weight, scale);
         const Tensor g = with_unit_columns(grads[0]);
         const Tensor scales = ctx->saved_data["scales"].toTensor(), t2_t = ctx->saved_data["t2_t"].toTensor();

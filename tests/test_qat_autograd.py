@@ -61,3 +61,27 @@ def test_a_batch_of_output_gradients(Linear):
     for i in range(3):
         for a, b in zip(got, torch.autograd.grad(y, inputs, v[i], retain_graph=True)):
             assert float((a[i] - b).norm() / b.norm()) < 1e-6  # both exact products summed in fp32
+
+
+def test_saved_tensors_that_come_back_otherwise(Linear):
+    (layer, x), _ = _twins(Linear, (20, 48))
+    v = torch.randn(20, 32, device="cuda")
+    inputs = [x, layer.weight, layer.bias]
+    want = torch.autograd.grad(layer(x), inputs, v)
+    start = layer.training_scale.clone()
+    # column by column instead of row by row
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t.t().contiguous(), lambda t: t.t()):
+        y = layer(x)
+    assert torch.equal(layer.training_scale, start)  # the same weight: the same step
+    for a, b in zip(torch.autograd.grad(y, inputs, v), want):
+        assert torch.equal(a, b)
+    # on another device: refused on the host
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t, lambda t: t.cpu()):
+        y = layer(x)
+    with pytest.raises(ValueError, match="saved tensors"):
+        y.sum().backward()
+    # and brought back from there
+    with torch.autograd.graph.save_on_cpu():
+        y = layer(x)
+    for a, b in zip(torch.autograd.grad(y, inputs, v), want):
+        assert torch.equal(a, b)
