@@ -109,7 +109,8 @@ __global__ void __launch_bounds__(256) qat_quantize_pack_kernel(const T *__restr
 
 // The rule compares w / scale, rounded, with the threshold, and keeps zeros (t81/qat.py:12-25).  Rounded division is
 // monotonic, so that is a comparison of |w| with the smallest value whose quotient reaches the threshold and is not
-// zero: bisected over the floats' bit patterns, from within four ulp of thr * scale where that brackets it.  
+// zero: bisected over the floats' bit patterns, from within four ulp of thr * scale where that brackets it.  Under a scale that is
+// not finite no quotient reaches anything (inf / inf is no number): the cut is no number then, and no weight reaches that.
 __device__ float quotient_cut(float thr, float scale) {
     auto reaches = [&](uint32_t bits) {
         const float q = __fdiv_rn(__uint_as_float(bits), scale);
@@ -118,6 +119,7 @@ __device__ float quotient_cut(float thr, float scale) {
     const uint32_t guess = __float_as_uint(__fmul_rn(thr, scale));
     uint32_t lo = guess > 4u ? guess - 4u : 0u, hi = guess + 4u;  // lo: below the cut, hi: at or above it
     if (reaches(lo) || !reaches(hi)) { lo = 0u; hi = 0x7F800000u; }
+    if (!reaches(hi)) return __uint_as_float(0x7FC00000u);
     while (hi - lo > 1u) {
         const uint32_t mid = lo + (hi - lo) / 2u;
         if (reaches(mid)) hi = mid;

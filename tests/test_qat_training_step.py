@@ -73,3 +73,18 @@ def test_weight_gradient_is_as_exact_as_fp32(lib_built, tokens, rows, cols, dtyp
     rms = lambda t: float((t.double() - want).norm() / want.norm())
     assert rms(ops.qat_weight_grad(g, x, w, scale)) <= rms(2.0 * (g.float().t() @ x.float()))
     assert _capi.kernel_status(reset=True) == 0
+
+
+# weights and scales that are not finite quantise as the division does: infinite weights keep their sign under a finite scale, and
+# nothing reaches the threshold under an infinite one
+@pytest.mark.parametrize("scale", [0.05, float("inf"), float("nan")])
+@pytest.mark.parametrize("threshold", [0.0, 0.45, 1.0])
+def test_quantiser_bytes_beyond_finite_values(lib_built, scale, threshold):
+    from t81lib_b200 import ops
+    w = np.random.default_rng(0).normal(0, 0.03, (40, 200)).astype(np.float32)
+    w.flat[:5] = [np.inf, -np.inf, np.nan, 3e38, -3e38]
+    with np.errstate(invalid="ignore", over="ignore"):
+        want = oracle.qat_quantize(w, np.float32(scale), threshold)
+    t2, t2_t, _ = ops.qat_quantize_t2(torch.from_numpy(w).cuda(), threshold, torch.tensor([scale]).cuda())
+    assert np.array_equal(t2.cpu().numpy(), oracle.pack_t2(want))
+    assert np.array_equal(t2_t.cpu().numpy(), oracle.pack_t2(np.ascontiguousarray(want.T)))
