@@ -656,14 +656,20 @@ int launch_tc_ct(int c_dtype, const TcShape &shape, const CUtensorMap &mw, const
 // Pre-pass for activations TMA cannot read in place: token-major rows of kpad elements in scratch memory.  16-bit
 // values are copied bit for bit; fp32 values become PLANES bf16 planes, plane i = bf16(x - planes before it).
 // Bound by memory: every element is read once and written once (PLANES x 2 bytes).
+// An infinity is the first plane's alone (what is left of it is no number), and a value that would round to one is
+// the largest bf16 number and the rest.
+__device__ __forceinline__ float plane_of(float r) { return isinf(r) ? r : fminf(fmaxf(r, -3.38953139e38f), 3.38953139e38f); }
+__device__ __forceinline__ float rest_of(float r, float plane) { return isinf(plane) ? 0.0f : r - plane; }
+
 template <int PLANES>
 __device__ __forceinline__ void store_planes(const float (&v)[4], __nv_bfloat16 *out, int64_t plane_elems) {
     float r[4] = {v[0], v[1], v[2], v[3]};
 #pragma unroll
     for (int pl = 0; pl < PLANES; ++pl) {
-        __nv_bfloat162 a = __floats2bfloat162_rn(r[0], r[1]), b = __floats2bfloat162_rn(r[2], r[3]);
+        const __nv_bfloat162 a = __floats2bfloat162_rn(plane_of(r[0]), plane_of(r[1])), b = __floats2bfloat162_rn(plane_of(r[2]), plane_of(r[3]));
         *reinterpret_cast<uint2 *>(out + pl * plane_elems) = make_uint2(bf162_bits(a), bf162_bits(b));
-        r[0] -= __low2float(a); r[1] -= __high2float(a); r[2] -= __low2float(b); r[3] -= __high2float(b);
+        r[0] = rest_of(r[0], __low2float(a)); r[1] = rest_of(r[1], __high2float(a));
+        r[2] = rest_of(r[2], __low2float(b)); r[3] = rest_of(r[3], __high2float(b));
     }
 }
 

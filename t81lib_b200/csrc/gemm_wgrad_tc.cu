@@ -149,14 +149,19 @@ __device__ __forceinline__ void emit_half(const WgradParams &p, const float (&w)
     }
 }
 
-// sum += 32 columns of an accumulator, 16 at a time (the sums of a whole tile take most of a thread's registers).
+// sum += 32 columns of an accumulator, 16 at a time (the sums of a whole tile take most of a thread's registers).  SMALL: the products
+// beside the large one, which say nothing where an operand is infinite (its other planes are zero).
+template <bool SMALL>
 __device__ __forceinline__ void add_columns(uint32_t taddr, float (&sum)[32]) {
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         uint32_t v[16];
         tmem_ld16(taddr + 16u * h, v);
 #pragma unroll
-        for (int i = 0; i < 16; ++i) sum[16 * h + i] += __uint_as_float(v[i]);
+        for (int i = 0; i < 16; ++i) {
+            const float x = __uint_as_float(v[i]);
+            sum[16 * h + i] += SMALL && !isfinite(x) ? 0.0f : x;
+        }
     }
 }
 
@@ -325,8 +330,8 @@ gemm_wgrad_tc_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_con
 #pragma unroll
                 for (int c = 0; c < MOST; ++c)
                     if (c < blocks) {
-                        add_columns(acc + 64u * c, sum[c]);
-                        if (p.planes > 1) add_columns(acc + 64u * c + 256u, sum[c]);  // fp32: the small products beside the large one
+                        add_columns<false>(acc + 64u * c, sum[c]);
+                        if (p.planes > 1) add_columns<true>(acc + 64u * c + 256u, sum[c]);
                     }
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();

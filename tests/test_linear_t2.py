@@ -137,3 +137,30 @@ def test_two_planes_lose_only_the_inputs_bits(dev, rows, K, tokens):
               ops.gemm_trit(packed, x.t().contiguous(), M=rows, K=K, layout="kn").t()):
         assert float((y.double() - want).norm() / want.norm()) < 2.0 ** -17 / 3 ** 0.5
     assert _capi.kernel_status(reset=True) == 0
+
+
+# an infinity among fp32 activations reaches the results as it does in fp32 arithmetic (signs kept, no number where a trit is zero), and
+# large values keep their size, on the limbs next to the largest there is (the other layout's codes are twice the trits): three planes,
+# two planes, both layouts
+@pytest.mark.parametrize("tokens,K", [(40, 96), (300, 96), (400, 1000)])
+def test_infinities_and_the_largest_values(dev, tokens, K):
+    from t81lib_b200 import ops
+    gen = torch.Generator(device="cuda").manual_seed(tokens)
+    trits = torch.randint(-1, 2, (256, K), generator=gen, device=dev).float()
+    packed = ops.quantize_pack(trits, 0.5, "fixed")[0]
+    t2 = ops.pack_t2(packed, 256, K)
+    x = torch.randn(tokens, K, generator=gen, device=dev)
+    x[1, 3], x[2, 5], x[5] = float("inf"), float("-inf"), 0.0
+    for largest in (1.5e38, 3.4e38):  # rounds to infinity in bf16; the very largest does with 16 mantissa bits too
+        x[5, 7] = -largest
+        want = x.double() @ trits.double().t()
+        outs = [ops.gemm_trit(packed, x.t().contiguous(), M=256, K=K, layout="kn").t()]
+        if largest < 1.7e38:
+            outs += [ops.linear_t2(t2, 256, x, K, None, None, torch.float32, planes) for planes in (2, 3)]
+        _compare_beyond_finite(outs, want)
+
+
+def _compare_beyond_finite(outs, want):
+    for y in outs:
+        assert torch.equal(y.isnan(), want.isnan()) and torch.equal(torch.where(y.isinf(), y, 0.0).double(), torch.where(want.isinf(), want, 0.0))
+        torch.testing.assert_close(y[5].double(), want[5], rtol=2.0 ** -16, atol=0)

@@ -88,3 +88,19 @@ def test_quantiser_bytes_beyond_finite_values(lib_built, scale, threshold):
     t2, t2_t, _ = ops.qat_quantize_t2(torch.from_numpy(w).cuda(), threshold, torch.tensor([scale]).cuda())
     assert np.array_equal(t2.cpu().numpy(), oracle.pack_t2(want))
     assert np.array_equal(t2_t.cpu().numpy(), oracle.pack_t2(np.ascontiguousarray(want.T)))
+
+
+# an infinity in either fp32 operand comes out where and as it does in fp32 arithmetic
+@pytest.mark.parametrize("tokens", [20, 600])
+def test_weight_gradient_of_infinities(lib_built, tokens):
+    from t81lib_b200 import ops
+    gen = torch.Generator(device="cuda").manual_seed(tokens)
+    w = torch.randn(70, 90, device="cuda", generator=gen) * 0.03
+    scale = w.abs().amax().reshape(1)
+    g, x = torch.randn(tokens, 70, device="cuda", generator=gen), torch.randn(tokens, 90, device="cuda", generator=gen)
+    g[3, 4], x[5, 6] = float("inf"), float("-inf")
+    want = (g.double().t() @ x.double()) * (((w / scale).abs() < 0.5).double() * 2.0)
+    got = ops.qat_weight_grad(g, x, w, scale)
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(torch.where(got.isinf(), got, 0.0).double(), torch.where(want.isinf(), want, 0.0))
+    finite = want.isfinite()
+    torch.testing.assert_close(got[finite].double(), want[finite], rtol=1e-5, atol=1e-4)  # fp32 sums of up to 600 products
