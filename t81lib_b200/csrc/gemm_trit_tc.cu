@@ -663,13 +663,15 @@ __device__ __forceinline__ float rest_of(float r, float plane) { return isinf(pl
 
 template <int PLANES>
 __device__ __forceinline__ void store_planes(const float (&v)[4], __nv_bfloat16 *out, int64_t plane_elems) {
-    float r[4] = {v[0], v[1], v[2], v[3]};
+    __nv_bfloat162 a = __floats2bfloat162_rn(plane_of(v[0]), plane_of(v[1])), b = __floats2bfloat162_rn(plane_of(v[2]), plane_of(v[3]));
+    *reinterpret_cast<uint2 *>(out) = make_uint2(bf162_bits(a), bf162_bits(b));
+    float r[4] = {rest_of(v[0], __low2float(a)), rest_of(v[1], __high2float(a)), rest_of(v[2], __low2float(b)), rest_of(v[3], __high2float(b))};
 #pragma unroll
-    for (int pl = 0; pl < PLANES; ++pl) {
-        const __nv_bfloat162 a = __floats2bfloat162_rn(plane_of(r[0]), plane_of(r[1])), b = __floats2bfloat162_rn(plane_of(r[2]), plane_of(r[3]));
+    for (int pl = 1; pl < PLANES; ++pl) {  // finite from here on
+        a = __floats2bfloat162_rn(r[0], r[1]);
+        b = __floats2bfloat162_rn(r[2], r[3]);
         *reinterpret_cast<uint2 *>(out + pl * plane_elems) = make_uint2(bf162_bits(a), bf162_bits(b));
-        r[0] = rest_of(r[0], __low2float(a)); r[1] = rest_of(r[1], __high2float(a));
-        r[2] = rest_of(r[2], __low2float(b)); r[3] = rest_of(r[3], __high2float(b));
+        r[0] -= __low2float(a); r[1] -= __high2float(a); r[2] -= __low2float(b); r[3] -= __high2float(b);
     }
 }
 
