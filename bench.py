@@ -321,7 +321,7 @@ def run_ours(args):
     # nothing is overwritten inside a step.  The last call of a step carries the flag exchange (its signal is
     # published after all earlier kernels of the stream have completed), and one wait closes the step: after it
     # every rank holds every result of the step, before the next step starts.  A consumer chained to a single
-    # Linear would need the flags on that call (about 8 us, see DESIGN.md); the stack's Linears read resident inputs.
+    # Linear would need the flags on that call (about 8 us); the stack's Linears read resident inputs.
     yd_peer = None
     if world > 1 and args.decode_shard:
         from t81lib_b200.nn.sharded import peer_order

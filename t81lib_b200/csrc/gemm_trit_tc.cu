@@ -7,7 +7,7 @@
 // halves, and each CTA keeps its 128 accumulator rows in TMEM (2 x 256 fp32 columns, double-buffered across tiles).
 // Measured against the one-CTA 128 x 256 kernel before it (bf16, weights in limbs there and in codes here):
 // 4096 x 14336 x 16384 tokens 1700 -> 1160 us (958 -> 1391 TFLOP/s in a long run under the power cap), 9216 x 3072 x 2048
-// 109 -> 86, 14336 x 4096 x 80 40.9 -> 20.3 us.
+// 109 -> 90, 14336 x 4096 x 80 40.9 -> 20.6 us.
 // What bounds the kernel is shared-memory bandwidth: a 64-deep step writes and reads 16 KB of expanded weights per CTA
 // and writes and reads the activations, against 512 clocks of MMA at 256 tokens.  Halving the activation share is what
 // the pair is for: a single CTA with a 128 x 256 tile needs 768 clocks of shared memory per 512 of MMA.
@@ -841,11 +841,11 @@ int gemm_trit_tc_launch(int fmt, int fp32_planes, const uint8_t *A, const float 
     memset(&mw, 0, sizeof mw);
     if (fmt == 0) {
         const int64_t row_bytes = (K + 47) / 48 * 16;
-        if (int rc = make_map_2d(&mw, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, A, (uint64_t)row_bytes, (uint64_t)M, (uint64_t)row_bytes, 64, BM,
+        if (int rc = make_map_2d(&mw, CU_TENSOR_MAP_DATA_TYPE_UINT8, A, (uint64_t)row_bytes, (uint64_t)M, (uint64_t)row_bytes, 64, BM,
                                  CU_TENSOR_MAP_SWIZZLE_NONE))
             return rc;
     }
-    if (int rc = make_map_2d(&mx, f16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, x_ptr, (uint64_t)K,
+    if (int rc = make_map_2d(&mx, f16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, x_ptr, (uint64_t)K,
                              (uint64_t)x_rows, (uint64_t)x_ld * 2, BK, (uint32_t)shape.bn / 2, CU_TENSOR_MAP_SWIZZLE_128B))
         return rc;
     TcParams p;
@@ -882,7 +882,7 @@ int gemm_trit_tc_launch(int fmt, int fp32_planes, const uint8_t *A, const float 
         const CUtensorMapDataType dt = c_dtype == T81B200_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
         for (int i = 0; i <= n_peers; ++i) {
             void *dst = i == 0 ? C : peer_C[i - 1];
-            if (int rc = make_map_2d(&om.m[i], dt, 2, dst, (uint64_t)M, (uint64_t)N, (uint64_t)ldc * 2, BM, OUT_TOKENS,
+            if (int rc = make_map_2d(&om.m[i], dt, dst, (uint64_t)M, (uint64_t)N, (uint64_t)ldc * 2, BM, OUT_TOKENS,
                                      CU_TENSOR_MAP_SWIZZLE_NONE))
                 return rc;
         }

@@ -19,11 +19,11 @@
 // 4096 tokens.  14336 x 4096 x 4096 tokens, bf16: 339 us in one piece, 405 in segments of 192, 375 with the weights brought to L2
 // ahead and long first segments (below); fp32 2048 x 2048 x 8192: 430 us in segments that met in memory, 329.
 //
-// Bound by the operands' way from L2: a pair tile takes 32 KB per CTA and 64 tokens of 16-bit operands.  The planes of
+// 14336 x 4096 x 4096 tokens in bf16: the tensor pipe is busy 76 % of the active cycles, L2 43 %, nothing is saturated; the rest are the
+// ends of tiles and 13 waves of them for 12.1.  A pair tile takes 32 KB per CTA and 64 tokens of 16-bit operands.  The planes of
 // fp32 operands are loaded together, once for all six products (2050 x 1537 x 1000 tokens: 64 us with a load per product,
-// 56 us this way).  Tiles
-// are walked in groups of eight row tiles so that what runs at a time shares its operands in L2.  The slope is applied in
-// the epilogue, on values that a trip through shared memory has turned into whole 128-byte rows, beside the weights.
+// 56 us this way).  Tiles are walked in groups of eight row tiles so that what runs at a time shares its operands in L2.  The slope
+// is applied in the epilogue, on values that a trip through shared memory has turned into whole 128-byte rows, beside the weights.
 #include "common.cuh"
 #include "tma.cuh"
 #include "umma.cuh"

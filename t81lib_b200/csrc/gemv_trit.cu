@@ -714,7 +714,7 @@ int gemv_trit_tma_launch(const GemvParams &base, int x_dtype, int c_dtype, cudaS
     tp.bar_offset = (int)(tp.part_offset + part_bytes);
     const size_t smem = (size_t)tp.bar_offset + 16 * (size_t)best_stages + 128;
     CUtensorMap map;
-    if (int rc = make_map_2d(&map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, base.A, (uint64_t)base.kl * 16, (uint64_t)base.M,
+    if (int rc = make_map_2d(&map, CU_TENSOR_MAP_DATA_TYPE_UINT8, base.A, (uint64_t)base.kl * 16, (uint64_t)base.M,
                              (uint64_t)base.kl * 16, 64, (uint32_t)rows, CU_TENSOR_MAP_SWIZZLE_NONE))
         return rc;
     switch (x_dtype) {

@@ -871,7 +871,7 @@ int make_plan(Plan &pl, const PlanKey &key, bool rules = true) {
         // the better split for K up to 3456 (9216 x 3072, 13 tokens: 8.69 -> 7.39).  Up to 8 tokens and from K = 8192 on, eight
         // slices of small CTAs, all resident at once (2048 x 14336, 3 tokens: 9.36 -> 6.95) — for up to 2048 rows: at 4096 x 14336
         // they win alone (10.5 -> 9.3), but in a chain of dependent launches they keep the next one from starting early and two
-        // decoder blocks lose 10 %.
+        // decoder blocks lose 10 %.  Where between the two the line belongs has not been measured.
         const int chunks = kl4 / 4;
         int64_t tiles32 = 0, tiles64 = 0;
         for (int i = 0; i < key.n_seg; ++i) { tiles32 += (key.M[i] + 31) / 32; tiles64 += (key.M[i] + 63) / 64; }
@@ -937,7 +937,7 @@ int make_plan(Plan &pl, const PlanKey &key, bool rules = true) {
         best.tile_begin[i] = tile;
         tile += (int)((key.M[i] + rows - 1) / rows);
         if (key.fmt == 1) continue;  // contiguous stages: bulk copies, no tensor map
-        if (int rc = make_map_2d(&best.map[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, key.A[i], (uint64_t)kl * 16, (uint64_t)key.M[i],
+        if (int rc = make_map_2d(&best.map[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, key.A[i], (uint64_t)kl * 16, (uint64_t)key.M[i],
                                  (uint64_t)kl * 16, 64, (uint32_t)rows, CU_TENSOR_MAP_SWIZZLE_NONE))
             return rc;
     }

@@ -1,12 +1,13 @@
-// Quantisation-aware-training forward of the ternary Linear (t81/nn/linear.py:72-99 with t81/qat.py:12-57 of the
-// reference), the two steps that touch every weight fused into two streaming kernels:
-//   1. the running scale: candidate = max |w| over the whole weight, clamped to >= 1e-6, blended into the stored
-//      scale with momentum 0.99 (_update_training_scale) — one reduction kernel, the blend done by the last CTA;
-//   2. quantise + pack: trit = Q(w / scale, threshold) with the reference's rule (clamp to [-1, 1], |.| >= threshold
-//      keeps the sign), written straight into the packed-limb layout, and the scale broadcast into a per-row
-//      vector — so the forward product runs on the packed-trit matmul kernels with that vector as row scale and
-//      no fp32 copy of the quantised weight is ever materialised (the reference builds quantized * scale in full).
-// Both read the weight once (4 bytes per weight for fp32) and write 1/3 byte per weight: HBM-bound streams.
+// Passes over the weight of the ternary Linear's training step (t81/nn/linear.py:72-99 with t81/qat.py:12-57 of the reference), and
+// the bias gradient:
+//   absmax_ema_kernel       the running scale: candidate = max |w| over the whole weight, clamped to >= 1e-6, blended into the stored
+//                           scale with momentum 0.99 (_update_training_scale) — one reduction, the blend done by the last CTA;
+//   qat_quantize_t2_kernel  trit = Q(w / scale, threshold) with the reference's rule (clamp to [-1, 1], |.| >= threshold keeps the sign)
+//                           straight into the decode-stream layout of the weight (forward) and of its transpose (input gradient), and
+//                           the scale as a vector of row scales: no fp32 copy of the quantised weight is ever made;
+//   qat_quantize_pack_kernel  the same quantiser into limbs, for callers of the C interface;
+//   column_sums_kernel      the output gradient summed over the tokens.
+// The first two read the weight once each (4 bytes per weight) and are bound by memory.
 #include "common.cuh"
 #include "launch_order.cuh"
 

@@ -98,9 +98,8 @@ inline int make_map(CUtensorMap *map, CUtensorMapDataType dt, int rank, const vo
     }
 }
 
-inline int make_map_2d(CUtensorMap *map, CUtensorMapDataType dt, size_t elem, const void *ptr, uint64_t inner, uint64_t outer,
+inline int make_map_2d(CUtensorMap *map, CUtensorMapDataType dt, const void *ptr, uint64_t inner, uint64_t outer,
                 uint64_t row_stride_bytes, uint32_t box_inner, uint32_t box_outer, CUtensorMapSwizzle swz) {
-    (void)elem;
     const cuuint64_t dims[2] = {inner, outer}, strides[1] = {row_stride_bytes};
     const cuuint32_t box[2] = {box_inner, box_outer};
     return make_map(map, dt, 2, ptr, dims, strides, box, swz);

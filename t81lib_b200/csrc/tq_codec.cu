@@ -34,7 +34,7 @@ __host__ __device__ constexpr int block_bytes(int format) { return format == T81
 // (trytes) and halfwords (blocks start on even bytes), each byte once; buffers that start on odd addresses (`wide` false)
 // are taken byte by byte.  Bound by instructions.
 // 14336 x 4096 TQ1_0 out and back: 349 us byte at a time (one CTA per block), 100 us with three blocks a warp and digits
-// by arithmetic, 61 us with twelve, 45 us now; 65 MB cross memory (10 us).
+// by arithmetic, 61 us with twelve, 49 us now (27 out, 22 in); 65 MB cross memory (10 us).
 constexpr int kRunBlocks = 9;
 constexpr int kPieces = kRunBlocks / 3;        // 256 trytes each: eight per lane
 constexpr int kBlockPitch = 76;                // words of digits from one block to the next
