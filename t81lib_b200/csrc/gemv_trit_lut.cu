@@ -125,6 +125,7 @@ struct GemvLutParams {
     int stages, stage_bytes;
     int ring0_stages;        // ring slots [0, ring0_stages) lie at offset 0, the others at ring1_offset
     int ring1_offset, xs_offset, part_offset, sb_offset, bar_offset;
+    uint32_t ntok_inv, row_blocks_inv, span_blocks_inv;  // inverse(d) of: ntok; eights of rows of a CTA; those that one CTA of a cluster finishes
     int vec_x;               // 1: rows of X start on 16-byte boundaries
     int bulk_x;              // 1: 16-bit activations, 16-byte aligned rows, K % 8 == 0: fetched by bulk copies
     int independent;         // 1: reads nothing the previous kernel of the stream wrote
@@ -136,6 +137,12 @@ struct GemvLutParams {
     uint32_t shl[8];         // FMT 1: 4^j.  Multiplying by a launch-time constant instead of shifting by a literal puts
                              // the shifts of the decode on the multiply-add pipe, beside the masks on the logic pipe
 };
+
+// i / d as (i * inverse(d)) >> 16, exact for i * (d - 1) < 65536: a division by a launch-time number costs 100 ns, and the kernel
+// has one on its way to the activations and two behind its last multiply: 14 products of two decoder blocks (8 tokens) 104.6 -> 102.3 us
+// without them and with the copies planned before the wait.
+__host__ __device__ constexpr uint32_t inverse(uint32_t d) { return (65535u + d) / d; }
+__device__ __forceinline__ int divided(int i, uint32_t inv) { return (int)(((uint32_t)i * inv) >> 16); }
 
 // fp16 activations multiply as fp16, everything else as bf16 (fp32 in two planes); weights are exact in both.
 template <bool F16>
@@ -431,16 +438,19 @@ gemv_trit_lut_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
             else mbar_arrive(x_bar + 8u * j);
         }
     };
-    auto issue_x = [&](int who, int n_who) {  // copies who, who + n_who, ... in piece order
-        const uint16_t *X = static_cast<const uint16_t *>(p.X);  // either 16-bit type
-        for (int i = who; i < kXPieces * p.ntok; i += n_who) {
-            const int j = i / p.ntok, tok = i - j * p.ntok;
-            int e0, e1;
-            x_piece(j, e0, e1);
-            if (e1 > e0)
-                bulk_load(smem_u32(xs + tok * tok_stride + e0 / 2), X + (int64_t)tok * p.ldx + (int64_t)L0 * 48 + e0,
-                          (uint32_t)(e1 - e0) * 2u, x_bar + 8u * j);
-        }
+    // Lane l of warp w has copy w + l * warps, in piece order; where from and where to is worked out before the wait for the
+    // kernel ahead.
+    struct { uint32_t dst, bytes, bar; const uint16_t *src; } x_copy = {0u, 0u, 0u, nullptr};
+    auto plan_x = [&](int i) {
+        x_copy.bytes = 0u;
+        if (i >= kXPieces * p.ntok) return;
+        const int j = divided(i, p.ntok_inv), tok = i - j * p.ntok;
+        int e0, e1;
+        x_piece(j, e0, e1);
+        x_copy.bytes = (uint32_t)(e1 - e0) * 2u;
+        x_copy.dst = smem_u32(xs + tok * tok_stride + e0 / 2);
+        x_copy.bar = x_bar + 8u * j;
+        x_copy.src = static_cast<const uint16_t *>(p.X) + (int64_t)tok * p.ldx + (int64_t)L0 * 48 + e0;  // either 16-bit type
     };
 
     constexpr int NACC = 2;
@@ -516,6 +526,7 @@ gemv_trit_lut_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
             }
         }
         if (p.bulk_x && threadIdx.x == 0) expect_x();
+        if (p.bulk_x) plan_x(warp + lane * consumer_warps);
         asm volatile("bar.sync 1, %0;" ::"r"(consumer_threads) : "memory");  // zero padding, expected bytes
         if (!p.independent) {
             asm volatile("griddepcontrol.wait;" ::: "memory");  // the activations may be the previous kernel's output
@@ -530,7 +541,11 @@ gemv_trit_lut_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
         }
         bool ok = true;
         if (p.bulk_x) {
-            issue_x(warp + lane * consumer_warps, 32 * consumer_warps);  // one copy per lane at most: one instruction per warp
+            if (x_copy.bytes) bulk_load(x_copy.dst, x_copy.src, x_copy.bytes, x_copy.bar);
+            for (int i = warp + (lane + 32) * consumer_warps; i < kXPieces * p.ntok; i += 32 * consumer_warps) {  // one warp only
+                plan_x(i);
+                if (x_copy.bytes) bulk_load(x_copy.dst, x_copy.src, x_copy.bytes, x_copy.bar);
+            }
         } else {
             stage_activations<XT, PLANES>(p, L0, nl, xs, tok_stride, plane_stride, threadIdx.x, consumer_threads);
             asm volatile("bar.sync 1, %0;" ::"r"(consumer_threads) : "memory");
@@ -709,11 +724,12 @@ gemv_trit_lut_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
     };
     if (slices == 1) {
         for (int item = threadIdx.x; item < kTokPad * blocks_per_tok; item += all_threads) {
-            const int tok = item / blocks_per_tok, r0 = (item - tok * blocks_per_tok) * 8;
+            const int tok = divided(item, p.row_blocks_inv), r0 = (item - tok * blocks_per_tok) * 8;
             float v[8];
             const float4 *src = reinterpret_cast<const float4 *>(part + tok * prow + r0);
             float4 lo = src[0], hi = src[1];
             v[0] = lo.x; v[1] = lo.y; v[2] = lo.z; v[3] = lo.w; v[4] = hi.x; v[5] = hi.y; v[6] = hi.z; v[7] = hi.w;
+#pragma unroll 4
             for (int w = 1; w < p.k_warps; ++w) {
                 src = reinterpret_cast<const float4 *>(part + (size_t)w * plane + tok * prow + r0);
                 lo = src[0]; hi = src[1];
@@ -731,15 +747,16 @@ gemv_trit_lut_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
         const int slot = kTokPad * spitch;       // floats per sender
         float *recv = part + (size_t)p.k_warps * plane;
         for (int item = threadIdx.x; item < kTokPad * blocks_per_tok; item += all_threads) {
-            const int tok = item / blocks_per_tok, r0 = (item - tok * blocks_per_tok) * 8;
+            const int tok = divided(item, p.row_blocks_inv), r0 = (item - tok * blocks_per_tok) * 8;
             const float4 *src = reinterpret_cast<const float4 *>(part + tok * prow + r0);
             float4 lo = src[0], hi = src[1];
+#pragma unroll 4
             for (int w = 1; w < p.k_warps; ++w) {
                 src = reinterpret_cast<const float4 *>(part + (size_t)w * plane + tok * prow + r0);
                 const float4 a = src[0], b = src[1];
                 lo.x += a.x; lo.y += a.y; lo.z += a.z; lo.w += a.w; hi.x += b.x; hi.y += b.y; hi.z += b.z; hi.w += b.w;
             }
-            const int dst = r0 / span;
+            const int dst = divided(r0 >> 3, p.span_blocks_inv);
             float4 *out = reinterpret_cast<float4 *>(cluster.map_shared_rank(recv, dst) + (size_t)slice * slot + tok * spitch + (r0 - dst * span));
             out[0] = lo;
             out[1] = hi;
@@ -747,8 +764,9 @@ gemv_trit_lut_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
         cluster.sync();
         const int span_blocks = span / 8;
         for (int item = threadIdx.x; item < kTokPad * span_blocks; item += all_threads) {
-            const int tok = item / span_blocks, r0 = (item - tok * span_blocks) * 8;
+            const int tok = divided(item, p.span_blocks_inv), r0 = (item - tok * span_blocks) * 8;
             float v[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll 4
             for (int rk = 0; rk < slices; ++rk) {
                 const float4 *src = reinterpret_cast<const float4 *>(recv + (size_t)rk * slot + tok * spitch + r0);
                 const float4 lo = src[0], hi = src[1];
@@ -1047,6 +1065,9 @@ int gemv_trit_lut_launch(int fmt, int n_seg, const uint8_t *const *A, const floa
     p.xs_offset = pl.xs_offset; p.part_offset = pl.part_offset; p.sb_offset = pl.sb_offset; p.bar_offset = pl.bar_offset;
     p.vec_x = reinterpret_cast<uintptr_t>(X) % 16 == 0 && (ldx * (int64_t)dtype_size(x_dtype)) % 16 == 0 ? 1 : 0;
     p.bulk_x = bulk_x;
+    p.ntok_inv = inverse((uint32_t)ntok);
+    p.row_blocks_inv = inverse((uint32_t)pl.row_warps * 4);
+    p.span_blocks_inv = inverse((uint32_t)pl.row_warps * 4 / pl.slices);
     p.n_peers = ctx ? ctx->n_peers : 0;
     for (int i = 0; i < T81B200_MAX_PEERS; ++i) p.peer_C[i] = i < p.n_peers ? ctx->peer_C[i] : nullptr;
     p.sync_local = ctx ? ctx->sync_local : nullptr;
