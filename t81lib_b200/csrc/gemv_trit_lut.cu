@@ -128,7 +128,7 @@ struct GemvLutParams {
     uint32_t ntok_inv, row_blocks_inv, span_blocks_inv;  // inverse(d) of: ntok; eights of rows of a CTA; those that one CTA of a cluster finishes
     int vec_x;               // 1: rows of X start on 16-byte boundaries
     int bulk_x;              // 1: 16-bit activations, 16-byte aligned rows, K % 8 == 0: fetched by bulk copies
-    int independent;         // 1: reads nothing the previous kernel of the stream wrote
+    int independent;         // reads nothing the previous kernel of the stream wrote: 1 stores without waiting for it too (the caller says so), 2 waits before it stores
     int n_peers;             // other GPUs whose result receives every output element too (one segment only)
     void *peer_C[T81B200_MAX_PEERS];
     uint32_t *sync_local;
@@ -415,8 +415,8 @@ gemv_trit_lut_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
     TRACE_STAMP(1);
     // Programmatic dependent launch: a kernel that depends on its predecessor lets its own successor start once
     // its input is complete (after its wait below); one that does not depend on it lets the successor start at
-    // once and waits for the predecessor at its very end instead, so that "this grid has completed" still implies
-    // "everything before it has".
+    // once and waits for the predecessor before its stores, or at its very end, so that "this grid has completed" still
+    // implies "everything before it has".
     if (p.independent) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
     // Activations by bulk copy (16-bit types, 16-byte aligned rows, K a multiple of 8): the copies bring exactly the
@@ -678,6 +678,7 @@ gemv_trit_lut_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
     }
     __syncthreads();
     TRACE_STAMP(5);
+    if (p.independent == 2) asm volatile("griddepcontrol.wait;" ::: "memory");
 
     // Fold the K-slices' partials in a fixed order (deterministic), then, with more than one CTA per cluster, the
     // ranks' partials through distributed shared memory (also in a fixed order).  A finishing thread owns eight consecutive rows of one
@@ -776,7 +777,7 @@ gemv_trit_lut_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
         }
     }
     TRACE_STAMP(6);
-    if (p.independent) asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (p.independent == 1) asm volatile("griddepcontrol.wait;" ::: "memory");
     if (p.sync_local) {
         // one system fence per CTA, by the signalling thread after the barrier: the barrier orders the CTA's stores before it
         __syncthreads();
@@ -821,10 +822,11 @@ struct PlanKey {
 };
 struct PlanKeyHash {
     size_t operator()(const PlanKey &k) const {
-        const unsigned char *b = reinterpret_cast<const unsigned char *>(&k);
-        uint64_t h = 1469598103934665603ull;
-        for (size_t i = 0; i < sizeof k; ++i) { h ^= b[i]; h *= 1099511628211ull; }
-        return (size_t)h;
+        static_assert(sizeof k % 8 == 0, "a key is hashed word by word");
+        uint64_t w[sizeof k / 8], h = 0;
+        memcpy(w, &k, sizeof k);
+        for (const uint64_t v : w) h = (h ^ v ^ (h >> 29)) * 0x9E3779B97F4A7C15ull;
+        return (size_t)(h ^ (h >> 32));
     }
 };
 struct Plan {
@@ -1020,6 +1022,49 @@ int launch_lut_xt(const Plan &pl, const GemvLutParams &p, int x_dtype, int c_dty
 
 extern thread_local int g_hint_independent;
 
+namespace {
+
+// Projections that share an input (q/k/v, gate/up) called one after the other wait for one another although they need not.  In a
+// graph capture that can be known: the stream names the nodes that the next launch will wait for.  Where that is one node alone,
+// and it is the streaming product that this thread captured last, everything ahead of that product is complete once all of its
+// CTAs have passed their wait and let the next launch start, and what it may still be writing is its own result.  A product
+// whose activations, scales and biases do not touch that result need not wait before it reads them (GemvLutParams::independent
+// == 2); it waits before it stores, so nothing is written earlier than it was, and whoever waits for it waits for both.
+// Products that started so add up: their results are kept here until one waits first again.  Outside a capture nothing tells
+// what else the stream holds, and every product waits.  Two decoder blocks of 14 products (8 tokens): 102.2 -> 94.2 to 96.2 us.
+struct Bytes {
+    uintptr_t from, to;
+};
+struct InFlight {
+    unsigned long long capture = 0;  // 0: none
+    cudaGraphNode_t node = nullptr;
+    int n = 0;
+    Bytes result[4 * kMaxSeg];
+};
+thread_local InFlight g_in_flight;
+
+// The capture that the stream is part of (0: none), and the node its next launch will wait for if that is a single one.
+unsigned long long capturing(cudaStream_t st, cudaGraphNode_t &node) {
+    unsigned long long capture = 0;
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    const cudaGraphNode_t *nodes = nullptr;
+    const cudaGraphEdgeData *edges = nullptr;
+    size_t n = 0;
+    if (cudaStreamGetCaptureInfo_v3(st, &status, &capture, nullptr, &nodes, &edges, &n) != cudaSuccess) {
+        (void)cudaGetLastError();  // the default stream beside another stream's capture
+        return 0;
+    }
+    node = n == 1 ? nodes[0] : nullptr;
+    return status == cudaStreamCaptureStatusActive ? capture : 0;
+}
+
+Bytes extent(const void *p, int64_t rows, int64_t ld, int64_t cols, size_t size) {
+    const uintptr_t at = reinterpret_cast<uintptr_t>(p);
+    return {at, p ? at + (uintptr_t)(((rows - 1) * ld + cols) * (int64_t)size) : at};
+}
+
+}  // namespace
+
 // Launch of the streaming kernel over n_seg weight matrices that share X.  NK layout, ntok in 1..16, every A
 // 16-byte aligned; fmt 0: A in the packed-limb layout (table decode), fmt 1: A in the decode-stream layout.
 // Returns T81B200_EALIGN when no launch shape fits (K too long for shared memory).
@@ -1074,11 +1119,33 @@ int gemv_trit_lut_launch(int fmt, int n_seg, const uint8_t *const *A, const floa
     for (int i = 0; i < T81B200_MAX_PEERS; ++i) p.sync_peer[i] = p.sync_local && i < ctx->n_peers ? ctx->sync_slots[i] : nullptr;
     p.independent = (g_hint_independent && !p.sync_local) ? 1 : 0;
     for (int j = 0; j < 8; ++j) p.shl[j] = 1u << (2 * j);
+    cudaGraphNode_t ahead = nullptr;
+    const unsigned long long capture = ctx || p.independent ? 0 : capturing(st, ahead);
+    if (capture && ahead && g_in_flight.capture == capture && g_in_flight.node == ahead && g_in_flight.n + n_seg <= (int)(sizeof g_in_flight.result / sizeof(Bytes))) {
+        bool apart = true;
+        auto reads = [&](const Bytes &b) {
+            for (int i = 0; i < g_in_flight.n; ++i) apart = apart && (b.to <= g_in_flight.result[i].from || g_in_flight.result[i].to <= b.from);
+        };
+        reads(extent(X, ntok, ldx, K, dtype_size(x_dtype)));
+        for (int i = 0; i < n_seg; ++i) {
+            reads(extent(p.seg[i].row_scale, 1, 0, M[i], 4));
+            reads(extent(p.seg[i].bias, 1, 0, M[i], 4));
+        }
+        if (apart) p.independent = 2;
+    }
+    if (p.independent != 2) g_in_flight.n = 0;
 #ifdef T81B200_GEMV_TRACE
     static std::atomic<int> trace_counter{0};
     p.trace_slot = trace_counter.fetch_add(1);
 #endif
-    return fmt == 1 ? launch_lut_xt<1>(pl, p, x_dtype, c_dtype, st) : launch_lut_xt<0>(pl, p, x_dtype, c_dtype, st);
+    const int rc = fmt == 1 ? launch_lut_xt<1>(pl, p, x_dtype, c_dtype, st) : launch_lut_xt<0>(pl, p, x_dtype, c_dtype, st);
+    g_in_flight.capture = 0;
+    if (rc == T81B200_OK && capture && capturing(st, ahead) == capture && ahead) {
+        for (int i = 0; i < n_seg; ++i) g_in_flight.result[g_in_flight.n++] = extent(C[i], ntok, ldc, M[i], dtype_size(c_dtype));
+        g_in_flight.capture = capture;
+        g_in_flight.node = ahead;
+    }
+    return rc;
 }
 
 #ifdef T81B200_GEMV_TRACE

@@ -98,7 +98,8 @@ class Linear(nn.Linear):
                 self.weight.detach(), threshold=self.ternary_threshold, rule=self.ternary_rule)
         product = ternary_weight._product
         if product is not None and t81_torch.DECODE_STREAM_LAYOUT:
-            y = product(x, self.bias)  # None: a call that needs a conversion, a copy or an autograd node
+            bias = self._parameters["bias"] if "bias" in self._parameters else self.bias  # past nn.Module.__getattr__ where it can be
+            y = product(x, bias)  # None: a call that needs a conversion, a copy or an autograd node
             if y is not None:
                 return y
         return self._packed_linear(x)

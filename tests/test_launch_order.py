@@ -114,3 +114,81 @@ def test_decode_sized_training_steps_follow_their_weights(ops, tokens):
         want = (x.cpu().numpy().astype(np.float64) @ trits.T) * scale
         # whole numbers below 2^24, times the scale: one rounding
         np.testing.assert_allclose(y.detach().cpu().numpy(), want, rtol=2.0 ** -23, atol=0)
+
+
+# Products of one input captured one after the other read it early; whatever lies between them, and inputs, scales and biases that
+# come from the product ahead, take the order that the stream gives.
+@pytest.mark.parametrize("dtype,tokens", [(torch.bfloat16, 8), (torch.float16, 13), (torch.float32, 3)])
+def test_captured_products_of_one_input(ops, dtype, tokens):
+    from t81lib_b200 import _capi
+    K, rows = 1024, 1024
+    gen = torch.Generator(device="cuda").manual_seed(tokens)
+
+    def weight():
+        trits = torch.randint(-1, 2, (rows, K), generator=gen, device="cuda").float()
+        trits *= torch.rand(rows, K, generator=gen, device="cuda") < 0.02  # results stay small whole numbers: exact in every type
+        return trits, ops.pack_t2(ops.quantize_pack(trits, 0.5, "fixed")[0], rows, K)
+    weights = [weight() for _ in range(10)]
+    x = torch.empty(tokens, K, device="cuda", dtype=dtype)
+    vector, shared = torch.zeros(rows, device="cuda"), torch.zeros(tokens, K, device="cuda", dtype=dtype)
+
+    def chain(product):
+        one = [product(i, x) for i in range(3)]               # q, k, v
+        shared.copy_(one[0].clamp(-2, 2))                     # another kernel between two products
+        two = [product(3, shared), product(4, shared)]
+        again = product(5, two[1].clamp(-2, 2))               # and products of the one ahead
+        follows = [product(6, again), product(7, again)]
+        follows.append(product(8, x))
+        vector.copy_(follows[2][0].float())
+        return one + two + [again] + follows + [product(9, x, vector)]
+
+    def device(i, a, bias=None):
+        return ops.linear_t2(weights[i][1], rows, a, K, None, bias)
+
+    def expected(i, a, bias=None):
+        y = a.double() @ weights[i][0].double().t()
+        return (y if bias is None else y + bias.double()).to(dtype)
+    x.zero_()
+    chain(device)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = chain(device)
+    for _ in range(20):
+        x.copy_(torch.randint(-1, 2, (tokens, K), generator=gen, device="cuda"))
+        graph.replay()
+        got_now = [g.clone() for g in got]
+        for g, want in zip(got_now, chain(expected)):
+            assert torch.equal(g, want)
+    assert _capi.kernel_status(reset=True) == 0
+
+
+# The result of one product lies in the input of the next, or the next one's result over its input: no early reading, no early writing.
+@pytest.mark.parametrize("overlap", ["reads what is written", "writes what is read", "apart"])
+def test_captured_products_whose_buffers_touch(ops, overlap):
+    from t81lib_b200 import _capi
+    K = rows = 512
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    trits = torch.randint(-1, 2, (rows, K), generator=gen, device="cuda").float() * (torch.rand(rows, K, generator=gen, device="cuda") < 0.01)
+    t2 = ops.pack_t2(ops.quantize_pack(trits, 0.5, "fixed")[0], rows, K)
+    a, b, c = (torch.zeros(4, K, device="cuda", dtype=torch.bfloat16) for _ in range(3))
+    into = lambda x, y: _capi.check(_capi.lib.t81b200_linear_t2(
+        t2.data_ptr(), None, None, y.data_ptr(), rows, x.data_ptr(), _capi.BF16, K, _capi.BF16, rows, 4, K, 1.0, 0.0, 2, None, 0,
+        torch.cuda.current_stream().cuda_stream))
+    steps = {"reads what is written": [(a, b), (b, c), (a, b), (b, a)], "writes what is read": [(a, b), (c, a), (a, c), (b, a)],
+             "apart": [(a, b), (a, c), (a, b), (a, c)]}[overlap]
+    into(a, b)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        for x, y in steps:
+            into(x, y)
+    for _ in range(20):
+        for t in (a, b, c):
+            t.copy_(torch.randint(-1, 2, (4, K), generator=gen, device="cuda"))
+        buffers = {id(t): t.double() for t in (a, b, c)}
+        graph.replay()
+        for x, y in steps:
+            buffers[id(y)] = (buffers[id(x)] @ trits.double().t()).to(torch.bfloat16).double()
+        for t in (a, b, c):
+            assert torch.equal(t.double(), buffers[id(t)])
