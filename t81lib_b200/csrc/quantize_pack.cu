@@ -226,11 +226,12 @@ quantize_pack_row_kernel(const T *__restrict__ w, int64_t rows, int cols, int64_
 // ---- the streaming form: rows land in a shared-memory ring by bulk copies ----
 //
 // quantize_pack_ring_kernel: one persistent CTA per SM.  A producer thread keeps a ring of whole rows in flight
-// (one bulk copy per row, up to 16 rows and ~220 KB per SM: the bytes in flight that HBM needs, which registers of
+// (one bulk copy per row, up to 12 rows and ~220 KB per SM: the bytes in flight that HBM needs, which registers of
 // resident CTAs cannot hold); TEAMS teams of four warps each take every TEAMS-th row of the CTA from the ring, with
 // the chunk ownership, the summation order and the pack step of the row kernel above, reading the row from
 // shared memory twice (sum, then pack) and handing the slot back after the second pass.
-// Needs 16-byte aligned rows of a multiple of 16 bytes and TEAMS rows in 226 KB; the row kernel covers the rest.
+// Rows may start and end anywhere: a copy brings the 16-byte pieces that hold the row, and groups are cut out of aligned pieces (two
+// loads instead of one, and a loop for each of the four shifts).  Needs TEAMS rows in 226 KB; the row kernel covers the rest.
 constexpr int kMaxTeams = 7;
 constexpr int kMaxSlots = 16;
 constexpr int kRingBytes = 226 * 1024;  // rows; barriers and team sums are static shared memory
@@ -238,26 +239,104 @@ constexpr int kRingBytes = 226 * 1024;  // rows; barriers and team sums are stat
 enum { QUANT_STATUS_TIMEOUT_PRODUCER = 9, QUANT_STATUS_TIMEOUT_CONSUMER = 10 };
 __device__ int g_quant_status = 0;
 
-template <typename T, bool ABSMEAN>
+// A row in shared memory lies SHIFT elements behind `row`, which is on a boundary of a group's size.  Where that is not 0 a group is cut
+// out of two aligned pieces.  TAIL: its columns may be no multiple of 4; what lies past the row's end reads as 0.
+template <typename T, bool ABSMEAN, int SHIFT, bool TAIL>
 __device__ __forceinline__ void load_chunk_shared(const T *row, int c, int lane, int cols, float (&v)[3][4], double &part) {
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         const int col = 4 * (kChunkGroups * c + 32 * k + lane);
-        if (col < cols) {  // whole groups: cols is a multiple of 4
+        if (col < cols) {
             if constexpr (sizeof(T) == 4) {
                 const float4 f = *reinterpret_cast<const float4 *>(row + col);
-                v[k][0] = f.x; v[k][1] = f.y; v[k][2] = f.z; v[k][3] = f.w;
+                float e[8] = {f.x, f.y, f.z, f.w, 0.0f, 0.0f, 0.0f, 0.0f};
+                if constexpr (SHIFT != 0) {
+                    const float4 g = *reinterpret_cast<const float4 *>(row + col + 4);
+                    e[4] = g.x; e[5] = g.y; e[6] = g.z; e[7] = g.w;
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i) v[k][i] = e[i + SHIFT];
             } else {
-                const uint2 u = *reinterpret_cast<const uint2 *>(row + col);
+                uint2 u = *reinterpret_cast<const uint2 *>(row + col);
+                if constexpr (SHIFT != 0) {
+                    const uint2 w = *reinterpret_cast<const uint2 *>(row + col + 4);
+                    if constexpr (SHIFT == 1) u = make_uint2(__byte_perm(u.x, u.y, 0x5432), __byte_perm(u.y, w.x, 0x5432));
+                    else if constexpr (SHIFT == 2) u = make_uint2(u.y, w.x);
+                    else u = make_uint2(__byte_perm(u.y, w.x, 0x5432), __byte_perm(w.x, w.y, 0x5432));
+                }
                 const T *e = reinterpret_cast<const T *>(&u);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) v[k][i] = to_float<T>(e[i]);
             }
+            if (TAIL && col + 4 > cols)
+#pragma unroll
+                for (int i = 1; i < 4; ++i)
+                    if (col + i >= cols) v[k][i] = 0.0f;
         } else { v[k][0] = v[k][1] = v[k][2] = v[k][3] = 0.0f; }
     }
     if constexpr (ABSMEAN) {
 #pragma unroll
         for (int k = 0; k < 3; ++k) part += group_abs_sum(v[k]);
+    }
+}
+
+// f with the row's shift as a constant; every shift has its own loops, a choice per group costs as much as packing it.
+template <bool ALIGNED, typename F>
+__device__ __forceinline__ void with_shift(int shift, F &&f) {
+    if constexpr (ALIGNED) f(std::integral_constant<int, 0>{});
+    else
+        switch (shift) {
+            case 0: f(std::integral_constant<int, 0>{}); break;
+            case 1: f(std::integral_constant<int, 1>{}); break;
+            case 2: f(std::integral_constant<int, 2>{}); break;
+            default: f(std::integral_constant<int, 3>{});
+        }
+}
+
+// Where a row that starts at `global` lies in its slot, which it enters at the same distance from a 16-byte boundary: the group boundary
+// at or before it, and the elements from there.
+template <typename T, bool ALIGNED>
+__device__ __forceinline__ const T *row_in_slot(const uint8_t *slot, const T *global, int &shift) {
+    shift = 0;
+    if constexpr (ALIGNED) return reinterpret_cast<const T *>(slot);
+    constexpr int kGroup = 4 * (int)sizeof(T);
+    const int lead = (int)(reinterpret_cast<uintptr_t>(global) & 15);
+    shift = lead % kGroup / (int)sizeof(T);
+    return reinterpret_cast<const T *>(slot + lead / kGroup * kGroup);
+}
+
+// Brings a row into a slot, for one thread: the 16-byte pieces that hold it, with the bytes of its neighbours in the first and
+// the last, except those that reach past the matrix (its first and last row): there its own elements alone, one by one.
+struct Matrix {
+    const uint8_t *begin, *end;
+};
+template <typename T, bool ALIGNED>
+__device__ __forceinline__ void fetch_row(const T *row, uint32_t row_bytes, const Matrix &m, uint8_t *slot, uint32_t slot_addr, uint32_t bar) {
+    if constexpr (ALIGNED) {
+        mbar_arrive_expect_tx(bar, row_bytes);
+        bulk_load(slot_addr, row, row_bytes, bar);
+    } else {
+        const uint8_t *start = reinterpret_cast<const uint8_t *>(row);
+        const uint32_t lead = (uint32_t)(reinterpret_cast<uintptr_t>(start) & 15), whole = (lead + row_bytes + 15) & ~15u;
+        const uint8_t *from = start - lead;
+        if (from >= m.begin && from + whole <= m.end) {
+            mbar_arrive_expect_tx(bar, whole);
+            bulk_load(slot_addr, from, whole, bar);
+            return;
+        }
+        const uint32_t first = from < m.begin ? 16 : 0, last = from + whole > m.end ? whole - 16 : whole;  // last may lie before first
+        auto single = [&](uint32_t a, uint32_t b) {
+            for (; a < b; a += sizeof(T)) *reinterpret_cast<T *>(slot + a) = *reinterpret_cast<const T *>(from + a);
+        };
+        if (first >= last) single(lead, lead + row_bytes);
+        else {
+            single(lead, first);
+            single(last, lead + row_bytes);
+        }
+        if (first < last) {
+            mbar_arrive_expect_tx(bar, last - first);
+            bulk_load(slot_addr + first, from + first, last - first, bar);
+        } else mbar_arrive(bar);
     }
 }
 
@@ -274,7 +353,7 @@ __device__ __forceinline__ bool team_all(int team, bool ok) {
     return r != 0;
 }
 
-template <typename T, bool ABSMEAN, int TEAMS>
+template <typename T, bool ABSMEAN, int TEAMS, bool ALIGNED>
 __global__ void __launch_bounds__(TEAMS * kRowThreads + 32, 1)
 quantize_pack_ring_kernel(const T *__restrict__ w, int rows, int cols, int64_t ld, float thr, uint8_t *__restrict__ packed,
                           float *__restrict__ row_scale, int slots, int slot_bytes) {
@@ -297,15 +376,12 @@ quantize_pack_ring_kernel(const T *__restrict__ w, int rows, int cols, int64_t l
     if (warp_in_cta == TEAMS * 4) {
         // producer: row i of this CTA goes to slot i % slots as soon as the slot's previous row was handed back
         if (lane == 0) {
+            const Matrix matrix = {reinterpret_cast<const uint8_t *>(w), reinterpret_cast<const uint8_t *>(w + (int64_t)(rows - 1) * ld + cols)};
             for (int i = 0; i < n_local; ++i) {
                 const int slot = i % slots, use = i / slots;
                 if (use > 0 && !mbar_wait(empty0 + 8u * slot, (uint32_t)(use - 1) & 1u)) { atomicCAS(&g_quant_status, 0, QUANT_STATUS_TIMEOUT_PRODUCER); break; }
                 const int64_t r = (int64_t)blockIdx.x + (int64_t)i * gridDim.x;
-                mbar_arrive_expect_tx(full0 + 8u * slot, row_bytes);
-                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                             ::"r"(smem_u32(ring) + (uint32_t)slot * (uint32_t)slot_bytes), "l"(w + r * ld), "r"(row_bytes),
-                               "r"(full0 + 8u * slot)
-                             : "memory");
+                fetch_row<T, ALIGNED>(w + r * ld, row_bytes, matrix, ring + (size_t)slot * slot_bytes, smem_u32(ring) + (uint32_t)slot * (uint32_t)slot_bytes, full0 + 8u * slot);
             }
         }
         return;
@@ -320,18 +396,20 @@ quantize_pack_ring_kernel(const T *__restrict__ w, int rows, int cols, int64_t l
         // slots is a multiple of the team count: every use of a slot is consumed by the same team, in order
         const int slot = i % slots, use = i / slots;
         const int64_t r = (int64_t)blockIdx.x + (int64_t)i * gridDim.x;
-        const T *row = reinterpret_cast<const T *>(ring + (size_t)slot * slot_bytes);
+        int shift;
+        const T *row = row_in_slot<T, ALIGNED>(ring + (size_t)slot * slot_bytes, w + r * ld, shift);
         uint32_t *out = reinterpret_cast<uint32_t *>(packed + r * (int64_t)kl * 16);
         bool ok = __all_sync(0xffffffffu, mbar_wait(full0 + 8u * slot, (uint32_t)use & 1u));
         float cut = thr;
         if constexpr (ABSMEAN) {
             double part = 0.0;
-            if (ok) {
-                for (int c = warp; c < nchunks; c += 4) {
-                    float v[3][4];
-                    load_chunk_shared<T, true>(row, c, lane, cols, v, part);
-                }
-            }
+            if (ok)
+                with_shift<ALIGNED>(shift, [&](auto s) {
+                    for (int c = warp; c < nchunks; c += 4) {
+                        float v[3][4];
+                        load_chunk_shared<T, true, decltype(s)::value, !ALIGNED>(row, c, lane, cols, v, part);
+                    }
+                });
 #pragma unroll
             for (int off = 16; off >= 1; off >>= 1) part += __shfl_down_sync(0xffffffffu, part, off);
             if (lane == 0) warp_sum[team][parity][warp] = part;
@@ -349,18 +427,105 @@ quantize_pack_ring_kernel(const T *__restrict__ w, int rows, int cols, int64_t l
         }
         // cut > 0 (the same in the whole team) takes the short form of the pack step; the branch stays outside the loop
         auto pack_row = [&](auto fast) {
-            for (int c = warp; c < nchunks; c += 4) {
-                float v[3][4];
-                double unused = 0.0;
-                load_chunk_shared<T, false>(row, c, lane, cols, v, unused);
-                const uint32_t word = pack_chunk<decltype(fast)::value>(v, c, lane, cols, cut, pc);
-                if (32 * c + lane < nwords) out[32 * c + lane] = word;
-            }
+            with_shift<ALIGNED>(shift, [&](auto s) {
+                for (int c = warp; c < nchunks; c += 4) {
+                    float v[3][4];
+                    double unused = 0.0;
+                    load_chunk_shared<T, false, decltype(s)::value, !ALIGNED>(row, c, lane, cols, v, unused);
+                    const uint32_t word = pack_chunk<decltype(fast)::value>(v, c, lane, cols, cut, pc);
+                    if (32 * c + lane < nwords) out[32 * c + lane] = word;
+                }
+            });
         };
         if (cut > 0.0f) pack_row(std::true_type{});
         else pack_row(std::false_type{});
         __syncwarp();
         if (lane == 0) mbar_arrive(empty0 + 8u * slot);  // this warp has read the row for the last time
+    }
+}
+
+// ---- rows of which many fit: a warp to a row ----
+//
+// quantize_pack_warp_kernel: three persistent CTAs per SM; every warp walks through rows of its own with one or two slots of shared
+// memory, filled by bulk copies that it starts itself; nothing is shared with other warps.  A team of four gives a row of a few
+// chunks little work beside its barrier, its hand-over and its wait for memory, and has fewer rows in flight.  (Four CTAs of eight warps
+// are 7 % slower than three, one CTA of 24 warps is 20 to 30 % slower for matrices of a few rows an SM.)  The summation
+// order is the same: chunk c belongs to partial sum c % 4 of the lane, each folded by itself.
+constexpr int kWarpRows = 8, kWarpCtas = 3;  // warps of a CTA, CTAs of an SM
+
+template <typename T, bool ABSMEAN, bool ALIGNED>
+__global__ void __launch_bounds__(kWarpRows * 32, kWarpCtas)
+quantize_pack_warp_kernel(const T *__restrict__ w, int rows, int cols, int64_t ld, float thr, uint8_t *__restrict__ packed,
+                          float *__restrict__ row_scale, int slots_each, int slot_bytes) {
+    extern __shared__ __align__(128) uint8_t ring[];
+    __shared__ __align__(8) uint64_t bars[kWarpRows][2];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int kl = (cols + 47) / 48, nwords = kl * 4, nchunks = (nwords + 31) / 32;
+    const uint32_t row_bytes = (uint32_t)cols * (uint32_t)sizeof(T), bar0 = smem_u32(bars[warp]);
+    uint8_t *slots = ring + (size_t)warp * slots_each * slot_bytes;
+    const Matrix matrix = {reinterpret_cast<const uint8_t *>(w), reinterpret_cast<const uint8_t *>(w + (int64_t)(rows - 1) * ld + cols)};
+    if (lane == 0) {
+        mbar_init(bar0, 1);
+        mbar_init(bar0 + 8u, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncwarp();
+    PackConsts pc;
+    make_pack_consts(lane, pc);
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // see quantize_pack_ring_kernel
+    const int64_t stride = (int64_t)gridDim.x * kWarpRows;
+    int64_t r = (int64_t)gridDim.x * warp + blockIdx.x;
+    if (lane == 0)
+        for (int i = 0; i < slots_each; ++i)
+            if (r + i * stride < rows) fetch_row<T, ALIGNED>(w + (r + i * stride) * ld, row_bytes, matrix, slots + i * slot_bytes, smem_u32(slots) + (uint32_t)(i * slot_bytes), bar0 + 8u * i);
+    int at = 0;  // slot
+    uint32_t phase = 0;
+    for (; r < rows; r += stride) {
+        int shift;
+        const T *row = row_in_slot<T, ALIGNED>(slots + at * slot_bytes, w + r * ld, shift);
+        uint32_t *out = reinterpret_cast<uint32_t *>(packed + r * (int64_t)kl * 16);
+        if (!__all_sync(0xffffffffu, mbar_wait(bar0 + 8u * at, phase))) {
+            if (lane == 0) atomicCAS(&g_quant_status, 0, QUANT_STATUS_TIMEOUT_CONSUMER);
+            break;
+        }
+        float cut = thr;
+        if constexpr (ABSMEAN) {
+            double part[4] = {0.0, 0.0, 0.0, 0.0};
+            with_shift<ALIGNED>(shift, [&](auto s) {
+                for (int c = 0; c < nchunks; c += 4)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        if (c + j < nchunks) {
+                            float v[3][4];
+                            load_chunk_shared<T, true, decltype(s)::value, !ALIGNED>(row, c + j, lane, cols, v, part[j]);
+                        }
+            });
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (j < nchunks)
+#pragma unroll
+                    for (int off = 16; off >= 1; off >>= 1) part[j] += __shfl_down_sync(0xffffffffu, part[j], off);
+            const float mean = __shfl_sync(0xffffffffu, __fdiv_rn((float)((part[0] + part[2]) + (part[1] + part[3])), (float)cols), 0);
+            cut = absmean_cut(mean, thr);
+            if (lane == 0) row_scale[r] = mean;
+        }
+        auto pack_row = [&](auto fast) {
+            with_shift<ALIGNED>(shift, [&](auto s) {
+                for (int c = 0; c < nchunks; ++c) {
+                    float v[3][4];
+                    double unused = 0.0;
+                    load_chunk_shared<T, false, decltype(s)::value, !ALIGNED>(row, c, lane, cols, v, unused);
+                    const uint32_t word = pack_chunk<decltype(fast)::value>(v, c, lane, cols, cut, pc);
+                    if (32 * c + lane < nwords) out[32 * c + lane] = word;
+                }
+            });
+        };
+        if (cut > 0.0f) pack_row(std::true_type{});
+        else pack_row(std::false_type{});
+        __syncwarp();
+        if (lane == 0 && r + slots_each * stride < rows)
+            fetch_row<T, ALIGNED>(w + (r + slots_each * stride) * ld, row_bytes, matrix, slots + at * slot_bytes, smem_u32(slots) + (uint32_t)(at * slot_bytes), bar0 + 8u * at);
+        if (++at == slots_each) { at = 0; phase ^= 1u; }
     }
 }
 
@@ -403,40 +568,62 @@ int launch_row_kernel(const void *w, int64_t rows, int64_t cols, int64_t ld, flo
     return T81B200_OK;
 }
 
-template <typename T, bool ABSMEAN, int TEAMS>
-int launch_ring_kernel(const T *w, int64_t rows, int64_t cols, int64_t ld, float thr, uint8_t *packed, float *row_scale,
-                       int slots, int slot_bytes, cudaStream_t st) {
-    static std::atomic<bool> configured[64];
+// Launch of a kernel whose rows wait in shared memory, behind the kernel ahead without a gap.
+template <typename K, typename... Args>
+int launch_staged(K kernel, std::atomic<bool> (&configured)[64], int ctas, int threads, size_t smem, cudaStream_t st, Args... args) {
     int dev = 0;
     T81_CUDA_TRY(cudaGetDevice(&dev));
-    auto kernel = quantize_pack_ring_kernel<T, ABSMEAN, TEAMS>;
     if (dev < 0 || dev >= 64 || !configured[dev].load(std::memory_order_acquire)) {
         T81_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRingBytes));
         if (dev >= 0 && dev < 64) configured[dev].store(true, std::memory_order_release);
     }
-    const int g = (int)(rows < sm_count() ? rows : sm_count());
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)g, 1, 1);
-    cfg.blockDim = dim3(TEAMS * kRowThreads + 32, 1, 1);
-    cfg.dynamicSmemBytes = (size_t)slots * slot_bytes;
+    cfg.gridDim = dim3((unsigned)ctas, 1, 1);
+    cfg.blockDim = dim3((unsigned)threads, 1, 1);
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    T81_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, w, (int)rows, (int)cols, ld, thr, packed, row_scale, slots, slot_bytes));
+    T81_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, args...));
     return T81B200_OK;
 }
 
-template <typename T, int TEAMS>
-int launch_ring(const T *w, int64_t rows, int64_t cols, int64_t ld, float thr, int rule, uint8_t *packed, float *row_scale,
-                int64_t slot_bytes, cudaStream_t st) {
+template <typename T, bool ABSMEAN, int TEAMS, bool ALIGNED>
+int launch_ring(const T *w, int64_t rows, int64_t cols, int64_t ld, float thr, uint8_t *packed, float *row_scale, int64_t slot_bytes, cudaStream_t st) {
+    static std::atomic<bool> configured[64];
     int slots = (int)(kRingBytes / slot_bytes) / TEAMS * TEAMS;
     slots = slots > kMaxSlots / TEAMS * TEAMS ? kMaxSlots / TEAMS * TEAMS : slots;
-    return rule == T81B200_RULE_ABSMEAN
-               ? launch_ring_kernel<T, true, TEAMS>(w, rows, cols, ld, thr, packed, row_scale, slots, (int)slot_bytes, st)
-               : launch_ring_kernel<T, false, TEAMS>(w, rows, cols, ld, thr, packed, row_scale, slots, (int)slot_bytes, st);
+    return launch_staged(quantize_pack_ring_kernel<T, ABSMEAN, TEAMS, ALIGNED>, configured, (int)(rows < sm_count() ? rows : sm_count()),
+                         TEAMS * kRowThreads + 32, (size_t)slots * slot_bytes, st, w, (int)rows, (int)cols, ld, thr, packed, row_scale, slots, (int)slot_bytes);
+}
+
+template <typename T, bool ABSMEAN, bool ALIGNED>
+int launch_warps(const T *w, int64_t rows, int64_t cols, int64_t ld, float thr, uint8_t *packed, float *row_scale, int64_t slot_bytes, int each, cudaStream_t st) {
+    static std::atomic<bool> configured[64];
+    const int64_t ctas = (rows + kWarpRows - 1) / kWarpRows, most = (int64_t)sm_count() * kWarpCtas;
+    return launch_staged(quantize_pack_warp_kernel<T, ABSMEAN, ALIGNED>, configured, (int)(ctas < most ? ctas : most), kWarpRows * 32,
+                         (size_t)(kWarpRows * each) * slot_bytes, st, w, (int)rows, (int)cols, ld, thr, packed, row_scale, each, (int)slot_bytes);
+}
+
+// The forms that stage rows in shared memory, for enough rows to give every SM a few; 1 where neither applies.  A warp to a row where 24
+// rows fit beside each other, else teams where four do: with fewer rows in flight the warps wait for memory (us, absmean, warps against
+// teams: 8000 x 4096 bf16 24.2 and 25.5, 9000 x 2816 fp32 23.2 and 22.8, 4096 x 4096 fp32 16.4 and 13.7, 4096 x 14336 bf16 51 and 36).
+// Rows on 16-byte boundaries, teams before and warps now: 14336 x 1024 bf16 31.7 -> 13.1, 14336 x 1152 fp32 30.7 -> 15.1, 9892 x 2936
+// bf16 26.7 -> 21.3.  Off them, by the row kernel before: 9892 x 2933 bf16 60.6 -> 29.5, 4095 x 9001 bf16 75.0 -> 29.5, 8006 x 3077 fp32
+// 34.9 -> 31.1, 1500 x 14335 fp32 42.4 -> 25.9.
+template <typename T, bool ABSMEAN, bool ALIGNED>
+int launch_staged_rows(const T *w, int64_t rows, int64_t cols, int64_t ld, float thr, uint8_t *packed, float *row_scale, cudaStream_t st) {
+    const int64_t row_bytes = cols * (int64_t)sizeof(T), slot_bytes = (row_bytes + (ALIGNED ? 0 : 30) + 127) / 128 * 128;
+    if (rows < 2 * (int64_t)sm_count() || rows >= (1ll << 31)) return 1;
+    const int64_t each = (kRingBytes / kWarpCtas - 1024) / (kWarpRows * slot_bytes);
+    if (each >= 1) return launch_warps<T, ABSMEAN, ALIGNED>(w, rows, cols, ld, thr, packed, row_scale, slot_bytes, each > 1 ? 2 : 1, st);
+    const int fit = (int)(kRingBytes / slot_bytes);  // rows the ring holds; a team needs one, and one more in flight
+    if (fit < 4) return 1;
+    if (fit >= 12) return launch_ring<T, ABSMEAN, 6, ALIGNED>(w, rows, cols, ld, thr, packed, row_scale, slot_bytes, st);
+    return launch_ring<T, ABSMEAN, 4, ALIGNED>(w, rows, cols, ld, thr, packed, row_scale, slot_bytes, st);
 }
 
 template <typename T>
@@ -444,17 +631,15 @@ int launch_quantize_pack(const void *w, int64_t rows, int64_t cols, int64_t ld, 
                          uint8_t *packed, float *row_scale, cudaStream_t st) {
     const bool vec = (reinterpret_cast<uintptr_t>(w) % (4 * sizeof(T)) == 0) && (ld % 4 == 0);
     const int64_t nchunks = ((cols + 47) / 48 * 4 + 31) / 32;  // 384 columns each
-    // the streaming form: rows that bulk copies can move (16-byte aligned, a multiple of 16 bytes), four or more
-    // of which fit the ring, and enough of them to give every SM a few; T81B200_QUANT_PATH=row (read once) turns it off
     const int64_t row_bytes = cols * (int64_t)sizeof(T);
-    const int64_t slot_bytes = (row_bytes + 127) / 128 * 128;
-    const bool movable = reinterpret_cast<uintptr_t>(w) % 16 == 0 && (ld * (int64_t)sizeof(T)) % 16 == 0 && row_bytes % 16 == 0;
-    static const bool ring_off = [] { const char *e = getenv("T81B200_QUANT_PATH"); return e && strcmp(e, "row") == 0; }();
+    const bool aligned = reinterpret_cast<uintptr_t>(w) % 16 == 0 && (ld * (int64_t)sizeof(T)) % 16 == 0 && row_bytes % 16 == 0;
+    static const bool staged_off = [] { const char *e = getenv("T81B200_QUANT_PATH"); return e && strcmp(e, "row") == 0; }();  // read once
     const T *wt = static_cast<const T *>(w);
-    if (!ring_off && movable && rows >= 2 * (int64_t)sm_count() && rows < (1ll << 31)) {
-        const int fit = (int)(kRingBytes / slot_bytes);  // rows the ring holds; a team needs one, and one more in flight
-        if (fit >= 12) return launch_ring<T, 6>(wt, rows, cols, ld, thr, rule, packed, row_scale, slot_bytes, st);
-        if (fit >= 4) return launch_ring<T, 4>(wt, rows, cols, ld, thr, rule, packed, row_scale, slot_bytes, st);
+    if (!staged_off && reinterpret_cast<uintptr_t>(w) % sizeof(T) == 0) {
+        const bool absmean = rule == T81B200_RULE_ABSMEAN;
+        const auto launch = aligned ? (absmean ? launch_staged_rows<T, true, true> : launch_staged_rows<T, false, true>)
+                                    : (absmean ? launch_staged_rows<T, true, false> : launch_staged_rows<T, false, false>);
+        if (const int rc = launch(wt, rows, cols, ld, thr, packed, row_scale, st); rc <= 0) return rc;
     }
     if (nchunks <= 4 * 3)  // up to 4608 columns
         return launch_row_kernel<T, 3>(w, rows, cols, ld, thr, rule, packed, row_scale, vec, st);
