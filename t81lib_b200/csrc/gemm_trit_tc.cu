@@ -95,6 +95,7 @@ struct TcParams {
                          // this many tensor maps (the local C first, then the peers'); 0: per-element stores
     int n_peers;         // other GPUs that receive a copy of every output element
     void *peer_C[T81B200_MAX_PEERS];  // their C, same strides as the local one
+    int c_rows;          // 1: a 16-bit token-major C that takes neither: blocks staged the same way, written by the epilogue warps
     int c_vec;           // 1: tokens are contiguous in C (the (M, N) argument order) and 16-byte aligned per 32-token block:
                          // a thread's 32 tokens of one feature are one run of memory, moved with 128-bit accesses
 };
@@ -127,6 +128,40 @@ struct OutStage {
     bool reused;       // an earlier store may still be reading the buffer
 };
 
+// A staged block to rows of C that TMA cannot write (off 16-byte boundaries): whole words, four warps take every fourth token.  Where a
+// row starts between two words its elements pair up the other way.  One element a lane, straight from the accumulators, is half the
+// bytes a store in twice the stores, and bounded short contractions: 13680 tokens of 834 x 834, bf16, 61 us, 40 this way
+// (8192 tokens of 2048 x 2047: 80 and 60; 51 where TMA writes, 2048 x 2048).
+template <typename CT>
+__device__ __forceinline__ void write_rows(const TcParams &p, const uint8_t *staged, int row0, int tok0, int quarter, int lane) {
+    const int features = (int)(p.M - row0 < BM ? p.M - row0 : BM), tokens = (int)(p.N - tok0 < OUT_TOKENS ? p.N - tok0 : OUT_TOKENS);
+    uint16_t *row = reinterpret_cast<uint16_t *>(static_cast<CT *>(p.C) + ((int64_t)tok0 + quarter) * p.c_tok_stride + row0);
+    const uint32_t *src = reinterpret_cast<const uint32_t *>(staged) + quarter * (BM / 2) + lane;
+    constexpr int kRows = OUT_TOKENS / 4, kNext = 2 * BM;  // words from one of the warp's rows to the next
+    uint32_t w[kRows][2], after[kRows][2];  // all loads first: the compiler cannot know the stores to miss them
+#pragma unroll
+    for (int i = 0; i < kRows; ++i)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            w[i][h] = src[i * kNext + 32 * h];
+            after[i][h] = src[i * kNext + 32 * h + (h == 0 || lane < 31 ? 1 : 0)];
+        }
+    const int64_t step = 4 * p.c_tok_stride;
+#pragma unroll
+    for (int i = 0; i < kRows; ++i, row += step) {
+        if (4 * i + quarter >= tokens) break;
+        const int odd = (int)(reinterpret_cast<uintptr_t>(row) >> 1 & 1);
+        if (odd && lane == 0 && features > 0) row[0] = (uint16_t)w[i][0];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int e = 2 * (lane + 32 * h) + odd;  // elements e and e + 1
+            const uint32_t pair = odd ? __byte_perm(w[i][h], after[i][h], 0x5432) : w[i][h];
+            if (e + 1 < features) *reinterpret_cast<uint32_t *>(row + e) = pair;
+            else if (e < features) row[e] = (uint16_t)pair;
+        }
+    }
+}
+
 // One 32-token block of this thread's output feature: scale, bias, beta, store.
 template <typename CT>
 __device__ __forceinline__ void emit_block(const TcParams &p, const TcOutMaps &omaps, const uint32_t (&v)[32], int row0, int64_t row,
@@ -151,6 +186,13 @@ __device__ __forceinline__ void emit_block(const TcParams &p, const TcOutMaps &o
                 for (int j = 0; j < p.n_out_maps; ++j) tma_store_2d(&omaps.m[j], out.smem, row0, tok0);
             asm volatile("cp.async.bulk.commit_group;" ::: "memory");
         }
+    } else if (sizeof(CT) == 2 && p.c_rows) {
+        CT *dst = reinterpret_cast<CT *>(out.gen) + (int)(row - row0);
+#pragma unroll
+        for (int i = 0; i < 32; ++i) dst[i * BM] = from_float<CT>(__uint_as_float(v[i]) * scale + bias);
+        // two buffers in turn: past this barrier every warp has read the other one
+        asm volatile("bar.sync %0, 128;" ::"r"(out.barrier) : "memory");
+        write_rows<CT>(p, out.gen, row0, tok0, (int)(row - row0) >> 5, threadIdx.x & 31);
     } else if (row_ok && p.c_vec && (int64_t)tok0 + 32 <= p.N) {
         // (M, N) argument order: the thread's 32 tokens are contiguous — whole 16-byte pieces, and with
         // beta the old values are all fetched before the first store
@@ -887,7 +929,7 @@ int gemm_trit_tc_launch(int fmt, int fp32_planes, const uint8_t *A, const float 
                 return rc;
         }
         p.n_out_maps = 1 + n_peers;
-    }
+    } else p.c_rows = dtype_size(c_dtype) == 2 && layout == T81B200_LAYOUT_NK && beta == 0.0f && n_peers == 0 && reinterpret_cast<uintptr_t>(C) % 2 == 0 ? 1 : 0;
     auto launch = [&](auto small) {
         constexpr int S = decltype(small)::value;
         return fmt == 1 ? launch_tc_ct<1, S>(c_dtype, shape, mw, mx, om, p, st) : launch_tc_ct<0, S>(c_dtype, shape, mw, mx, om, p, st);

@@ -167,3 +167,24 @@ def test_host_pointer_entry_point(dev):
     assert rel_err(C, want) < 5e-5
     rc = _capi.lib.t81b200_gemm_trit_host(A.ctypes.data_as(vp), B.ctypes.data_as(vp), C.ctypes.data_as(vp), -1, N, K, 1.0, 0.0)
     assert rc == _capi.EINVAL and "non-negative" in _capi.last_error()
+
+
+# 16-bit results whose rows start anywhere, and activations whose rows do: widths around words, warps and tiles, tokens around blocks.
+# Whole numbers below 256 throughout, so that every type holds them exactly.
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("out_f,in_f,tokens", [(1, 577, 33), (2, 576, 40), (63, 201, 100), (65, 203, 64), (127, 385, 31), (129, 1001, 300), (255, 66, 257), (257, 95, 1000),
+                                               (386, 833, 2100), (4093, 301, 50), (1999, 2047, 90)])
+def test_tc_rows_off_boundaries(dev, dtype, out_f, in_f, tokens):
+    from t81lib_b200 import _capi, ops
+    gen = torch.Generator(device="cuda").manual_seed(out_f + tokens)
+    trits = torch.randint(-1, 2, (out_f, in_f), generator=gen, device="cuda").float()
+    t2 = ops.pack_t2(ops.quantize_pack(trits, 0.5, "fixed")[0], out_f, in_f)
+    x = torch.randint(-1, 2, (tokens, in_f), generator=gen, device="cuda").to(dtype)
+    x[torch.rand(tokens, in_f, generator=gen, device="cuda") < 0.5] = 0
+    want = (x.double() @ trits.double().t()).to(dtype)
+    got = ops.linear_t2(t2, out_f, x, in_f, None, None)
+    assert torch.equal(got, want)
+    wide = torch.full((tokens, in_f + 3), float("nan"), device="cuda", dtype=dtype)  # nothing beside the rows is used
+    wide[:, 1:in_f + 1] = x
+    assert torch.equal(ops.linear_t2(t2, out_f, wide[:, 1:in_f + 1], in_f, None, None), want)
+    assert _capi.kernel_status(reset=True) == 0
