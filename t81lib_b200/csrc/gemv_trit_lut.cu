@@ -730,7 +730,6 @@ gemv_trit_lut_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
             const float4 *src = reinterpret_cast<const float4 *>(part + tok * prow + r0);
             float4 lo = src[0], hi = src[1];
             v[0] = lo.x; v[1] = lo.y; v[2] = lo.z; v[3] = lo.w; v[4] = hi.x; v[5] = hi.y; v[6] = hi.z; v[7] = hi.w;
-#pragma unroll 4
             for (int w = 1; w < p.k_warps; ++w) {
                 src = reinterpret_cast<const float4 *>(part + (size_t)w * plane + tok * prow + r0);
                 lo = src[0]; hi = src[1];
@@ -751,7 +750,6 @@ gemv_trit_lut_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
             const int tok = divided(item, p.row_blocks_inv), r0 = (item - tok * blocks_per_tok) * 8;
             const float4 *src = reinterpret_cast<const float4 *>(part + tok * prow + r0);
             float4 lo = src[0], hi = src[1];
-#pragma unroll 4
             for (int w = 1; w < p.k_warps; ++w) {
                 src = reinterpret_cast<const float4 *>(part + (size_t)w * plane + tok * prow + r0);
                 const float4 a = src[0], b = src[1];
@@ -767,7 +765,6 @@ gemv_trit_lut_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
         for (int item = threadIdx.x; item < kTokPad * span_blocks; item += all_threads) {
             const int tok = divided(item, p.span_blocks_inv), r0 = (item - tok * span_blocks) * 8;
             float v[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll 4
             for (int rk = 0; rk < slices; ++rk) {
                 const float4 *src = reinterpret_cast<const float4 *>(recv + (size_t)rk * slot + tok * spitch + r0);
                 const float4 lo = src[0], hi = src[1];
