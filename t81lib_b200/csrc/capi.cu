@@ -155,6 +155,13 @@ extern "C" size_t t81b200_gemm_trit_workspace_bytes(int b_dtype, int layout, int
 // Contractions up to this length always have a launch shape of the streaming kernel (16 fp32 rows of B included).
 constexpr int64_t kT2StreamingMaxK = 14336;
 
+// The hint for the slice from row n0 on of a call of N rows.  Where the first slice waits, it releases the others once everything
+// ahead of the call is complete, and they run on the hint.  Where a capture lets it start early, each of the others is held against
+// what may still run and waits before it stores (gemv_trit_lut_launch), which costs more from five slices on than the early start
+// gives (behind a product of 16 rows, 512 x 512, 64 / 80 / 128 rows: 11.9 / 13.9 / 20.0 us with it, 12.4 / 13.3 / 16.2 without;
+// 2048 x 2048: 13.6 / 15.7 / 22.8 and 15.2 / 17.2 / 22.3): there the first one waits, hint -1.
+static int slice_hint(int hint, int64_t n0, int64_t N) { return n0 > 0 ? 1 : (hint == 0 && N > 64 ? -1 : hint); }
+
 static int gemm_trit_local(const uint8_t *A, const float *row_scale, const void *B, int b_dtype, int layout,
                            int64_t ldb, const float *bias, void *C, int c_dtype, int64_t ldc, int64_t M,
                            int64_t N, int64_t K, float alpha, float beta, void *workspace,
@@ -327,9 +334,8 @@ static int gemm_trit_local(const uint8_t *A, const float *row_scale, const void 
     if (a_aligned && layout == T81B200_LAYOUT_NK && N <= 16 && K > 0)
         return gemv_trit_launch(A, row_scale, B, b_dtype, ldb, bias, C, c_dtype, ldc, M, (int)N, K, alpha, beta, st, ctx);
     // 17 to 128 rows of B: one launch of the streaming kernel per 16 rows where streaming_wins says so, or where the tiles would
-    // need scratch memory that the caller has not lent.  A later slice reads and writes nothing an earlier one touches and is
-    // released by it only once its own input is complete: the slices are flagged independent and overlap.  Not with peers: the
-    // exchange protocol counts calls, not slices.
+    // need scratch memory that the caller has not lent.  A later slice reads and writes nothing an earlier one touches: the slices
+    // are flagged independent and overlap (slice_hint).  Not with peers: the exchange protocol counts calls, not slices.
     const size_t need = gemm_trit_tc_scratch(B, b_dtype, layout, ldb, N, K, 2);
     const bool tiles = need == 0 || (workspace && workspace_bytes >= need && reinterpret_cast<uintptr_t>(workspace) % 16 == 0 && worth_staging(M, N, K));
     if (a_aligned && layout == T81B200_LAYOUT_NK && K > 0 && !ctx && N <= T81B200_T2_MAX_ROWS && !(b_dtype == T81B200_F32 && fp32_exact(M, N, K)) && (!tiles || streaming_wins(M, N, K, 1.4))) {
@@ -337,7 +343,7 @@ static int gemm_trit_local(const uint8_t *A, const float *row_scale, const void 
         const int hint = t81b200::g_hint_independent;
         int rc = T81B200_OK;
         for (int64_t n0 = 0; n0 < N && rc == T81B200_OK; n0 += 16) {
-            if (n0 > 0) t81b200::g_hint_independent = 1;
+            t81b200::g_hint_independent = slice_hint(hint, n0, N);
             rc = gemv_trit_launch(A, row_scale, static_cast<const char *>(B) + n0 * ldb * esz_b, b_dtype, ldb, bias,
                                   static_cast<char *>(C) + n0 * ldc * esz_c, c_dtype, ldc, M, (int)(N - n0 < 16 ? N - n0 : 16), K, alpha,
                                   beta, st, nullptr);
@@ -387,15 +393,14 @@ extern "C" int t81b200_gemm_trit_t2(int n_group, const uint8_t *const *t2, const
     if (int rc = check_device()) return rc;
     if (N == 0) return T81B200_OK;
     // The kernel takes 16 rows of B at a time; more rows run as one launch per 16.  A later slice reads and writes
-    // nothing an earlier one touches, and an earlier slice releases it only once its own input is complete, so the
-    // slices are flagged independent of their predecessor and overlap.
+    // nothing an earlier one touches, so the slices are flagged independent of their predecessor and overlap (slice_hint).
     const int64_t esz_b = (int64_t)dtype_size(b_dtype), esz_c = (int64_t)dtype_size(c_dtype);
     const int hint = t81b200::g_hint_independent;
     int rc = T81B200_OK;
     for (int64_t n0 = 0; n0 < N && rc == T81B200_OK; n0 += 16) {
         void *Cs[T81B200_MAX_GROUP];
         for (int i = 0; i < n_group; ++i) Cs[i] = static_cast<char *>(C[i]) + n0 * ldc * esz_c;
-        if (n0 > 0) t81b200::g_hint_independent = 1;
+        t81b200::g_hint_independent = slice_hint(hint, n0, N);
         rc = gemv_trit_lut_launch(1, n_group, t2, row_scale, bias, Cs, M, static_cast<const char *>(B) + n0 * ldb * esz_b, b_dtype, ldb,
                                   c_dtype, ldc, (int)(N - n0 < 16 ? N - n0 : 16), K, alpha, beta, static_cast<cudaStream_t>(stream), nullptr);
     }

@@ -646,11 +646,12 @@ size_t gemv_smem_bytes(int planes, int ntok, int tokpad, int lps, int warps, int
 // Shape choice and launch of the TMA-fed kernel.  Returns T81B200_EALIGN when no configuration
 // fits (the caller then uses the register-prefetch kernel).
 extern thread_local int g_hint_independent;
+bool hint_holds(cudaStream_t st);  // gemv_trit_lut.cu: not behind a product that a capture started early
 
 int gemv_trit_tma_launch(const GemvParams &base, int x_dtype, int c_dtype, cudaStream_t st, const PeerCtx *ctx) {
     GemvTmaParams tp;
     tp.g = base;
-    tp.independent = (g_hint_independent && !(ctx && ctx->sync_local)) ? 1 : 0;
+    tp.independent = (g_hint_independent > 0 && !(ctx && ctx->sync_local) && hint_holds(st)) ? 1 : 0;
     tp.sync_local = ctx ? ctx->sync_local : nullptr;
     for (int i = 0; i < T81B200_MAX_PEERS; ++i) tp.sync_peer[i] = tp.sync_local && i < ctx->n_peers ? ctx->sync_slots[i] : nullptr;
     const int ntok = base.ntok;

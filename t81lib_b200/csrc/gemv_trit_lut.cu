@@ -128,7 +128,7 @@ struct GemvLutParams {
     uint32_t ntok_inv, row_blocks_inv, span_blocks_inv;  // inverse(d) of: ntok; eights of rows of a CTA; those that one CTA of a cluster finishes
     int vec_x;               // 1: rows of X start on 16-byte boundaries
     int bulk_x;              // 1: 16-bit activations, 16-byte aligned rows, K % 8 == 0: fetched by bulk copies
-    int independent;         // reads nothing the previous kernel of the stream wrote: 1 stores without waiting for it too (the caller says so), 2 waits before it stores
+    int independent;         // reads nothing the previous kernel of the stream wrote: 1 stores without waiting for it too (the caller says so), 2 waits before it stores (gemv_trit_lut_launch)
     int n_peers;             // other GPUs whose result receives every output element too (one segment only)
     void *peer_C[T81B200_MAX_PEERS];
     uint32_t *sync_local;
@@ -1017,7 +1017,7 @@ int launch_lut_xt(const Plan &pl, const GemvLutParams &p, int x_dtype, int c_dty
 
 }  // namespace
 
-extern thread_local int g_hint_independent;
+extern thread_local int g_hint_independent;  // 1: t81b200_hint_independent; -1: waits whatever is ahead (slice_hint in capi.cu)
 
 namespace {
 
@@ -1028,15 +1028,23 @@ namespace {
 // whose activations, scales and biases do not touch that result need not wait before it reads them (GemvLutParams::independent
 // == 2); it waits before it stores, so nothing is written earlier than it was, and whoever waits for it waits for both.
 // Products that started so add up: their results are kept here until one waits first again.  Outside a capture nothing tells
-// what else the stream holds, and every product waits.  Two decoder blocks of 14 products (8 tokens): 102.2 -> 94.2 to 96.2 us.
+// what else the stream holds, and every product waits.  Two decoder blocks of 14 products (8 tokens): 102.2 -> 96.5 us.
+//
+// A product that started early has let its successor start with the one ahead of it still running, which the promise of
+// t81b200_hint_independent does not cover: it speaks of the kernels back to the last unhinted one.  So in a capture a hinted product
+// (one of the later slices of 17 to 128 rows, too) takes the caller's word (independent == 1) only behind a product that this
+// thread knows to have waited first or to have been hinted behind such a one; behind one that started early it is looked at like
+// any other, and waits before it stores at the least.
 struct Bytes {
     uintptr_t from, to;
 };
 struct InFlight {
     unsigned long long capture = 0;  // 0: none
-    cudaGraphNode_t node = nullptr;
+    cudaGraphNode_t node = nullptr;  // the product captured last
+    bool early = false;              // it let its successor start before what is ahead of it was complete, on its own account
+    bool listed = false;             // `result` has all that may still be written once its CTAs have started
     int n = 0;
-    Bytes result[4 * kMaxSeg];
+    Bytes result[8 * kMaxSeg];
 };
 thread_local InFlight g_in_flight;
 
@@ -1055,12 +1063,22 @@ unsigned long long capturing(cudaStream_t st, cudaGraphNode_t &node) {
     return status == cudaStreamCaptureStatusActive ? capture : 0;
 }
 
+bool known_ahead(unsigned long long capture, cudaGraphNode_t ahead) {
+    return capture && ahead && g_in_flight.capture == capture && g_in_flight.node == ahead;
+}
+
 Bytes extent(const void *p, int64_t rows, int64_t ld, int64_t cols, size_t size) {
     const uintptr_t at = reinterpret_cast<uintptr_t>(p);
     return {at, p ? at + (uintptr_t)(((rows - 1) * ld + cols) * (int64_t)size) : at};
 }
 
 }  // namespace
+
+bool hint_holds(cudaStream_t st) {
+    cudaGraphNode_t ahead = nullptr;
+    const unsigned long long capture = capturing(st, ahead);
+    return !capture || (known_ahead(capture, ahead) && !g_in_flight.early);
+}
 
 // Launch of the streaming kernel over n_seg weight matrices that share X.  NK layout, ntok in 1..16, every A
 // 16-byte aligned; fmt 0: A in the packed-limb layout (table decode), fmt 1: A in the decode-stream layout.
@@ -1114,11 +1132,12 @@ int gemv_trit_lut_launch(int fmt, int n_seg, const uint8_t *const *A, const floa
     for (int i = 0; i < T81B200_MAX_PEERS; ++i) p.peer_C[i] = i < p.n_peers ? ctx->peer_C[i] : nullptr;
     p.sync_local = ctx ? ctx->sync_local : nullptr;
     for (int i = 0; i < T81B200_MAX_PEERS; ++i) p.sync_peer[i] = p.sync_local && i < ctx->n_peers ? ctx->sync_slots[i] : nullptr;
-    p.independent = (g_hint_independent && !p.sync_local) ? 1 : 0;
     for (int j = 0; j < 8; ++j) p.shl[j] = 1u << (2 * j);
     cudaGraphNode_t ahead = nullptr;
-    const unsigned long long capture = ctx || p.independent ? 0 : capturing(st, ahead);
-    if (capture && ahead && g_in_flight.capture == capture && g_in_flight.node == ahead && g_in_flight.n + n_seg <= (int)(sizeof g_in_flight.result / sizeof(Bytes))) {
+    const unsigned long long capture = capturing(st, ahead);
+    const bool known = known_ahead(capture, ahead);
+    p.independent = g_hint_independent > 0 && !p.sync_local && (!capture || (known && !g_in_flight.early)) ? 1 : 0;
+    if (!p.independent && g_hint_independent >= 0 && known && g_in_flight.listed && !ctx && g_in_flight.n + n_seg <= (int)(sizeof g_in_flight.result / sizeof(Bytes))) {
         bool apart = true;
         auto reads = [&](const Bytes &b) {
             for (int i = 0; i < g_in_flight.n; ++i) apart = apart && (b.to <= g_in_flight.result[i].from || g_in_flight.result[i].to <= b.from);
@@ -1138,9 +1157,11 @@ int gemv_trit_lut_launch(int fmt, int n_seg, const uint8_t *const *A, const floa
     const int rc = fmt == 1 ? launch_lut_xt<1>(pl, p, x_dtype, c_dtype, st) : launch_lut_xt<0>(pl, p, x_dtype, c_dtype, st);
     g_in_flight.capture = 0;
     if (rc == T81B200_OK && capture && capturing(st, ahead) == capture && ahead) {
-        for (int i = 0; i < n_seg; ++i) g_in_flight.result[g_in_flight.n++] = extent(C[i], ntok, ldc, M[i], dtype_size(c_dtype));
         g_in_flight.capture = capture;
         g_in_flight.node = ahead;
+        g_in_flight.early = p.independent == 2;
+        g_in_flight.listed = p.independent != 1 && !ctx;
+        for (int i = 0; g_in_flight.listed && i < n_seg; ++i) g_in_flight.result[g_in_flight.n++] = extent(C[i], ntok, ldc, M[i], dtype_size(c_dtype));
     }
     return rc;
 }

@@ -1,6 +1,7 @@
 """Decode-sized products fetch their weights ahead of the kernel before them, except behind one that wrote weights: the kinds of edges
 in a captured graph, which is where the launches' order can be read, and training steps whose weights change from step to step."""
 
+import contextlib
 import ctypes
 
 import numpy as np
@@ -8,6 +9,7 @@ import pytest
 import torch
 
 import oracle
+from _graph_nodes import capture, kernels
 
 pytestmark = pytest.mark.gpu
 
@@ -192,3 +194,140 @@ def test_captured_products_whose_buffers_touch(ops, overlap):
             buffers[id(y)] = (buffers[id(x)] @ trits.double().t()).to(torch.bfloat16).double()
         for t in (a, b, c):
             assert torch.equal(t.double(), buffers[id(t)])
+
+
+def _products(graph):
+    """The parameter blocks of a graph's streaming products, in the order of their capture."""
+    return [parameter(3) for name, parameter in kernels(graph) if "gemv_trit_lut_kernel" in name]  # three tensor maps, then the block
+
+
+@pytest.fixture(scope="module")
+def forms(ops):
+    """What a graph's products do, in order: "waits" before anything, "reads" early and waits before it stores, or "runs" on the caller's
+    word.  Where a parameter block says so is found from one product captured twice, whose second launch differs in that alone."""
+    trits = torch.ones(32, 192, device="cuda")
+    t2, x, y = ops.pack_t2(ops.quantize_pack(trits, 0.5, "fixed")[0], 32, 192), torch.ones(1, 192, device="cuda", dtype=torch.bfloat16), []
+    out = torch.empty(1, 32, device="cuda", dtype=torch.bfloat16)
+    a, b = _products(capture(lambda: [ops.gemm_trit_t2([t2], [32], x, K=192, outs=[out]) for _ in range(2)]))
+    (at,) = np.nonzero(a != b)[0]
+    assert (a[at], b[at]) == (0, 2)
+    return lambda graph: [("waits", "runs", "reads")[block[at]] for block in _products(graph)]
+
+
+class _Weights:
+    """Sparse weights, in either layout: products of small whole numbers are small whole numbers, exact in every type and order."""
+
+    def __init__(self, ops, layout, n=4, size=512):
+        gen = torch.Generator(device="cuda").manual_seed(size)
+        self.ops, self.layout, self.size = ops, layout, size
+        self.trits = [torch.randint(-1, 2, (size, size), generator=gen, device="cuda").float() * (torch.rand(size, size, generator=gen, device="cuda") < 0.01)
+                      for _ in range(n)]
+        packed = [ops.quantize_pack(t, 0.5, "fixed")[0] for t in self.trits]
+        self.packed = packed if layout == "limbs" else [ops.pack_t2(p, size, size) for p in packed]
+
+    def __call__(self, i, x, out, scale=None, bias=None, beta=0.0):
+        if self.layout == "limbs":
+            return self.ops.gemm_trit(self.packed[i], x, M=self.size, K=self.size, layout="nk", row_scale=scale, bias=bias, C=out, beta=beta)
+        return self.ops.gemm_trit_t2([self.packed[i]], [self.size], x, K=self.size, row_scales=[scale], biases=[bias], outs=[out], beta=beta)[0]
+
+    def want(self, i, x, out=None, scale=None, bias=None, beta=0.0):
+        y = (x.double() @ self.trits[i].double().t()) * (1.0 if scale is None else scale.double()) + (0.0 if bias is None else bias.double())
+        return y if beta == 0.0 else y + beta * out.double()
+
+
+def _replayed(graph, tensors, check, seed=0):
+    """Replays on new whole numbers in every tensor; `check` gets copies of what they held before."""
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    for _ in range(20):
+        for t in tensors:
+            t.copy_(torch.randint(-1, 2, t.shape, generator=gen, device="cuda"))
+        before = [t.clone() for t in tensors]
+        graph.replay()
+        check(*before)
+
+
+# Calls of more than 16 rows are slices of the kernel; behind a product that writes the rows of a later slice, and one whose input lies
+# where a later slice stores, no slice runs on the word of the call alone.
+@pytest.mark.parametrize("layout", ["limbs", "codes"])
+@pytest.mark.parametrize("case", ["reads", "stores", "adds"])
+def test_slices_behind_a_captured_product(ops, forms, layout, case):
+    w, bf = _Weights(ops, layout), torch.bfloat16
+    x, buf, out = (torch.zeros(r, w.size, device="cuda", dtype=bf) for r in (16, 32, 32))
+    first = torch.empty(16, w.size, device="cuda", dtype=bf)
+    if case == "reads":      # the second slice's input is the product's result
+        work = lambda: (w(0, x, buf[16:]), w(1, buf, out))
+    elif case == "stores":   # the second slice's result lies over the product's input
+        work = lambda: (w(0, out[16:], first), w(1, buf, out))
+    else:                    # and adds to what the product wrote
+        work = lambda: (w(0, x, out[16:]), w(1, buf, out, beta=1.0))
+    graph = capture(work)
+
+    def check(x0, buf0, out0):
+        if case == "reads":
+            buf0[16:] = w.want(0, x0).to(bf)
+            assert torch.equal(buf, buf0) and torch.equal(out, w.want(1, buf0).to(bf))
+        elif case == "stores":
+            assert torch.equal(first, w.want(0, out0[16:]).to(bf)) and torch.equal(out, w.want(1, buf0).to(bf))
+        else:
+            out0[16:] = w.want(0, x0).to(bf)
+            assert torch.equal(out, w.want(1, buf0, out0, beta=1.0).to(bf))
+    assert forms(graph) == {"reads": ["waits", "reads", "waits"], "stores": ["waits", "reads", "reads"], "adds": ["waits", "reads", "reads"]}[case]
+    _replayed(graph, (x, buf, out), check)
+
+
+# From five slices on the first one waits, and the others run beside it.
+def test_many_slices_behind_a_captured_product(ops, forms):
+    w = _Weights(ops, "codes")
+    x, buf, out = (torch.zeros(r, w.size, device="cuda", dtype=torch.bfloat16) for r in (16, 80, 80))
+    graph = capture(lambda: (w(0, x, buf[64:]), w(1, buf, out)))
+    assert forms(graph) == ["waits", "waits", "runs", "runs", "runs", "runs"]
+
+    def check(x0, buf0, _):
+        buf0[64:] = w.want(0, x0).to(torch.bfloat16)
+        assert torch.equal(out, w.want(1, buf0).to(torch.bfloat16))
+    _replayed(graph, (x, buf, out), check)
+
+
+# A hint speaks of the kernels back to the last unhinted one: it is taken at its word behind one that waited first, not behind one that
+# started early, nor behind what another thread captured.
+@pytest.mark.parametrize("layout", ["limbs", "codes"])
+def test_hints_behind_captured_products(ops, forms, layout):
+    w = _Weights(ops, layout)
+    x, a, b, c, d = (torch.zeros(8, w.size, device="cuda", dtype=torch.bfloat16) for _ in range(5))
+    hinted = ops.independent_of_previous
+
+    def chain(*steps):
+        def work():
+            for i, (hint, src, dst) in enumerate(steps):
+                with hinted() if hint else contextlib.nullcontext():
+                    w(i, src, dst)
+
+        graph = capture(work)
+
+        def check(*before):
+            held = {t.data_ptr(): v for t, v in zip((x, a, b, c, d), before)}
+            for i, (_, src, dst) in enumerate(steps):
+                held[dst.data_ptr()] = w.want(i, held[src.data_ptr()]).to(torch.bfloat16)
+            for t in (x, a, b, c, d):
+                assert torch.equal(t, held[t.data_ptr()])
+        _replayed(graph, (x, a, b, c, d), check)
+        return forms(graph)
+    assert chain((0, x, a), (0, x, b), (1, a, c)) == ["waits", "reads", "waits"]
+    assert chain((0, x, a), (0, x, b), (1, x, c), (1, x, d)) == ["waits", "reads", "reads", "reads"]
+    assert chain((0, x, a), (0, x, b), (1, a, c), (1, x, d)) == ["waits", "reads", "waits", "runs"]
+    assert chain((0, x, a), (1, x, b), (1, x, c), (0, x, d)) == ["waits", "runs", "runs", "waits"]
+
+    import threading
+
+    def work():
+        stream = torch.cuda.current_stream()
+
+        def other():
+            with torch.cuda.stream(stream), hinted():
+                w(2, a, c)
+        w(0, x, a)
+        w(1, x, b)
+        thread = threading.Thread(target=other)
+        thread.start()
+        thread.join()
+    assert forms(capture(work)) == ["waits", "reads", "waits"]
