@@ -608,20 +608,47 @@ int launch_warps(const T *w, int64_t rows, int64_t cols, int64_t ld, float thr, 
                          (size_t)(kWarpRows * each) * slot_bytes, st, w, (int)rows, (int)cols, ld, thr, packed, row_scale, each, (int)slot_bytes);
 }
 
-// The forms that stage rows in shared memory, for enough rows to give every SM a few; 1 where neither applies.  A warp to a row where 24
-// rows fit beside each other, else teams where four do: with fewer rows in flight the warps wait for memory (us, absmean, warps against
-// teams: 8000 x 4096 bf16 24.2 and 25.5, 9000 x 2816 fp32 23.2 and 22.8, 4096 x 4096 fp32 16.4 and 13.7, 4096 x 14336 bf16 51 and 36).
-// Rows on 16-byte boundaries, teams before and warps now: 14336 x 1024 bf16 31.7 -> 13.1, 14336 x 1152 fp32 30.7 -> 15.1, 9892 x 2936
-// bf16 26.7 -> 21.3.  Off them, by the row kernel before: 9892 x 2933 bf16 60.6 -> 29.5, 4095 x 9001 bf16 75.0 -> 29.5, 8006 x 3077 fp32
-// 34.9 -> 31.1, 1500 x 14335 fp32 42.4 -> 25.9.
+// The forms that stage rows in shared memory, for enough rows to give every SM a few; 1 where the row kernel is to take them.
+//
+// A warp to a row keeps 24 rows of an SM in flight and shares nothing, but a row is one warp's work: with few rows an SM most of
+// the 24 have none, and a long row takes long.  So the shorter the rows (in chunks of 384 columns), the fewer of them it needs.
+// Under the absmean rule, which goes through a row twice, rows of which one warp has no second slot need whole waves of 24 an SM,
+// the last at least two thirds full over all.  Off 16-byte boundaries groups are cut out of aligned pieces, which short rows of
+// few-row matrices do not win back; the row kernel, six CTAs an SM, steps up behind six rows an SM.  us a call, absmean, row kernel / teams / warps, at 297, 800, 1184, 3552, 4096, 10000 rows:
+//   1024 fp32                    2.5 2.9 2.8   3.8 3.9 3.2   5.5 4.7 3.9   9.7 9.1 5.8    10.8 10.3 7.2   21.5 22.2 12.6
+//   4096 bf16                    4.6 3.5 5.1   8.7 5.1 6.4   14.5 6.0 6.8  28.8 12.6 12.5 33.5 14.6 15.9  78.8 31.9 28.7
+//   2049 fp32, off boundaries    3.1 4.0 5.0   5.4 5.7 6.3   7.6 6.5 6.7   14.7 12.7 11.2 16.4 14.3 14.9  35.1 31.7 25.4
+//   4097 bf16, off boundaries    5.5 4.7 7.7   10.8 6.6 9.0  16.6 8.0 9.5  32.1 16.1 16.6 36.5 18.6 23.0  89.3 40.9 41.1
+// Over 13 x 33 sizes from 297 x 64 to 14336 x 6144, both rules, fp32 and bf16, the choice is 0.2 % behind the best form on average.
+template <bool ABSMEAN, bool ALIGNED>
+bool suits_warps(int64_t rows, int64_t chunks, size_t element, int64_t slots_each) {
+    const int64_t sms = sm_count(), wave = sms * kWarpRows * kWarpCtas, waves = (rows + wave - 1) / wave;
+    if (slots_each < 1) return false;
+    if (!ABSMEAN && ALIGNED) return slots_each > 1 || chunks <= 6 || rows >= (chunks <= 8 ? 3 * sms : wave);
+    if (!ABSMEAN && slots_each > 1) return element == 2 || chunks <= 2 ? 3 * rows >= 10 * sms : rows >= 4 * sms;
+    if (!ABSMEAN) return chunks <= 9 ? rows > 6 * sms : rows >= wave;
+    if (rows >= wave && 3 * rows >= 2 * waves * wave) return true;
+    if (ALIGNED) return chunks <= 3 || ((slots_each > 1 || chunks <= 4) && rows >= 5 * sms);
+    return chunks <= 3 ? rows >= 5 * sms : (chunks <= 5 ? rows > 6 * sms : chunks == 6 && slots_each > 1 && rows >= 8 * sms);
+}
+// Teams or the row kernel, off 16-byte boundaries: the row kernel reads single elements there, but has all rows of a small matrix
+// under way at once.
+bool suits_teams_off_boundaries(int64_t rows, int64_t chunks, size_t element) {
+    const int64_t sms = sm_count();
+    if (chunks < 6) return false;
+    if (element == 2) return 3 * rows >= 10 * sms || chunks >= 11;
+    return rows > 6 * sms || chunks >= 16 || (rows >= 5 * sms && chunks >= 13);
+}
+
 template <typename T, bool ABSMEAN, bool ALIGNED>
 int launch_staged_rows(const T *w, int64_t rows, int64_t cols, int64_t ld, float thr, uint8_t *packed, float *row_scale, cudaStream_t st) {
     const int64_t row_bytes = cols * (int64_t)sizeof(T), slot_bytes = (row_bytes + (ALIGNED ? 0 : 30) + 127) / 128 * 128;
     if (rows < 2 * (int64_t)sm_count() || rows >= (1ll << 31)) return 1;
-    const int64_t each = (kRingBytes / kWarpCtas - 1024) / (kWarpRows * slot_bytes);
-    if (each >= 1) return launch_warps<T, ABSMEAN, ALIGNED>(w, rows, cols, ld, thr, packed, row_scale, slot_bytes, each > 1 ? 2 : 1, st);
+    const int64_t chunks = (cols + 4 * kChunkGroups - 1) / (4 * kChunkGroups), each = (kRingBytes / kWarpCtas - 1024) / (kWarpRows * slot_bytes);
+    if (suits_warps<ABSMEAN, ALIGNED>(rows, chunks, sizeof(T), each))
+        return launch_warps<T, ABSMEAN, ALIGNED>(w, rows, cols, ld, thr, packed, row_scale, slot_bytes, each > 1 ? 2 : 1, st);
     const int fit = (int)(kRingBytes / slot_bytes);  // rows the ring holds; a team needs one, and one more in flight
-    if (fit < 4) return 1;
+    if (fit < 4 || (!ALIGNED && !suits_teams_off_boundaries(rows, chunks, sizeof(T)))) return 1;
     if (fit >= 12) return launch_ring<T, ABSMEAN, 6, ALIGNED>(w, rows, cols, ld, thr, packed, row_scale, slot_bytes, st);
     return launch_ring<T, ABSMEAN, 4, ALIGNED>(w, rows, cols, ld, thr, packed, row_scale, slot_bytes, st);
 }
