@@ -718,19 +718,26 @@ __device__ __forceinline__ void store_planes(const float (&v)[4], __nv_bfloat16 
     }
 }
 
-// (N, K) layout: a thread moves four consecutive k of one token, eight of a 16-bit type; whole 16- / 8-byte loads where the rows allow
-// them.  16-bit rows elsewhere are read in words, which lie one element off those of the result where a row starts between two
-// of them (8192 tokens of 2047: 17.5 us element by element, 13.4 so); no word reaches past the row.
-template <int PLANES> constexpr int kStageWidth = PLANES == 0 ? 8 : 4;
-template <typename T, int PLANES>
+// (N, K) layout: a thread moves WIDTH consecutive k of one token; whole 16- / 8-byte loads where the rows allow them.  Four, and eight
+// of much 16-bit data: there rows elsewhere are read in words, which lie one element off those of the result where a row starts
+// between two of them (8192 tokens of 2047: 17.5 us element by element, 13.4 so); no word reaches past the row.
+template <typename T, int PLANES, int WIDTH>
 __global__ void __launch_bounds__(256) stage_rows_kernel(const T *__restrict__ B, int64_t ldb, int64_t N, int64_t K, __nv_bfloat16 *__restrict__ out,
                                                          int64_t kpad, int64_t plane_elems, bool vec) {
     wait_for_kernel_ahead();
-    const int64_t n = (int64_t)blockIdx.x * blockDim.y + threadIdx.y, k = ((int64_t)blockIdx.y * blockDim.x + threadIdx.x) * kStageWidth<PLANES>;
+    const int64_t n = (int64_t)blockIdx.x * blockDim.y + threadIdx.y, k = ((int64_t)blockIdx.y * blockDim.x + threadIdx.x) * WIDTH;
     if (n >= N || k >= kpad) return;
     const T *src = B + n * ldb + k;
     __nv_bfloat16 *dst = out + n * kpad + k;
-    if constexpr (PLANES == 0) {  // bit copy of a 16-bit type
+    if constexpr (PLANES == 0 && WIDTH == 4) {  // bit copy of a 16-bit type
+        uint16_t e[4] = {0, 0, 0, 0};
+        const uint16_t *s16 = reinterpret_cast<const uint16_t *>(src);
+        if (vec && k + 4 <= K) *reinterpret_cast<uint2 *>(e) = *reinterpret_cast<const uint2 *>(src);
+        else
+#pragma unroll
+            for (int i = 0; i < 4; ++i) if (k + i < K) e[i] = s16[i];
+        *reinterpret_cast<uint2 *>(dst) = *reinterpret_cast<const uint2 *>(e);
+    } else if constexpr (PLANES == 0) {
         const uint16_t *s16 = reinterpret_cast<const uint16_t *>(src);
         uint32_t w[4] = {0u, 0u, 0u, 0u};
         if (k + 8 > K) {
@@ -804,12 +811,24 @@ int launch_stage(const void *B, int layout, int64_t ldb, int64_t N, int64_t K, _
         if (grid.y > 65535u) return fail(T81B200_ELIMIT, "gemm_trit: K too large");
         T81_CUDA_TRY(launch_behind(stage_columns_kernel<T, PLANES>, grid, 256, st, src, ldb, N, K, out, kpad, plane_elems));
     } else {
-        // a row's pieces side by side, and as many rows of few pieces as 256 threads take
-        const int64_t pieces = (kpad + kStageWidth<PLANES> - 1) / kStageWidth<PLANES>, across = pieces < 256 ? (pieces + 31) / 32 * 32 : 256;
-        const dim3 block((unsigned)across, (unsigned)(256 / across)), grid((unsigned)((N + block.y - 1) / block.y), (unsigned)((pieces + 255) / 256));
-        if (grid.y > 65535u) return fail(T81B200_ELIMIT, "gemm_trit: K too large");
         const bool vec = reinterpret_cast<uintptr_t>(B) % (4 * sizeof(T)) == 0 && ldb % 4 == 0;
-        T81_CUDA_TRY(launch_behind(stage_rows_kernel<T, PLANES>, grid, block, st, src, ldb, N, K, out, kpad, plane_elems, vec));
+        auto launch = [&](auto width) -> int {
+            constexpr int W = decltype(width)::value;
+            // a row's pieces side by side, and as many rows of few pieces as 256 threads take
+            const int64_t pieces = (kpad + W - 1) / W, across = pieces < 256 ? (pieces + 31) / 32 * 32 : 256;
+            const dim3 block((unsigned)across, (unsigned)(256 / across)), grid((unsigned)((N + block.y - 1) / block.y), (unsigned)((pieces + 255) / 256));
+            if (grid.y > 65535u) return fail(T81B200_ELIMIT, "gemm_trit: K too large");
+            T81_CUDA_TRY(launch_behind(stage_rows_kernel<T, PLANES, W>, grid, block, st, src, ldb, N, K, out, kpad, plane_elems, vec));
+            return T81B200_OK;
+        };
+        // Eight k a thread are half the loads in flight and no shorter a chain, so up to 1.5 million elements four are faster, or up to a
+        // third of that where four leave more than a tenth of the lanes idle (whole products, us, eight and four: 1000 tokens of 1023 by
+        // 2048 features 13.36 and 12.78, 200 of 4095 by 4096 18.89 and 17.99, 3000 of 513 by 600 12.20 and 13.78).
+        if constexpr (PLANES == 0) {
+            const int64_t pieces = (kpad + 3) / 4, lanes = pieces < 256 ? (pieces + 31) / 32 * 32 : (pieces + 255) / 256 * 256;
+            if (plane_elems > (10 * pieces >= 9 * lanes ? 3 << 19 : 1 << 19)) return launch(std::integral_constant<int, 8>{});
+        }
+        return launch(std::integral_constant<int, 4>{});
     }
     return T81B200_OK;
 }

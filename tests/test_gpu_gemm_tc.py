@@ -6,6 +6,7 @@ import pytest
 import torch
 
 import oracle
+from _graph_nodes import capture, kernels
 
 pytestmark = pytest.mark.gpu
 
@@ -188,3 +189,19 @@ def test_tc_rows_off_boundaries(dev, dtype, out_f, in_f, tokens):
     wide[:, 1:in_f + 1] = x
     assert torch.equal(ops.linear_t2(t2, out_f, wide[:, 1:in_f + 1], in_f, None, None), want)
     assert _capi.kernel_status(reset=True) == 0
+
+
+# Staged 16-bit rows: four k a thread up to a size, eight beyond it; less where four leave many lanes idle (513: 130 pieces on 160 lanes).
+@pytest.mark.parametrize("in_f,tokens,width", [(1023, 1536, 4), (1023, 1537, 8), (513, 1008, 4), (513, 1009, 8), (2047, 17, 4), (2047, 768, 4), (2047, 769, 8)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_staged_rows_by_size(dev, in_f, tokens, width, dtype):
+    from t81lib_b200 import ops
+    gen = torch.Generator(device="cuda").manual_seed(tokens)
+    trits = torch.randint(-1, 2, (130, in_f), generator=gen, device="cuda").float()
+    t2 = ops.pack_t2(ops.quantize_pack(trits, 0.5, "fixed")[0], 130, in_f)
+    x = torch.randint(-1, 2, (tokens, in_f), generator=gen, device="cuda").to(dtype)
+    x[torch.rand(tokens, in_f, generator=gen, device="cuda") < 0.8] = 0
+    got = []
+    staging = [name for name, _ in kernels(capture(lambda: got.append(ops.linear_t2(t2, 130, x, in_f, None, None)))) if "stage_rows_kernel" in name]
+    assert len(staging) == 1 and f"Li0ELi{width}E" in staging[0]
+    assert torch.equal(got[0], (x.double() @ trits.double().t()).to(dtype))
