@@ -331,3 +331,59 @@ def test_hints_behind_captured_products(ops, forms, layout):
         thread.start()
         thread.join()
     assert forms(capture(work)) == ["waits", "reads", "waits"]
+
+
+# Scales and biases that a product in flight writes, of one matrix and of any of a group's; groups of which nothing touches it read early.
+@pytest.mark.parametrize("touch", ["scale", "bias", "a group's scale", "a group's bias", "nothing"])
+def test_vectors_of_a_captured_product(ops, forms, touch):
+    w = _Weights(ops, "codes")
+    x = torch.zeros(1, w.size, device="cuda")
+    vector, y, z = (torch.zeros(1, w.size, device="cuda") for _ in range(3))
+    at = lambda kind: vector[0] if kind in touch else None
+
+    def work():
+        w(0, x, vector)
+        if "group" in touch or touch == "nothing":
+            ops.gemm_trit_t2(w.packed[1:3], [w.size] * 2, x, K=w.size, outs=[y, z], row_scales=[None, at("scale")], biases=[None, at("bias")])
+        else:
+            w(2, x, z, scale=at("scale"), bias=at("bias"))
+    graph = capture(work)
+    assert forms(graph) == ["waits", "reads" if touch == "nothing" else "waits"]
+
+    def check(x0, *_):
+        held = w.want(0, x0)
+        assert torch.equal(vector, held.float())
+        scale, bias = (held[0] if kind in touch else None for kind in ("scale", "bias"))
+        assert torch.equal(z, w.want(2, x0, scale=scale, bias=bias).float())
+        if "group" in touch or touch == "nothing":
+            assert torch.equal(y, w.want(1, x0).float())
+    _replayed(graph, (x, vector, y, z), check)
+
+
+# Two streams in one capture: what follows a join, or another stream's product, waits.
+def test_captured_streams_that_fork_and_join(ops, forms):
+    w = _Weights(ops, "codes", n=6)
+    x, a, b, c, d, e, f = (torch.zeros(8, w.size, device="cuda", dtype=torch.bfloat16) for _ in range(7))
+    side = torch.cuda.Stream()
+
+    def work():
+        main = torch.cuda.current_stream()
+        w(0, x, a)
+        side.wait_stream(main)
+        w(1, x, b)
+        with torch.cuda.stream(side):
+            w(2, a, c)
+            w(3, a, d)
+        main.wait_stream(side)
+        w(4, d, e)
+        w(5, b, f)
+    graph = capture(work)
+    assert forms(graph) == ["waits", "reads", "waits", "reads", "waits", "reads"]
+
+    def check(x0, *_):
+        held = [w.want(0, x0).to(torch.bfloat16), w.want(1, x0).to(torch.bfloat16)]
+        held += [w.want(i, held[0]).to(torch.bfloat16) for i in (2, 3)]
+        held += [w.want(4, held[3]).to(torch.bfloat16), w.want(5, held[1]).to(torch.bfloat16)]
+        for got, want in zip((a, b, c, d, e, f), held):
+            assert torch.equal(got, want)
+    _replayed(graph, (x, a, b, c, d, e, f), check)
