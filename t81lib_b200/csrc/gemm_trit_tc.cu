@@ -723,8 +723,8 @@ __device__ __forceinline__ void store_planes(const float (&v)[4], __nv_bfloat16 
 // between two of them (8192 tokens of 2047: 17.5 us element by element, 13.4 so); no word reaches past the row.
 template <typename T, int PLANES, int WIDTH>
 __global__ void __launch_bounds__(256) stage_rows_kernel(const T *__restrict__ B, int64_t ldb, int64_t N, int64_t K, __nv_bfloat16 *__restrict__ out,
-                                                         int64_t kpad, int64_t plane_elems, bool vec) {
-    wait_for_kernel_ahead();
+                                                         int64_t kpad, int64_t plane_elems, bool vec, bool release) {
+    wait_for_kernel_ahead(release);
     const int64_t n = (int64_t)blockIdx.x * blockDim.y + threadIdx.y, k = ((int64_t)blockIdx.y * blockDim.x + threadIdx.x) * WIDTH;
     if (n >= N || k >= kpad) return;
     const T *src = B + n * ldb + k;
@@ -812,13 +812,17 @@ int launch_stage(const void *B, int layout, int64_t ldb, int64_t N, int64_t K, _
         T81_CUDA_TRY(launch_behind(stage_columns_kernel<T, PLANES>, grid, 256, st, src, ldb, N, K, out, kpad, plane_elems));
     } else {
         const bool vec = reinterpret_cast<uintptr_t>(B) % (4 * sizeof(T)) == 0 && ldb % 4 == 0;
+        // The product's CTAs wait beside this pass, or come as its blocks end.  The first is up to 3 % faster, except for many tokens of
+        // contractions up to four chunks, whose tiles then load and store all at once (fp32, 600 features, us, released early and
+        // late: 6000 tokens of 513 27.3 and 25.3, 9000 of 600 46.0 and 43.0).
+        const bool release = K > 768 || N < 2000;
         auto launch = [&](auto width) -> int {
             constexpr int W = decltype(width)::value;
             // a row's pieces side by side, and as many rows of few pieces as 256 threads take
             const int64_t pieces = (kpad + W - 1) / W, across = pieces < 256 ? (pieces + 31) / 32 * 32 : 256;
             const dim3 block((unsigned)across, (unsigned)(256 / across)), grid((unsigned)((N + block.y - 1) / block.y), (unsigned)((pieces + 255) / 256));
             if (grid.y > 65535u) return fail(T81B200_ELIMIT, "gemm_trit: K too large");
-            T81_CUDA_TRY(launch_behind(stage_rows_kernel<T, PLANES, W>, grid, block, st, src, ldb, N, K, out, kpad, plane_elems, vec));
+            T81_CUDA_TRY(launch_behind(stage_rows_kernel<T, PLANES, W>, grid, block, st, src, ldb, N, K, out, kpad, plane_elems, vec, release));
             return T81B200_OK;
         };
         // Eight k a thread are half the loads in flight and no shorter a chain, so up to 1.5 million elements four are faster, or up to a

@@ -13,11 +13,12 @@ namespace t81b200 {
 
 // A kernel that starts while the one ahead ends (programmatic stream serialization), and whose first statement is
 // wait_for_kernel_ahead: it touches no global memory before all of that kernel's writes are visible, and lets its own successor
-// start; so the order of memory is the stream's, and what overlaps is the launch (1 to 2 us between two short kernels).  Not for
-// kernels of many warps behind long ones, whose SMs they wait on: the absmax reduction behind a weight gradient cost that 2 %.
-__device__ __forceinline__ void wait_for_kernel_ahead() {
+// start (there, or with `release` false as its blocks end); so the order of memory is the stream's, and what overlaps is the launch
+// (1 to 2 us between two short kernels).  Not for kernels of many warps behind long ones, whose SMs they wait on: the absmax
+// reduction behind a weight gradient cost that 2 %.
+__device__ __forceinline__ void wait_for_kernel_ahead(bool release = true) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (release) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 template <typename... Params, typename... Args>
 cudaError_t launch_behind(void (*kernel)(Params...), dim3 grid, dim3 block, cudaStream_t st, Args &&...args) {

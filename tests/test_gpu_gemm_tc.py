@@ -192,7 +192,8 @@ def test_tc_rows_off_boundaries(dev, dtype, out_f, in_f, tokens):
 
 
 # Staged 16-bit rows: four k a thread up to a size, eight beyond it; less where four leave many lanes idle (513: 130 pieces on 160 lanes).
-@pytest.mark.parametrize("in_f,tokens,width", [(1023, 1536, 4), (1023, 1537, 8), (513, 1008, 4), (513, 1009, 8), (2047, 17, 4), (2047, 768, 4), (2047, 769, 8)])
+@pytest.mark.parametrize("in_f,tokens,width", [(1023, 1536, 4), (1023, 1537, 8), (513, 1008, 4), (513, 1009, 8), (2047, 17, 4), (2047, 768, 4), (2047, 769, 8), (703, 2000, 4),
+                                               (513, 2000, 8)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_staged_rows_by_size(dev, in_f, tokens, width, dtype):
     from t81lib_b200 import ops
