@@ -333,6 +333,7 @@ __device__ __forceinline__ void fetch_row(const T *row, uint32_t row_bytes, cons
             single(lead, first);
             single(last, lead + row_bytes);
         }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // this slot's later copies come behind these stores
         if (first < last) {
             mbar_arrive_expect_tx(bar, last - first);
             bulk_load(slot_addr + first, from + first, last - first, bar);
