@@ -809,7 +809,7 @@ int launch_stage(const void *B, int layout, int64_t ldb, int64_t N, int64_t K, _
     if (layout == T81B200_LAYOUT_KN) {
         const dim3 grid((unsigned)((N + 31) / 32), (unsigned)((kpad + 63) / 64));
         if (grid.y > 65535u) return fail(T81B200_ELIMIT, "gemm_trit: K too large");
-        T81_CUDA_TRY(launch_behind(stage_columns_kernel<T, PLANES>, grid, 256, st, src, ldb, N, K, out, kpad, plane_elems));
+        T81_CUDA_TRY(launch_behind(stage_columns_kernel<T, PLANES>, grid, 256, 0, st, src, ldb, N, K, out, kpad, plane_elems));
     } else {
         const bool vec = reinterpret_cast<uintptr_t>(B) % (4 * sizeof(T)) == 0 && ldb % 4 == 0;
         // The product's CTAs wait beside this pass, or come as its blocks end.  The first is up to 3 % faster, except for many tokens of
@@ -822,7 +822,7 @@ int launch_stage(const void *B, int layout, int64_t ldb, int64_t N, int64_t K, _
             const int64_t pieces = (kpad + W - 1) / W, across = pieces < 256 ? (pieces + 31) / 32 * 32 : 256;
             const dim3 block((unsigned)across, (unsigned)(256 / across)), grid((unsigned)((N + block.y - 1) / block.y), (unsigned)((pieces + 255) / 256));
             if (grid.y > 65535u) return fail(T81B200_ELIMIT, "gemm_trit: K too large");
-            T81_CUDA_TRY(launch_behind(stage_rows_kernel<T, PLANES, W>, grid, block, st, src, ldb, N, K, out, kpad, plane_elems, vec, release));
+            T81_CUDA_TRY(launch_behind(stage_rows_kernel<T, PLANES, W>, grid, block, 0, st, src, ldb, N, K, out, kpad, plane_elems, vec, release));
             return T81B200_OK;
         };
         // Eight k a thread are half the loads in flight and no shorter a chain, so up to 1.5 million elements four are faster, or up to a

@@ -11,9 +11,9 @@
 
 namespace t81b200 {
 
-// A kernel that starts while the one ahead ends (programmatic stream serialization), and whose first statement is
-// wait_for_kernel_ahead: it touches no global memory before all of that kernel's writes are visible, and lets its own successor
-// start (there, or with `release` false as its blocks end); so the order of memory is the stream's, and what overlaps is the launch
+// launch_behind: a kernel that starts while the one ahead ends (programmatic stream serialization).  It touches no global memory before
+// its griddepcontrol.wait, behind which all of that kernel's writes are visible.  wait_for_kernel_ahead is that wait as a first
+// statement, and lets the kernel's own successor start (there, or with `release` false as its blocks end).  So the order of memory is the stream's, and what overlaps is the launch
 // (1 to 2 us between two short kernels).  Not for kernels of many warps behind long ones, whose SMs they wait on: the absmax
 // reduction behind a weight gradient cost that 2 %.
 __device__ __forceinline__ void wait_for_kernel_ahead(bool release = true) {
@@ -21,10 +21,11 @@ __device__ __forceinline__ void wait_for_kernel_ahead(bool release = true) {
     if (release) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 template <typename... Params, typename... Args>
-cudaError_t launch_behind(void (*kernel)(Params...), dim3 grid, dim3 block, cudaStream_t st, Args &&...args) {
+cudaError_t launch_behind(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args &&...args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;

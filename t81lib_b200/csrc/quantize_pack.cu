@@ -232,7 +232,6 @@ quantize_pack_row_kernel(const T *__restrict__ w, int64_t rows, int cols, int64_
 // shared memory twice (sum, then pack) and handing the slot back after the second pass.
 // Rows may start and end anywhere: a copy brings the 16-byte pieces that hold the row, and groups are cut out of aligned pieces (two
 // loads instead of one, and a loop for each of the four shifts).  Needs TEAMS rows in 226 KB; the row kernel covers the rest.
-constexpr int kMaxTeams = 7;
 constexpr int kMaxSlots = 16;
 constexpr int kRingBytes = 226 * 1024;  // rows; barriers and team sums are static shared memory
 
@@ -578,17 +577,7 @@ int launch_staged(K kernel, std::atomic<bool> (&configured)[64], int ctas, int t
         T81_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRingBytes));
         if (dev >= 0 && dev < 64) configured[dev].store(true, std::memory_order_release);
     }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)ctas, 1, 1);
-    cfg.blockDim = dim3((unsigned)threads, 1, 1);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    T81_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, args...));
+    T81_CUDA_TRY(launch_behind(kernel, dim3((unsigned)ctas), dim3((unsigned)threads), smem, st, args...));
     return T81B200_OK;
 }
 
