@@ -273,7 +273,9 @@ T81B200_API int t81b200_exchange_signal(uint32_t *sync_local, uint32_t *const *s
  * the predecessor has, so later calls can rely on stream order as usual.  A hinted kernel
  * releases ITS successor at once, so in a run of consecutive hinted calls each one must be
  * independent of every kernel back to and including the last unhinted one (q, k*, v*: v may
- * run beside q, not only beside k).  The promise is the caller's; a false one is a data
+ * run beside q, not only beside k).  In a stream capture the library lets unhinted products
+ * of one input start early by itself; a hinted call behind such a one waits where it has to,
+ * so the promise stays the same.  The promise is the caller's; a false one is a data
  * race the library cannot detect.  Other kernels ignore the hint.  No counterpart in the
  * reference. */
 T81B200_API void t81b200_hint_independent(int on);
