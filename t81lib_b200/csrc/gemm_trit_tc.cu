@@ -96,7 +96,6 @@ struct TcParams {
                          // this many tensor maps (the local C first, then the peers'); 0: per-element stores
     int n_peers;         // other GPUs that receive a copy of every output element
     void *peer_C[T81B200_MAX_PEERS];  // their C, same strides as the local one
-    int c_rows;          // 1: a 16-bit token-major C that takes neither: blocks staged the same way, written by the epilogue warps
     int c_vec;           // 1: tokens are contiguous in C (the (M, N) argument order) and 16-byte aligned per 32-token block:
                          // a thread's 32 tokens of one feature are one run of memory, moved with 128-bit accesses
 };
@@ -131,8 +130,8 @@ struct OutStage {
 
 // A staged block to rows of C that TMA cannot write (off 16-byte boundaries): whole words, four warps take every fourth token.  Where a
 // row starts between two words its elements pair up the other way.  One element a lane, straight from the accumulators, is half the
-// bytes a store in twice the stores, and bounded short contractions: 13680 tokens of 834 x 834, bf16, 61 us, 40 this way
-// (8192 tokens of 2048 x 2047: 80 and 60; 51 where TMA writes, 2048 x 2048).
+// bytes a store in twice the stores, and bounded short contractions: 13680 tokens of 834 x 834, bf16, with their staging 70 us, 45
+// this way (8192 tokens of 2048 x 2047: 78 and 55; 47 where TMA writes, 2048 x 2048).
 template <typename CT>
 __device__ __forceinline__ void write_rows(const TcParams &p, const uint8_t *staged, int row0, int tok0, int quarter, int lane) {
     const int features = (int)(p.M - row0 < BM ? p.M - row0 : BM), tokens = (int)(p.N - tok0 < OUT_TOKENS ? p.N - tok0 : OUT_TOKENS);
@@ -164,9 +163,20 @@ __device__ __forceinline__ void write_rows(const TcParams &p, const uint8_t *sta
 }
 
 // One 32-token block of this thread's output feature: scale, bias, beta, store.
-template <typename CT>
+// ROWS: a 16-bit token-major C that TMA cannot write, without beta or peers, in blocks staged the same way.  A kernel of its own: as one
+// more branch it cost the others registers (spills in bf16) and 0.2 to 0.3 us (51 tokens of 624 by 2592, bf16: 8.26 -> 8.42 us).
+template <typename CT, bool ROWS>
 __device__ __forceinline__ void emit_block(const TcParams &p, const TcOutMaps &omaps, const uint32_t (&v)[32], int row0, int64_t row,
                                            float scale, float bias, int tok0, const OutStage &out) {
+    if constexpr (ROWS) {
+        CT *dst = reinterpret_cast<CT *>(out.gen) + (int)(row - row0);
+#pragma unroll
+        for (int i = 0; i < 32; ++i) dst[i * BM] = from_float<CT>(__uint_as_float(v[i]) * scale + bias);
+        // two buffers in turn: past this barrier every warp has read the other one
+        asm volatile("bar.sync %0, 128;" ::"r"(out.barrier) : "memory");
+        write_rows<CT>(p, out.gen, row0, tok0, (int)(row - row0) >> 5, threadIdx.x & 31);
+        return;
+    }
     const bool row_ok = row < p.M;
     CT *crow = static_cast<CT *>(p.C) + row * p.c_row_stride;
     if (p.n_out_maps > 0) {
@@ -187,13 +197,6 @@ __device__ __forceinline__ void emit_block(const TcParams &p, const TcOutMaps &o
                 for (int j = 0; j < p.n_out_maps; ++j) tma_store_2d(&omaps.m[j], out.smem, row0, tok0);
             asm volatile("cp.async.bulk.commit_group;" ::: "memory");
         }
-    } else if (sizeof(CT) == 2 && p.c_rows) {
-        CT *dst = reinterpret_cast<CT *>(out.gen) + (int)(row - row0);
-#pragma unroll
-        for (int i = 0; i < 32; ++i) dst[i * BM] = from_float<CT>(__uint_as_float(v[i]) * scale + bias);
-        // two buffers in turn: past this barrier every warp has read the other one
-        asm volatile("bar.sync %0, 128;" ::"r"(out.barrier) : "memory");
-        write_rows<CT>(p, out.gen, row0, tok0, (int)(row - row0) >> 5, threadIdx.x & 31);
     } else if (row_ok && p.c_vec && (int64_t)tok0 + 32 <= p.N) {
         // (M, N) argument order: the thread's 32 tokens are contiguous — whole 16-byte pieces, and with
         // beta the old values are all fetched before the first store
@@ -317,7 +320,8 @@ __device__ __forceinline__ void expand_chunk(const RawChunk<FMT> &raw, uint8_t *
 }
 
 // SMALL: 0, or with two or three activation planes the columns from a tile's accumulator to the one of all planes but the first.
-template <typename CT, int FMT, int SMALL>
+// ROWS: see emit_block.
+template <typename CT, int FMT, int SMALL, bool ROWS>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_trit_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ TcOutMaps omaps, const __grid_constant__ TcParams p) {
     extern __shared__ uint8_t smem_raw[];
@@ -511,7 +515,7 @@ gemm_trit_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                 uint32_t v[32];
                 load_sums<SMALL>(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * 256 + c * 32), v);
                 const uint32_t stage = out_off + (uint32_t)(out_count++ & 1) * OUT_STAGE_BYTES;
-                emit_block<CT>(p, omaps, v, row0, row, scale, bias, n0 + c * 32,
+                emit_block<CT, ROWS>(p, omaps, v, row0, row, scale, bias, n0 + c * 32,
                                OutStage{gen_base + stage, base + stage, 2, threadIdx.x == EPILOGUE_WARP0 * 32, true});
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -583,7 +587,7 @@ gemm_trit_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                 load_sums<SMALL>(t_lane + (uint32_t)(b * 32), v);
                 if (S > 1) fold_partials(v, gen_base, b, S, slice, lane_row);
                 const uint32_t stage = b_off + (uint32_t)b * OUT_STAGE_BYTES;
-                emit_block<CT>(p, omaps, v, row0, own_row, own_scale, own_bias, n0 + b * 32, OutStage{gen_base + stage, base + stage, (uint32_t)(2 + group), first, false});
+                emit_block<CT, ROWS>(p, omaps, v, row0, own_row, own_scale, own_bias, n0 + b * 32, OutStage{gen_base + stage, base + stage, (uint32_t)(2 + group), first, false});
             }
             if (first) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
         }
@@ -655,9 +659,9 @@ TcShape pick_shape(int64_t M, int64_t N, int64_t K, int planes) {
     return best;
 }
 
-template <typename CT, int FMT, int SMALL>
+template <typename CT, int FMT, int SMALL, bool ROWS>
 int launch_tc(const TcShape &shape, const CUtensorMap &mw, const CUtensorMap &mx, const TcOutMaps &om, const TcParams &p, cudaStream_t st) {
-    auto kern = gemm_trit_tc_kernel<CT, FMT, SMALL>;
+    auto kern = gemm_trit_tc_kernel<CT, FMT, SMALL, ROWS>;
     // the shared-memory limit is a per-device attribute of the function: set it once on every device
     static std::atomic<bool> configured[64];
     int dev = 0;
@@ -687,11 +691,11 @@ int launch_tc(const TcShape &shape, const CUtensorMap &mw, const CUtensorMap &mx
 }
 
 template <int FMT, int SMALL>
-int launch_tc_ct(int c_dtype, const TcShape &shape, const CUtensorMap &mw, const CUtensorMap &mx, const TcOutMaps &om, const TcParams &p, cudaStream_t st) {
+int launch_tc_ct(int c_dtype, bool rows, const TcShape &shape, const CUtensorMap &mw, const CUtensorMap &mx, const TcOutMaps &om, const TcParams &p, cudaStream_t st) {
     switch (c_dtype) {
-        case T81B200_F32: return launch_tc<float, FMT, SMALL>(shape, mw, mx, om, p, st);
-        case T81B200_BF16: return launch_tc<__nv_bfloat16, FMT, SMALL>(shape, mw, mx, om, p, st);
-        case T81B200_F16: return launch_tc<__half, FMT, SMALL>(shape, mw, mx, om, p, st);
+        case T81B200_F32: return launch_tc<float, FMT, SMALL, false>(shape, mw, mx, om, p, st);
+        case T81B200_BF16: return rows ? launch_tc<__nv_bfloat16, FMT, SMALL, true>(shape, mw, mx, om, p, st) : launch_tc<__nv_bfloat16, FMT, SMALL, false>(shape, mw, mx, om, p, st);
+        case T81B200_F16: return rows ? launch_tc<__half, FMT, SMALL, true>(shape, mw, mx, om, p, st) : launch_tc<__half, FMT, SMALL, false>(shape, mw, mx, om, p, st);
     }
     return fail(T81B200_EINVAL, "gemm_trit: unknown output dtype %d", c_dtype);
 }
@@ -852,7 +856,7 @@ int resident_pair_clusters(int splits) {
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return sm_count() / (2 * splits + 1);
     int n = known[dev][splits].load(std::memory_order_relaxed);
     if (n > 0) return n;
-    auto kern = gemm_trit_tc_kernel<__nv_bfloat16, 1, 0>;
+    auto kern = gemm_trit_tc_kernel<__nv_bfloat16, 1, 0, false>;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(2 * splits), 1, 1);
     cfg.blockDim = dim3(NUM_THREADS, 1, 1);
@@ -974,10 +978,11 @@ int gemm_trit_tc_launch(int fmt, int fp32_planes, const uint8_t *A, const float 
                 return rc;
         }
         p.n_out_maps = 1 + n_peers;
-    } else p.c_rows = dtype_size(c_dtype) == 2 && layout == T81B200_LAYOUT_NK && beta == 0.0f && n_peers == 0 && reinterpret_cast<uintptr_t>(C) % 2 == 0 ? 1 : 0;
+    }
+    const bool rows = !tma_out && dtype_size(c_dtype) == 2 && layout == T81B200_LAYOUT_NK && beta == 0.0f && n_peers == 0 && reinterpret_cast<uintptr_t>(C) % 2 == 0;
     auto launch = [&](auto small) {
         constexpr int S = decltype(small)::value;
-        return fmt == 1 ? launch_tc_ct<1, S>(c_dtype, shape, mw, mx, om, p, st) : launch_tc_ct<0, S>(c_dtype, shape, mw, mx, om, p, st);
+        return fmt == 1 ? launch_tc_ct<1, S>(c_dtype, rows, shape, mw, mx, om, p, st) : launch_tc_ct<0, S>(c_dtype, rows, shape, mw, mx, om, p, st);
     };
     if (planes == 1) return launch(std::integral_constant<int, 0>{});
     return shape.bn <= 128 ? launch(std::integral_constant<int, 128>{}) : launch(std::integral_constant<int, 256>{});

@@ -206,3 +206,17 @@ def test_staged_rows_by_size(dev, in_f, tokens, width, dtype):
     staging = [name for name, _ in kernels(capture(lambda: got.append(ops.linear_t2(t2, 130, x, in_f, None, None)))) if "stage_rows_kernel" in name]
     assert len(staging) == 1 and f"Li0ELi{width}E" in staging[0]
     assert torch.equal(got[0], (x.double() @ trits.double().t()).to(dtype))
+
+
+# 16-bit results that TMA cannot write have a kernel of their own; everything else stays out of it.
+@pytest.mark.parametrize("out_f,dtype,out_dtype,own", [(256, torch.bfloat16, None, 0), (255, torch.bfloat16, None, 1), (260, torch.float16, None, 1),
+                                                       (255, torch.bfloat16, torch.float32, 0), (255, torch.float32, torch.bfloat16, 1), (264, torch.float32, torch.float16, 0)])
+def test_rows_off_boundaries_have_their_own_kernel(dev, out_f, dtype, out_dtype, own):
+    from t81lib_b200 import ops
+    gen = torch.Generator(device="cuda").manual_seed(out_f)
+    trits = torch.randint(-1, 2, (out_f, 192), generator=gen, device="cuda").float()
+    t2 = ops.pack_t2(ops.quantize_pack(trits, 0.5, "fixed")[0], out_f, 192)
+    x, got = torch.randint(-1, 2, (70, 192), generator=gen, device="cuda").to(dtype), []
+    names = [name for name, _ in kernels(capture(lambda: got.append(ops.linear_t2(t2, out_f, x, 192, None, None, out_dtype)))) if "gemm_trit_tc_kernel" in name]
+    assert len(names) == 1 and f"ELb{own}EEE" in names[0], names
+    assert torch.equal(got[0], (x.double() @ trits.double().t()).to(out_dtype or dtype))
