@@ -604,7 +604,8 @@ int launch_warps(const T *w, int64_t rows, int64_t cols, int64_t ld, float thr, 
 // the 24 have none, and a long row takes long.  So the shorter the rows (in chunks of 384 columns), the fewer of them it needs.
 // Under the absmean rule, which goes through a row twice, rows of which one warp has no second slot need whole waves of 24 an SM,
 // the last at least two thirds full over all.  Off 16-byte boundaries groups are cut out of aligned pieces, which short rows of
-// few-row matrices do not win back; the row kernel, six CTAs an SM, steps up behind six rows an SM.  us a call, absmean, row kernel / teams / warps, at 297, 800, 1184, 3552, 4096, 10000 rows:
+// few-row matrices do not win back; the row kernel, six CTAs an SM, steps up behind six rows an SM.  us a call, absmean, row kernel /
+// teams / warps, at 297, 800, 1184, 3552, 4096 and 10000 rows:
 //   1024 fp32                    2.5 2.9 2.8   3.8 3.9 3.2   5.5 4.7 3.9   9.7 9.1 5.8    10.8 10.3 7.2   21.5 22.2 12.6
 //   4096 bf16                    4.6 3.5 5.1   8.7 5.1 6.4   14.5 6.0 6.8  28.8 12.6 12.5 33.5 14.6 15.9  78.8 31.9 28.7
 //   2049 fp32, off boundaries    3.1 4.0 5.0   5.4 5.7 6.3   7.6 6.5 6.7   14.7 12.7 11.2 16.4 14.3 14.9  35.1 31.7 25.4
