@@ -16,14 +16,14 @@
 // 1.1e-6 for fp32 ones.  So an accumulator takes a segment of the tokens only, and the epilogue warps add the segments up in
 // registers, while the MMAs fill the other accumulator: 16-bit operands 64 tokens below 512 of them, 128 below 1024 and 192 from
 // there on, fp32 ones 256; each the longest that is no further off than those sums were.  The results are 1.9e-7 to 2.9e-7 off at
-// 4096 tokens.  14336 x 4096 x 4096 tokens, bf16: 339 us in one piece, 405 in segments of 192, 375 with the weights brought to L2
-// ahead and long first segments (below); fp32 2048 x 2048 x 8192: 430 us in segments that met in memory, 329.
+// 4096 tokens.  A segment of 64 tokens costs 960 clocks, 500 of MMA: from an accumulator handed back to the next one full are 1300, and
+// there are two.
 //
-// 14336 x 4096 x 4096 tokens in bf16: the tensor pipe is busy 76 % of the active cycles, L2 43 %, nothing is saturated; the rest are the
-// ends of tiles and 13 waves of them for 12.1.  A pair tile takes 32 KB per CTA and 64 tokens of 16-bit operands.  The planes of
+// 14336 x 4096 x 4096 tokens in bf16, back to back: 365 us (390 to 400 with the weights in registers at the end of a tile); nothing is
+// saturated: the rest are the ends of tiles and 13 waves of them for 12.1.  A pair tile takes 32 KB per CTA and 64 tokens of 16-bit operands.  The planes of
 // fp32 operands are loaded together, once for all six products (2050 x 1537 x 1000 tokens: 64 us with a load per product,
 // 56 us this way).  Tiles are walked in groups of eight row tiles so that what runs at a time shares its operands in L2.  The slope
-// is applied in the epilogue, on values that a trip through shared memory has turned into whole 128-byte rows, beside the weights.
+// is applied in the epilogue, in the shared memory that the weights have come to (below).
 #include "common.cuh"
 #include "tma.cuh"
 #include "umma.cuh"
@@ -43,9 +43,10 @@ constexpr int EPILOGUE_WARPS = 8;             // two per quarter of the rows: ea
 constexpr int NUM_THREADS = (2 + EPILOGUE_WARPS) * 32;
 constexpr int EPILOGUE_WARP0 = 2;
 constexpr int MAX_SPLITS = 4;
-constexpr int TURN_PITCH = 36;                // floats per row of the turning buffer: 16-byte aligned, conflict-free
-constexpr int TURN_BYTES = EPILOGUE_WARPS * 32 * TURN_PITCH * 4;
-constexpr int BARRIER_BYTES = 256;
+constexpr int BLOCK_BYTES = 32 * 128;         // a block of the epilogue: 32 columns of a warp's 32 rows, fp32
+constexpr int MOST_BLOCKS = 4;                // of a warp: 256 columns / 64
+constexpr int MAX_SLOTS = 3;                  // blocks whose weights a warp has in shared memory or on their way there
+constexpr int BARRIER_BYTES = 512;
 constexpr int SMEM_LIMIT = 227 * 1024;
 
 enum { WGRAD_STATUS_PRODUCER = 11, WGRAD_STATUS_MMA = 12, WGRAD_STATUS_EPILOGUE = 13 };
@@ -60,7 +61,8 @@ struct WgradParams {
     int segment, lead;                // token stages an accumulator takes before the epilogue adds it up; those of a tile's first two
     int splits, stages;
     uint32_t idesc;
-    int vec;                          // 128-bit accesses to w and out
+    int slots;                        // blocks of weights a warp of the epilogue holds
+    int vec;                          // TMA reads w and writes out
 };
 
 // Plane pair i of an fp32 product: planes of g and of x.
@@ -91,103 +93,125 @@ __device__ __forceinline__ void tile_at(const WgradParams &p, int tile, int &m, 
     n = r / height;
 }
 
-// A block is 32 columns of this warp's 32 rows, half a block 16 of the rows.  VEC: a lane moves four columns of rows 4 i + lane / 8
-// (whole 128-byte row pieces, 16 bytes a lane); otherwise one column of all rows.
+// A block is 32 columns of a warp's 32 rows.  Its weights come into a slot of shared memory (rows of 128 bytes, 16-byte piece j of row
+// r at (j ^ (r & 7)) * 16) long before the block's sums are there, the thread that has a row's sums turns them into the gradient in
+// place, and the slot leaves as it came.  VEC: both ways one TMA box; otherwise, rows off 16-byte boundaries, a word a lane and row.
+// Few tokens leave little beside this: with the weights in registers, half a block ahead, a tile took 7000 clocks to put out, 3800 this
+// way (9472 x 4096, 64 to 511 tokens: 67 to 99 us, 60 to 78; 310 MB cross memory in 47).  Copies of the 16-byte pieces that hold an
+// unaligned row, and stores of them, took longer than words do (512 tokens of 12402 by 2988: 151 us before, 124 in words, 160).
 template <bool VEC>
-__device__ __forceinline__ void load_weights(const WgradParams &p, int64_t row0, int64_t col0, int lane, int half, float (&w)[16]) {
+__device__ __forceinline__ void load_block(const WgradParams &p, const CUtensorMap *map_w, uint32_t slot, uint32_t bar, int row0, int col0, int lane) {
     if constexpr (VEC) {
-        const int64_t col = col0 + (lane & 7) * 4;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int64_t row = row0 + 16 * half + 4 * i + (lane >> 3);
-            const float4 q = row < p.rows && col < p.cols ? __ldg(reinterpret_cast<const float4 *>(p.w + row * p.ldw + col)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            w[4 * i] = q.x; w[4 * i + 1] = q.y; w[4 * i + 2] = q.z; w[4 * i + 3] = q.w;
+        if (lane == 0) {
+            mbar_arrive_expect_tx(bar, BLOCK_BYTES);
+            tma_load_2d(slot, map_w, col0, row0, bar);
         }
     } else {
-        const int64_t row = row0 + 16 * half;
-        const int n = col0 + lane < p.cols ? (int)(p.rows - row < 16 ? p.rows - row : 16) : 0;
-        const float *src = p.w + row * p.ldw + col0 + lane;
+        const int n = col0 + lane < p.cols ? (int)(p.rows - row0 < 32 ? p.rows - row0 : 32) : 0;
+        const float *src = p.w + (int64_t)row0 * p.ldw + col0 + lane;
+        const uint32_t dst = slot + (uint32_t)(lane & 3) * 4u;
 #pragma unroll
-        for (int i = 0; i < 16; ++i, src += p.ldw) w[i] = i < n ? __ldg(src) : 0.0f;
+        for (int r = 0; r < 32; ++r, src += p.ldw)
+            if (r < n)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + (uint32_t)r * 128u + (uint32_t)(((lane >> 2) ^ (r & 7)) << 4)), "l"(src) : "memory");
+        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
     }
 }
 
-// The block's sums into the turning buffer.
-__device__ __forceinline__ void turn_block(const float (&sum)[32], float *turn, int lane) {
-    __syncwarp();
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-        *reinterpret_cast<float4 *>(turn + lane * TURN_PITCH + 4 * i) = make_float4(sum[4 * i], sum[4 * i + 1], sum[4 * i + 2], sum[4 * i + 3]);
-    __syncwarp();
-}
-
-// Half of the block in the turning buffer, multiplied with the slope and stored.
-template <bool VEC>
-__device__ __forceinline__ void emit_half(const WgradParams &p, const float (&w)[16], const float *turn, int64_t row0, int64_t col0, int lane, int half,
-                                          float half_scale) {
+// The weights in the slot have arrived: they become the gradient, which leaves for memory.  `refill` runs between the two, when the
+// stores of the block before have had the most time to read their slot.
+template <bool VEC, typename F>
+__device__ __forceinline__ void emit_block(const WgradParams &p, const CUtensorMap *map_out, const float2 (&sum)[16], uint8_t *slot, int row0, int col0,
+                                           int lane, float half_scale, F &&refill) {
     // |w / scale| < 0.5 exactly where |w| < scale / 2: two floats that differ do so by 2^-24 of their size or more,
     // and a quotient 2^-24 below one half does not round up to it
-    auto sloped = [&](float sum, float weight) { return sum * (fabsf(weight) < half_scale ? 2.0f : 0.0f); };
-    if constexpr (VEC) {
-        const int64_t col = col0 + (lane & 7) * 4;
-        if (col >= p.cols) return;
+    auto sloped = [&](float v, float weight) { return v * (fabsf(weight) < half_scale ? 2.0f : 0.0f); };
+    uint8_t *row = slot + lane * 128;
+    const int turn = (lane & 7) << 4;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int r = 16 * half + 4 * i + (lane >> 3);
-            if (row0 + r >= p.rows) continue;
-            const float4 s = *reinterpret_cast<const float4 *>(turn + r * TURN_PITCH + (lane & 7) * 4);
-            *reinterpret_cast<float4 *>(p.out + (row0 + r) * p.cols + col) =
-                make_float4(sloped(s.x, w[4 * i]), sloped(s.y, w[4 * i + 1]), sloped(s.z, w[4 * i + 2]), sloped(s.w, w[4 * i + 3]));
+    for (int h = 0; h < 8; h += 4) {
+        float4 w[4];  // all of them before the first store: the compiler cannot know the stores to miss them
+#pragma unroll
+        for (int j = 0; j < 4; ++j) w[j] = *reinterpret_cast<const float4 *>(row + (((h + j) << 4) ^ turn));
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float2 a = sum[2 * (h + j)], b = sum[2 * (h + j) + 1];
+            *reinterpret_cast<float4 *>(row + (((h + j) << 4) ^ turn)) = make_float4(sloped(a.x, w[j].x), sloped(a.y, w[j].y), sloped(b.x, w[j].z), sloped(b.y, w[j].w));
+        }
+    }
+    if constexpr (VEC) {
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+        refill();
+        __syncwarp();
+        if (lane == 0) {
+            if (row0 < p.rows && col0 < p.cols) tma_store_2d(map_out, smem_u32(slot), col0, row0);
+            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
         }
     } else {
-        const int64_t row = row0 + 16 * half;
-        const int n = col0 + lane < p.cols ? (int)(p.rows - row < 16 ? p.rows - row : 16) : 0;
-        float *out = p.out + row * p.cols + col0 + lane;
+        refill();
+        __syncwarp();
+        const int n = col0 + lane < p.cols ? (int)(p.rows - row0 < 32 ? p.rows - row0 : 32) : 0;
+        float *out = p.out + (int64_t)row0 * p.cols + col0 + lane;
+        const uint8_t *src = slot + (lane & 3) * 4;
 #pragma unroll
-        for (int i = 0; i < 16; ++i, out += p.cols)
-            if (i < n) *out = sloped(turn[(16 * half + i) * TURN_PITCH + lane], w[i]);
+        for (int r = 0; r < 32; ++r, out += p.cols)
+            if (r < n) *out = *reinterpret_cast<const float *>(src + r * 128 + (((lane >> 2) ^ (r & 7)) << 4));
+        __syncwarp();
     }
 }
 
-// sum += 32 columns of an accumulator, 16 at a time (the sums of a whole tile take most of a thread's registers).  SMALL: the products
-// beside the large one, which say nothing where an operand is infinite (its other planes are zero).
+// sum += 32 columns of each of the warp's blocks, which lie 64 columns apart; eight columns are on their way while the eight before are
+// added (the sums of a whole tile take most of a thread's registers).  SMALL: the products beside the large one, which say nothing where
+// an operand is infinite (its other planes are zero).
 template <bool SMALL>
-__device__ __forceinline__ void add_columns(uint32_t taddr, float (&sum)[32]) {
+__device__ __forceinline__ void add_blocks(uint32_t taddr, int blocks, float2 (&sum)[MOST_BLOCKS][16]) {
+    uint32_t v[2][8];
+    tmem_ld8_start(taddr, v[0]);
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        uint32_t v[16];
-        tmem_ld16(taddr + 16u * h, v);
+    for (int q = 0; q < 4 * MOST_BLOCKS; ++q) {
+        if (q / 4 >= blocks) break;
+        tmem_ld8_wait(v[q & 1]);
+        if (q + 1 < 4 * MOST_BLOCKS && (q + 1) / 4 < blocks) tmem_ld8_start(taddr + (uint32_t)((q + 1) / 4 * 64 + (q + 1) % 4 * 8), v[(q + 1) & 1]);
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            const float x = __uint_as_float(v[i]);
-            sum[16 * h + i] += SMALL && !isfinite(x) ? 0.0f : x;
+        for (int i = 0; i < 4; ++i) {
+            float2 x = make_float2(__uint_as_float(v[q & 1][2 * i]), __uint_as_float(v[q & 1][2 * i + 1]));
+            if (SMALL && !isfinite(x.x)) x.x = 0.0f;
+            if (SMALL && !isfinite(x.y)) x.y = 0.0f;
+            float2 &to = sum[q / 4][4 * (q % 4) + i];
+            to = __fadd2_rn(to, x);
         }
     }
 }
 
-__device__ __forceinline__ void store_columns(uint32_t taddr, const float (&sum)[32]) {
+__device__ __forceinline__ void store_columns(uint32_t taddr, const float2 (&sum)[16]) {
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         uint32_t v[16];
 #pragma unroll
-        for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(sum[16 * h + i]);
+        for (int i = 0; i < 8; ++i) {
+            v[2 * i] = __float_as_uint(sum[8 * h + i].x);
+            v[2 * i + 1] = __float_as_uint(sum[8 * h + i].y);
+        }
         tmem_st16(taddr + 16u * h, v);
     }
 }
 
 template <bool VEC>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
-gemm_wgrad_tc_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ WgradParams p) {
+gemm_wgrad_tc_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
+                     const __grid_constant__ CUtensorMap map_out, const __grid_constant__ WgradParams p) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t *gen_base = smem_raw + (base - smem_u32(smem_raw));
     const uint32_t group = (uint32_t)group_bytes(p.planes), stage_bytes = (2u + (uint32_t)p.bn / 128u) * group;
-    const uint32_t turn_off = (uint32_t)p.stages * stage_bytes, bars = base + turn_off + TURN_BYTES;
+    const uint32_t slot_off = (uint32_t)p.stages * stage_bytes, bars = base + slot_off + (uint32_t)(EPILOGUE_WARPS * p.slots * BLOCK_BYTES);
     auto full = [&](int s) { return bars + 8u * s; };
     auto empty = [&](int s) { return bars + 8u * (MAX_STAGES + s); };
     auto acc_full = [&](int s) { return bars + 8u * (2 * MAX_STAGES + s); };
     auto acc_empty = [&](int s) { return bars + 8u * (2 * MAX_STAGES + 2 + s); };
-    const uint32_t tmem_slot = bars + 8u * (2 * MAX_STAGES + 4);
+    auto slot_full = [&](int warp, int s) { return bars + 8u * (2 * MAX_STAGES + 4 + warp * MAX_SLOTS + s); };
+    const uint32_t tmem_slot = bars + 8u * (2 * MAX_STAGES + 4 + EPILOGUE_WARPS * MAX_SLOTS);
 
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const uint32_t rank = cluster_rank();
@@ -196,6 +220,7 @@ gemm_wgrad_tc_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_con
     if (threadIdx.x == 0) {
         for (int s = 0; s < MAX_STAGES; ++s) { mbar_init(full(s), 1); mbar_init(empty(s), 1); }
         for (int s = 0; s < 2; ++s) { mbar_init(acc_full(s), 1); mbar_init(acc_empty(s), 2 * EPILOGUE_WARPS); }
+        for (int s = 0; s < EPILOGUE_WARPS * MAX_SLOTS; ++s) mbar_init(slot_full(0, s), VEC ? 1 : 32);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncwarp();
@@ -298,66 +323,90 @@ gemm_wgrad_tc_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_con
         }
     }
 
-    // ---- epilogue: two warps per quarter of the rows, each with every other 32-column block of the tile ----
+    // ---- epilogue: two warps per quarter of the rows, each with every other 32-column block of the tile, or of its slice of it ----
     const bool epilogue = warp >= EPILOGUE_WARP0;
-    const int quarter = warp & 3, first = (warp - EPILOGUE_WARP0) >> 2;
-    float *turn = reinterpret_cast<float *>(gen_base + turn_off) + (warp - EPILOGUE_WARP0) * 32 * TURN_PITCH;
+    const int ew = warp - EPILOGUE_WARP0, quarter = warp & 3, first = ew >> 2;
     const uint32_t t_lane = tmem_base + ((uint32_t)(quarter * 32) << 16);
+    const int block0 = p.splits == 1 ? first : slice + p.splits * first, block_step = 2 * p.splits;
+    // the warp's blocks in order, one slot after the other
+    const uint32_t slot0 = slot_off + (uint32_t)(ew * p.slots * BLOCK_BYTES);
+    struct Place { int row, col; };  // first row, and column of block 0
+    auto place_of = [&](int tile) {
+        int m, n;
+        tile_at(p, tile, m, n);
+        return Place{(2 * m + half) * 128 + quarter * 32, n * p.bn};
+    };
+    int ahead = p.slots, fetch_block = block0;  // blocks that may still be fetched
+    Place place = place_of(cluster_id), next = place;
+    bool in_next = false;  // where the fetches are; the last one of the next tile does not come before this tile's last block has left
+    Ring fill, use;
+    auto fetch = [&](bool has_next) {
+        for (; ahead > 0; --ahead) {
+            if (fetch_block >= p.bn / 32) {
+                if (in_next || !has_next) return;
+                in_next = true;
+                fetch_block = block0;
+            }
+            load_block<VEC>(p, &map_w, base + slot0 + (uint32_t)(fill.stage * BLOCK_BYTES), slot_full(ew, fill.stage), in_next ? next.row : place.row,
+                            (in_next ? next.col : place.col) + fetch_block * 32, lane);
+            fill.advance(p.slots);
+            fetch_block += block_step;
+        }
+    };
+    // `freed`: the slot of the block before may be filled again once that block has been read
+    auto put_out = [&](const float2 (&sum)[16], int block, bool freed, bool has_next) {
+        const bool ok = __all_sync(0xffffffffu, mbar_wait(slot_full(ew, use.stage), use.phase));
+        if (!ok) return false;
+        emit_block<VEC>(p, &map_out, sum, gen_base + slot0 + use.stage * BLOCK_BYTES, place.row, place.col + block * 32, lane, half_scale, [&] {
+            ahead += freed ? 1 : 0;
+            fetch(has_next);
+        });
+        use.advance(p.slots);
+        return true;
+    };
     if (epilogue) {
-        constexpr int MOST = 4;  // blocks of a warp: 256 columns / 64
         const int blocks = p.bn / 64;
         bool ok = true;
         int it = 0;
+        bool freed = false;
+        fetch(false);
         for (int tile = cluster_id; tile < total_tiles && ok; tile += n_clusters) {
-            int m, n;
-            tile_at(p, tile, m, n);
-            const int64_t row0 = (int64_t)(2 * m + half) * 128 + quarter * 32, col0 = (int64_t)n * p.bn + first * 32;
-            // the tile's weights on their way to L2 while its products are summed: what follows the last segment keeps the MMAs waiting
-            if (p.splits == 1 && row0 + lane < p.rows)
-                for (int c = 0; c < blocks && col0 + 64 * c < p.cols; ++c)
-                    asm volatile("prefetch.global.L2 [%0];" ::"l"(p.w + (row0 + lane) * p.ldw + col0 + 64 * c));
-            float sum[MOST][32];
+            const bool has_next = tile + n_clusters < total_tiles;
+            float2 sum[MOST_BLOCKS][16];
 #pragma unroll
-            for (int c = 0; c < MOST; ++c)
+            for (int c = 0; c < MOST_BLOCKS; ++c)
 #pragma unroll
-                for (int i = 0; i < 32; ++i) sum[c][i] = 0.0f;
+                for (int i = 0; i < 16; ++i) sum[c][i] = make_float2(0.0f, 0.0f);
             for (int s = s0; s < s1; s = segment_end(s), ++it) {
                 const int buf = it % n_bufs;
                 ok = __all_sync(0xffffffffu, mbar_wait(acc_full(buf), (uint32_t)(it / n_bufs) & 1u));
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t acc = t_lane + (uint32_t)(buf * 256 + first * 32);
-#pragma unroll
-                for (int c = 0; c < MOST; ++c)
-                    if (c < blocks) {
-                        add_columns<false>(acc + 64u * c, sum[c]);
-                        if (p.planes > 1) add_columns<true>(acc + 64u * c + 256u, sum[c]);
-                    }
+                add_blocks<false>(acc, blocks, sum);
+                if (p.planes > 1) add_blocks<true>(acc + 256u, blocks, sum);
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
                 if (lane == 0) mbar_arrive_leader(acc_empty(buf));
+                if (s == s0 && has_next) next = place_of(tile + n_clusters);
             }
             if (!ok) break;
             if (p.splits > 1) {  // back to where the pairs of the cluster take them from
 #pragma unroll
-                for (int c = 0; c < MOST; ++c)
+                for (int c = 0; c < MOST_BLOCKS; ++c)
                     if (c < blocks) store_columns(t_lane + (uint32_t)(first * 32 + 64 * c), sum[c]);
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 break;
             }
-            float w[2][16];  // the weights of half a block are fetched while the half before it is put out: their latency bounded this loop
-            turn_block(sum[0], turn, lane);
-            load_weights<VEC>(p, row0, col0, lane, 0, w[0]);
 #pragma unroll
-            for (int c = 0; c < MOST; ++c)
-                if (c < blocks) {
-                    if (c > 0) turn_block(sum[c], turn, lane);
-                    load_weights<VEC>(p, row0, col0 + 64 * c, lane, 1, w[1]);
-                    emit_half<VEC>(p, w[0], turn, row0, col0 + 64 * c, lane, 0, half_scale);
-                    if (c + 1 < blocks) load_weights<VEC>(p, row0, col0 + 64 * (c + 1), lane, 0, w[0]);
-                    emit_half<VEC>(p, w[1], turn, row0, col0 + 64 * c, lane, 1, half_scale);
+            for (int c = 0; c < MOST_BLOCKS; ++c)
+                if (c < blocks && ok) {
+                    ok = put_out(sum[c], first + 2 * c, freed, has_next);
+                    freed = true;
                 }
+            place = next;
+            in_next = false;
         }
         if (!ok) give_up(&g_wgrad_status, WGRAD_STATUS_EPILOGUE);
     }
@@ -381,25 +430,20 @@ gemm_wgrad_tc_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_con
         __syncthreads();
         cluster_barrier();
         if (epilogue) {
-            int m, n;
-            tile_at(p, cluster_id, m, n);
-            const int64_t row0 = (int64_t)(2 * m + half) * 128 + quarter * 32;
-            for (int b = slice + S * first; b < blocks; b += 2 * S) {
-                const int64_t col = (int64_t)n * p.bn + b * 32;
-                float w[2][16], sums[32];
-                load_weights<VEC>(p, row0, col, lane, 0, w[0]);
-                load_weights<VEC>(p, row0, col, lane, 1, w[1]);
+            bool ok = true;
+            for (int b = block0; b < blocks && ok; b += block_step) {
                 uint32_t v[32];
                 tmem_ld32(t_lane + (uint32_t)(b * 32), v);
                 fold_partials(v, gen_base, b, S, slice, lane_row);
+                float2 sums[16];
 #pragma unroll
-                for (int i = 0; i < 32; ++i) sums[i] = __uint_as_float(v[i]);
-                turn_block(sums, turn, lane);
-                emit_half<VEC>(p, w[0], turn, row0, col, lane, 0, half_scale);
-                emit_half<VEC>(p, w[1], turn, row0, col, lane, 1, half_scale);
+                for (int i = 0; i < 16; ++i) sums[i] = make_float2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]));
+                ok = put_out(sums, b, b != block0, false);
             }
+            if (!ok) give_up(&g_wgrad_status, WGRAD_STATUS_EPILOGUE);
         }
     }
+    if (VEC && epilogue && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");  // every store has completed
 
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -417,7 +461,7 @@ int make_map_3d(CUtensorMap *map, CUtensorMapDataType dt, const void *ptr, uint6
 }
 
 template <bool VEC>
-int launch_wgrad(const cudaLaunchConfig_t &cfg, const CUtensorMap &mg, const CUtensorMap &mx, const WgradParams &p) {
+int launch_wgrad(const cudaLaunchConfig_t &cfg, const CUtensorMap &mg, const CUtensorMap &mx, const CUtensorMap &mw, const CUtensorMap &mo, const WgradParams &p) {
     // the shared-memory limit is a per-device attribute of the function: set it once on every device
     static std::atomic<bool> configured[64];
     int dev = 0;
@@ -426,7 +470,7 @@ int launch_wgrad(const cudaLaunchConfig_t &cfg, const CUtensorMap &mg, const CUt
         T81_CUDA_TRY(cudaFuncSetAttribute(gemm_wgrad_tc_kernel<VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT));
         if (dev >= 0 && dev < 64) configured[dev].store(true, std::memory_order_release);
     }
-    T81_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_wgrad_tc_kernel<VEC>, mg, mx, p));
+    T81_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_wgrad_tc_kernel<VEC>, mg, mx, mw, mo, p));
     return T81B200_OK;
 }
 
@@ -511,10 +555,21 @@ extern "C" int t81b200_qat_weight_grad(const void *g, int g_dtype, int64_t ldg, 
     p.segment = p.planes > 1 ? 256 / token_step(3) : (tokens < 512 ? 1 : (tokens < 1024 ? 2 : 3));  // how long: see the top
     p.n_tiles = (int)((cols + p.bn - 1) / p.bn);
     const int stage = (2 + p.bn / 128) * group_bytes(p.planes);
-    const int fit = (SMEM_LIMIT - 1024 - TURN_BYTES - BARRIER_BYTES) / stage;
+    p.vec = cols % 4 == 0 && ldw % 4 == 0 && ldw < (1ll << 37) && reinterpret_cast<uintptr_t>(w) % 16 == 0 && reinterpret_cast<uintptr_t>(out) % 16 == 0 ? 1 : 0;
+    // Three slots a warp leave four stages of 16-bit operands, two leave five.  Few tokens are over before two have been read and filled
+    // again, many want the stages (16-bit, us, two and three: 304 tokens of 2416 by 4965 35.2 and 30.9, 1104 of 12192 by 12476 405 and
+    // 380, 4096 of 4096 by 14336 365 and 371); fp32 stages and rows that lanes copy word by word gain nothing from a third.
+    p.slots = p.planes == 1 && p.vec && p.bn == 256 && tokens <= 2048 ? 3 : 2;
+    const int fit = (SMEM_LIMIT - 1024 - EPILOGUE_WARPS * p.slots * BLOCK_BYTES - BARRIER_BYTES) / stage;
     p.stages = fit < MAX_STAGES ? fit : MAX_STAGES;
     p.idesc = umma_instr_desc(p.bn, g_dtype == T81B200_F16, true, true);
-    p.vec = cols % 4 == 0 && ldw % 4 == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0 && reinterpret_cast<uintptr_t>(out) % 16 == 0 ? 1 : 0;
+    CUtensorMap mw, mo;
+    memset(&mw, 0, sizeof mw);
+    memset(&mo, 0, sizeof mo);
+    if (p.vec) {
+        if (int rc = make_map_2d(&mw, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, w, (uint64_t)cols, (uint64_t)rows, (uint64_t)ldw * 4, 32, 32, CU_TENSOR_MAP_SWIZZLE_128B)) return rc;
+        if (int rc = make_map_2d(&mo, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, out, (uint64_t)cols, (uint64_t)rows, (uint64_t)cols * 4, 32, 32, CU_TENSOR_MAP_SWIZZLE_128B)) return rc;
+    }
     const int64_t tiles = (int64_t)p.m_tiles * p.n_tiles;
     const int64_t clusters = p.splits > 1 || tiles < resident_pair_clusters(1) ? tiles : resident_pair_clusters(1);
     // While the epilogue puts a tile out, the MMAs of the next one have two accumulators to go on with: an eighth of the tokens each
@@ -524,7 +579,7 @@ extern "C" int t81b200_qat_weight_grad(const void *g, int g_dtype, int64_t ldg, 
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(clusters * 2 * p.splits), 1, 1);
     cfg.blockDim = dim3(NUM_THREADS, 1, 1);
-    cfg.dynamicSmemBytes = (size_t)p.stages * stage + TURN_BYTES + BARRIER_BYTES + 1024;
+    cfg.dynamicSmemBytes = (size_t)p.stages * stage + EPILOGUE_WARPS * p.slots * BLOCK_BYTES + BARRIER_BYTES + 1024;
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -534,5 +589,5 @@ extern "C" int t81b200_qat_weight_grad(const void *g, int g_dtype, int64_t ldg, 
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    return p.vec ? launch_wgrad<true>(cfg, mg, mx, p) : launch_wgrad<false>(cfg, mg, mx, p);
+    return p.vec ? launch_wgrad<true>(cfg, mg, mx, mw, mo, p) : launch_wgrad<false>(cfg, mg, mx, mw, mo, p);
 }

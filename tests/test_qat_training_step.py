@@ -90,6 +90,24 @@ def test_quantiser_bytes_beyond_finite_values(lib_built, scale, threshold):
     assert np.array_equal(t2_t.cpu().numpy(), oracle.pack_t2(np.ascontiguousarray(want.T)))
 
 
+# weights whose rows TMA reads, with and without gaps, and rows that go word by word: blocks at the edges of the matrix, slots that are
+# filled again inside a tile and for the tile that follows, three and two of them, tokens split over a cluster
+@pytest.mark.parametrize("gap,skip", [(0, 0), (4, 0), (4, 1), (3, 0)])
+@pytest.mark.parametrize("tokens,rows,cols", [(64, 33, 36), (130, 300, 1540), (70, 4000, 4340), (300, 4000, 4340), (2100, 4000, 4341), (20, 4100, 700)])
+def test_weight_gradient_of_strided_weights(lib_built, tokens, rows, cols, gap, skip):
+    from t81lib_b200 import _capi, ops
+    gen = torch.Generator(device="cuda").manual_seed(tokens + rows + cols + gap)
+    w = (torch.randn(rows, cols + gap, device="cuda", generator=gen) * 0.03)[:, skip:skip + cols]
+    scale = w.abs().amax().reshape(1)
+    g, x = (torch.randn(tokens, n, device="cuda", generator=gen).bfloat16() for n in (rows, cols))
+    slope = ((w / scale).abs() < 0.5).double() * 2.0
+    sums = g.double().t() @ x.double()
+    got = ops.qat_weight_grad(g, x, w, scale)
+    bound = 2 * 5 * (tokens / 16 + 3) * 2.0 ** -23  # as above
+    assert float((got.double() - sums * slope).abs().max() / sums.pow(2).mean().sqrt()) < bound
+    assert _capi.kernel_status(reset=True) == 0
+
+
 # an infinity in either fp32 operand comes out where and as it does in fp32 arithmetic
 @pytest.mark.parametrize("tokens", [20, 600])
 def test_weight_gradient_of_infinities(lib_built, tokens):
