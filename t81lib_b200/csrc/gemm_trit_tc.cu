@@ -128,69 +128,57 @@ struct OutStage {
     bool reused;       // an earlier store may still be reading the buffer
 };
 
-// A staged block to rows of C that TMA cannot write (off 16-byte boundaries): whole words, four warps take every fourth token.  Where a
-// row starts between two words its elements pair up the other way.  One element a lane, straight from the accumulators, is half the
-// bytes a store in twice the stores, and bounded short contractions: 13680 tokens of 834 x 834, bf16, with their staging 70 us, 45
-// this way (8192 tokens of 2048 x 2047: 78 and 55; 47 where TMA writes, 2048 x 2048).
-template <typename CT>
-__device__ __forceinline__ void write_rows(const TcParams &p, const uint8_t *staged, int row0, int tok0, int quarter, int lane) {
-    const int features = (int)(p.M - row0 < BM ? p.M - row0 : BM), tokens = (int)(p.N - tok0 < OUT_TOKENS ? p.N - tok0 : OUT_TOKENS);
-    uint16_t *row = reinterpret_cast<uint16_t *>(static_cast<CT *>(p.C) + ((int64_t)tok0 + quarter) * p.c_tok_stride + row0);
-    const uint32_t *src = reinterpret_cast<const uint32_t *>(staged) + quarter * (BM / 2) + lane;
-    constexpr int kRows = OUT_TOKENS / 4, kNext = 2 * BM;  // words from one of the warp's rows to the next
-    uint32_t w[kRows][2], after[kRows][2];  // all loads first: the compiler cannot know the stores to miss them
+// One element a lane and token, 32 features of a token side by side.  One address that moves on: a 64-bit product and a compare per
+// element made a block 3500 clocks long, and short contractions twice as long (2444 tokens of 576 by 8064, fp32: 90.9 us, 38.9 now).
+// OFTEN: whole blocks without a compare per token; the other forms' kernels go without that code (16-bit results that TMA writes lose 2 %
+// to it).
+template <typename CT, bool OFTEN>
+__device__ __forceinline__ void store_rows(const TcParams &p, const uint32_t (&v)[32], CT *dst, float scale, float bias, int tokens) {
+    auto next = [&](auto *&at) {
+        at += p.c_tok_stride;
+        asm("" : "+l"(at));  // 32 addresses worked out ahead take registers from the whole kernel
+    };
+    float y[32];
 #pragma unroll
-    for (int i = 0; i < kRows; ++i)
+    for (int i = 0; i < 32; ++i) y[i] = __uint_as_float(v[i]) * scale + bias;
+    if (p.beta != 0.0f) {  // the old values are all fetched before the first store (the compiler cannot know the stores to miss them)
+        const CT *was = dst;
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            w[i][h] = src[i * kNext + 32 * h];
-            after[i][h] = src[i * kNext + 32 * h + (h == 0 || lane < 31 ? 1 : 0)];
-        }
-    const int64_t step = 4 * p.c_tok_stride;
+        for (int i = 0; i < 32; ++i, next(was))
+            if (i < tokens) y[i] += p.beta * to_float<CT>(*was);
+    }
+    if (OFTEN && tokens >= 32) {
 #pragma unroll
-    for (int i = 0; i < kRows; ++i, row += step) {
-        if (4 * i + quarter >= tokens) break;
-        const int odd = (int)(reinterpret_cast<uintptr_t>(row) >> 1 & 1);
-        if (odd && lane == 0 && features > 0) row[0] = (uint16_t)w[i][0];
+        for (int i = 0; i < 32; ++i, next(dst)) *dst = from_float<CT>(y[i]);
+    } else {
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int e = 2 * (lane + 32 * h) + odd;  // elements e and e + 1
-            const uint32_t pair = odd ? __byte_perm(w[i][h], after[i][h], 0x5432) : w[i][h];
-            if (e + 1 < features) *reinterpret_cast<uint32_t *>(row + e) = pair;
-            else if (e < features) row[e] = (uint16_t)pair;
-        }
+        for (int i = 0; i < 32; ++i, next(dst))
+            if (i < tokens) *dst = from_float<CT>(y[i]);
     }
 }
 
 // One 32-token block of this thread's output feature: scale, bias, beta, store.
-// ROWS: a 16-bit token-major C that TMA cannot write, without beta or peers, in blocks staged the same way.  A kernel of its own: as one
-// more branch it cost the others registers (spills in bf16) and 0.2 to 0.3 us (51 tokens of 624 by 2592, bf16: 8.26 -> 8.42 us).
+// ROWS: a 16-bit token-major C that TMA cannot write, without beta or peers.  A kernel of its own, since every form of the epilogue costs
+// the others registers.  Blocks staged in shared memory and written as words took three times as long as storing the elements (1024
+// tokens of 768 by 7885, bf16: 27.7 us, 17.6 now; 8192 of 2047 by 2048 57 and 52).
 template <typename CT, bool ROWS>
 __device__ __forceinline__ void emit_block(const TcParams &p, const TcOutMaps &omaps, const uint32_t (&v)[32], int row0, int64_t row,
                                            float scale, float bias, int tok0, const OutStage &out) {
-    if constexpr (ROWS) {
-        CT *dst = reinterpret_cast<CT *>(out.gen) + (int)(row - row0);
-#pragma unroll
-        for (int i = 0; i < 32; ++i) dst[i * BM] = from_float<CT>(__uint_as_float(v[i]) * scale + bias);
-        // two buffers in turn: past this barrier every warp has read the other one
-        asm volatile("bar.sync %0, 128;" ::"r"(out.barrier) : "memory");
-        write_rows<CT>(p, out.gen, row0, tok0, (int)(row - row0) >> 5, threadIdx.x & 31);
-        return;
-    }
     const bool row_ok = row < p.M;
     CT *crow = static_cast<CT *>(p.C) + row * p.c_row_stride;
+    if constexpr (ROWS) {
+        if (row_ok) store_rows<CT, true>(p, v, crow + (int64_t)tok0 * p.c_tok_stride, scale, bias, (int)(p.N - tok0));
+        return;
+    }
     if (p.n_out_maps > 0) {
         // 16-bit output, token-major C: stage [32 tokens][128 features] blocks in shared memory and let
         // TMA write them (whole 256-byte rows; the tensor map clips rows and tokens past the end)
-        if (out.reused) {
-            // two buffers in turn: the store issued from this one two blocks ago must have read it
-            if (out.first) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-            asm volatile("bar.sync %0, 128;" ::"r"(out.barrier) : "memory");
-        }
         CT *dst = reinterpret_cast<CT *>(out.gen) + (int)(row - row0);
 #pragma unroll
         for (int i = 0; i < 32; ++i) dst[i * BM] = from_float<CT>(__uint_as_float(v[i]) * scale + bias);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        // two buffers in turn: past this barrier the other one, stored from a block ago, has been read
+        if (out.reused && out.first) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
         asm volatile("bar.sync %0, 128;" ::"r"(out.barrier) : "memory");
         if (out.first) {
             if (row0 < p.M && tok0 < p.N)
@@ -220,16 +208,7 @@ __device__ __forceinline__ void emit_block(const TcParams &p, const TcOutMaps &o
             dst[q] = *reinterpret_cast<const uint4 *>(out);
         }
     } else if (row_ok) {
-        // with beta the old values are all fetched before the first store (the compiler cannot know the stores to miss them)
-        float y[32];
-#pragma unroll
-        for (int i = 0; i < 32; ++i) {
-            y[i] = __uint_as_float(v[i]) * scale + bias;
-            if (p.beta != 0.0f && (int64_t)tok0 + i < p.N) y[i] += p.beta * to_float<CT>(crow[((int64_t)tok0 + i) * p.c_tok_stride]);
-        }
-#pragma unroll
-        for (int i = 0; i < 32; ++i)
-            if ((int64_t)tok0 + i < p.N) crow[((int64_t)tok0 + i) * p.c_tok_stride] = from_float<CT>(y[i]);
+        store_rows<CT, sizeof(CT) == 4>(p, v, crow + (int64_t)tok0 * p.c_tok_stride, scale, bias, (int)(p.N - tok0));
         // column-sharded Linear: the same elements go into every peer's result over NVLink
         for (int pj = 0; pj < p.n_peers; ++pj) {
             CT *prow = static_cast<CT *>(p.peer_C[pj]) + row * p.c_row_stride;
@@ -979,7 +958,7 @@ int gemm_trit_tc_launch(int fmt, int fp32_planes, const uint8_t *A, const float 
         }
         p.n_out_maps = 1 + n_peers;
     }
-    const bool rows = !tma_out && dtype_size(c_dtype) == 2 && layout == T81B200_LAYOUT_NK && beta == 0.0f && n_peers == 0 && reinterpret_cast<uintptr_t>(C) % 2 == 0;
+    const bool rows = !tma_out && dtype_size(c_dtype) == 2 && layout == T81B200_LAYOUT_NK && beta == 0.0f && n_peers == 0;
     auto launch = [&](auto small) {
         constexpr int S = decltype(small)::value;
         return fmt == 1 ? launch_tc_ct<1, S>(c_dtype, rows, shape, mw, mx, om, p, st) : launch_tc_ct<0, S>(c_dtype, rows, shape, mw, mx, om, p, st);
