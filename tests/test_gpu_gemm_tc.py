@@ -220,3 +220,25 @@ def test_rows_off_boundaries_have_their_own_kernel(dev, out_f, dtype, out_dtype,
     names = [name for name, _ in kernels(capture(lambda: got.append(ops.linear_t2(t2, out_f, x, 192, None, None, out_dtype)))) if "gemm_trit_tc_kernel" in name]
     assert len(names) == 1 and f"ELb{own}EEE" in names[0], names
     assert torch.equal(got[0], (x.double() @ trits.double().t()).to(out_dtype or dtype))
+
+
+# The planes of float32 activations side by side in one product (up to 96 tokens a tile), apart (128) and wide (192 to 256, tiles alone):
+# tokens at the edges of the widths, one tile, tiles that follow one another and a contraction split over a cluster.
+@pytest.mark.parametrize("planes", [2, 3])
+@pytest.mark.parametrize("out_f,in_f,tokens", [(300, 700, 17), (256, 4000, 32), (300, 4000, 33), (260, 4000, 64), (5000, 3000, 65), (20000, 200, 96), (20000, 200, 97), (300, 9000, 128),
+                                               (2600, 1000, 513), (20000, 193, 129), (5530, 6000, 249), (20000, 500, 250), (700, 130, 6000)])
+def test_planes_of_float32_by_width(dev, out_f, in_f, tokens, planes):
+    from t81lib_b200 import _capi, ops
+    gen = torch.Generator(device="cuda").manual_seed(out_f + tokens)
+    trits = torch.randint(-1, 2, (out_f, in_f), generator=gen, device="cuda").float()
+    t2 = ops.pack_t2(ops.quantize_pack(trits, 0.5, "fixed")[0], out_f, in_f)
+    x = torch.randn(tokens, in_f, generator=gen, device="cuda")
+    # small planes say much: values whose second and third plane are of one sign
+    x = (x.bfloat16().float() * (1.0 + 2.0 ** -9 + 2.0 ** -18)).contiguous()
+    want = x.double() @ trits.double().t()
+    got = ops.linear_t2(t2, out_f, x, in_f, None, None, torch.float32, planes)
+    # two planes leave 2^-17 of a value out, three 2^-25; an accumulator is cut off at 2^-23 of its sum, which grows with its root, every
+    # 16 columns: the first plane's with the values' 8 bits hardly ever, the others' always, but they are 2^-8 of it
+    err = float((got.double() - want).norm() / want.norm())
+    assert err < (2.0 ** -16 if planes == 2 else 2.0 ** -20)
+    assert _capi.kernel_status(reset=True) == 0
