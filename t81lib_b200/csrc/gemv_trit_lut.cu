@@ -7,7 +7,8 @@
 //     on the previous kernel of the stream, so it starts before the programmatic-dependent-launch wait;
 //   * the activations arrive by bulk copies (cp.async.bulk, one per token and piece of the contraction range, no
 //     per-thread round trips) after that wait, in their natural order, each piece behind its own barrier so
-//     that the first chunks are multiplied while the rest is still on its way from L2;
+//     that the first chunks are multiplied while the rest is still on its way from L2; 16-bit rows off 16-byte
+//     boundaries come whole and are moved into place (move_piece), fp32 ones are converted by the consumer warps;
 //   * consumer warp (rw, kw) takes chunks kw, kw + KW, ... of rows 32*rw .. 32*rw+31: lane (g, t) reads
 //     limb t of rows g, g+8, g+16, g+24 with 128-bit shared loads and expands every tryte byte with ONE
 //     shared-memory table look-up into exact bf16 {-1,0,+1}: the byte is dropped into bits 8..15 of the
@@ -127,7 +128,7 @@ struct GemvLutParams {
     int ring1_offset, xs_offset, part_offset, sb_offset, bar_offset;
     uint32_t ntok_inv, row_blocks_inv, span_blocks_inv;  // inverse(d) of: ntok; eights of rows of a CTA; those that one CTA of a cluster finishes
     int vec_x;               // 1: rows of X start on 16-byte boundaries
-    int bulk_x;              // 1: 16-bit activations, 16-byte aligned rows, K % 8 == 0: fetched by bulk copies
+    int bulk_x;              // activations that bulk copies fetch: 1: 16-bit, 16-byte aligned rows, K % 8 == 0; 2: other 16-bit ones (move_piece)
     int independent;         // reads nothing the previous kernel of the stream wrote: 1 stores without waiting for it too (the caller says so), 2 waits before it stores (gemv_trit_lut_launch)
     int n_peers;             // other GPUs whose result receives every output element too (one segment only)
     void *peer_C[T81B200_MAX_PEERS];
@@ -217,116 +218,59 @@ template <typename XT> struct LutPlanes { static constexpr int value = 1; };
 template <> struct LutPlanes<float> { static constexpr int value = 2; };
 
 // Activations of the CTA's limbs [0, nl) (limb 0 = limb L0 of the row) for every token, in natural order, zero beyond
-// K, eight elements at a time.  16-bit values as they are; fp32 as bf16(x) and bf16(x - that) (PLANES == 2: 16 mantissa
-// bits).  Rows on 16-byte boundaries (vec_x) are read with 128-bit loads, others element by element, four (two) eights in
-// flight per thread.  For what bulk copies cannot take (see bulk_x).
-template <typename XT, int PLANES>
+// K, eight elements at a time, as bf16(x) and bf16(x - that) (16 mantissa bits).  Rows on 16-byte boundaries (vec_x) are read with
+// 128-bit loads, others element by element, four (two) eights in flight per thread.
 __device__ __forceinline__ void stage_activations(const GemvLutParams &p, int L0, int nl, uint32_t *xs, int tok_stride, int plane_stride,
                                                   int tid, int nthreads) {
-    const XT *X = static_cast<const XT *>(p.X);
+    const float *X = static_cast<const float *>(p.X);
     const int per_tok = nl * 6;
     if (per_tok == 0) return;
     const int64_t k_first = (int64_t)L0 * 48;
     int tok = 0, r = tid;  // eight r of token tok
     auto settle = [&]() { while (r >= per_tok && tok < p.ntok) { r -= per_tok; ++tok; } };
-    auto put = [&](uint32_t *dst, const XT (&e)[8]) {
-        if constexpr (PLANES == 1) {
-            uint4 q;
-            memcpy(&q, e, 16);
-            *reinterpret_cast<uint4 *>(dst) = q;
-        } else {
-            uint32_t hi[4], lo[4];
+    auto put = [&](uint32_t *dst, const float (&e)[8]) {
+        uint32_t hi[4], lo[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float e0 = to_float<XT>(e[2 * i]), e1 = to_float<XT>(e[2 * i + 1]);
-                hi[i] = pack_bf16_pair(e0, e1);
-                const __nv_bfloat162 hv = *reinterpret_cast<const __nv_bfloat162 *>(&hi[i]);
-                lo[i] = pack_bf16_pair(e0 - __low2float(hv), e1 - __high2float(hv));
-            }
-            *reinterpret_cast<uint4 *>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-            *reinterpret_cast<uint4 *>(dst + plane_stride) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+        for (int i = 0; i < 4; ++i) {
+            hi[i] = pack_bf16_pair(e[2 * i], e[2 * i + 1]);
+            const __nv_bfloat162 hv = *reinterpret_cast<const __nv_bfloat162 *>(&hi[i]);
+            lo[i] = pack_bf16_pair(e[2 * i] - __low2float(hv), e[2 * i + 1] - __high2float(hv));
         }
+        *reinterpret_cast<uint4 *>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+        *reinterpret_cast<uint4 *>(dst + plane_stride) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
     };
-    auto load_elements = [&](const XT *src, int64_t k, XT (&e)[8]) {
+    auto load_elements = [&](const float *src, int64_t k, float (&e)[8]) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) e[i] = k + i < p.K ? __ldcg(src + i) : from_float<XT>(0.0f);
+        for (int i = 0; i < 8; ++i) e[i] = k + i < p.K ? __ldcg(src + i) : 0.0f;
     };
     settle();
     if (p.vec_x) {
-        constexpr int U = 4, LOADS = (int)sizeof(XT) / 2;
+        constexpr int U = 4;
         while (tok < p.ntok) {
-            uint4 q[U][LOADS];
+            float e[U][8];
             uint32_t *dst[U];
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 const int64_t k = k_first + 8 * r;
-                const XT *src = X + (int64_t)tok * p.ldx + k;
+                const float *src = X + (int64_t)tok * p.ldx + k;
                 dst[u] = tok < p.ntok ? xs + tok * tok_stride + 4 * r : nullptr;
                 if (dst[u] && k + 8 <= p.K) {
 #pragma unroll
-                    for (int l = 0; l < LOADS; ++l) q[u][l] = __ldcg(reinterpret_cast<const uint4 *>(src) + l);
-                } else {
-                    XT e[8];
-                    if (dst[u]) load_elements(src, k, e);
-                    memcpy(&q[u], e, sizeof e);
-                }
+                    for (int l = 0; l < 2; ++l) reinterpret_cast<float4 *>(e[u])[l] = __ldcg(reinterpret_cast<const float4 *>(src) + l);
+                } else if (dst[u]) load_elements(src, k, e[u]);
                 r += nthreads;
                 settle();
             }
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 if (!dst[u]) break;
-                XT e[8];
-                memcpy(e, &q[u], sizeof e);
-                put(dst[u], e);
-            }
-        }
-    } else if constexpr (PLANES == 1) {
-        // 16-bit rows off those boundaries: three or four whole words, and single elements where the row starts on an odd
-        // place.  The loads of all eights come first and are put together afterwards: a wait per eight cost 3 us a call.
-        constexpr int U = 4;
-        while (tok < p.ntok) {
-            uint32_t w[U][5];
-            const XT *src[U];
-            uint32_t *dst[U];
-            int64_t at[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int64_t k = k_first + 8 * r;
-                src[u] = X + (int64_t)tok * p.ldx + k;
-                dst[u] = tok < p.ntok ? xs + tok * tok_stride + 4 * r : nullptr;
-                at[u] = k;
-                const bool odd = reinterpret_cast<uintptr_t>(src[u]) % 4 != 0;
-                const uint32_t *words = reinterpret_cast<const uint32_t *>(src[u] + (odd ? 1 : 0));
-                const uint16_t *halves = reinterpret_cast<const uint16_t *>(src[u]);
-                const bool load = dst[u] && k + 8 <= p.K;
-#pragma unroll
-                for (int i = 0; i < 3; ++i) w[u][i] = load ? __ldcg(words + i) : 0u;
-                w[u][3] = load && !odd ? __ldcg(words + 3) : 0u;
-                w[u][4] = 0u;
-                if (load && odd) {
-                    w[u][3] = __ldcg(halves + 7);
-                    w[u][4] = __ldcg(halves);
-                }
-                r += nthreads;
-                settle();
-            }
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                if (!dst[u]) break;
-                uint4 q = make_uint4(w[u][0], w[u][1], w[u][2], w[u][3]);
-                if (reinterpret_cast<uintptr_t>(src[u]) % 4 != 0)
-                    q = make_uint4(__byte_perm(w[u][4], q.x, 0x5410), __funnelshift_l(q.x, q.y, 16), __funnelshift_l(q.y, q.z, 16), __byte_perm(q.z, q.w, 0x5432));
-                XT e[8];
-                if (at[u] + 8 <= p.K) memcpy(e, &q, 16);
-                else load_elements(src[u], at[u], e);
-                put(dst[u], e);
+                put(dst[u], e[u]);
             }
         }
     } else {
         constexpr int U = 2;
         while (tok < p.ntok) {
-            XT e[U][8];
+            float e[U][8];
             uint32_t *dst[U];
 #pragma unroll
             for (int u = 0; u < U; ++u) {
@@ -345,7 +289,56 @@ __device__ __forceinline__ void stage_activations(const GemvLutParams &p, int L0
     }
 }
 
-template <typename XT, typename CT, int TOKB, int FMT>
+// 16-bit rows off 16-byte boundaries, or of a length that is no multiple of eight: a copy brings the aligned pieces of memory that hold
+// a token's share, its elements starting `shift` bytes into them, and a warp moves them down to where they belong, 2 KB at a
+// time (front to back, in place: what a step writes, later ones do not read), with zeros from element `valid` on.  `words`: the
+// share's length, a multiple of 96; four words more belong to it.  Consumer warps that loaded and converted such rows by
+// themselves took 4 to 5 us a launch longer than copies of aligned rows (a decode step of hidden 3073 / ffn 8193, 13 tokens, fp16:
+// 55.9 us, 36.7 at 3072 / 8192; 45.2 this way, with
+// results that leave in words).
+__device__ __forceinline__ void move_piece(uint32_t *at, int shift, int valid, int words, int lane) {
+    constexpr int U = 4;
+    for (int w0 = shift == 0 ? valid / 256 * 128 : 0; w0 < words; w0 += 128 * U) {  // what lies right and is whole stays
+        uint32_t v[U][8];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int w = w0 + 128 * u + 4 * lane;
+            if (w >= words) continue;
+            const uint4 a = *reinterpret_cast<const uint4 *>(at + w), b = *reinterpret_cast<const uint4 *>(at + w + 4);
+            v[u][0] = a.x; v[u][1] = a.y; v[u][2] = a.z; v[u][3] = a.w; v[u][4] = b.x; v[u][5] = b.y; v[u][6] = b.z; v[u][7] = b.w;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int w = w0 + 128 * u + 4 * lane;
+            if (w >= words) continue;
+            if (shift & 8) {
+#pragma unroll
+                for (int i = 0; i < 6; ++i) v[u][i] = v[u][i + 2];
+            }
+            if (shift & 4) {
+#pragma unroll
+                for (int i = 0; i < 5; ++i) v[u][i] = v[u][i + 1];
+            }
+            if (shift & 2) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) v[u][i] = __byte_perm(v[u][i], v[u][i + 1], 0x5432);
+            }
+            if (2 * w + 8 > valid) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int left = valid - 2 * (w + i);
+                    v[u][i] = left >= 2 ? v[u][i] : (left == 1 ? v[u][i] & 0xFFFFu : 0u);
+                }
+            }
+            *reinterpret_cast<uint4 *>(at + w) = make_uint4(v[u][0], v[u][1], v[u][2], v[u][3]);
+        }
+        __syncwarp();
+    }
+}
+
+// MOVED: bulk_x == 2.  A kernel of its own: as a run-time choice it cost aligned rows 1 to 3 %.
+template <typename XT, typename CT, int TOKB, int FMT, bool MOVED>
 __global__ void __launch_bounds__(kThreads, 1)
 gemv_trit_lut_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ CUtensorMap map1,
                      const __grid_constant__ CUtensorMap map2, const GemvLutParams p) {
@@ -375,6 +368,7 @@ gemv_trit_lut_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
     auto empty_bar = [&](int st) { return bars + 8u * (p.stages + st); };
     const uint32_t x_bar = bars + 8u * (2 * p.stages);
     const uint32_t lut_bar = x_bar + 8u * kXPieces, sb_bar = lut_bar + 8u;  // decode tables; row scales and biases have landed
+    const uint32_t moved_bar = sb_bar + 8u;  // a piece of the activations has been moved into place
     auto ring_offset = [&](int st) { return st < p.ring0_stages ? st * p.stage_bytes : p.ring1_offset + (st - p.ring0_stages) * p.stage_bytes; };
 
     cg::cluster_group cluster = cg::this_cluster();
@@ -406,9 +400,12 @@ gemv_trit_lut_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
 
     // x arrives in up to kXPieces pieces of x_group chunks each, every piece behind its own barrier: the first
     // chunks can be multiplied while the rest of the activations is still on its way from L2
-    const int x_group = (chunks_cta + kXPieces - 1) / kXPieces > 0 ? (chunks_cta + kXPieces - 1) / kXPieces : 1;
+    // (MOVED: in one; moving four took the warps longer than it hid: a decode step of hidden 4097, 8 tokens, 110 and 120 us)
+    constexpr int kPieces = MOVED ? 1 : kXPieces;
+    const int x_group = (chunks_cta + kPieces - 1) / kPieces > 0 ? (chunks_cta + kPieces - 1) / kPieces : 1;
     if (threadIdx.x < p.stages) { mbar_init(full_bar(threadIdx.x), 1); mbar_init(empty_bar(threadIdx.x), p.row_warps); }
-    if (threadIdx.x >= kMaxStages && threadIdx.x < kMaxStages + kXPieces) mbar_init(x_bar + 8u * (threadIdx.x - kMaxStages), 1);
+    if (threadIdx.x >= kMaxStages && threadIdx.x < kMaxStages + kXPieces) mbar_init(x_bar + 8u * (threadIdx.x - kMaxStages), MOVED ? p.ntok : 1);
+    if (MOVED && threadIdx.x == kMaxStages) mbar_init(moved_bar, p.ntok);
     if (threadIdx.x == kMaxStages + kXPieces) { mbar_init(lut_bar, 1); mbar_init(sb_bar, 1); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     __syncthreads();
@@ -443,7 +440,7 @@ gemv_trit_lut_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
     struct { uint32_t dst, bytes, bar; const uint16_t *src; } x_copy = {0u, 0u, 0u, nullptr};
     auto plan_x = [&](int i) {
         x_copy.bytes = 0u;
-        if (i >= kXPieces * p.ntok) return;
+        if (i >= kPieces * p.ntok) return;
         const int j = divided(i, p.ntok_inv), tok = i - j * p.ntok;
         int e0, e1;
         x_piece(j, e0, e1);
@@ -451,6 +448,16 @@ gemv_trit_lut_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
         x_copy.dst = smem_u32(xs + tok * tok_stride + e0 / 2);
         x_copy.bar = x_bar + 8u * j;
         x_copy.src = static_cast<const uint16_t *>(p.X) + (int64_t)tok * p.ldx + (int64_t)L0 * 48 + e0;  // either 16-bit type
+        if (MOVED && x_copy.bytes) {
+            const uint32_t shift = (uint32_t)(reinterpret_cast<uintptr_t>(x_copy.src) & 15);
+            x_copy.src -= shift / 2;
+            x_copy.bytes = (x_copy.bytes + shift + 15u) & ~15u;
+        }
+    };
+    auto copy_x = [&]() {
+        if (!x_copy.bytes) return;
+        if (MOVED) mbar_arrive_expect_tx(x_copy.bar, x_copy.bytes);
+        bulk_load(x_copy.dst, x_copy.src, x_copy.bytes, x_copy.bar);
     };
 
     constexpr int NACC = 2;
@@ -518,14 +525,14 @@ gemv_trit_lut_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
         rw = warp % p.row_warps;
         kw = warp / p.row_warps;
         // what lies between K and the end of the CTA's padded range is zero and is written now, before the wait
-        if (p.bulk_x) {
+        if (!MOVED && p.bulk_x) {
             const int zero_words = nl * 24 - (int)(valid / 2);
             for (int item = threadIdx.x; item < p.ntok * zero_words; item += consumer_threads) {
                 const int tok = item / zero_words;
                 xs[tok * tok_stride + (int)(valid / 2) + (item - tok * zero_words)] = 0u;
             }
         }
-        if (p.bulk_x && threadIdx.x == 0) expect_x();
+        if (!MOVED && p.bulk_x && threadIdx.x == 0) expect_x();
         if (p.bulk_x) plan_x(warp + lane * consumer_warps);
         asm volatile("bar.sync 1, %0;" ::"r"(consumer_threads) : "memory");  // zero padding, expected bytes
         if (!p.independent) {
@@ -541,13 +548,13 @@ gemv_trit_lut_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
         }
         bool ok = true;
         if (p.bulk_x) {
-            if (x_copy.bytes) bulk_load(x_copy.dst, x_copy.src, x_copy.bytes, x_copy.bar);
-            for (int i = warp + (lane + 32) * consumer_warps; i < kXPieces * p.ntok; i += 32 * consumer_warps) {  // one warp only
+            copy_x();
+            for (int i = warp + (lane + 32) * consumer_warps; i < kPieces * p.ntok; i += 32 * consumer_warps) {  // one warp only
                 plan_x(i);
-                if (x_copy.bytes) bulk_load(x_copy.dst, x_copy.src, x_copy.bytes, x_copy.bar);
+                copy_x();
             }
-        } else {
-            stage_activations<XT, PLANES>(p, L0, nl, xs, tok_stride, plane_stride, threadIdx.x, consumer_threads);
+        } else if constexpr (PLANES == 2) {
+            stage_activations(p, L0, nl, xs, tok_stride, plane_stride, threadIdx.x, consumer_threads);
             asm volatile("bar.sync 1, %0;" ::"r"(consumer_threads) : "memory");
         }
         // row scales and biases the producer's bulk copies do not bring (see there), while the activations land; absent ones are 1 and 0
@@ -557,6 +564,15 @@ gemv_trit_lut_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
         if (!bias_by_copy)
             for (int r = threadIdx.x; r < rows_per_cta; r += consumer_threads)
                 sb[rows_per_cta + r] = cta_row0 + r < S.M && S.bias ? S.bias[cta_row0 + r] : 0.0f;
+        if (MOVED && valid > 0) {
+            ok = __all_sync(0xffffffffu, mbar_wait(x_bar, 0));
+            for (int tok = warp; tok < p.ntok && ok; tok += consumer_warps) {
+                const uint16_t *src = static_cast<const uint16_t *>(p.X) + (int64_t)tok * p.ldx + (int64_t)L0 * 48;
+                move_piece(xs + tok * tok_stride, (int)(reinterpret_cast<uintptr_t>(src) & 15), (int)valid, chunks_cta * 96, lane);
+                if (lane == 0) mbar_arrive(moved_bar);
+            }
+        }
+        const uint32_t ready_bar = MOVED ? moved_bar : x_bar;
         TRACE_STAMP(3);
 
         int tok_off[TOKB];
@@ -572,7 +588,7 @@ gemv_trit_lut_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
         for (int c = kw; c < chunks_cta && ok; c += p.k_warps, st += p.k_warps, xc += p.k_warps) {
             if (st >= p.stages) { st -= p.stages; phase ^= 1u; }
             while (xc >= x_group) { xc -= x_group; ++xg; }
-            ok = __all_sync(0xffffffffu, mbar_wait(full_bar(st), phase) && (!p.bulk_x || mbar_wait(x_bar + 8u * xg, 0)));
+            ok = __all_sync(0xffffffffu, mbar_wait(full_bar(st), phase) && (!p.bulk_x || mbar_wait(ready_bar + 8u * xg, 0)));
             if (!ok) break;
             if constexpr (FMT == 1) {
                 const uint8_t *tile = smem + ring_offset(st) + rw * 1536 + lane * 48;
@@ -713,6 +729,24 @@ gemv_trit_lut_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
             }
             return;
         }
+        if (p.beta == 0.0f && p.n_peers == 0 && row + 8 <= S.M) {  // whole words where there are any
+            if constexpr (sizeof(CT) == 2) {
+                uint32_t *words = reinterpret_cast<uint32_t *>(reinterpret_cast<uintptr_t>(c + 1) & ~(uintptr_t)3);
+                if (reinterpret_cast<uintptr_t>(c) & 2) {
+                    c[0] = from_float<CT>(y[0]);
+#pragma unroll
+                    for (int i = 0; i < 3; ++i) words[i] = pack_pair<CT>(y[2 * i + 1], y[2 * i + 2]);
+                    c[7] = from_float<CT>(y[7]);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) words[i] = pack_pair<CT>(y[2 * i], y[2 * i + 1]);
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) c[i] = from_float<CT>(y[i]);
+            }
+            return;
+        }
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             if (row + i >= S.M) continue;
@@ -848,7 +882,7 @@ bool lay_out(Plan &pl, int fmt, int planes, int ntok, int tokpad, int rwv, int k
     // partial sums of the K-slices, and behind them the receive slots of the cluster fold (one per rank)
     const size_t part_bytes = align_up((size_t)kwv * tokpad * (rows + 4) * 4 + (s > 1 ? (size_t)tokpad * (rows + 4 * s) * 4 : 0), 128);
     const size_t sb_bytes = align_up((size_t)2 * rows * 4, 128);
-    const size_t bar_bytes = 1024;  // 2 * 48 + 4 + 2 barriers
+    const size_t bar_bytes = 1024;  // 2 * 48 + 4 + 3 barriers
     size_t off = fmt == 1 ? 0 : kWindowHi;  // no table, no window to keep free
     pl.xs_offset = (int)off; off += xs_bytes;
     pl.part_offset = (int)off; off += part_bytes;
@@ -965,9 +999,9 @@ int make_plan(Plan &pl, const PlanKey &key, bool rules = true) {
     return T81B200_OK;
 }
 
-template <typename XT, typename CT, int TOKB, int FMT>
+template <typename XT, typename CT, int TOKB, int FMT, bool MOVED>
 int launch_lut(const Plan &pl, const GemvLutParams &p, cudaStream_t st) {
-    auto kern = gemv_trit_lut_kernel<XT, CT, TOKB, FMT>;
+    auto kern = gemv_trit_lut_kernel<XT, CT, TOKB, FMT, MOVED>;
     // the shared-memory limit is a per-device attribute of the function: raised once per device
     static std::atomic<bool> configured[64];
     int dev = 0;
@@ -994,13 +1028,19 @@ int launch_lut(const Plan &pl, const GemvLutParams &p, cudaStream_t st) {
     return T81B200_OK;
 }
 
+template <typename XT, typename CT, int FMT>
+int launch_lut_form(const Plan &pl, const GemvLutParams &p, cudaStream_t st) {
+    if constexpr (!std::is_same<XT, float>::value)
+        if (p.bulk_x == 2) return p.ntok > 8 ? launch_lut<XT, CT, 2, FMT, true>(pl, p, st) : launch_lut<XT, CT, 1, FMT, true>(pl, p, st);
+    return p.ntok > 8 ? launch_lut<XT, CT, 2, FMT, false>(pl, p, st) : launch_lut<XT, CT, 1, FMT, false>(pl, p, st);
+}
+
 template <typename XT, int FMT>
 int launch_lut_ct(const Plan &pl, const GemvLutParams &p, int c_dtype, cudaStream_t st) {
-    const bool wide = p.ntok > 8;
     switch (c_dtype) {
-        case T81B200_F32: return wide ? launch_lut<XT, float, 2, FMT>(pl, p, st) : launch_lut<XT, float, 1, FMT>(pl, p, st);
-        case T81B200_BF16: return wide ? launch_lut<XT, __nv_bfloat16, 2, FMT>(pl, p, st) : launch_lut<XT, __nv_bfloat16, 1, FMT>(pl, p, st);
-        case T81B200_F16: return wide ? launch_lut<XT, __half, 2, FMT>(pl, p, st) : launch_lut<XT, __half, 1, FMT>(pl, p, st);
+        case T81B200_F32: return launch_lut_form<XT, float, FMT>(pl, p, st);
+        case T81B200_BF16: return launch_lut_form<XT, __nv_bfloat16, FMT>(pl, p, st);
+        case T81B200_F16: return launch_lut_form<XT, __half, FMT>(pl, p, st);
     }
     return fail(T81B200_EINVAL, "gemm_trit: unknown output dtype %d", c_dtype);
 }
@@ -1089,7 +1129,7 @@ int gemv_trit_lut_launch(int fmt, int n_seg, const uint8_t *const *A, const floa
     PlanKey key;
     memset(&key, 0, sizeof key);
     for (int i = 0; i < n_seg; ++i) { key.A[i] = A[i]; key.M[i] = M[i]; }
-    const int bulk_x = x_dtype != T81B200_F32 && reinterpret_cast<uintptr_t>(X) % 16 == 0 && (ldx * 2) % 16 == 0 && K % 8 == 0 ? 1 : 0;
+    const int bulk_x = x_dtype == T81B200_F32 ? 0 : (reinterpret_cast<uintptr_t>(X) % 16 == 0 && (ldx * 2) % 16 == 0 && K % 8 == 0 ? 1 : 2);
     key.bulk_x = bulk_x;
     key.K = K; key.n_seg = n_seg; key.ntok = ntok; key.x_dtype = x_dtype; key.c_dtype = c_dtype; key.fmt = fmt;
     T81_CUDA_TRY(cudaGetDevice(&key.device));

@@ -151,3 +151,29 @@ def test_every_row_length_has_a_launch_shape(dev, rows, tokens):
         assert torch.equal(got, want), K
         assert torch.equal(ops.linear_t2(t2, rows, x, K, None, None, torch.float32), want), K
     assert _capi.kernel_status(reset=True) == 0
+
+
+# 16-bit rows off 16-byte boundaries and of lengths that are no multiple of eight, which warps move into place behind the copies: every
+# distance from a boundary, rows of one piece and of several, one to sixteen tokens, clusters; nothing beside the rows is used.
+@pytest.mark.gpu
+@pytest.mark.parametrize("fmt", ["t2", "limbs"])
+@pytest.mark.parametrize("rows,k", [(32, 1), (70, 7), (33, 191), (64, 193), (96, 513), (4096, 1001), (300, 2050), (1000, 4100), (64, 14335), (14336, 775)])
+def test_rows_off_boundaries_are_moved_into_place(lib_built, rows, k, fmt):
+    from t81lib_b200 import _capi, ops
+    gen = torch.Generator(device="cuda").manual_seed(rows + k)
+    trits = torch.randint(-1, 2, (rows, k), generator=gen, device="cuda").float()
+    packed = ops.quantize_pack(trits, 0.5, "fixed")[0]
+    t2 = ops.pack_t2(packed, rows, k)
+    for tokens in (1, 3, 8, 9, 16):
+        for skip in range(8):
+            dtype = torch.bfloat16 if (skip + tokens) % 2 else torch.float16
+            wide = torch.full((tokens, k + skip + tokens % 4), float("nan"), device="cuda", dtype=dtype)
+            x = wide[:, skip:skip + k]
+            x.copy_(torch.randint(-1, 2, (tokens, k), generator=gen, device="cuda"))
+            want = (x.double() @ trits.double().t()).to(torch.float32)
+            if fmt == "t2":
+                got = ops.linear_t2(t2, rows, x, k, None, None, torch.float32)
+            else:
+                got = ops.gemm_trit(packed, x, M=rows, K=k, layout="nk", out_dtype=torch.float32)
+            assert torch.equal(got, want), (tokens, skip)
+    assert _capi.kernel_status(reset=True) == 0
