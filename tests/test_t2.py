@@ -165,8 +165,8 @@ def test_rows_off_boundaries_are_moved_into_place(lib_built, rows, k, fmt):
     packed = ops.quantize_pack(trits, 0.5, "fixed")[0]
     t2 = ops.pack_t2(packed, rows, k)
     for tokens in (1, 3, 8, 9, 16):
-        for skip in range(8):
-            dtype = torch.bfloat16 if (skip + tokens) % 2 else torch.float16
+        for skip in range(12):  # the last four: float32 rows, converted from the pieces that hold them
+            dtype = torch.float32 if skip >= 8 else (torch.bfloat16 if (skip + tokens) % 2 else torch.float16)
             wide = torch.full((tokens, k + skip + tokens % 4), float("nan"), device="cuda", dtype=dtype)
             x = wide[:, skip:skip + k]
             x.copy_(torch.randint(-1, 2, (tokens, k), generator=gen, device="cuda"))
