@@ -6,8 +6,8 @@
 // its shared memory and loads half of the tile's activation rows by TMA; the even CTA issues the MMAs, which read both
 // halves, and each CTA keeps its 128 accumulator rows in TMEM (2 x 256 fp32 columns, double-buffered across tiles).
 // Measured against the one-CTA 128 x 256 kernel before it (bf16, weights in limbs there and in codes here):
-// 4096 x 14336 x 16384 tokens 1700 -> 1160 us (958 -> 1391 TFLOP/s in a long run under the power cap), 9216 x 3072 x 2048
-// 109 -> 90, 14336 x 4096 x 80 40.9 -> 20.6 us.
+// 4096 x 14336 x 16384 tokens 958 -> 1529 TFLOP/s in a long run under the power cap, 9216 x 3072 x 2048 109 -> 83 us, 14336 x 4096 x 80
+// 40.9 -> 19.2 us.
 // What bounds the kernel is shared-memory bandwidth: a 64-deep step writes and reads 16 KB of expanded weights per CTA
 // and writes and reads the activations, against 512 clocks of MMA at 256 tokens.  Halving the activation share is what
 // the pair is for: a single CTA with a 128 x 256 tile needs 768 clocks of shared memory per 512 of MMA.
@@ -21,7 +21,7 @@
 // 192 columns are four limbs and three 64-column operand atoms: the unit in which converters hand weights to the MMAs.
 //
 // Activations: 16-bit types as they are (A and B of one MMA have the same type), fp32 as bf16 planes (x = hi + lo, 16
-// mantissa bits) that are multiplied one after the other with the same expanded weights.  Rows TMA cannot read
+// mantissa bits) that are multiplied with the same expanded weights, side by side or in turn (Mode).  Rows TMA cannot read
 // (unaligned, the (K, N) layout, fp32) are first copied into token-major planes in the caller's workspace.
 // All planes but the first have an accumulator of their own beside it, and the epilogue adds the two.  The tensor core cuts an
 // accumulator off at every 16 columns instead of rounding it.  With the first plane alone little is cut (trits times 8-bit
