@@ -222,8 +222,8 @@ def test_rows_off_boundaries_have_their_own_kernel(dev, out_f, dtype, out_dtype,
     assert torch.equal(got[0], (x.double() @ trits.double().t()).to(out_dtype or dtype))
 
 
-# The planes of float32 activations side by side in one product (up to 96 tokens a tile), apart (128) and wide (192 to 256, tiles alone):
-# tokens at the edges of the widths, one tile, tiles that follow one another and a contraction split over a cluster.
+# The planes of float32 activations in tiles of up to 128 tokens and of 192 to 256 (tiles alone): tokens at the edges of the widths, one
+# tile, tiles that follow one another and a contraction split over a cluster.
 @pytest.mark.parametrize("planes", [2, 3])
 @pytest.mark.parametrize("out_f,in_f,tokens", [(300, 700, 17), (256, 4000, 32), (300, 4000, 33), (260, 4000, 64), (5000, 3000, 65), (20000, 200, 96), (20000, 200, 97), (300, 9000, 128),
                                                (2600, 1000, 513), (20000, 193, 129), (5530, 6000, 249), (20000, 500, 250), (700, 130, 6000)])
