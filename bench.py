@@ -564,11 +564,27 @@ def run_ours(args):
         os._exit(0)
 
 
+def link_rates(torch, dev, host, out):
+    """The prefill's copies by themselves: what share of an end-to-end step the host link takes on this machine."""
+    dst = {w: torch.empty_like(t, device=dev) for w, t in host.items()}
+    src = torch.empty_like(out, device=dev)
+    rates = {}
+    for name, copies in (("h2d_gbs", [(dst[w], t) for w, t in host.items()]), ("d2h_gbs", [(out, src)])):
+        t0, t1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        t0.record()
+        for to, frm in copies:
+            to.copy_(frm, non_blocking=True)
+        t1.record()
+        torch.cuda.synchronize()
+        rates[name] = sum(t.numel() * t.element_size() for t, _ in copies) / (t0.elapsed_time(t1) * 1e-3) / 1e9
+    return rates
+
+
 def e2e_public_api(torch, dev, Linear, layers, args, world=1, rank=0):
     """Same job through nn.Module calls: pinned host activations are copied in for the
     prefill and for every decode step, the last Linear's output is copied back."""
     import t81lib_b200.torch as t81_torch
-    from t81lib_b200 import ops
+    from t81lib_b200 import _capi, ops
     mods = []
     for layer in layers:
         row = []
@@ -718,6 +734,8 @@ def e2e_public_api(torch, dev, Linear, layers, args, world=1, rank=0):
     e1.record()
     torch.cuda.synchronize()
     sec = e0.elapsed_time(e1) * 1e-3 / steps
+    assert _capi.kernel_status(reset=True) == 0, "a kernel reported a timed-out wait"
+    link = link_rates(torch, dev, host_p, out_p) if rank == 0 else None
     if world > 1:
         import torch.distributed as dist
         t = torch.tensor([sec], device=dev, dtype=torch.float64)
@@ -726,7 +744,7 @@ def e2e_public_api(torch, dev, Linear, layers, args, world=1, rank=0):
     h2d = 2 * (ptok + DECODE * dtok) * (HIDDEN + FFN)
     d2h = 2 * (ptok + DECODE * dtok) * HIDDEN
     return {"value": BATCH * (PREFILL + DECODE) / sec, "unit": "tokens/s", "h2d_bytes_per_step": h2d,
-            "d2h_bytes_per_step": d2h, "steps": steps, "api": ("t81lib_b200.nn.Linear.forward" if world == 1 else
+            "d2h_bytes_per_step": d2h, "steps": steps, "copies_alone": link, "api": ("t81lib_b200.nn.Linear.forward" if world == 1 else
                                                                     "t81lib_b200.nn.sharded.ShardedLinear.forward (prefill: exchange='p2p'; decode: " +
                                                                     ("step_ordered + close_step" if step_sharded else "whole-matrix t81lib_b200.nn.Linear on every rank") + ")")
                    + " (prefill eager; decode pass replayed from a torch.cuda.CUDAGraph)" +
