@@ -568,6 +568,9 @@ gemv_trit_lut_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
             if (threadIdx.x == 0 && !exchange_wait(p.sync_local, p.n_peers))
                 atomicCAS(&g_lut_status, LUT_STATUS_OK, LUT_STATUS_TIMEOUT_EXCHANGE);
             asm volatile("bar.sync 1, %0;" ::"r"(consumer_threads) : "memory");
+            // Their stores and the acquire above are of the generic proxy, the copies below are not, and no kernel's end lies between:
+            // every thread that may issue one orders the two.
+            asm volatile("fence.proxy.async.global;" ::: "memory");
         }
         bool ok = true;
         if (p.bulk_x) {

@@ -51,6 +51,26 @@ def main() -> int:
     layer.exchange_for(8, torch.bfloat16, dev).flags.wait()
     torch.cuda.synchronize()
     ok = ok and torch.equal(outs[-1], want) and torch.equal(outs[-2], want)
+    # The same through layers whose widths are no multiples of eight (16-bit rows off 16-byte boundaries): each reads what the peers
+    # stored for the one before, with no kernel's end between those stores and the read.  Whole numbers: exact in any order of the sums.
+    odd = [torch.randint(-1, 2, (o, i), generator=gen, device=dev).float() for o, i in ((770, 521), (1030, 770), (522, 1030))]
+    for tokens, dtype in ((8, torch.bfloat16), (3, torch.float16), (16, torch.float32)):
+        x = want = torch.randint(-1, 2, (tokens, 521), generator=gen, device=dev).to(dtype)
+        chain = [ShardedLinear(m, None, threshold=0.5, rule="fixed", exchange="p2p") for m in odd]
+        for m in odd:
+            want = (want.double() @ m.double().t()).to(dtype)
+        for layer_ in chain:
+            layer_.defer_wait = True
+        for _ in range(20):
+            y = x
+            for layer_ in chain:
+                y = layer_(y)
+            chain[-1].exchange_for(tokens, dtype, dev).flags.wait()
+            torch.cuda.synchronize()
+            same = torch.equal(y, want)
+            ok = ok and same
+            if rank == 0 and not same:
+                print(f"CHAIN MISMATCH tokens={tokens} dtype={dtype}", flush=True)
     # A result is read AFTER the next same-shape call has been issued, while the peer runs ahead: rank 0 stalls
     # its stream before the read, the other ranks go on issuing calls that store into rank 0's buffers.  With
     # three buffers per shape the peers' stores of call j + 2 cannot land in the buffer that holds result j.
