@@ -439,10 +439,11 @@ gemv_trit_lut_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
     // implies "everything before it has".
     if (p.independent) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
-    // Activations by bulk copy (16-bit types, 16-byte aligned rows, K a multiple of 8): the copies bring exactly the
-    // elements below K, one copy per token and piece; piece j holds the elements of chunks
-    // [j * x_group, (j + 1) * x_group) that exist.  Issuing a copy costs its warp tens of nanoseconds, so the
-    // consumer warps share them out (lane 0 of each), in piece order: no warp starts its chunks late.
+    // Activations by bulk copy (16-bit types), one copy per token and piece; piece j holds the elements of chunks
+    // [j * x_group, (j + 1) * x_group) that exist.  Of 16-byte aligned rows, K a multiple of 8, they bring exactly the elements
+    // below K; of others (MOVED) the 16-byte pieces that hold them, up to 14 bytes beside them on either side, which nothing uses.
+    // Issuing a copy costs its warp tens of nanoseconds, so the consumer warps share them out, in piece order: no warp
+    // starts its chunks late.
     int64_t valid = p.K - (int64_t)L0 * 48;  // elements of this CTA's range that exist
     valid = valid < 0 ? 0 : (valid > (int64_t)nl * 48 ? (int64_t)nl * 48 : valid);
     auto x_piece = [&](int j, int &e0, int &e1) {
@@ -940,7 +941,7 @@ int make_plan(Plan &pl, const PlanKey &key, bool rules = true) {
     Switches sw = switches();
     const bool forced = sw.rw != 0;
     if (rules && key.fmt == 1 && key.bulk_x && !forced) {
-        // Where bulk copies bring the activations (no warp converts them), short rows need no cluster: its fold costs about a
+        // Where bulk copies bring the activations (no warp converts them; moved rows: below), short rows need no cluster: its fold costs about a
         // microsecond, and one CTA's copy of the activations is small.  Over 122 shapes in every launch shape the model below is
         // 16 and 11 % behind the best for K up to 1152 and 1728, and a warp row of four K-slices is within 4 % of it for every
         // number of tokens as long as the CTAs are at most three per SM (5504 x 1536, 8 tokens: 4.65 -> 3.85 us; 9216 x 1280, 10
@@ -952,9 +953,22 @@ int make_plan(Plan &pl, const PlanKey &key, bool rules = true) {
         const int chunks = kl4 / 4;
         int64_t tiles32 = 0, tiles64 = 0;
         for (int i = 0; i < key.n_seg; ++i) { tiles32 += (key.M[i] + 31) / 32; tiles64 += (key.M[i] + 63) / 64; }
-        if (chunks >= 4 && chunks <= 9 && tiles32 <= 3 * sms) { sw.rw = 1; sw.kw = 4; sw.s = 1; }
-        else if (key.ntok > 8 && chunks >= 10 && chunks <= 18 && tiles64 <= sms) { sw.rw = 2; sw.kw = 4; sw.s = 2; }
-        else if (key.ntok <= 8 && chunks >= 43 && tiles64 >= 8 && tiles64 <= 32) { sw.rw = 2; sw.kw = 2; sw.s = 8; }
+        // Rows that are moved into place (bulk_x == 2) take the same shapes, 570 of them measured with and without the rules: 0.72,
+        // 0.90 and 0.99 of the time on average, and 1.2 to 1.7 times in two places that are left to the model.  Nine chunks and more
+        // than nine tokens of two CTAs an SM, where the model's 64-row tiles are one wave (16 tokens of 1700 by 8200: 7.3 and 4.4 us;
+        // 12 tokens 5.3 and 4.2), and with 16 tokens, three of whose CTAs no SM holds, any number above one an SM.  And eight slices
+        // of more than 24 tiles whose CTAs are too large for four an SM, so that not all are resident (7 tokens of 13050 by 1792: 5.9
+        // and 4.5 us); from 31 tiles and 69 chunks on the model's own choice is slower still (8 of 14086 by 2024: 6.5 and 9.0).
+        const bool moved = key.bulk_x == 2;
+        const bool crowded = moved && chunks == 9 && key.ntok > 9 && tiles32 > sms && (tiles32 <= 2 * sms || key.ntok > 15);
+        Plan eighth;
+        const bool all_resident = !moved || tiles64 <= 24 || (tiles64 > 30 && chunks >= 69) ||
+                                  (lay_out(eighth, 1, planes, key.ntok, tokpad, 2, 2, 8, (chunks + 7) / 8 * 4, (chunks + 7) / 8, kSmemBudget) &&
+                                   4 * (eighth.smem + 1024) <= 228 * 1024);
+        if (chunks >= 4 && chunks <= 9 && tiles32 <= 3 * sms) {
+            if (!crowded) { sw.rw = 1; sw.kw = 4; sw.s = 1; }
+        } else if (key.ntok > 8 && chunks >= 10 && chunks <= 18 && tiles64 <= sms) { sw.rw = 2; sw.kw = 4; sw.s = 2; }
+        else if (key.ntok <= 8 && chunks >= 43 && tiles64 >= 8 && tiles64 <= 32 && all_resident) { sw.rw = 2; sw.kw = 2; sw.s = 8; }
     }
     double best_t = 1e30;
     Plan best;

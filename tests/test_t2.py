@@ -177,3 +177,18 @@ def test_rows_off_boundaries_are_moved_into_place(lib_built, rows, k, fmt):
                 got = ops.gemm_trit(packed, x, M=rows, K=k, layout="nk", out_dtype=torch.float32)
             assert torch.equal(got, want), (tokens, skip)
     assert _capi.kernel_status(reset=True) == 0
+
+
+# Moved rows where the launch shape changes hands: nine chunks with one, two and three CTAs an SM, eight slices whose CTAs are all
+# resident and those whose are not.
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,k,tokens", [(4736, 1699, 16), (4737, 1699, 16), (9473, 1699, 16), (4737, 1601, 10), (9472, 1601, 10), (9473, 1601, 15), (1536, 13051, 7), (1537, 13051, 7),
+                                           (1792, 11011, 8), (1985, 13300, 8), (1921, 13051, 6), (1600, 14085, 5)])
+def test_moved_rows_by_launch_shape(lib_built, rows, k, tokens):
+    from t81lib_b200 import _capi, ops
+    gen = torch.Generator(device="cuda").manual_seed(rows + k)
+    trits = torch.randint(-1, 2, (rows, k), generator=gen, device="cuda").float()
+    t2 = ops.pack_t2(ops.quantize_pack(trits, 0.5, "fixed")[0], rows, k)
+    x = torch.randint(-1, 2, (tokens, k), generator=gen, device="cuda").bfloat16()
+    assert torch.equal(ops.linear_t2(t2, rows, x, k, None, None, torch.float32), (x.double() @ trits.double().t()).float())
+    assert _capi.kernel_status(reset=True) == 0
