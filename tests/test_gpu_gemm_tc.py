@@ -242,3 +242,61 @@ def test_planes_of_float32_by_width(dev, out_f, in_f, tokens, planes):
     err = float((got.double() - want).norm() / want.norm())
     assert err < (2.0 ** -16 if planes == 2 else 2.0 ** -20)
     assert _capi.kernel_status(reset=True) == 0
+
+
+# Every form in which planes meet: accumulators 128 or 256 columns apart, tiles alone, one after the other and split over a cluster.  The
+# form is read from what was launched, so that other step costs cannot drop one unseen.
+TC_PARAM_WIDTH, TC_PARAM_SPLITS, TC_PARAM_M_TILES, TC_PARAM_N_TILES = 21, 26, 19, 20  # TcParams in 32-bit words
+
+
+@pytest.mark.parametrize("planes", [2, 3])
+@pytest.mark.parametrize("out_f,in_f,tokens,apart,split,alone", [
+    (10152, 11900, 114, 128, False, True), (7391, 13254, 101, 128, True, True), (6000, 3000, 120, 128, True, True), (20000, 200, 97, 128, False, False),
+    (700, 130, 6000, 256, False, True), (2807, 9347, 475, 256, True, True)])
+def test_planes_of_float32_in_every_form(dev, out_f, in_f, tokens, apart, split, alone, planes):
+    from t81lib_b200 import _capi, ops
+    gen = torch.Generator(device="cuda").manual_seed(out_f + tokens)
+    trits = torch.randint(-1, 2, (out_f, in_f), generator=gen, device="cuda").float()
+    t2 = ops.pack_t2(ops.quantize_pack(trits, 0.5, "fixed")[0], out_f, in_f)
+    x = torch.randn(tokens, in_f, generator=gen, device="cuda")
+    x = (x.bfloat16().float() * (1.0 + 2.0 ** -9 + 2.0 ** -18)).contiguous()
+    got = []
+    graph = capture(lambda: got.append(ops.linear_t2(t2, out_f, x, in_f, None, None, torch.float32, planes)))  # its parameters live as long as it does
+    launched = [(name, params(3)) for name, params in kernels(graph) if "gemm_trit_tc_kernel" in name]
+    graph.replay()
+    assert len(launched) == 1 and f"Li1ELi{apart}E" in launched[0][0], launched[0][0]
+    words = launched[0][1]
+    assert (words[TC_PARAM_SPLITS] > 1) == split and words[TC_PARAM_WIDTH] % 32 == 0 and (words[TC_PARAM_WIDTH] > 128) == (apart == 256)
+    assert (split or words[TC_PARAM_M_TILES] * words[TC_PARAM_N_TILES] <= 74) == alone
+    want = x.double() @ trits.double().t()
+    for y in got:  # the call before the capture, and the captured one
+        assert float((y.double() - want).norm() / want.norm()) < (2.0 ** -16 if planes == 2 else 2.0 ** -20)  # as above
+    assert _capi.kernel_status(reset=True) == 0
+
+
+# Products of every tile width one behind the other, each in a part of the chip's pairs so that the next one's set-up runs beside it; the
+# last pair's odd CTA has no weights.  A wait that runs out shows in the status, and in sums that are not whole.
+def test_products_of_every_width_one_behind_the_other(dev):
+    from t81lib_b200 import _capi, ops
+    gen = torch.Generator(device="cuda").manual_seed(160)
+    shapes = [(11392, 10808, (143,)), (11392, 2056, (30, 60, 90, 120, 143, 190, 220, 250)), (5504, 4104, (160, 288, 130, 448))]
+    work = []
+    for out_f, in_f, rows in shapes:
+        trits = torch.randint(-1, 2, (out_f, in_f), generator=gen, device="cuda").float()
+        t2 = ops.pack_t2(ops.quantize_pack(trits, 0.5, "fixed")[0], out_f, in_f)
+        for tokens in rows:
+            x = torch.randint(-1, 2, (tokens, in_f), generator=gen, device="cuda").bfloat16()
+            work.append((t2, out_f, x, in_f, (x.double() @ trits.double().t()).bfloat16()))
+        del trits
+    for _ in range(20):
+        for t2, out_f, x, in_f, want in work:
+            assert torch.equal(ops.linear_t2(t2, out_f, x, in_f, None, None), want)
+    for step in (1, 5):  # without anything between the products
+        got = []
+        graph = capture(lambda: got.append([ops.linear_t2(*work[step * i % len(work)][:4], None, None) for i in range(2 * len(work))]))
+        for _ in range(20):
+            graph.replay()
+            torch.cuda.synchronize()
+        for i, y in enumerate(got[-1]):
+            assert torch.equal(y, work[step * i % len(work)][4])
+    assert _capi.kernel_status(reset=True) == 0
