@@ -131,8 +131,8 @@ struct OutStage {
 // One element a lane and token, 32 features of a token side by side.  One address that moves on: a 64-bit product and a compare per
 // element made a block 3500 clocks long, and short contractions twice as long (2444 tokens of 576 by 8064, fp32: 90.9 us, 38.9 now).
 // OFTEN: whole blocks without a compare per token; the other forms' kernels go without that code (16-bit results that TMA writes lose 2 %
-// to it).
-template <typename CT, bool OFTEN>
+// to it).  BETA: there may be one.
+template <typename CT, bool OFTEN, bool BETA>
 __device__ __forceinline__ void store_rows(const TcParams &p, const uint32_t (&v)[32], CT *dst, float scale, float bias, int tokens) {
     auto next = [&](auto *&at) {
         at += p.c_tok_stride;
@@ -141,7 +141,7 @@ __device__ __forceinline__ void store_rows(const TcParams &p, const uint32_t (&v
     float y[32];
 #pragma unroll
     for (int i = 0; i < 32; ++i) y[i] = __uint_as_float(v[i]) * scale + bias;
-    if (p.beta != 0.0f) {  // the old values are all fetched before the first store (the compiler cannot know the stores to miss them)
+    if (BETA && p.beta != 0.0f) {  // the old values are all fetched before the first store (the compiler cannot know the stores to miss them)
         const CT *was = dst;
 #pragma unroll
         for (int i = 0; i < 32; ++i, next(was))
@@ -167,7 +167,7 @@ __device__ __forceinline__ void emit_block(const TcParams &p, const TcOutMaps &o
     const bool row_ok = row < p.M;
     CT *crow = static_cast<CT *>(p.C) + row * p.c_row_stride;
     if constexpr (ROWS) {
-        if (row_ok) store_rows<CT, true>(p, v, crow + (int64_t)tok0 * p.c_tok_stride, scale, bias, (int)(p.N - tok0));
+        if (row_ok) store_rows<CT, true, false>(p, v, crow + (int64_t)tok0 * p.c_tok_stride, scale, bias, (int)(p.N - tok0));
         return;
     }
     if (p.n_out_maps > 0) {
@@ -208,7 +208,7 @@ __device__ __forceinline__ void emit_block(const TcParams &p, const TcOutMaps &o
             dst[q] = *reinterpret_cast<const uint4 *>(out);
         }
     } else if (row_ok) {
-        store_rows<CT, sizeof(CT) == 4>(p, v, crow + (int64_t)tok0 * p.c_tok_stride, scale, bias, (int)(p.N - tok0));
+        store_rows<CT, sizeof(CT) == 4, true>(p, v, crow + (int64_t)tok0 * p.c_tok_stride, scale, bias, (int)(p.N - tok0));
         // column-sharded Linear: the same elements go into every peer's result over NVLink
         for (int pj = 0; pj < p.n_peers; ++pj) {
             CT *prow = static_cast<CT *>(p.peer_C[pj]) + row * p.c_row_stride;
