@@ -134,6 +134,8 @@ T81B200_API int t81b200_gemm_limb_host(const uint8_t *A, const uint8_t *B, float
  *   A          (M, ceil(K/48)) limbs, M = output features
  *   row_scale  M floats or NULL (= 1)
  *   B          dense, K x N logical, b_dtype, layout per `layout`, leading dim ldb elements
+ *              (rows that start or end off 16-byte boundaries may be read in the whole 16-byte pieces that hold them: up to 14 bytes
+ *              beside a row, which are not used; they may change meanwhile, but a race or initialisation checker sees the reads)
  *   bias       M floats or NULL
  *   C          c_dtype, layout per `layout`, leading dim ldc elements; read only if beta != 0
  *   M, N, K    output features, tokens, contraction length (K need not be a multiple of 48;

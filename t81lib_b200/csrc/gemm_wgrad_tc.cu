@@ -558,7 +558,8 @@ extern "C" int t81b200_qat_weight_grad(const void *g, int g_dtype, int64_t ldg, 
     p.vec = cols % 4 == 0 && ldw % 4 == 0 && ldw < (1ll << 37) && reinterpret_cast<uintptr_t>(w) % 16 == 0 && reinterpret_cast<uintptr_t>(out) % 16 == 0 ? 1 : 0;
     // Three slots a warp leave four stages of 16-bit operands, two leave five.  Few tokens are over before two have been read and filled
     // again, many want the stages (16-bit, us, two and three: 304 tokens of 2416 by 4965 35.2 and 30.9, 1104 of 12192 by 12476 405 and
-    // 380, 4096 of 4096 by 14336 365 and 371); fp32 stages and rows that lanes copy word by word gain nothing from a third.
+    // 380, 4096 of 4096 by 14336 365 and 371; over eight layers, three against two: 0.88 to 1.0 at 700 tokens, 0.95 to 1.02 at 2048 and 2400, 0.97
+    // to 1.06 at 2800, 0.91 to 1.07 at 4096, 1.01 to 1.25 at 6000); fp32 stages and rows that lanes copy word by word gain nothing from a third.
     p.slots = p.planes == 1 && p.vec && p.bn == 256 && tokens <= 2048 ? 3 : 2;
     const int fit = (SMEM_LIMIT - 1024 - EPILOGUE_WARPS * p.slots * BLOCK_BYTES - BARRIER_BYTES) / stage;
     p.stages = fit < MAX_STAGES ? fit : MAX_STAGES;

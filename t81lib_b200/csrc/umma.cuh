@@ -107,7 +107,10 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16
           "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
         : "memory");
 }
-// Eight columns in two steps: what `v` holds may be read past the wait only, which is for every load before it.
+// Eight columns in two steps: what `v` holds may be read past the wait only, which is for every load before it.  The first step names
+// registers as written that the load fills later, and the second takes and gives back the same ones, so that every use of `v` comes
+// behind the wait.  What the language does not promise is that no copy of them is made in between: `v` is an array that only
+// these two touch until then, in straight-line code, and the tests compare every column of the sums.
 __device__ __forceinline__ void tmem_ld8_start(uint32_t taddr, uint32_t (&v)[8]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                  : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
