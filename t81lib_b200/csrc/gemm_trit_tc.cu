@@ -371,7 +371,10 @@ gemm_trit_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         if (++raw_c >= c1) { raw_c = c0; raw_tile += n_clusters; }
     };
 
-    // launched with programmatic stream serialization: everything above overlaps the tail of the previous kernel
+    // Launched with programmatic stream serialization: everything above overlaps the tail of the previous kernel.  No more than that: with the
+    // accumulators' allocation and the cluster's meeting before this wait, tensor maps fetched there and issuing loops without a loop
+    // over planes, waits of later launches ran out or the context was lost (143 tokens of 10808 by 11392, bf16, in most processes once,
+    // behind freshly prepared launches), and reading found no cause.
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (warp == 0) {
