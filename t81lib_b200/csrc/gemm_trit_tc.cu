@@ -59,7 +59,13 @@ constexpr int CHUNK = 192;       // columns converted at a time: 3 atoms
 constexpr int A_ATOM_BYTES = BM * BK * 2;        // 16 KB
 constexpr int A_CHUNK_BYTES = 3 * A_ATOM_BYTES;  // 48 KB
 constexpr int A_MAX = 3, B_MAX = 12;             // ring slots that have barriers
-constexpr int RAW_STAGES = 3;                    // packed weights of a chunk (128 rows): 8 KB of limbs, 6 KB of codes
+// Packed weights of a chunk (128 rows): 8 KB of limbs, 6 KB of codes.  The two groups of converters take alternate chunks, so an even number of
+// slots leaves each slot to one group.  With three, a group came to a slot whose last use had been the other's, and a wait that
+// tells phases by parity passes at once if that use has not even landed: chunk 0's copy later than chunk 1's by the time chunk 1
+// takes to expand (weights whose pages are not in the TLB), and the group went on with whatever lay there and handed the slot back once
+// too often, from where on nothing fits together: waits that run out, wrong sums, a lost context.
+constexpr int RAW_STAGES = 4;
+static_assert(RAW_STAGES % 2 == 0, "a slot belongs to one of the two groups of converters");
 constexpr int MAX_SPLITS = 4;                    // clusters of up to 8 CTAs
 constexpr int NUM_THREADS = 14 * 32;
 constexpr int EPILOGUE_WARP0 = 2, CONVERTER_WARP0 = 6;
@@ -68,7 +74,7 @@ constexpr int OUT_STAGE_BYTES = OUT_TOKENS * BM * 2;  // [token][feature] block 
 constexpr int BARRIER_BYTES = 512;
 constexpr int SMEM_LIMIT = 227 * 1024;
 template <int FMT> constexpr int kRawBytes = FMT == 1 ? 4 * 1536 : BM * 64;
-constexpr int SMEM_FIXED = RAW_STAGES * 8192 + 2 * OUT_STAGE_BYTES + BARRIER_BYTES + 1024 /*alignment*/;
+constexpr int SMEM_FIXED = 2 * OUT_STAGE_BYTES + BARRIER_BYTES + 1024 /*alignment*/;  // and the packed weights
 
 enum { STATUS_OK = 0, STATUS_TIMEOUT_PRODUCER = 1, STATUS_TIMEOUT_MMA = 2, STATUS_TIMEOUT_EPILOGUE = 3, STATUS_TIMEOUT_CONVERTER = 4 };
 
@@ -371,10 +377,7 @@ gemm_trit_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         if (++raw_c >= c1) { raw_c = c0; raw_tile += n_clusters; }
     };
 
-    // Launched with programmatic stream serialization: everything above overlaps the tail of the previous kernel.  No more than that: with the
-    // accumulators' allocation and the cluster's meeting before this wait, tensor maps fetched there and issuing loops without a loop
-    // over planes, waits of later launches ran out or the context was lost (143 tokens of 10808 by 11392, bf16, in most processes once,
-    // behind freshly prepared launches), and reading found no cause.
+    // launched with programmatic stream serialization: everything above overlaps the tail of the previous kernel
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (warp == 0) {
@@ -512,7 +515,10 @@ gemm_trit_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         Ring a, raw;
         if (group == 1) { a.advance(p.a_stages); raw.advance(RAW_STAGES); }
         bool ok = true;
-        int c = c0 + group;  // the groups take alternate chunks of the CTA's whole sequence
+        // The groups take alternate chunks of the CTA's whole sequence.  Slots of the operand ring change hands where there are three: there a
+        // group waits for the MMAs of the slot's last chunk, k - 3.  It has seen those of k - 5 end when it took its own last chunk, and MMAs
+        // end in order, so those of k - 6, the slot's use before, have ended too, and the wait cannot be a whole use behind.
+        int c = c0 + group;
         for (int left = my_tiles * span - group; left > 0; left -= 2) {
             while (c >= c1) c -= span;
             ok = __all_sync(0xffffffffu, mbar_wait(raw_full(raw.stage), raw.phase));
@@ -610,7 +616,7 @@ double step_cost(int bn, int planes) {
 // no pair has a second tile (5530 x 11021 x 249: 83 us at 128 tokens, 66 at 256).  The width 160 is left out for several planes:
 // a launch at it (728 tiles, two planes, fp32 result) failed with an unspecified error on a variant of this kernel that had other
 // issuing loops, and the cause is not known.
-TcShape pick_shape(int64_t M, int64_t N, int64_t K, int planes) {
+TcShape pick_shape(int64_t M, int64_t N, int64_t K, int planes, int raw_bytes) {
     const int64_t m_tiles = (M + 255) / 256, chunks = (K + CHUNK - 1) / CHUNK, wide = (N + 255) / 256, narrow = (N + 127) / 128;
     const int64_t least = planes > 1 && wide > resident_pair_clusters(1) ? narrow : wide, most = (planes > 1 ? narrow : wide) + 8;
     TcShape best;
@@ -632,12 +638,12 @@ TcShape pick_shape(int64_t M, int64_t N, int64_t K, int planes) {
     // One barrier per chunk instead of one per step where two stages of a chunk fit (up to 224 tokens) and the planes are not
     // several (those fill the time between two barriers anyway, and do better with a deeper ring: 200 against 220 us at
     // 4096 x 4096 x 4096, fp32, 192 tokens).  With one plane: 192 tokens 408 -> 314 us at 14336 x 4096 x 4096.
-    best.b_step = best.bn <= 128 || (planes == 1 && best.bn <= 224) ? 3 : 1;
     best.a_stages = best.bn <= 96 ? 3 : 2;
-    const int stage = best.bn * BK * best.b_step;
-    int b = (SMEM_LIMIT - SMEM_FIXED - best.a_stages * A_CHUNK_BYTES) / stage;
+    const int fixed = SMEM_FIXED + RAW_STAGES * raw_bytes, room = SMEM_LIMIT - fixed - best.a_stages * A_CHUNK_BYTES;
+    best.b_step = (best.bn <= 128 || (planes == 1 && best.bn <= 224)) && room >= 6 * best.bn * BK ? 3 : 1;
+    const int stage = best.bn * BK * best.b_step, b = room / stage;
     best.b_stages = b > B_MAX ? B_MAX : b;
-    best.smem = (size_t)best.a_stages * A_CHUNK_BYTES + (size_t)best.b_stages * stage + SMEM_FIXED;
+    best.smem = (size_t)best.a_stages * A_CHUNK_BYTES + (size_t)best.b_stages * stage + fixed;
     return best;
 }
 
@@ -871,7 +877,7 @@ bool gemm_trit_tc_eligible(int64_t M, int64_t N, int64_t K) {
 
 // Time of a launch without staging: 6 us of launch, set-up and last stores on top of the planner's figure (13.5 us estimated and 12.4
 // measured at 4096 x 4096 x 32, 18.8 and 20.3 at 14336 x 4096 x 80, both bf16).
-double gemm_trit_tc_estimate_us(int64_t M, int64_t N, int64_t K) { return 6.0 + 1.7e-3 * pick_shape(M, N, K, 1).cost; }
+double gemm_trit_tc_estimate_us(int64_t M, int64_t N, int64_t K) { return 6.0 + 1.7e-3 * pick_shape(M, N, K, 1, kRawBytes<1>).cost; }
 
 // Scratch bytes for the activations: none when they are read in place.  `planes`: bf16 planes of fp32 activations.
 size_t gemm_trit_tc_scratch_most(int b_dtype, int64_t N, int64_t K, int planes) {
@@ -908,7 +914,7 @@ int gemm_trit_tc_launch(int fmt, int fp32_planes, const uint8_t *A, const float 
         if (int rc = stage_planes(B, b_dtype, layout, ldb, N, K, planes, workspace, st)) return rc;
         x_ptr = workspace; x_ld = scratch_row(K);
     }
-    const TcShape shape = pick_shape(M, N, K, planes);
+    const TcShape shape = pick_shape(M, N, K, planes, fmt == 1 ? kRawBytes<1> : kRawBytes<0>);
     const bool f16 = b_dtype == T81B200_F16;
     CUtensorMap mw, mx;
     memset(&mw, 0, sizeof mw);

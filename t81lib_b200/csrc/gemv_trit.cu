@@ -681,6 +681,8 @@ int gemv_trit_tma_launch(const GemvParams &base, int x_dtype, int c_dtype, cudaS
                 if (xs_bytes + part_bytes + 1024 + 2 * stage_bytes * kwv > budget) continue;
                 int stages = (int)((budget - xs_bytes - part_bytes - 1024) / stage_bytes);
                 if (stages > kTmaMaxStages) stages = kTmaMaxStages;
+                // a slot that is used again belongs to the warps of one K-slice: only who has waited for its last use knows that it landed
+                if (stages < chunks) stages -= stages % kwv;
                 if (stages > chunks) stages = chunks;
                 if (stages < 2 * kwv && stages < chunks) continue;
                 // Cost model fitted to a sweep over the Llama / Phi shapes (zero regret on it): a warp needs

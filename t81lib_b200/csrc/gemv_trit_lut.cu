@@ -920,6 +920,9 @@ bool lay_out(Plan &pl, int fmt, int planes, int ntok, int tokpad, int rwv, int k
     int stages1 = (int)(((size_t)budget - off) / stage_bytes);
     int stages = stages0 + stages1;
     if (stages > kMaxStages) stages = kMaxStages;
+    // A slot that is used again belongs to the warps of one K-slice: a wait that tells phases by parity passes at once if the slot's last
+    // use has not landed yet, and only who has waited for that use knows that it has.
+    if (stages < chunks) stages -= stages % kwv;
     if (stages > chunks) stages = chunks;
     if (stages < 2 * kwv && stages < chunks) return false;
     if (stages0 > stages) stages0 = stages;
