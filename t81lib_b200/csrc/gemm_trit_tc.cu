@@ -6,8 +6,8 @@
 // its shared memory and loads half of the tile's activation rows by TMA; the even CTA issues the MMAs, which read both
 // halves, and each CTA keeps its 128 accumulator rows in TMEM (2 x 256 fp32 columns, double-buffered across tiles).
 // Measured against the one-CTA 128 x 256 kernel before it (bf16, weights in limbs there and in codes here):
-// 4096 x 14336 x 16384 tokens 1700 -> 1160 us (958 -> 1391 TFLOP/s in a long run under the power cap), 9216 x 3072 x 2048
-// 109 -> 90, 14336 x 4096 x 80 40.9 -> 20.6 us.
+// 4096 x 14336 x 16384 tokens 958 -> 1529 TFLOP/s in a long run under the power cap, 9216 x 3072 x 2048 109 -> 83 us, 14336 x 4096 x 80
+// 40.9 -> 19.2 us.
 // What bounds the kernel is shared-memory bandwidth: a 64-deep step writes and reads 16 KB of expanded weights per CTA
 // and writes and reads the activations, against 512 clocks of MMA at 256 tokens.  Halving the activation share is what
 // the pair is for: a single CTA with a 128 x 256 tile needs 768 clocks of shared memory per 512 of MMA.
@@ -21,7 +21,7 @@
 // 192 columns are four limbs and three 64-column operand atoms: the unit in which converters hand weights to the MMAs.
 //
 // Activations: 16-bit types as they are (A and B of one MMA have the same type), fp32 as bf16 planes (x = hi + lo, 16
-// mantissa bits) that are multiplied one after the other with the same expanded weights.  Rows TMA cannot read
+// mantissa bits) that are multiplied with the same expanded weights, side by side or in turn (Mode).  Rows TMA cannot read
 // (unaligned, the (K, N) layout, fp32) are first copied into token-major planes in the caller's workspace.
 // All planes but the first have an accumulator of their own beside it, and the epilogue adds the two.  The tensor core cuts an
 // accumulator off at every 16 columns instead of rounding it.  With the first plane alone little is cut (trits times 8-bit
@@ -74,7 +74,6 @@ constexpr int OUT_STAGE_BYTES = OUT_TOKENS * BM * 2;  // [token][feature] block 
 constexpr int BARRIER_BYTES = 512;
 constexpr int SMEM_LIMIT = 227 * 1024;
 template <int FMT> constexpr int kRawBytes = FMT == 1 ? 4 * 1536 : BM * 64;
-constexpr int SMEM_FIXED = 2 * OUT_STAGE_BYTES + BARRIER_BYTES + 1024 /*alignment*/;  // and the packed weights
 
 enum { STATUS_OK = 0, STATUS_TIMEOUT_PRODUCER = 1, STATUS_TIMEOUT_MMA = 2, STATUS_TIMEOUT_EPILOGUE = 3, STATUS_TIMEOUT_CONVERTER = 4 };
 
@@ -91,11 +90,13 @@ struct TcParams {
     int bn;                  // tokens per tile: a multiple of 32
     int n_atoms, n_chunks;
     int planes, plane_rows;  // activation planes and their row distance in the tensor map
+    int b_rows;              // rows of activations that a CTA loads per atom
     int splits;              // pairs of a cluster that share a tile's contraction
     int a_stages, b_stages;
+    int out_bytes;           // of staged output blocks beside the rings: two, or none
     int b_step;              // atoms behind one barrier of the activation ring: 1, or 3 (a whole chunk)
     int one_tile;            // no cluster has more than one tile: all warps but the first two finish it
-    uint32_t idesc;
+    uint32_t idesc, idesc_rest;  // of the first product, and of the third plane's beside two in one
     uint32_t one_mask;       // FMT 0: bits of bf16 +-1 that stay (all for bf16, 0xBC00 per half for fp16)
     float alpha, beta;
     int n_out_maps;      // > 0: the epilogue stages output blocks in shared memory and stores them by TMA through
@@ -227,15 +228,25 @@ __device__ __forceinline__ void emit_block(const TcParams &p, const TcOutMaps &o
     }
 }
 
-// 32 columns of a tile's sums.
-template <int SMALL>
-__device__ __forceinline__ void load_sums(uint32_t taddr, uint32_t (&v)[32]) {
+// How the activation planes of a tile meet its weights.
+//   ONE    one plane.
+//   SIDE   up to 96 tokens: the first two planes side by side are the columns of one product, each CTA loads one of them, and the sums
+//          of the second come out beside those of the first; a third plane is a product of its own that adds to the second's.  The
+//          weights are read once for both planes, which is what bounds narrow products.
+//   APART  128 tokens: a product per plane, the sums 128 columns apart.
+//   WIDE   192 to 256, where no pair has a second tile: the same, 256 columns apart.
+enum Mode { ONE, SIDE, APART, WIDE };
+
+// 32 columns of a tile's sums; all planes but the first have theirs `rest` columns further.
+template <Mode MODE>
+__device__ __forceinline__ void load_sums(const TcParams &p, uint32_t taddr, uint32_t (&v)[32]) {
     tmem_ld32(taddr, v);
-    if constexpr (SMALL > 0) {
+    if constexpr (MODE != ONE) {
+        const uint32_t rest = MODE == SIDE ? (uint32_t)p.bn : (MODE == APART ? 128u : 256u);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {  // eight at a time: a whole block beside v costs the kernel spills
             uint32_t small[8];
-            tmem_ld8(taddr + (uint32_t)(SMALL + 8 * q), small);
+            tmem_ld8(taddr + rest + (uint32_t)(8 * q), small);
 #pragma unroll
             for (int i = 0; i < 8; ++i) v[8 * q + i] = __float_as_uint(__uint_as_float(v[8 * q + i]) + __uint_as_float(small[i]));
         }
@@ -304,20 +315,19 @@ __device__ __forceinline__ void expand_chunk(const RawChunk<FMT> &raw, uint8_t *
     }
 }
 
-// SMALL: 0, or with two or three activation planes the columns from a tile's accumulator to the one of all planes but the first.
 // ROWS: see emit_block.
-template <typename CT, int FMT, int SMALL, bool ROWS>
+template <typename CT, int FMT, Mode MODE, bool ROWS>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_trit_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ TcOutMaps omaps, const __grid_constant__ TcParams p) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t *gen_base = smem_raw + (base - smem_u32(smem_raw));
-    const uint32_t b_atom_bytes = (uint32_t)p.bn * (BK * 2 / 2);  // this CTA's half of the tokens
+    const uint32_t b_atom_bytes = MODE == SIDE ? (uint32_t)p.b_rows * (BK * 2) : (uint32_t)p.bn * (BK * 2 / 2);  // this CTA's half of the tokens
     const uint32_t b_stage_bytes = b_atom_bytes * (uint32_t)p.b_step;
     const uint32_t b_off = (uint32_t)p.a_stages * A_CHUNK_BYTES;
     const uint32_t raw_off = b_off + (uint32_t)p.b_stages * b_stage_bytes;
     const uint32_t out_off = raw_off + RAW_STAGES * kRawBytes<FMT>;
-    const uint32_t bars = base + out_off + 2 * OUT_STAGE_BYTES;
+    const uint32_t bars = base + out_off + (uint32_t)p.out_bytes;
     auto a_full = [&](int s) { return bars + 8u * s; };
     auto a_empty = [&](int s) { return bars + 8u * (A_MAX + s); };
     auto b_full = [&](int s) { return bars + 8u * (2 * A_MAX + s); };
@@ -400,21 +410,27 @@ gemm_trit_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         Ring b;
         bool ok = fill_ok;
         for (int tile = cluster_id; tile < total_tiles && ok; tile += n_clusters) {
-            const int row = (tile / p.m_tiles) * p.bn + half * (p.bn / 2);
+            const int row = (tile / p.m_tiles) * p.bn + (MODE == SIDE ? half * p.plane_rows : half * (p.bn / 2));
             for (int c = c0; c < c1 && ok; ++c) {
                 load_raw();
                 ok = fill_ok;
                 const int a_end = 3 * c + 3 < p.n_atoms ? 3 * c + 3 : p.n_atoms;
                 for (int a0 = 3 * c; a0 < a_end && ok; a0 += p.b_step) {
                     const int a1 = a0 + p.b_step < a_end ? a0 + p.b_step : a_end;
-                    for (int pl = 0; pl < p.planes; ++pl) {
+                    for (int pl = 0; pl < (MODE == APART || MODE == WIDE ? p.planes : 1); ++pl) {
                         ok = mbar_wait(b_empty(b.stage), b.phase ^ 1);
                         if (!ok) break;
                         if (elect_one()) {
                             if (half == 0) mbar_arrive_expect_tx(b_full(b.stage), 2 * (uint32_t)(a1 - a0) * b_atom_bytes);
                             uint32_t dst = base + b_off + (uint32_t)b.stage * b_stage_bytes;
-                            for (int a = a0; a < a1; ++a, dst += b_atom_bytes)
+                            for (int a = a0; a < a1; ++a, dst += b_atom_bytes) {
                                 tma_load_2d_pair(dst, &map_x, a * BK, pl * p.plane_rows + row, b_full(b.stage));
+                                if (MODE == SIDE && p.planes == 3) {  // boxes of half a tile: the rest of this CTA's plane, and half of the third
+                                    const uint32_t half_bytes = (uint32_t)p.bn * (BK * 2 / 2);
+                                    tma_load_2d_pair(dst + half_bytes, &map_x, a * BK, row + p.bn / 2, b_full(b.stage));
+                                    tma_load_2d_pair(dst + 2 * half_bytes, &map_x, a * BK, 2 * p.plane_rows + (tile / p.m_tiles) * p.bn + half * (p.bn / 2), b_full(b.stage));
+                                }
+                            }
                         }
                         __syncwarp();
                         b.advance(p.b_stages);
@@ -449,12 +465,12 @@ gemm_trit_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                     const uint32_t a_base = base + (uint32_t)a.stage * A_CHUNK_BYTES;
                     for (int j0 = 0; j0 < atoms && ok; j0 += p.b_step) {
                         const int j1 = j0 + p.b_step < atoms ? j0 + p.b_step : atoms;
-                        for (int pl = 0; pl < p.planes; ++pl) {
+                        for (int pl = 0; pl < (MODE == APART || MODE == WIDE ? p.planes : 1); ++pl) {
                             ok = mbar_wait(b_full(b.stage), b.phase);
                             if (!ok) break;
                             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                            const uint32_t d_tmem = d_tile + (pl > 0 ? (uint32_t)SMALL : 0u);
-                            const uint32_t accumulate = c > c0 || j0 > 0 || pl > (SMALL > 0 ? 1 : 0) ? 1u : 0u;
+                            const uint32_t d_tmem = d_tile + (pl > 0 ? (MODE == APART ? 128u : 256u) : 0u);
+                            const uint32_t accumulate = c > c0 || j0 > 0 || pl > 1 ? 1u : 0u;
                             if (elect_one()) {
                                 uint64_t bd = umma_desc_k(base + b_off + (uint32_t)b.stage * b_stage_bytes);
                                 uint64_t ad = umma_desc_k(a_base + (uint32_t)j0 * A_ATOM_BYTES);
@@ -462,6 +478,15 @@ gemm_trit_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 #pragma unroll
                                     for (int k = 0; k < BK / 16; ++k)
                                         umma_pair(d_tmem, ad + (uint64_t)(2 * k), bd + (uint64_t)(2 * k), p.idesc, k == 0 && j == j0 ? accumulate : 1u);
+                                }
+                                if (MODE == SIDE && p.planes == 3) {
+                                    bd = umma_desc_k(base + b_off + (uint32_t)b.stage * b_stage_bytes + (uint32_t)p.bn * (BK * 2));
+                                    ad = umma_desc_k(a_base + (uint32_t)j0 * A_ATOM_BYTES);
+                                    for (int j = j0; j < j1; ++j, ad += A_ATOM_BYTES >> 4, bd += b_atom_bytes >> 4) {
+#pragma unroll
+                                        for (int k = 0; k < BK / 16; ++k)
+                                            umma_pair(d_tile + (uint32_t)p.bn, ad + (uint64_t)(2 * k), bd + (uint64_t)(2 * k), p.idesc_rest, 1u);
+                                    }
                                 }
                                 umma_commit_pair(b_empty(b.stage), pair_mask);
                             }
@@ -498,7 +523,7 @@ gemm_trit_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 #pragma unroll 1
             for (int c = 0; c < p.bn / 32; ++c) {
                 uint32_t v[32];
-                load_sums<SMALL>(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * 256 + c * 32), v);
+                load_sums<MODE>(p, tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * 256 + c * 32), v);
                 const uint32_t stage = out_off + (uint32_t)(out_count++ & 1) * OUT_STAGE_BYTES;
                 emit_block<CT, ROWS>(p, omaps, v, row0, row, scale, bias, n0 + c * 32,
                                OutStage{gen_base + stage, base + stage, 2, threadIdx.x == EPILOGUE_WARP0 * 32, true});
@@ -562,7 +587,7 @@ gemm_trit_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                     const int to = b % S;
                     if (to == slice) continue;
                     uint32_t v[32];
-                    load_sums<SMALL>(t_lane + (uint32_t)(b * 32), v);
+                    load_sums<MODE>(p, t_lane + (uint32_t)(b * 32), v);
                     push_partial(v, base + partial_slot(b, S, slice, to) * 16384u + lane_row * 4u, (uint32_t)(2 * to + half));
                 }
             __syncthreads();
@@ -572,7 +597,7 @@ gemm_trit_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             const bool first = quarter == 2 && lane == 0;
             for (int b = slice + S * group; b < blocks; b += 3 * S) {
                 uint32_t v[32];
-                load_sums<SMALL>(t_lane + (uint32_t)(b * 32), v);
+                load_sums<MODE>(p, t_lane + (uint32_t)(b * 32), v);
                 if (S > 1) fold_partials(v, gen_base, b, S, slice, lane_row);
                 const uint32_t stage = b_off + (uint32_t)b * OUT_STAGE_BYTES;
                 emit_block<CT, ROWS>(p, omaps, v, row0, own_row, own_scale, own_bias, n0 + b * 32, OutStage{gen_base + stage, base + stage, (uint32_t)(2 + group), first, false});
@@ -594,21 +619,34 @@ gemm_trit_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 
 // Everything a launch needs to know about the sizes.
 struct TcShape {
-    int bn = 0, n_tiles = 0, splits = 1, a_stages = 2, b_stages = 2, b_step = 1;
+    Mode mode = ONE;
+    int bn = 0, n_tiles = 0, splits = 1, a_stages = 2, b_stages = 2, b_step = 1, b_rows = 0, out_bytes = 0;
     size_t smem = 0;
     double cost = 0.0;  // pick_shape's estimate, in units of 1.7 ns
 };
 
-// Time of a 64-deep step of one activation plane at tile width bn, in units of 1.7 ns (measured with 32 to 224 steps a tile):
-// its tokens, and no less than 104 of them whatever the width (reading 256 rows of weights bounds it); from 160 tokens on the
-// time grows slowly, since the issuing warps' own path between two barriers is a large part of it (290, 303 and 362 ns at 192,
-// 224 and 256 tokens with a barrier per chunk up to 224; 310, 320 and 370 ns with one per step, as several planes have it).
-double step_cost(int bn, int planes) {
-    if (bn <= 128) return bn > 104 ? bn : 104;
-    if (bn > 224) return 213;
-    return planes == 1 ? 178 - 0.25 * (224 - bn) : 188 - 0.2 * (224 - bn);
+// Time of a 64-deep step of one product at width n, in units of 1.7 ns (measured with 32 to 224 steps a tile): its columns, and no less
+// than 104 of them whatever the width (reading 256 rows of weights bounds it); from 160 on the time grows slowly, since the issuing
+// warps' own path between two barriers is a large part of it (290, 303 and 362 ns at 192, 224 and 256 columns with a barrier per chunk
+// up to 224; 310, 320 and 370 ns with one per step, as products of planes apart have it).
+double product_cost(int n, bool apart) {
+    if (n <= 128) return n > 104 ? n : 104;
+    if (n > 224) return 213;
+    return apart ? 188 - 0.2 * (224 - n) : 178 - 0.25 * (224 - n);
+}
+Mode mode_of(int bn, int planes) { return planes == 1 ? ONE : (bn <= 96 ? SIDE : (bn <= 128 ? APART : WIDE)); }
+// The same of a step of all planes.  Products of 128 tokens apart take turns without a gap, 184 ns each; side by side, at 256
+// columns, they took 420 ns a step, since two stages are all that fits (1500 tokens of 9000 by 1200, fp32: 75 and 82 us).
+double step_cost(Mode mode, int bn, int planes) {
+    if (mode == ONE) return product_cost(bn, false);
+    if (mode == APART) return planes * 108.0;
+    if (mode == WIDE) return planes * product_cost(bn, true);
+    return product_cost(2 * bn, false) + (planes == 3 ? product_cost(bn, false) : 0.0);
 }
 
+// Planes side by side against apart, at the width that each form is best at (us, fp32): 777 tokens of 3001 by 1999 26.9 -> 22.8, 300
+// of 1000 by 9000 21.5 -> 17.0, 64 of 4096 by 14336 25.7 -> 21.8, 17 of 4096 by 4096 15.1 -> 13.9.
+//
 // Tile width and split: the smallest estimate, in step_cost's units.  Fitted to every width and split of 50 shapes from
 // 512 x 528 x 256 to 14336 x 4096 x 4096: the steps; a tile 400 more; writing the last tiles out, 3 a token; sharing partial
 // sums 1300 and 3 a token.  Several planes take two accumulators a tile, so tiles that follow one another in a pair are at most
@@ -616,7 +654,7 @@ double step_cost(int bn, int planes) {
 // no pair has a second tile (5530 x 11021 x 249: 83 us at 128 tokens, 66 at 256).  The width 160 is left out for several planes:
 // a launch at it (728 tiles, two planes, fp32 result) failed with an unspecified error on a variant of this kernel that had other
 // issuing loops, and the cause is not known.
-TcShape pick_shape(int64_t M, int64_t N, int64_t K, int planes, int raw_bytes) {
+TcShape pick_shape(int64_t M, int64_t N, int64_t K, int planes, int raw_bytes, bool staged) {
     const int64_t m_tiles = (M + 255) / 256, chunks = (K + CHUNK - 1) / CHUNK, wide = (N + 255) / 256, narrow = (N + 127) / 128;
     const int64_t least = planes > 1 && wide > resident_pair_clusters(1) ? narrow : wide, most = (planes > 1 ? narrow : wide) + 8;
     TcShape best;
@@ -628,28 +666,36 @@ TcShape pick_shape(int64_t M, int64_t N, int64_t K, int planes, int raw_bytes) {
             const int resident = resident_pair_clusters(s);
             if (s > chunks || (s > 1 && tiles > resident)) continue;
             if (planes > 1 && bn > 128 && (bn < 192 || tiles > resident)) continue;
-            const double atom = planes * step_cost(bn, planes);
+            const double atom = step_cost(mode_of(bn, planes), bn, planes);
             const double t = (double)((tiles + resident - 1) / resident) * (3.0 * (double)((chunks + s - 1) / s) * atom + 400.0) +
                              3.0 * bn + (s > 1 ? 1300.0 + 3.0 * bn : 0.0);
             if (t < best_t) { best_t = t; best.bn = bn; best.n_tiles = (int)n_tiles; best.splits = s; }
         }
     }
     best.cost = best_t;
-    // One barrier per chunk instead of one per step where two stages of a chunk fit (up to 224 tokens) and the planes are not
-    // several (those fill the time between two barriers anyway, and do better with a deeper ring: 200 against 220 us at
-    // 4096 x 4096 x 4096, fp32, 192 tokens).  With one plane: 192 tokens 408 -> 314 us at 14336 x 4096 x 4096.
-    best.a_stages = best.bn <= 96 ? 3 : 2;
-    const int fixed = SMEM_FIXED + RAW_STAGES * raw_bytes, room = SMEM_LIMIT - fixed - best.a_stages * A_CHUNK_BYTES;
-    best.b_step = (best.bn <= 128 || (planes == 1 && best.bn <= 224)) && room >= 6 * best.bn * BK ? 3 : 1;
-    const int stage = best.bn * BK * best.b_step, b = room / stage;
+    const bool alone = best.splits > 1 || m_tiles * best.n_tiles <= resident_pair_clusters(1);
+    best.mode = mode_of(best.bn, planes);
+    const int columns = best.mode == SIDE ? 2 * best.bn : best.bn;
+    best.b_rows = (columns + (best.mode == SIDE && planes == 3 ? best.bn : 0)) / 2;
+    best.a_stages = columns <= 96 ? 3 : 2;
+    const int atom = best.b_rows * BK * 2;
+    // Output blocks are staged beside the rings only where tiles follow one another and TMA writes them; what is left goes to the
+    // activation ring (4096 tokens of 4096 by 4096, fp32: 191 -> 183 us with a fourth stage, 500 in bf16 20.6 -> 19.4).
+    best.out_bytes = staged && !alone ? 2 * OUT_STAGE_BYTES : 0;
+    const int fixed = RAW_STAGES * raw_bytes + best.out_bytes + BARRIER_BYTES + 1024, room = SMEM_LIMIT - fixed - best.a_stages * A_CHUNK_BYTES;
+    // One barrier per chunk instead of one per step where two stages of a chunk fit (up to 224 columns) and the planes do not fill the time
+    // between two barriers anyway (wide ones do better with a deeper ring: 200 against 220 us at 4096 x 4096 x 4096, fp32, 192
+    // tokens).  With one plane: 192 tokens 408 -> 314 us at 14336 x 4096 x 4096; 256 columns in two stages 76 -> 81 at 9216 x 3072 x 2048.
+    best.b_step = best.mode != WIDE && best.bn <= 224 && room >= 6 * atom ? 3 : 1;
+    const int stage = atom * best.b_step, b = room / stage;
     best.b_stages = b > B_MAX ? B_MAX : b;
     best.smem = (size_t)best.a_stages * A_CHUNK_BYTES + (size_t)best.b_stages * stage + fixed;
     return best;
 }
 
-template <typename CT, int FMT, int SMALL, bool ROWS>
+template <typename CT, int FMT, Mode MODE, bool ROWS>
 int launch_tc(const TcShape &shape, const CUtensorMap &mw, const CUtensorMap &mx, const TcOutMaps &om, const TcParams &p, cudaStream_t st) {
-    auto kern = gemm_trit_tc_kernel<CT, FMT, SMALL, ROWS>;
+    auto kern = gemm_trit_tc_kernel<CT, FMT, MODE, ROWS>;
     // the shared-memory limit is a per-device attribute of the function: set it once on every device
     static std::atomic<bool> configured[64];
     int dev = 0;
@@ -678,12 +724,12 @@ int launch_tc(const TcShape &shape, const CUtensorMap &mw, const CUtensorMap &mx
     return T81B200_OK;
 }
 
-template <int FMT, int SMALL>
+template <int FMT, Mode MODE>
 int launch_tc_ct(int c_dtype, bool rows, const TcShape &shape, const CUtensorMap &mw, const CUtensorMap &mx, const TcOutMaps &om, const TcParams &p, cudaStream_t st) {
     switch (c_dtype) {
-        case T81B200_F32: return launch_tc<float, FMT, SMALL, false>(shape, mw, mx, om, p, st);
-        case T81B200_BF16: return rows ? launch_tc<__nv_bfloat16, FMT, SMALL, true>(shape, mw, mx, om, p, st) : launch_tc<__nv_bfloat16, FMT, SMALL, false>(shape, mw, mx, om, p, st);
-        case T81B200_F16: return rows ? launch_tc<__half, FMT, SMALL, true>(shape, mw, mx, om, p, st) : launch_tc<__half, FMT, SMALL, false>(shape, mw, mx, om, p, st);
+        case T81B200_F32: return launch_tc<float, FMT, MODE, false>(shape, mw, mx, om, p, st);
+        case T81B200_BF16: return rows ? launch_tc<__nv_bfloat16, FMT, MODE, true>(shape, mw, mx, om, p, st) : launch_tc<__nv_bfloat16, FMT, MODE, false>(shape, mw, mx, om, p, st);
+        case T81B200_F16: return rows ? launch_tc<__half, FMT, MODE, true>(shape, mw, mx, om, p, st) : launch_tc<__half, FMT, MODE, false>(shape, mw, mx, om, p, st);
     }
     return fail(T81B200_EINVAL, "gemm_trit: unknown output dtype %d", c_dtype);
 }
@@ -844,7 +890,7 @@ int resident_pair_clusters(int splits) {
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return sm_count() / (2 * splits + 1);
     int n = known[dev][splits].load(std::memory_order_relaxed);
     if (n > 0) return n;
-    auto kern = gemm_trit_tc_kernel<__nv_bfloat16, 1, 0, false>;
+    auto kern = gemm_trit_tc_kernel<__nv_bfloat16, 1, ONE, false>;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(2 * splits), 1, 1);
     cfg.blockDim = dim3(NUM_THREADS, 1, 1);
@@ -877,7 +923,7 @@ bool gemm_trit_tc_eligible(int64_t M, int64_t N, int64_t K) {
 
 // Time of a launch without staging: 6 us of launch, set-up and last stores on top of the planner's figure (13.5 us estimated and 12.4
 // measured at 4096 x 4096 x 32, 18.8 and 20.3 at 14336 x 4096 x 80, both bf16).
-double gemm_trit_tc_estimate_us(int64_t M, int64_t N, int64_t K) { return 6.0 + 1.7e-3 * pick_shape(M, N, K, 1, kRawBytes<1>).cost; }
+double gemm_trit_tc_estimate_us(int64_t M, int64_t N, int64_t K) { return 6.0 + 1.7e-3 * pick_shape(M, N, K, 1, kRawBytes<1>, true).cost; }
 
 // Scratch bytes for the activations: none when they are read in place.  `planes`: bf16 planes of fp32 activations.
 size_t gemm_trit_tc_scratch_most(int b_dtype, int64_t N, int64_t K, int planes) {
@@ -914,7 +960,12 @@ int gemm_trit_tc_launch(int fmt, int fp32_planes, const uint8_t *A, const float 
         if (int rc = stage_planes(B, b_dtype, layout, ldb, N, K, planes, workspace, st)) return rc;
         x_ptr = workspace; x_ld = scratch_row(K);
     }
-    const TcShape shape = pick_shape(M, N, K, planes, fmt == 1 ? kRawBytes<1> : kRawBytes<0>);
+    // TMA-store epilogue: 16-bit output, token-major C (features contiguous), no read-modify-write, and every
+    // result 16-byte aligned with a 16-byte multiple as its row pitch
+    bool tma_out = dtype_size(c_dtype) == 2 && layout == T81B200_LAYOUT_NK && beta == 0.0f && (ldc * 2) % 16 == 0 &&
+                   reinterpret_cast<uintptr_t>(C) % 16 == 0;
+    for (int i = 0; i < n_peers; ++i) tma_out = tma_out && reinterpret_cast<uintptr_t>(peer_C[i]) % 16 == 0;
+    const TcShape shape = pick_shape(M, N, K, planes, fmt == 1 ? kRawBytes<1> : kRawBytes<0>, tma_out);
     const bool f16 = b_dtype == T81B200_F16;
     CUtensorMap mw, mx;
     memset(&mw, 0, sizeof mw);
@@ -925,7 +976,7 @@ int gemm_trit_tc_launch(int fmt, int fp32_planes, const uint8_t *A, const float 
             return rc;
     }
     if (int rc = make_map_2d(&mx, f16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, x_ptr, (uint64_t)K,
-                             (uint64_t)x_rows, (uint64_t)x_ld * 2, BK, (uint32_t)shape.bn / 2, CU_TENSOR_MAP_SWIZZLE_128B))
+                             (uint64_t)x_rows, (uint64_t)x_ld * 2, BK, (uint32_t)(shape.mode == SIDE && planes == 2 ? shape.bn : shape.bn / 2), CU_TENSOR_MAP_SWIZZLE_128B))
         return rc;
     TcParams p;
     memset(&p, 0, sizeof p);
@@ -938,11 +989,12 @@ int gemm_trit_tc_launch(int fmt, int fp32_planes, const uint8_t *A, const float 
     p.bn = shape.bn;
     p.n_atoms = (int)((K + BK - 1) / BK);
     p.n_chunks = (int)((K + CHUNK - 1) / CHUNK);
-    p.planes = planes; p.plane_rows = (int)N;
+    p.planes = planes; p.plane_rows = (int)N; p.b_rows = shape.b_rows; p.out_bytes = shape.out_bytes;
     p.splits = shape.splits;
     p.a_stages = shape.a_stages; p.b_stages = shape.b_stages; p.b_step = shape.b_step;
     p.one_tile = shape.splits > 1 || p.m_tiles * p.n_tiles <= resident_pair_clusters(1) ? 1 : 0;
-    p.idesc = umma_instr_desc(shape.bn, f16);
+    p.idesc = umma_instr_desc(shape.mode == SIDE ? 2 * shape.bn : shape.bn, f16);
+    p.idesc_rest = umma_instr_desc(shape.bn, f16);
     p.one_mask = f16 ? 0xBC00BC00u : 0xFFFFFFFFu;
     p.alpha = fmt == 1 ? 0.5f * alpha : alpha;
     p.beta = beta;
@@ -950,13 +1002,8 @@ int gemm_trit_tc_launch(int fmt, int fp32_planes, const uint8_t *A, const float 
     for (int i = 0; i < n_peers; ++i) p.peer_C[i] = peer_C[i];
     p.c_vec = layout == T81B200_LAYOUT_KN && n_peers == 0 && reinterpret_cast<uintptr_t>(C) % 16 == 0 &&
                       (ldc * (int64_t)dtype_size(c_dtype)) % 16 == 0 ? 1 : 0;
-    // TMA-store epilogue: 16-bit output, token-major C (features contiguous), no read-modify-write, and every
-    // result 16-byte aligned with a 16-byte multiple as its row pitch
     TcOutMaps om;
     memset(&om, 0, sizeof om);
-    bool tma_out = dtype_size(c_dtype) == 2 && layout == T81B200_LAYOUT_NK && beta == 0.0f && (ldc * 2) % 16 == 0 &&
-                   reinterpret_cast<uintptr_t>(C) % 16 == 0;
-    for (int i = 0; i < n_peers; ++i) tma_out = tma_out && reinterpret_cast<uintptr_t>(peer_C[i]) % 16 == 0;
     if (tma_out) {
         const CUtensorMapDataType dt = c_dtype == T81B200_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
         for (int i = 0; i <= n_peers; ++i) {
@@ -968,12 +1015,16 @@ int gemm_trit_tc_launch(int fmt, int fp32_planes, const uint8_t *A, const float 
         p.n_out_maps = 1 + n_peers;
     }
     const bool rows = !tma_out && dtype_size(c_dtype) == 2 && layout == T81B200_LAYOUT_NK && beta == 0.0f && n_peers == 0;
-    auto launch = [&](auto small) {
-        constexpr int S = decltype(small)::value;
-        return fmt == 1 ? launch_tc_ct<1, S>(c_dtype, rows, shape, mw, mx, om, p, st) : launch_tc_ct<0, S>(c_dtype, rows, shape, mw, mx, om, p, st);
+    auto launch = [&](auto mode) {
+        constexpr Mode MODE = decltype(mode)::value;
+        return fmt == 1 ? launch_tc_ct<1, MODE>(c_dtype, rows, shape, mw, mx, om, p, st) : launch_tc_ct<0, MODE>(c_dtype, rows, shape, mw, mx, om, p, st);
     };
-    if (planes == 1) return launch(std::integral_constant<int, 0>{});
-    return shape.bn <= 128 ? launch(std::integral_constant<int, 128>{}) : launch(std::integral_constant<int, 256>{});
+    switch (shape.mode) {
+        case SIDE: return launch(std::integral_constant<Mode, SIDE>{});
+        case APART: return launch(std::integral_constant<Mode, APART>{});
+        case WIDE: return launch(std::integral_constant<Mode, WIDE>{});
+        default: return launch(std::integral_constant<Mode, ONE>{});
+    }
 }
 
 }  // namespace t81b200

@@ -222,8 +222,8 @@ def test_rows_off_boundaries_have_their_own_kernel(dev, out_f, dtype, out_dtype,
     assert torch.equal(got[0], (x.double() @ trits.double().t()).to(out_dtype or dtype))
 
 
-# The planes of float32 activations in tiles of up to 128 tokens and of 192 to 256 (tiles alone): tokens at the edges of the widths, one
-# tile, tiles that follow one another and a contraction split over a cluster.
+# The planes of float32 activations side by side in one product (up to 96 tokens a tile), apart (128) and wide (192 to 256, tiles alone):
+# tokens at the edges of the widths, one tile, tiles that follow one another and a contraction split over a cluster.
 @pytest.mark.parametrize("planes", [2, 3])
 @pytest.mark.parametrize("out_f,in_f,tokens", [(300, 700, 17), (256, 4000, 32), (300, 4000, 33), (260, 4000, 64), (5000, 3000, 65), (20000, 200, 96), (20000, 200, 97), (300, 9000, 128),
                                                (2600, 1000, 513), (20000, 193, 129), (5530, 6000, 249), (20000, 500, 250), (700, 130, 6000)])
@@ -244,16 +244,18 @@ def test_planes_of_float32_by_width(dev, out_f, in_f, tokens, planes):
     assert _capi.kernel_status(reset=True) == 0
 
 
-# Every form in which planes meet: accumulators 128 or 256 columns apart, tiles alone, one after the other and split over a cluster.  The
-# form is read from what was launched, so that other step costs cannot drop one unseen.
-TC_PARAM_WIDTH, TC_PARAM_SPLITS, TC_PARAM_M_TILES, TC_PARAM_N_TILES = 21, 26, 19, 20  # TcParams in 32-bit words
+# Every form in which planes meet (Mode): side by side in one product, apart and wide, of tiles alone, one after the other and split over a
+# cluster.  The form is read from what was launched, so that other step costs cannot drop one unseen.
+TC_PARAM_WIDTH, TC_PARAM_SPLITS, TC_PARAM_M_TILES, TC_PARAM_N_TILES = 21, 27, 19, 20  # TcParams in 32-bit words
+SIDE, APART, WIDE = 1, 2, 3
 
 
 @pytest.mark.parametrize("planes", [2, 3])
-@pytest.mark.parametrize("out_f,in_f,tokens,apart,split,alone", [
-    (10152, 11900, 114, 128, False, True), (7391, 13254, 101, 128, True, True), (6000, 3000, 120, 128, True, True), (20000, 200, 97, 128, False, False),
-    (700, 130, 6000, 256, False, True), (2807, 9347, 475, 256, True, True)])
-def test_planes_of_float32_in_every_form(dev, out_f, in_f, tokens, apart, split, alone, planes):
+@pytest.mark.parametrize("out_f,in_f,tokens,mode,split,alone", [
+    (2600, 1000, 513, SIDE, False, True), (5000, 3000, 65, SIDE, True, True), (20000, 200, 96, SIDE, False, False),
+    (10152, 11900, 114, APART, False, True), (7391, 13254, 101, APART, True, True), (20000, 500, 250, APART, False, False),
+    (700, 130, 6000, WIDE, False, True), (2807, 9347, 475, WIDE, True, True)])
+def test_planes_of_float32_in_every_form(dev, out_f, in_f, tokens, mode, split, alone, planes):
     from t81lib_b200 import _capi, ops
     gen = torch.Generator(device="cuda").manual_seed(out_f + tokens)
     trits = torch.randint(-1, 2, (out_f, in_f), generator=gen, device="cuda").float()
@@ -264,9 +266,9 @@ def test_planes_of_float32_in_every_form(dev, out_f, in_f, tokens, apart, split,
     graph = capture(lambda: got.append(ops.linear_t2(t2, out_f, x, in_f, None, None, torch.float32, planes)))  # its parameters live as long as it does
     launched = [(name, params(3)) for name, params in kernels(graph) if "gemm_trit_tc_kernel" in name]
     graph.replay()
-    assert len(launched) == 1 and f"Li1ELi{apart}E" in launched[0][0], launched[0][0]
+    assert len(launched) == 1 and f"ModeE{mode}E" in launched[0][0], launched[0][0]
     words = launched[0][1]
-    assert (words[TC_PARAM_SPLITS] > 1) == split and words[TC_PARAM_WIDTH] % 32 == 0 and (words[TC_PARAM_WIDTH] > 128) == (apart == 256)
+    assert (words[TC_PARAM_SPLITS] > 1) == split and words[TC_PARAM_WIDTH] in ((), (32, 64, 96), (128,), (192, 224, 256))[mode]
     assert (split or words[TC_PARAM_M_TILES] * words[TC_PARAM_N_TILES] <= 74) == alone
     want = x.double() @ trits.double().t()
     for y in got:  # the call before the capture, and the captured one
