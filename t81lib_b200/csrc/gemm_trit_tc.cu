@@ -387,7 +387,15 @@ gemm_trit_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         if (++raw_c >= c1) { raw_c = c0; raw_tile += n_clusters; }
     };
 
-    // launched with programmatic stream serialization: everything above overlaps the tail of the previous kernel
+    // launched with programmatic stream serialization: everything above overlaps the tail of the previous kernel.  So do the tensor maps
+    // and, as far as L2 (the kernel ahead may have written them), the first tile's weights.
+    if (warp == 0) {
+        if (lane == 0) {
+            prefetch_map(&map_x);
+            if (FMT == 0) prefetch_map(&map_w);
+            if (p.n_out_maps > 0) prefetch_map(&omaps.m[0]);
+        }
+    }
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (warp == 0) {

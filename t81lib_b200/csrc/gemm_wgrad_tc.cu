@@ -225,6 +225,14 @@ gemm_wgrad_tc_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_con
     }
     __syncwarp();
     if (warp == 1) tmem_alloc_pair(tmem_slot);
+    if (threadIdx.x == 0) {
+        prefetch_map(&map_g);
+        prefetch_map(&map_x);
+        if (VEC) {
+            prefetch_map(&map_w);
+            prefetch_map(&map_out);
+        }
+    }
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");

@@ -57,6 +57,11 @@ __device__ __forceinline__ void bulk_prefetch(const void *src, uint32_t bytes) {
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
 }
 
+// A tensor map on its way to where copies look it up (the first copy through it waits some hundred ns otherwise).
+__device__ __forceinline__ void prefetch_map(const CUtensorMap *map) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
+}
+
 struct Ring {
     int stage = 0;
     uint32_t phase = 0;
