@@ -634,31 +634,29 @@ struct TcShape {
     double cost = 0.0;  // pick_shape's estimate, in units of 1.7 ns
 };
 
-// Time of a 64-deep step of one product at width n, in units of 1.7 ns (measured with 32 to 224 steps a tile): its columns, and no less
-// than 104 of them whatever the width (reading 256 rows of weights bounds it); from 160 on the time grows slowly, since the issuing
-// warps' own path between two barriers is a large part of it (290, 303 and 362 ns at 192, 224 and 256 columns with a barrier per chunk
-// up to 224; 310, 320 and 370 ns with one per step, as products of planes apart have it).
-double product_cost(int n, bool apart) {
-    if (n <= 128) return n > 104 ? n : 104;
-    if (n > 224) return 213;
-    return apart ? 188 - 0.2 * (224 - n) : 178 - 0.25 * (224 - n);
+// Time of a 64-deep step of one product of n columns, in units of 1.7 ns, measured in tiles of 24 to 96 steps, one and three to a pair:
+// up to 160 columns it is the weights' own time, through shared memory and out of it again.
+double product_cost(int n) {
+    constexpr double cost[8] = {115, 119, 122, 125, 130, 153, 169, 187};  // 32, 64, .. 256 columns
+    return cost[n / 32 - 1];
 }
 Mode mode_of(int bn, int planes) { return planes == 1 ? ONE : (bn <= 96 ? SIDE : (bn <= 128 ? APART : WIDE)); }
-// The same of a step of all planes.  Products of 128 tokens apart take turns without a gap, 184 ns each; side by side, at 256
-// columns, they took 420 ns a step, since two stages are all that fits (1500 tokens of 9000 by 1200, fp32: 75 and 82 us).
+// The same of a step of all planes.  Products of 128 tokens apart take turns without a gap; side by side, at 256 columns, they took
+// 420 ns a step, since two stages are all that fits (1500 tokens of 9000 by 1200, fp32: 75 and 82 us).
 double step_cost(Mode mode, int bn, int planes) {
-    if (mode == ONE) return product_cost(bn, false);
-    if (mode == APART) return planes * 108.0;
-    if (mode == WIDE) return planes * product_cost(bn, true);
-    return product_cost(2 * bn, false) + (planes == 3 ? product_cost(bn, false) : 0.0);
+    if (mode == ONE) return product_cost(bn);
+    if (mode == APART) return planes * 98.0;
+    if (mode == WIDE) return planes * product_cost(bn);
+    return product_cost(2 * bn) + (planes == 3 ? product_cost(bn) : 0.0);
 }
 
 // Planes side by side against apart, at the width that each form is best at (us, fp32): 777 tokens of 3001 by 1999 26.9 -> 22.8, 300
 // of 1000 by 9000 21.5 -> 17.0, 64 of 4096 by 14336 25.7 -> 21.8, 17 of 4096 by 4096 15.1 -> 13.9.
 //
 // Tile width and split: the smallest estimate, in step_cost's units.  Fitted to every width and split of 50 shapes from
-// 512 x 528 x 256 to 14336 x 4096 x 4096: the steps; a tile 400 more; writing the last tiles out, 3 a token; sharing partial
-// sums 1300 and 3 a token.  Several planes take two accumulators a tile, so tiles that follow one another in a pair are at most
+// 512 x 528 x 256 to 14336 x 4096 x 4096: the steps; a tile 400 more; writing the last tiles out, 3 a token; sharing partial sums 1300
+// and 3 a token (the steps' costs refitted since: 900 tokens of 3000 by 5000, bf16, 34.3 -> 26.2 us, 400 of 6000 by 3000 25.3 -> 23.4, 200 of 2000
+// by 2000, fp32, 13.7 -> 12.8; 27 others as they were).  Several planes take two accumulators a tile, so tiles that follow one another in a pair are at most
 // 128 tokens wide there (4096 x 4096 x 4096 in two planes 202 us, 208 at 256 tokens with one accumulator); wider ones only where
 // no pair has a second tile (5530 x 11021 x 249: 83 us at 128 tokens, 66 at 256).  The width 160 is left out for several planes:
 // a launch at it (728 tiles, two planes, fp32 result) failed with an unspecified error on a variant of this kernel that had other
@@ -930,9 +928,9 @@ bool gemm_trit_tc_eligible(int64_t M, int64_t N, int64_t K) {
     return M >= 1 && N >= 1 && K >= 1 && M < (1ll << 31) && N < (1ll << 29) && K < (1ll << 31);
 }
 
-// Time of a launch without staging: 6 us of launch, set-up and last stores on top of the planner's figure (13.5 us estimated and 12.4
-// measured at 4096 x 4096 x 32, 18.8 and 20.3 at 14336 x 4096 x 80, both bf16).
-double gemm_trit_tc_estimate_us(int64_t M, int64_t N, int64_t K) { return 6.0 + 1.7e-3 * pick_shape(M, N, K, 1, kRawBytes<1>, true).cost; }
+// Time of a launch without staging: 5.5 us of launch, set-up and last stores on top of the planner's figure (20.4 us estimated and 19.1
+// measured at 14336 x 4096 x 80, 9.9 and 7.8 at 4096 x 1024 x 30, both bf16).
+double gemm_trit_tc_estimate_us(int64_t M, int64_t N, int64_t K) { return 5.5 + 1.7e-3 * pick_shape(M, N, K, 1, kRawBytes<1>, true).cost; }
 
 // Scratch bytes for the activations: none when they are read in place.  `planes`: bf16 planes of fp32 activations.
 size_t gemm_trit_tc_scratch_most(int b_dtype, int64_t N, int64_t K, int planes) {
