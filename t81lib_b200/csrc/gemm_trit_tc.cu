@@ -59,13 +59,14 @@ constexpr int CHUNK = 192;       // columns converted at a time: 3 atoms
 constexpr int A_ATOM_BYTES = BM * BK * 2;        // 16 KB
 constexpr int A_CHUNK_BYTES = 3 * A_ATOM_BYTES;  // 48 KB
 constexpr int A_MAX = 3, B_MAX = 12;             // ring slots that have barriers
-// Packed weights of a chunk (128 rows): 8 KB of limbs, 6 KB of codes.  The two groups of converters take alternate chunks, so an even number of
-// slots leaves each slot to one group.  With three, a group came to a slot whose last use had been the other's, and a wait that
+constexpr int RAW_STAGES = 3;                    // packed weights of a chunk (128 rows): 8 KB of limbs, 6 KB of codes
+// The two groups of converters take alternate chunks, so a slot's uses go from one to the other; the barrier that tells a chunk's arrival is
+// one of its group's own three.  With a barrier per slot a group came to one whose use before had been the other's, and a wait that
 // tells phases by parity passes at once if that use has not even landed: chunk 0's copy later than chunk 1's by the time chunk 1
-// takes to expand (weights whose pages are not in the TLB), and the group went on with whatever lay there and handed the slot back once
-// too often, from where on nothing fits together: waits that run out, wrong sums, a lost context.
-constexpr int RAW_STAGES = 4;
-static_assert(RAW_STAGES % 2 == 0, "a slot belongs to one of the two groups of converters");
+// takes to expand (weights whose pages are not in the TLB).  The group then took whatever lay there and handed the slot back once
+// too often, and nothing fitted together from there on: waits that ran out, wrong sums, a lost context.  (Four slots are as safe, but cost
+// the activation ring a stage: 1463 tokens of 6384 by 3192, bf16, 50.7 and 59.7 us.)
+constexpr int RAW_BARRIERS = 2 * RAW_STAGES;
 constexpr int MAX_SPLITS = 4;                    // clusters of up to 8 CTAs
 constexpr int NUM_THREADS = 14 * 32;
 constexpr int EPILOGUE_WARP0 = 2, CONVERTER_WARP0 = 6;
@@ -335,8 +336,8 @@ gemm_trit_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     auto acc_full = [&](int s) { return bars + 8u * (2 * A_MAX + 2 * B_MAX + s); };
     auto acc_empty = [&](int s) { return bars + 8u * (2 * A_MAX + 2 * B_MAX + 2 + s); };
     auto raw_full = [&](int s) { return bars + 8u * (2 * A_MAX + 2 * B_MAX + 4 + s); };
-    auto raw_empty = [&](int s) { return bars + 8u * (2 * A_MAX + 2 * B_MAX + 4 + RAW_STAGES + s); };
-    const uint32_t tmem_slot = bars + 8u * (2 * A_MAX + 2 * B_MAX + 4 + 2 * RAW_STAGES);
+    auto raw_empty = [&](int s) { return bars + 8u * (2 * A_MAX + 2 * B_MAX + 4 + RAW_BARRIERS + s); };
+    const uint32_t tmem_slot = bars + 8u * (2 * A_MAX + 2 * B_MAX + 4 + RAW_BARRIERS + RAW_STAGES);
 
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const uint32_t rank = cluster_rank();
@@ -346,7 +347,8 @@ gemm_trit_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         for (int s = 0; s < A_MAX; ++s) { mbar_init(a_full(s), 8); mbar_init(a_empty(s), 1); }
         for (int s = 0; s < B_MAX; ++s) { mbar_init(b_full(s), 1); mbar_init(b_empty(s), 1); }
         for (int s = 0; s < 2; ++s) { mbar_init(acc_full(s), 1); mbar_init(acc_empty(s), 8); }
-        for (int s = 0; s < RAW_STAGES; ++s) { mbar_init(raw_full(s), 1); mbar_init(raw_empty(s), 4); }
+        for (int s = 0; s < RAW_BARRIERS; ++s) mbar_init(raw_full(s), 1);
+        for (int s = 0; s < RAW_STAGES; ++s) mbar_init(raw_empty(s), 4);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();  // barriers initialised (this CTA)
@@ -358,7 +360,7 @@ gemm_trit_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 
     // The producer's weight loads run two chunks ahead of the activations; the first ones touch nothing but this CTA's
     // memory and start before the cluster has met.
-    Ring raw_fill;
+    Ring raw_fill, raw_told;
     bool fill_ok = true;
     int raw_tile = cluster_id, raw_c = c0;
     auto load_raw = [&]() {
@@ -366,7 +368,7 @@ gemm_trit_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         fill_ok = mbar_wait(raw_empty(raw_fill.stage), raw_fill.phase ^ 1);
         if (!fill_ok) return;
         const int row0 = ((raw_tile % p.m_tiles) * 2 + half) * BM;
-        const uint32_t dst = base + raw_off + (uint32_t)raw_fill.stage * (uint32_t)kRawBytes<FMT>, bar = raw_full(raw_fill.stage);
+        const uint32_t dst = base + raw_off + (uint32_t)raw_fill.stage * (uint32_t)kRawBytes<FMT>, bar = raw_full(raw_told.stage);
         if (elect_one()) {
             if constexpr (FMT == 1) {
                 // the row tiles of a chunk are contiguous; past the matrix's last one nothing is loaded (those rows
@@ -384,6 +386,7 @@ gemm_trit_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         }
         __syncwarp();
         raw_fill.advance(RAW_STAGES);
+        raw_told.advance(RAW_BARRIERS);
         if (++raw_c >= c1) { raw_c = c0; raw_tile += n_clusters; }
     };
 
@@ -547,7 +550,7 @@ gemm_trit_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         const int rt = (warp - CONVERTER_WARP0) & 3, group = (warp - CONVERTER_WARP0) >> 2;
         const int span = c1 - c0, my_tiles = cluster_id < total_tiles ? (total_tiles - 1 - cluster_id) / n_clusters + 1 : 0;
         Ring a, raw;
-        if (group == 1) { a.advance(p.a_stages); raw.advance(RAW_STAGES); }
+        if (group == 1) { a.advance(p.a_stages); raw.advance(RAW_BARRIERS); }
         bool ok = true;
         // The groups take alternate chunks of the CTA's whole sequence.  Slots of the operand ring change hands where there are three: there a
         // group waits for the MMAs of the slot's last chunk, k - 3.  It has seen those of k - 5 end when it took its own last chunk, and MMAs
@@ -558,9 +561,10 @@ gemm_trit_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             ok = __all_sync(0xffffffffu, mbar_wait(raw_full(raw.stage), raw.phase));
             if (!ok) break;
             RawChunk<FMT> words;
-            read_chunk<FMT>(p, gen_base + raw_off + raw.stage * kRawBytes<FMT>, rt, c, lane, words);
+            const int slot = raw.stage < RAW_STAGES ? raw.stage : raw.stage - RAW_STAGES;
+            read_chunk<FMT>(p, gen_base + raw_off + slot * kRawBytes<FMT>, rt, c, lane, words);
             __syncwarp();
-            if (lane == 0) mbar_arrive(raw_empty(raw.stage));
+            if (lane == 0) mbar_arrive(raw_empty(slot));
             ok = __all_sync(0xffffffffu, mbar_wait(a_empty(a.stage), a.phase ^ 1));
             if (!ok) break;
             expand_chunk<FMT>(words, gen_base + a.stage * A_CHUNK_BYTES + rt * 4096, lane, p.one_mask);
@@ -570,8 +574,8 @@ gemm_trit_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             if (lane == 0) mbar_arrive_leader(a_full(a.stage));
             a.advance(p.a_stages);
             a.advance(p.a_stages);
-            raw.advance(RAW_STAGES);
-            raw.advance(RAW_STAGES);
+            raw.advance(RAW_BARRIERS);
+            raw.advance(RAW_BARRIERS);
             c += 2;
         }
         if (!ok) give_up(&g_tc_status, STATUS_TIMEOUT_CONVERTER);

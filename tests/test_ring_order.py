@@ -10,30 +10,32 @@ import pytest
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "t81lib_b200", "csrc")
 
 
-def read_too_early(slots, groups, chunks, late):
+def read_too_early(slots, groups, chunks, late, barriers=None):
     """The first chunk that a group takes before it has landed, or None.  Group g takes chunks g, g + groups, .., chunk k from slot k % slots,
-    and hands the slot back; chunk k + slots is fetched once chunk k's slot is free."""
-    landed, issued, freed, phases, at = set(), 0, set(), [0] * slots, list(range(groups))
+    whose arrival barrier k % barriers (one per slot by default) tells, and hands the slot back; chunk k + slots is fetched once chunk
+    k's slot is free."""
+    barriers = barriers or slots
+    landed, issued, freed, phases, at = set(), 0, set(), [0] * barriers, list(range(groups))
     while any(k < chunks for k in at):
         moved = False
         while issued < chunks and (issued < slots or issued - slots in freed):
             if issued != late:
                 landed.add(issued)
-                phases[issued % slots] += 1
+                phases[issued % barriers] += 1
             issued += 1
             moved = True
         for g in range(groups):
             k = at[g]
-            if k < chunks and phases[k % slots] & 1 != (k // slots) & 1:  # the barrier's wait for the parity of use k // slots
+            if k < chunks and phases[k % barriers] & 1 != (k // barriers) & 1:  # the barrier's wait for the parity of use k // barriers
                 if k not in landed:
                     return k
                 freed.add(k)
                 at[g] += groups
                 moved = True
         if not moved:
-            assert late is not None and late not in landed, "stuck"
+            assert late not in landed, "stuck"
             landed.add(late)
-            phases[late % slots] += 1
+            phases[late % barriers] += 1
     return None
 
 
@@ -46,7 +48,8 @@ def test_model_finds_slots_that_change_hands():
 def test_packed_weights_of_the_tensor_core_product():
     source = open(os.path.join(CSRC, "gemm_trit_tc.cu")).read()
     slots = int(re.search(r"constexpr int RAW_STAGES = (\d+);", source).group(1))
-    assert all(read_too_early(slots, 2, 24, late) is None for late in range(24))
+    barriers = slots * int(re.search(r"constexpr int RAW_BARRIERS = (\d+) \* RAW_STAGES;", source).group(1))
+    assert all(read_too_early(slots, 2, 24, late, barriers) is None for late in range(24))
 
 
 # GemvLutParams in 32-bit words
