@@ -932,9 +932,12 @@ bool gemm_trit_tc_eligible(int64_t M, int64_t N, int64_t K) {
     return M >= 1 && N >= 1 && K >= 1 && M < (1ll << 31) && N < (1ll << 29) && K < (1ll << 31);
 }
 
-// Time of a launch without staging: 5.5 us of launch, set-up and last stores on top of the planner's figure (20.4 us estimated and 19.1
-// measured at 14336 x 4096 x 80, 9.9 and 7.8 at 4096 x 1024 x 30, both bf16).
-double gemm_trit_tc_estimate_us(int64_t M, int64_t N, int64_t K) { return 5.5 + 1.7e-3 * pick_shape(M, N, K, 1, kRawBytes<1>, true).cost; }
+// Time of a launch without staging, for the choice between tiles and slices of the streaming kernel: the planner's figure and 5.6 us.  A
+// launch, its set-up and last stores take 4.6 on average on top of the figure (648 products of 17 to 80 tokens, 256 to 6144 features of
+// 256 to 8192, bf16, captured one behind the other: 3.8 to 6.3), but slices take 1.0 to 2.7 times their estimate, and the line is what
+// decides: with 5.6 the slower of the two is taken for 3.8 % on average, with 5.5 sizes beside the line went from the faster one to
+// the slower (64 tokens of 1536 by 1024: 8.9 -> 9.6 us); 4.0 would leave 1.4 %.
+double gemm_trit_tc_estimate_us(int64_t M, int64_t N, int64_t K) { return 5.6 + 1.7e-3 * pick_shape(M, N, K, 1, kRawBytes<1>, true).cost; }
 
 // Scratch bytes for the activations: none when they are read in place.  `planes`: bf16 planes of fp32 activations.
 size_t gemm_trit_tc_scratch_most(int b_dtype, int64_t N, int64_t K, int planes) {
