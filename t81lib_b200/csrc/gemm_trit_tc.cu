@@ -6,7 +6,7 @@
 // its shared memory and loads half of the tile's activation rows by TMA; the even CTA issues the MMAs, which read both
 // halves, and each CTA keeps its 128 accumulator rows in TMEM (2 x 256 fp32 columns, double-buffered across tiles).
 // Measured against the one-CTA 128 x 256 kernel before it (bf16, weights in limbs there and in codes here):
-// 4096 x 14336 x 16384 tokens 958 -> 1529 TFLOP/s in a long run under the power cap, 9216 x 3072 x 2048 109 -> 83 us, 14336 x 4096 x 80
+// 4096 x 14336 x 16384 tokens 958 -> 1506 TFLOP/s in a long run under the power cap, 9216 x 3072 x 2048 109 -> 84 us, 14336 x 4096 x 80
 // 40.9 -> 19.2 us.
 // What bounds the kernel is shared-memory bandwidth: a 64-deep step writes and reads 16 KB of expanded weights per CTA
 // and writes and reads the activations, against 512 clocks of MMA at 256 tokens.  Halving the activation share is what
@@ -358,8 +358,8 @@ gemm_trit_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     const int c0 = p.n_chunks * slice / p.splits, c1 = p.n_chunks * (slice + 1) / p.splits;
     const uint16_t pair_mask = (uint16_t)(3u << (rank & ~1u));
 
-    // The producer's weight loads run two chunks ahead of the activations; the first ones touch nothing but this CTA's
-    // memory and start before the cluster has met.
+    // The producer's weight loads run two chunks ahead of the activations; the first two start right behind the wait for the kernel ahead,
+    // for which the cluster has met already.
     Ring raw_fill, raw_told;
     bool fill_ok = true;
     int raw_tile = cluster_id, raw_c = c0;
@@ -662,9 +662,8 @@ double step_cost(Mode mode, int bn, int planes) {
 // and 3 a token (the steps' costs refitted since: 900 tokens of 3000 by 5000, bf16, 34.3 -> 26.2 us, 400 of 6000 by 3000 25.3 -> 23.4, 200 of 2000
 // by 2000, fp32, 13.7 -> 12.8; 27 others as they were).  Several planes take two accumulators a tile, so tiles that follow one another in a pair are at most
 // 128 tokens wide there (4096 x 4096 x 4096 in two planes 202 us, 208 at 256 tokens with one accumulator); wider ones only where
-// no pair has a second tile (5530 x 11021 x 249: 83 us at 128 tokens, 66 at 256).  The width 160 is left out for several planes:
-// a launch at it (728 tiles, two planes, fp32 result) failed with an unspecified error on a variant of this kernel that had other
-// issuing loops, and the cause is not known.
+// no pair has a second tile (5530 x 11021 x 249: 83 us at 128 tokens, 66 at 256).  The widths between 128 and 192 are left out for several
+// planes: tiles that follow one another have no room for the second accumulator there, and tiles alone have not been measured.
 TcShape pick_shape(int64_t M, int64_t N, int64_t K, int planes, int raw_bytes, bool staged) {
     const int64_t m_tiles = (M + 255) / 256, chunks = (K + CHUNK - 1) / CHUNK, wide = (N + 255) / 256, narrow = (N + 127) / 128;
     const int64_t least = planes > 1 && wide > resident_pair_clusters(1) ? narrow : wide, most = (planes > 1 ? narrow : wide) + 8;
